@@ -55,7 +55,7 @@ extern "C" {
 typedef struct lact_scan_config {
   int64_t B, L, D, H; /* merged batch*heads, tokens, head dim, fast-weight hidden dim */
   int64_t out_len;    /* tokens in o (== L except for operator lists that concatenate applies) */
-  int32_t act_dtype;  /* dtype of q, k, v, o (LACT_BF16; LACT_F32 = split-precision fp32 mode) */
+  int32_t act_dtype;  /* dtype of q, k, v, o (LACT_BF16; LACT_F32: lact_scan_f32_fwd) */
   int32_t lr_dtype;   /* dtype of lr0, lr1, lr2 */
   int32_t mom_dtype;  /* dtype of momentum */
   int32_t w_dtype;    /* dtype of w0, w1, w2 (inputs); outputs and state are always fp32 */
@@ -408,11 +408,18 @@ int lact_momentum_bwd(void *dg0, void *dg1, void *carry0, void *carry1, const vo
                       int32_t add_carry, void *stream);
 
 /* fp32 mode (fp32 activations; the reference's CPU configuration, e.g. bidirectional_lact_layer.py with fp32 inputs):
- * plain FFMA kernels for accuracy, no tensor cores.  The Python package runs the step program with them.
+ * FFMA kernels, no tensor cores.
+ *   lact_scan_f32_fwd: lact_scan_fwd on fp32 q, k, v, o (act_dtype LACT_F32; D a multiple of 4, H of 8, of 8 both with
+ *     Muon); forward only: io.state_dump and io.ns_trace are ignored;
  *   lact_sgemm_f32: c[batch, M, N] = a b^T (+ beta[batch] * c when accumulate; beta NULL = 1), a stored [M][K] (a_t = 0) or [K][M], b stored [N][K] (b_t = 0) or [K][N]
  *     (replaces torch.bmm on fp32 tensors, e.g. ttt_operation.py:141-168);
  *   lact_swiglu_planes_f32: hidden (*lr1) and, when dh is given, dy0*lr0 | dy2*lr2 from y0|y2 (ttt_operation.py:149-160);
  *   lact_add_renorm: w <- renorm((quirk ? g : w) + (x ? x : g)) on fp32 masters (ttt_operation.py:189-200). */
+int lact_scan_f32_workspace_bytes(const lact_scan_config *cfg, int32_t n_steps, const int32_t *kind, const int64_t *start,
+                                  const int64_t *end, size_t *bytes_out);
+int lact_scan_f32_fwd(const lact_scan_config *cfg, const lact_scan_io *io, int32_t n_steps, const int32_t *kind,
+                      const int64_t *start, const int64_t *end, const int64_t *out_start, void *workspace,
+                      size_t workspace_bytes, void *stream);
 int lact_sgemm_f32(const void *a, int32_t a_t, const void *b, int32_t b_t, void *c, int32_t accumulate,
                    const void *beta, int64_t batch, int64_t M, int64_t N, int64_t K, void *stream);
 int lact_swiglu_planes_f32(const void *y02, const void *dh, const void *lr0, const void *lr1, const void *lr2,

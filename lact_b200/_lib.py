@@ -79,6 +79,8 @@ def _declare(lib: C.CDLL) -> None:
     lib.lact_ns_trace_result_offset.restype = C.c_int
     lib.lact_scan_fwd.argtypes = [C.POINTER(ScanConfig), C.POINTER(ScanIO), i32, C.POINTER(i32), C.POINTER(i64),
                                   C.POINTER(i64), C.POINTER(i64), vp, C.c_size_t, vp]
+    lib.lact_scan_f32_workspace_bytes.argtypes = lib.lact_scan_workspace_bytes.argtypes
+    lib.lact_scan_f32_fwd.argtypes = lib.lact_scan_fwd.argtypes
     lib.lact_swiglu_ffn_workspace_bytes.argtypes = [i64, i64, i64, i64, szp]
     lib.lact_swiglu_ffn_fwd.argtypes = [vp, vp, vp, vp, i64, i64, i64, i64, vp, C.c_size_t, vp]
     lib.lact_static_scratch_bytes.restype = C.c_size_t
@@ -125,7 +127,7 @@ def _declare(lib: C.CDLL) -> None:
     lib.lact_swiglu_planes_f32.argtypes = [vp, vp, vp, vp, vp, i32, f32, vp, vp, i64, i64, vp]
     lib.lact_add_renorm.argtypes = [vp, vp, vp, vp, vp, vp, i64, i64, i64, i32, i32, i32, i32, vp]
     for name in ("lact_read_status", "lact_set_wait_limit_ns", "lact_debug_wait_timeout", "lact_static_status",
-                 "lact_scan_workspace_bytes", "lact_scan_fwd", "lact_swiglu_ffn_workspace_bytes",
+                 "lact_scan_workspace_bytes", "lact_scan_fwd", "lact_scan_f32_workspace_bytes", "lact_scan_f32_fwd", "lact_swiglu_ffn_workspace_bytes",
                  "lact_swiglu_ffn_fwd", "lact_fw_grad_workspace_bytes", "lact_fw_grad",
                  "lact_newton_schulz_workspace_bytes", "lact_newton_schulz", "lact_l2_norm_add",
                  "lact_prenorm_momentum_l2norm", "lact_bmm_bf16", "lact_bmm2_bf16", "lact_bmm2_strided_bf16", "lact_swiglu_bwd_planes",

@@ -1,6 +1,7 @@
 """Builds liblact_b200.so in-tree with nvcc for sm_100a (cross-compiles without a GPU)."""
 from __future__ import annotations
 
+import glob
 import os
 import shutil
 import subprocess
@@ -8,7 +9,7 @@ import subprocess
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 SRC = os.path.join(PKG_DIR, "csrc", "lact_b200.cu")
 LIB = os.path.join(PKG_DIR, "liblact_b200.so")
-DEPS = [os.path.join(PKG_DIR, "csrc", f) for f in ("lact_b200.cu", "ops.cuh", "umma_gemm.cuh", "ns_fused.cuh", "ptx.cuh")] + [
+DEPS = sorted(glob.glob(os.path.join(PKG_DIR, "csrc", "*.cu*"))) + [
     os.path.join(os.path.dirname(PKG_DIR), "include", "lact_b200.h")]
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "--shared",

@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "../../include/lact_b200.h"
+#include "f32_gemm.cuh"
 #include "ns_bwd_fused.cuh"
 #include "swa_bwd.cuh"
 
@@ -1075,6 +1076,63 @@ int scan_ns_trace_layout(const lact_scan_config& c, size_t* stride, size_t* g0_b
   return LACT_OK;
 }
 
+// Momentum state the program starts from: the caller's, or zeros.
+int load_momentum_state(const lact_scan_config& c, const lact_scan_io& io, float* G02, float* G1, cudaStream_t stream) {
+  const size_t B = c.B, D = c.D, H = c.H;
+  if (io.m0_in && io.m1_in && io.m2_in) {
+    LACT_CUDA(cudaMemcpy2DAsync(G02, 2 * H * D * 4, io.m0_in, H * D * 4, H * D * 4, B, cudaMemcpyDeviceToDevice, stream));
+    LACT_CUDA(cudaMemcpy2DAsync(G02 + H * D, 2 * H * D * 4, io.m2_in, H * D * 4, H * D * 4, B, cudaMemcpyDeviceToDevice,
+                                stream));
+    LACT_CUDA(cudaMemcpyAsync(G1, io.m1_in, B * D * H * 4, cudaMemcpyDeviceToDevice, stream));
+  } else {
+    LACT_CUDA(cudaMemsetAsync(G02, 0, B * 2 * H * D * 4, stream));
+    LACT_CUDA(cudaMemsetAsync(G1, 0, B * D * H * 4, stream));
+  }
+  return LACT_OK;
+}
+
+// Per-update momentum factors beta[u][b], all UPDATE steps at once.
+int launch_momentum_means(const lact_scan_config& c, const lact_scan_io& io, int32_t n_steps, const int32_t* kind,
+                          const int64_t* start, const int64_t* end, float* beta, cudaStream_t stream) {
+  MeanArgs ma;
+  std::memset(&ma, 0, sizeof(ma));
+  int u = 0, first_u = 0;
+  auto flush = [&]() -> int {
+    if (ma.n == 0) return LACT_OK;
+    KernelScope scope(kClsMomentumMean, stream);
+    momentum_mean_kernel<<<dim3(static_cast<unsigned>(c.B), ma.n), 256, 0, stream>>>(
+        io.momentum, c.mom_dtype == LACT_F32, c.L, ma, beta + first_u * c.B, static_cast<int>(c.B));
+    LACT_CUDA(cudaGetLastError());
+    first_u = u;
+    ma.n = 0;
+    return LACT_OK;
+  };
+  for (int i = 0; i < n_steps; ++i) {
+    if (kind[i] != LACT_STEP_UPDATE) continue;
+    ma.s[ma.n] = static_cast<int32_t>(start[i]);
+    ma.e[ma.n] = static_cast<int32_t>(end[i]);
+    ++ma.n; ++u;
+    if (ma.n == kMeanBatch) LACT_TRY(flush());
+  }
+  return flush();
+}
+
+// Final fast weights and momentum state into the caller's arrays (those that are given).
+int store_state(const lact_scan_config& c, const lact_scan_io& io, const float* W02, const float* W1, const float* G02,
+                const float* G1, cudaStream_t stream) {
+  const size_t B = c.B, D = c.D, H = c.H;
+  auto half = [&](void* dst, const float* src) {
+    return cudaMemcpy2DAsync(dst, H * D * 4, src, 2 * H * D * 4, H * D * 4, B, cudaMemcpyDeviceToDevice, stream);
+  };
+  if (io.w0_out) LACT_CUDA(half(io.w0_out, W02));
+  if (io.w2_out) LACT_CUDA(half(io.w2_out, W02 + H * D));
+  if (io.w1_out) LACT_CUDA(cudaMemcpyAsync(io.w1_out, W1, B * D * H * 4, cudaMemcpyDeviceToDevice, stream));
+  if (io.m0_out) LACT_CUDA(half(io.m0_out, G02));
+  if (io.m2_out) LACT_CUDA(half(io.m2_out, G02 + H * D));
+  if (io.m1_out) LACT_CUDA(cudaMemcpyAsync(io.m1_out, G1, B * D * H * 4, cudaMemcpyDeviceToDevice, stream));
+  return LACT_OK;
+}
+
 int scan_fwd(const lact_scan_config& c, const lact_scan_io& io, int32_t n_steps, const int32_t* kind,
              const int64_t* start, const int64_t* end, const int64_t* out_start, void* workspace, size_t ws_bytes,
              cudaStream_t stream) {
@@ -1115,43 +1173,8 @@ int scan_fwd(const lact_scan_config& c, const lact_scan_io& io, int32_t n_steps,
                                                                   p.n02, p.n1, p.W02b, p.W1b);
     LACT_CUDA(cudaGetLastError());
   }
-  // gradient / momentum state
-  if (io.m0_in && io.m1_in && io.m2_in) {
-    LACT_CUDA(cudaMemcpy2DAsync(p.G02, 2 * H * D * 4, io.m0_in, H * D * 4, H * D * 4, B, cudaMemcpyDeviceToDevice,
-                                stream));
-    LACT_CUDA(cudaMemcpy2DAsync(p.G02 + H * D, 2 * H * D * 4, io.m2_in, H * D * 4, H * D * 4, B,
-                                cudaMemcpyDeviceToDevice, stream));
-    LACT_CUDA(cudaMemcpyAsync(p.G1, io.m1_in, B * D * H * 4, cudaMemcpyDeviceToDevice, stream));
-  } else {
-    LACT_CUDA(cudaMemsetAsync(p.G02, 0, B * 2 * H * D * 4, stream));
-    LACT_CUDA(cudaMemsetAsync(p.G1, 0, B * D * H * 4, stream));
-  }
-
-  // per-update momentum factors, all steps at once
-  if (c.use_momentum) {
-    MeanArgs ma;
-    std::memset(&ma, 0, sizeof(ma));
-    int u = 0;
-    auto flush = [&](int first_u) -> int {
-      if (ma.n == 0) return LACT_OK;
-      KernelScope scope(kClsMomentumMean, stream);
-      momentum_mean_kernel<<<dim3(static_cast<unsigned>(B), ma.n), 256, 0, stream>>>(
-          io.momentum, c.mom_dtype == LACT_F32, c.L, ma, p.beta + static_cast<int64_t>(first_u) * B,
-          static_cast<int>(B));
-      LACT_CUDA(cudaGetLastError());
-      return LACT_OK;
-    };
-    ma.n = 0;
-    int first_u = 0;
-    for (int i = 0; i < n_steps; ++i) {
-      if (kind[i] != LACT_STEP_UPDATE) continue;
-      ma.s[ma.n] = static_cast<int32_t>(start[i]);
-      ma.e[ma.n] = static_cast<int32_t>(end[i]);
-      ++ma.n; ++u;
-      if (ma.n == kMeanBatch) { LACT_TRY(flush(first_u)); first_u = u; ma.n = 0; }
-    }
-    LACT_TRY(flush(first_u));
-  }
+  LACT_TRY(load_momentum_state(c, io, p.G02, p.G1, stream));
+  if (c.use_momentum) LACT_TRY(launch_momentum_means(c, io, n_steps, kind, start, end, p.beta, stream));
 
   // training with Muon: per-update Newton-Schulz traces in the caller's buffer (see lact_scan_ns_trace_bytes)
   size_t ns_trace_stride = 0, ns_trace_g0 = 0;
@@ -1276,18 +1299,212 @@ int scan_fwd(const lact_scan_config& c, const lact_scan_io& io, int32_t n_steps,
       W1cur = rn[1].master;
     }
   }
-  // final state out
-  if (io.w0_out) LACT_CUDA(cudaMemcpy2DAsync(io.w0_out, H * D * 4, p.W02c, 2 * H * D * 4, H * D * 4, B,
-                                             cudaMemcpyDeviceToDevice, stream));
-  if (io.w2_out) LACT_CUDA(cudaMemcpy2DAsync(io.w2_out, H * D * 4, p.W02c + H * D, 2 * H * D * 4, H * D * 4, B,
-                                             cudaMemcpyDeviceToDevice, stream));
-  if (io.w1_out) LACT_CUDA(cudaMemcpyAsync(io.w1_out, p.W1c, B * D * H * 4, cudaMemcpyDeviceToDevice, stream));
-  if (io.m0_out) LACT_CUDA(cudaMemcpy2DAsync(io.m0_out, H * D * 4, G02cur, 2 * H * D * 4, H * D * 4, B,
-                                             cudaMemcpyDeviceToDevice, stream));
-  if (io.m2_out) LACT_CUDA(cudaMemcpy2DAsync(io.m2_out, H * D * 4, G02cur + H * D, 2 * H * D * 4, H * D * 4, B,
-                                             cudaMemcpyDeviceToDevice, stream));
-  if (io.m1_out) LACT_CUDA(cudaMemcpyAsync(io.m1_out, G1cur, B * D * H * 4, cudaMemcpyDeviceToDevice, stream));
+  return store_state(c, io, p.W02c, p.W1c, G02cur, G1cur, stream);
+}
+
+// ------------------------------------------------------------------------------------------
+// fp32 mode: the same step programs on fp32 activations (FFMA contractions, f32_gemm.cuh)
+// ------------------------------------------------------------------------------------------
+F32Mat f32_mat(const float* p, int64_t ld, int64_t bs, int t, int64_t rows, int64_t k) {
+  const int64_t contiguous = t ? rows : k;
+  const bool vec = (reinterpret_cast<uintptr_t>(p) & 15) == 0 && (ld % 4) == 0 && (bs % 4) == 0 && (contiguous % 4) == 0;
+  return F32Mat{p, ld, bs, t, vec ? 1 : 0};
+}
+
+template <int MODE>
+int launch_f32_gemm(F32Args& a, cudaStream_t stream) {
+  const dim3 grid(ceil_div(a.N, MODE == kF32Store ? kFN : 32), ceil_div(a.M, kFM), static_cast<unsigned>(a.batch * a.splits));
+  if (a.M < 1 || a.N < 1 || a.K < 1 || grid.y > 65535 || static_cast<int64_t>(a.batch) * a.splits > 65535) return LACT_ERR_SHAPE;
+  KernelScope scope(kClsOther, stream);
+  LACT_CUDA(launch_pdl(f32_gemm_kernel<MODE>, grid, dim3(kFThreads), 0, stream, a));
   return LACT_OK;
+}
+
+// Splits of a token contraction (output R x C per entry, `len` tokens): enough that the grid fills the four CTAs an SM
+// holds, at least 64 tokens each.  At 4 entries of 192 x 192 and 4096 tokens one split would be 24 CTAs.
+int f32_splits(int64_t R, int64_t C, int64_t B, int64_t len) {
+  const int64_t tiles = B * ceil_div(R, kFM) * ceil_div(C, kFN);
+  const int64_t want = (4 * static_cast<int64_t>(sm_count()) + tiles - 1) / tiles;
+  return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>({want, (len + 63) / 64, 64})));
+}
+
+struct ScanF32Plan {
+  int32_t* status;
+  float *W02, *W1, *W02c, *W1c, *n02, *n1, *G02, *G1, *beta, *hidden, *dy02, *part02, *part1;
+  NsPlan ns;
+  size_t bytes;
+};
+
+int plan_scan_f32(const lact_scan_config& c, int32_t n_steps, const int32_t* kind, const int64_t* start, const int64_t* end,
+                  void* base, ScanF32Plan* p) {
+  int64_t max_apply = 0, max_update = 0;
+  for (int i = 0; i < n_steps; ++i) {
+    if (start[i] < 0 || end[i] > c.L || end[i] < start[i]) return LACT_ERR_STEPS;
+    const int64_t len = end[i] - start[i];
+    if (kind[i] == LACT_STEP_APPLY) max_apply = std::max(max_apply, len);
+    else if (kind[i] == LACT_STEP_UPDATE) max_update = std::max(max_update, len);
+    else return LACT_ERR_STEPS;
+  }
+  Carver cv(base);
+  const size_t B = c.B, D = c.D, H = c.H;
+  p->status = cv.take<int32_t>(64);
+  p->W02 = cv.take<float>(B * 2 * H * D);
+  p->W1 = cv.take<float>(B * D * H);
+  p->W02c = cv.take<float>(B * 2 * H * D);
+  p->W1c = cv.take<float>(B * D * H);
+  p->n02 = cv.take<float>(B * 2 * H);
+  p->n1 = cv.take<float>(B * D);
+  p->G02 = cv.take<float>(B * 2 * H * D);
+  p->G1 = cv.take<float>(B * D * H);
+  p->beta = cv.take<float>(B * static_cast<size_t>(std::max(1, n_steps)));
+  p->hidden = cv.take<float>(B * static_cast<size_t>(std::max(max_apply, max_update)) * H);
+  p->dy02 = cv.take<float>(B * static_cast<size_t>(max_update) * 2 * H);
+  // (splits grow with the token count: the longest update needs the most)
+  p->part02 = cv.take<float>(max_update > 0 ? static_cast<size_t>(f32_splits(2 * c.H, c.D, c.B, max_update)) * B * 2 * H * D : 0);
+  p->part1 = cv.take<float>(max_update > 0 ? static_cast<size_t>(f32_splits(c.D, c.H, c.B, max_update)) * B * D * H : 0);
+  p->ns.ngroups = 0;
+  if (c.use_muon && max_update > 0) plan_ns(cv, c.B, c.D, c.H, c.ns_concat, c.ns_gram_right, &p->ns);
+  p->bytes = cv.off + 256;
+  return LACT_OK;
+}
+
+int validate_scan_f32(const lact_scan_config& c) {
+  if (c.B < 1 || c.L < 1 || c.D < 4 || c.H < 8 || c.out_len < 0 || (c.D % 4) != 0 || (c.H % 8) != 0) return LACT_ERR_SHAPE;
+  if (c.B > 65535 / 64 || c.L > (1ll << 30)) return LACT_ERR_SHAPE;
+  if (c.act_dtype != LACT_F32) return LACT_ERR_DTYPE;
+  if (c.use_muon) {
+    if (c.ns_steps < 0 || c.ns_steps > 64 || (c.D % 8) != 0) return LACT_ERR_CONFIG;
+    if (!c.ns_const_coeffs && c.ns_steps != 5) return LACT_ERR_CONFIG;
+  }
+  if (c.renorm < 0 || c.renorm > 2) return LACT_ERR_CONFIG;
+  return LACT_OK;
+}
+
+int scan_fwd_f32(const lact_scan_config& c, const lact_scan_io& io, int32_t n_steps, const int32_t* kind, const int64_t* start,
+                 const int64_t* end, const int64_t* out_start, void* workspace, size_t ws_bytes, cudaStream_t stream) {
+  LACT_TRY(check_device());
+  LACT_TRY(validate_scan_f32(c));
+  if (!io.w0 || !io.w1 || !io.w2 || !io.q || !io.k || !io.v || !io.lr0 || !io.lr1 || !io.lr2 || !io.o) return LACT_ERR_NULL;
+  if (c.use_momentum && !io.momentum) return LACT_ERR_NULL;
+  if (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 255) != 0) return LACT_ERR_WORKSPACE;
+  ScanF32Plan p;
+  LACT_TRY(plan_scan_f32(c, n_steps, kind, start, end, workspace, &p));
+  if (p.bytes > ws_bytes) return LACT_ERR_WORKSPACE;
+  for (int i = 0; i < n_steps; ++i)
+    if (kind[i] == LACT_STEP_APPLY && (out_start[i] < 0 || out_start[i] + (end[i] - start[i]) > c.out_len)) return LACT_ERR_STEPS;
+  const int64_t B = c.B, D = c.D, H = c.H;
+  if (D > kRenormMaxCols || H > kRenormMaxCols) return LACT_ERR_SHAPE;
+  LACT_CUDA(cudaMemsetAsync(p.status, 0, 256, stream));
+  {
+    KernelScope scope(kClsPrepare, stream);
+    prepare_weights_kernel<<<ceil_div(B * (2 * H + D), 8), 256, 0, stream>>>(
+        io.w0, io.w1, io.w2, c.w_dtype == LACT_F32, static_cast<int>(B), static_cast<int>(H), static_cast<int>(D), p.W02, p.W1,
+        p.W02c, p.W1c, p.n02, p.n1, nullptr, nullptr);
+    LACT_CUDA(cudaGetLastError());
+  }
+  if (c.use_momentum) LACT_TRY(load_momentum_state(c, io, p.G02, p.G1, stream));
+  if (c.use_momentum) LACT_TRY(launch_momentum_means(c, io, n_steps, kind, start, end, p.beta, stream));
+  const float* W02 = c.prenorm ? p.W02c : p.W02;  // the weights the steps compute with
+  const float* W1 = c.prenorm ? p.W1c : p.W1;
+  const float *q = static_cast<const float*>(io.q), *k = static_cast<const float*>(io.k), *v = static_cast<const float*>(io.v);
+  int update_idx = 0;
+  for (int i = 0; i < n_steps; ++i) {
+    const int64_t len = end[i] - start[i];
+    if (len <= 0) {
+      update_idx += kind[i] == LACT_STEP_UPDATE;
+      continue;
+    }
+    F32Args a;
+    std::memset(&a, 0, sizeof(a));
+    a.batch = static_cast<int32_t>(B);
+    a.splits = 1;
+    a.M = static_cast<int32_t>(len); a.N = static_cast<int32_t>(H); a.K = a.kper = static_cast<int32_t>(D);
+    a.c = p.hidden; a.c_ld = H; a.c_bs = len * H;
+    a.b = f32_mat(W02, D, 2 * H * D, 0, 2 * H, D);
+    if (kind[i] == LACT_STEP_APPLY) {
+      a.a = f32_mat(q + start[i] * c.q_ts, c.q_ts, c.q_bs, 0, len, D);
+      LACT_TRY(launch_f32_gemm<kF32Gate>(a, stream));
+      F32Args d;
+      std::memset(&d, 0, sizeof(d));
+      d.batch = a.batch; d.splits = 1;
+      d.M = a.M; d.N = static_cast<int32_t>(D); d.K = d.kper = static_cast<int32_t>(H);
+      d.a = f32_mat(p.hidden, H, len * H, 0, len, H);
+      d.b = f32_mat(W1, H, D * H, 0, D, H);
+      d.c = static_cast<float*>(io.o) + out_start[i] * c.o_ts; d.c_ld = c.o_ts; d.c_bs = c.o_bs;
+      LACT_TRY(launch_f32_gemm<kF32Store>(d, stream));
+      continue;
+    }
+    const int u = update_idx++;
+    a.a = f32_mat(k + start[i] * c.k_ts, c.k_ts, c.k_bs, 0, len, D);
+    a.a2 = f32_mat(v + start[i] * c.v_ts, c.v_ts, c.v_bs, 0, len, D);
+    a.b2 = f32_mat(W1, H, D * H, 1, H, D);  // dh = v w1: w1 is [D][H], k = D rows
+    a.c2 = p.dy02; a.c2_ld = 2 * H; a.c2_bs = len * 2 * H;
+    const int64_t esz = c.lr_dtype == LACT_F32 ? 4 : 2;
+    auto at = [&](const void* t) { return static_cast<const uint8_t*>(t) + start[i] * esz; };
+    a.lr0 = at(io.lr0); a.lr1 = at(io.lr1); a.lr2 = at(io.lr2);
+    a.lr_f32 = c.lr_dtype == LACT_F32;
+    a.lr_bs = c.L;
+    a.w_scale = c.w_scale;
+    LACT_TRY(launch_f32_gemm<kF32Grad>(a, stream));
+    F32ReduceArgs red;
+    std::memset(&red, 0, sizeof(red));
+    red.batch = static_cast<int32_t>(B);
+    red.accumulate = c.use_momentum;
+    red.beta = c.use_momentum ? p.beta + static_cast<int64_t>(u) * B : nullptr;
+    for (int w = 0; w < 2; ++w) {  // [dw0; dw2] = dy^T k, dw1 = v^T hidden
+      const int64_t R = w == 0 ? 2 * H : D, C = w == 0 ? D : H;
+      F32Args g;
+      std::memset(&g, 0, sizeof(g));
+      g.batch = a.batch;
+      g.M = static_cast<int32_t>(R); g.N = static_cast<int32_t>(C); g.K = static_cast<int32_t>(len);
+      const int splits = f32_splits(R, C, B, len);
+      g.kper = ceil_div(ceil_div(len, splits), kFK) * kFK;
+      g.splits = ceil_div(len, g.kper);
+      if (w == 0) {
+        g.a = f32_mat(p.dy02, 2 * H, len * 2 * H, 1, R, len);
+        g.b = f32_mat(k + start[i] * c.k_ts, c.k_ts, c.k_bs, 1, C, len);
+      } else {
+        g.a = f32_mat(v + start[i] * c.v_ts, c.v_ts, c.v_bs, 1, R, len);
+        g.b = f32_mat(p.hidden, H, len * H, 1, C, len);
+      }
+      g.c = w == 0 ? p.part02 : p.part1;
+      g.c_ld = C; g.c_bs = R * C;
+      LACT_TRY(launch_f32_gemm<kF32Store>(g, stream));
+      red.part[w] = g.c;
+      red.c[w] = w == 0 ? p.G02 : p.G1;
+      red.n[w] = R * C;
+      red.splits[w] = g.splits;
+    }
+    {
+      KernelScope scope(kClsOther, stream);
+      LACT_CUDA(launch_pdl(f32_reduce_kernel, dim3(ceil_div((red.n[0] + red.n[1]) * B / 4, 256)), dim3(256), 0, stream, red));
+    }
+    const bf16* xres[2] = {nullptr, nullptr};
+    if (c.use_muon) {
+      const void* srcs[2] = {p.G02, p.G1};
+      LACT_TRY(launch_ns_prepare(p.ns.grp, 2, srcs, 1, 1, stream));
+      int rc = try_ns_fused(p.ns.grp, 2, c.ns_steps, c.ns_const_coeffs, p.status, stream, xres);
+      if (rc == LACT_ERR_CONFIG)
+        rc = run_ns_iterations(p.ns.grp, 2, c.ns_steps, c.ns_const_coeffs, xres, p.status, stream);
+      LACT_TRY(rc);
+    }
+    RenormArgs rn[2];
+    for (int w = 0; w < 2; ++w) {
+      RenormArgs& r = rn[w];
+      std::memset(&r, 0, sizeof(r));
+      r.R = static_cast<int>(w == 0 ? 2 * H : D); r.C = static_cast<int>(w == 0 ? D : H);
+      r.B = static_cast<int>(B);
+      r.master = w == 0 ? p.W02 : p.W1;
+      r.compute = !c.prenorm ? nullptr : (w == 0 ? p.W02c : p.W1c);
+      r.n0 = w == 0 ? p.n02 : p.n1;
+      r.g = w == 0 ? p.G02 : p.G1;
+      r.x = xres[w];
+      r.x_bs = static_cast<int64_t>(r.R) * r.C;
+      r.mode = c.renorm; r.prenorm = c.prenorm; r.prenorm_bf16 = c.prenorm_bf16; r.quirk = c.overwrite_quirk;
+    }
+    LACT_TRY(launch_add_renorm(rn[0], rn[1], stream));
+  }
+  return store_state(c, io, W02, W1, p.G02, p.G1, stream);
 }
 
 }  // namespace
@@ -1420,6 +1637,24 @@ int lact_scan_fwd(const lact_scan_config* cfg, const lact_scan_io* io, int32_t n
   if (!cfg || !io || (n_steps > 0 && (!kind || !start || !end || !out_start))) return LACT_ERR_NULL;
   return scan_fwd(*cfg, *io, n_steps, kind, start, end, out_start, workspace, workspace_bytes,
                   static_cast<cudaStream_t>(stream));
+}
+
+int lact_scan_f32_workspace_bytes(const lact_scan_config* cfg, int32_t n_steps, const int32_t* kind, const int64_t* start,
+                                  const int64_t* end, size_t* bytes_out) {
+  if (!cfg || !bytes_out || (n_steps > 0 && (!kind || !start || !end))) return LACT_ERR_NULL;
+  LACT_TRY(validate_scan_f32(*cfg));
+  ScanF32Plan p;
+  LACT_TRY(plan_scan_f32(*cfg, n_steps, kind, start, end, nullptr, &p));
+  *bytes_out = p.bytes;
+  return LACT_OK;
+}
+
+int lact_scan_f32_fwd(const lact_scan_config* cfg, const lact_scan_io* io, int32_t n_steps, const int32_t* kind,
+                      const int64_t* start, const int64_t* end, const int64_t* out_start, void* workspace,
+                      size_t workspace_bytes, void* stream) {
+  if (!cfg || !io || (n_steps > 0 && (!kind || !start || !end || !out_start))) return LACT_ERR_NULL;
+  return scan_fwd_f32(*cfg, *io, n_steps, kind, start, end, out_start, workspace, workspace_bytes,
+                      static_cast<cudaStream_t>(stream));
 }
 
 // ---------------------------------------------------------------- sub-ops
@@ -2338,15 +2573,19 @@ int lact_momentum_bwd(void* dg0, void* dg1, void* carry0, void* carry1, const vo
 int lact_sgemm_f32(const void* a, int32_t a_t, const void* b, int32_t b_t, void* c, int32_t accumulate,
                    const void* beta, int64_t batch, int64_t M, int64_t N, int64_t K, void* stream) {
   if (!a || !b || !c) return LACT_ERR_NULL;
-  if (batch < 1 || batch > 65535 || M < 1 || N < 1 || K < 1) return LACT_ERR_SHAPE;
-  dim3 grid(ceil_div(N, 64), ceil_div(M, 64), static_cast<unsigned>(batch));
-  if (grid.y > 65535) return LACT_ERR_SHAPE;
-  KernelScope scope(kClsOther, static_cast<cudaStream_t>(stream));
-  sgemm_f32_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const float*>(a), a_t, static_cast<const float*>(b), b_t, static_cast<float*>(c), accumulate,
-      static_cast<const float*>(beta), static_cast<int>(M), static_cast<int>(N), static_cast<int>(K));
-  LACT_CUDA(cudaGetLastError());
-  return LACT_OK;
+  if (batch < 1 || batch > 65535 || M < 1 || N < 1 || K < 1 || M > (1ll << 30) || N > (1ll << 30) || K > (1ll << 30))
+    return LACT_ERR_SHAPE;
+  F32Args g;
+  std::memset(&g, 0, sizeof(g));
+  g.a = f32_mat(static_cast<const float*>(a), a_t ? M : K, M * K, a_t ? 1 : 0, M, K);
+  g.b = f32_mat(static_cast<const float*>(b), b_t ? N : K, N * K, b_t ? 1 : 0, N, K);
+  g.M = static_cast<int32_t>(M); g.N = static_cast<int32_t>(N); g.K = g.kper = static_cast<int32_t>(K);
+  g.batch = static_cast<int32_t>(batch);
+  g.splits = 1;
+  g.c = static_cast<float*>(c); g.c_ld = N; g.c_bs = M * N;
+  g.accumulate = accumulate;
+  g.beta = static_cast<const float*>(beta);
+  return launch_f32_gemm<kF32Store>(g, static_cast<cudaStream_t>(stream));
 }
 
 int lact_swiglu_planes_f32(const void* y02, const void* dh, const void* lr0, const void* lr1, const void* lr2,

@@ -499,7 +499,7 @@ __global__ void prepare_weights_kernel(const void* w0, const void* w1, const voi
     ss += x * x;
     dm[doff + c] = x;
     dc[doff + c] = x;
-    db[doff + c] = __float2bfloat16_rn(x);
+    if (db != nullptr) db[doff + c] = __float2bfloat16_rn(x);
   }
   ss = warp_sum(ss);
   if (lane == 0) *dn = sqrtf(ss);
@@ -675,7 +675,7 @@ struct RenormArgs {
   float* master;     // [B][R][C] fp32, in/out
   const float* master_in;  // nullptr, or where the current master is read from (`master` is then written only)
   float* compute;    // [B][R][C] fp32 out (may be nullptr): the weights the next step computes with
-  bf16* shadow;      // [B][R][C] bf16 out
+  bf16* shadow;      // [B][R][C] bf16 out (nullptr in fp32 mode)
   const float* n0;   // [B][R]
   const float* g;    // [B][R][C] fp32 gradient (after momentum)
   const bf16* x;     // Newton-Schulz result in the weight's own orientation, or nullptr (update = g)
@@ -735,7 +735,8 @@ __device__ __forceinline__ void renorm_row(const RenormArgs& a, int64_t row, int
       const float4 yv = make_float4(y[0], y[1], y[2], y[3]);
       *reinterpret_cast<float4*>(a.master + off + c) = a.prenorm ? w[i] : yv;
       if (a.compute != nullptr) *reinterpret_cast<float4*>(a.compute + off + c) = yv;
-      *reinterpret_cast<uint2*>(a.shadow + off + c) = make_uint2(pack_bf16x2(y[0], y[1]), pack_bf16x2(y[2], y[3]));
+      if (a.shadow != nullptr)
+        *reinterpret_cast<uint2*>(a.shadow + off + c) = make_uint2(pack_bf16x2(y[0], y[1]), pack_bf16x2(y[2], y[3]));
     }
   }
 }
@@ -1047,59 +1048,8 @@ __global__ void __launch_bounds__(1024) momentum_bwd_kernel(const MomentumBwdArg
 }
 
 // ------------------------------------------------------------------------------------------
-// fp32 mode (parity path for fp32 activations): plain FFMA kernels, no tensor cores.
-// tcgen05 has no fp32 x fp32 MMA; this path exists for accuracy (max relative error ~1e-6 when
-// Muon is off), not for throughput.
+// fp32 mode: pointwise stages as kernels of their own (the recurrence itself fuses them, f32_gemm.cuh)
 // ------------------------------------------------------------------------------------------
-// c[b][m][n] = sum_k A(b, m, k) * B(b, n, k) (+ beta[b] * c[b][m][n] when accumulating; beta = 1
-// without a beta vector); A stored [M][K] (a_t = 0) or [K][M] (a_t = 1), B stored [N][K] (b_t = 0)
-// or [K][N] (b_t = 1); all contiguous.  64 x 64 tile, 256 threads, 4 x 4 per thread.
-__global__ void __launch_bounds__(256) sgemm_f32_kernel(const float* A, int a_t, const float* B, int b_t, float* C,
-                                                        int accumulate, const float* beta, int M, int N, int K) {
-  __shared__ float As[16][65];
-  __shared__ float Bs[16][65];
-  const int b = blockIdx.z;
-  A += static_cast<int64_t>(b) * M * K;
-  B += static_cast<int64_t>(b) * N * K;
-  C += static_cast<int64_t>(b) * M * N;
-  const float cb = beta != nullptr ? beta[b] : 1.f;
-  const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  float acc[4][4] = {};
-  for (int k0 = 0; k0 < K; k0 += 16) {
-    for (int i = threadIdx.x; i < 16 * 64; i += 256) {
-      const int kk = a_t ? i / 64 : i % 16, mm = a_t ? i % 64 : i / 16;
-      const int gm = m0 + mm, gk = k0 + kk;
-      As[kk][mm] = (gm < M && gk < K) ? (a_t ? A[static_cast<int64_t>(gk) * M + gm] : A[static_cast<int64_t>(gm) * K + gk]) : 0.f;
-      const int kb = b_t ? i / 64 : i % 16, nn = b_t ? i % 64 : i / 16;
-      const int gn = n0 + nn, gkb = k0 + kb;
-      Bs[kb][nn] = (gn < N && gkb < K) ? (b_t ? B[static_cast<int64_t>(gkb) * N + gn] : B[static_cast<int64_t>(gn) * K + gkb]) : 0.f;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < 16; ++kk) {
-      float a[4], bb[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) { a[i] = As[kk][ty * 4 + i]; bb[i] = Bs[kk][tx * 4 + i]; }
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], bb[j], acc[i][j]);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int gm = m0 + ty * 4 + i, gn = n0 + tx * 4 + j;
-      if (gm < M && gn < N) {
-        float* o = C + static_cast<int64_t>(gm) * N + gn;
-        *o = accumulate ? fmaf(*o, cb, acc[i][j]) : acc[i][j];
-      }
-    }
-}
-
 // fp32 planes: hidden = silu(y0) * y2 (lr pointers null and dh null), or the lr-weighted gradient
 // planes (hidden*lr1, dy0*lr0, dy2*lr2).  Exact expf / division.  One warp per token row.
 __global__ void __launch_bounds__(256) swiglu_planes_f32_kernel(const float* y02, const float* dh, const void* lr0,

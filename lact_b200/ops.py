@@ -3,7 +3,7 @@
 Same names, positional order, keyword defaults and return types as the reference functions
 (cited per function); the arithmetic runs in the sm_100a kernels of liblact_b200.so through the
 C ABI.  bf16 activations run the fused tcgen05 program (with a training backward); fp32 activations
-run the accuracy path of `fp32_mode` (forward only).
+run the same programs on the FP32 pipes (forward only).
 """
 from __future__ import annotations
 
@@ -49,6 +49,14 @@ def _act(t: torch.Tensor, name: str) -> torch.Tensor:
     return t
 
 
+def _act_f32(t: torch.Tensor, name: str) -> torch.Tensor:
+    if t.dim() != 3:
+        raise ValueError(f"{name} must be [b, l, d]")
+    if t.stride(2) != 1 or t.stride(1) % 4 or t.stride(0) % 4 or t.data_ptr() % 16:
+        t = t.contiguous()
+    return t
+
+
 def _vec(t: torch.Tensor, B: int, Ltok: int, name: str) -> torch.Tensor:
     """[b, l, 1] or [b, l] per-token scalar -> contiguous [b, l] in fp32 or bf16."""
     if t.dim() == 3:
@@ -78,13 +86,10 @@ def scan_eager(w0, w1, w2, q, k, v, lr0, lr1, lr2, steps: Sequence[P.Step], *, o
     """Forward of the general chunk recurrence, straight through the C ABI (`lact_scan_fwd`), no
     autograd.  `scan` is the public, differentiable and compilable entry point."""
     dev = _need_cuda(w0, w1, w2, q, k, v, lr0, lr1, lr2, momentum)
-    if q.dtype == k.dtype == v.dtype == torch.float32:
-        return _scan_f32(dev, w0, w1, w2, q, k, v, lr0, lr1, lr2, steps, out_len, momentum, m_init,
-                         dict(use_muon=use_muon, ns_steps=ns_steps, ns_const_coeffs=ns_const_coeffs,
-                              ns_concat=ns_concat, ns_gram_right=ns_gram_right, renorm=renorm, prenorm=prenorm,
-                              prenorm_bf16=prenorm_bf16, overwrite_quirk=overwrite_quirk, w_scale=w_scale,
-                              return_state=return_state, return_momentum=return_momentum), _state_dump)
-    q, k, v = _act(q, "q"), _act(k, "k"), _act(v, "v")
+    f32 = q.dtype == k.dtype == v.dtype == torch.float32   # fp32 mode: FFMA contractions, forward only
+    if f32 and _state_dump is not None:
+        raise NotImplementedError("the per-update state dump is a bf16-mode feature")
+    q, k, v = ((_act_f32 if f32 else _act)(t, n) for t, n in ((q, "q"), (k, "k"), (v, "v")))
     B, Ltok, D = k.shape
     H = w0.shape[1]
     if q.shape[0] != B or q.shape[2] != D or v.shape != k.shape:
@@ -112,11 +117,11 @@ def scan_eager(w0, w1, w2, q, k, v, lr0, lr1, lr2, steps: Sequence[P.Step], *, o
             break
         covered = max(covered, s_[1])
     full = full and covered >= out_len
-    o = (torch.empty if full else torch.zeros)(B, out_len, D, dtype=BF16, device=dev)
+    o = (torch.empty if full else torch.zeros)(B, out_len, D, dtype=q.dtype, device=dev)
 
     cfg = L.ScanConfig()
     cfg.B, cfg.L, cfg.D, cfg.H, cfg.out_len = B, Ltok, D, H, out_len
-    cfg.act_dtype = L.LACT_BF16
+    cfg.act_dtype = L.LACT_F32 if f32 else L.LACT_BF16
     cfg.lr_dtype = L.dtype_code(lr0)
     cfg.mom_dtype = L.dtype_code(momentum) if momentum is not None else L.LACT_F32
     cfg.w_dtype = L.dtype_code(w0)
@@ -137,7 +142,9 @@ def scan_eager(w0, w1, w2, q, k, v, lr0, lr1, lr2, steps: Sequence[P.Step], *, o
     outs = (C.c_int64 * n)(*[s[3] for s in steps])
     lib = L.lib()
     need = C.c_size_t(0)
-    L.check(lib.lact_scan_workspace_bytes(C.byref(cfg), n, kind, start, end, C.byref(need)), "lact_scan_workspace_bytes")
+    query, forward = (lib.lact_scan_f32_workspace_bytes, lib.lact_scan_f32_fwd) if f32 else \
+        (lib.lact_scan_workspace_bytes, lib.lact_scan_fwd)
+    L.check(query(C.byref(cfg), n, kind, start, end, C.byref(need)), "lact_scan_workspace_bytes")
     ws = L.workspace(need.value, dev)
 
     io = L.ScanIO()
@@ -167,8 +174,8 @@ def scan_eager(w0, w1, w2, q, k, v, lr0, lr1, lr2, steps: Sequence[P.Step], *, o
                torch.empty(B, H, D, dtype=torch.float32, device=dev))
         io.m0_out, io.m1_out, io.m2_out = (t.data_ptr() for t in mom)
     with torch.cuda.device(dev):
-        L.check(lib.lact_scan_fwd(C.byref(cfg), C.byref(io), n, kind, start, end, outs, ws.data_ptr(), ws.numel(),
-                                  L.stream_ptr()), "lact_scan_fwd")
+        L.check(forward(C.byref(cfg), C.byref(io), n, kind, start, end, outs, ws.data_ptr(), ws.numel(), L.stream_ptr()),
+                "lact_scan_fwd")
     L.mark_pending(ws)
     res = [o]
     if return_state:
@@ -194,26 +201,6 @@ def ns_trace_layout(B, Ltok, D, H, opts) -> Tuple[int, int]:
     if rc != 0:
         return 0, 0
     return int(stride.value), int(off.value)
-
-
-def _scan_f32(dev, w0, w1, w2, q, k, v, lr0, lr1, lr2, steps, out_len, momentum, m_init, opts, state_dump):
-    """fp32 activations: validate as `scan` does and run the step program in `fp32_mode`."""
-    from .fp32_mode import scan_f32
-    if state_dump is not None:
-        raise NotImplementedError("the per-update state dump is a bf16-mode feature")
-    for t, name in ((q, "q"), (k, "k"), (v, "v")):
-        if t.dim() != 3:
-            raise ValueError(f"{name} must be [b, l, d]")
-    B, Ltok, D = k.shape
-    H = w0.shape[1]
-    if q.shape[0] != B or q.shape[2] != D or v.shape != k.shape or q.shape[1] != Ltok:
-        raise ValueError("q, k, v shapes disagree")
-    w0, w1, w2 = _weight(w0, (B, H, D), "w0"), _weight(w1, (B, D, H), "w1"), _weight(w2, (B, H, D), "w2")
-    lr0, lr1, lr2 = (_vec(t, B, Ltok, n).float() for t, n in ((lr0, "lr0"), (lr1, "lr1"), (lr2, "lr2")))
-    if momentum is not None:
-        momentum = _vec(momentum, B, Ltok, "momentum")
-    return scan_f32(w0, w1, w2, q, k, v, lr0, lr1, lr2, steps, out_len=out_len, momentum=momentum, m_init=m_init,
-                    **opts)
 
 
 # ----------------------------------------------------------------------------------------------
