@@ -90,6 +90,9 @@ typedef struct lact_scan_io {
    * lact_ns_trace_bwd reads (lact_scan_ns_trace_bytes per step; 256-byte aligned), so that the backward does not
    * recompute them; or NULL */
   void *ns_trace;
+  /* training: the bf16 copies of the weights, [w0w2 | w1] per slot: slot 0 the initial weights, slot u the weights after
+   * update u (number of UPDATE steps + 1 slots); or NULL */
+  void *shadow_dump;
 } lact_scan_io;
 
 /* Library version (major * 1000 + minor).  No counterpart in the reference. */
@@ -129,6 +132,10 @@ int64_t lact_stream_sync_count(void);
  * time-out path can be exercised without any fault: `status_word` (device memory, zero before
  * the call) holds 101 once the kernel has run.  No counterpart in the reference. */
 int lact_set_wait_limit_ns(uint64_t limit_ns);
+/* A word of pinned host memory (one per device, made at the first call) in which every kernel that records a non-zero
+ * device status also leaves it: a host that reads it now and then learns of a failure without copies or waits.  The
+ * host clears it.  Make the first call outside stream capture.  No counterpart in the reference. */
+int lact_status_host_word(int32_t **word_out);
 int lact_debug_wait_timeout(int32_t *status_word, void *stream);
 
 /* Scratch bytes needed by lact_scan_fwd for this configuration and step list. */
@@ -160,6 +167,11 @@ int lact_scan_fwd(const lact_scan_config *cfg, const lact_scan_io *io, int32_t n
 int lact_swiglu_ffn_workspace_bytes(int64_t B, int64_t N, int64_t D, int64_t H, size_t *bytes_out);
 int lact_swiglu_ffn_fwd(const void *w0w2, const void *w1, const void *x, void *out, int64_t B, int64_t N,
                         int64_t D, int64_t H, void *workspace, size_t workspace_bytes, void *stream);
+
+/* lact_swiglu_ffn_fwd with its scratch and its status word given one by one: hidden = bf16 [B, N, H]; status_word = device
+ * word the caller has cleared (it is not cleared here, so that consecutive calls can share one). */
+int lact_swiglu_ffn_apply(const void *w0w2, const void *w1, const void *x, void *out, void *hidden, int64_t B, int64_t N,
+                          int64_t D, int64_t H, int32_t *status_word, void *stream);
 
 /* The same computation as lact_swiglu_ffn_fwd for callers that must not allocate and cannot hand
  * over a workspace.  No counterpart in the reference.
@@ -251,6 +263,19 @@ int lact_qkv_prologue_rope(const void *xq, const void *xk, const void *xv, int64
 int lact_lr_prologue(const void *lr_proj, int32_t proj_dtype, int64_t proj_ld, float base_lr_inv, const void *mom_logits,
                      int32_t logits_dtype, int64_t logits_ld, void *lr0, void *lr1, void *lr2, void *momentum, int64_t b,
                      int64_t s, int64_t n_heads, void *stream);
+
+/* Backward of lact_lr_prologue: g0, g1, g2, gm = gradients of its outputs (fp32 [(b n_heads)][s], NULL = zero), dproj
+ * [b][s][3 n_heads] and dlogits [b][s][n_heads] contiguous in the projections' dtypes, written. */
+int lact_lr_prologue_bwd(const void *lr_proj, int32_t proj_dtype, int64_t proj_ld, float base_lr_inv, const void *mom_logits,
+                         int32_t logits_dtype, int64_t logits_ld, const void *g0, const void *g1, const void *g2, const void *gm,
+                         void *dproj, void *dlogits, int64_t b, int64_t s, int64_t n_heads, void *stream);
+
+/* out[cols] = sums of the columns of x [rows][cols] (fp32, fixed order): adds the partial rows of lact_out_epilogue_bwd. */
+int lact_column_sums(const float *x, float *out, int64_t rows, int64_t cols, void *stream);
+
+/* out[t] = first token of the packed sequence token t belongs to, from cu_seqlens (int32 [n_sequences + 1], device): the
+ * seq_start argument of the prologue and of attention. */
+int lact_seq_start(const int32_t *cu_seqlens, int64_t n_sequences, int64_t n_tokens, int32_t *out, void *stream);
 
 /* Causal sliding-window attention forward, the other half of each hybrid layer, on the same q / k / v layout as
  * the layer's projections: o[b, l, h, d] = softmax over keys (i - window, i] of q_i . k_j * softmax_scale, times v.
@@ -374,7 +399,9 @@ int lact_swiglu_bwd_planes(const void *y02, const void *dh, const void *lr0, con
 int lact_fw_grad_bwd_pointwise(const void *y02, const void *dh, const void *g_dy02, const void *g_hid,
                                const void *lr0, const void *lr1, const void *lr2, int32_t lr_dtype, float w_scale,
                                void *g_y02, void *g_dh, void *dy02, void *hid, void *g_lr0, void *g_lr1, void *g_lr2,
-                               int64_t rows, int64_t H, void *stream);
+                               int64_t B, int64_t n, int64_t H,
+                               int64_t lr_bs, int64_t g_lr_bs /* batch strides of lr* and g_lr* (token stride 1) */,
+                               int32_t g_lr_add /* 1: add to g_lr* */, void *stream);
 int lact_renorm_bwd(const void *base, const void *upd, int32_t upd_dtype, const void *n0, const void *dy, void *dw,
                     void *dw_bf16 /* optional bf16 copy of dw, or NULL */, void *dn0, int64_t rows, int64_t C,
                     int32_t mode, void *stream);
@@ -383,8 +410,8 @@ int lact_renorm_bwd(const void *base, const void *upd, int32_t upd_dtype, const 
  *     dx0 [nmat][n] (fp32, in/out) <- dx0 / den - bf16(g) <dx0, bf16(g)> / (den^2 nrm), nrm = bf16(||bf16(g)||),
  *     den = bf16(nrm + 1e-7), g [nmat][n] fp32;
  *   lact_momentum_bwd: momentum step (ttt_operation.py:170-179) for both gradient arrays (n0, n1 fp32 elements per
- *     batch entry): dg += carry (if add_carry); sum over s of dbeta[b][s] = <dg, mprev> (mprev NULL at the first update);
- *     carry <- dg * beta[b]; dgb = bf16(dg).  carry / beta NULL: no momentum (bf16 copy only). */
+ *     batch entry), d = dg (+ carry if add_carry): sum over s of dbeta[b][s] = <d, mprev> (mprev NULL at the first
+ *     update); carry <- d * beta[b]; dgb = bf16(d).  carry / beta NULL: no momentum (bf16 copy only). */
 /* The same backward for one or two groups of matrices (e.g. the [w0; w2] and the w1 gradients of one update) in ONE
  * cooperative launch, followed by the normalisation backward: dg = d loss / d G (fp32, written).  Needs the trace of
  * lact_ns_trace_fwd / the training scan (steps <= 5).  LACT_ERR_CONFIG when no fused instantiation covers the shapes:
@@ -403,9 +430,21 @@ int lact_ns_trace_bwd_fused(const lact_ns_bwd_group *groups, int32_t ngroups, in
 int lact_ns_norm_bwd(const void *g, void *dx0, void *partials /* fp32 scratch, nmat * 2 * lact_momentum_bwd_slices() */,
                      int64_t nmat, int64_t elems_per_matrix, void *stream);
 int lact_momentum_bwd_slices(void); /* slices per batch entry: dbeta of lact_momentum_bwd is [B][slices] partial sums */
-int lact_momentum_bwd(void *dg0, void *dg1, void *carry0, void *carry1, const void *mprev0, const void *mprev1,
+int lact_momentum_bwd(const void *dg0, const void *dg1, void *carry0, void *carry1, const void *mprev0, const void *mprev1,
                       void *dgb0, void *dgb1, const void *beta, void *dbeta, int64_t B, int64_t n0, int64_t n1,
                       int32_t add_carry, void *stream);
+
+/* Ends of the reverse sweep: momentum factors beta[n][B] = mean of momentum[b, start:end] per update
+ * (ttt_operation.py:170-172), the gradient of the momentum gate from dbeta [n][B][slices] (every token of [B, L] written),
+ * and the gradients of the initial weights (caller's layout and dtype) from the stacked state gradients: dW (+ dWm)
+ * + dn[row] * W / n[row] (dn NULL: target norms detached). */
+int lact_momentum_means(const void *momentum, int32_t dtype, int64_t B, int64_t L, int32_t n, const int64_t *start,
+                        const int64_t *end, float *beta, void *stream);
+int lact_momentum_gate_grad(const float *dbeta, int64_t B, int64_t L, int32_t n, const int64_t *start, const int64_t *end,
+                            void *out, int32_t out_dtype, void *stream);
+int lact_weight_grad(const float *dW02, const float *dW1, const float *dWm02, const float *dWm1, const float *dn02,
+                     const float *dn1, const float *n02, const float *n1, const float *W02, const float *W1, void *dw0,
+                     void *dw1, void *dw2, int32_t dtype, int64_t B, int64_t D, int64_t H, void *stream);
 
 /* fp32 mode (fp32 activations; the reference's CPU configuration, e.g. bidirectional_lact_layer.py with fp32 inputs):
  * FFMA kernels, no tensor cores.

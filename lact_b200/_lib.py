@@ -6,12 +6,13 @@ from __future__ import annotations
 
 import ctypes as C
 import os
-from typing import Dict, Optional
+from typing import Optional
 
 import torch
 
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(PKG_DIR, "liblact_b200.so")
+OPS_PATH = os.path.join(PKG_DIR, "liblact_b200_torch.so")
 
 LACT_F32, LACT_BF16 = 0, 1
 RENORM_NONE, RENORM_EPS_OUTSIDE, RENORM_EPS_INSIDE = 0, 1, 2
@@ -28,7 +29,7 @@ class ScanConfig(C.Structure):
 class ScanIO(C.Structure):
     _fields_ = [(n, C.c_void_p) for n in ("w0", "w1", "w2", "q", "k", "v", "lr0", "lr1", "lr2", "momentum", "m0_in",
                                           "m1_in", "m2_in", "o", "w0_out", "w1_out", "w2_out", "m0_out", "m1_out",
-                                          "m2_out", "state_dump", "ns_trace")]
+                                          "m2_out", "state_dump", "ns_trace", "shadow_dump")]
 
 
 ERR_CONFIG = -5  # LACT_ERR_CONFIG
@@ -103,8 +104,7 @@ def _declare(lib: C.CDLL) -> None:
     lib.lact_lr_prologue.argtypes = [vp, i32, i64, f32, vp, i32, i64, vp, vp, vp, vp, i64, i64, i64, vp]
     lib.lact_out_epilogue.argtypes = [vp, vp, vp, i64, vp, i64, vp, i64, i64, i64, i64, i64, f32, vp]
     lib.lact_swiglu_bwd_planes.argtypes = [vp, vp, vp, vp, vp, i32, f32, vp, vp, i64, i64, vp]
-    lib.lact_fw_grad_bwd_pointwise.argtypes = [vp, vp, vp, vp, vp, vp, vp, i32, f32, vp, vp, vp, vp, vp, vp, vp, i64,
-                                               i64, vp]
+    lib.lact_fw_grad_bwd_pointwise.argtypes = [vp] * 7 + [i32, f32] + [vp] * 7 + [i64] * 5 + [i32, vp]
     lib.lact_renorm_bwd.argtypes = [vp, vp, i32, vp, vp, vp, vp, vp, i64, i64, i32, vp]
     lib.lact_ns_norm_bwd.argtypes = [vp, vp, vp, i64, i64, vp]
     lib.lact_momentum_bwd_slices.restype = C.c_int
@@ -149,6 +149,43 @@ def lib() -> C.CDLL:
     return _lib
 
 
+# The registered operators (torch.ops.lact_b200) live in a second library on top of the first.
+_ops_loaded = False
+_ops_lib: Optional[C.CDLL] = None
+
+
+def load_ops() -> None:
+    """Loads the operator library (once) and registers its shape-only implementations.  Raises if it has not been built."""
+    global _ops_loaded, _ops_lib
+    if _ops_loaded:
+        return
+    lib()
+    if not os.path.exists(OPS_PATH):
+        raise ImportError(f"{OPS_PATH} is missing: build it with `python -m lact_b200.build` "
+                          "(there is no fallback implementation)")
+    torch.ops.load_library(OPS_PATH)
+    _ops_lib = C.CDLL(OPS_PATH)
+    _ops_lib.lact_torch_take_status.argtypes = [C.c_int]
+    _ops_lib.lact_torch_take_status.restype = C.c_int
+    from . import _fakes  # noqa: F401
+    _ops_loaded = True
+
+
+def call(op, *args):
+    """One operator call; a device status or a CUDA error the operator reports becomes a LactError."""
+    if torch.compiler.is_compiling():
+        return op(*args)
+    try:
+        out = op(*args)
+    except RuntimeError as e:
+        if str(e).startswith("lact_b200: "):
+            raise LactError(str(e).split("\n", 1)[0]) from None
+        raise
+    if SYNC_CHECK:
+        synchronize_and_check()
+    return out
+
+
 class LactError(RuntimeError):
     pass
 
@@ -174,99 +211,30 @@ def stream_ptr() -> int:
     return torch.cuda.current_stream().cuda_stream
 
 
-# One growing scratch buffer per (device, stream), taken from PyTorch's caching allocator.  Kernels
-# of consecutive calls on one stream are ordered, so reuse is safe.
-_workspaces: Dict[tuple, torch.Tensor] = {}
+# LACT_B200_SYNC_CHECK=1 waits for the device and checks its status after every operator call (debugging).
 SYNC_CHECK = os.environ.get("LACT_B200_SYNC_CHECK", "0") == "1"
 
 
-def _key(device: torch.device) -> tuple:
-    return (device.index if device.index is not None else torch.cuda.current_device(), stream_ptr())
-
-
 def workspace(nbytes: int, device: torch.device) -> torch.Tensor:
-    """Scratch for one call on the current stream.  Never waits for the device."""
-    key = _key(device)
-    buf = _workspaces.get(key)
-    if buf is None or buf.numel() < nbytes:
-        buf = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
-        _workspaces[key] = buf
-    return buf
+    """Scratch for one call on the current stream, from PyTorch's caching allocator (stream-ordered: giving it back right
+    after the call has been enqueued is safe)."""
+    return torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
 
 
-class _StatusRing:
-    """Device status words of finished calls, copied to pinned host memory WITHOUT waiting.
-
-    Every call's kernels leave a status word at the head of its workspace (0 = ok, 101 = a bounded
-    wait ran out).  The next call on the stream clears that word, so right after a call has been
-    enqueued an asynchronous 4-byte copy into the next slot of a pinned ring is enqueued behind
-    it.  The host looks at slots whose copy has completed (an event query, no wait) whenever a
-    later call is made, and at all of them in `synchronize_and_check`.  A slot is waited for only
-    when the ring wraps around while its copy is still in flight (256 calls ahead of the device).
-    """
-    SLOTS = 256
-
-    def __init__(self):
-        self.host = torch.zeros(self.SLOTS, dtype=torch.int32).pin_memory()
-        self.events = [None] * self.SLOTS
-        self.head = 0  # next slot to use
-        self.tail = 0  # oldest slot not yet examined
-
-    def _examine(self, slot: int) -> None:
-        self.events[slot] = None
-        st = int(self.host[slot])
-        if st != 0:
-            self.host[slot] = 0
-            raise LactError("device status: " + lib().lact_error_string(st).decode() + f" (code {st})")
-
-    def poll(self, wait: bool = False) -> None:
-        """Examines finished slots in order; with `wait`, all of them."""
-        while self.tail != self.head:
-            slot = self.tail % self.SLOTS
-            ev = self.events[slot]
-            if ev is not None:
-                if wait:
-                    ev.synchronize()
-                elif not ev.query():
-                    return
-            self.tail += 1
-            self._examine(slot)
-
-    def post(self, ws: torch.Tensor) -> None:
-        if self.head - self.tail >= self.SLOTS:  # the ring is full: the oldest copy must have landed
-            slot = self.tail % self.SLOTS
-            if self.events[slot] is not None:
-                self.events[slot].synchronize()
-            self.tail += 1
-            self._examine(slot)
-        slot = self.head % self.SLOTS
-        self.host[slot:slot + 1].copy_(ws[:4].view(torch.int32), non_blocking=True)
-        ev = torch.cuda.Event()
-        ev.record()
-        self.events[slot] = ev
-        self.head += 1
-
-
-_rings: Dict[int, _StatusRing] = {}
+def _take_status(index: int) -> None:
+    load_ops()
+    st = _ops_lib.lact_torch_take_status(index)
+    if st != 0:
+        raise LactError("device status: " + lib().lact_error_string(st).decode() + f" (code {st})")
 
 
 def mark_pending(ws: torch.Tensor) -> None:
-    """Called after a library call has been enqueued with `ws` as its workspace: arranges for the
-    call's device status word to reach the host without blocking (see `_StatusRing`), and raises
-    for any EARLIER call whose word has arrived non-zero.  Inside CUDA-graph stream capture
-    nothing is recorded.  LACT_B200_SYNC_CHECK=1 checks synchronously instead (debugging)."""
-    if torch.cuda.is_current_stream_capturing():
-        return
+    """Called after a library call has been enqueued with `ws` as its workspace.  Kernels that give up leave their status
+    in a word of mapped host memory (`lact_status_host_word`): reading it here raises for any EARLIER call that has
+    failed by now, without copies, events or waits."""
     if SYNC_CHECK:
         read_status(ws)
-        return
-    idx = ws.device.index
-    ring = _rings.get(idx)
-    if ring is None:
-        ring = _rings[idx] = _StatusRing()
-    with torch.cuda.device(ws.device):
-        ring.post(ws)
-        ring.poll()
+    _take_status(ws.device.index)
 
 
 def read_status(ws: torch.Tensor) -> None:
@@ -277,11 +245,15 @@ def read_status(ws: torch.Tensor) -> None:
 
 
 def synchronize_and_check() -> None:
-    """Waits for every status word posted so far and raises if any call recorded a device-side
-    error (a bounded wait that ran out).  The op calls themselves never wait."""
-    for idx, ring in list(_rings.items()):
-        with torch.cuda.device(idx):
-            ring.poll(wait=True)
+    """Waits for the work enqueued so far and raises if any call recorded a device-side error (a bounded wait that ran
+    out).  The op calls themselves never wait."""
+    if not _ops_loaded or not torch.cuda.is_initialized():
+        return
+    for idx in range(torch.cuda.device_count()):
+        if torch.cuda.device_count() > 1 and torch.cuda.memory_reserved(idx) == 0:
+            continue
+        torch.cuda.synchronize(idx)
+        _take_status(idx)
 
 
 def stream_sync_count() -> int:

@@ -1076,10 +1076,12 @@ int scan_ns_trace_layout(const lact_scan_config& c, size_t* stride, size_t* g0_b
   return LACT_OK;
 }
 
-// Momentum state the program starts from: the caller's, or zeros.
+// Momentum state the program starts from: the caller's.  Without one the first update has nothing to add to its gradient
+// (it runs without a momentum factor), and zeros are written only for a program that hands the state back untouched.
+inline bool has_initial_momentum(const lact_scan_io& io) { return io.m0_in && io.m1_in && io.m2_in; }
 int load_momentum_state(const lact_scan_config& c, const lact_scan_io& io, float* G02, float* G1, cudaStream_t stream) {
   const size_t B = c.B, D = c.D, H = c.H;
-  if (io.m0_in && io.m1_in && io.m2_in) {
+  if (has_initial_momentum(io)) {
     LACT_CUDA(cudaMemcpy2DAsync(G02, 2 * H * D * 4, io.m0_in, H * D * 4, H * D * 4, B, cudaMemcpyDeviceToDevice, stream));
     LACT_CUDA(cudaMemcpy2DAsync(G02 + H * D, 2 * H * D * 4, io.m2_in, H * D * 4, H * D * 4, B, cudaMemcpyDeviceToDevice,
                                 stream));
@@ -1151,7 +1153,6 @@ int scan_fwd(const lact_scan_config& c, const lact_scan_io& io, int32_t n_steps,
       return LACT_ERR_STEPS;
 
   const int64_t B = c.B, D = c.D, H = c.H;
-  LACT_CUDA(cudaMemsetAsync(p.status, 0, 256, stream));
   // Training (post-norm): the per-update state the backward needs is not copied out, it LIVES in the caller's dump:
   // update u reads its master weights from slot u and writes the new ones into slot u + 1 (the last update into the
   // workspace), and the gradient / momentum state of update u is written into slot u while slot u - 1 is read.
@@ -1162,6 +1163,10 @@ int scan_fwd(const lact_scan_config& c, const lact_scan_io& io, int32_t n_steps,
   auto slot = [&](int u) { return static_cast<float*>(io.state_dump) + static_cast<size_t>(u) * 2 * (n02 + n1); };
   float* W02cur = dump_in_place ? slot(0) : p.W02;   // master weights in force
   float* W1cur = dump_in_place ? slot(0) + n02 : p.W1;
+  // bf16 copies of the weights in force (MMA operands); training keeps those of every update in the caller's buffer
+  bf16 *W02b = p.W02b, *W1b = p.W1b;
+  auto shadow_slot = [&](int u) { return static_cast<bf16*>(io.shadow_dump) + static_cast<size_t>(u) * (n02 + n1); };
+  if (io.shadow_dump != nullptr) { W02b = shadow_slot(0); W1b = W02b + n02; }
   float* G02cur = p.G02;                              // gradient / momentum state after the latest update
   float* G1cur = p.G1;
   {
@@ -1170,10 +1175,10 @@ int scan_fwd(const lact_scan_config& c, const lact_scan_io& io, int32_t n_steps,
     prepare_weights_kernel<<<ceil_div(rows, 8), 256, 0, stream>>>(io.w0, io.w1, io.w2, c.w_dtype == LACT_F32,
                                                                   static_cast<int>(B), static_cast<int>(H),
                                                                   static_cast<int>(D), W02cur, W1cur, p.W02c, p.W1c,
-                                                                  p.n02, p.n1, p.W02b, p.W1b);
+                                                                  p.n02, p.n1, W02b, W1b, p.status);
     LACT_CUDA(cudaGetLastError());
   }
-  LACT_TRY(load_momentum_state(c, io, p.G02, p.G1, stream));
+  if (has_initial_momentum(io) || n_updates == 0) LACT_TRY(load_momentum_state(c, io, p.G02, p.G1, stream));
   if (c.use_momentum) LACT_TRY(launch_momentum_means(c, io, n_steps, kind, start, end, p.beta, stream));
 
   // training with Muon: per-update Newton-Schulz traces in the caller's buffer (see lact_scan_ns_trace_bytes)
@@ -1185,12 +1190,13 @@ int scan_fwd(const lact_scan_config& c, const lact_scan_io& io, int32_t n_steps,
   int update_idx = 0;
   for (int i = 0; i < n_steps; ++i) {
     if (kind[i] == LACT_STEP_APPLY) {
-      ApplyArgs a{p.W02b, p.W1b, io.q, c.q_bs, c.q_ts, start[i], end[i], io.o, c.o_bs, c.o_ts, out_start[i],
+      ApplyArgs a{W02b, W1b, io.q, c.q_bs, c.q_ts, start[i], end[i], io.o, c.o_bs, c.o_ts, out_start[i],
                   p.hidden, B, D, H};
       LACT_TRY(run_apply(a, p.status, stream));
       continue;
     }
-    const float* beta = c.use_momentum ? p.beta + static_cast<int64_t>(update_idx) * B : nullptr;
+    const float* beta = c.use_momentum && (update_idx > 0 || has_initial_momentum(io))
+                            ? p.beta + static_cast<int64_t>(update_idx) * B : nullptr;
     float* dump = nullptr;
     if (io.state_dump != nullptr && !dump_in_place) {
       // training (pre-norm): the weights this update computed with and (below) its gradient after momentum are copied
@@ -1207,7 +1213,7 @@ int scan_fwd(const lact_scan_config& c, const lact_scan_io& io, int32_t n_steps,
       G1cur = slot(update_idx) + 2 * n02 + n1;
     }
     ++update_idx;
-    GradArgs g{p.W02b, p.W1b, io.k, io.v, c.k_bs, c.k_ts, c.v_bs, c.v_ts, start[i], end[i], io.lr0, io.lr1, io.lr2,
+    GradArgs g{W02b, W1b, io.k, io.v, c.k_bs, c.k_ts, c.v_bs, c.v_ts, start[i], end[i], io.lr0, io.lr1, io.lr2,
                c.lr_dtype == LACT_F32, c.L, c.w_scale, p.dy02, p.hid, G02cur, G1cur, 1, beta, B, D, H};
     g.g02_prev = G02prev;
     g.g1_prev = G1prev;
@@ -1237,7 +1243,8 @@ int scan_fwd(const lact_scan_config& c, const lact_scan_io& io, int32_t n_steps,
     }
 
     // add + renormalise arguments (the update is the Newton-Schulz result when Muon is on)
-    const bool want_compute = c.prenorm || !has_later_update(kind, n_steps, i);
+    // (the fp32 copy of the normalised weights is what pre-norm computes with and what the final export reads)
+    const bool want_compute = c.prenorm || (io.w0_out != nullptr && !has_later_update(kind, n_steps, i));
     RenormArgs rn[2];
     for (int w = 0; w < 2; ++w) {
       RenormArgs& r = rn[w];
@@ -1250,7 +1257,8 @@ int scan_fwd(const lact_scan_config& c, const lact_scan_io& io, int32_t n_steps,
         if (update_idx < n_updates) r.master = w == 0 ? slot(update_idx) : slot(update_idx) + n02;
       }
       r.compute = want_compute ? (w == 0 ? p.W02c : p.W1c) : nullptr;
-      r.shadow = w == 0 ? p.W02b : p.W1b;
+      r.shadow = w == 0 ? W02b : W1b;
+      if (io.shadow_dump != nullptr) r.shadow = w == 0 ? shadow_slot(update_idx) : shadow_slot(update_idx) + n02;
       r.n0 = w == 0 ? p.n02 : p.n1;
       r.g = w == 0 ? G02cur : G1cur;
       r.x = nullptr;
@@ -1294,6 +1302,8 @@ int scan_fwd(const lact_scan_config& c, const lact_scan_io& io, int32_t n_steps,
       rn[1].x = xres[1];
     }
     LACT_TRY(launch_add_renorm(rn[0], rn[1], stream));
+    W02b = rn[0].shadow;
+    W1b = rn[1].shadow;
     if (dump_in_place) {
       W02cur = rn[0].master;
       W1cur = rn[1].master;
@@ -1394,15 +1404,14 @@ int scan_fwd_f32(const lact_scan_config& c, const lact_scan_io& io, int32_t n_st
     if (kind[i] == LACT_STEP_APPLY && (out_start[i] < 0 || out_start[i] + (end[i] - start[i]) > c.out_len)) return LACT_ERR_STEPS;
   const int64_t B = c.B, D = c.D, H = c.H;
   if (D > kRenormMaxCols || H > kRenormMaxCols) return LACT_ERR_SHAPE;
-  LACT_CUDA(cudaMemsetAsync(p.status, 0, 256, stream));
   {
     KernelScope scope(kClsPrepare, stream);
     prepare_weights_kernel<<<ceil_div(B * (2 * H + D), 8), 256, 0, stream>>>(
         io.w0, io.w1, io.w2, c.w_dtype == LACT_F32, static_cast<int>(B), static_cast<int>(H), static_cast<int>(D), p.W02, p.W1,
-        p.W02c, p.W1c, p.n02, p.n1, nullptr, nullptr);
+        p.W02c, p.W1c, p.n02, p.n1, nullptr, nullptr, p.status);
     LACT_CUDA(cudaGetLastError());
   }
-  if (c.use_momentum) LACT_TRY(load_momentum_state(c, io, p.G02, p.G1, stream));
+  if (has_initial_momentum(io) || io.m0_out) LACT_TRY(load_momentum_state(c, io, p.G02, p.G1, stream));
   if (c.use_momentum) LACT_TRY(launch_momentum_means(c, io, n_steps, kind, start, end, p.beta, stream));
   const float* W02 = c.prenorm ? p.W02c : p.W02;  // the weights the steps compute with
   const float* W1 = c.prenorm ? p.W1c : p.W1;
@@ -1449,8 +1458,8 @@ int scan_fwd_f32(const lact_scan_config& c, const lact_scan_io& io, int32_t n_st
     F32ReduceArgs red;
     std::memset(&red, 0, sizeof(red));
     red.batch = static_cast<int32_t>(B);
-    red.accumulate = c.use_momentum;
-    red.beta = c.use_momentum ? p.beta + static_cast<int64_t>(u) * B : nullptr;
+    red.accumulate = c.use_momentum && (u > 0 || has_initial_momentum(io));
+    red.beta = red.accumulate ? p.beta + static_cast<int64_t>(u) * B : nullptr;
     for (int w = 0; w < 2; ++w) {  // [dw0; dw2] = dy^T k, dw1 = v^T hidden
       const int64_t R = w == 0 ? 2 * H : D, C = w == 0 ? D : H;
       F32Args g;
@@ -1590,6 +1599,26 @@ int lact_read_status(const void* workspace, void* stream) {
 
 int64_t lact_stream_sync_count(void) { return g_stream_syncs.load(); }
 
+int lact_status_host_word(int32_t** word_out) {
+  if (!word_out) return LACT_ERR_NULL;
+  static std::mutex mu;
+  static int32_t* words[64] = {nullptr};
+  int dev = 0;
+  LACT_CUDA(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64) return LACT_ERR_DEVICE;
+  std::lock_guard<std::mutex> lock(mu);
+  if (words[dev] == nullptr) {
+    void *h = nullptr, *d = nullptr;
+    LACT_CUDA(cudaHostAlloc(&h, sizeof(int32_t), cudaHostAllocMapped | cudaHostAllocPortable));
+    *static_cast<int32_t*>(h) = 0;
+    LACT_CUDA(cudaHostGetDevicePointer(&d, h, 0));
+    LACT_CUDA(cudaMemcpyToSymbol(g_host_status, &d, sizeof(d)));
+    words[dev] = static_cast<int32_t*>(h);
+  }
+  *word_out = words[dev];
+  return LACT_OK;
+}
+
 int lact_set_wait_limit_ns(uint64_t limit_ns) {
   if (limit_ns == 0) limit_ns = kDefaultWaitLimitNs;
   LACT_CUDA(cudaMemcpyToSymbol(g_wait_limit_ns, &limit_ns, sizeof(limit_ns)));
@@ -1603,7 +1632,7 @@ __global__ void wait_timeout_probe_kernel(int32_t* status) {
   if (threadIdx.x == 0) {
     mbar_init(&bar, 1);
     fence_mbar_init();
-    if (!mbar_wait(&bar, 0)) atomicCAS(status, kStatusOk, kStatusWaitTimeout);
+    if (!mbar_wait(&bar, 0)) report_timeout(status);
   }
 }
 
@@ -1683,6 +1712,16 @@ int lact_swiglu_ffn_fwd(const void* w0w2, const void* w1, const void* x, void* o
   ApplyArgs a{static_cast<const bf16*>(w0w2), static_cast<const bf16*>(w1), x, N * D, D, 0, N, out, N * D, D, 0,
               reinterpret_cast<bf16*>(static_cast<uint8_t*>(workspace) + 256), B, D, H};
   return run_apply(a, static_cast<int32_t*>(workspace), s);
+}
+
+int lact_swiglu_ffn_apply(const void* w0w2, const void* w1, const void* x, void* out, void* hidden, int64_t B, int64_t N,
+                          int64_t D, int64_t H, int32_t* status_word, void* stream) {
+  if (!w0w2 || !w1 || !x || !out || !hidden || !status_word) return LACT_ERR_NULL;
+  LACT_TRY(check_device());
+  LACT_TRY(check_dims(B, N, D, H));
+  const ApplyArgs a{static_cast<const bf16*>(w0w2), static_cast<const bf16*>(w1), x, N * D, D, 0, N, out, N * D, D, 0,
+                    static_cast<bf16*>(hidden), B, D, H};
+  return run_apply(a, status_word, static_cast<cudaStream_t>(stream));
 }
 
 // ---------------------------------------------------------------- allocation-free variant
@@ -2117,6 +2156,50 @@ int lact_lr_prologue(const void* lr_proj, int32_t proj_dtype, int64_t proj_ld, f
   return LACT_OK;
 }
 
+int lact_lr_prologue_bwd(const void* lr_proj, int32_t proj_dtype, int64_t proj_ld, float base_lr_inv, const void* mom_logits,
+                         int32_t logits_dtype, int64_t logits_ld, const void* g0, const void* g1, const void* g2, const void* gm,
+                         void* dproj, void* dlogits, int64_t b, int64_t s, int64_t n_heads, void* stream) {
+  if (!lr_proj || !dproj || ((mom_logits == nullptr) != (dlogits == nullptr))) return LACT_ERR_NULL;
+  LACT_TRY(check_device());
+  if (b < 1 || s < 1 || n_heads < 1 || b > 65535 || s > (1ll << 30) || n_heads > 4096) return LACT_ERR_SHAPE;
+  if (proj_ld < 3 * n_heads || (mom_logits && logits_ld < n_heads)) return LACT_ERR_SHAPE;
+  LrPrologueBwdArgs a;
+  std::memset(&a, 0, sizeof(a));
+  a.proj = lr_proj; a.logits = mom_logits;
+  a.proj_f32 = proj_dtype == LACT_F32; a.logits_f32 = logits_dtype == LACT_F32;
+  a.proj_ld = proj_ld; a.logits_ld = logits_ld;
+  a.base_lr_inv = base_lr_inv;
+  a.g[0] = static_cast<const float*>(g0); a.g[1] = static_cast<const float*>(g1); a.g[2] = static_cast<const float*>(g2);
+  a.gm = static_cast<const float*>(gm);
+  a.dproj = dproj; a.dlogits = dlogits;
+  a.b = static_cast<int32_t>(b); a.s = static_cast<int32_t>(s); a.n_h = static_cast<int32_t>(n_heads);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  KernelScope scope(kClsOther, st);
+  lr_prologue_bwd_kernel<<<static_cast<unsigned>(ceil_div(b * s * n_heads, 256)), 256, 0, st>>>(a);
+  LACT_CUDA(cudaGetLastError());
+  return LACT_OK;
+}
+
+int lact_column_sums(const float* x, float* out, int64_t rows, int64_t cols, void* stream) {
+  if (!x || !out) return LACT_ERR_NULL;
+  if (rows < 1 || cols < 1 || cols > (1ll << 30)) return LACT_ERR_SHAPE;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  KernelScope scope(kClsOther, st);
+  column_sums_kernel<<<static_cast<unsigned>(ceil_div(cols, 32)), 256, 0, st>>>(x, out, rows, cols);
+  LACT_CUDA(cudaGetLastError());
+  return LACT_OK;
+}
+
+int lact_seq_start(const int32_t* cu_seqlens, int64_t n_sequences, int64_t n_tokens, int32_t* out, void* stream) {
+  if (!cu_seqlens || !out) return LACT_ERR_NULL;
+  if (n_sequences < 1 || n_tokens < 1 || n_tokens > (1ll << 30)) return LACT_ERR_SHAPE;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  KernelScope scope(kClsOther, st);
+  seq_start_kernel<<<static_cast<unsigned>(ceil_div(n_tokens, 256)), 256, 0, st>>>(cu_seqlens, n_sequences, n_tokens, out);
+  LACT_CUDA(cudaGetLastError());
+  return LACT_OK;
+}
+
 int lact_out_epilogue(const void* fw_x, const void* weight, const void* gate_proj, int64_t gate_ld, const void* resid,
                       int64_t resid_ld, void* out, int64_t out_ld, int64_t b, int64_t s, int64_t n_heads, int64_t d,
                       float eps, void* stream) {
@@ -2454,16 +2537,18 @@ int lact_swiglu_bwd_planes(const void* y02, const void* dh, const void* lr0, con
 
 int lact_fw_grad_bwd_pointwise(const void* y02, const void* dh, const void* g_dy02, const void* g_hid, const void* lr0,
                                const void* lr1, const void* lr2, int32_t lr_dtype, float w_scale, void* g_y02,
-                               void* g_dh, void* dy02, void* hid, void* g_lr0, void* g_lr1, void* g_lr2, int64_t rows,
-                               int64_t H, void* stream) {
+                               void* g_dh, void* dy02, void* hid, void* g_lr0, void* g_lr1, void* g_lr2, int64_t B,
+                               int64_t n, int64_t H, int64_t lr_bs, int64_t g_lr_bs, int32_t g_lr_add, void* stream) {
   if (!y02 || !dh || !g_dy02 || !g_hid || !lr0 || !lr1 || !lr2 || !g_y02 || !g_dh || !dy02 || !hid || !g_lr0 ||
       !g_lr1 || !g_lr2)
     return LACT_ERR_NULL;
-  if (rows < 1 || H < 8 || (H % 8) != 0) return LACT_ERR_SHAPE;  // planes move as 16-byte vectors
-  const PlaneArgs a = make_plane_args(y02, dh, g_dy02, g_hid, lr0, lr1, lr2, lr_dtype, w_scale, dy02, hid, g_y02, g_dh,
-                                      g_lr0, g_lr1, g_lr2, rows, H);
+  if (B < 1 || B > 65535 || n < 1 || H < 8 || (H % 8) != 0) return LACT_ERR_SHAPE;  // planes move as 16-byte vectors
+  const int64_t rows = B * n;
+  PlaneArgs a = make_plane_args(y02, dh, g_dy02, g_hid, lr0, lr1, lr2, lr_dtype, w_scale, dy02, hid, g_y02, g_dh,
+                                g_lr0, g_lr1, g_lr2, rows, H);
+  a.n = n; a.lr_bs = lr_bs; a.g_lr_bs = g_lr_bs; a.g_lr_add = g_lr_add;
   KernelScope scope(kClsOther, static_cast<cudaStream_t>(stream));
-  fw_grad_bwd_pointwise_kernel<<<ceil_div(rows, 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(a);
+  fw_grad_bwd_pointwise_kernel<<<dim3(ceil_div(n, 8), static_cast<unsigned>(B)), 256, 0, static_cast<cudaStream_t>(stream)>>>(a);
   LACT_CUDA(cudaGetLastError());
   return LACT_OK;
 }
@@ -2547,7 +2632,7 @@ int lact_ns_trace_bwd_fused(const lact_ns_bwd_group* groups, int32_t ngroups, in
 
 int lact_momentum_bwd_slices(void) { return kNormBwdSlices; }
 
-int lact_momentum_bwd(void* dg0, void* dg1, void* carry0, void* carry1, const void* mprev0, const void* mprev1,
+int lact_momentum_bwd(const void* dg0, const void* dg1, void* carry0, void* carry1, const void* mprev0, const void* mprev1,
                       void* dgb0, void* dgb1, const void* beta, void* dbeta, int64_t B, int64_t n0, int64_t n1,
                       int32_t add_carry, void* stream) {
   if (!dg0 || !dg1 || !dgb0 || !dgb1) return LACT_ERR_NULL;
@@ -2555,7 +2640,7 @@ int lact_momentum_bwd(void* dg0, void* dg1, void* carry0, void* carry1, const vo
   if (B < 1 || B > 65535 * 16 || n0 < 4 || n1 < 4 || (n0 % 4) != 0 || (n1 % 4) != 0) return LACT_ERR_SHAPE;
   MomentumBwdArgs a;
   std::memset(&a, 0, sizeof(a));
-  a.dg[0] = static_cast<float*>(dg0); a.dg[1] = static_cast<float*>(dg1);
+  a.dg[0] = static_cast<const float*>(dg0); a.dg[1] = static_cast<const float*>(dg1);
   a.carry[0] = static_cast<float*>(carry0); a.carry[1] = static_cast<float*>(carry1);
   a.mprev[0] = static_cast<const float*>(mprev0); a.mprev[1] = static_cast<const float*>(mprev1);
   a.dgb[0] = static_cast<bf16*>(dgb0); a.dgb[1] = static_cast<bf16*>(dgb1);
@@ -2565,6 +2650,60 @@ int lact_momentum_bwd(void* dg0, void* dg1, void* carry0, void* carry1, const vo
   a.add_carry = add_carry;
   KernelScope scope(kClsOther, static_cast<cudaStream_t>(stream));
   momentum_bwd_kernel<<<dim3(static_cast<unsigned>(B), kNormBwdSlices), 512, 0, static_cast<cudaStream_t>(stream)>>>(a);
+  LACT_CUDA(cudaGetLastError());
+  return LACT_OK;
+}
+
+int lact_momentum_means(const void* momentum, int32_t dtype, int64_t B, int64_t L, int32_t n, const int64_t* start,
+                        const int64_t* end, float* beta, void* stream) {
+  if (!momentum || !beta || (n > 0 && (!start || !end))) return LACT_ERR_NULL;
+  if (B < 1 || B > 65535 || L < 1 || n < 0) return LACT_ERR_SHAPE;
+  for (int32_t i = 0; i < n; ++i)
+    if (start[i] < 0 || end[i] > L || end[i] <= start[i]) return LACT_ERR_STEPS;
+  lact_scan_config c;
+  std::memset(&c, 0, sizeof(c));
+  c.B = B; c.L = L; c.mom_dtype = dtype;
+  lact_scan_io io;
+  std::memset(&io, 0, sizeof(io));
+  io.momentum = momentum;
+  const std::vector<int32_t> kind(static_cast<size_t>(n), LACT_STEP_UPDATE);
+  return launch_momentum_means(c, io, n, kind.data(), start, end, beta, static_cast<cudaStream_t>(stream));
+}
+
+int lact_momentum_gate_grad(const float* dbeta, int64_t B, int64_t L, int32_t n, const int64_t* start, const int64_t* end,
+                            void* out, int32_t out_dtype, void* stream) {
+  if (!dbeta || !out || (n > 0 && (!start || !end))) return LACT_ERR_NULL;
+  if (B < 1 || B > 65535 || L < 1 || n < 0) return LACT_ERR_SHAPE;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  int first = 0;
+  do {
+    MeanArgs ma;
+    std::memset(&ma, 0, sizeof(ma));
+    ma.n = std::min(kMeanBatch, n - first);
+    for (int i = 0; i < ma.n; ++i) {
+      ma.s[i] = static_cast<int32_t>(start[first + i]);
+      ma.e[i] = static_cast<int32_t>(end[first + i]);
+    }
+    KernelScope scope(kClsOther, s);
+    momentum_gate_grad_kernel<<<dim3(ceil_div(L, 256), static_cast<unsigned>(B)), 256, 0, s>>>(
+        ma, dbeta, kNormBwdSlices, static_cast<int>(B), first, first > 0, out, out_dtype == LACT_F32, L);
+    LACT_CUDA(cudaGetLastError());
+    first += kMeanBatch;
+  } while (first < n);
+  return LACT_OK;
+}
+
+int lact_weight_grad(const float* dW02, const float* dW1, const float* dWm02, const float* dWm1, const float* dn02,
+                     const float* dn1, const float* n02, const float* n1, const float* W02, const float* W1, void* dw0,
+                     void* dw1, void* dw2, int32_t dtype, int64_t B, int64_t D, int64_t H, void* stream) {
+  if (!dW02 || !dW1 || !dw0 || !dw1 || !dw2 || ((dWm02 == nullptr) != (dWm1 == nullptr))) return LACT_ERR_NULL;
+  if (dn02 != nullptr && (!dn1 || !n02 || !n1 || !W02 || !W1)) return LACT_ERR_NULL;
+  if (B < 1 || D < 1 || H < 1 || B * (2 * H + D) > (1ll << 33)) return LACT_ERR_SHAPE;
+  const WeightGradArgs a{dW02, dW1, dWm02, dWm1, dn02, dn1, n02, n1, W02, W1, dw0, dw1, dw2, dtype == LACT_F32,
+                         static_cast<int32_t>(B), static_cast<int32_t>(H), static_cast<int32_t>(D)};
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  KernelScope scope(kClsOther, s);
+  weight_grad_kernel<<<ceil_div(B * (2 * H + D), 8), 256, 0, s>>>(a);
   LACT_CUDA(cudaGetLastError());
   return LACT_OK;
 }

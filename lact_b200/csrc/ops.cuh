@@ -462,12 +462,13 @@ __device__ __forceinline__ float warp_sum(float x) {
 
 // Splits the caller's w0, w1, w2 into the internal state: fp32 masters W02 = [w0; w2] ([B,2H,D])
 // and W1 ([B,D,H]), their row norms n0, the fp32 compute copies and the bf16 shadows.
-// One warp per weight row.
+// One warp per weight row.  Also clears the program's status word.
 __global__ void prepare_weights_kernel(const void* w0, const void* w1, const void* w2, int w_f32, int B, int H, int D,
                                        float* W02, float* W1, float* W02c, float* W1c, float* n02, float* n1,
-                                       bf16* W02b, bf16* W1b) {
+                                       bf16* W02b, bf16* W1b, int32_t* status) {
   griddep_launch_dependents();
   griddep_wait();
+  if (blockIdx.x == 0 && threadIdx.x == 0) *status = kStatusOk;  // the first kernel of a program
   const int rows_per_b = 2 * H + D;
   const int64_t r = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (r >= static_cast<int64_t>(B) * rows_per_b) return;
@@ -768,9 +769,12 @@ struct PlaneArgs {
   bf16* hid;    // out [rows][H]: hidden*lr1
   bf16* g_y02;  // out [rows][2H] (second-order only)
   bf16* g_dh;   // out [rows][H]  (second-order only)
-  float *g_lr0, *g_lr1, *g_lr2;  // out [rows] (second-order only)
+  float *g_lr0, *g_lr1, *g_lr2;  // out (second-order only), indexed like the learning rates
   int64_t rows;
   int32_t H;
+  // second-order kernel: row = entry * n + token; learning rates and their gradients at entry * bs + token
+  int64_t n, lr_bs, g_lr_bs;
+  int32_t g_lr_add;              // 1: the learning-rate gradients are added to what is there
 };
 
 // eight consecutive bf16 values as floats / back (16-byte accesses; column counts here are multiples of 8)
@@ -823,12 +827,14 @@ __global__ void __launch_bounds__(256) swiglu_bwd_planes_kernel(const PlaneArgs 
 //   g_y0 = g_hid*A*y2*l1 + g_dy0*A'*y2*dh*l0 + g_dy2*A*dh*l2,   g_y2 = g_hid*sw*l1 + g_dy0*A*dh*l0,
 //   g_dh = g_dy0*A*y2*l0 + g_dy2*sw*l2,   g_lr = row sums (deterministic: one warp per row).
 __global__ void __launch_bounds__(256, 4) fw_grad_bwd_pointwise_kernel(const PlaneArgs a) {
-  const int64_t row = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (row >= a.rows) return;
+  // grid (token blocks, entries)
+  const int64_t entry = blockIdx.y, tok = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (tok >= a.n) return;
   const int lane = threadIdx.x & 31;
-  const float l0 = load_scalar(a.lr0, a.lr_f32, row) * a.w_scale;
-  const float l1 = load_scalar(a.lr1, a.lr_f32, row) * a.w_scale;
-  const float l2 = load_scalar(a.lr2, a.lr_f32, row) * a.w_scale;
+  const int64_t row = entry * a.n + tok, li = entry * a.lr_bs + tok;
+  const float l0 = load_scalar(a.lr0, a.lr_f32, li) * a.w_scale;
+  const float l1 = load_scalar(a.lr1, a.lr_f32, li) * a.w_scale;
+  const float l2 = load_scalar(a.lr2, a.lr_f32, li) * a.w_scale;
   const int H = a.H;
   float s0 = 0.f, s1 = 0.f, s2 = 0.f;
   for (int c = lane * 8; c < H; c += 256) {
@@ -864,9 +870,10 @@ __global__ void __launch_bounds__(256, 4) fw_grad_bwd_pointwise_kernel(const Pla
   }
   s0 = warp_sum(s0); s1 = warp_sum(s1); s2 = warp_sum(s2);
   if (lane == 0) {
-    a.g_lr0[row] = s0 * a.w_scale;
-    a.g_lr1[row] = s1 * a.w_scale;
-    a.g_lr2[row] = s2 * a.w_scale;
+    const int64_t gi = entry * a.g_lr_bs + tok;
+    a.g_lr0[gi] = s0 * a.w_scale + (a.g_lr_add ? a.g_lr0[gi] : 0.f);
+    a.g_lr1[gi] = s1 * a.w_scale + (a.g_lr_add ? a.g_lr1[gi] : 0.f);
+    a.g_lr2[gi] = s2 * a.w_scale + (a.g_lr_add ? a.g_lr2[gi] : 0.f);
   }
 }
 
@@ -1001,12 +1008,13 @@ __global__ void __launch_bounds__(512) ns_norm_bwd_apply_kernel(const float* g, 
 }
 
 // Momentum step of the reverse sweep for one batch entry per block, over the two gradient arrays (n0 and n1 elements
-// per entry):  dG += carry (the gradient that reaches this update's momentum state from the NEXT update, if any);
-// dbeta[b] = <dG, Mprev> (Mprev: momentum state before this update, or nullptr at the first update);
-// carry <- dG * beta[b] (what reaches the previous update's state); and a bf16 copy of dG for the contractions of
-// the fast-weight-gradient backward.  beta == nullptr: no momentum (only dG += 0 and the bf16 copy).
+// per entry), with d = dG + carry (the gradient that reaches this update's momentum state from the NEXT update, if any):
+// dbeta[b] = <d, Mprev> (Mprev: momentum state before this update, or nullptr at the first update);
+// carry <- d * beta[b] (what reaches the previous update's state); and bf16(d) for the contractions of the
+// fast-weight-gradient backward.  dG itself is only read: nothing else needs d in fp32.  beta == nullptr: no momentum
+// (only the bf16 copy).
 struct MomentumBwdArgs {
-  float* dg[2];          // in/out
+  const float* dg[2];
   float* carry[2];       // in/out, or nullptr when there is no momentum
   const float* mprev[2]; // or nullptr
   bf16* dgb[2];          // out
@@ -1032,7 +1040,6 @@ __global__ void __launch_bounds__(1024) momentum_bwd_kernel(const MomentumBwdArg
       if (a.carry[w] != nullptr && a.add_carry) {
         const float4 c = *reinterpret_cast<const float4*>(a.carry[w] + off + i);
         d.x += c.x; d.y += c.y; d.z += c.z; d.w += c.w;
-        *reinterpret_cast<float4*>(a.dg[w] + off + i) = d;
       }
       if (a.mprev[w] != nullptr) {
         const float4 m = *reinterpret_cast<const float4*>(a.mprev[w] + off + i);
@@ -1045,6 +1052,65 @@ __global__ void __launch_bounds__(1024) momentum_bwd_kernel(const MomentumBwdArg
   }
   block_sum2(dot, unused, scratch);
   if (threadIdx.x == 0 && a.dbeta != nullptr) a.dbeta[b * gridDim.y + blockIdx.y] = dot;
+}
+
+// Gradient of the momentum gate: token t of entry b receives sum over updates u whose range [s_u, e_u) holds t of
+// sum_slices dbeta[u][b][slice] / (e_u - s_u).  Grid (token blocks, entries); `first` = index of the launch's first
+// update; `add`: 0 writes (also the tokens no update covers), 1 adds (programs of more than kMeanBatch updates).
+__global__ void __launch_bounds__(256) momentum_gate_grad_kernel(const MeanArgs ma, const float* dbeta, int slices, int B,
+                                                                 int first, int add, void* out, int out_f32, int64_t L) {
+  __shared__ float per_u[kMeanBatch];
+  const int b = blockIdx.y;
+  for (int u = threadIdx.x; u < ma.n; u += blockDim.x) {
+    float x = 0.f;
+    for (int i = 0; i < slices; ++i) x += dbeta[(static_cast<int64_t>(first + u) * B + b) * slices + i];
+    per_u[u] = x / static_cast<float>(ma.e[u] - ma.s[u]);
+  }
+  __syncthreads();
+  const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (t >= L) return;
+  const int64_t i = b * L + t;
+  float x = add ? load_scalar(out, out_f32, i) : 0.f;
+  for (int u = 0; u < ma.n; ++u)
+    if (t >= ma.s[u] && t < ma.e[u]) x += per_u[u];
+  if (out_f32) static_cast<float*>(out)[i] = x;
+  else static_cast<bf16*>(out)[i] = __float2bfloat16_rn(x);
+}
+
+// End of the reverse sweep: gradients of the initial weights in the caller's layout and dtype,
+//   dw = dW (+ dWm) + dn0[row] * W0 / n0[row]    (the target row norms are functions of the initial weights; dn nullptr: detached)
+// from the stacked state arrays [B][2H][D] / [B][D][H].  One warp per row.
+struct WeightGradArgs {
+  const float *dW02, *dW1, *dWm02, *dWm1;  // dWm: gradient through the un-normalised masters (pre-norm), or nullptr
+  const float *dn02, *dn1;                 // [B][2H], [B][D], or nullptr
+  const float *n02, *n1;
+  const float *W02, *W1;                   // initial weights (read only with dn)
+  void *dw0, *dw1, *dw2;
+  int32_t f32, B, H, D;
+};
+__global__ void __launch_bounds__(256) weight_grad_kernel(const WeightGradArgs a) {
+  const int64_t r = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int rows_per_b = 2 * a.H + a.D;
+  if (r >= static_cast<int64_t>(a.B) * rows_per_b) return;
+  const int lane = threadIdx.x & 31;
+  const int b = static_cast<int>(r / rows_per_b), rr = static_cast<int>(r % rows_per_b);
+  const bool second = rr >= 2 * a.H;
+  const int len = second ? a.H : a.D;
+  const int64_t row = second ? static_cast<int64_t>(b) * a.D + rr - 2 * a.H : static_cast<int64_t>(b) * 2 * a.H + rr;
+  const float* dW = (second ? a.dW1 : a.dW02) + row * len;
+  const float* dWm = second ? a.dWm1 : a.dWm02;
+  const float* W = (second ? a.W1 : a.W02) + row * len;
+  const float k = a.dn02 == nullptr ? 0.f
+                                    : (second ? a.dn1[row] : a.dn02[row]) / fmaxf(second ? a.n1[row] : a.n02[row], 1e-30f);
+  void* out = second ? a.dw1 : (rr < a.H ? a.dw0 : a.dw2);
+  const int64_t off = (second ? row : static_cast<int64_t>(b) * a.H + (rr < a.H ? rr : rr - a.H)) * len;
+  for (int c = lane; c < len; c += 32) {
+    float x = dW[c];
+    if (dWm != nullptr) x += dWm[row * len + c];
+    if (a.dn02 != nullptr) x += k * W[c];
+    if (a.f32) static_cast<float*>(out)[off + c] = x;
+    else static_cast<bf16*>(out)[off + c] = __float2bfloat16_rn(x);
+  }
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1282,6 +1348,77 @@ __global__ void __launch_bounds__(256) lr_prologue_kernel(const LrPrologueArgs a
     const float sg = 1.f / (1.f + expf(-x));
     a.mom[i] = a.logits_f32 ? sg : bf16_round(sg);
   }
+}
+
+// Backward of lr_prologue_kernel: d softplus = sigmoid(x) (1 beyond the threshold of 20), d sigmoid = m (1 - m), on the
+// saved projections.  One thread per (batch, token, head), heads fastest: the three gradients of a head are adjacent in
+// the output row.  A null gradient counts as zero.
+struct LrPrologueBwdArgs {
+  const void *proj, *logits;
+  int32_t proj_f32, logits_f32;
+  int64_t proj_ld, logits_ld;
+  float base_lr_inv;
+  const float *g[3], *gm;  // [(b n_h)][s]
+  void *dproj, *dlogits;   // [b][s][3 n_h], [b][s][n_h] contiguous, in the projections' dtypes
+  int32_t b, s, n_h;
+};
+__global__ void __launch_bounds__(256) lr_prologue_bwd_kernel(const LrPrologueBwdArgs a) {
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= static_cast<int64_t>(a.b) * a.s * a.n_h) return;
+  const int h = static_cast<int>(i % a.n_h);
+  const int64_t row = i / a.n_h;
+  const int64_t bi = row / a.s, tok = row - bi * a.s, gi = (bi * a.n_h + h) * a.s + tok;
+  auto put = [](void* p, int f32, int64_t at, float x) {
+    if (f32) static_cast<float*>(p)[at] = x;
+    else static_cast<bf16*>(p)[at] = __float2bfloat16_rn(x);
+  };
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    const float x = load_scalar(a.proj, a.proj_f32, row * a.proj_ld + h * 3 + j) + a.base_lr_inv;
+    const float g = a.g[j] != nullptr ? a.g[j][gi] : 0.f;
+    put(a.dproj, a.proj_f32, i * 3 + j, x > 20.f ? g : g / (1.f + expf(-x)));
+  }
+  if (a.logits != nullptr) {
+    const float sg = 1.f / (1.f + expf(-load_scalar(a.logits, a.logits_f32, row * a.logits_ld + h)));
+    put(a.dlogits, a.logits_f32, i, a.gm != nullptr ? a.gm[gi] * sg * (1.f - sg) : 0.f);
+  }
+}
+
+// Sums of the columns of an [rows][cols] fp32 matrix (partial sums of many blocks) in a fixed order: a block owns 32
+// columns, its eight warps every eighth row.
+__global__ void __launch_bounds__(256) column_sums_kernel(const float* x, float* out, int64_t rows, int64_t cols) {
+  __shared__ float part[8][33];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t c = static_cast<int64_t>(blockIdx.x) * 32 + lane;
+  float s[4] = {};
+  if (c < cols) {
+    int64_t r = warp;
+    for (; r + 24 < rows; r += 32)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s[j] += x[(r + 8 * j) * cols + c];
+    for (; r < rows; r += 8) s[0] += x[r * cols + c];
+  }
+  part[warp][lane] = (s[0] + s[1]) + (s[2] + s[3]);
+  __syncthreads();
+  if (warp == 0 && c < cols) {
+    float t = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) t += part[w][lane];
+    out[c] = t;
+  }
+}
+
+// First token of the sequence every token of a packed entry belongs to: the last boundary at or before it.
+__global__ void __launch_bounds__(256) seq_start_kernel(const int32_t* cu, int64_t n_seq, int64_t n_tokens, int32_t* out) {
+  const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (t >= n_tokens) return;
+  int64_t lo = 0, hi = n_seq;  // cu[lo] <= t < cu[hi]
+  while (hi - lo > 1) {
+    const int64_t mid = (lo + hi) / 2;
+    if (cu[mid] <= t) lo = mid;
+    else hi = mid;
+  }
+  out[t] = cu[lo];
 }
 
 // Output side of the layer: y = bf16(x * rsqrt(mean(x^2) + eps) * weight) per head row (fp32 arithmetic, as the

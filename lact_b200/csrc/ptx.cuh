@@ -14,6 +14,18 @@ enum : int32_t {
   kStatusWaitTimeout = 101,  // a bounded mbarrier wait ran out
 };
 
+// A failure is recorded twice: in the call's device status word (later kernels of the call look at it and stand aside)
+// and, if the host asked for it (lact_status_host_word), in a word of mapped host memory that the host reads like any
+// other variable: no copy, no event and no wait per call, and nothing at all on the path without a failure.
+__device__ int32_t* g_host_status = nullptr;
+__device__ __forceinline__ void report_timeout(int32_t* status) {
+  atomicCAS(status, kStatusOk, kStatusWaitTimeout);
+  if (g_host_status != nullptr) {
+    *reinterpret_cast<volatile int32_t*>(g_host_status) = kStatusWaitTimeout;
+    __threadfence_system();
+  }
+}
+
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }

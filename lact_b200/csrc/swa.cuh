@@ -320,7 +320,7 @@ __global__ void __launch_bounds__(320, 1) swa_fwd_kernel(const __grid_constant__
   // a wait that ran out: raise the flag so the other roles stop, record the status
   if (failed && *reinterpret_cast<volatile int32_t*>(a.status) == kStatusOk) {
     *abort_flag = 1;
-    atomicCAS(a.status, kStatusOk, kStatusWaitTimeout);
+    report_timeout(a.status);
   }
   tc_fence_before();
   __syncthreads();

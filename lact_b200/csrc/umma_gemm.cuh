@@ -617,7 +617,7 @@ __device__ __forceinline__ void gemm_setup(GemmCtx& cx, uint8_t* smem_raw, int r
 __device__ __forceinline__ void gemm_teardown(GemmCtx& cx, bool failed, int32_t* status, uint32_t tmem_cols) {
   if (failed) {
     *cx.abort_flag = 1;
-    atomicCAS(status, kStatusOk, kStatusWaitTimeout);
+    report_timeout(status);
   }
   tc_fence_before();
   __syncthreads();

@@ -101,6 +101,11 @@ def ar_inference_program(L: int, mini_batch_size: int = -1, do_update: bool = Fa
     return steps
 
 
+def flatten(steps: Sequence[Step]) -> List[int]:
+    """The program as one list of integers (what the registered operators take)."""
+    return [int(x) for st in steps for x in st]
+
+
 import collections  # noqa: E402
 
 # Same field names as the reference's operator tuple (lact_nvs/lact_ttt.py:10).
