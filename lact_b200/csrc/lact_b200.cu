@@ -16,6 +16,7 @@
 #include "../../include/lact_b200.h"
 #include "f32_gemm.cuh"
 #include "ns_bwd_fused.cuh"
+#include "ns_chip.cuh"
 #include "swa_bwd.cuh"
 
 namespace lact {
@@ -729,6 +730,76 @@ int try_ns_fused(const NsGroup* grp, int ngroups, int steps, int const_coeffs, i
   return LACT_ERR_CONFIG;
 }
 
+// All of Newton-Schulz, normalisation included, by one CTA per matrix (ns_chip.cuh); every group must fit an SM.
+// src[g]: gradients (read unless `unscaled`, when the bf16 gradient is already in grp[g].xa); parts[g]: partial sums of
+// squares per matrix in grp[g].partial, or 0 / nullptr: the kernel adds them up itself.
+int launch_ns_chip(const NsGroup* grp, int ngroups, const void* const* src, int src_f32, const int* parts, int unscaled,
+                   int steps, int const_coeffs, int32_t* status, cudaStream_t stream, const bf16** result, const NsKeep* keep) {
+  static std::mutex mu;
+  static bool configured[64] = {false};
+  int dev = 0;
+  LACT_CUDA(cudaGetDevice(&dev));
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    if (dev >= 64 || !configured[dev]) {
+      LACT_CUDA(cudaFuncSetAttribute(ns_chip_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kNsChipSmem));
+      if (dev < 64) configured[dev] = true;
+    }
+  }
+  NsChipArgs a;
+  std::memset(&a, 0, sizeof(a));
+  int64_t ctas = 0;
+  for (int g = 0; g < ngroups; ++g) {
+    const NsGroup& G = grp[g];
+    NsChipGroup& K = a.grp[g];
+    const int64_t rc = static_cast<int64_t>(G.R) * G.C, mm = static_cast<int64_t>(G.m) * G.m;
+    K.nmat = G.nmat; K.R = G.R; K.C = G.C; K.m = G.m; K.n = G.n; K.tall = G.transposed;
+    K.box_rows = G.R <= 256 ? G.R : G.R / 2;
+    K.src = src[g]; K.src_f32 = src_f32;
+    K.nparts = parts != nullptr ? parts[g] : 0;
+    K.partial = K.nparts > 0 ? G.partial : nullptr;
+    if (unscaled) LACT_TRY(encode_map(&K.x_in, Mat{G.xa, G.R, G.C, G.C, G.nmat, rc}, static_cast<uint32_t>(K.box_rows)));
+    bf16* out = keep != nullptr ? keep[g].X : G.xb;
+    LACT_TRY(encode_map(&K.x_out, Mat{out, G.R, G.C, G.C, keep != nullptr ? static_cast<int64_t>(steps + 1) * G.nmat : G.nmat, rc},
+                        static_cast<uint32_t>(K.box_rows)));
+    result[g] = keep != nullptr ? keep[g].X + rc * G.nmat * steps : G.xb;
+    if (keep != nullptr) {
+      const int64_t all = static_cast<int64_t>(steps) * G.nmat;
+      LACT_TRY(encode_map(&K.s_out, Mat{keep[g].A, G.m, G.m, G.m, all, mm}, static_cast<uint32_t>(G.m)));
+      LACT_TRY(encode_map(&K.p_out, Mat{keep[g].P, G.m, G.m, G.m, all, mm}, static_cast<uint32_t>(G.m)));
+    }
+    ctas += G.nmat;
+  }
+  for (int it = 0; it < steps; ++it) {
+    const float* co = const_coeffs ? kNsConst : kNsTuned[it];
+    a.coef[it][0] = co[0]; a.coef[it][1] = co[1]; a.coef[it][2] = co[2];
+  }
+  a.ngroups = ngroups;
+  a.steps = steps;
+  a.load = unscaled;
+  a.keep = keep != nullptr;
+  a.status = status;
+  KernelScope scope(kClsNsFused, stream);
+  LACT_CUDA(launch_pdl(ns_chip_kernel, dim3(static_cast<unsigned>(ctas)), dim3(kNsChipThreads), kNsChipSmem, stream, a));
+  return LACT_OK;
+}
+
+// Newton-Schulz of one or two groups by the best path: one CTA per matrix where the matrices fit an SM, else the
+// preparation kernels and the dataflow kernel, else one launch per product.  `unscaled`: grp[g].xa holds bf16(G) and
+// the normalisation is folded into the first iteration.
+int run_newton_schulz(NsGroup* grp, int ngroups, const void* const* src, int src_f32, const int* parts, int unscaled, int steps,
+                      int const_coeffs, int32_t* status, cudaStream_t stream, const bf16** result, const NsKeep* keep = nullptr) {
+  bool chip = steps >= 1 && steps <= 16 && (const_coeffs || steps == 5);
+  for (int g = 0; g < ngroups; ++g) chip = chip && ns_chip_fits(grp[g].R, grp[g].C, grp[g].transposed);
+  const bool given = parts != nullptr && parts[0] > 0;
+  if (chip) return launch_ns_chip(grp, ngroups, src, src_f32, given ? parts : nullptr, unscaled, steps, const_coeffs, status, stream,
+                                  result, keep);
+  LACT_TRY(launch_ns_prepare(grp, ngroups, src, src_f32, !unscaled, stream, given ? parts : nullptr));
+  const int rc = try_ns_fused(grp, ngroups, steps, const_coeffs, status, stream, result, unscaled, keep);
+  if (rc != LACT_ERR_CONFIG || keep != nullptr) return rc;
+  return run_ns_iterations(grp, ngroups, steps, const_coeffs, result, status, stream, unscaled);
+}
+
 // ------------------------------------------------------------------------------------------
 // workspace planning
 // ------------------------------------------------------------------------------------------
@@ -1283,8 +1354,7 @@ int scan_fwd(const lact_scan_config& c, const lact_scan_io& io, int32_t n_steps,
         tg[gi].xa = t.X;
         keep[gi] = NsKeep{t.X, t.A, t.P};
       }
-      LACT_TRY(launch_ns_prepare(tg, 2, srcs, 1, 1, stream, fused_parts[0] > 0 ? fused_parts : nullptr));
-      LACT_TRY(try_ns_fused(tg, 2, c.ns_steps, c.ns_const_coeffs, p.status, stream, xres, 0, keep));
+      LACT_TRY(run_newton_schulz(tg, 2, srcs, 1, fused_parts, 0, c.ns_steps, c.ns_const_coeffs, p.status, stream, xres, keep));
       rn[0].x = xres[0];
       rn[1].x = xres[1];
     } else if (c.use_muon) {
@@ -1292,12 +1362,8 @@ int scan_fwd(const lact_scan_config& c, const lact_scan_io& io, int32_t n_steps,
       const bf16* xres[2] = {nullptr, nullptr};
       const void* srcs[2] = {G02cur, G1cur};
       const int unscaled = g.gb02 != nullptr ? 1 : 0;
-      LACT_TRY(launch_ns_prepare(ns.grp, ns.ngroups, srcs, 1, !unscaled, stream,
-                                 fused_parts[0] > 0 ? fused_parts : nullptr));
-      int rc = try_ns_fused(ns.grp, ns.ngroups, c.ns_steps, c.ns_const_coeffs, p.status, stream, xres, unscaled);
-      if (rc == LACT_ERR_CONFIG)
-        rc = run_ns_iterations(ns.grp, ns.ngroups, c.ns_steps, c.ns_const_coeffs, xres, p.status, stream, unscaled);
-      LACT_TRY(rc);
+      LACT_TRY(run_newton_schulz(ns.grp, ns.ngroups, srcs, 1, fused_parts, unscaled, c.ns_steps, c.ns_const_coeffs, p.status,
+                                 stream, xres));
       rn[0].x = xres[0];
       rn[1].x = xres[1];
     }
@@ -1491,11 +1557,7 @@ int scan_fwd_f32(const lact_scan_config& c, const lact_scan_io& io, int32_t n_st
     const bf16* xres[2] = {nullptr, nullptr};
     if (c.use_muon) {
       const void* srcs[2] = {p.G02, p.G1};
-      LACT_TRY(launch_ns_prepare(p.ns.grp, 2, srcs, 1, 1, stream));
-      int rc = try_ns_fused(p.ns.grp, 2, c.ns_steps, c.ns_const_coeffs, p.status, stream, xres);
-      if (rc == LACT_ERR_CONFIG)
-        rc = run_ns_iterations(p.ns.grp, 2, c.ns_steps, c.ns_const_coeffs, xres, p.status, stream);
-      LACT_TRY(rc);
+      LACT_TRY(run_newton_schulz(p.ns.grp, 2, srcs, 1, nullptr, 0, c.ns_steps, c.ns_const_coeffs, p.status, stream, xres));
     }
     RenormArgs rn[2];
     for (int w = 0; w < 2; ++w) {
@@ -1829,10 +1891,7 @@ int lact_newton_schulz(const void* g, int32_t g_dtype, void* x, int64_t B, int64
   carve_ns_group(cv, grp);
   const bf16* res = nullptr;
   const void* srcs[2] = {g, g};
-  LACT_TRY(launch_ns_prepare(&grp, 1, srcs, g_dtype == LACT_F32, 1, s));
-  int rc = try_ns_fused(&grp, 1, steps, const_coeffs, status, s, &res);
-  if (rc == LACT_ERR_CONFIG) rc = run_ns_iterations(&grp, 1, steps, const_coeffs, &res, status, s);
-  LACT_TRY(rc);
+  LACT_TRY(run_newton_schulz(&grp, 1, srcs, g_dtype == LACT_F32, nullptr, 0, steps, const_coeffs, status, s, &res));
   LACT_CUDA(cudaMemcpyAsync(x, res, static_cast<size_t>(B) * R * C * 2, cudaMemcpyDeviceToDevice, s));
   return LACT_OK;
 }
@@ -1871,14 +1930,15 @@ int lact_ns_trace_fwd(const void* g, int32_t g_dtype, void* x_out, int64_t B, in
   const size_t rc = static_cast<size_t>(B) * R * C, mm = static_cast<size_t>(B) * t.grp.m * t.grp.m;
   t.grp.xa = t.X;
   const void* srcs[2] = {g, g};
-  LACT_TRY(launch_ns_prepare(&t.grp, 1, srcs, g_dtype == LACT_F32, 1, s));  // X[0] = normalised bf16(g)
-  // all iterations in one dataflow launch that keeps every iterate (up to five: both coefficient schedules of the
-  // reference's drivers); longer constant-coefficient runs go iteration by iteration
+  // all iterations in one launch that keeps every iterate (up to five: both coefficient schedules of the reference's
+  // drivers); longer constant-coefficient runs go iteration by iteration
   int rc_f = LACT_ERR_CONFIG;
   if (steps <= 5) {
     const NsKeep keep{t.X, t.A, t.P};
     const bf16* res = nullptr;
-    rc_f = try_ns_fused(&t.grp, 1, steps, const_coeffs, status_word, s, &res, 0, &keep);
+    rc_f = run_newton_schulz(&t.grp, 1, srcs, g_dtype == LACT_F32, nullptr, 0, steps, const_coeffs, status_word, s, &res, &keep);
+  } else {
+    LACT_TRY(launch_ns_prepare(&t.grp, 1, srcs, g_dtype == LACT_F32, 1, s));  // X[0] = normalised bf16(g)
   }
   if (rc_f == LACT_ERR_CONFIG) {
     for (int it = 0; it < steps; ++it) {
