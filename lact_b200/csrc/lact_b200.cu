@@ -755,6 +755,7 @@ int launch_ns_chip(const NsGroup* grp, int ngroups, const void* const* src, int 
     const int64_t rc = static_cast<int64_t>(G.R) * G.C, mm = static_cast<int64_t>(G.m) * G.m;
     K.nmat = G.nmat; K.R = G.R; K.C = G.C; K.m = G.m; K.n = G.n; K.tall = G.transposed;
     K.box_rows = G.R <= 256 ? G.R : G.R / 2;
+    K.two = ns_chip_fits(G.R, G.C, G.transposed, true);
     K.src = src[g]; K.src_f32 = src_f32;
     K.nparts = parts != nullptr ? parts[g] : 0;
     K.partial = K.nparts > 0 ? G.partial : nullptr;

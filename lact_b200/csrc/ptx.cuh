@@ -41,6 +41,13 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
                : "memory");
 }
+__device__ __forceinline__ void mbar_expect_tx_if(uint32_t leader, uint64_t* bar, uint32_t bytes) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t"
+      "@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(smem_u32(bar)),
+      "r"(bytes), "r"(leader)
+      : "memory");
+}
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
@@ -67,15 +74,25 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
 constexpr uint64_t kDefaultWaitLimitNs = 2000000000ull;
 __constant__ uint64_t g_wait_limit_ns = kDefaultWaitLimitNs;
 __device__ __forceinline__ uint64_t wait_limit_ns() { return g_wait_limit_ns; }
+// The time is looked at only after 64 failed tries (each of which the hardware lets sleep a while), so a wait that ends
+// soon -- nearly all of them -- never reads the global timer.
+struct WaitClock {
+  uint64_t t0 = 0;
+  // false once the limit has passed since the first look
+  __device__ __forceinline__ bool within_limit() {
+    const uint64_t now = globaltimer_ns();
+    if (t0 == 0) t0 = now;
+    return now - t0 <= wait_limit_ns();
+  }
+};
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag = nullptr) {
   if (mbar_try_wait(bar, parity)) return true;
-  const uint64_t t0 = globaltimer_ns();
-  const uint64_t limit = wait_limit_ns();
+  WaitClock clock;
   for (uint32_t i = 1;; ++i) {
     if (mbar_try_wait(bar, parity)) return true;
     if ((i & 63u) == 0) {
       if (abort_flag != nullptr && *abort_flag != 0) return false;
-      if (globaltimer_ns() - t0 > limit) return false;
+      if (!clock.within_limit()) return false;
     }
   }
 }
@@ -88,6 +105,35 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
 // Both are no-ops for kernels launched without the attribute.
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// ---------------------------------------------------------------- warp-uniform roles
+// TMA and tcgen05 instructions take their addresses and descriptors from uniform registers.  In code that only one lane
+// executes (`if (lane == 0)`) the compiler has to move every operand over one by one: about 100 clocks per MMA (measured:
+// 8 MMAs of 128 x 128 x 16 issued in 827 clocks, where the tensor pipe needs 512 and the loop below reaches that).  So a
+// role's warp runs its loop as a whole on warp-uniform values, and the single-thread instructions are predicated on the
+// leader lane.
+__device__ __forceinline__ int uniform_warp_index() { return __shfl_sync(0xFFFFFFFFu, static_cast<int>(threadIdx.x >> 5), 0); }
+__device__ __forceinline__ uint32_t uniform(uint32_t x) { return __shfl_sync(0xFFFFFFFFu, x, 0); }
+// 1 in one lane of the (fully active) warp, the same lane every time
+__device__ __forceinline__ uint32_t elect_leader() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "elect.sync _|q, 0xFFFFFFFF;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(p));
+  return p;
+}
+
+// Bounded wait of a whole warp with a warp-uniform answer (so that the loops around it stay uniform for the compiler).
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag) {
+  if (__all_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity))) return true;
+  WaitClock clock;
+  for (uint32_t i = 1;; ++i) {
+    if (__all_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity))) return true;
+    if ((i & 63u) == 0 && __any_sync(0xFFFFFFFFu, *abort_flag != 0 || !clock.within_limit())) return false;
+  }
+}
 
 // ---------------------------------------------------------------- fences
 __device__ __forceinline__ void fence_async_proxy() {
@@ -123,6 +169,26 @@ __device__ __forceinline__ void tma_load_4d(uint32_t smem_dst, const CUtensorMap
       "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
       " [%0], [%1, {%3, %4, %5, %6}], [%2];"
       ::"r"(smem_dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+      : "memory");
+}
+
+// the same two loads issued by the leader lane of a warp-uniform role
+__device__ __forceinline__ void tma_load_3d_if(uint32_t leader, uint32_t smem_dst, const CUtensorMap* map, uint64_t* bar, int c0,
+                                               int c1, int c2) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %6, 0;\n\t"
+      "@q cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%3, %4, %5}], [%2];\n\t}"
+      ::"r"(smem_dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(leader)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_4d_if(uint32_t leader, uint32_t smem_dst, const CUtensorMap* map, uint64_t* bar, int c0,
+                                               int c1, int c2, int c3) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %7, 0;\n\t"
+      "@q cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%3, %4, %5, %6}], [%2];\n\t}"
+      ::"r"(smem_dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(leader)
       : "memory");
 }
 
@@ -187,6 +253,15 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr, uint32_t lbo_
   d |= static_cast<uint64_t>(2) << 61;  // layout type: 128-byte swizzle
   return d;
 }
+// The descriptors of one operand's tiles: they differ in the start address alone (16-byte units, low word).
+struct SmemDescBase {
+  uint32_t lo, hi;
+  __device__ __forceinline__ explicit SmemDescBase(uint32_t lbo_bytes)
+      : lo(((lbo_bytes >> 4) & 0x3FFFu) << 16), hi(((1024u >> 4) & 0x3FFFu) | (1u << 14) | (2u << 29)) {}
+  __device__ __forceinline__ uint64_t at(uint32_t saddr16) const {
+    return (static_cast<uint64_t>(hi) << 32) | (lo + saddr16);
+  }
+};
 // Instruction descriptor for kind::f16 with bf16 operands and fp32 accumulation.
 __host__ __device__ __forceinline__ uint32_t make_idesc_bf16(uint32_t m, uint32_t n, uint32_t a_mn_major,
                                                              uint32_t b_mn_major) {
@@ -214,6 +289,25 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint6
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                : "memory");
+}
+
+// the same two instructions issued by the leader lane of a warp-uniform role
+__device__ __forceinline__ void umma_bf16_if(uint32_t leader, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                             uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(leader)
+      : "memory");
+}
+__device__ __forceinline__ void umma_commit_if(uint32_t leader, uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)),
+      "r"(leader)
+      : "memory");
 }
 
 // ---------------------------------------------------------------- small numeric helpers

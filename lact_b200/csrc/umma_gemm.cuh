@@ -90,30 +90,21 @@ constexpr int kGemmThreadsFlow = kGemmThreadsV2 + 64;  // + dependency scout war
 // With KB = 2 a K-major tile arrives as one box of a 4-D map when the operand allows it (k4d), an
 // MN-major tile as one 128-k-row box per atom.
 template <int ROWS, int KB>
-__device__ __forceinline__ void load_operand_tile(uint32_t dst, const CUtensorMap* map, const OperandInfo& oi,
+__device__ __forceinline__ void load_operand_tile(uint32_t leader, uint32_t dst, const CUtensorMap* map, const OperandInfo& oi,
                                                   int mn0, int kc, int batch, uint64_t* bar) {
   if (!oi.mn_major) {
     if (KB == 2 && oi.k4d) {
-      tma_load_4d(dst, map, bar, 0, oi.mn_off + mn0, (oi.k_off + kc) / kBK, oi.batch_off + batch);
+      tma_load_4d_if(leader, dst, map, bar, 0, oi.mn_off + mn0, (oi.k_off + kc) / kBK, oi.batch_off + batch);
     } else {
 #pragma unroll
       for (int kk = 0; kk < KB; ++kk)
-        tma_load_3d(dst + kk * (ROWS * kBK * 2), map, bar, oi.k_off + kc + kk * kBK, oi.mn_off + mn0, oi.batch_off + batch);
+        tma_load_3d_if(leader, dst + kk * (ROWS * kBK * 2), map, bar, oi.k_off + kc + kk * kBK, oi.mn_off + mn0, oi.batch_off + batch);
     }
   } else {
 #pragma unroll
     for (int j = 0; j < ROWS / 64; ++j)
-      tma_load_3d(dst + j * (KB * kAtomBytes), map, bar, oi.mn_off + mn0 + 64 * j, oi.k_off + kc, oi.batch_off + batch);
+      tma_load_3d_if(leader, dst + j * (KB * kAtomBytes), map, bar, oi.mn_off + mn0 + 64 * j, oi.k_off + kc, oi.batch_off + batch);
   }
-}
-
-// Descriptor of the k-block `kk`, 16-element k-slice `k4`, of an operand tile of ROWS_BYTES = rows * 128.
-template <int KB>
-__device__ __forceinline__ uint64_t operand_desc(uint32_t tile, int mn_major, uint32_t rows_bytes, int kk, int k4) {
-  // K-major: advance 16 elements (32 bytes) inside the swizzled 128-byte row.
-  // MN-major: advance 16 k-rows (2 groups of 8 rows x 128 bytes); atoms are KB * 8 KB apart.
-  return mn_major ? make_smem_desc(tile + kk * kAtomBytes + k4 * 2048, KB * kAtomBytes, 1024)
-                  : make_smem_desc(tile + kk * rows_bytes + k4 * 32, 0, 1024);
 }
 
 struct TileCoord {
@@ -190,10 +181,10 @@ __device__ __forceinline__ void st_release_cta_shared_u32(uint32_t* p, uint32_t 
 // Bounded spin until *ctr >= need (global memory, written by other CTAs).
 __device__ __forceinline__ bool dep_wait(const uint32_t* ctr, uint32_t need, volatile uint32_t* abort_flag) {
   if (need == 0 || ld_acquire_gpu_u32(ctr) >= need) return true;
-  const uint64_t t0 = globaltimer_ns();
+  WaitClock clock;
   for (uint32_t i = 1;; ++i) {
     if (ld_acquire_gpu_u32(ctr) >= need) return true;
-    if ((i & 31u) == 0 && (*abort_flag != 0 || globaltimer_ns() - t0 > wait_limit_ns())) return false;
+    if ((i & 31u) == 0 && (*abort_flag != 0 || !clock.within_limit())) return false;
   }
 }
 // Storing thread: once all its stores have landed, publish the completion of a tile.
@@ -207,10 +198,10 @@ __device__ __forceinline__ void flow_publish(uint32_t* counter) {
 // running number `seq` (0-based).
 __device__ __forceinline__ bool flow_wait_verified(const GemmCtx& cx, uint32_t seq) {
   if (ld_acquire_cta_shared_u32(cx.dep_ok) > seq) return true;
-  const uint64_t t0 = globaltimer_ns();
+  WaitClock clock;
   for (uint32_t i = 1;; ++i) {
     if (ld_acquire_cta_shared_u32(cx.dep_ok) > seq) return true;
-    if ((i & 63u) == 0 && (*cx.abort_flag != 0 || globaltimer_ns() - t0 > wait_limit_ns())) return false;
+    if ((i & 255u) == 0 && (*cx.abort_flag != 0 || !clock.within_limit())) return false;
   }
 }
 
@@ -290,11 +281,12 @@ __device__ __forceinline__ bool gemm_phase(GemmCtx& cx, const GemmProblem<Op>* p
   };
   if constexpr (Deps::kOn) cx.rot = (cx.rot + static_cast<uint32_t>(total_tiles)) % gridDim.x;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
   bool failed = false;
   if (warp == 0) {
-    // ---------------- TMA producer (one thread); the ring keeps running across tiles
-    if (lane == 0) {
+    // ---------------- TMA producer (warp-uniform, issued by its leader lane); the ring keeps running across tiles
+    const uint32_t leader = elect_leader();
+    {
       for (int tile_i = 0; tile_i < rounds && !failed; ++tile_i) {
         const int tile = tile_at(tile_i);
         if (tile >= total_tiles) continue;
@@ -302,30 +294,31 @@ __device__ __forceinline__ bool gemm_phase(GemmCtx& cx, const GemmProblem<Op>* p
         const GemmProblem<Op>& P = probs[tc.prob];
         const int num_kb = (P.K + kBK - 1) / kBK;
         if constexpr (Deps::kOn) {
-          if (!flow_wait_verified(cx, cx.ptile++)) { failed = true; break; }  // the scout warp checked this tile
+          if (!__all_sync(0xFFFFFFFFu, flow_wait_verified(cx, cx.ptile++))) { failed = true; break; }  // the scout warp checked this tile
           asm volatile("fence.proxy.async;" ::: "memory");
         }
         const int num_sb = (num_kb + KB - 1) / KB;  // ring stages of KB k-blocks
         for (int sb = 0; sb < num_sb; ++sb, ++cx.it) {
           const int s = cx.it % RING;
           const uint32_t ph = (cx.it / RING) & 1;
-          if (!mbar_wait(&cx.empty_bar[s], ph ^ 1, cx.abort_flag)) { failed = true; break; }
-          mbar_expect_tx(&cx.full_bar[s], kStageBytes);
+          if (!mbar_wait_warp(&cx.empty_bar[s], ph ^ 1, cx.abort_flag)) { failed = true; break; }
+          mbar_expect_tx_if(leader, &cx.full_bar[s], kStageBytes);
           const uint32_t st = cx.smem_base + s * cx.stage_stride;
           const int kc = sb * KB * kBK;
 #pragma unroll
           for (int i = 0; i < NA; ++i)
-            load_operand_tile<kBM, KB>(st + i * (KB * kATileBytes), &P.a[i], P.ai[i], tc.m0, kc, tc.batch, &cx.full_bar[s]);
+            load_operand_tile<kBM, KB>(leader, st + i * (KB * kATileBytes), &P.a[i], P.ai[i], tc.m0, kc, tc.batch, &cx.full_bar[s]);
 #pragma unroll
           for (int i = 0; i < NB; ++i)
-            load_operand_tile<BT, KB>(st + NA * (KB * kATileBytes) + i * (KB * kBTileBytes), &P.b[i], P.bi[i], tc.n0, kc,
+            load_operand_tile<BT, KB>(leader, st + NA * (KB * kATileBytes) + i * (KB * kBTileBytes), &P.b[i], P.bi[i], tc.n0, kc,
                                       tc.batch, &cx.full_bar[s]);
         }
       }
     }
   } else if (warp == 1) {
-    // ---------------- MMA issuer (one thread)
-    if (lane == 0) {
+    // ---------------- MMA issuer (warp-uniform, issued by its leader lane)
+    const uint32_t leader = elect_leader();
+    {
       for (int tile_i = 0; tile_i < rounds && !failed; ++tile_i) {
         const int tile = tile_at(tile_i);
         if (tile >= total_tiles) continue;
@@ -333,37 +326,47 @@ __device__ __forceinline__ bool gemm_phase(GemmCtx& cx, const GemmProblem<Op>* p
         const GemmProblem<Op>& P = probs[tc.prob];
         const int num_kb = (P.K + kBK - 1) / kBK;
         const uint32_t as = cx.tcount & 1, aph = (cx.tcount >> 1) & 1;
-        if (!mbar_wait(&cx.acc_empty_bar[as], aph ^ 1, cx.abort_flag)) { failed = true; break; }
+        if (!mbar_wait_warp(&cx.acc_empty_bar[as], aph ^ 1, cx.abort_flag)) { failed = true; break; }
         tc_fence_after();
         const uint32_t acc_base = cx.tmem_base + as * kAccStride;
         const int num_sb = (num_kb + KB - 1) / KB;
+        // K-major tiles: 16 elements = 32 bytes on inside the swizzled 128-byte row, k-blocks a tile apart; MN-major tiles:
+        // 16 k-rows of 128 bytes on, k-blocks 64 rows apart, 64-wide atoms KB * 8 KB apart (the leading offset)
+        uint32_t idesc[Op::NTERMS], step_a[Op::NTERMS], step_b[Op::NTERMS], blk_a[Op::NTERMS], blk_b[Op::NTERMS];
+#pragma unroll
+        for (int t = 0; t < Op::NTERMS; ++t) {
+          const int a_mn = P.ai[Op::term_a(t)].mn_major, b_mn = P.bi[Op::term_b(t)].mn_major;
+          idesc[t] = make_idesc_bf16(kBM, Op::term_n(t), a_mn, b_mn);
+          step_a[t] = a_mn ? 128 : 2;
+          step_b[t] = b_mn ? 128 : 2;
+          blk_a[t] = (a_mn ? kAtomBytes : kATileBytes) >> 4;
+          blk_b[t] = (b_mn ? kAtomBytes : kBTileBytes) >> 4;
+        }
+        const SmemDescBase desc(KB * kAtomBytes);  // (K-major descriptors ignore the leading offset)
         for (int sb = 0; sb < num_sb; ++sb, ++cx.it) {
           const int s = cx.it % RING;
           const uint32_t ph = (cx.it / RING) & 1;
-          if (!mbar_wait(&cx.full_bar[s], ph, cx.abort_flag)) { failed = true; break; }
+          if (!mbar_wait_warp(&cx.full_bar[s], ph, cx.abort_flag)) { failed = true; break; }
           tc_fence_after();
-          const uint32_t st = cx.smem_base + s * cx.stage_stride;
+          const uint32_t st = (cx.smem_base + s * cx.stage_stride) >> 4;
 #pragma unroll
           for (int kk = 0; kk < KB; ++kk) {
             if (sb * KB + kk >= num_kb) break;  // a trailing half-empty stage
 #pragma unroll
             for (int t = 0; t < Op::NTERMS; ++t) {
-              const int ia = Op::term_a(t), ib = Op::term_b(t);
-              const int a_mn = P.ai[ia].mn_major, b_mn = P.bi[ib].mn_major;
-              const uint32_t idesc = make_idesc_bf16(kBM, Op::term_n(t), a_mn, b_mn);
-              const uint32_t a_tile = st + ia * (KB * kATileBytes);
-              const uint32_t b_tile = st + NA * (KB * kATileBytes) + ib * (KB * kBTileBytes);
+              const uint32_t a_tile = st + Op::term_a(t) * (KB * kATileBytes >> 4) + kk * blk_a[t];
+              const uint32_t b_tile = st + (NA * (KB * kATileBytes) + Op::term_b(t) * (KB * kBTileBytes) >> 4) + kk * blk_b[t];
 #pragma unroll
               for (int k4 = 0; k4 < kBK / kUmmaK; ++k4) {
                 const uint32_t acc = (sb > 0 || kk > 0 || k4 > 0 || !Op::term_first(t)) ? 1u : 0u;
-                umma_bf16(acc_base + Op::term_col(t), operand_desc<KB>(a_tile, a_mn, kATileBytes, kk, k4),
-                          operand_desc<KB>(b_tile, b_mn, kBTileBytes, kk, k4), idesc, acc);
+                umma_bf16_if(leader, acc_base + Op::term_col(t), desc.at(a_tile + k4 * step_a[t]), desc.at(b_tile + k4 * step_b[t]),
+                             idesc[t], acc);
               }
             }
           }
-          umma_commit(&cx.empty_bar[s]);  // frees the stage once these MMAs have read it
+          umma_commit_if(leader, &cx.empty_bar[s]);  // frees the stage once these MMAs have read it
         }
-        if (!failed) umma_commit(&cx.acc_full_bar[as]);
+        if (!failed) umma_commit_if(leader, &cx.acc_full_bar[as]);
         ++cx.tcount;
       }
     }
@@ -611,7 +614,7 @@ __device__ __forceinline__ void gemm_setup(GemmCtx& cx, uint8_t* smem_raw, int r
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  cx.tmem_base = *tmem_slot;
+  cx.tmem_base = uniform(*tmem_slot);
 }
 
 __device__ __forceinline__ void gemm_teardown(GemmCtx& cx, bool failed, int32_t* status, uint32_t tmem_cols) {
