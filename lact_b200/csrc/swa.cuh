@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(320, 1) swa_fwd_kernel(const __grid_constant__
   volatile uint32_t* abort_flag = tmem_slot + 1;
   float* xch = reinterpret_cast<float*>(aligned + SM::kBars + 256);   // [2 halves][128 rows]
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
     for (int s = 0; s < 2; ++s) {
@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(320, 1) swa_fwd_kernel(const __grid_constant__
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = uniform(*tmem_slot);
 
   // this CTA's query tile and the key tiles its window touches
   const int qt = blockIdx.x % a.q_tiles;
@@ -115,51 +115,53 @@ __global__ void __launch_bounds__(320, 1) swa_fwd_kernel(const __grid_constant__
     kv_hi = a.Lk;
   }
   const int T = (kv_hi - kv_lo + 127) / 128;
-  bool failed = *reinterpret_cast<volatile int32_t*>(a.status) != kStatusOk;
+  bool failed = uniform(static_cast<uint32_t>(*reinterpret_cast<volatile int32_t*>(a.status))) != kStatusOk;
 
   if (warp == 0) {
-    if (lane == 0 && !failed) {
-      mbar_expect_tx(q_full, SM::kTile);
-      for (int j = 0; j < KBD; ++j) tma_load_4d(base + SM::kQ + j * kBox, &a.q, q_full, 64 * j, q0, head, batch);
+    const uint32_t leader = elect_leader();
+    if (!failed) {
+      mbar_expect_tx_if(leader, q_full, SM::kTile);
+      for (int j = 0; j < KBD; ++j) tma_load_4d_if(leader, base + SM::kQ + j * kBox, &a.q, q_full, 64 * j, q0, head, batch);
       for (int t = 0; t < T && !failed; ++t) {
         const int sb = t & 1;
-        if (t >= 2 && !mbar_wait(&k_empty[sb], ((t - 2) >> 1) & 1, abort_flag)) { failed = true; break; }
-        mbar_expect_tx(&k_full[sb], SM::kTile);
+        if (t >= 2 && !mbar_wait_warp(&k_empty[sb], ((t - 2) >> 1) & 1, abort_flag)) { failed = true; break; }
+        mbar_expect_tx_if(leader, &k_full[sb], SM::kTile);
         for (int j = 0; j < KBD; ++j)
-          tma_load_4d(base + SM::kK + sb * SM::kTile + j * kBox, &a.k, &k_full[sb], 64 * j, kv_lo + t * 128, head, batch);
-        if (t >= 2 && !mbar_wait(&pv_done[sb], ((t - 2) >> 1) & 1, abort_flag)) { failed = true; break; }
-        mbar_expect_tx(&v_full[sb], SM::kTile);
+          tma_load_4d_if(leader, base + SM::kK + sb * SM::kTile + j * kBox, &a.k, &k_full[sb], 64 * j, kv_lo + t * 128, head, batch);
+        if (t >= 2 && !mbar_wait_warp(&pv_done[sb], ((t - 2) >> 1) & 1, abort_flag)) { failed = true; break; }
+        mbar_expect_tx_if(leader, &v_full[sb], SM::kTile);
         for (int j = 0; j < KBD; ++j)
-          tma_load_4d(base + SM::kV + sb * SM::kTile + j * kBox, &a.v, &v_full[sb], 64 * j, kv_lo + t * 128, head, batch);
+          tma_load_4d_if(leader, base + SM::kV + sb * SM::kTile + j * kBox, &a.v, &v_full[sb], 64 * j, kv_lo + t * 128, head, batch);
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && !failed) {
+    const uint32_t leader = elect_leader();
+    if (!failed) {
       const uint32_t idesc_s = make_idesc_bf16(128, 128, 0, 0);
       const uint32_t idesc_o = make_idesc_bf16(128, HD, 0, 1);
       auto issue_s = [&](int u) -> bool {
         const int sb = u & 1;
-        if (!mbar_wait(&k_full[sb], (u >> 1) & 1, abort_flag)) return false;
-        if (u >= 2 && !mbar_wait(&s_empty[sb], ((u - 2) >> 1) & 1, abort_flag)) return false;
+        if (!mbar_wait_warp(&k_full[sb], (u >> 1) & 1, abort_flag)) return false;
+        if (u >= 2 && !mbar_wait_warp(&s_empty[sb], ((u - 2) >> 1) & 1, abort_flag)) return false;
         tc_fence_after();
         const uint32_t qa = base + SM::kQ, kb = base + SM::kK + sb * SM::kTile;
 #pragma unroll
         for (int kk = 0; kk < KBD; ++kk)
 #pragma unroll
           for (int k4 = 0; k4 < 4; ++k4)
-            umma_bf16(tmem + sb * 128, make_smem_desc(qa + kk * kBox + k4 * 32, 0, 1024),
+            umma_bf16_if(leader, tmem + sb * 128, make_smem_desc(qa + kk * kBox + k4 * 32, 0, 1024),
                       make_smem_desc(kb + kk * kBox + k4 * 32, 0, 1024), idesc_s, (kk | k4) != 0);
-        umma_commit(&s_full[sb]);
-        umma_commit(&k_empty[sb]);
+        umma_commit_if(leader, &s_full[sb]);
+        umma_commit_if(leader, &k_empty[sb]);
         return true;
       };
-      if (!mbar_wait(q_full, 0, abort_flag)) failed = true;
+      if (!mbar_wait_warp(q_full, 0, abort_flag)) failed = true;
       for (int t = 0; t < T && !failed; ++t) {
         const int sb = t & 1;
         if (t == 0 && !issue_s(0)) { failed = true; break; }
         if (t + 1 < T && !issue_s(t + 1)) { failed = true; break; }
-        if (!mbar_wait(&p_full[sb], (t >> 1) & 1, abort_flag) || !mbar_wait(&v_full[sb], (t >> 1) & 1, abort_flag) ||
-            (t >= 2 && !mbar_wait(&o_empty[sb], ((t - 2) >> 1) & 1, abort_flag))) {
+        if (!mbar_wait_warp(&p_full[sb], (t >> 1) & 1, abort_flag) || !mbar_wait_warp(&v_full[sb], (t >> 1) & 1, abort_flag) ||
+            (t >= 2 && !mbar_wait_warp(&o_empty[sb], ((t - 2) >> 1) & 1, abort_flag))) {
           failed = true;
           break;
         }
@@ -171,9 +173,9 @@ __global__ void __launch_bounds__(320, 1) swa_fwd_kernel(const __grid_constant__
         for (int kk = 0; kk < 2; ++kk)
 #pragma unroll
           for (int k4 = 0; k4 < 4; ++k4)
-            umma_bf16(tmem + 256 + sb * HD, make_smem_desc(pa + kk * kBox + k4 * 32, 0, 1024),
+            umma_bf16_if(leader, tmem + 256 + sb * HD, make_smem_desc(pa + kk * kBox + k4 * 32, 0, 1024),
                       make_smem_desc(vb + kk * kAtomBytes + k4 * 2048, kBox, 1024), idesc_o, (kk | k4) != 0);
-        umma_commit(&pv_done[sb]);
+        umma_commit_if(leader, &pv_done[sb]);
       }
     }
   } else {

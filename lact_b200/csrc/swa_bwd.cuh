@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(320, 1) swa_bwd_kernel(const __grid_constant__
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     mbar_init(outer_full, 1);
     for (int s = 0; s < NI; ++s) {
@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(320, 1) swa_bwd_kernel(const __grid_constant__
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = uniform(*tmem_slot);
 
   const int ot = blockIdx.x % a.tiles;
   const int head = (blockIdx.x / a.tiles) % a.heads;
@@ -117,39 +117,41 @@ __global__ void __launch_bounds__(320, 1) swa_bwd_kernel(const __grid_constant__
     if (!a.causal) t_lo = 0, t_hi = (a.Lk - 1) / 64;  // every key tile
   }
   const int T = t_hi - t_lo + 1;
-  bool failed = *reinterpret_cast<volatile int32_t*>(a.status) != kStatusOk;
+  bool failed = uniform(static_cast<uint32_t>(*reinterpret_cast<volatile int32_t*>(a.status))) != kStatusOk;
   const CUtensorMap* outer_a = MODE == 0 ? &a.k : &a.q;          // outer pair: (K, V) or (Q, dO)
   const CUtensorMap* outer_b = MODE == 0 ? &a.v : &a.dout;
   const CUtensorMap* inner_a = MODE == 0 ? &a.q64 : &a.k64;      // inner pair: (Q, dO) or (K, V)
   const CUtensorMap* inner_b = MODE == 0 ? &a.dout64 : &a.v64;
 
   if (warp == 0) {
-    if (lane == 0 && !failed) {
-      mbar_expect_tx(outer_full, 2 * SM::kOTile);
+    const uint32_t leader = elect_leader();
+    if (!failed) {
+      mbar_expect_tx_if(leader, outer_full, 2 * SM::kOTile);
       for (int j = 0; j < KBD; ++j) {
-        tma_load_4d(base + SM::kOuter + j * kBox, outer_a, outer_full, 64 * j, o0, head, batch);
-        tma_load_4d(base + SM::kOuter + SM::kOTile + j * kBox, outer_b, outer_full, 64 * j, o0, head, batch);
+        tma_load_4d_if(leader, base + SM::kOuter + j * kBox, outer_a, outer_full, 64 * j, o0, head, batch);
+        tma_load_4d_if(leader, base + SM::kOuter + SM::kOTile + j * kBox, outer_b, outer_full, 64 * j, o0, head, batch);
       }
       for (int t = 0; t < T && !failed; ++t) {
         const int s = t % NI;
-        if (t >= NI && !mbar_wait(&inner_empty[s], (t / NI - 1) & 1, abort_flag)) { failed = true; break; }
-        mbar_expect_tx(&inner_full[s], 2 * SM::kITile);
+        if (t >= NI && !mbar_wait_warp(&inner_empty[s], (t / NI - 1) & 1, abort_flag)) { failed = true; break; }
+        mbar_expect_tx_if(leader, &inner_full[s], 2 * SM::kITile);
         const uint32_t dst = base + SM::kInner + s * 2 * SM::kITile;
         for (int j = 0; j < KBD; ++j) {
-          tma_load_4d(dst + j * kIBox, inner_a, &inner_full[s], 64 * j, (t_lo + t) * 64, head, batch);
-          tma_load_4d(dst + SM::kITile + j * kIBox, inner_b, &inner_full[s], 64 * j, (t_lo + t) * 64, head, batch);
+          tma_load_4d_if(leader, dst + j * kIBox, inner_a, &inner_full[s], 64 * j, (t_lo + t) * 64, head, batch);
+          tma_load_4d_if(leader, dst + SM::kITile + j * kIBox, inner_b, &inner_full[s], 64 * j, (t_lo + t) * 64, head, batch);
         }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && !failed) {
+    const uint32_t leader = elect_leader();
+    if (!failed) {
       const uint32_t idesc_first = make_idesc_bf16(128, 64, 0, 0);   // [outer x inner], both operands K-major (features)
       const uint32_t idesc_acc = make_idesc_bf16(128, HD, 0, 1);     // [outer x HD]: A = P / dS tile K-major, B = inner tile MN-major
       const uint32_t o_a = base + SM::kOuter, o_b = o_a + SM::kOTile;
       // first products of inner tile t into its stage's columns
       auto first = [&](int t) -> bool {
         const int s = t & 1, si = t % NI;
-        if (!mbar_wait(&inner_full[si], (t / NI) & 1, abort_flag)) return false;
+        if (!mbar_wait_warp(&inner_full[si], (t / NI) & 1, abort_flag)) return false;
         tc_fence_after();
         const uint32_t i_a = base + SM::kInner + si * 2 * SM::kITile, i_b = i_a + SM::kITile;
         const uint32_t col = tmem + s * 128;
@@ -157,24 +159,24 @@ __global__ void __launch_bounds__(320, 1) swa_bwd_kernel(const __grid_constant__
         for (int kk = 0; kk < KBD; ++kk)
 #pragma unroll
           for (int k4 = 0; k4 < 4; ++k4)
-            umma_bf16(col, make_smem_desc(o_a + kk * kBox + k4 * 32, 0, 1024),
+            umma_bf16_if(leader, col, make_smem_desc(o_a + kk * kBox + k4 * 32, 0, 1024),
                       make_smem_desc(i_a + kk * kIBox + k4 * 32, 0, 1024), idesc_first, (kk | k4) != 0);
 #pragma unroll
         for (int kk = 0; kk < KBD; ++kk)
 #pragma unroll
           for (int k4 = 0; k4 < 4; ++k4)
-            umma_bf16(col + 64, make_smem_desc(o_b + kk * kBox + k4 * 32, 0, 1024),
+            umma_bf16_if(leader, col + 64, make_smem_desc(o_b + kk * kBox + k4 * 32, 0, 1024),
                       make_smem_desc(i_b + kk * kIBox + k4 * 32, 0, 1024), idesc_first, (kk | k4) != 0);
-        umma_commit(&sdp_full[s]);
+        umma_commit_if(leader, &sdp_full[s]);
         return true;
       };
-      if (!mbar_wait(outer_full, 0, abort_flag)) failed = true;
+      if (!mbar_wait_warp(outer_full, 0, abort_flag)) failed = true;
       if (!failed && !first(0)) failed = true;
       for (int t = 0; t < T && !failed; ++t) {
         const int s = t & 1;
         // (the other stage's columns were read by the softmax threads of tile t - 1: awaited one iteration ago)
         if (t + 1 < T && !first(t + 1)) { failed = true; break; }
-        if (!mbar_wait(&pds_full[s], (t >> 1) & 1, abort_flag)) { failed = true; break; }
+        if (!mbar_wait_warp(&pds_full[s], (t >> 1) & 1, abort_flag)) { failed = true; break; }
         tc_fence_after();
         const int si = t % NI;
         const uint32_t i_a = base + SM::kInner + si * 2 * SM::kITile, i_b = i_a + SM::kITile;
@@ -183,19 +185,19 @@ __global__ void __launch_bounds__(320, 1) swa_bwd_kernel(const __grid_constant__
 #pragma unroll
         for (int k4 = 0; k4 < 4; ++k4) {
           if (MODE == 0) {
-            umma_bf16(tmem + 256, make_smem_desc(w_p + k4 * 32, 0, 1024), make_smem_desc(i_b + k4 * 2048, kIBox, 1024),
+            umma_bf16_if(leader, tmem + 256, make_smem_desc(w_p + k4 * 32, 0, 1024), make_smem_desc(i_b + k4 * 2048, kIBox, 1024),
                       idesc_acc, (t | k4) != 0);            // dV += P^T dO
-            umma_bf16(tmem + 256 + HD, make_smem_desc(w_ds + k4 * 32, 0, 1024), make_smem_desc(i_a + k4 * 2048, kIBox, 1024),
+            umma_bf16_if(leader, tmem + 256 + HD, make_smem_desc(w_ds + k4 * 32, 0, 1024), make_smem_desc(i_a + k4 * 2048, kIBox, 1024),
                       idesc_acc, (t | k4) != 0);            // dK += dS^T Q
           } else {
-            umma_bf16(tmem + 256, make_smem_desc(w_ds + k4 * 32, 0, 1024), make_smem_desc(i_a + k4 * 2048, kIBox, 1024),
+            umma_bf16_if(leader, tmem + 256, make_smem_desc(w_ds + k4 * 32, 0, 1024), make_smem_desc(i_a + k4 * 2048, kIBox, 1024),
                       idesc_acc, (t | k4) != 0);            // dQ += dS K
           }
         }
-        umma_commit(&inner_empty[si]);
-        umma_commit(&w_empty[s]);
+        umma_commit_if(leader, &inner_empty[si]);
+        umma_commit_if(leader, &w_empty[s]);
       }
-      if (!failed) umma_commit(acc_full);
+      if (!failed) umma_commit_if(leader, acc_full);
     }
   } else {
     // ---------------- softmax / epilogue: two threads per tensor-memory lane (outer row), 32 inner columns each
