@@ -17,6 +17,7 @@
 #include "f32_gemm.cuh"
 #include "ns_bwd_fused.cuh"
 #include "ns_chip.cuh"
+#include "row_passes.cuh"
 #include "swa_bwd.cuh"
 
 namespace lact {
@@ -2045,7 +2046,13 @@ static int qkv_prologue_impl(const void* xq, const void* xk, const void* xv, int
   KernelScope scope(kClsOther, static_cast<cudaStream_t>(stream));
   const unsigned grid = static_cast<unsigned>(ceil_div(rows, 8));
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (a.rope_hd != 0) {
+  const bool exact = n_heads <= 65535 / 3 && with_row_shape(d, [&](auto lpr, auto v) {
+    const dim3 g(ceil_div(s, 256 / lpr.value), static_cast<unsigned>(3 * n_heads), static_cast<unsigned>(b));
+    if (a.rope_hd != 0) qkv_rows_kernel<lpr.value, v.value, true><<<g, 256, 0, st>>>(a);
+    else qkv_rows_kernel<lpr.value, v.value, false><<<g, 256, 0, st>>>(a);
+  });
+  if (exact) {
+  } else if (a.rope_hd != 0) {
     switch (ceil_div(d, 256)) {
       case 1: qkv_prologue_kernel<1, true><<<grid, 256, 0, st>>>(a); break;
       case 2: qkv_prologue_kernel<2, true><<<grid, 256, 0, st>>>(a); break;
@@ -2112,7 +2119,13 @@ int lact_qkv_prologue_bwd(const void* xq, const void* xk, const void* xv, int64_
   KernelScope scope(kClsOther, static_cast<cudaStream_t>(stream));
   const unsigned grid = static_cast<unsigned>(ceil_div(rows, 8));
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (a.rope_hd != 0) {
+  const bool exact = n_heads <= 65535 / 3 && with_row_shape(d, [&](auto lpr, auto v) {
+    const dim3 g(ceil_div(s, 256 / lpr.value), static_cast<unsigned>(3 * n_heads), static_cast<unsigned>(b));
+    if (a.rope_hd != 0) qkv_rows_bwd_kernel<lpr.value, v.value, true><<<g, 256, 0, st>>>(a);
+    else qkv_rows_bwd_kernel<lpr.value, v.value, false><<<g, 256, 0, st>>>(a);
+  });
+  if (exact) {
+  } else if (a.rope_hd != 0) {
     switch (ceil_div(d, 256)) {
       case 1: qkv_prologue_bwd_kernel<1, true><<<grid, 256, 0, st>>>(a); break;
       case 2: qkv_prologue_bwd_kernel<2, true><<<grid, 256, 0, st>>>(a); break;
@@ -2131,7 +2144,7 @@ int lact_qkv_prologue_bwd(const void* xq, const void* xk, const void* xv, int64_
   return LACT_OK;
 }
 
-int lact_out_epilogue_bwd_blocks(void) { return sm_count() * 4; }
+int lact_out_epilogue_bwd_blocks(void) { return sm_count() * 2; }  // what an SM holds of out_rows_bwd_kernel
 
 int lact_out_epilogue_bwd(const void* fw_x, const void* weight, const void* gate_proj, int64_t gate_ld, const void* dout,
                           int64_t dout_ld, void* dx, void* dgate, void* dw_partial, int64_t b, int64_t s, int64_t n_heads,
@@ -2164,7 +2177,8 @@ int lact_out_epilogue_bwd(const void* fw_x, const void* weight, const void* gate
   KernelScope scope(kClsOther, static_cast<cudaStream_t>(stream));
   const unsigned grid = static_cast<unsigned>(lact_out_epilogue_bwd_blocks());
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  switch (ceil_div(d, 256)) {
+  const bool exact = with_row_shape(d, [&](auto lpr, auto v) { out_rows_bwd_kernel<lpr.value, v.value><<<grid, 256, 0, st>>>(a); });
+  if (!exact) switch (ceil_div(d, 256)) {
     case 1: out_epilogue_bwd_kernel<1><<<grid, 256, 0, st>>>(a); break;
     case 2: out_epilogue_bwd_kernel<2><<<grid, 256, 0, st>>>(a); break;
     case 3: out_epilogue_bwd_kernel<3><<<grid, 256, 0, st>>>(a); break;
@@ -2289,7 +2303,11 @@ int lact_out_epilogue(const void* fw_x, const void* weight, const void* gate_pro
   KernelScope scope(kClsOther, static_cast<cudaStream_t>(stream));
   const unsigned grid = static_cast<unsigned>(ceil_div(rows, 8));
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  switch (ceil_div(d, 256)) {
+  const bool exact = n_heads <= 65535 && with_row_shape(d, [&](auto lpr, auto v) {
+    const dim3 g(ceil_div(s, 256 / lpr.value), static_cast<unsigned>(n_heads), static_cast<unsigned>(b));
+    out_rows_kernel<lpr.value, v.value><<<g, 256, 0, st>>>(a);
+  });
+  if (!exact) switch (ceil_div(d, 256)) {
     case 1: out_epilogue_kernel<1><<<grid, 256, 0, st>>>(a); break;
     case 2: out_epilogue_kernel<2><<<grid, 256, 0, st>>>(a); break;
     case 3: out_epilogue_kernel<3><<<grid, 256, 0, st>>>(a); break;
@@ -2364,9 +2382,10 @@ int lact_swa_bwd(const void* q, const void* k, const void* v, const void* o, con
     da.delta = static_cast<float*>(delta);
     da.b = static_cast<int32_t>(b); da.L = static_cast<int32_t>(l);
     da.heads = static_cast<int32_t>(n_heads); da.d = static_cast<int32_t>(d);
-    const int64_t rows = b * l * n_heads;
+    const int64_t rows = l * n_heads;
     KernelScope scope(kClsOther, st);
-    swa_delta_kernel<<<static_cast<unsigned>(ceil_div(rows, 8)), 256, 0, st>>>(da);
+    if (d == 64) swa_delta_rows_kernel<4><<<dim3(ceil_div(rows, 64), static_cast<unsigned>(b)), 256, 0, st>>>(da);
+    else swa_delta_rows_kernel<8><<<dim3(ceil_div(rows, 32), static_cast<unsigned>(b)), 256, 0, st>>>(da);
     LACT_CUDA(cudaGetLastError());
   }
   SwaBwdArgs a;

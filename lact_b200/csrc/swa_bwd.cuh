@@ -379,26 +379,5 @@ struct SwaDeltaArgs {
   float* delta;              // [b][h][l]
   int32_t b, L, heads, d;
 };
-__global__ void __launch_bounds__(256) swa_delta_kernel(const SwaDeltaArgs a) {
-  const int64_t row = static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
-  const int64_t rows = static_cast<int64_t>(a.b) * a.L * a.heads;
-  if (row >= rows) return;
-  const int lane = threadIdx.x & 31;
-  const int h = static_cast<int>(row % a.heads);
-  const int64_t bl = row / a.heads;
-  const int tok = static_cast<int>(bl % a.L), bi = static_cast<int>(bl / a.L);
-  const bf16* po = a.o + bi * a.o_bs + tok * a.o_ts + static_cast<int64_t>(h) * a.d;
-  const bf16* pd = a.dout + bi * a.d_bs + tok * a.d_ts + static_cast<int64_t>(h) * a.d;
-  float acc = 0.f;
-  for (int c = lane * 4; c < a.d; c += 128) {
-    const uint2 uo = *reinterpret_cast<const uint2*>(po + c), ud = *reinterpret_cast<const uint2*>(pd + c);
-    acc += __uint_as_float(uo.x << 16) * __uint_as_float(ud.x << 16) +
-           __uint_as_float(uo.x & 0xFFFF0000u) * __uint_as_float(ud.x & 0xFFFF0000u) +
-           __uint_as_float(uo.y << 16) * __uint_as_float(ud.y << 16) +
-           __uint_as_float(uo.y & 0xFFFF0000u) * __uint_as_float(ud.y & 0xFFFF0000u);
-  }
-  acc = warp_sum(acc);
-  if (lane == 0) a.delta[(static_cast<int64_t>(bi) * a.heads + h) * a.L + tok] = acc;
-}
 
 }  // namespace lact
