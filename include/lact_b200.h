@@ -362,6 +362,13 @@ typedef struct lact_bmm_desc {
   int32_t a0_mn, b0_mn, a1_mn, b1_mn, c_dtype, accumulate;
 } lact_bmm_desc;
 int lact_bmm_group_bf16(const lact_bmm_desc *problems, int32_t n, int32_t *status_word, void *stream);
+/* The same where the contraction may be cut into several units per output tile (a long K over few tiles leaves SMs idle
+ * otherwise): `scratch` holds the units' fp32 sums, which the last unit of a tile adds in a fixed order.
+ * lact_bmm_group_split_bytes: bytes of scratch and uint32 words of counters the group takes, 0 where it is not cut.  The
+ * counters are zero before the first call and zero again after every one; calls that share them must follow one another. */
+int lact_bmm_group_split_bytes(const lact_bmm_desc *problems, int32_t n, size_t *bytes, int64_t *counters);
+int lact_bmm_group_split_bf16(const lact_bmm_desc *problems, int32_t n, void *counters, void *scratch, size_t scratch_bytes,
+                              int32_t *status_word, void *stream);
 
 /* The pointwise stage of lact_fw_grad alone: dy02[B, N, 2H] = [dy0 * lr0 | dy2 * lr2], hid[B, N, H] = hidden * lr1
  * (bf16) from k, v [B, N, D] (bf16; token / batch strides in elements) -- lact_fw_grad.py:25-58.  A NULL learning

@@ -114,6 +114,8 @@ def _declare(lib: C.CDLL) -> None:
     lib.lact_swa_fwd.argtypes = [vp, vp, vp, vp] + [i64] * 14 + [f32, vp, vp, vp, vp]
     lib.lact_swa_bwd.argtypes = [vp] * 10 + [i64] * 16 + [f32, vp, vp, vp]
     lib.lact_bmm_group_bf16.argtypes = [C.POINTER(BmmDesc), i32, vp, vp]
+    lib.lact_bmm_group_split_bytes.argtypes = [C.POINTER(BmmDesc), i32, szp, C.POINTER(i64)]
+    lib.lact_bmm_group_split_bf16.argtypes = [C.POINTER(BmmDesc), i32, vp, vp, C.c_size_t, vp, vp]
     lib.lact_fw_grad_pointwise.argtypes = [vp, vp, vp, i64, i64, vp, i64, i64, vp, vp, vp, i32, i64, f32, vp, vp, i64, i64,
                                            i64, i64, vp, vp]
     lib.lact_ns_trace_bwd_fused.argtypes = [C.POINTER(NsBwdGroup), i32, i32, i32, i32, vp, vp]

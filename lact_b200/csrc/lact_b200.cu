@@ -261,7 +261,7 @@ int launch_gemm(const GemmArgs<Op, NPROB>& args, cudaStream_t stream, int cls, i
   for (int p = 0; p < nprob; ++p) {
     const auto& P = args.prob[p];
     if (P.M < 1 || P.N < 1 || P.batch < 1 || P.K < 1) return LACT_ERR_SHAPE;
-    tiles += static_cast<int64_t>((P.M + kBM - 1) / kBM) * ((P.N + Op::BT - 1) / Op::BT) * P.batch;
+    tiles += static_cast<int64_t>((P.M + kBM - 1) / kBM) * ((P.N + Op::BT - 1) / Op::BT) * P.batch * std::max(1, P.splits);
   }
   if (tiles > (1ll << 30)) return LACT_ERR_SHAPE;
   const int grid = static_cast<int>(std::min<int64_t>(tiles, sm_count()));
@@ -285,6 +285,37 @@ int choose_bt(std::initializer_list<NW> probs) {
     if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = bt; }
   }
   return best;
+}
+
+// Split of a long contraction: into how many units each output tile is cut.  Few entries or small heads have few output
+// tiles (16 heads of 192: 80 on 148 SMs), and a tile of 49152 tokens is 768 k-blocks of serial work; shorter units fill the
+// SMs and even out the last round.  The rule looks at the length of the sum alone, never at the number of entries: an
+// entry's result is the same bits in any batch.  From 96 k-blocks up three units per tile, from 192 five (both odd, so that
+// tile counts just above half the SMs do not double their rounds): 16 entries of 192 and 768 k-blocks 366 -> 278 us (twelve
+// units: 335, their partial sums cost more than the rounds they even out), 8 entries and 128 k-blocks 70 -> 43 us (four:
+// 52).  Below that nothing is gained: at 32 k-blocks (4 entries of 384) 25 us either way, at 25 (12 of 128 x 256) 19 -> 23.
+struct Split {
+  int splits, kb_per_split;
+};
+Split choose_split(int64_t num_kb) {
+  if (num_kb < 96) return Split{1, static_cast<int>(num_kb)};
+  const int64_t want = num_kb < 192 ? 3 : 5;
+  const int64_t per = ((num_kb + want - 1) / want + 1) & ~1ll;  // whole ring stages of two k-blocks
+  return Split{static_cast<int>((num_kb + per - 1) / per), static_cast<int>(per)};
+}
+inline int64_t output_tiles(int64_t M, int64_t N, int64_t batch, int bt) {
+  return static_cast<int64_t>(ceil_div(M, kBM)) * ceil_div(N, bt) * batch;
+}
+struct SplitScratch {
+  float* part = nullptr;      // fp32 sums of all units: tiles x splits x 128 x bt
+  uint32_t* count = nullptr;  // a word per tile, zero
+};
+template <class P>
+void set_split(P& prob, const Split& sp, const SplitScratch& ws) {
+  prob.splits = sp.splits;
+  prob.kb_per_split = sp.kb_per_split;
+  prob.part = ws.part;
+  prob.count = ws.count;
 }
 
 // Instantiates OpT<BT> for the chosen tile width; `fill(args, bt)` populates the problems.
@@ -389,9 +420,14 @@ struct GradArgs {
   bf16* gb1 = nullptr;
   const float* g02_prev = nullptr;  // optional: momentum state read from here instead of g02 / g1 (fp32)
   const float* g1_prev = nullptr;
+  SplitScratch split;               // optional: scratch for a split contraction
 };
 
 inline int contract_bt(int64_t D, int64_t H) { return choose_bt({{D, 2 * H}, {H, D}}); }
+inline int64_t contract_tiles(int64_t B, int64_t D, int64_t H) {
+  const int bt = contract_bt(D, H);
+  return output_tiles(2 * H, D, B, bt) + output_tiles(D, H, B, bt);
+}
 
 // Pointwise stage: dy02 = [dy0 | dy2] ([B][len][2H]) and hid = hidden * lr1 ([B][len][H]) for tokens [start, end).
 int run_grad_pointwise(const GradArgs& a, int32_t* status, cudaStream_t stream) {
@@ -434,6 +470,7 @@ int run_grad(const GradArgs& a, int32_t* status, cudaStream_t stream) {
   const Mat hid{a.hid, len, a.H, a.H, a.B, len * a.H};
   // token contraction: [dw0; dw2] = dy02^T k  and  dw1 = v^T hidden
   const int bt = contract_bt(a.D, a.H);
+  const Split split = a.split.part != nullptr ? choose_split(ceil_div(len, kBK)) : Split{1, 0};
   auto fill = [&](auto& g, int btv) -> int {
     auto& P0 = g.prob[0];
     LACT_TRY(make_operand(kb_of(P0), &P0.a[0], &P0.ai[0], dy, 1, kBM, 0, 0));
@@ -449,6 +486,8 @@ int run_grad(const GradArgs& a, int32_t* status, cudaStream_t stream) {
     P1.batch = static_cast<int>(a.B);
     P1.ep = EpiDW{a.g1, a.D * a.H, a.H, a.beta, 1, a.g_f32, a.partial1, ceil_div(a.D, kBM), ceil_div(a.H, btv),
                   a.gb1, a.g1_prev};
+    set_split(P0, split, a.split);
+    set_split(P1, split, a.split);
     g.status = status;
     return LACT_OK;
   };
@@ -1054,6 +1093,8 @@ struct ScanPlan {
   int32_t* status;
   float *W02, *W1, *W02c, *W1c, *n02, *n1, *G02, *G1, *beta;
   bf16 *W02b, *W1b, *hidden, *dy02, *hid;
+  SplitScratch split;
+  int32_t split_tiles;
   NsPlan ns;
   size_t bytes;
 };
@@ -1087,6 +1128,13 @@ int plan_scan(const lact_scan_config& c, int32_t n_steps, const int32_t* kind, c
   p->hidden = cv.take<bf16>(B * static_cast<size_t>(max_apply) * H);
   p->dy02 = cv.take<bf16>(B * static_cast<size_t>(max_update) * 2 * H);
   p->hid = cv.take<bf16>(B * static_cast<size_t>(max_update) * H);
+  p->split = SplitScratch{};
+  const int splits = choose_split(ceil_div(max_update, kBK)).splits;  // (the longest update is cut into the most units)
+  p->split_tiles = splits > 1 ? static_cast<int32_t>(contract_tiles(c.B, c.D, c.H)) : 0;
+  if (splits > 1) {
+    p->split.count = cv.take<uint32_t>(p->split_tiles);
+    p->split.part = cv.take<float>(static_cast<size_t>(p->split_tiles) * splits * kBM * contract_bt(c.D, c.H));
+  }
   p->ns.ngroups = 0;
   if (c.use_muon && max_update > 0) plan_ns(cv, c.B, c.D, c.H, c.ns_concat, c.ns_gram_right, &p->ns);
   p->bytes = cv.off + 256;
@@ -1248,7 +1296,8 @@ int scan_fwd(const lact_scan_config& c, const lact_scan_io& io, int32_t n_steps,
     prepare_weights_kernel<<<ceil_div(rows, 8), 256, 0, stream>>>(io.w0, io.w1, io.w2, c.w_dtype == LACT_F32,
                                                                   static_cast<int>(B), static_cast<int>(H),
                                                                   static_cast<int>(D), W02cur, W1cur, p.W02c, p.W1c,
-                                                                  p.n02, p.n1, W02b, W1b, p.status);
+                                                                  p.n02, p.n1, W02b, W1b, p.status, p.split.count,
+                                                                  p.split_tiles);
     LACT_CUDA(cudaGetLastError());
   }
   if (has_initial_momentum(io) || n_updates == 0) LACT_TRY(load_momentum_state(c, io, p.G02, p.G1, stream));
@@ -1290,6 +1339,7 @@ int scan_fwd(const lact_scan_config& c, const lact_scan_io& io, int32_t n_steps,
                c.lr_dtype == LACT_F32, c.L, c.w_scale, p.dy02, p.hid, G02cur, G1cur, 1, beta, B, D, H};
     g.g02_prev = G02prev;
     g.g1_prev = G1prev;
+    g.split = p.split;
     // The Frobenius norms Newton-Schulz needs are gathered per output tile by the contraction when a
     // tile never straddles two matrices (concatenated [2H, D], or H a multiple of the 128-row tile).
     int fused_parts[2] = {0, 0};
@@ -1476,7 +1526,7 @@ int scan_fwd_f32(const lact_scan_config& c, const lact_scan_io& io, int32_t n_st
     KernelScope scope(kClsPrepare, stream);
     prepare_weights_kernel<<<ceil_div(B * (2 * H + D), 8), 256, 0, stream>>>(
         io.w0, io.w1, io.w2, c.w_dtype == LACT_F32, static_cast<int>(B), static_cast<int>(H), static_cast<int>(D), p.W02, p.W1,
-        p.W02c, p.W1c, p.n02, p.n1, nullptr, nullptr, p.status);
+        p.W02c, p.W1c, p.n02, p.n1, nullptr, nullptr, p.status, nullptr, 0);
     LACT_CUDA(cudaGetLastError());
   }
   if (has_initial_momentum(io) || io.m0_out) LACT_TRY(load_momentum_state(c, io, p.G02, p.G1, stream));
@@ -2456,7 +2506,20 @@ int lact_prenorm_momentum_l2norm(const void* x, const void* dx, const void* m, c
 
 // One or two independent problems c (+)= alpha (a0 b0^T [+ a1 b1^T]) in one persistent launch (both single-product
 // or both two-product; one tile width for the launch).
-static int bmm_group(const lact_bmm_desc* d, int n, int32_t* status_word, void* stream, float alpha) {
+static int group_bt(const lact_bmm_desc* d, int n) {
+  const lact_bmm_desc& l = d[n - 1];
+  const int bt = choose_bt({{d[0].N, d[0].M * d[0].batch}, {l.N, n > 1 ? l.M * l.batch : 0}});
+  return d[0].a1 != nullptr ? std::min(bt, 192) : bt;
+}
+// Split of a group whose problems are one long contraction each (single products of one K), else one unit per tile.
+static Split group_split(const lact_bmm_desc* d, int n) {
+  for (int p = 0; p < n; ++p)
+    if (d[p].a1 != nullptr || d[p].K != d[0].K) return Split{1, 0};
+  return choose_split(ceil_div(d[0].K, kBK));
+}
+
+static int bmm_group(const lact_bmm_desc* d, int n, int32_t* status_word, void* stream, float alpha,
+                     const SplitScratch& scratch = SplitScratch{}) {
   if (!d || !status_word) return LACT_ERR_NULL;
   if (n < 1 || n > 2) return LACT_ERR_CONFIG;
   LACT_TRY(check_device());
@@ -2484,9 +2547,8 @@ static int bmm_group(const lact_bmm_desc* d, int n, int32_t* status_word, void* 
   auto mat = [](const lact_bmm_desc& q, const void* ptr, int mn, int64_t rows, int64_t ld, int64_t bs) {
     return mn ? Mat{ptr, q.K, rows, ld, q.batch, bs} : Mat{ptr, rows, q.K, ld, q.batch, bs};
   };
-  const lact_bmm_desc& l = d[n - 1];
-  int bt = choose_bt({{d[0].N, d[0].M * d[0].batch}, {l.N, n > 1 ? l.M * l.batch : 0}});
-  if (two) bt = std::min(bt, 192);
+  const int bt = group_bt(d, n);
+  const Split split = scratch.part != nullptr ? group_split(d, n) : Split{1, 0};
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   auto fill = [&](auto& g, int btv) -> int {
     for (int p = 0; p < n; ++p) {
@@ -2501,12 +2563,41 @@ static int bmm_group(const lact_bmm_desc* d, int n, int32_t* status_word, void* 
       P.M = static_cast<int>(q.M); P.N = static_cast<int>(q.N); P.K = static_cast<int>(q.K);
       P.batch = static_cast<int>(q.batch);
       P.ep = EpiStore{q.c, q.c_bs, q.c_ld, 0, q.c_dtype == LACT_F32, q.accumulate, alpha};
+      set_split(P, split, scratch);
     }
     g.status = status_word;
     return LACT_OK;
   };
   if (n == 1) return two ? launch_op<OpStore2T, 1>(bt, fill, s, kClsOther, 1) : launch_op<OpStoreDirectT, 1>(bt, fill, s, kClsOther, 1);
   return two ? launch_op<OpStore2T, 2>(bt, fill, s, kClsOther, 2) : launch_op<OpStoreDirectT, 2>(bt, fill, s, kClsOther, 2);
+}
+
+int lact_bmm_group_split_bytes(const lact_bmm_desc* problems, int32_t n, size_t* bytes, int64_t* counters) {
+  if (!problems || !bytes || !counters) return LACT_ERR_NULL;
+  if (n < 1 || n > 2) return LACT_ERR_CONFIG;
+  *bytes = 0;
+  *counters = 0;
+  for (int p = 0; p < n; ++p)
+    if (problems[p].batch < 1 || problems[p].M < 1 || problems[p].N < 1 || problems[p].K < 1) return LACT_ERR_SHAPE;
+  const int splits = group_split(problems, n).splits, bt = group_bt(problems, n);
+  if (splits == 1) return LACT_OK;
+  for (int p = 0; p < n; ++p) *counters += output_tiles(problems[p].M, problems[p].N, problems[p].batch, bt);
+  *bytes = static_cast<size_t>(*counters) * splits * kBM * bt * sizeof(float);
+  return LACT_OK;
+}
+
+int lact_bmm_group_split_bf16(const lact_bmm_desc* problems, int32_t n, void* counters, void* scratch, size_t scratch_bytes,
+                              int32_t* status_word, void* stream) {
+  size_t need = 0;
+  int64_t words = 0;
+  LACT_TRY(lact_bmm_group_split_bytes(problems, n, &need, &words));
+  SplitScratch ws;
+  if (need > 0) {
+    if (!counters || !scratch) return LACT_ERR_NULL;
+    if (scratch_bytes < need || (reinterpret_cast<uintptr_t>(scratch) & 15) != 0) return LACT_ERR_WORKSPACE;
+    ws = SplitScratch{static_cast<float*>(scratch), static_cast<uint32_t*>(counters)};
+  }
+  return bmm_group(problems, n, status_word, stream, 1.0f, ws);
 }
 
 int lact_bmm_group_bf16(const lact_bmm_desc* problems, int32_t n, int32_t* status_word, void* stream) {

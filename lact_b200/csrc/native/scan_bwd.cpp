@@ -14,6 +14,17 @@
 
 namespace lact_torch {
 
+void TokenBackward::contraction(const lact_bmm_desc* d) {
+  size_t need = 0;
+  int64_t words = 0;
+  check(lact_bmm_group_split_bytes(d, 2, &need, &words), "lact_bmm_group_split_bytes");
+  if (need > 0 && (!split_count_.defined() || split_count_.numel() < words))
+    split_count_ = at::zeros({words}, like_.options().dtype(at::kInt).requires_grad(false));
+  if (need > 0 && (!split_.defined() || split_.numel() < static_cast<int64_t>(need))) split_ = bytes(need, like_);
+  check(lact_bmm_group_split_bf16(d, 2, need > 0 ? ptr(split_count_) : nullptr, need > 0 ? ptr(split_) : nullptr, need, status_, stream_),
+        "lact_bmm_group_split_bf16");
+}
+
 void TokenBackward::apply(View w02, View w1, View q, View dO, int64_t n, View dW02, View dW1, bool accumulate, View dq) {
   const View dy = plane(a_, n, 2 * H_), hid = plane(b_, n, H_);
   // pre-activations y0, y2 = q w0^T, q w2^T and dh = dO w1 with the pointwise stage in their epilogue
@@ -22,7 +33,7 @@ void TokenBackward::apply(View w02, View w1, View q, View dO, int64_t n, View dW
         "lact_fw_grad_pointwise");
   const lact_bmm_desc dw[2] = {product(dy, true, q, true, dW02, LACT_F32, accumulate, B_, 2 * H_, D_, n),
                                product(dO, true, hid, true, dW1, LACT_F32, accumulate, B_, D_, H_, n)};
-  check(lact_bmm_group_bf16(dw, 2, status_, stream_), "lact_bmm_group_bf16");
+  contraction(dw);
   const lact_bmm_desc dx = product(dy, false, w02, true, dq, LACT_BF16, false, B_, n, D_, 2 * H_);
   check(lact_bmm_group_bf16(&dx, 1, status_, stream_), "lact_bmm_group_bf16");
 }
@@ -49,7 +60,7 @@ void TokenBackward::gradient(View w02, View w1, View k, View v, int64_t n, const
   check(lact_bmm_group_bf16(p2, 2, status_, stream_), "lact_bmm_group_bf16");
   const lact_bmm_desc p3[2] = {product(gy, true, k, true, dW02, LACT_F32, accumulate, B_, 2 * H_, D_, n),
                                product(v, true, gdh, true, dW1, LACT_F32, accumulate, B_, D_, H_, n)};
-  check(lact_bmm_group_bf16(p3, 2, status_, stream_), "lact_bmm_group_bf16");
+  contraction(p3);
 }
 
 namespace {

@@ -49,6 +49,7 @@ class TokenBackward {
                 bool glr_add);
 
  private:
+  void contraction(const lact_bmm_desc* d);  // two products summed over tokens
   View plane(Tensor& t, int64_t n, int64_t width) {
     if (!t.defined() || t.size(1) != n || t.size(2) != width) t = empty({B_, n, width}, at::kBFloat16, like_);
     return View(t);
@@ -58,6 +59,7 @@ class TokenBackward {
   int32_t* status_;
   void* stream_;
   Tensor a_, b_, c_, d_, e_, f_, g_, h_;
+  Tensor split_, split_count_;  // scratch of split contractions, once one is
 };
 
 }  // namespace lact_torch

@@ -182,6 +182,7 @@ __host__ __device__ constexpr int ring_depth(uint32_t stage_bytes, uint32_t stag
 // c = a b^T, one accumulator, direct (register) epilogue `EpiT`; output tile 128 x BT.
 template <class EpiT, int BT_>
 struct OpBmm {
+  static constexpr bool kSplitK = true;
   static constexpr int NA = 1, NB = 1, NACC = 1, BT = BT_, NTERMS = 1, NOUT = 0;
   static constexpr bool kTileReduce = false;
   static constexpr bool kWarpTranspose = true, kReverseBatch = false;
@@ -207,6 +208,7 @@ struct OpBmm {
 // then warp shuffle; the consumer adds them in a fixed order, so the norm is deterministic).
 template <int BT_>
 struct OpDW {
+  static constexpr bool kSplitK = true;
   static constexpr int NA = 1, NB = 1, NACC = 1, BT = BT_, NTERMS = 1, NOUT = 0;
   static constexpr bool kTileReduce = true;
   static constexpr bool kWarpTranspose = true;                   // results reach global memory through `EpiDW::warp_block`
@@ -465,10 +467,12 @@ __device__ __forceinline__ float warp_sum(float x) {
 // One warp per weight row.  Also clears the program's status word.
 __global__ void prepare_weights_kernel(const void* w0, const void* w1, const void* w2, int w_f32, int B, int H, int D,
                                        float* W02, float* W1, float* W02c, float* W1c, float* n02, float* n1,
-                                       bf16* W02b, bf16* W1b, int32_t* status) {
+                                       bf16* W02b, bf16* W1b, int32_t* status, uint32_t* split_count, int split_tiles) {
   griddep_launch_dependents();
   griddep_wait();
   if (blockIdx.x == 0 && threadIdx.x == 0) *status = kStatusOk;  // the first kernel of a program
+  // arrival counters of the program's split contractions
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < split_tiles; i += gridDim.x * blockDim.x) split_count[i] = 0;
   const int rows_per_b = 2 * H + D;
   const int64_t r = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (r >= static_cast<int64_t>(B) * rows_per_b) return;

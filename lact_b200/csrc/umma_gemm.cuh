@@ -43,6 +43,13 @@ struct GemmProblem {
   OutInfo oi[Op::NOUT > 0 ? Op::NOUT : 1];
   int32_t M, N, K, batch;
   typename Op::Epi ep;
+  // Split contraction (ops with `kSplitK`; `splits` > 1): the k-blocks of every output tile are dealt to `splits` units of
+  // `kb_per_split` k-blocks each.  A unit leaves its fp32 sums in `part`; the unit that finds the tile's word of `count` at
+  // splits - 1 is the last to arrive, adds all of them in their order (the same result whoever is last), runs the epilogue
+  // and sets the word back to zero.  Nothing waits for another unit.
+  int32_t splits, kb_per_split;
+  float* part;      // [tile of the launch][split][128 * BT]
+  uint32_t* count;  // [tile of the launch], zero before and after the launch
 };
 
 template <class Op, int NPROB>
@@ -109,6 +116,7 @@ __device__ __forceinline__ void load_operand_tile(uint32_t leader, uint32_t dst,
 
 struct TileCoord {
   int prob, batch, m0, n0;
+  int slot, split;  // split contractions: running number of the output tile, and which share of its k-blocks
 };
 
 // Ops whose output is a symmetric M x M matrix (both operands the same rows) may declare `kSymmetric`: only the
@@ -123,6 +131,12 @@ template <class Op>
 __host__ __device__ constexpr uint32_t gemm_staging_bytes() {
   return (Op::NOUT + (op_symmetric<Op>::value ? 1 : 0)) * kBM * Op::BT * 2 + Op::kEpiScratch;
 }
+
+// Ops whose contraction may be split over several units (see GemmProblem): direct epilogues, single-phase kernels.
+template <class Op, class = void>
+struct op_split { static constexpr bool value = false; };
+template <class Op>
+struct op_split<Op, decltype(void(Op::kSplitK))> { static constexpr bool value = Op::kSplitK; };
 
 // Per-thread view of the CTA's pipeline resources and of this thread's progress counters.  The
 // producer thread advances `it`, the MMA thread `it` and `tcount`, epilogue threads `tcount`;
@@ -142,6 +156,7 @@ struct GemmCtx {
   uint32_t ptile = 0;            // tiles whose dependency has been verified (scout) / consumed (producer)
   uint32_t sround = 0;           // staging hand-overs so far (epilogue threads and the storing thread count alike)
   uint32_t* dep_ok = nullptr;    // shared-memory word: tiles verified by the scout warp, read by the producer thread
+  volatile uint32_t* last_unit = nullptr;  // shared-memory word: this unit completes its tile (split contractions)
 };
 
 struct NoPatch {
@@ -235,7 +250,9 @@ __device__ __forceinline__ bool gemm_phase(GemmCtx& cx, const GemmProblem<Op>* p
 
   constexpr bool SYM = op_symmetric<Op>::value;
   static_assert(!SYM || (BT == kBM && Op::NOUT == 1 && Deps::kOn), "symmetric ops: 128-wide tiles, one staged output, dataflow");
-  int tiles_of[kMaxProb], tn_of[kMaxProb], tm_of[kMaxProb], per_batch_of[kMaxProb];
+  constexpr bool SPLIT = op_split<Op>::value;
+  static_assert(!SPLIT || (Op::NOUT == 0 && Op::kWarpTranspose && !Deps::kOn), "split contractions: direct epilogue, one phase");
+  int tiles_of[kMaxProb], tn_of[kMaxProb], tm_of[kMaxProb], per_batch_of[kMaxProb], splits_of[kMaxProb];
   int total_tiles = 0;
 #pragma unroll
   for (int p = 0; p < kMaxProb; ++p) {
@@ -243,9 +260,10 @@ __device__ __forceinline__ bool gemm_phase(GemmCtx& cx, const GemmProblem<Op>* p
       tn_of[p] = (probs[p].N + BT - 1) / BT;
       tm_of[p] = (probs[p].M + kBM - 1) / kBM;
       per_batch_of[p] = SYM ? tm_of[p] * (tm_of[p] + 1) / 2 : tn_of[p] * tm_of[p];
-      tiles_of[p] = per_batch_of[p] * probs[p].batch;
+      splits_of[p] = SPLIT && probs[p].splits > 1 ? probs[p].splits : 1;
+      tiles_of[p] = per_batch_of[p] * probs[p].batch * splits_of[p];
     } else {
-      tn_of[p] = tm_of[p] = per_batch_of[p] = 1;
+      tn_of[p] = tm_of[p] = per_batch_of[p] = splits_of[p] = 1;
       tiles_of[p] = 0;
     }
     total_tiles += tiles_of[p];
@@ -253,10 +271,21 @@ __device__ __forceinline__ bool gemm_phase(GemmCtx& cx, const GemmProblem<Op>* p
   auto coord = [&](int tile) {
     TileCoord c;
     c.prob = 0;
-    if (tile >= tiles_of[0]) { tile -= tiles_of[0]; c.prob = 1; }
+    c.slot = c.split = 0;
+    if (tile >= tiles_of[0]) {
+      tile -= tiles_of[0];
+      c.prob = 1;
+      if constexpr (SPLIT) c.slot = tiles_of[0] / splits_of[0];
+    }
     const int per_batch = per_batch_of[c.prob];
     c.batch = tile / per_batch;
     int r = tile - c.batch * per_batch;
+    if constexpr (SPLIT) {  // the units of one batch entry and split are consecutive: they share operand tiles
+      const int unit = c.batch;
+      c.batch = unit / splits_of[c.prob];
+      c.split = unit - c.batch * splits_of[c.prob];
+      c.slot += c.batch * per_batch + r;
+    }
     // a consumer of large intermediates walks the batch entries backwards: the entries its producer wrote last
     // are the ones still in L2
     if constexpr (Op::kReverseBatch) c.batch = probs[c.prob].batch - 1 - c.batch;
@@ -271,6 +300,18 @@ __device__ __forceinline__ bool gemm_phase(GemmCtx& cx, const GemmProblem<Op>* p
       c.n0 = (r % tn_of[c.prob]) * BT;
     }
     return c;
+  };
+
+  // the k-blocks [first, last) of a unit
+  auto k_range = [&](const GemmProblem<Op>& P, const TileCoord& tc, int& first, int& last) {
+    first = 0;
+    last = (P.K + kBK - 1) / kBK;
+    if constexpr (SPLIT) {
+      if (splits_of[tc.prob] > 1) {
+        first = tc.split * P.kb_per_split;
+        last = min(last, first + P.kb_per_split);
+      }
+    }
   };
 
   const int rounds = (total_tiles + gridDim.x - 1) / gridDim.x;
@@ -292,19 +333,20 @@ __device__ __forceinline__ bool gemm_phase(GemmCtx& cx, const GemmProblem<Op>* p
         if (tile >= total_tiles) continue;
         const TileCoord tc = coord(tile);
         const GemmProblem<Op>& P = probs[tc.prob];
-        const int num_kb = (P.K + kBK - 1) / kBK;
+        int kb0, kb1;
+        k_range(P, tc, kb0, kb1);
         if constexpr (Deps::kOn) {
           if (!__all_sync(0xFFFFFFFFu, flow_wait_verified(cx, cx.ptile++))) { failed = true; break; }  // the scout warp checked this tile
           asm volatile("fence.proxy.async;" ::: "memory");
         }
-        const int num_sb = (num_kb + KB - 1) / KB;  // ring stages of KB k-blocks
+        const int num_sb = (kb1 - kb0 + KB - 1) / KB;  // ring stages of KB k-blocks
         for (int sb = 0; sb < num_sb; ++sb, ++cx.it) {
           const int s = cx.it % RING;
           const uint32_t ph = (cx.it / RING) & 1;
           if (!mbar_wait_warp(&cx.empty_bar[s], ph ^ 1, cx.abort_flag)) { failed = true; break; }
           mbar_expect_tx_if(leader, &cx.full_bar[s], kStageBytes);
           const uint32_t st = cx.smem_base + s * cx.stage_stride;
-          const int kc = sb * KB * kBK;
+          const int kc = (kb0 + sb * KB) * kBK;
 #pragma unroll
           for (int i = 0; i < NA; ++i)
             load_operand_tile<kBM, KB>(leader, st + i * (KB * kATileBytes), &P.a[i], P.ai[i], tc.m0, kc, tc.batch, &cx.full_bar[s]);
@@ -324,7 +366,9 @@ __device__ __forceinline__ bool gemm_phase(GemmCtx& cx, const GemmProblem<Op>* p
         if (tile >= total_tiles) continue;
         const TileCoord tc = coord(tile);
         const GemmProblem<Op>& P = probs[tc.prob];
-        const int num_kb = (P.K + kBK - 1) / kBK;
+        int kb0, kb1;
+        k_range(P, tc, kb0, kb1);
+        const int num_kb = kb1 - kb0;
         const uint32_t as = cx.tcount & 1, aph = (cx.tcount >> 1) & 1;
         if (!mbar_wait_warp(&cx.acc_empty_bar[as], aph ^ 1, cx.abort_flag)) { failed = true; break; }
         tc_fence_after();
@@ -476,7 +520,75 @@ __device__ __forceinline__ bool gemm_phase(GemmCtx& cx, const GemmProblem<Op>* p
         named_barrier_sync(1, kEpiThreads);
         if (cx.abort_flag[1] != 0) { failed = true; break; }
       } else {
+        if constexpr (SPLIT) {
+          // (as above: the warps of a split tile meet at named barriers, so they give up together)
+          if (splits_of[tc.prob] > 1) {
+            if (!got) cx.abort_flag[1] = 1;
+            named_barrier_sync(1, kEpiThreads);
+            got = cx.abort_flag[1] == 0;
+          }
+        }
         if (!got) { failed = true; break; }
+      }
+      if constexpr (SPLIT) {
+        if (splits_of[tc.prob] > 1) {
+          // this unit's sums: 32 x 32 blocks, sixteen bytes per lane and store
+          const int splits = splits_of[tc.prob];
+          constexpr int kTileF4 = kBM * BT / 4;
+          float4* const tile_part = reinterpret_cast<float4*>(P.part) + static_cast<int64_t>(tc.slot) * splits * kTileF4;
+          float4* const mine = tile_part + static_cast<int64_t>(tc.split) * kTileF4;
+          for (int c = half * 32; c < BT; c += 64) {
+            if (tc.n0 + c >= P.N) break;
+            uint32_t bits[32];
+            tmem_ld32(acc_base + c, bits);
+            tmem_ld_wait();
+            float4* const blk = mine + (quarter * (BT / 32) + (c >> 5)) * 256 + lane;
+#pragma unroll
+            for (int g = 0; g < 8; ++g)
+              __stcg(blk + g * 32, make_float4(__uint_as_float(bits[g * 4]), __uint_as_float(bits[g * 4 + 1]),
+                                               __uint_as_float(bits[g * 4 + 2]), __uint_as_float(bits[g * 4 + 3])));
+          }
+          tc_fence_before();
+          __threadfence();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&cx.acc_empty_bar[as]);
+          named_barrier_sync(2, kEpiThreads);
+          if (elected) {
+            const bool last = atomicAdd(P.count + tc.slot, 1u) == static_cast<uint32_t>(splits - 1);
+            __threadfence();
+            if (last) P.count[tc.slot] = 0;
+            *cx.last_unit = last;
+          }
+          named_barrier_sync(1, kEpiThreads);
+          if (*cx.last_unit != 0) {
+            for (int c = half * 32; c < BT; c += 64) {
+              if (tc.n0 + c >= P.N) break;
+              float v[NACC][32];
+#pragma unroll
+              for (int j = 0; j < 32; ++j) v[0][j] = 0.f;
+              const float4* blk = tile_part + (quarter * (BT / 32) + (c >> 5)) * 256 + lane;
+              for (int s = 0; s < splits; ++s, blk += kTileF4) {
+                float4 x[8];
+#pragma unroll
+                for (int g = 0; g < 8; ++g) x[g] = __ldcg(blk + g * 32);
+#pragma unroll
+                for (int g = 0; g < 8; ++g) {
+                  v[0][g * 4] += x[g].x; v[0][g * 4 + 1] += x[g].y; v[0][g * 4 + 2] += x[g].z; v[0][g * 4 + 3] += x[g].w;
+                }
+              }
+              Op::epilogue_warp(ep, tc.batch, tc.m0 + quarter * 32, tc.n0 + c, P.M, P.N, v, pf,
+                                cx.staging + (warp - 2) * (32 * 144), lane);
+            }
+            if constexpr (Op::kTileReduce) {
+              float tv = Op::tile_value(pf);
+#pragma unroll
+              for (int o = 16; o > 0; o >>= 1) tv += __shfl_xor_sync(0xFFFFFFFFu, tv, o);
+              if (lane == 0) Op::tile_store(ep, tc.batch, tc.m0 / kBM, tc.n0 / BT, warp - 2, tv);
+            }
+          }
+          ++cx.tcount;
+          continue;
+        }
       }
       for (int c = half * 32; c < BT; c += 64) {
         if (tc.n0 + c >= P.N) break;  // warp-uniform
@@ -591,6 +703,7 @@ __device__ __forceinline__ void gemm_setup(GemmCtx& cx, uint8_t* smem_raw, int r
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(cx.stg_empty_bar + 1);
   cx.abort_flag = tmem_slot + 1;  // [2]
   cx.dep_ok = tmem_slot + 3;
+  cx.last_unit = tmem_slot + 4;
   if (threadIdx.x == 0) {
     for (int s = 0; s < ring; ++s) {
       mbar_init(&cx.full_bar[s], 1);
