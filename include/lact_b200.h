@@ -296,6 +296,15 @@ int lact_swa_fwd(const void *q, const void *k, const void *v, void *o, int64_t b
                  int64_t d, int64_t q_ts, int64_t q_bs, int64_t k_ts, int64_t k_bs, int64_t v_ts, int64_t v_bs, int64_t o_ts,
                  int64_t o_bs, int64_t window, float softmax_scale, const int32_t *seq_start, void *lse,
                  int32_t *status_word, void *stream);
+/* The same with query tiles cut over their keys where whole tiles would leave SMs idle (few of them, or a short last round).
+ * lact_swa_fwd_split_bytes: bytes of scratch (16-byte aligned) and uint32 words of counters (zero before every call) it
+ * takes; both 0 where nothing is cut.  counters or scratch NULL: nothing is cut. */
+int lact_swa_fwd_split_bytes(int64_t b, int64_t l, int64_t lk, int64_t n_heads, int64_t d, int64_t window, size_t *bytes,
+                             int64_t *counters);
+int lact_swa_fwd_split(const void *q, const void *k, const void *v, void *o, int64_t b, int64_t l, int64_t lk, int64_t n_heads,
+                 int64_t d, int64_t q_ts, int64_t q_bs, int64_t k_ts, int64_t k_bs, int64_t v_ts, int64_t v_bs, int64_t o_ts,
+                 int64_t o_bs, int64_t window, float softmax_scale, const int32_t *seq_start, void *lse,
+                 void *counters, void *scratch, size_t scratch_bytes, int32_t *status_word, void *stream);
 
 /* Backward of lact_swa_fwd: dq (bf16, contiguous [b, l, n_heads, d]) and dk, dv ([b, lk, n_heads, d]), written, from the forward's inputs, its
  * output o, its lse and the output gradient dout (bf16, token / batch strides in elements).  delta: fp32 scratch

@@ -112,6 +112,8 @@ def _declare(lib: C.CDLL) -> None:
     lib.lact_out_epilogue_bwd_blocks.restype = C.c_int
     lib.lact_out_epilogue_bwd.argtypes = [vp, vp, vp, i64, vp, i64, vp, vp, vp, i64, i64, i64, i64, f32, vp]
     lib.lact_swa_fwd.argtypes = [vp, vp, vp, vp] + [i64] * 14 + [f32, vp, vp, vp, vp]
+    lib.lact_swa_fwd_split_bytes.argtypes = [i64] * 6 + [szp, C.POINTER(i64)]
+    lib.lact_swa_fwd_split.argtypes = [vp, vp, vp, vp] + [i64] * 14 + [f32, vp, vp, vp, vp, C.c_size_t, vp, vp]
     lib.lact_swa_bwd.argtypes = [vp] * 10 + [i64] * 16 + [f32, vp, vp, vp]
     lib.lact_bmm_group_bf16.argtypes = [C.POINTER(BmmDesc), i32, vp, vp]
     lib.lact_bmm_group_split_bytes.argtypes = [C.POINTER(BmmDesc), i32, szp, C.POINTER(i64)]

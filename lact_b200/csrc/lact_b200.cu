@@ -2367,10 +2367,55 @@ int lact_out_epilogue(const void* fw_x, const void* weight, const void* gate_pro
   return LACT_OK;
 }
 
+// Which query tiles of an attention launch are cut over their keys, and into how many CTAs.  Whole tiles fill whole rounds
+// of the SMs (a CTA takes an SM's shared memory); the rest, all tiles where there are fewer than SMs, are cut so that the
+// launch ends sooner: a CTA takes about 4 us plus 1.5 us per 128 keys (1.2 at d = 64), combining about 0.6 us per share.
+// Measured: 1560 queries over 4680 keys, 12 heads of 128 (156 tiles on 148 SMs, the last 8 cut in 8) 110 -> 80 us.
+struct SwaSplit {
+  int64_t whole;
+  int splits;
+};
+static SwaSplit swa_split(int64_t b, int64_t l, int64_t lk, int64_t heads, int64_t d, int64_t window) {
+  const int64_t sms = sm_count(), tiles = b * heads * ceil_div(l, 128);
+  const int64_t span = window < 0 ? (lk > 0 ? lk : l) : window > 0 && window < l ? std::min(l, window + 127) : l;
+  const int64_t T = ceil_div(span, 128), rest = tiles % sms;
+  SwaSplit best{tiles, 1};
+  if (rest == 0 || tiles > 64 * sms) return best;
+  const double per_tile = d == 64 ? 1.2 : 1.5;
+  double cost = T * per_tile + 4.0;
+  for (int s = 2; s <= 16 && s <= T; ++s) {
+    const double c = ((rest * s + sms - 1) / sms) * (((T + s - 1) / s) * per_tile + 4.0) + 2.0 + 0.6 * s;
+    if (c < 0.9 * cost) {
+      cost = c;
+      best = SwaSplit{tiles - rest, s};
+    }
+  }
+  return best;
+}
+
+int lact_swa_fwd_split_bytes(int64_t b, int64_t l, int64_t lk, int64_t n_heads, int64_t d, int64_t window, size_t* bytes,
+                             int64_t* counters) {
+  if (!bytes || !counters) return LACT_ERR_NULL;
+  if ((d != 64 && d != 128) || b < 1 || l < 1 || n_heads < 1 || b > 65535 || n_heads > 65535 || l > (1ll << 30) || lk > (1ll << 30))
+    return LACT_ERR_SHAPE;
+  const SwaSplit sp = swa_split(b, l, lk, n_heads, d, window);
+  *counters = sp.splits > 1 ? b * n_heads * ceil_div(l, 128) - sp.whole : 0;
+  *bytes = static_cast<size_t>(*counters) * sp.splits * (128 * d * sizeof(float) + 256 * sizeof(float2));
+  return LACT_OK;
+}
+
 int lact_swa_fwd(const void* q, const void* k, const void* v, void* o, int64_t b, int64_t l, int64_t lk, int64_t n_heads,
                  int64_t d, int64_t q_ts, int64_t q_bs, int64_t k_ts, int64_t k_bs, int64_t v_ts, int64_t v_bs, int64_t o_ts,
                  int64_t o_bs, int64_t window, float softmax_scale, const int32_t* seq_start, void* lse, int32_t* status_word,
                  void* stream) {
+  return lact_swa_fwd_split(q, k, v, o, b, l, lk, n_heads, d, q_ts, q_bs, k_ts, k_bs, v_ts, v_bs, o_ts, o_bs, window, softmax_scale,
+                            seq_start, lse, nullptr, nullptr, 0, status_word, stream);
+}
+
+int lact_swa_fwd_split(const void* q, const void* k, const void* v, void* o, int64_t b, int64_t l, int64_t lk, int64_t n_heads,
+                       int64_t d, int64_t q_ts, int64_t q_bs, int64_t k_ts, int64_t k_bs, int64_t v_ts, int64_t v_bs, int64_t o_ts,
+                       int64_t o_bs, int64_t window, float softmax_scale, const int32_t* seq_start, void* lse, void* counters,
+                       void* scratch, size_t scratch_bytes, int32_t* status_word, void* stream) {
   if (!q || !k || !v || !o || !status_word) return LACT_ERR_NULL;
   if (seq_start != nullptr && b != 1) return LACT_ERR_CONFIG;   // packed sequences live in one batch entry
   const bool causal = window >= 0;
@@ -2399,8 +2444,25 @@ int lact_swa_fwd(const void* q, const void* k, const void* v, void* o, int64_t b
   a.lse = static_cast<float*>(lse);
   a.seq_start = seq_start;
   a.status = status_word;
-  const int64_t ctas = b * n_heads * a.q_tiles;
+  int64_t ctas = b * n_heads * a.q_tiles;
   if (ctas > 0x7FFFFFFFll) return LACT_ERR_SHAPE;
+  a.whole = static_cast<int32_t>(ctas);
+  a.splits = 1;
+  if (scratch != nullptr && counters != nullptr) {
+    const SwaSplit sp = swa_split(b, l, lk, n_heads, d, window);
+    const int64_t rest = ctas - sp.whole;
+    const size_t rows = static_cast<size_t>(rest) * sp.splits;
+    if (sp.splits > 1) {
+      if (scratch_bytes < rows * (128 * d * sizeof(float) + 256 * sizeof(float2)) || (reinterpret_cast<uintptr_t>(scratch) & 15) != 0)
+        return LACT_ERR_WORKSPACE;
+      a.whole = static_cast<int32_t>(sp.whole);
+      a.splits = sp.splits;
+      a.part = static_cast<float4*>(scratch);
+      a.ml = reinterpret_cast<float2*>(static_cast<uint8_t*>(scratch) + rows * 128 * d * sizeof(float));
+      a.count = static_cast<uint32_t*>(counters);
+      ctas = sp.whole + rest * sp.splits;
+    }
+  }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   return d == 64 ? launch_swa<64>(a, ctas, st) : launch_swa<128>(a, ctas, st);
 }

@@ -34,9 +34,18 @@ std::vector<Tensor> swa(const Tensor& q_, const Tensor& k_, const Tensor& v_, in
   const Tensor q = head_view(q_), k = head_view(k_), v = head_view(v_);
   const int64_t b = q.size(0), l = q.size(1), h = q.size(2), d = q.size(3), lk = k.size(1);
   Tensor o = empty({b, l, h, d}, at::kBFloat16, q), lse = empty({b, h, l}, at::kFloat, q);
-  check(lact_swa_fwd(ptr(q), ptr(k), ptr(v), ptr(o), b, l, lk, h, d, q.stride(1), q.stride(0), k.stride(1), k.stride(0), v.stride(1),
+  size_t need = 0;
+  int64_t words = 0;
+  if (lact_swa_fwd_split_bytes(b, l, lk, h, d, window, &need, &words) != LACT_OK) need = 0;  // the call below reports it
+  Tensor scratch, counters;
+  if (need > 0) {
+    scratch = bytes(need, q);
+    counters = at::zeros({words}, q.options().dtype(at::kInt).requires_grad(false));
+  }
+  check(lact_swa_fwd_split(ptr(q), ptr(k), ptr(v), ptr(o), b, l, lk, h, d, q.stride(1), q.stride(0), k.stride(1), k.stride(0), v.stride(1),
                      v.stride(0), o.stride(1), o.stride(0), window, static_cast<float>(scale), static_cast<const int32_t*>(ptr(seq)),
-                     ptr(lse), status_word(q), stream_of(q)),
+                     ptr(lse), need > 0 ? ptr(counters) : nullptr, need > 0 ? ptr(scratch) : nullptr, need, status_word(q),
+                     stream_of(q)),
         "lact_swa_fwd");
   return {o, lse};
 }

@@ -32,6 +32,14 @@ struct SwaArgs {
                              // keys before it are invisible), or nullptr: one sequence per batch entry
   float* lse;            // optional [b][h][l]: log2-domain log-sum-exp of every row (the backward's input), or nullptr
   int32_t* status;
+  // Tiles from `whole` on (in grid order) are cut into `splits` CTAs, each over a share of the tile's key tiles: fewer query
+  // tiles than SMs, or a last round of them, would leave SMs idle.  A CTA leaves its unnormalised output rows, maxima and
+  // sums in `part` / `ml`; the last of a tile to arrive (its word of `count`, zero at launch) combines all of them in their
+  // order and writes the result.  Nothing waits.
+  int32_t whole, splits;
+  float4* part;      // [tile - whole][split][HD / 8][256 threads]
+  float2* ml;        // [tile - whole][split][256 threads]: maximum, this thread's share of the sum
+  uint32_t* count;   // [tile - whole]
 };
 
 // 2^x by the hardware approximation (2^-inf = 0)
@@ -71,6 +79,7 @@ __global__ void __launch_bounds__(320, 1) swa_fwd_kernel(const __grid_constant__
   uint64_t* o_empty = bars + 15;      // [2]  8 arrivals
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
   volatile uint32_t* abort_flag = tmem_slot + 1;
+  volatile uint32_t* last_flag = tmem_slot + 2;   // this CTA completes a split tile
   float* xch = reinterpret_cast<float*>(aligned + SM::kBars + 256);   // [2 halves][128 rows]
 
   const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
@@ -99,9 +108,16 @@ __global__ void __launch_bounds__(320, 1) swa_fwd_kernel(const __grid_constant__
   const uint32_t tmem = uniform(*tmem_slot);
 
   // this CTA's query tile and the key tiles its window touches
-  const int qt = blockIdx.x % a.q_tiles;
-  const int head = (blockIdx.x / a.q_tiles) % a.heads;
-  const int batch = blockIdx.x / (a.q_tiles * a.heads);
+  int tile = blockIdx.x, splits = 1, split = 0;
+  if (tile >= a.whole) {
+    const int u = tile - a.whole;
+    splits = a.splits;
+    tile = a.whole + u / splits;
+    split = u % splits;
+  }
+  const int qt = tile % a.q_tiles;
+  const int head = (tile / a.q_tiles) % a.heads;
+  const int batch = tile / (a.q_tiles * a.heads);
   const int q0 = qt * 128;
   const int window = a.window > 0 ? a.window : a.L;
   int kv_lo = q0 - (window - 1);
@@ -114,12 +130,17 @@ __global__ void __launch_bounds__(320, 1) swa_fwd_kernel(const __grid_constant__
     kv_lo = 0;
     kv_hi = a.Lk;
   }
-  const int T = (kv_hi - kv_lo + 127) / 128;
+  int T = (kv_hi - kv_lo + 127) / 128;
+  if (splits > 1) {   // this CTA's share of the key tiles (none, if there are fewer of them than shares)
+    const int per = (T + splits - 1) / splits, t0 = min(T, split * per);
+    T = min(T, t0 + per) - t0;
+    kv_lo += t0 * 128;
+  }
   bool failed = uniform(static_cast<uint32_t>(*reinterpret_cast<volatile int32_t*>(a.status))) != kStatusOk;
 
   if (warp == 0) {
     const uint32_t leader = elect_leader();
-    if (!failed) {
+    if (!failed && T > 0) {
       mbar_expect_tx_if(leader, q_full, SM::kTile);
       for (int j = 0; j < KBD; ++j) tma_load_4d_if(leader, base + SM::kQ + j * kBox, &a.q, q_full, 64 * j, q0, head, batch);
       for (int t = 0; t < T && !failed; ++t) {
@@ -155,7 +176,7 @@ __global__ void __launch_bounds__(320, 1) swa_fwd_kernel(const __grid_constant__
         umma_commit_if(leader, &k_empty[sb]);
         return true;
       };
-      if (!mbar_wait_warp(q_full, 0, abort_flag)) failed = true;
+      if (T > 0 && !mbar_wait_warp(q_full, 0, abort_flag)) failed = true;
       for (int t = 0; t < T && !failed; ++t) {
         const int sb = t & 1;
         if (t == 0 && !issue_s(0)) { failed = true; break; }
@@ -302,8 +323,50 @@ __global__ void __launch_bounds__(320, 1) swa_fwd_kernel(const __grid_constant__
       a_prev = alpha;
     }
     if (!failed && T > 0 && !fold(T - 1, a_prev)) failed = true;
+    bool store = true;
+    if (splits > 1) {
+      // (every softmax thread meets the others here, whatever its waits returned)
+      const int thr = threadIdx.x - 64;
+      constexpr int kO4 = OC / 4;
+      const int64_t first = static_cast<int64_t>(tile - a.whole) * splits;
+      float4* const mine = a.part + (first + split) * (kO4 * 256) + thr;
+#pragma unroll
+      for (int c = 0; c < kO4; ++c) __stcg(mine + c * 256, make_float4(O[4 * c], O[4 * c + 1], O[4 * c + 2], O[4 * c + 3]));
+      __stcg(a.ml + (first + split) * 256 + thr, make_float2(m, l));
+      __threadfence();
+      named_barrier_sync(5, 256);
+      if (thr == 0) {
+        *last_flag = atomicAdd(a.count + (tile - a.whole), 1u) == static_cast<uint32_t>(splits - 1);
+        __threadfence();
+      }
+      named_barrier_sync(5, 256);
+      store = *last_flag != 0;
+      if (store && !failed) {
+        const float2* const ml = a.ml + first * 256 + thr;
+        m = -INFINITY;
+        for (int s = 0; s < splits; ++s) m = fmaxf(m, __ldcg(ml + s * 256).x);
+        l = 0.f;
+#pragma unroll
+        for (int j = 0; j < OC; ++j) O[j] = 0.f;
+        const float4* src = a.part + first * (kO4 * 256) + thr;
+        for (int s = 0; s < splits; ++s, src += kO4 * 256) {
+          const float2 ms = __ldcg(ml + s * 256);
+          if (ms.x == -INFINITY) continue;   // this share saw no key of the row
+          const float w = fast_exp2(ms.x - m);
+          l = fmaf(ms.y, w, l);
+#pragma unroll
+          for (int c = 0; c < kO4; ++c) {
+            const float4 x = __ldcg(src + c * 256);
+            O[4 * c] = fmaf(x.x, w, O[4 * c]);
+            O[4 * c + 1] = fmaf(x.y, w, O[4 * c + 1]);
+            O[4 * c + 2] = fmaf(x.z, w, O[4 * c + 2]);
+            O[4 * c + 3] = fmaf(x.w, w, O[4 * c + 3]);
+          }
+        }
+      }
+    }
     const float l_other = exchange(l);
-    if (!failed && qi < a.L) {
+    if (!failed && store && qi < a.L) {
       const float tot = l + l_other;
       const float inv = tot > 0.f ? 1.0f / tot : 0.f;
       if (a.lse != nullptr && half == 0) a.lse[(static_cast<int64_t>(batch) * a.heads + head) * a.L + qi] = m + log2f(tot);
