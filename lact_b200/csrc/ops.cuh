@@ -1246,8 +1246,8 @@ __global__ void __launch_bounds__(256, ROPE ? (NCH <= 2 ? 4 : 2) : (NCH <= 2 ? 8
           if (a.silu[t]) {
             // fast exponential and divide: their fp32 error (a few ulp) moves the bf16 rounding of about one value
             // in ten thousand by one ulp
-            lo = bf16_round(__fdividef(lo, 1.f + __expf(-lo)));
-            hi = bf16_round(__fdividef(hi, 1.f + __expf(-hi)));
+            lo = bf16_round(lo * sigmoidf_fast(lo));
+            hi = bf16_round(hi * sigmoidf_fast(hi));
           }
           y[c][2 * i] = lo;
           y[c][2 * i + 1] = hi;
@@ -1475,7 +1475,7 @@ __global__ void __launch_bounds__(256, NCH <= 2 ? 8 : 4) out_epilogue_kernel(con
       float gt[8];
       load8_bf16(a.gate + bs_idx * a.gate_ld + off + col, gt);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) y[j] = bf16_round(y[j] * bf16_round(__fdividef(gt[j], 1.f + __expf(-gt[j]))));
+      for (int j = 0; j < 8; ++j) y[j] = bf16_round(y[j] * bf16_round(gt[j] * sigmoidf_fast(gt[j])));
     }
     if (a.resid != nullptr) {
       float r[8];
@@ -1535,7 +1535,7 @@ __global__ void __launch_bounds__(256, (ROPE || NCH > 1) ? 2 : 4) qkv_prologue_b
         if (a.dz[t] != nullptr) load8_bf16(a.dz[t] + z_off + col, g[c]);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          u[c][i] = a.silu[t] ? bf16_round(__fdividef(xv[c][i], 1.f + __expf(-xv[c][i]))) : xv[c][i];
+          u[c][i] = a.silu[t] ? bf16_round(xv[c][i] * sigmoidf_fast(xv[c][i])) : xv[c][i];
           ss += u[c][i] * u[c][i];
         }
       }
@@ -1659,7 +1659,7 @@ __global__ void __launch_bounds__(256, 2) out_epilogue_bwd_kernel(const Epilogue
         for (int j = 0; j < 8; ++j) {
           const float n = v[c][j] * rstd * w[c][j];
           dg[j] = dn[c][j] * n * silu_grad(gt[j]);
-          dn[c][j] *= __fdividef(gt[j], 1.f + __expf(-gt[j]));
+          dn[c][j] *= gt[j] * sigmoidf_fast(gt[j]);
         }
         if (a.dgate != nullptr) store8_bf16(a.dgate + bs_idx * (static_cast<int64_t>(a.n_h) * a.d) + off + col, dg);
       }

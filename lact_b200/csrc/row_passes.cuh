@@ -28,7 +28,7 @@ __device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
   return make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
 }
 __device__ __forceinline__ uint4 load_unit(const bf16* p) { return *reinterpret_cast<const uint4*>(p); }
-__device__ __forceinline__ float silu_bf16(float x) { return bf16_round(__fdividef(x, 1.f + __expf(-x))); }
+__device__ __forceinline__ float silu_bf16(float x) { return bf16_round(x * sigmoidf_fast(x)); }
 
 // The rotation partner of unit u sits hd / 16 units away inside its attention head (hd a power of two): another lane of
 // the row's group, or another unit of the same lane.

@@ -42,13 +42,6 @@ struct SwaArgs {
   uint32_t* count;   // [tile - whole]
 };
 
-// 2^x by the hardware approximation (2^-inf = 0)
-__device__ __forceinline__ float fast_exp2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
 template <int HD>
 struct SwaSmem {
   static constexpr uint32_t kTile = 128 * HD * 2;          // one Q / K / V tile
@@ -277,7 +270,7 @@ __global__ void __launch_bounds__(320, 1) swa_fwd_kernel(const __grid_constant__
       mx = fmaxf(mx, exchange(mx));
       if (failed) continue;
       const float m_new = fmaxf(m, mx * a.scale_log2);
-      const float alpha = m_new == -INFINITY ? 1.f : fast_exp2(m - m_new);
+      const float alpha = m_new == -INFINITY ? 1.f : exp2_ftz(m - m_new);
       const float shift = m_new == -INFINITY ? 0.f : m_new;
       float sum = 0.f;
       const uint32_t p_row = base + SM::kP + sb * SM::kPTile + half * kBox + r * 128;   // this thread's 64-key panel
@@ -289,7 +282,7 @@ __global__ void __launch_bounds__(320, 1) swa_fwd_kernel(const __grid_constant__
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
             const int j = g * 8 + e;
-            const float x = fast_exp2(fmaf(__uint_as_float(bits[j]), a.scale_log2, -shift));
+            const float x = exp2_ftz(fmaf(__uint_as_float(bits[j]), a.scale_log2, -shift));
             p[e] = (!masked || (c + j >= j_lo && c + j <= j_hi)) ? x : 0.f;
             sum += p[e];
           }
@@ -352,7 +345,7 @@ __global__ void __launch_bounds__(320, 1) swa_fwd_kernel(const __grid_constant__
         for (int s = 0; s < splits; ++s, src += kO4 * 256) {
           const float2 ms = __ldcg(ml + s * 256);
           if (ms.x == -INFINITY) continue;   // this share saw no key of the row
-          const float w = fast_exp2(ms.x - m);
+          const float w = exp2_ftz(ms.x - m);
           l = fmaf(ms.y, w, l);
 #pragma unroll
           for (int c = 0; c < kO4; ++c) {

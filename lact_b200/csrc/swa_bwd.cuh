@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(320, 1) swa_bwd_kernel(const __grid_constant__
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                   const int j = g * 4 + e;
-                  p[j] = fast_exp2(fmaf(__uint_as_float(sb[j]), a.scale_log2, -lv[e]));
+                  p[j] = exp2_ftz(fmaf(__uint_as_float(sb[j]), a.scale_log2, -lv[e]));
                   ds[j] = p[j] * fmaf(__uint_as_float(db[j]), a.scale, -dv[e]);
                 }
               }
@@ -278,7 +278,7 @@ __global__ void __launch_bounds__(320, 1) swa_bwd_kernel(const __grid_constant__
                 for (int e = 0; e < 4; ++e) {
                   const int j = g * 4 + e, qi = i0 + c0 + j;
                   const bool ok = (!a.causal || (row <= qi && row >= qi - (window - 1) && row >= sv[e])) && qi < a.L && row < a.Lk;
-                  p[j] = ok ? fast_exp2(fmaf(__uint_as_float(sb[j]), a.scale_log2, -lv[e])) : 0.f;
+                  p[j] = ok ? exp2_ftz(fmaf(__uint_as_float(sb[j]), a.scale_log2, -lv[e])) : 0.f;
                   ds[j] = p[j] * fmaf(__uint_as_float(db[j]), a.scale, -dv[e]);
                 }
               }
@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(320, 1) swa_bwd_kernel(const __grid_constant__
             if (interior) {
 #pragma unroll
               for (int j = 0; j < 32; ++j) {
-                p[j] = fast_exp2(fmaf(__uint_as_float(sb[j]), a.scale_log2, -lse_r));
+                p[j] = exp2_ftz(fmaf(__uint_as_float(sb[j]), a.scale_log2, -lse_r));
                 ds[j] = p[j] * fmaf(__uint_as_float(db[j]), a.scale, -delta_r);
               }
             } else {
@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(320, 1) swa_bwd_kernel(const __grid_constant__
               for (int j = 0; j < 32; ++j) {
                 const int kv = i0 + c0 + j;
                 const bool ok = kv >= k_lo && kv <= k_hi;
-                p[j] = ok ? fast_exp2(fmaf(__uint_as_float(sb[j]), a.scale_log2, -lse_r)) : 0.f;
+                p[j] = ok ? exp2_ftz(fmaf(__uint_as_float(sb[j]), a.scale_log2, -lse_r)) : 0.f;
                 ds[j] = p[j] * fmaf(__uint_as_float(db[j]), a.scale, -delta_r);
               }
             }
