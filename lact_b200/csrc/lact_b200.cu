@@ -2781,7 +2781,12 @@ int lact_fw_grad_bwd_pointwise(const void* y02, const void* dh, const void* g_dy
                                 g_lr0, g_lr1, g_lr2, rows, H);
   a.n = n; a.lr_bs = lr_bs; a.g_lr_bs = g_lr_bs; a.g_lr_add = g_lr_add;
   KernelScope scope(kClsOther, static_cast<cudaStream_t>(stream));
-  fw_grad_bwd_pointwise_kernel<<<dim3(ceil_div(n, 8), static_cast<unsigned>(B)), 256, 0, static_cast<cudaStream_t>(stream)>>>(a);
+  // lanes per token: the most that divide its units, or a warp where eight do not
+  const cudaStream_t st = static_cast<cudaStream_t>(stream);
+  auto grid = [&](int lanes) { return dim3(ceil_div(n, 256 / lanes), static_cast<unsigned>(B)); };
+  if (H % 256 != 0 && H % 128 == 0) fw_grad_bwd_pointwise_kernel<16><<<grid(16), 256, 0, st>>>(a);
+  else if (H % 256 != 0 && H % 64 == 0) fw_grad_bwd_pointwise_kernel<8><<<grid(8), 256, 0, st>>>(a);
+  else fw_grad_bwd_pointwise_kernel<32><<<grid(32), 256, 0, st>>>(a);
   LACT_CUDA(cudaGetLastError());
   return LACT_OK;
 }

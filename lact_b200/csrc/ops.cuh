@@ -830,50 +830,77 @@ __global__ void __launch_bounds__(256) swiglu_bwd_planes_kernel(const PlaneArgs 
 // (lact_llm/lact_model/lact_triton_kernels/lact_fw_grad.py:178-260): with A = d silu / dy0,
 //   g_y0 = g_hid*A*y2*l1 + g_dy0*A'*y2*dh*l0 + g_dy2*A*dh*l2,   g_y2 = g_hid*sw*l1 + g_dy0*A*dh*l0,
 //   g_dh = g_dy0*A*y2*l0 + g_dy2*sw*l2,   g_lr = row sums (deterministic: one warp per row).
-__global__ void __launch_bounds__(256, 4) fw_grad_bwd_pointwise_kernel(const PlaneArgs a) {
+// LPR lanes share a token (H / 8 units of 16 bytes, six planes in and six out), so that a head size of 64, 128, 192, 256, 384
+// or 512 leaves no lane without a unit, and the next unit's six loads are in flight while one is computed.  HBM bounds it:
+// 32 entries x 2048 tokens of H = 384 move 604 MB (91 us at the copy rate): 106 us; with a warp per token, whose second
+// pass had half its lanes idle, 159 us.
+template <int LPR>
+__global__ void __launch_bounds__(256, 3) fw_grad_bwd_pointwise_kernel(const PlaneArgs a) {
   // grid (token blocks, entries)
-  const int64_t entry = blockIdx.y, tok = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (tok >= a.n) return;
-  const int lane = threadIdx.x & 31;
+  const int64_t entry = blockIdx.y, want = static_cast<int64_t>(blockIdx.x) * (256 / LPR) + threadIdx.x / LPR;
+  const bool live = want < a.n;  // (every lane takes part in the sums' shuffles)
+  const int64_t tok = live ? want : a.n - 1;
+  const int lane = threadIdx.x % LPR;
   const int64_t row = entry * a.n + tok, li = entry * a.lr_bs + tok;
+  const int H = a.H;
+  const bf16* const src[6] = {a.y02 + row * 2 * H, a.y02 + row * 2 * H + H,       a.dh + row * H,
+                              a.g_dy02 + row * 2 * H, a.g_dy02 + row * 2 * H + H, a.g_hid + row * H};
+  uint4 raw[6];
+  auto fetch = [&](int c) {
+#pragma unroll
+    for (int p = 0; p < 6; ++p) raw[p] = *reinterpret_cast<const uint4*>(src[p] + c);
+  };
+  int c = lane * 8;
+  if (c < H) fetch(c);
   const float l0 = load_scalar(a.lr0, a.lr_f32, li) * a.w_scale;
   const float l1 = load_scalar(a.lr1, a.lr_f32, li) * a.w_scale;
   const float l2 = load_scalar(a.lr2, a.lr_f32, li) * a.w_scale;
-  const int H = a.H;
   float s0 = 0.f, s1 = 0.f, s2 = 0.f;
-  for (int c = lane * 8; c < H; c += 256) {
-    float y0[8], y2[8], dh[8], gd0[8], gd2[8], gh[8];
-    load8_bf16(a.y02 + row * 2 * H + c, y0);
-    load8_bf16(a.y02 + row * 2 * H + H + c, y2);
-    load8_bf16(a.dh + row * H + c, dh);
-    load8_bf16(a.g_dy02 + row * 2 * H + c, gd0);
-    load8_bf16(a.g_dy02 + row * 2 * H + H + c, gd2);
-    load8_bf16(a.g_hid + row * H + c, gh);
-    float gy0[8], gy2[8], gdh[8], oh[8], o0[8], o2[8];
+  for (; c < H; c += LPR * 8) {
+    uint4 in[6];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float sg = sigmoidf_fast(y0[j]), sw = sg * y0[j];
-      const float A = sg * (1.0f + y0[j] * (1.0f - sg));
-      const float Ap = sg * (1.0f - sg) * (2.0f + y0[j] * (1.0f - 2.0f * sg));
-      gy0[j] = gh[j] * A * y2[j] * l1 + gd0[j] * Ap * y2[j] * dh[j] * l0 + gd2[j] * A * dh[j] * l2;
-      gy2[j] = gh[j] * sw * l1 + gd0[j] * A * dh[j] * l0;
-      gdh[j] = gd0[j] * A * y2[j] * l0 + gd2[j] * sw * l2;
-      oh[j] = sw * y2[j] * l1;
-      o0[j] = A * y2[j] * dh[j] * l0;
-      o2[j] = sw * dh[j] * l2;
-      s0 += gd0[j] * A * y2[j] * dh[j];
-      s1 += gh[j] * sw * y2[j];
-      s2 += gd2[j] * sw * dh[j];
+    for (int p = 0; p < 6; ++p) in[p] = raw[p];
+    if (c + LPR * 8 < H) fetch(c + LPR * 8);
+    const uint32_t* const w = reinterpret_cast<const uint32_t*>(in);
+    uint4 out[6];
+    uint32_t* const ow = reinterpret_cast<uint32_t*>(out);
+#pragma unroll
+    for (int j2 = 0; j2 < 4; ++j2) {
+      float r[6][2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        auto at = [&](int p) { return __uint_as_float(e == 0 ? w[p * 4 + j2] << 16 : w[p * 4 + j2] & 0xFFFF0000u); };
+        const float y0 = at(0), y2 = at(1), dh = at(2), gd0 = at(3), gd2 = at(4), gh = at(5);
+        const float sg = sigmoidf_fast(y0), sw = sg * y0;
+        const float A = sg * (1.0f + y0 * (1.0f - sg));
+        const float Ap = sg * (1.0f - sg) * (2.0f + y0 * (1.0f - 2.0f * sg));
+        r[0][e] = gh * A * y2 * l1 + gd0 * Ap * y2 * dh * l0 + gd2 * A * dh * l2;  // g_y0
+        r[1][e] = gh * sw * l1 + gd0 * A * dh * l0;                                // g_y2
+        r[2][e] = gd0 * A * y2 * l0 + gd2 * sw * l2;                               // g_dh
+        r[3][e] = sw * y2 * l1;                                                    // hidden
+        r[4][e] = A * y2 * dh * l0;                                                // dy0
+        r[5][e] = sw * dh * l2;                                                    // dy2
+        s0 += gd0 * A * y2 * dh;
+        s1 += gh * sw * y2;
+        s2 += gd2 * sw * dh;
+      }
+#pragma unroll
+      for (int p = 0; p < 6; ++p) ow[p * 4 + j2] = pack_bf16x2(r[p][0], r[p][1]);
     }
-    store8_bf16(a.g_y02 + row * 2 * H + c, gy0);
-    store8_bf16(a.g_y02 + row * 2 * H + H + c, gy2);
-    store8_bf16(a.g_dh + row * H + c, gdh);
-    store8_bf16(a.hid + row * H + c, oh);
-    store8_bf16(a.dy02 + row * 2 * H + c, o0);
-    store8_bf16(a.dy02 + row * 2 * H + H + c, o2);
+    if (live) {
+      bf16* const dst[6] = {a.g_y02 + row * 2 * H, a.g_y02 + row * 2 * H + H, a.g_dh + row * H,
+                            a.hid + row * H,       a.dy02 + row * 2 * H,      a.dy02 + row * 2 * H + H};
+#pragma unroll
+      for (int p = 0; p < 6; ++p) *reinterpret_cast<uint4*>(dst[p] + c) = out[p];
+    }
   }
-  s0 = warp_sum(s0); s1 = warp_sum(s1); s2 = warp_sum(s2);
-  if (lane == 0) {
+#pragma unroll
+  for (int o = LPR / 2; o > 0; o >>= 1) {
+    s0 += __shfl_xor_sync(0xFFFFFFFFu, s0, o);
+    s1 += __shfl_xor_sync(0xFFFFFFFFu, s1, o);
+    s2 += __shfl_xor_sync(0xFFFFFFFFu, s2, o);
+  }
+  if (live && lane == 0) {
     const int64_t gi = entry * a.g_lr_bs + tok;
     a.g_lr0[gi] = s0 * a.w_scale + (a.g_lr_add ? a.g_lr0[gi] : 0.f);
     a.g_lr1[gi] = s1 * a.w_scale + (a.g_lr_add ? a.g_lr1[gi] : 0.f);
