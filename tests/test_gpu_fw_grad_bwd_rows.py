@@ -30,8 +30,9 @@ def test_fw_grad_bwd_pointwise(H, B, n, add):
     sw, A, Ap = s * y0, s * (1 + y0 * (1 - s)), s * (1 - s) * (2 + y0 * (1 - 2 * s))
     want = [torch.cat([gh * A * y2 * l1 + d0 * Ap * y2 * h * l0 + d2 * A * h * l2, gh * sw * l1 + d0 * A * h * l0], -1),
             d0 * A * y2 * l0 + d2 * sw * l2, torch.cat([A * y2 * h * l0, sw * h * l2], -1), sw * y2 * l1]
-    for got, w in zip((gy, gdh, dy, hid), want):   # one rounding to bf16 of fp32 arithmetic: 2^-9 of every value
-        assert float((got.double() - w).norm() / w.norm()) <= 2 ** -9
+    # one rounding to bf16 (8 significant bits: at most 2^-8 of a value) of fp32 arithmetic with approximate sigmoids (1e-5)
+    for got, w in zip((gy, gdh, dy, hid), want):
+        assert float((got.double() - w).norm() / w.norm()) <= 2 ** -8 + 1e-5
     sums = [(d0 * A * y2 * h), (gh * sw * y2), (d2 * sw * h)]
     for got, w in zip(glr, sums):   # fp32 sums of H terms with approximate sigmoids (1e-6 each)
         err = (got[:, :n].double() - w.sum(-1) - (1 if add else 0)).abs()
