@@ -829,7 +829,7 @@ __global__ void __launch_bounds__(256) swiglu_bwd_planes_kernel(const PlaneArgs 
 // Second-order pointwise stage of the fast-weight-gradient backward
 // (lact_llm/lact_model/lact_triton_kernels/lact_fw_grad.py:178-260): with A = d silu / dy0,
 //   g_y0 = g_hid*A*y2*l1 + g_dy0*A'*y2*dh*l0 + g_dy2*A*dh*l2,   g_y2 = g_hid*sw*l1 + g_dy0*A*dh*l0,
-//   g_dh = g_dy0*A*y2*l0 + g_dy2*sw*l2,   g_lr = row sums (deterministic: one warp per row).
+//   g_dh = g_dy0*A*y2*l0 + g_dy2*sw*l2,   g_lr = row sums (deterministic: one group of lanes per row).
 // LPR lanes share a token (H / 8 units of 16 bytes, six planes in and six out), so that a head size of 64, 128, 192, 256, 384
 // or 512 leaves no lane without a unit, and the next unit's six loads are in flight while one is computed.  HBM bounds it:
 // 32 entries x 2048 tokens of H = 384 move 604 MB (91 us at the copy rate): 106 us; with a warp per token, whose second
