@@ -344,8 +344,8 @@ __global__ void __launch_bounds__(320, 1) swa_fwd_kernel(const __grid_constant__
         const float4* src = a.part + first * (kO4 * 256) + thr;
         for (int s = 0; s < splits; ++s, src += kO4 * 256) {
           const float2 ms = __ldcg(ml + s * 256);
-          if (ms.x == -INFINITY) continue;   // this share saw no key of the row
-          const float w = exp2_ftz(ms.x - m);
+          // (a maximum of -inf is a share without a visible key, all zeros, or one whose scores are all NaN: those pass through)
+          const float w = ms.x == -INFINITY ? 1.f : exp2_ftz(ms.x - m);
           l = fmaf(ms.y, w, l);
 #pragma unroll
           for (int c = 0; c < kO4; ++c) {
