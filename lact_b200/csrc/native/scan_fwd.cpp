@@ -44,8 +44,12 @@ std::vector<Tensor> scan_fwd(const Tensor& w0_, const Tensor& w1_, const Tensor&
     TORCH_CHECK_TYPE(f32 || t->scalar_type() == at::kBFloat16, "q, k, v must be bfloat16, or all float32 (got ", t->scalar_type(), ")");
     TORCH_CHECK_VALUE(t->dim() == 3, "q, k, v must be [b, l, d]");
   }
-  for (const Tensor* t : {&w0_, &w1_, &w2_, &q_, &v_, &lr0_, &lr1_, &lr2_})
+  const Tensor mom_ = value(momentum_), state_[3] = {value(m0), value(m1), value(m2)};
+  for (const Tensor* t : {&w0_, &w1_, &w2_, &q_, &v_, &lr0_, &lr1_, &lr2_, &mom_, &state_[0], &state_[1], &state_[2]}) {
+    if (!t->defined()) continue;
+    TORCH_CHECK(t->is_cuda(), "lact_b200 runs on CUDA tensors only (there is no CPU implementation)");
     TORCH_CHECK_VALUE(t->device() == k_.device(), "all tensors must be on the same device");
+  }
   const Tensor q = aligned(q_, f32 ? 4 : 8), k = aligned(k_, f32 ? 4 : 8), v = aligned(v_, f32 ? 4 : 8);
   const int64_t B = k.size(0), L = k.size(1), D = k.size(2);
   TORCH_CHECK_VALUE(w0_.dim() == 3, "w0 must be [b, d_h, d]");
@@ -57,7 +61,7 @@ std::vector<Tensor> scan_fwd(const Tensor& w0_, const Tensor& w1_, const Tensor&
   Tensor lr0 = per_token(lr0_, B, L, "lr0"), lr1 = per_token(lr1_, B, L, "lr1"), lr2 = per_token(lr2_, B, L, "lr2");
   same_dtype(lr0, lr1, lr2);
   Tensor mom;
-  if (given(momentum_)) mom = per_token(*momentum_, B, L, "momentum");
+  if (mom_.defined()) mom = per_token(mom_, B, L, "momentum");
 
   lact_scan_config c = base_config(o, B, L, D, H);
   // The reference drivers start from torch.zeros_like(q): tokens no APPLY step covers stay zero.
@@ -82,11 +86,10 @@ std::vector<Tensor> scan_fwd(const Tensor& w0_, const Tensor& w1_, const Tensor&
   io.momentum = mom.defined() ? ptr(mom) : nullptr;
   io.o = ptr(out);
   Tensor mi[3];
-  if (given(m0)) {
-    const OptTensor* ms[3] = {&m0, &m1, &m2};
+  if (state_[0].defined()) {
     for (int i = 0; i < 3; ++i) {
-      TORCH_CHECK_VALUE(given(*ms[i]), "the momentum state has three parts");
-      mi[i] = (*ms[i])->to(at::kFloat).contiguous();
+      TORCH_CHECK_VALUE(state_[i].defined(), "the momentum state has three parts");
+      mi[i] = state_[i].to(at::kFloat).contiguous();
       TORCH_CHECK_VALUE(mi[i].numel() == B * D * H, "momentum state: one value per weight");
     }
     io.m0_in = ptr(mi[0]); io.m1_in = ptr(mi[1]); io.m2_in = ptr(mi[2]);
