@@ -111,13 +111,27 @@ std::vector<Tensor> scan_bwd(const Tensor& w0, const Tensor& w1, const Tensor& w
     dv.narrow(1, s, e - s).zero_();
     for (Tensor& t : dlr) t.narrow(1, s, e - s).zero_();
   }
-  std::vector<std::pair<int64_t, int64_t>> q_done, kv_done;
-  auto first = [](std::vector<std::pair<int64_t, int64_t>>& done, int64_t s, int64_t e) {
+  // (in part, if ranges overlap: what no step has written yet of a range that is added to is zeroed first)
+  using Ranges = std::vector<std::pair<int64_t, int64_t>>;
+  Ranges q_done, kv_done;
+  // Whether [s, e) has been written nowhere; otherwise `missing` receives the parts of it that have not.
+  auto first = [](Ranges& done, int64_t s, int64_t e, Ranges& missing) {
     bool ok = true;
-    for (auto& [a, b] : done) ok = ok && (e <= a || s >= b);
+    missing.assign(1, {s, e});
+    for (auto& [a, b] : done) {
+      if (e <= a || s >= b) continue;
+      ok = false;
+      Ranges left;
+      for (auto& [x, y] : missing) {
+        if (x < std::min(y, a)) left.emplace_back(x, std::min(y, a));
+        if (std::max(x, b) < y) left.emplace_back(std::max(x, b), y);
+      }
+      missing.swap(left);
+    }
     done.emplace_back(s, e);
     return ok;
   };
+  Ranges missing;
 
   TokenBackward tok(B, D, H, k, sw.status, stream);
   int cnt = st.updates;
@@ -125,12 +139,15 @@ std::vector<Tensor> scan_bwd(const Tensor& w0, const Tensor& w1, const Tensor& w
     const int64_t s = st.start[i], e = st.end[i], n = e - s;
     if (n <= 0) continue;
     if (st.kind[i] == kApply) {
-      const bool own = first(q_done, s, e);
+      const bool own = first(q_done, s, e, missing);
       Tensor tmp = own ? Tensor() : empty({B, n, D}, BF, k);
       tok.apply(W02b(cnt), W1b(cnt), tokens(q, s), tokens(dO, st.out[i]), n, View(dW02), View(dW1), !fresh,
                 own ? tokens(dq, s) : View(tmp));
       fresh = false;
-      if (!own) dq.narrow(1, s, n).add_(tmp);
+      if (!own) {
+        for (auto& [a, b] : missing) dq.narrow(1, a, b - a).zero_();
+        dq.narrow(1, s, n).add_(tmp);
+      }
       continue;
     }
     const int u = --cnt;
@@ -190,9 +207,17 @@ std::vector<Tensor> scan_bwd(const Tensor& w0, const Tensor& w1, const Tensor& w
     for (int j = 0; j < 3; ++j) lr[j] = static_cast<const uint8_t*>(ptr(lrv[j])) + s * lr_esz;
     float* glr[3];
     for (int j = 0; j < 3; ++j) glr[j] = dlr[j].data_ptr<float>() + s;
-    const bool own = first(kv_done, s, e);
+    const bool own = first(kv_done, s, e, missing);
     Tensor tk, tv;
-    if (!own) { tk = empty({B, n, D}, BF, k); tv = empty({B, n, D}, BF, k); }
+    if (!own) {
+      tk = empty({B, n, D}, BF, k);
+      tv = empty({B, n, D}, BF, k);
+      for (auto& [a, b] : missing) {
+        dk.narrow(1, a, b - a).zero_();
+        dv.narrow(1, a, b - a).zero_();
+        for (Tensor& t : dlr) t.narrow(1, a, b - a).zero_();
+      }
+    }
     tok.gradient(W02b(u), W1b(u), tokens(k, s), tokens(v, s), n, lr, dtype_code(lrv[0]), L, static_cast<float>(w_scale), View(g02b),
                  View(g1b), View(dW02), View(dW1), !fresh, own ? tokens(dk, s) : View(tk), own ? tokens(dv, s) : View(tv), glr, L,
                  !own);
