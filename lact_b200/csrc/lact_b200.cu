@@ -1529,12 +1529,13 @@ int scan_fwd_f32(const lact_scan_config& c, const lact_scan_io& io, int32_t n_st
         p.W02c, p.W1c, p.n02, p.n1, nullptr, nullptr, p.status, nullptr, 0);
     LACT_CUDA(cudaGetLastError());
   }
-  if (has_initial_momentum(io) || io.m0_out) LACT_TRY(load_momentum_state(c, io, p.G02, p.G1, stream));
+  if (has_initial_momentum(io) || io.m0_out || io.m1_out || io.m2_out) LACT_TRY(load_momentum_state(c, io, p.G02, p.G1, stream));
   if (c.use_momentum) LACT_TRY(launch_momentum_means(c, io, n_steps, kind, start, end, p.beta, stream));
   const float* W02 = c.prenorm ? p.W02c : p.W02;  // the weights the steps compute with
   const float* W1 = c.prenorm ? p.W1c : p.W1;
   const float *q = static_cast<const float*>(io.q), *k = static_cast<const float*>(io.k), *v = static_cast<const float*>(io.v);
   int update_idx = 0;
+  bool state_written = has_initial_momentum(io);  // by the caller, or by an update that had tokens
   for (int i = 0; i < n_steps; ++i) {
     const int64_t len = end[i] - start[i];
     if (len <= 0) {
@@ -1576,8 +1577,9 @@ int scan_fwd_f32(const lact_scan_config& c, const lact_scan_io& io, int32_t n_st
     F32ReduceArgs red;
     std::memset(&red, 0, sizeof(red));
     red.batch = static_cast<int32_t>(B);
-    red.accumulate = c.use_momentum && (u > 0 || has_initial_momentum(io));
+    red.accumulate = c.use_momentum && state_written;
     red.beta = red.accumulate ? p.beta + static_cast<int64_t>(u) * B : nullptr;
+    state_written = true;
     for (int w = 0; w < 2; ++w) {  // [dw0; dw2] = dy^T k, dw1 = v^T hidden
       const int64_t R = w == 0 ? 2 * H : D, C = w == 0 ? D : H;
       F32Args g;

@@ -1,0 +1,31 @@
+"""fp32 mode at the edges of what it takes."""
+import pytest
+import torch
+
+from test_gpu_overlapping_ranges import fill_free_memory
+
+pytestmark = pytest.mark.gpu
+NAMES = ("w0", "w1", "w2", "q", "k", "v", "lr0", "lr1", "lr2")
+
+
+def _inputs(B, L, D, H, seed=1):
+    from oracle import lact_oracle as orc
+    return {n: t.cuda() for n, t in orc.make_inputs(B, L, D, H, seed=seed).items()}
+
+
+def test_momentum_after_an_empty_first_update():
+    import lact_b200 as lb
+    from lact_b200 import ops
+    from lact_b200 import program as P
+    L, n = 96, 48
+    i = _inputs(2, L, 32, 16)
+    args = [i[x] for x in NAMES]
+    steps = [(P.APPLY, 0, n, 0), (P.UPDATE, 0, n, 0), (P.APPLY, n, L, n), (P.UPDATE, n, L, 0)]
+    want = ops.scan(*args, steps, momentum=i["momentum"], return_state=True, return_momentum=True)
+    for empty in (1, 2):
+        fill_free_memory()
+        got = ops.scan(*args, [(P.UPDATE, 0, 0, 0)] * empty + steps, momentum=i["momentum"], return_state=True, return_momentum=True)
+        got_o = ops.scan(*args, [(P.UPDATE, 0, 0, 0)] * empty + steps, momentum=i["momentum"], return_state=True)
+        lb.synchronize_and_check()
+        for a, b in zip(list(got) + list(got_o), list(want) + list(want[:4])):
+            assert torch.equal(a, b)
