@@ -53,9 +53,16 @@ inline Tensor bytes(size_t n, const Tensor& like) {
   return empty({static_cast<int64_t>(n < 256 ? 256 : n)}, at::kByte, like);
 }
 
-// Device status word of the calls on (device of `like`, current stream): cleared once, shared by consecutive calls.
-// Throws if a call has recorded a failure since the last look (see status.cpp); costs one read of host memory.
-int32_t* status_word(const Tensor& like);
+// Device status word of the calls on (device of `like`, current stream): cleared once, shared by consecutive calls.  A
+// call that is being captured gets a word of its own, which the graph clears at every replay: keep the object for as long
+// as kernels that use the word are enqueued.  Throws if a call has recorded a failure since the last look (see status.cpp);
+// costs one read of host memory and a query of the stream.
+struct StatusWord {
+  Tensor own;  // defined inside a capture
+  int32_t* word;
+  operator int32_t*() const { return word; }
+};
+StatusWord status_word(const Tensor& like);
 void poll_status(const Tensor& like);
 
 // A [batch, rows, cols] bf16 activation whose last axis is contiguous and whose strides and base keep 16-byte alignment

@@ -137,7 +137,7 @@ class Sweep {
   const Steps& st_;
   Tensor like_;
   int64_t B, L, D, H, n02, n1;
-  int32_t* status;
+  StatusWord status;
   void* stream;
 };
 

@@ -38,8 +38,8 @@ inline lact_bmm_desc& plus(lact_bmm_desc& d, View a, bool a_mn, View b, bool b_m
 // count; `w02` / `w1` are the bf16 weights the step computed with.
 class TokenBackward {
  public:
-  TokenBackward(int64_t B, int64_t D, int64_t H, const Tensor& like, int32_t* status, void* stream)
-      : B_(B), D_(D), H_(H), like_(like), status_(status), stream_(stream) {}
+  TokenBackward(int64_t B, int64_t D, int64_t H, const Tensor& like, StatusWord status, void* stream)
+      : B_(B), D_(D), H_(H), like_(like), status_(std::move(status)), stream_(stream) {}
   // o = w1 (silu(w0 q) * (w2 q)): weight gradients (+)= into dW02 / dW1 (fp32), dq (bf16) written.
   void apply(View w02, View w1, View q, View dO, int64_t n, View dW02, View dW1, bool accumulate, View dq);
   // lr-weighted fast-weight gradient, given the bf16 gradients g02 / g1 of its outputs: weight gradients (+)=, dk, dv
@@ -56,7 +56,7 @@ class TokenBackward {
   }
   int64_t B_, D_, H_;
   Tensor like_;
-  int32_t* status_;
+  StatusWord status_;
   void* stream_;
   Tensor a_, b_, c_, d_, e_, f_, g_, h_;
   Tensor split_, split_count_;  // scratch of split contractions, once one is

@@ -2,6 +2,8 @@
 // (lact_status_host_word).  An operator reads that word before it enqueues (one load); a non-zero word is reported as an
 // exception and cleared together with the device-side words.  This replaced a 4-byte device-to-host copy, an event and
 // a memset per call: about 5 us of stream time and 12 us of host time each.
+#include <c10/cuda/CUDAGraphsC10Utils.h>
+
 #include <atomic>
 #include <mutex>
 #include <unordered_map>
@@ -45,8 +47,14 @@ void poll_status(const Tensor& like) {
   TORCH_CHECK(false, "lact_b200: device status: ", lact_error_string(st), " (code ", st, ")");
 }
 
-int32_t* status_word(const Tensor& like) {
+StatusWord status_word(const Tensor& like) {
   poll_status(like);
+  if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) {
+    // The stream's shared word would be cleared (or not) by whatever runs between the replays, and if its clearing fell
+    // into this capture it would only be recorded.
+    Tensor own = empty({64}, at::kInt, like).zero_();
+    return {own, own.data_ptr<int32_t>()};
+  }
   const int dev = like.device().index();
   const auto stream = c10::cuda::getCurrentCUDAStream(dev);
   const uint64_t key = (static_cast<uint64_t>(dev) << 56) ^ static_cast<uint64_t>(reinterpret_cast<uintptr_t>(stream.stream()));
@@ -58,7 +66,7 @@ int32_t* status_word(const Tensor& like) {
     w.buf.zero_();
     w.epoch = epoch;
   }
-  return w.buf.data_ptr<int32_t>();
+  return {Tensor(), w.buf.data_ptr<int32_t>()};
 }
 
 }  // namespace lact_torch

@@ -1,0 +1,68 @@
+"""Device status and stream capture."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+SETUP = """
+import ctypes as C, torch
+import lact_b200 as lb
+from lact_b200 import _lib as L
+from lact_b200 import layer_ops as lo
+g = torch.Generator(device="cuda").manual_seed(0)
+rn = lambda *s: torch.randn(*s, device="cuda", generator=g)
+bf = lambda *s: rn(*s).to(torch.bfloat16)
+def scan_args(B=1, n=256, D=64, H=64):
+    unit = lambda t: (t / t.norm(dim=-1, keepdim=True)).to(torch.bfloat16)
+    return [rn(B, H, D) / 8, rn(B, D, H) / 8, rn(B, H, D) / 8, unit(rn(B, n, D)), unit(rn(B, n, D)), bf(B, n, D)] + [torch.rand(B, n, 1, device="cuda") / 8 for _ in range(3)]
+def train(leaves, dout):
+    o = lb.block_causal_lact_swiglu(*leaves, chunk_size=64, use_muon=True)
+    return [o.detach()] + list(torch.autograd.grad(o, leaves, dout))
+def make(kind):
+    if kind == "attention":
+        t = [bf(1, 300, 2, 64) for _ in range(3)]
+        return lambda: [lo.sliding_window_attention(*t, 128)]
+    if kind == "ffn":
+        t = bf(2, 128, 64) / 8, bf(2, 64, 64) / 8, bf(2, 40, 64)
+        return lambda: [lb.fused_swiglu_ffn_fwd(*t)]
+    if kind == "train":
+        leaves, dout = [t.requires_grad_(True) for t in scan_args()], bf(1, 256, 64)
+        return lambda: train(leaves, dout)
+    if kind == "newton_schulz":
+        t = rn(2, 64, 128)
+        return lambda: [lb.zeropower_via_newtonschulz5(t)]
+    t = scan_args()
+    return lambda: [lb.block_causal_lact_swiglu(*t, chunk_size=64, use_muon=True)]
+"""
+
+
+@pytest.mark.parametrize("kind", ["attention", "ffn", "train"])
+def test_graphs_of_one_stream_replay_in_any_order(kind):
+    ns = {}
+    exec(SETUP + f"\ncall = make({kind!r})", ns)
+    call, lb = ns["call"], ns["lb"]
+    want = call()
+    lb.synchronize_and_check()
+    stream, pool = torch.cuda.Stream(), torch.cuda.graph_pool_handle()
+    filler, first, second = (torch.cuda.CUDAGraph() for _ in range(3))
+    with torch.cuda.graph(filler, pool=pool, stream=stream):   # leaves non-zero words in the pool's memory
+        junk = [torch.full((n,), 1, dtype=torch.int32, device="cuda") for n in (1 << 20, 1 << 16, 1 << 12, 128) for _ in range(24)]
+        del junk
+    filler.replay()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(first, pool=pool, stream=stream):
+        out1 = call()
+    with torch.cuda.graph(second, pool=pool, stream=stream):
+        out2 = call()
+    for graph, out in ((second, out2), (first, out1), (second, out2)):
+        filler.replay()
+        for t in out:
+            t.fill_(float("nan"))
+        graph.replay()
+        torch.cuda.synchronize()
+        for a, b in zip(out, want):
+            assert torch.equal(a, b)
+    again = call()   # and eager calls after them
+    lb.synchronize_and_check()
+    for a, b in zip(again, want):
+        assert torch.equal(a, b)
