@@ -134,7 +134,7 @@ int64_t lact_stream_sync_count(void);
 int lact_set_wait_limit_ns(uint64_t limit_ns);
 /* A word of pinned host memory (one per device, made at the first call) in which every kernel that records a non-zero
  * device status also leaves it: a host that reads it now and then learns of a failure without copies or waits.  The
- * host clears it.  Make the first call outside stream capture.  No counterpart in the reference. */
+ * host clears it.  May be called while a stream is being captured.  No counterpart in the reference. */
 int lact_status_host_word(int32_t **word_out);
 int lact_debug_wait_timeout(int32_t *status_word, void *stream);
 

@@ -1715,6 +1715,34 @@ int lact_read_status(const void* workspace, void* stream) {
 
 int64_t lact_stream_sync_count(void) { return g_stream_syncs.load(); }
 
+// Makes a device's word of mapped host memory and tells its kernels where it is.  The call that needs it first may be inside
+// a stream capture, which forbids this thread allocations and stream 0: the relaxed mode and a stream of its own keep the
+// capture out of it.
+static int make_status_host_word(int32_t** word) {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  LACT_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+  auto make = [&]() -> int {
+    void *h = nullptr, *d = nullptr;
+    LACT_CUDA(cudaHostAlloc(&h, sizeof(int32_t), cudaHostAllocMapped | cudaHostAllocPortable));
+    *static_cast<int32_t*>(h) = 0;
+    cudaStream_t s = nullptr;
+    cudaError_t e = cudaHostGetDevicePointer(&d, h, 0);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaMemcpyToSymbolAsync(g_host_status, &d, sizeof(d), 0, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (s != nullptr) cudaStreamDestroy(s);
+    if (e != cudaSuccess) {
+      cudaFreeHost(h);
+      return LACT_ERR_CUDA;
+    }
+    *word = static_cast<int32_t*>(h);
+    return LACT_OK;
+  };
+  const int rc = make();
+  LACT_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+  return rc;
+}
+
 int lact_status_host_word(int32_t** word_out) {
   if (!word_out) return LACT_ERR_NULL;
   static std::mutex mu;
@@ -1723,14 +1751,7 @@ int lact_status_host_word(int32_t** word_out) {
   LACT_CUDA(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64) return LACT_ERR_DEVICE;
   std::lock_guard<std::mutex> lock(mu);
-  if (words[dev] == nullptr) {
-    void *h = nullptr, *d = nullptr;
-    LACT_CUDA(cudaHostAlloc(&h, sizeof(int32_t), cudaHostAllocMapped | cudaHostAllocPortable));
-    *static_cast<int32_t*>(h) = 0;
-    LACT_CUDA(cudaHostGetDevicePointer(&d, h, 0));
-    LACT_CUDA(cudaMemcpyToSymbol(g_host_status, &d, sizeof(d)));
-    words[dev] = static_cast<int32_t*>(h);
-  }
+  if (words[dev] == nullptr) LACT_TRY(make_status_host_word(&words[dev]));
   *word_out = words[dev];
   return LACT_OK;
 }

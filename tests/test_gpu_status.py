@@ -1,8 +1,13 @@
 """Device status and stream capture."""
+import os
+import subprocess
+import sys
+
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 SETUP = """
 import ctypes as C, torch
@@ -36,6 +41,12 @@ def make(kind):
 """
 
 
+def _python(code, **env):
+    r = subprocess.run([sys.executable, "-c", SETUP + code], cwd=ROOT, capture_output=True, text=True, timeout=300, env={**os.environ, **env})
+    assert r.returncode == 0, r.stdout + r.stderr
+    return r.stdout
+
+
 @pytest.mark.parametrize("kind", ["attention", "ffn", "train"])
 def test_graphs_of_one_stream_replay_in_any_order(kind):
     ns = {}
@@ -66,3 +77,19 @@ def test_graphs_of_one_stream_replay_in_any_order(kind):
     lb.synchronize_and_check()
     for a, b in zip(again, want):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("kind", ["attention", "ffn", "train", "scan", "newton_schulz"])
+def test_first_call_of_a_process_inside_a_capture(kind):
+    _python(f"""
+call = make({kind!r})
+torch.cuda.synchronize()
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    out = call()
+graph.replay()
+torch.cuda.synchronize()
+want = call()
+lb.synchronize_and_check()
+assert all(torch.equal(a, b) for a, b in zip(out, want))
+""")
