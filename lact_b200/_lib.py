@@ -171,6 +171,8 @@ def load_ops() -> None:
     _ops_lib = C.CDLL(OPS_PATH)
     _ops_lib.lact_torch_take_status.argtypes = [C.c_int]
     _ops_lib.lact_torch_take_status.restype = C.c_int
+    _ops_lib.lact_torch_prepare_status.argtypes = [C.c_int]
+    _ops_lib.lact_torch_prepare_status.restype = C.c_int
     from . import _fakes  # noqa: F401
     _ops_loaded = True
 
@@ -222,7 +224,20 @@ SYNC_CHECK = os.environ.get("LACT_B200_SYNC_CHECK", "0") == "1"
 def workspace(nbytes: int, device: torch.device) -> torch.Tensor:
     """Scratch for one call on the current stream, from PyTorch's caching allocator (stream-ordered: giving it back right
     after the call has been enqueued is safe)."""
+    prepare_status(device)
     return torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
+
+
+_prepared = set()   # devices whose failures have a place to be reported in
+
+
+def prepare_status(device: torch.device) -> None:
+    """Before a library call that is not a registered operator: its kernels find the word that failures are left in."""
+    index = device.index if device.index is not None else torch.cuda.current_device()
+    if index not in _prepared:
+        load_ops()
+        check(_ops_lib.lact_torch_prepare_status(index), "lact_status_host_word")
+        _prepared.add(index)
 
 
 def _take_status(index: int) -> None:

@@ -18,6 +18,7 @@ def _status_word(dev: torch.device) -> torch.Tensor:
     """Device status word of the backward kernels, one per (device, stream)."""
     key = (dev.index if dev.index is not None else torch.cuda.current_device(), L.stream_ptr())
     if key not in _status:
+        L.prepare_status(dev)
         _status[key] = torch.zeros(64, dtype=torch.int32, device=dev)
     return _status[key]
 

@@ -83,3 +83,15 @@ extern "C" int lact_torch_take_status(int device) {
   }
   return st;
 }
+
+// Makes the word failures on `device` are reported in, if no operator has yet: called before kernels are launched past the
+// operators.  Returns the C ABI's code.
+extern "C" int lact_torch_prepare_status(int device) {
+  if (device < 0 || device >= lact_torch::kMaxDevices) return LACT_ERR_DEVICE;
+  if (lact_torch::g_host[device].load(std::memory_order_acquire) != nullptr) return LACT_OK;
+  const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
+  int32_t* w = nullptr;
+  const int rc = lact_status_host_word(&w);
+  if (rc == LACT_OK) lact_torch::g_host[device].store(w, std::memory_order_release);
+  return rc;
+}

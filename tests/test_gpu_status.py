@@ -93,3 +93,24 @@ want = call()
 lb.synchronize_and_check()
 assert all(torch.equal(a, b) for a, b in zip(out, want))
 """)
+
+
+def test_failure_in_a_process_that_calls_no_registered_operator():
+    _python("""
+lb.zeropower_via_newtonschulz5(rn(1, 64, 64))
+dev = torch.device("cuda", 0)
+ws = L.workspace(1 << 20, dev)
+ws[:256].zero_()
+L.check(L.lib().lact_set_wait_limit_ns(1_000_000), "limit")
+L.check(L.lib().lact_debug_wait_timeout(ws.data_ptr(), L.stream_ptr()), "timeout")
+torch.cuda.synchronize()
+try:
+    L.mark_pending(ws)
+    lb.synchronize_and_check()
+except lb.LactError:
+    pass
+else:
+    raise SystemExit("not reported")
+lb.zeropower_via_newtonschulz5(rn(1, 64, 64))
+lb.synchronize_and_check()
+""")
