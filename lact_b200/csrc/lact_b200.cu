@@ -1449,11 +1449,12 @@ int launch_f32_gemm(F32Args& a, cudaStream_t stream) {
 }
 
 // Splits of a token contraction (output R x C per entry, `len` tokens): enough that the grid fills the four CTAs an SM
-// holds, at least 64 tokens each.  At 4 entries of 192 x 192 and 4096 tokens one split would be 24 CTAs.
+// holds, at least 64 tokens each, and no more than the grid's third axis takes (B x splits).  At 4 entries of 192 x 192 and
+// 4096 tokens one split would be 24 CTAs.
 int f32_splits(int64_t R, int64_t C, int64_t B, int64_t len) {
   const int64_t tiles = B * ceil_div(R, kFM) * ceil_div(C, kFN);
   const int64_t want = (4 * static_cast<int64_t>(sm_count()) + tiles - 1) / tiles;
-  return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>({want, (len + 63) / 64, 64})));
+  return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>({want, (len + 63) / 64, 64, 65535 / B})));
 }
 
 struct ScanF32Plan {
@@ -1498,7 +1499,7 @@ int plan_scan_f32(const lact_scan_config& c, int32_t n_steps, const int32_t* kin
 
 int validate_scan_f32(const lact_scan_config& c) {
   if (c.B < 1 || c.L < 1 || c.D < 4 || c.H < 8 || c.out_len < 0 || (c.D % 4) != 0 || (c.H % 8) != 0) return LACT_ERR_SHAPE;
-  if (c.B > 65535 / 64 || c.L > (1ll << 30)) return LACT_ERR_SHAPE;
+  if (c.B > 65535 || c.L > (1ll << 30)) return LACT_ERR_SHAPE;
   if (c.act_dtype != LACT_F32) return LACT_ERR_DTYPE;
   if (c.use_muon) {
     if (c.ns_steps < 0 || c.ns_steps > 64 || (c.D % 8) != 0) return LACT_ERR_CONFIG;

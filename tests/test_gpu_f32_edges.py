@@ -13,6 +13,11 @@ def _inputs(B, L, D, H, seed=1):
     return {n: t.cuda() for n, t in orc.make_inputs(B, L, D, H, seed=seed).items()}
 
 
+def _close(a, b, tol):
+    assert torch.isfinite(a).all()
+    assert float((a - b).abs().max()) <= tol * float(b.abs().max())
+
+
 def test_momentum_after_an_empty_first_update():
     import lact_b200 as lb
     from lact_b200 import ops
@@ -29,3 +34,13 @@ def test_momentum_after_an_empty_first_update():
         lb.synchronize_and_check()
         for a, b in zip(list(got) + list(got_o), list(want) + list(want[:4])):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("B,L", [(1100, 9), (1025, 150)])
+def test_many_entries(B, L):
+    import lact_b200 as lb
+    i = _inputs(B, L, 4, 8)
+    chunk = 4 if L < 100 else 149
+    run = lambda s, e: lb.block_causal_lact_swiglu(*[i[n][s:e] for n in NAMES], chunk_size=chunk, momentum=i["momentum"][s:e])
+    got = run(0, B)
+    _close(got, torch.cat([run(0, 513), run(513, B)]), 1e-5)   # fp32 sums of at most 149 terms, split differently
