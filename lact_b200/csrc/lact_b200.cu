@@ -1460,6 +1460,7 @@ int f32_splits(int64_t R, int64_t C, int64_t B, int64_t len) {
 struct ScanF32Plan {
   int32_t* status;
   float *W02, *W1, *W02c, *W1c, *n02, *n1, *G02, *G1, *beta, *hidden, *dy02, *part02, *part1;
+  bool updates;  // some update has tokens
   NsPlan ns;
   size_t bytes;
 };
@@ -1488,6 +1489,7 @@ int plan_scan_f32(const lact_scan_config& c, int32_t n_steps, const int32_t* kin
   p->beta = cv.take<float>(B * static_cast<size_t>(std::max(1, n_steps)));
   p->hidden = cv.take<float>(B * static_cast<size_t>(std::max(max_apply, max_update)) * H);
   p->dy02 = cv.take<float>(B * static_cast<size_t>(max_update) * 2 * H);
+  p->updates = max_update > 0;
   // (splits grow with the token count: the longest update needs the most)
   p->part02 = cv.take<float>(max_update > 0 ? static_cast<size_t>(f32_splits(2 * c.H, c.D, c.B, max_update)) * B * 2 * H * D : 0);
   p->part1 = cv.take<float>(max_update > 0 ? static_cast<size_t>(f32_splits(c.D, c.H, c.B, max_update)) * B * D * H : 0);
@@ -1522,7 +1524,7 @@ int scan_fwd_f32(const lact_scan_config& c, const lact_scan_io& io, int32_t n_st
   for (int i = 0; i < n_steps; ++i)
     if (kind[i] == LACT_STEP_APPLY && (out_start[i] < 0 || out_start[i] + (end[i] - start[i]) > c.out_len)) return LACT_ERR_STEPS;
   const int64_t B = c.B, D = c.D, H = c.H;
-  if (D > kRenormMaxCols || H > kRenormMaxCols) return LACT_ERR_SHAPE;
+  if (p.updates && (D > kRenormMaxCols || H > kRenormMaxCols)) return LACT_ERR_SHAPE;  // (rows of an update's renormalisation)
   {
     KernelScope scope(kClsPrepare, stream);
     prepare_weights_kernel<<<ceil_div(B * (2 * H + D), 8), 256, 0, stream>>>(

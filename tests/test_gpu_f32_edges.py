@@ -44,3 +44,15 @@ def test_many_entries(B, L):
     run = lambda s, e: lb.block_causal_lact_swiglu(*[i[n][s:e] for n in NAMES], chunk_size=chunk, momentum=i["momentum"][s:e])
     got = run(0, B)
     _close(got, torch.cat([run(0, 513), run(513, B)]), 1e-5)   # fp32 sums of at most 149 terms, split differently
+
+
+@pytest.mark.parametrize("D,H", [(1036, 8), (16, 1048)])
+def test_rows_longer_than_an_update_takes(D, H):
+    import lact_b200 as lb
+    i = _inputs(1, 20, D, H)
+    got = lb.block_causal_lact_swiglu(*[i[n] for n in NAMES], chunk_size=32)   # one chunk: no update
+    w0, w1, w2, q = (i[n].double() for n in ("w0", "w1", "w2", "q"))
+    want = (torch.nn.functional.silu(q @ w0.transpose(1, 2)) * (q @ w2.transpose(1, 2))) @ w1.transpose(1, 2)
+    _close(got.double(), want, 1e-5)
+    with pytest.raises(ValueError):
+        lb.block_causal_lact_swiglu(*[i[n] for n in NAMES], chunk_size=8)
