@@ -62,6 +62,7 @@ std::vector<Tensor> scan_fwd(const Tensor& w0_, const Tensor& w1_, const Tensor&
   same_dtype(lr0, lr1, lr2);
   Tensor mom;
   if (mom_.defined()) mom = per_token(mom_, B, L, "momentum");
+  if (mom.defined() && f32) mom = mom.to(at::kFloat);  // (the mean of a bf16 gate is rounded to bf16, as a bf16 model's is)
 
   lact_scan_config c = base_config(o, B, L, D, H);
   // The reference drivers start from torch.zeros_like(q): tokens no APPLY step covers stay zero.

@@ -56,3 +56,11 @@ def test_rows_longer_than_an_update_takes(D, H):
     _close(got.double(), want, 1e-5)
     with pytest.raises(ValueError):
         lb.block_causal_lact_swiglu(*[i[n] for n in NAMES], chunk_size=8)
+
+
+def test_bf16_gate_is_averaged_in_fp32():
+    import lact_b200 as lb
+    i = _inputs(2, 90, 32, 16)
+    gate = i["momentum"].to(torch.bfloat16)
+    run = lambda m: lb.block_causal_lact_swiglu(*[i[n] for n in NAMES], chunk_size=30, momentum=m)
+    assert torch.equal(run(gate), run(gate.float()))
