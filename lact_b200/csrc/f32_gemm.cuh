@@ -30,6 +30,7 @@ struct F32Args {
   int32_t batch, splits, kper;  // split s covers k in [s * kper, min(K, (s + 1) * kper)); partial s at c + s * batch * c_bs
   float* c;
   int64_t c_ld, c_bs;
+  int32_t c_vec;        // kF32Store: rows of c start on 16 bytes (set by the launch)
   int32_t accumulate;   // kF32Store, splits = 1: c = acc + beta[batch] * c (beta nullptr: 1)
   const float* beta;
   // kF32Grad
@@ -165,7 +166,7 @@ __global__ void __launch_bounds__(kFThreads, MODE == kF32Grad ? 3 : 4) f32_gemm_
       for (int g = 0; g < 2; ++g) {
         const int n = n0 + g * 32 + tx * 4;
         float* o = C + static_cast<int64_t>(m) * a.c_ld + n;
-        if (n + 4 <= a.N && (a.c_ld & 3) == 0) {
+        if (n + 4 <= a.N && a.c_vec) {
           float4 r = make_float4(acc[i][g * 4], acc[i][g * 4 + 1], acc[i][g * 4 + 2], acc[i][g * 4 + 3]);
           if (a.accumulate) {
             const float4 old = *reinterpret_cast<const float4*>(o);

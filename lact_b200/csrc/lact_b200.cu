@@ -1443,6 +1443,7 @@ template <int MODE>
 int launch_f32_gemm(F32Args& a, cudaStream_t stream) {
   const dim3 grid(ceil_div(a.N, MODE == kF32Store ? kFN : 32), ceil_div(a.M, kFM), static_cast<unsigned>(a.batch * a.splits));
   if (a.M < 1 || a.N < 1 || a.K < 1 || grid.y > 65535 || static_cast<int64_t>(a.batch) * a.splits > 65535) return LACT_ERR_SHAPE;
+  a.c_vec = (reinterpret_cast<uintptr_t>(a.c) & 15) == 0 && (a.c_ld % 4) == 0 && (a.c_bs % 4) == 0;
   KernelScope scope(kClsOther, stream);
   LACT_CUDA(launch_pdl(f32_gemm_kernel<MODE>, grid, dim3(kFThreads), 0, stream, a));
   return LACT_OK;

@@ -64,3 +64,17 @@ def test_bf16_gate_is_averaged_in_fp32():
     gate = i["momentum"].to(torch.bfloat16)
     run = lambda m: lb.block_causal_lact_swiglu(*[i[n] for n in NAMES], chunk_size=30, momentum=m)
     assert torch.equal(run(gate), run(gate.float()))
+
+
+@pytest.mark.parametrize("M,N,K", [(3, 4, 5), (130, 64, 17), (65, 72, 16)])
+@pytest.mark.parametrize("shift", [(0, 0, 1), (1, 0, 0), (1, 3, 2)])
+def test_product_of_arrays_off_sixteen_bytes(M, N, K, shift):
+    """lact_sgemm_f32 takes arrays that start on any element."""
+    from lact_b200 import _lib as L
+    g = torch.Generator(device="cuda").manual_seed(M)
+    at = lambda n, s: torch.randn(n + s, device="cuda", generator=g)[s:]
+    a, b, c = at(2 * M * K, shift[0]), at(2 * N * K, shift[1]), at(2 * M * N, shift[2])
+    want = a.view(2, M, K).double() @ b.view(2, N, K).double().transpose(1, 2) + c.view(2, M, N).double()
+    L.check(L.lib().lact_sgemm_f32(a.data_ptr(), 0, b.data_ptr(), 0, c.data_ptr(), 1, None, 2, M, N, K, L.stream_ptr()), "sgemm")
+    torch.cuda.synchronize()
+    _close(c.view(2, M, N).double(), want, 1e-5)   # fp32 sums of at most 18 terms
