@@ -215,7 +215,7 @@ int lact_fw_grad(const void *w0w2, const void *w1, const void *k, const void *v,
 /* x[B, R, C] (bf16) = Newton-Schulz orthogonalisation of g[B, R, C] (g_dtype), bf16 arithmetic.
  * const_coeffs = 0: zeropower_via_newtonschulz5(G) (lact_llm/lact_model/ttt_operation.py:30-66),
  * steps must be 5; const_coeffs = 1: zeropower_via_newtonschulz5(G, steps)
- * (lact_nvs/lact_ttt.py:32-67). */
+ * (lact_nvs/lact_ttt.py:32-67).  g starts on four of its elements (else LACT_ERR_SHAPE). */
 int lact_newton_schulz_workspace_bytes(int64_t B, int64_t R, int64_t C, size_t *bytes_out);
 int lact_newton_schulz(const void *g, int32_t g_dtype, void *x, int64_t B, int64_t R, int64_t C, int32_t steps,
                        int32_t const_coeffs, void *workspace, size_t workspace_bytes, void *stream);

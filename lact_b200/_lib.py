@@ -228,6 +228,12 @@ def workspace(nbytes: int, device: torch.device) -> torch.Tensor:
     return torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
 
 
+def on_16_bytes(t: torch.Tensor) -> torch.Tensor:
+    """`t` (contiguous), copied if it starts off a 16-byte boundary (a view into a packed buffer): kernels read it 16 bytes
+    at a time."""
+    return t if t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format)
+
+
 _prepared = set()   # devices whose failures have a place to be reported in
 
 

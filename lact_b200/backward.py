@@ -93,6 +93,7 @@ def ns_forward_saved(G, steps, const_coeffs, gram_right):
     nmat, R, Cc = G.shape
     if G.dtype not in (torch.float32, BF16):
         G = G.float()
+    G = L.on_16_bytes(G)
     if int(steps) == 0:   # no iteration (lact_nvs/lact_ttt.py with muon_update_steps = 0): the normalisation alone
         from . import ops
         U = ops.zeropower_via_newtonschulz5(G, 0)

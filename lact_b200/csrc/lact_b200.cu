@@ -831,7 +831,8 @@ int launch_ns_chip(const NsGroup* grp, int ngroups, const void* const* src, int 
 int run_newton_schulz(NsGroup* grp, int ngroups, const void* const* src, int src_f32, const int* parts, int unscaled, int steps,
                       int const_coeffs, int32_t* status, cudaStream_t stream, const bf16** result, const NsKeep* keep = nullptr) {
   bool chip = steps >= 1 && steps <= 16 && (const_coeffs || steps == 5);
-  for (int g = 0; g < ngroups; ++g) chip = chip && ns_chip_fits(grp[g].R, grp[g].C, grp[g].transposed);
+  for (int g = 0; g < ngroups; ++g)  // (that kernel reads 16 bytes of the gradients at a time, the others half of that in bf16)
+    chip = chip && ns_chip_fits(grp[g].R, grp[g].C, grp[g].transposed) && (reinterpret_cast<uintptr_t>(src[g]) & 15) == 0;
   const bool given = parts != nullptr && parts[0] > 0;
   if (chip) return launch_ns_chip(grp, ngroups, src, src_f32, given ? parts : nullptr, unscaled, steps, const_coeffs, status, stream,
                                   result, keep);
@@ -1953,6 +1954,11 @@ int lact_newton_schulz_workspace_bytes(int64_t B, int64_t R, int64_t C, size_t* 
   return LACT_OK;
 }
 
+// The gradients are read four at a time.
+static bool ns_source_aligned(const void* g, int32_t g_dtype) {
+  return (reinterpret_cast<uintptr_t>(g) & (g_dtype == LACT_F32 ? 15 : 7)) == 0;
+}
+
 int lact_newton_schulz(const void* g, int32_t g_dtype, void* x, int64_t B, int64_t R, int64_t C, int32_t steps,
                        int32_t const_coeffs, void* workspace, size_t workspace_bytes, void* stream) {
   if (!g || !x) return LACT_ERR_NULL;
@@ -1961,6 +1967,7 @@ int lact_newton_schulz(const void* g, int32_t g_dtype, void* x, int64_t B, int64
   LACT_TRY(lact_newton_schulz_workspace_bytes(B, R, C, &need));
   if (!workspace || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 255)) return LACT_ERR_WORKSPACE;
   if (steps < 0 || steps > 64 || (!const_coeffs && steps != 5)) return LACT_ERR_CONFIG;
+  if (!ns_source_aligned(g, g_dtype)) return LACT_ERR_SHAPE;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   LACT_CUDA(cudaMemsetAsync(workspace, 0, 256, s));
   Carver cv(workspace);
@@ -2002,6 +2009,7 @@ int lact_ns_trace_fwd(const void* g, int32_t g_dtype, void* x_out, int64_t B, in
   LACT_TRY(check_device());
   if ((reinterpret_cast<uintptr_t>(trace) & 255) != 0) return LACT_ERR_WORKSPACE;
   if (!const_coeffs && steps != 5) return LACT_ERR_CONFIG;
+  if (!ns_source_aligned(g, g_dtype)) return LACT_ERR_SHAPE;
   NsTrace t;
   LACT_TRY(plan_ns_trace(trace, B, R, C, steps, gram_right, &t));
   if (t.bytes > trace_bytes) return LACT_ERR_WORKSPACE;

@@ -285,7 +285,7 @@ def zeropower_via_newtonschulz5(G: torch.Tensor, steps: Optional[int] = None) ->
         return _NewtonSchulz.apply(G, steps)
     if G.dtype not in (torch.float32, BF16):
         G = G.float()
-    G = G.contiguous()
+    G = L.on_16_bytes(G.contiguous())
     B, R, Cc = G.shape
     x = torch.empty(B, R, Cc, dtype=BF16, device=dev)
     lib = L.lib()
