@@ -1368,7 +1368,7 @@ int scan_fwd(const lact_scan_config& c, const lact_scan_io& io, int32_t n_steps,
 
     // add + renormalise arguments (the update is the Newton-Schulz result when Muon is on)
     // (the fp32 copy of the normalised weights is what pre-norm computes with and what the final export reads)
-    const bool want_compute = c.prenorm || (io.w0_out != nullptr && !has_later_update(kind, n_steps, i));
+    const bool want_compute = c.prenorm || ((io.w0_out || io.w1_out || io.w2_out) && !has_later_update(kind, n_steps, i));
     RenormArgs rn[2];
     for (int w = 0; w < 2; ++w) {
       RenormArgs& r = rn[w];

@@ -1,4 +1,6 @@
 """Arguments of the recurrence that reach past its usual form."""
+import ctypes as C
+
 import pytest
 import torch
 
@@ -31,3 +33,37 @@ def test_tensors_off_the_device_are_refused(act, train):
             a["w0"] = i["w0"]
         with pytest.raises((RuntimeError, ValueError), match="CUDA tensors only|same device"):
             ops.scan(*[a[n] for n in NAMES], P.causal_program(64, 32), momentum=a["momentum"], m_init=m)
+
+
+@pytest.mark.parametrize("which", [("w0",), ("w1",), ("w2",), ("w1", "w2")])
+def test_c_abi_returns_each_weight_by_itself(which):
+    """The final weights are optional one by one (each out pointer may be NULL)."""
+    from lact_b200 import _lib as L
+    from lact_b200 import ops
+    from lact_b200 import program as P
+    B, n, D, H = 2, 128, 64, 32
+    i = _inputs(B, n, D, H)
+    steps = P.causal_program(n, 64)
+    want = dict(zip(("o", "w0", "w1", "w2"), ops.scan(*[i[x] for x in NAMES], steps, return_state=True)))
+    cfg, io = L.ScanConfig(), L.ScanIO()
+    cfg.B, cfg.L, cfg.D, cfg.H, cfg.out_len, cfg.act_dtype, cfg.renorm, cfg.w_scale = B, n, D, H, n, L.LACT_BF16, L.RENORM_EPS_OUTSIDE, 1.0
+    for x in ("q", "k", "v", "o"):
+        setattr(cfg, x + "_bs", n * D)
+        setattr(cfg, x + "_ts", D)
+    out = {x: torch.full(want[x].shape, float("nan"), device="cuda") for x in which}
+    o = torch.empty(B, n, D, dtype=BF16, device="cuda")
+    for x in NAMES:
+        setattr(io, x, i[x].data_ptr())
+    io.o = o.data_ptr()
+    for x in which:
+        setattr(io, x + "_out", out[x].data_ptr())
+    m = len(steps)
+    kind, start, end, outs = ((t * m)(*[s[j] for s in steps]) for j, t in enumerate((C.c_int32, C.c_int64, C.c_int64, C.c_int64)))
+    need = C.c_size_t(0)
+    L.check(L.lib().lact_scan_workspace_bytes(C.byref(cfg), m, kind, start, end, C.byref(need)), "bytes")
+    ws = torch.empty(need.value, dtype=torch.uint8, device="cuda")
+    L.check(L.lib().lact_scan_fwd(C.byref(cfg), C.byref(io), m, kind, start, end, outs, ws.data_ptr(), need, L.stream_ptr()), "scan")
+    torch.cuda.synchronize()
+    assert torch.equal(o, want["o"])
+    for x in which:
+        assert torch.equal(out[x], want[x]), x
