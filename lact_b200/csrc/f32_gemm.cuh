@@ -226,6 +226,7 @@ struct F32ReduceArgs {
   int64_t n[2];
   int32_t splits[2];
   int32_t batch, accumulate;
+  int32_t fresh;  // accumulate: c counts as zeros and is not read
   const float* beta;
 };
 __global__ void __launch_bounds__(256) f32_reduce_kernel(const F32ReduceArgs a) {
@@ -245,7 +246,7 @@ __global__ void __launch_bounds__(256) f32_reduce_kernel(const F32ReduceArgs a) 
   float4* o = reinterpret_cast<float4*>(a.c[w] + i * 4);
   if (a.accumulate) {
     const float bt = a.beta != nullptr ? a.beta[i * 4 / a.n[w]] : 1.f;
-    const float4 old = *o;
+    const float4 old = a.fresh ? make_float4(0.f, 0.f, 0.f, 0.f) : *o;
     s = make_float4(fmaf(old.x, bt, s.x), fmaf(old.y, bt, s.y), fmaf(old.z, bt, s.z), fmaf(old.w, bt, s.w));
   }
   *o = s;

@@ -420,6 +420,7 @@ struct GradArgs {
   bf16* gb1 = nullptr;
   const float* g02_prev = nullptr;  // optional: momentum state read from here instead of g02 / g1 (fp32)
   const float* g1_prev = nullptr;
+  int32_t fresh = 0;                // 1: the momentum state is still zero
   SplitScratch split;               // optional: scratch for a split contraction
 };
 
@@ -478,14 +479,14 @@ int run_grad(const GradArgs& a, int32_t* status, cudaStream_t stream) {
     P0.M = static_cast<int>(2 * a.H); P0.N = static_cast<int>(a.D); P0.K = static_cast<int>(len);
     P0.batch = static_cast<int>(a.B);
     P0.ep = EpiDW{a.g02, 2 * a.H * a.D, a.D, a.beta, 1, a.g_f32, a.partial02, ceil_div(2 * a.H, kBM),
-                  ceil_div(a.D, btv), a.gb02, a.g02_prev};
+                  ceil_div(a.D, btv), a.gb02, a.g02_prev, a.fresh};
     auto& P1 = g.prob[1];
     LACT_TRY(make_operand(kb_of(P1), &P1.a[0], &P1.ai[0], vm, 1, kBM, 0, static_cast<int>(a.start)));
     LACT_TRY(make_operand(kb_of(P1), &P1.b[0], &P1.bi[0], hid, 1, btv, 0, 0));
     P1.M = static_cast<int>(a.D); P1.N = static_cast<int>(a.H); P1.K = static_cast<int>(len);
     P1.batch = static_cast<int>(a.B);
     P1.ep = EpiDW{a.g1, a.D * a.H, a.H, a.beta, 1, a.g_f32, a.partial1, ceil_div(a.D, kBM), ceil_div(a.H, btv),
-                  a.gb1, a.g1_prev};
+                  a.gb1, a.g1_prev, a.fresh};
     set_split(P0, split, a.split);
     set_split(P1, split, a.split);
     g.status = status;
@@ -1198,8 +1199,8 @@ int scan_ns_trace_layout(const lact_scan_config& c, size_t* stride, size_t* g0_b
   return LACT_OK;
 }
 
-// Momentum state the program starts from: the caller's.  Without one the first update has nothing to add to its gradient
-// (it runs without a momentum factor), and zeros are written only for a program that hands the state back untouched.
+// Momentum state the program starts from: the caller's.  Without one the first update adds its factor times zero without
+// reading it, and zeros are written only for a program that hands the state back untouched.
 inline bool has_initial_momentum(const lact_scan_io& io) { return io.m0_in && io.m1_in && io.m2_in; }
 int load_momentum_state(const lact_scan_config& c, const lact_scan_io& io, float* G02, float* G1, cudaStream_t stream) {
   const size_t B = c.B, D = c.D, H = c.H;
@@ -1318,8 +1319,8 @@ int scan_fwd(const lact_scan_config& c, const lact_scan_io& io, int32_t n_steps,
       LACT_TRY(run_apply(a, p.status, stream));
       continue;
     }
-    const float* beta = c.use_momentum && (update_idx > 0 || has_initial_momentum(io))
-                            ? p.beta + static_cast<int64_t>(update_idx) * B : nullptr;
+    const float* beta = c.use_momentum ? p.beta + static_cast<int64_t>(update_idx) * B : nullptr;
+    const bool fresh = update_idx == 0 && !has_initial_momentum(io);
     float* dump = nullptr;
     if (io.state_dump != nullptr && !dump_in_place) {
       // training (pre-norm): the weights this update computed with and (below) its gradient after momentum are copied
@@ -1340,6 +1341,7 @@ int scan_fwd(const lact_scan_config& c, const lact_scan_io& io, int32_t n_steps,
                c.lr_dtype == LACT_F32, c.L, c.w_scale, p.dy02, p.hid, G02cur, G1cur, 1, beta, B, D, H};
     g.g02_prev = G02prev;
     g.g1_prev = G1prev;
+    g.fresh = fresh;
     g.split = p.split;
     // The Frobenius norms Newton-Schulz needs are gathered per output tile by the contraction when a
     // tile never straddles two matrices (concatenated [2H, D], or H a multiple of the 128-row tile).
@@ -1582,8 +1584,9 @@ int scan_fwd_f32(const lact_scan_config& c, const lact_scan_io& io, int32_t n_st
     F32ReduceArgs red;
     std::memset(&red, 0, sizeof(red));
     red.batch = static_cast<int32_t>(B);
-    red.accumulate = c.use_momentum && state_written;
-    red.beta = red.accumulate ? p.beta + static_cast<int64_t>(u) * B : nullptr;
+    red.accumulate = c.use_momentum;
+    red.fresh = !state_written;
+    red.beta = c.use_momentum ? p.beta + static_cast<int64_t>(u) * B : nullptr;
     state_written = true;
     for (int w = 0; w < 2; ++w) {  // [dw0; dw2] = dy^T k, dw1 = v^T hidden
       const int64_t R = w == 0 ? 2 * H : D, C = w == 0 ? D : H;

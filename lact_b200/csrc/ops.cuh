@@ -85,6 +85,7 @@ struct EpiDW {
   // optional: the momentum state is read from here instead of `g` (same layout, fp32): training keeps every update's
   // state in its own slot, so the previous one is read and the next one written without a copy in between
   const float* g_prev = nullptr;
+  int32_t fresh = 0;  // 1: the state is all zeros and is not read (beta * 0 is added: a NaN or infinite gate shows)
   // One warp's 32 x 32 block of results, thread `lane` holding row `row0 + lane` in v[0..31].  The block goes
   // through `scratch` (this warp's 32 x 144 bytes of shared memory) so that the read-modify-write of the fp32
   // state is issued with eight lanes per 128-byte row segment (four full lines per instruction) instead of one
@@ -111,7 +112,7 @@ struct EpiDW {
     for (int i = 0; i < 8; ++i) {
       const int row = row0 + i * 4 + rsub;
       old[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (rmw && col_ok && row < M)
+      if (rmw && !fresh && col_ok && row < M)
         old[i] = *reinterpret_cast<const float4*>((g_prev != nullptr ? g_prev : reinterpret_cast<const float*>(g)) + base +
                                                   static_cast<int64_t>(row) * ld);
     }

@@ -67,3 +67,18 @@ def test_c_abi_returns_each_weight_by_itself(which):
     assert torch.equal(o, want["o"])
     for x in which:
         assert torch.equal(out[x], want[x]), x
+
+
+@pytest.mark.parametrize("act", [BF16, torch.float32])
+@pytest.mark.parametrize("muon", [False, True])
+def test_nan_gate_of_the_first_chunk_reaches_the_weights(act, muon):
+    import lact_b200 as lb
+    i = _inputs(2, 256, 64, 64, act)
+    clean = lb.block_causal_lact_swiglu(*[i[n] for n in NAMES], chunk_size=64, use_muon=muon, momentum=i["momentum"])
+    for bad in (float("nan"), float("inf")):
+        m = i["momentum"].clone()
+        m[1, 3] = bad
+        o = lb.block_causal_lact_swiglu(*[i[n] for n in NAMES], chunk_size=64, use_muon=muon, momentum=m)
+        lb.synchronize_and_check()
+        assert torch.equal(o[0], clean[0]) and torch.equal(o[1, :64], clean[1, :64])
+        assert bool(o[1, 64:].isnan().all())   # bad * 0 (the state before the first update)
