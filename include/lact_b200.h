@@ -451,11 +451,13 @@ int lact_momentum_bwd(const void *dg0, const void *dg1, void *carry0, void *carr
                       int32_t add_carry, void *stream);
 
 /* Ends of the reverse sweep: momentum factors beta[n][B] = mean of momentum[b, start:end] per update
- * (ttt_operation.py:170-172), the gradient of the momentum gate from dbeta [n][B][slices] (every token of [B, L] written),
+ * (ttt_operation.py:170-172), the gradient of the momentum gate from dbeta [n][B][slices] (every token of [B, L] written;
+ * in launches of LACT_GATE_GRAD_UPDATES updates, later ones adding to `out`: with more updates use an fp32 `out`),
  * and the gradients of the initial weights (caller's layout and dtype) from the stacked state gradients: dW (+ dWm)
  * + dn[row] * W / n[row] (dn NULL: target norms detached). */
 int lact_momentum_means(const void *momentum, int32_t dtype, int64_t B, int64_t L, int32_t n, const int64_t *start,
                         const int64_t *end, float *beta, void *stream);
+#define LACT_GATE_GRAD_UPDATES 64
 int lact_momentum_gate_grad(const float *dbeta, int64_t B, int64_t L, int32_t n, const int64_t *start, const int64_t *end,
                             void *out, int32_t out_dtype, void *stream);
 int lact_weight_grad(const float *dW02, const float *dW1, const float *dWm02, const float *dWm1, const float *dn02,

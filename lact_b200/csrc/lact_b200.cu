@@ -2950,6 +2950,7 @@ int lact_momentum_gate_grad(const float* dbeta, int64_t B, int64_t L, int32_t n,
                             void* out, int32_t out_dtype, void* stream) {
   if (!dbeta || !out || (n > 0 && (!start || !end))) return LACT_ERR_NULL;
   if (B < 1 || B > 65535 || L < 1 || n < 0) return LACT_ERR_SHAPE;
+  static_assert(kMeanBatch == LACT_GATE_GRAD_UPDATES, "the header names the launch's size");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   int first = 0;
   do {

@@ -243,7 +243,8 @@ std::vector<Tensor> scan_bwd(const Tensor& w0, const Tensor& w1, const Tensor& w
   std::vector<Tensor> r{dw0.to(w0.scalar_type()), dw1.to(w1.scalar_type()), dw2.to(w2.scalar_type()), dq.to(q_.scalar_type()),
                         dk.to(k_.scalar_type()), dv.to(v_.scalar_type()), like(dlr[0], lr0), like(dlr[1], lr1), like(dlr[2], lr2)};
   if (has_mom) {
-    const bool mb = momentum->scalar_type() == BF;
+    // (bf16 only where one launch writes it: later ones add to what is there)
+    const bool mb = momentum->scalar_type() == BF && st.updates <= LACT_GATE_GRAD_UPDATES;
     Tensor dm = empty({B, L}, mb ? BF : F, k);
     if (st.updates > 0)
       check(lact_momentum_gate_grad(dbeta.data_ptr<float>(), B, L, st.updates, us.data(), ue.data(), ptr(dm), mb ? LACT_BF16 : LACT_F32,

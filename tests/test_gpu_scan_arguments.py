@@ -82,3 +82,19 @@ def test_nan_gate_of_the_first_chunk_reaches_the_weights(act, muon):
         lb.synchronize_and_check()
         assert torch.equal(o[0], clean[0]) and torch.equal(o[1, :64], clean[1, :64])
         assert bool(o[1, 64:].isnan().all())   # bad * 0 (the state before the first update)
+
+
+def test_gate_gradient_over_many_updates_is_summed_in_fp32():
+    from lact_b200 import ops
+    from lact_b200 import program as P
+    i = _inputs(2, 64, 32, 32)
+    steps = [(P.UPDATE, 0, 32, 0)] * 150 + [(P.APPLY, 0, 64, 0)]
+    dO = torch.randn(2, 64, 32, device="cuda", generator=torch.Generator(device="cuda").manual_seed(3)).to(BF16)
+
+    def grad(m):
+        m = m.requires_grad_(True)
+        return torch.autograd.grad(ops.scan(*[i[n] for n in NAMES], steps, momentum=m), m, dO)[0]
+    gate = torch.full((2, 64, 1), 0.5, device="cuda")   # its mean is exact in bf16
+    a, b = grad(gate.to(BF16)), grad(gate)
+    assert a.dtype == BF16 and float(b.abs().max()) > 0
+    assert torch.equal(a, b.to(BF16))
