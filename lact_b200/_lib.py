@@ -173,21 +173,17 @@ def load_ops() -> None:
     _ops_lib.lact_torch_take_status.restype = C.c_int
     _ops_lib.lact_torch_prepare_status.argtypes = [C.c_int]
     _ops_lib.lact_torch_prepare_status.restype = C.c_int
+    _ops_lib.lact_torch_set_error_type.argtypes = [C.py_object]
+    _ops_lib.lact_torch_set_error_type.restype = None
+    _ops_lib.lact_torch_set_error_type(LactError)   # what a device status or a CUDA error is raised as
     from . import _fakes  # noqa: F401
     _ops_loaded = True
 
 
 def call(op, *args):
-    """One operator call; a device status or a CUDA error the operator reports becomes a LactError."""
-    if torch.compiler.is_compiling():
-        return op(*args)
-    try:
-        out = op(*args)
-    except RuntimeError as e:
-        if str(e).startswith("lact_b200: "):
-            raise LactError(str(e).split("\n", 1)[0]) from None
-        raise
-    if SYNC_CHECK:
+    """One operator call; with LACT_B200_SYNC_CHECK=1 it is waited for and its status checked."""
+    out = op(*args)
+    if SYNC_CHECK and not torch.compiler.is_compiling():
         synchronize_and_check()
     return out
 

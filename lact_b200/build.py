@@ -46,13 +46,15 @@ def _run(cmd, what: str, verbose: bool) -> None:
 
 def build_torch(verbose: bool = False) -> str:
     """Compiles the operator library against the installed PyTorch (the sources in parallel, then one link)."""
+    import sysconfig
     import tempfile
     from concurrent.futures import ThreadPoolExecutor
 
     import torch
     from torch.utils import cpp_extension
     cuda = os.path.dirname(os.path.dirname(find_nvcc()))
-    inc = [f for p in cpp_extension.include_paths() + [os.path.join(cuda, "include")] for f in ("-isystem", p)]
+    inc = [f for p in cpp_extension.include_paths() + [os.path.join(cuda, "include"), sysconfig.get_path("include")]
+           for f in ("-isystem", p)]
     abi = f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"
     libdir = os.path.join(os.path.dirname(torch.__file__), "lib")
     # the system compiler, as nvcc uses it: its libstdc++ is the shared one PyTorch is linked with (a compiler that links its
@@ -64,7 +66,7 @@ def build_torch(verbose: bool = False) -> str:
         with ThreadPoolExecutor(max(1, min(len(jobs), os.cpu_count() or 1))) as pool:
             list(pool.map(lambda c: _run(c, "g++", verbose), jobs))
         _run([cxx, "-shared", "-o", TORCH_LIB, *objs, "-L" + PKG_DIR, "-l:liblact_b200.so", "-L" + libdir, "-lc10", "-lc10_cuda",
-              "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-Wl,-rpath,$ORIGIN"], "link", verbose)
+              "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python", "-Wl,-rpath,$ORIGIN"], "link", verbose)
     return TORCH_LIB
 
 

@@ -22,14 +22,17 @@ using torch::autograd::variable_list;
 
 enum Step : int64_t { kApply = LACT_STEP_APPLY, kUpdate = LACT_STEP_UPDATE };
 
-// Return code of the C ABI -> exception (ValueError for arguments, RuntimeError for the device).
+// Throws the Python package's LactError, from forwards and backwards alike (status.cpp).
+[[noreturn]] void fail(const std::string& message);
+
+// Return code of the C ABI -> exception (ValueError for arguments, LactError for the device).
 inline void check(int rc, const char* what) {
   if (rc == LACT_OK) return;
   const char* msg = lact_error_string(rc);
   TORCH_CHECK_VALUE(!(rc == LACT_ERR_NULL || rc == LACT_ERR_SHAPE || rc == LACT_ERR_DTYPE || rc == LACT_ERR_CONFIG ||
                       rc == LACT_ERR_STEPS),
                     what, ": ", msg, " (code ", rc, ")");
-  TORCH_CHECK(false, "lact_b200: ", what, ": ", msg, " (code ", rc, ")");
+  fail(c10::str("lact_b200: ", what, ": ", msg, " (code ", rc, ")"));
 }
 
 inline int dtype_code(const Tensor& t) {

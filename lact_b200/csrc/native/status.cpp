@@ -2,7 +2,10 @@
 // (lact_status_host_word).  An operator reads that word before it enqueues (one load); a non-zero word is reported as an
 // exception and cleared together with the device-side words.  This replaced a 4-byte device-to-host copy, an event and
 // a memset per call: about 5 us of stream time and 12 us of host time each.
+#include <Python.h>
+
 #include <c10/cuda/CUDAGraphsC10Utils.h>
+#include <torch/csrc/Exceptions.h>
 
 #include <atomic>
 #include <mutex>
@@ -12,6 +15,17 @@
 
 namespace lact_torch {
 namespace {
+
+std::atomic<PyObject*> g_error_type{nullptr};  // lact_b200.LactError, kept alive by its module
+
+// PyTorch turns exceptions of this kind into Python ones of their type, also those that leave an autograd node.
+struct Failure : torch::PyTorchError {
+  using torch::PyTorchError::PyTorchError;
+  PyObject* python_type() override {
+    PyObject* t = g_error_type.load();
+    return t != nullptr ? t : PyExc_RuntimeError;
+  }
+};
 
 constexpr int kMaxDevices = 64;
 std::atomic<int32_t*> g_host[kMaxDevices];
@@ -36,6 +50,8 @@ volatile int32_t* host_word(int dev) {
 
 }  // namespace
 
+void fail(const std::string& message) { throw Failure(message); }
+
 void poll_status(const Tensor& like) {
   const int dev = like.device().index();
   TORCH_CHECK(dev >= 0 && dev < kMaxDevices, "unsupported device index");
@@ -44,7 +60,7 @@ void poll_status(const Tensor& like) {
   if (st == 0) return;
   *w = 0;
   g_epoch.fetch_add(1);
-  TORCH_CHECK(false, "lact_b200: device status: ", lact_error_string(st), " (code ", st, ")");
+  fail(c10::str("lact_b200: device status: ", lact_error_string(st), " (code ", st, ")"));
 }
 
 StatusWord status_word(const Tensor& like) {
@@ -95,3 +111,6 @@ extern "C" int lact_torch_prepare_status(int device) {
   if (rc == LACT_OK) lact_torch::g_host[device].store(w, std::memory_order_release);
   return rc;
 }
+
+// The class of `fail`'s exceptions.
+extern "C" void lact_torch_set_error_type(PyObject* type) { lact_torch::g_error_type.store(type); }

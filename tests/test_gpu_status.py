@@ -1,4 +1,5 @@
 """Device status and stream capture."""
+import ctypes as C
 import os
 import subprocess
 import sys
@@ -114,3 +115,36 @@ else:
 lb.zeropower_via_newtonschulz5(rn(1, 64, 64))
 lb.synchronize_and_check()
 """)
+
+
+def _fail_on_host():
+    from lact_b200 import _lib as L
+    word = C.POINTER(C.c_int32)()
+    L.check(L.lib().lact_status_host_word(C.byref(word)), "word")
+    word[0] = 101
+
+
+@pytest.mark.parametrize("kind", ["scan", "attention", "ffn", "grads"])
+def test_failure_found_in_a_backward_is_a_lact_error(kind):
+    ns = {}
+    exec(SETUP, ns)
+    lb, lo, bf, rn = (ns[n] for n in ("lb", "lo", "bf", "rn"))
+    leaf = lambda t: t.requires_grad_(True)
+    if kind == "scan":
+        o = lb.block_causal_lact_swiglu(*[leaf(t) for t in ns["scan_args"]()], chunk_size=64)
+    elif kind == "attention":
+        o = lo.sliding_window_attention(*[leaf(bf(1, 300, 2, 64)) for _ in range(3)], 128)
+    elif kind == "ffn":
+        o = lb.fused_swiglu_ffn_fwd(leaf(bf(2, 128, 64)), leaf(bf(2, 64, 64)), leaf(bf(2, 40, 64)))
+    else:
+        o = lb.fused_lact_swiglu_ffn_fast_weight_grads(leaf(bf(2, 128, 64)), leaf(bf(2, 64, 64)), leaf(bf(2, 40, 64)), leaf(bf(2, 40, 64)),
+                                                       *[torch.rand(2, 40, device="cuda") for _ in range(3)])[0]
+    lb.synchronize_and_check()
+    _fail_on_host()
+    with pytest.raises(lb.LactError, match="101"):
+        o.backward(torch.ones_like(o))
+    with pytest.raises(ValueError):   # (arguments stay ValueError)
+        lb.block_causal_lact_swiglu(*ns["scan_args"]()[:8], torch.rand(1, 3, 1, device="cuda"), chunk_size=64)
+    _fail_on_host()
+    with pytest.raises(lb.LactError, match="101"):
+        lb.block_causal_lact_swiglu(*ns["scan_args"](), chunk_size=64)
