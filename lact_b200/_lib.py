@@ -183,7 +183,7 @@ def load_ops() -> None:
 def call(op, *args):
     """One operator call; with LACT_B200_SYNC_CHECK=1 it is waited for and its status checked."""
     out = op(*args)
-    if SYNC_CHECK and not torch.compiler.is_compiling():
+    if SYNC_CHECK and not torch.compiler.is_compiling() and not torch.cuda.is_current_stream_capturing():
         synchronize_and_check()
     return out
 
@@ -213,7 +213,8 @@ def stream_ptr() -> int:
     return torch.cuda.current_stream().cuda_stream
 
 
-# LACT_B200_SYNC_CHECK=1 waits for the device and checks its status after every operator call (debugging).
+# LACT_B200_SYNC_CHECK=1 waits for the device and checks its status after every operator call, backwards included, outside
+# stream captures (debugging).
 SYNC_CHECK = os.environ.get("LACT_B200_SYNC_CHECK", "0") == "1"
 
 
@@ -253,7 +254,7 @@ def mark_pending(ws: torch.Tensor) -> None:
     """Called after a library call has been enqueued with `ws` as its workspace.  Kernels that give up leave their status
     in a word of mapped host memory (`lact_status_host_word`): reading it here raises for any EARLIER call that has
     failed by now, without copies, events or waits."""
-    if SYNC_CHECK:
+    if SYNC_CHECK and not torch.cuda.is_current_stream_capturing():
         read_status(ws)
     _take_status(ws.device.index)
 

@@ -64,6 +64,7 @@ std::vector<Tensor> swa_bwd(const Tensor& q_, const Tensor& k_, const Tensor& v_
                      dout.stride(1), dout.stride(0), window, static_cast<float>(scale), static_cast<const int32_t*>(ptr(seq)),
                      status_word(q), stream_of(q)),
         "lact_swa_bwd");
+  settle(q);
   return {dq, dk, dv};
 }
 

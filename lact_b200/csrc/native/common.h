@@ -67,6 +67,9 @@ struct StatusWord {
 };
 StatusWord status_word(const Tensor& like);
 void poll_status(const Tensor& like);
+// End of a backward: with LACT_B200_SYNC_CHECK=1 (and no capture) waits for the stream and reports what it has left (forwards
+// are waited for in Python).
+void settle(const Tensor& like);
 
 // A [batch, rows, cols] bf16 activation whose last axis is contiguous and whose strides and base keep 16-byte alignment
 // (views of fused projections pass through); anything else is copied.

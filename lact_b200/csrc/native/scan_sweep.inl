@@ -253,6 +253,7 @@ std::vector<Tensor> scan_bwd(const Tensor& w0, const Tensor& w1, const Tensor& w
     else dm.zero_();
     r.push_back(like(dm, *momentum));
   }
+  settle(k);
   return r;
 }
 

@@ -8,7 +8,9 @@
 #include <torch/csrc/Exceptions.h>
 
 #include <atomic>
+#include <cstdlib>
 #include <mutex>
+#include <string_view>
 #include <unordered_map>
 
 #include "common.h"
@@ -63,9 +65,21 @@ void poll_status(const Tensor& like) {
   fail(c10::str("lact_b200: device status: ", lact_error_string(st), " (code ", st, ")"));
 }
 
+static bool capturing() { return c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None; }
+
+void settle(const Tensor& like) {
+  static const bool on = [] {
+    const char* v = std::getenv("LACT_B200_SYNC_CHECK");
+    return v != nullptr && std::string_view(v) == "1";
+  }();
+  if (!on || capturing()) return;
+  c10::cuda::getCurrentCUDAStream(like.device().index()).synchronize();
+  poll_status(like);
+}
+
 StatusWord status_word(const Tensor& like) {
   poll_status(like);
-  if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) {
+  if (capturing()) {
     // The stream's shared word would be cleared (or not) by whatever runs between the replays, and if its clearing fell
     // into this capture it would only be recorded.
     Tensor own = empty({64}, at::kInt, like).zero_();

@@ -41,6 +41,7 @@ std::vector<Tensor> ffn_bwd(const Tensor& w02_, const Tensor& w1_, const Tensor&
   Tensor dw02 = empty(w02.sizes(), at::kFloat, x), dw1 = empty(w1.sizes(), at::kFloat, x), dx = empty({B, N, D}, at::kBFloat16, x);
   TokenBackward tok(B, D, H, x, status_word(x), stream_of(x));
   tok.apply(View(w02), View(w1), View(x), View(g), N, View(dw02), View(dw1), false, View(dx));
+  settle(x);
   return {dw02.to(at::kBFloat16), dw1.to(at::kBFloat16), dx};
 }
 
@@ -102,6 +103,7 @@ std::vector<Tensor> grads_bwd(const Tensor& w02, const Tensor& w1, const Tensor&
   TokenBackward tok(B, D, H, k, status_word(k), stream_of(k));
   tok.gradient(View(w02), View(w1), View(k), View(v), N, lp, dtype_code(lr0), N, 1.0f, View(g02), View(g1), View(dw02), View(dw1),
                false, View(dk), View(dv), gp, N, false);
+  settle(k);
   return {dw02.to(BF), dw1.to(BF), dk, dv, glr[0].to(lr0.scalar_type()), glr[1].to(lr1.scalar_type()), glr[2].to(lr2.scalar_type())};
 }
 

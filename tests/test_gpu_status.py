@@ -148,3 +148,22 @@ def test_failure_found_in_a_backward_is_a_lact_error(kind):
     _fail_on_host()
     with pytest.raises(lb.LactError, match="101"):
         lb.block_causal_lact_swiglu(*ns["scan_args"](), chunk_size=64)
+
+
+def test_sync_check_covers_backwards():
+    out = _python("""
+leaves, dout = [t.requires_grad_(True) for t in scan_args()], bf(1, 256, 64)
+o = lb.block_causal_lact_swiglu(*leaves, chunk_size=64)
+torch.cuda.set_sync_debug_mode("error")
+try:
+    torch.autograd.grad(o, leaves, dout)
+except RuntimeError as e:
+    print("waited" if "synchronizing" in str(e) else e)
+torch.cuda.set_sync_debug_mode("default")
+# and a capture is left alone
+call = make("train")
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    call()
+""", LACT_B200_SYNC_CHECK="1")
+    assert "waited" in out
