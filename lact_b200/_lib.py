@@ -167,6 +167,10 @@ def load_ops() -> None:
     if not os.path.exists(OPS_PATH):
         raise ImportError(f"{OPS_PATH} is missing: build it with `python -m lact_b200.build` "
                           "(there is no fallback implementation)")
+    from . import build
+    if not build.built_for_this_torch(OPS_PATH):
+        raise ImportError(f"{OPS_PATH} was built for another PyTorch than {torch.__version__}: rebuild it with "
+                          "`python -m lact_b200.build`")
     torch.ops.load_library(OPS_PATH)
     _ops_lib = C.CDLL(OPS_PATH)
     _ops_lib.lact_torch_take_status.argtypes = [C.c_int]

@@ -34,6 +34,17 @@ def is_stale(lib: str = LIB, deps=DEPS) -> bool:
     return any(os.path.getmtime(d) > t for d in deps if os.path.exists(d))
 
 
+def torch_stamp() -> str:
+    """What the operator library built here carries: it fits the PyTorch it was compiled against and no other."""
+    import torch
+    return f"lact_b200 operators for PyTorch {torch.__version__};"
+
+
+def built_for_this_torch(lib: str = TORCH_LIB) -> bool:
+    with open(lib, "rb") as f:
+        return torch_stamp().encode() in f.read()
+
+
 def _run(cmd, what: str, verbose: bool) -> None:
     if verbose:
         print(" ".join(cmd))
@@ -62,7 +73,8 @@ def build_torch(verbose: bool = False) -> str:
     cxx = shutil.which("g++") or "c++"
     with tempfile.TemporaryDirectory() as tmp:
         objs = [os.path.join(tmp, os.path.basename(s) + ".o") for s in TORCH_SRC]
-        jobs = [[cxx, "-O2", "-std=c++20", "-fPIC", "-w", abi, *inc, "-c", s, "-o", o] for s, o in zip(TORCH_SRC, objs)]
+        stamp = f'-DLACT_TORCH_BUILD="{torch_stamp()}"'
+        jobs = [[cxx, "-O2", "-std=c++20", "-fPIC", "-w", abi, stamp, *inc, "-c", s, "-o", o] for s, o in zip(TORCH_SRC, objs)]
         with ThreadPoolExecutor(max(1, min(len(jobs), os.cpu_count() or 1))) as pool:
             list(pool.map(lambda c: _run(c, "g++", verbose), jobs))
         _run([cxx, "-shared", "-o", TORCH_LIB, *objs, "-L" + PKG_DIR, "-l:liblact_b200.so", "-L" + libdir, "-lc10", "-lc10_cuda",
@@ -77,7 +89,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if verbose:
             cmd.insert(1, "-Xptxas=-v")
         _run(cmd, "nvcc", verbose)
-    if force or is_stale(TORCH_LIB, TORCH_DEPS):
+    if force or is_stale(TORCH_LIB, TORCH_DEPS) or not built_for_this_torch():
         build_torch(verbose)
     return LIB
 

@@ -126,5 +126,8 @@ extern "C" int lact_torch_prepare_status(int device) {
   return rc;
 }
 
+// The PyTorch this library was compiled against (LACT_TORCH_BUILD, from build.py, which looks for it in the file).
+extern "C" const char lact_torch_build[] = LACT_TORCH_BUILD;
+
 // The class of `fail`'s exceptions.
 extern "C" void lact_torch_set_error_type(PyObject* type) { lact_torch::g_error_type.store(type); }
