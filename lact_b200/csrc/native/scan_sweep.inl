@@ -113,7 +113,7 @@ std::vector<Tensor> scan_bwd(const Tensor& w0, const Tensor& w1, const Tensor& w
   }
   // (in part, if ranges overlap: what no step has written yet of a range that is added to is zeroed first)
   using Ranges = std::vector<std::pair<int64_t, int64_t>>;
-  Ranges q_done, kv_done;
+  Ranges q_done, kv_done, o_done;
   // Whether [s, e) has been written nowhere; otherwise `missing` receives the parts of it that have not.
   auto first = [](Ranges& done, int64_t s, int64_t e, Ranges& missing) {
     bool ok = true;
@@ -131,7 +131,7 @@ std::vector<Tensor> scan_bwd(const Tensor& w0, const Tensor& w1, const Tensor& w
     done.emplace_back(s, e);
     return ok;
   };
-  Ranges missing;
+  Ranges missing, kept_out;
 
   TokenBackward tok(B, D, H, k, sw.status, stream);
   int cnt = st.updates;
@@ -139,10 +139,22 @@ std::vector<Tensor> scan_bwd(const Tensor& w0, const Tensor& w1, const Tensor& w
     const int64_t s = st.start[i], e = st.end[i], n = e - s;
     if (n <= 0) continue;
     if (st.kind[i] == kApply) {
+      // (of outputs that a later step writes again, only the last has a gradient)
+      const int64_t at = st.out[i];
+      Tensor last;
+      View go = tokens(dO, at);
+      if (!first(o_done, at, at + n, kept_out)) {
+        last = at::zeros({B, n, D}, dO.options());
+        for (auto& [a, b] : kept_out) last.narrow(1, a - at, b - a).copy_(dO.narrow(1, a, b - a));
+        go = View(last);
+      }
       const bool own = first(q_done, s, e, missing);
+      if (last.defined() && kept_out.empty()) {
+        for (auto& [a, b] : missing) dq.narrow(1, a, b - a).zero_();
+        continue;
+      }
       Tensor tmp = own ? Tensor() : empty({B, n, D}, BF, k);
-      tok.apply(W02b(cnt), W1b(cnt), tokens(q, s), tokens(dO, st.out[i]), n, View(dW02), View(dW1), !fresh,
-                own ? tokens(dq, s) : View(tmp));
+      tok.apply(W02b(cnt), W1b(cnt), tokens(q, s), go, n, View(dW02), View(dW1), !fresh, own ? tokens(dq, s) : View(tmp));
       fresh = false;
       if (!own) {
         for (auto& [a, b] : missing) dq.narrow(1, a, b - a).zero_();

@@ -43,3 +43,45 @@ def test_overlapping_update_and_apply_ranges(order):
         assert torch.isfinite(a).all(), n
         # bf16 operands in the backward's products (2^-9 each, a few of them in a row)
         assert orc.rel_max(a, b) <= 3e-2 and orc.cosine(a, b) >= 0.999, (n, orc.rel_max(a, b))
+
+
+def test_outputs_that_a_later_apply_overwrites():
+    """num_repeat > 1 applies every token range once per repetition and keeps the last result: earlier ones have no gradient."""
+    import lact_b200 as lb
+    from oracle import lact_oracle as orc
+    B, L, D, H = 2, 256, 64, 64
+    i = orc.make_inputs(B, L, D, H, seed=13, act_dtype=BF16)
+    dO = torch.randn(B, L, D, generator=torch.Generator().manual_seed(6)).to(BF16)
+    kw = dict(num_repeat=2, mini_batch_size=64, update_every=64)
+    ref = {n: i[n].float().clone().requires_grad_(True) for n in NAMES}
+    orc.ar_mini_batch(*[ref[n] for n in NAMES], 1.0, **kw)[0].backward(dO.float())
+    got = {n: i[n].cuda().requires_grad_(True) for n in NAMES}
+    o = lb.ar_fast_weight_swish_glu_weight_norm_mini_batch(*[got[n] for n in NAMES], 1.0, **kw)[0]
+    d = dO.cuda()
+    fill_free_memory()
+    o.backward(d)
+    lb.synchronize_and_check()
+    for n in NAMES:
+        a, b = got[n].grad.float().cpu(), ref[n].grad.float()
+        assert orc.rel_max(a, b) <= 3e-2 and orc.cosine(a, b) >= 0.999, (n, orc.rel_max(a, b))
+
+
+def test_outputs_overwritten_in_part():
+    """Against the same program whose applies stop where a later one writes."""
+    import lact_b200 as lb
+    from lact_b200 import ops
+    from lact_b200 import program as P
+    from oracle import lact_oracle as orc
+    i = orc.make_inputs(2, 192, 64, 64, seed=17, act_dtype=BF16)
+    leaves = [i[n].cuda().requires_grad_(True) for n in NAMES]
+    A, U = P.APPLY, P.UPDATE
+    d = torch.randn(2, 192, 64, generator=torch.Generator().manual_seed(8)).to(BF16).cuda()
+    grads = []
+    for steps in ([(A, 0, 192, 0), (U, 0, 64, 0), (A, 40, 100, 60), (U, 64, 150, 0), (A, 100, 150, 100)],
+                  [(A, 0, 60, 0), (A, 150, 192, 150), (U, 0, 64, 0), (A, 40, 80, 60), (U, 64, 150, 0), (A, 100, 150, 100)]):
+        o = ops.scan(*leaves, steps)
+        fill_free_memory()
+        grads.append((o.detach(), *torch.autograd.grad(o, leaves, d)))
+    lb.synchronize_and_check()
+    for a, b in zip(*grads):   # the same values; bf16 products of other shapes, their sums in another order
+        assert orc.rel_max(a.float().cpu(), b.float().cpu()) <= 2e-2
