@@ -291,9 +291,12 @@ int choose_bt(std::initializer_list<NW> probs) {
 // tiles (16 heads of 192: 80 on 148 SMs), and a tile of 49152 tokens is 768 k-blocks of serial work; shorter units fill the
 // SMs and even out the last round.  The rule looks at the length of the sum alone, never at the number of entries: an
 // entry's result is the same bits in any batch.  From 96 k-blocks up three units per tile, from 192 five (both odd, so that
-// tile counts just above half the SMs do not double their rounds): 16 entries of 192 and 768 k-blocks 366 -> 278 us (twelve
-// units: 335, their partial sums cost more than the rounds they even out), 8 entries and 128 k-blocks 70 -> 43 us (four:
-// 52).  Below that nothing is gained: at 32 k-blocks (4 entries of 384) 25 us either way, at 25 (12 of 128 x 256) 19 -> 23.
+// tile counts just above half the SMs do not double their rounds): 16 entries of 192 and 768 k-blocks 315 -> 270 us (twelve
+// units take longer: their partial sums cost more than the rounds they even out), 8 entries of 256 and 192 k-blocks 126 -> 93,
+// 37 of 192 and 128 k-blocks 142 -> 130.  Below 96 nothing is gained: at 32 k-blocks (4 entries of 384) 25 us either way, at
+// 25 (12 of 128 x 256) 19 -> 23.  Where the tiles fill the chip anyway the partial sums cost what they are: nothing at 64
+// entries of 192 (204 us either way), 345 -> 378 at 128 of them, 255 -> 288 at 96 of 128 x 256; entries of 384 gain alone
+// (49 -> 33 at 128 k-blocks) and in fours (60 -> 58), and lose in eights (70 -> 82) and beyond (32: 219 -> 256).
 struct Split {
   int splits, kb_per_split;
 };
@@ -826,8 +829,10 @@ int launch_ns_chip(const NsGroup* grp, int ngroups, const void* const* src, int 
   return LACT_OK;
 }
 
-// Newton-Schulz of one or two groups by the best path: one CTA per matrix where the matrices fit an SM, else the
-// preparation kernels and the dataflow kernel, else one launch per product.  `unscaled`: grp[g].xa holds bf16(G) and
+// Newton-Schulz of one or two groups by the best path: one CTA per matrix where the matrices fit an SM, however many there
+// are, else the preparation kernels and the dataflow kernel, else one launch per product.  (The whole call, one CTA per matrix
+// against preparation and dataflow, us: 64 x 128, 1 / 32 / 192 / 1200 matrices 25 / 27 / 43 / 153 against 86 / 87 / 111 / 260;
+// 128 x 256 39 / 39 / 72 / 299 against 99 / 104 / 135 / 545; 192 x 192 53 / 55 / 104 / 442 against 104 / 119 / 172 / 901.)  `unscaled`: grp[g].xa holds bf16(G) and
 // the normalisation is folded into the first iteration.
 int run_newton_schulz(NsGroup* grp, int ngroups, const void* const* src, int src_f32, const int* parts, int unscaled, int steps,
                       int const_coeffs, int32_t* status, cudaStream_t stream, const bf16** result, const NsKeep* keep = nullptr) {
@@ -1650,7 +1655,7 @@ using namespace lact;
 
 extern "C" {
 
-int lact_version(void) { return 1000; }
+int lact_version(void) { return 1001; }
 
 const char* lact_error_string(int code) {
   switch (code) {
@@ -2232,7 +2237,9 @@ int lact_qkv_prologue_bwd(const void* xq, const void* xk, const void* xv, int64_
   return LACT_OK;
 }
 
-int lact_out_epilogue_bwd_blocks(void) { return sm_count() * 2; }  // what an SM holds of out_rows_bwd_kernel
+// Two blocks per SM: what an SM holds of out_rows_bwd_kernel, and the better number for the general kernel too (2 batches x
+// 8192 tokens x 4 heads of 72 / 320 / 640 / 896: 71 / 118 / 169 / 255 us; with four per SM 75 / 122 / 177 / 263).
+int lact_out_epilogue_bwd_blocks(void) { return sm_count() * 2; }
 
 int lact_out_epilogue_bwd(const void* fw_x, const void* weight, const void* gate_proj, int64_t gate_ld, const void* dout,
                           int64_t dout_ld, void* dx, void* dgate, void* dw_partial, int64_t b, int64_t s, int64_t n_heads,

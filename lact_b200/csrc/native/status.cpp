@@ -1,7 +1,7 @@
 // Device status without copies: every kernel that gives up leaves its code in a word of mapped host memory
 // (lact_status_host_word).  An operator reads that word before it enqueues (one load); a non-zero word is reported as an
-// exception and cleared together with the device-side words.  This replaced a 4-byte device-to-host copy, an event and
-// a memset per call: about 5 us of stream time and 12 us of host time each.
+// exception and cleared together with the device-side words.  (A 4-byte device-to-host copy, an event and a memset per
+// call cost about 5 us of stream time and 12 us of host time.)
 #include <Python.h>
 
 #include <c10/cuda/CUDAGraphsC10Utils.h>

@@ -162,17 +162,8 @@ __device__ __forceinline__ void tma_load_3d(uint32_t smem_dst, const CUtensorMap
       : "memory");
 }
 
-// 4-D tiled load (same completion mechanism); c0 is the innermost coordinate.
-__device__ __forceinline__ void tma_load_4d(uint32_t smem_dst, const CUtensorMap* map, uint64_t* bar, int c0,
-                                            int c1, int c2, int c3) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%3, %4, %5, %6}], [%2];"
-      ::"r"(smem_dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-      : "memory");
-}
-
-// the same two loads issued by the leader lane of a warp-uniform role
+// 3-D and 4-D tiled loads (same completion mechanism; c0 is the innermost coordinate) issued by the leader lane of a
+// warp-uniform role
 __device__ __forceinline__ void tma_load_3d_if(uint32_t leader, uint32_t smem_dst, const CUtensorMap* map, uint64_t* bar, int c0,
                                                int c1, int c2) {
   asm volatile(
@@ -275,23 +266,7 @@ __host__ __device__ __forceinline__ uint32_t make_idesc_bf16(uint32_t m, uint32_
   d |= (m >> 4) << 24;
   return d;
 }
-// D[tmem] (+)= A[smem] * B[smem]; issued by ONE thread.
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                          uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// Arrives on the mbarrier once every previously issued MMA of this thread has completed.
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-               : "memory");
-}
-
-// the same two instructions issued by the leader lane of a warp-uniform role
+// D[tmem] (+)= A[smem] * B[smem], issued by the leader lane of a warp-uniform role.
 __device__ __forceinline__ void umma_bf16_if(uint32_t leader, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                              uint32_t accumulate) {
   asm volatile(
@@ -302,6 +277,7 @@ __device__ __forceinline__ void umma_bf16_if(uint32_t leader, uint32_t tmem_d, u
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(leader)
       : "memory");
 }
+// Arrives on the mbarrier once every MMA the leader lane has issued has completed.
 __device__ __forceinline__ void umma_commit_if(uint32_t leader, uint64_t* bar) {
   asm volatile(
       "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
@@ -316,8 +292,7 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
 }
-// 2^x and 1 / x by the hardware approximations alone, subnormal numbers as zero: without `ftz` every call also scales its
-// argument and its result around the approximation, four to six more instructions
+// 2^x and 1 / x by the hardware approximations alone, subnormal numbers as zero
 __device__ __forceinline__ float exp2_ftz(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
