@@ -95,7 +95,10 @@ typedef struct lact_scan_io {
   void *shadow_dump;
 } lact_scan_io;
 
-/* Library version (major * 1000 + minor).  No counterpart in the reference. */
+/* Library version (major * 1000 + minor).  1001: lact_fw_grad_bwd_pointwise takes entries, tokens and the batch strides of
+ * lr* and g_lr* in place of a row count; lact_momentum_bwd reads dg0 / dg1 and no longer adds the carry to them; lact_scan_io
+ * ends with shadow_dump.  A caller compiled against 1000 that uses one of these must be compiled again.  No counterpart in
+ * the reference. */
 int lact_version(void);
 
 /* Human-readable text for a return code.  No counterpart in the reference. */
