@@ -296,7 +296,8 @@ int choose_bt(std::initializer_list<NW> probs) {
 // 37 of 192 and 128 k-blocks 142 -> 130.  Below 96 nothing is gained: at 32 k-blocks (4 entries of 384) 25 us either way, at
 // 25 (12 of 128 x 256) 19 -> 23.  Where the tiles fill the chip anyway the partial sums cost what they are: nothing at 64
 // entries of 192 (204 us either way), 345 -> 378 at 128 of them, 255 -> 288 at 96 of 128 x 256; entries of 384 gain alone
-// (49 -> 33 at 128 k-blocks) and in fours (60 -> 58), and lose in eights (70 -> 82) and beyond (32: 219 -> 256).
+// (49 -> 33 at 128 k-blocks) and in fours (60 -> 58), and lose in eights (70 -> 82) and beyond (32: 219 -> 256; 64 at 96
+// k-blocks: 365 -> 485).
 struct Split {
   int splits, kb_per_split;
 };

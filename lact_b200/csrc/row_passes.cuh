@@ -1,10 +1,10 @@
 // Row-wise passes of the layer for the usual head sizes: LPR lanes share one (batch, token, head) row of d = 8 * LPR * V
 // features, V 16-byte units per lane (unit u = lane + LPR * i), so no lane idles and a lane has all its loads in flight.
 // Grid (token blocks, heads [x tensors], batch entries): no index divisions, and a block's rows are consecutive tokens.
-// What bounds them is HBM: at d = 384 the former warp-per-row kernels left a quarter of the lanes without a unit and two
-// to eight warps of latency uncovered (2 batches x 8192 tokens x 4 heads: prologue forward 144 us, backward 324 us,
-// epilogue 59 and 111 us, i.e. 20 - 50 % of the measured copy rate).  Head sizes without a (LPR, V) of this table keep the
-// warp-per-row kernels of ops.cuh.
+// What bounds them is HBM and the instructions between the loads: 2 batches x 8192 tokens x 4 heads of 384 take 83 us in the
+// prologue forward (302 MB: 3.6 TB/s) and 125 backward, 40 and 52 in the epilogue.  (A warp per row leaves a quarter of the
+// lanes without a unit at that size and the loads of too few warps in flight: 144, 324, 59 and 111 us.)  Head sizes without a
+// (LPR, V) of this table take the warp-per-row kernels of ops.cuh.
 #pragma once
 #include "swa_bwd.cuh"
 
