@@ -316,6 +316,7 @@ struct OpNsT {
   static constexpr int KB = kb_per_stage(kATileBytes + BT_ * kBK * 2, kStagingTiles);
   static constexpr int STAGES = ring_depth(KB * (kATileBytes + BT_ * kBK * 2), kStagingTiles);
   using Epi = EpiNs;
+  __host__ __device__ static constexpr int diag_a(int) { return 0; }  // S = X X^T, P ~ S S: one matrix on both sides
   __host__ __device__ static constexpr int term_a(int) { return 0; }
   __host__ __device__ static constexpr int term_b(int) { return 0; }
   __host__ __device__ static constexpr int term_col(int) { return 0; }
@@ -354,6 +355,7 @@ struct OpNs2T {
   static constexpr int KB = 1;
   static constexpr int STAGES = ring_depth(2 * (kATileBytes + BT_ * kBK * 2), (SYM_ ? 2 : 1) * kBM * BT_ * 2);
   using Epi = EpiNs;
+  __host__ __device__ static constexpr int diag_a(int b) { return 1 - b; }  // U V^T + V U^T: a0 = b1 = U, a1 = b0 = V
   __host__ __device__ static constexpr int term_a(int t) { return t; }
   __host__ __device__ static constexpr int term_b(int t) { return t; }
   __host__ __device__ static constexpr int term_col(int) { return 0; }

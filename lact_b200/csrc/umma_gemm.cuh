@@ -122,6 +122,10 @@ struct TileCoord {
 // Ops whose output is a symmetric M x M matrix (both operands the same rows) may declare `kSymmetric`: only the
 // 128 x 128 tiles on and above the diagonal are computed, and every off-diagonal tile is stored twice, as it is and
 // transposed (from a second staging tile the epilogue fills).  Needs BT = 128, one staged output, dataflow mode.
+// On the diagonal the B tiles are the very rows of the A tiles, read the same way: they are not loaded a second time, the
+// products read A tile `diag_a(b)` in place of B tile b.  What these kernels share as a limit is the rate at which operands
+// come out of L2 (8 to 10 TB/s over the chip, profiles of all GEMM classes alike), and at three row blocks half of the
+// computed tiles lie on the diagonal: a quarter of the operand bytes of these phases.
 template <class Op, class = void>
 struct op_symmetric { static constexpr bool value = false; };
 template <class Op>
@@ -340,16 +344,18 @@ __device__ __forceinline__ bool gemm_phase(GemmCtx& cx, const GemmProblem<Op>* p
           asm volatile("fence.proxy.async;" ::: "memory");
         }
         const int num_sb = (kb1 - kb0 + KB - 1) / KB;  // ring stages of KB k-blocks
+        const bool diagonal = SYM && tc.m0 == tc.n0;
         for (int sb = 0; sb < num_sb; ++sb, ++cx.it) {
           const int s = cx.it % RING;
           const uint32_t ph = (cx.it / RING) & 1;
           if (!mbar_wait_warp(&cx.empty_bar[s], ph ^ 1, cx.abort_flag)) { failed = true; break; }
-          mbar_expect_tx_if(leader, &cx.full_bar[s], kStageBytes);
+          mbar_expect_tx_if(leader, &cx.full_bar[s], diagonal ? KB * NA * kATileBytes : kStageBytes);
           const uint32_t st = cx.smem_base + s * cx.stage_stride;
           const int kc = (kb0 + sb * KB) * kBK;
 #pragma unroll
           for (int i = 0; i < NA; ++i)
             load_operand_tile<kBM, KB>(leader, st + i * (KB * kATileBytes), &P.a[i], P.ai[i], tc.m0, kc, tc.batch, &cx.full_bar[s]);
+          if (diagonal) continue;
 #pragma unroll
           for (int i = 0; i < NB; ++i)
             load_operand_tile<BT, KB>(leader, st + NA * (KB * kATileBytes) + i * (KB * kBTileBytes), &P.b[i], P.bi[i], tc.n0, kc,
@@ -374,6 +380,7 @@ __device__ __forceinline__ bool gemm_phase(GemmCtx& cx, const GemmProblem<Op>* p
         tc_fence_after();
         const uint32_t acc_base = cx.tmem_base + as * kAccStride;
         const int num_sb = (num_kb + KB - 1) / KB;
+        const bool diagonal = SYM && tc.m0 == tc.n0;
         // K-major tiles: 16 elements = 32 bytes on inside the swizzled 128-byte row, k-blocks a tile apart; MN-major tiles:
         // 16 k-rows of 128 bytes on, k-blocks 64 rows apart, 64-wide atoms KB * 8 KB apart (the leading offset)
         uint32_t idesc[Op::NTERMS], step_a[Op::NTERMS], step_b[Op::NTERMS], blk_a[Op::NTERMS], blk_b[Op::NTERMS];
@@ -399,7 +406,11 @@ __device__ __forceinline__ bool gemm_phase(GemmCtx& cx, const GemmProblem<Op>* p
 #pragma unroll
             for (int t = 0; t < Op::NTERMS; ++t) {
               const uint32_t a_tile = st + Op::term_a(t) * (KB * kATileBytes >> 4) + kk * blk_a[t];
-              const uint32_t b_tile = st + (NA * (KB * kATileBytes) + Op::term_b(t) * (KB * kBTileBytes) >> 4) + kk * blk_b[t];
+              uint32_t b_off = NA * (KB * kATileBytes) + Op::term_b(t) * (KB * kBTileBytes);
+              if constexpr (SYM) {
+                if (diagonal) b_off = Op::diag_a(Op::term_b(t)) * (KB * kATileBytes);
+              }
+              const uint32_t b_tile = st + (b_off >> 4) + kk * blk_b[t];
 #pragma unroll
               for (int k4 = 0; k4 < kBK / kUmmaK; ++k4) {
                 const uint32_t acc = (sb > 0 || kk > 0 || k4 > 0 || !Op::term_first(t)) ? 1u : 0u;
