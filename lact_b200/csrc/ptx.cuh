@@ -41,12 +41,15 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
                : "memory");
 }
-__device__ __forceinline__ void mbar_expect_tx_if(uint32_t leader, uint64_t* bar, uint32_t bytes) {
+__device__ __forceinline__ void mbar_expect_tx_if(uint32_t leader, uint32_t bar, uint32_t bytes) {
   asm volatile(
       "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t"
-      "@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(smem_u32(bar)),
+      "@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(bar),
       "r"(bytes), "r"(leader)
       : "memory");
+}
+__device__ __forceinline__ void mbar_expect_tx_if(uint32_t leader, uint64_t* bar, uint32_t bytes) {
+  mbar_expect_tx_if(leader, smem_u32(bar), bytes);
 }
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -164,23 +167,27 @@ __device__ __forceinline__ void tma_load_3d(uint32_t smem_dst, const CUtensorMap
 
 // 3-D and 4-D tiled loads (same completion mechanism; c0 is the innermost coordinate) issued by the leader lane of a
 // warp-uniform role
-__device__ __forceinline__ void tma_load_3d_if(uint32_t leader, uint32_t smem_dst, const CUtensorMap* map, uint64_t* bar, int c0,
+__device__ __forceinline__ void tma_load_3d_if(uint32_t leader, uint32_t smem_dst, const CUtensorMap* map, uint32_t bar, int c0,
                                                int c1, int c2) {
   asm volatile(
       "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %6, 0;\n\t"
       "@q cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
       " [%0], [%1, {%3, %4, %5}], [%2];\n\t}"
-      ::"r"(smem_dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(leader)
+      ::"r"(smem_dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(leader)
       : "memory");
 }
-__device__ __forceinline__ void tma_load_4d_if(uint32_t leader, uint32_t smem_dst, const CUtensorMap* map, uint64_t* bar, int c0,
+__device__ __forceinline__ void tma_load_4d_if(uint32_t leader, uint32_t smem_dst, const CUtensorMap* map, uint32_t bar, int c0,
                                                int c1, int c2, int c3) {
   asm volatile(
       "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %7, 0;\n\t"
       "@q cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
       " [%0], [%1, {%3, %4, %5, %6}], [%2];\n\t}"
-      ::"r"(smem_dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(leader)
+      ::"r"(smem_dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(leader)
       : "memory");
+}
+__device__ __forceinline__ void tma_load_4d_if(uint32_t leader, uint32_t smem_dst, const CUtensorMap* map, uint64_t* bar, int c0,
+                                               int c1, int c2, int c3) {
+  tma_load_4d_if(leader, smem_dst, map, smem_u32(bar), c0, c1, c2, c3);
 }
 
 // 3-D tiled store shared -> global (bulk async-group completion).  Elements outside the tensor's
