@@ -17,6 +17,7 @@
 #include "f32_gemm.cuh"
 #include "ns_bwd_fused.cuh"
 #include "ns_chip.cuh"
+#include "pair_gemm.cuh"
 #include "row_passes.cuh"
 #include "swa_bwd.cuh"
 
@@ -46,8 +47,9 @@ struct Mat {
   int64_t rows, cols, ld, batch, bs;  // ld / bs: row / batch stride in elements
 };
 
-// Encodes a 3-D map (cols, rows, batch) with a {64, box_rows, 1} box and 128-byte swizzle.
-int encode_map(CUtensorMap* map, const Mat& m, uint32_t box_rows) {
+// Encodes a 3-D map (cols, rows, batch) with a {64, box_rows, 1} box and 128-byte swizzle, or a {32, box_rows, 1} box and
+// 64-byte swizzle.
+int encode_map(CUtensorMap* map, const Mat& m, uint32_t box_rows, uint32_t box_cols = 64) {
   EncodeFn fn = get_encode_fn();
   if (fn == nullptr) return LACT_ERR_CUDA;
   if ((reinterpret_cast<uintptr_t>(m.ptr) & 15) != 0 || (m.ld % 8) != 0 || (m.batch > 1 && (m.bs % 8) != 0))
@@ -57,11 +59,11 @@ int encode_map(CUtensorMap* map, const Mat& m, uint32_t box_rows) {
                         static_cast<cuuint64_t>(m.batch)};
   const int64_t bs = m.batch > 1 ? m.bs : m.ld * m.rows;
   cuuint64_t strides[2] = {static_cast<cuuint64_t>(m.ld) * 2, static_cast<cuuint64_t>(bs) * 2};
-  cuuint32_t box[3] = {64, box_rows, 1};
+  cuuint32_t box[3] = {box_cols, box_rows, 1};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(m.ptr), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, box_cols == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? LACT_OK : LACT_ERR_CUDA;
 }
 
@@ -240,6 +242,8 @@ int sm_count() {
   return cached[dev];
 }
 
+inline int ceil_div(int64_t a, int64_t b) { return static_cast<int>((a + b - 1) / b); }
+
 // Launches the first `nprob` problems of `args` as one persistent grid (one CTA per SM at most).
 template <class Op, int NPROB>
 int launch_gemm(const GemmArgs<Op, NPROB>& args, cudaStream_t stream, int cls, int nprob = NPROB) {
@@ -270,7 +274,66 @@ int launch_gemm(const GemmArgs<Op, NPROB>& args, cudaStream_t stream, int cls, i
   return LACT_OK;
 }
 
-inline int ceil_div(int64_t a, int64_t b) { return static_cast<int>((a + b - 1) / b); }
+// Whether a product of `batch` x `M` tokens with N columns in tiles of `bt` goes to pairs of SMs (pair_gemm.cuh).  It does where
+// a pair keeps its weights for at least six tiles of 256 tokens: a launch of clusters costs about 2 us more than a plain one, and
+// with fewer tiles the halves of the last one stand idle.  Measured, us per launch, pairs against single SMs: 1.3 tiles per pair
+// (4 entries of 384, 2048 tokens) gate 16.2 / 14.7, down 12.7 / 10.7, pointwise 21.8 / 21.0; 2.3 to 4.7 (12 entries of 128 x 256,
+// 1560 tokens) 16.8 / 16.6, 12.7 / 10.7, 20.9 / 20.9; 7 to 10.7 (32 of 384, 2048) 43 / 48, 28.8 / 31.5, 96 / 99; 128 (16 of 192,
+// 49152) pointwise 314 / 347.
+inline int64_t pair_tiles(int64_t batch, int64_t M) { return ceil_div(M, kPairRows) * batch; }
+inline bool pair_pays(int64_t tiles, int64_t N, int bt, int64_t K) {
+  const int64_t tn = ceil_div(N, bt);
+  return K <= kPairMaxKb * kBK && tiles * tn >= 6 * (sm_count() / 2) && tn <= sm_count() / 2;
+}
+
+// The same launch on pairs of SMs with the weights kept in shared memory; all problems have the same K and N.
+template <class Op, int NPROB>
+int launch_pair(const GemmArgs<Op, NPROB>& args, cudaStream_t stream, int cls, int nprob = NPROB) {
+  auto kernel = pair_gemm_kernel<Op, NPROB>;
+  static std::mutex mu;
+  static bool configured[64] = {false};
+  int dev = 0;
+  LACT_CUDA(cudaGetDevice(&dev));
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    if (dev >= 64 || !configured[dev]) {
+      LACT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448));
+      if (dev < 64) configured[dev] = true;
+    }
+  }
+  int64_t tiles = 0;
+  for (int p = 0; p < nprob; ++p) {
+    const auto& P = args.prob[p];
+    if (P.M < 1 || P.N < 1 || P.batch < 1 || P.K < 1 || P.K != args.prob[0].K || P.N != args.prob[0].N) return LACT_ERR_SHAPE;
+    tiles += pair_tiles(P.batch, P.M);
+  }
+  const int tn = ceil_div(args.prob[0].N, Op::BT), teams = static_cast<int>(std::min<int64_t>(tiles, sm_count() / 2 / tn));
+  if (tiles > (1ll << 30) || teams < 1) return LACT_ERR_SHAPE;
+  const int num_kb = ceil_div(args.prob[0].K, kBK), ring = pair_ring<Op>(num_kb);
+  if (num_kb > kPairMaxKb || ring < 2) return LACT_ERR_CONFIG;
+  const size_t smem = 1024 + kPairBars + pair_panels<Op>() * kPairPanel + pair_b_bytes<Op>(num_kb) + ring * pair_stage_bytes<Op>();
+  KernelScope scope(cls, stream);
+  LACT_CUDA(launch_pdl(kernel, dim3(2 * teams * tn), dim3(kGemmThreadsV2), smem, stream, args, nprob, ring));
+  return LACT_OK;
+}
+// c = a b^T of every problem in bf16 tiles `bt` wide; `fill` as for launch_op, with B boxes of half a tile.
+template <int NPROB, class Fill>
+int launch_pair_store(int bt, Fill&& fill, cudaStream_t stream, int cls, int nprob) {
+#define LACT_PAIR_CASE(BTV)                                  \
+  case BTV: {                                                \
+    GemmArgs<OpBmmStore<BTV>, NPROB> g;                      \
+    std::memset(&g, 0, sizeof(g));                           \
+    LACT_TRY(fill(g, BTV / 2));                              \
+    return launch_pair(g, stream, cls, nprob);               \
+  }
+  switch (bt) {
+    LACT_PAIR_CASE(128)
+    LACT_PAIR_CASE(192)
+    LACT_PAIR_CASE(256)
+    default: return LACT_ERR_CONFIG;
+  }
+#undef LACT_PAIR_CASE
+}
 
 // Output-tile width for a single-accumulator GEMM: the candidate with the least padded work over
 // the problems of the launch (ties go to the wider tile, whose MMA shape is more efficient).
@@ -373,6 +436,7 @@ int launch_gate(const ApplyArgs& a, const Mat& x, const Mat& w02, int64_t len, i
   P.M = static_cast<int>(len); P.N = static_cast<int>(a.H); P.K = static_cast<int>(a.D);
   P.batch = static_cast<int>(a.B);
   g.status = status;
+  if (pair_pays(pair_tiles(a.B, len), a.H, BT, a.D)) return launch_pair(g, stream, kClsGate);
   return launch_gemm(g, stream, kClsGate);
 }
 
@@ -398,6 +462,7 @@ int run_apply(const ApplyArgs& a, int32_t* status, cudaStream_t stream) {
     g.status = status;
     return LACT_OK;
   };
+  if (bt >= 128 && pair_pays(pair_tiles(a.B, len), a.D, bt, a.H)) return launch_pair_store<1>(bt, fill, stream, kClsDown, 1);
   return launch_op<OpBmmStore, 1>(bt, fill, stream, kClsDown, 1);
 }
 
@@ -463,6 +528,10 @@ int run_grad_pointwise(const GradArgs& a, int32_t* status, cudaStream_t stream) 
   LACT_TRY(make_output(&P.out[1], &P.oi[1], dy2m, 0, 0));
   LACT_TRY(make_output(&P.out[2], &P.oi[2], hid, 0, 0));
   g.status = status;
+  if (pair_pays(pair_tiles(a.B, len), a.H, BT, a.D)) {
+    LACT_TRY(encode_map(&P.b[2], w1, 64, 32));  // a CTA's half of these columns: atoms of 32
+    return launch_pair(g, stream, kClsGradPointwise);
+  }
   return launch_gemm(g, stream, kClsGradPointwise);
 }
 

@@ -425,25 +425,33 @@ struct OpFwGradPointwise {
   __host__ __device__ static constexpr int term_col(int t) { return t == 0 ? 0 : 128; }
   __host__ __device__ static constexpr int term_n(int t) { return t == 0 ? 128 : 64; }
   __host__ __device__ static constexpr bool term_first(int) { return true; }
+  // The learning rates of a row as they are stored (fp32 or bf16 bits): nothing waits for the loads before the epilogue uses
+  // the values, a tile later.
+  static constexpr bool kFetchAhead = true;
   struct Prefetch {
-    float l0, l1, l2;
+    uint32_t r[3];
   };
   __device__ static __forceinline__ void prefetch(const Epi& ep, int batch, int row, int, int, int M, int,
                                                   Prefetch& pf) {
-    pf.l0 = pf.l1 = pf.l2 = 0.f;
-    if (row < M) {
-      const int64_t li = batch * ep.lr_bs + ep.tok_off + row;
+    const void* const lr[3] = {ep.lr0, ep.lr1, ep.lr2};
+    const int64_t li = batch * ep.lr_bs + ep.tok_off + row;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
       // (a null learning rate stands for 1: the backward of apply is this same pointwise stage on (q, dO))
-      pf.l0 = (ep.lr0 ? load_scalar(ep.lr0, ep.lr_f32, li) : 1.f) * ep.w_scale;
-      pf.l1 = (ep.lr1 ? load_scalar(ep.lr1, ep.lr_f32, li) : 1.f) * ep.w_scale;
-      pf.l2 = (ep.lr2 ? load_scalar(ep.lr2, ep.lr_f32, li) : 1.f) * ep.w_scale;
+      pf.r[i] = ep.lr_f32 ? 0x3F800000u : 0x3F80u;
+      if (row >= M) pf.r[i] = 0;
+      else if (lr[i] != nullptr)
+        pf.r[i] = ep.lr_f32 ? reinterpret_cast<const uint32_t*>(lr[i])[li] : reinterpret_cast<const uint16_t*>(lr[i])[li];
     }
   }
+  __device__ static __forceinline__ float rate(const Epi& ep, uint32_t r) {
+    return __uint_as_float(ep.lr_f32 ? r : r << 16) * ep.w_scale;
+  }
   __device__ static __forceinline__ bool skip_store(const Epi&, int) { return false; }
-  __device__ static __forceinline__ void epilogue_staged(const Epi&, int, int, int, int, int,
+  __device__ static __forceinline__ void epilogue_staged(const Epi& ep, int, int, int, int, int,
                                                          const float (&v)[3][32], float (&o)[3][32],
                                                          Prefetch& pf) {
-    const float l0 = pf.l0, l1 = pf.l1, l2 = pf.l2;
+    const float l0 = rate(ep, pf.r[0]), l1 = rate(ep, pf.r[1]), l2 = rate(ep, pf.r[2]);
 #pragma unroll
     for (int j = 0; j < 32; ++j) {
       const float y0 = v[0][j], y2 = v[1][j], dh = v[2][j];

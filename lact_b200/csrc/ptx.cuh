@@ -201,7 +201,9 @@ __device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, uint32_t sm
 __device__ __forceinline__ void bulk_commit_group() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // waits until the sources of all committed bulk groups have been read (shared memory reusable)
 __device__ __forceinline__ void bulk_wait_read_all() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-// all but the most recently committed group have finished reading shared memory
+// all but the N most recently committed groups have finished reading shared memory
+template <int N>
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
 // waits until all committed bulk groups have completed (global writes performed)
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 // named barrier among `count` threads (barrier 0 is __syncthreads)
@@ -254,6 +256,12 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr, uint32_t lbo_
 // The descriptors of one operand's tiles: they differ in the start address alone (16-byte units, low word).
 struct SmemDescBase {
   uint32_t lo, hi;
+  // 64-byte swizzle: an MN-major operand one 32-element atom wide (rows of 64 bytes, 8-k-row groups 512 bytes apart)
+  __device__ static __forceinline__ SmemDescBase half_atom() {
+    SmemDescBase d(0);
+    d.hi = (512u >> 4) | (1u << 14) | (4u << 29);
+    return d;
+  }
   __device__ __forceinline__ explicit SmemDescBase(uint32_t lbo_bytes)
       : lo(((lbo_bytes >> 4) & 0x3FFFu) << 16), hi(((1024u >> 4) & 0x3FFFu) | (1u << 14) | (2u << 29)) {}
   __device__ __forceinline__ uint64_t at(uint32_t saddr16) const {
@@ -290,6 +298,65 @@ __device__ __forceinline__ void umma_commit_if(uint32_t leader, uint64_t* bar) {
       "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
       "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)),
       "r"(leader)
+      : "memory");
+}
+
+// ---------------------------------------------------------------- pairs of SMs (clusters of two CTAs, cta_group::2)
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// Barrier among all threads of the cluster (every thread reaches it: it has no time limit).
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Address, in the cluster's shared window, of the leader's (rank 0) copy of a shared-memory object.
+__device__ __forceinline__ uint32_t leader_address(const void* p) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(smem_u32(p)));
+  return a;
+}
+__device__ __forceinline__ void mbar_arrive_leader(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(leader_address(bar)) : "memory");
+}
+// As tma_load_3d_if, into this CTA's shared memory; `bar` (a cluster address) may be the peer's.
+__device__ __forceinline__ void tma_load_3d_pair_if(uint32_t leader, uint32_t smem_dst, const CUtensorMap* map, uint32_t bar, int c0,
+                                                    int c1, int c2) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %6, 0;\n\t"
+      "@q cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2"
+      " [%0], [%1, {%3, %4, %5}], [%2];\n\t}"
+      ::"r"(smem_dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(leader)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_result, uint32_t ncols) {
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_result)), "r"(ncols)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_relinquish_pair() {
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+// Product of the pair: A is 128 rows in each CTA's shared memory, B half of its rows in each; results stay with the rows of A.
+__device__ __forceinline__ void umma_bf16_pair_if(uint32_t leader, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                                  uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(leader)
+      : "memory");
+}
+// Arrives on both CTAs' copies of the barrier once every product the leader lane has issued has completed.
+__device__ __forceinline__ void umma_commit_pair_if(uint32_t leader, uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %2;\n\t}" ::"r"(smem_u32(bar)),
+      "r"(leader), "h"(static_cast<uint16_t>(3))
       : "memory");
 }
 

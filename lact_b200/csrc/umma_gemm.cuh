@@ -164,6 +164,14 @@ struct op_split { static constexpr bool value = false; };
 template <class Op>
 struct op_split<Op, decltype(void(Op::kSplitK))> { static constexpr bool value = Op::kSplitK; };
 
+// Ops whose epilogue reads per-row values from global memory may declare `kFetchAhead`: `prefetch` then only issues the loads
+// and is called a tile ahead.  Where the epilogue sets the pace (the pointwise stage at 192 features, 4570 clocks a tile) 2000
+// of them went on waiting for the learning rates of the tile in hand.
+template <class Op, class = void>
+struct op_fetch_ahead { static constexpr bool value = false; };
+template <class Op>
+struct op_fetch_ahead<Op, decltype(void(Op::kFetchAhead))> { static constexpr bool value = Op::kFetchAhead; };
+
 // Per-thread view of the CTA's pipeline resources and of this thread's progress counters.  The
 // producer thread advances the ring stage, the MMA thread stage and `tcount`, epilogue threads `tcount`;
 // all three walk the same tile sequence, so their private copies stay consistent.  The counters
@@ -532,6 +540,14 @@ __device__ __forceinline__ bool gemm_phase(GemmCtx& cx, const GemmProblem<Op>* p
       const int t = tile_at(r);
       return t < total_tiles ? t : -1;
     };
+    [[maybe_unused]] typename Op::Prefetch pf_next;
+    [[maybe_unused]] auto fetch = [&](int tile) {
+      if (tile < 0) return;
+      const TileCoord tc = coord(tile);
+      const GemmProblem<Op>& P = probs[tc.prob];
+      Op::prefetch(P.ep, tc.batch, tc.m0 + row_local, tc.n0, half, P.M, P.N, pf_next);
+    };
+    if constexpr (op_fetch_ahead<Op>::value) fetch(tile_of_round(0));
     for (int tile_i = 0; tile_i < rounds; ++tile_i) {
       const int tile = tile_of_round(tile_i);
       if (tile < 0) continue;
@@ -542,9 +558,14 @@ __device__ __forceinline__ bool gemm_phase(GemmCtx& cx, const GemmProblem<Op>* p
       const uint32_t stg = cx.staging;
       const uint32_t as = cx.tcount & 1, aph = (cx.tcount >> 1) & 1;
       const int row = tc.m0 + row_local;
-      // global operands of the epilogue are fetched while the tile's MMAs are still running
+      // global operands of the epilogue are fetched while the tile's MMAs are still running, or a tile ahead
       typename Op::Prefetch pf;
-      Op::prefetch(ep, tc.batch, row, tc.n0, half, P.M, P.N, pf);
+      if constexpr (op_fetch_ahead<Op>::value) {
+        pf = pf_next;
+        fetch(tile_of_round(tile_i + 1));
+      } else {
+        Op::prefetch(ep, tc.batch, row, tc.n0, half, P.M, P.N, pf);
+      }
       bool got = mbar_wait(&cx.acc_full_bar[as], aph, cx.abort_flag);
       tc_fence_after();
       const uint32_t acc_base = cx.tmem_base + as * kAccStride + (static_cast<uint32_t>(quarter * 32) << 16);

@@ -1,0 +1,70 @@
+"""Token x weight products on pairs of SMs: the same bits as the one-SM kernel gives entry by entry, and the fp32 reference."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+
+# (entries, d, h, tokens): enough tiles of 256 tokens for the pairs in the batch and too few in a single entry.  Token counts at
+# the edges of a tile and of either CTA's half of it, heads whose columns end inside a tile or whose k ends inside a k-block, the
+# longest k that is kept in shared memory, two batch entries per pair and several
+CASES = [(12, 384, 384, 3329), (40, 384, 384, 1025), (48, 192, 192, 1024), (90, 192, 192, 1409), (30, 256, 256, 2048 + 127),
+         (64, 128, 256, 1560), (40, 512, 512, 1281), (60, 144, 80, 2560), (100, 64, 64, 1300), (36, 320, 208, 1152 + 255)]
+
+
+def _inputs(b, d, h, n, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    rn = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    w02, w1 = (rn(b, 2 * h, d) / d ** 0.5).bfloat16(), (rn(b, d, h) / h ** 0.5).bfloat16()
+    kv = rn(b, n, 3 * d).bfloat16()   # k and v are views of a fused projection
+    return w02, w1, kv[..., :d], kv[..., d:2 * d], [F.softplus(rn(b, n) - 2) for _ in range(3)]
+
+
+def _close(got, want):
+    # one rounding to bf16 (2^-9 relative) of fp32 sums, and of the hidden plane before the down projection
+    assert float((got.double() - want).norm() / want.norm()) < 2.0 ** -7
+
+
+@pytest.mark.parametrize("b,d,h,n", CASES)
+def test_apply(b, d, h, n):
+    import lact_b200 as lb
+    w02, w1, k, _, _ = _inputs(b, d, h, n, n)
+    x = k.contiguous()
+    out = lb.fused_swiglu_ffn_fwd(w02, w1, x)
+    for i in range(0, b, max(1, b // 4)):
+        assert torch.equal(out[i], lb.fused_swiglu_ffn_fwd(w02[i:i + 1], w1[i:i + 1], x[i:i + 1])[0])
+    y = x[-1].double() @ w02[-1].double().T
+    _close(out[-1], (F.silu(y[:, :h]) * y[:, h:]) @ w1[-1].double().T)
+    lb.synchronize_and_check()
+
+
+@pytest.mark.parametrize("b,d,h,n", CASES)
+@pytest.mark.parametrize("lr_dtype", [torch.float32, torch.bfloat16, None])
+def test_pointwise(b, d, h, n, lr_dtype):
+    from lact_b200 import _lib as L
+    w02, w1, k, v, lr = _inputs(b, d, h, n, n + 1)
+    lr = [None] * 3 if lr_dtype is None else [t.to(lr_dtype) for t in lr]
+    status = torch.zeros(64, dtype=torch.int32, device="cuda")
+
+    def run(s):
+        m = w02[s].shape[0]
+        guard = torch.full((m * n * 3 * h + 2 * h,), -7.0, dtype=torch.bfloat16, device="cuda")
+        dy, hid = guard[:m * n * 2 * h].view(m, n, 2 * h), guard[m * n * 2 * h:m * n * 3 * h].view(m, n, h)
+        ptr = [t[s].data_ptr() if t is not None else None for t in lr]
+        L.check(L.lib().lact_fw_grad_pointwise(w02[s].data_ptr(), w1[s].data_ptr(), k[s].data_ptr(), 3 * d, 3 * d * n, v[s].data_ptr(),
+                                               3 * d, 3 * d * n, *ptr, 1 if lr_dtype == torch.bfloat16 else 0, n, 0.5, dy.data_ptr(),
+                                               hid.data_ptr(), m, n, d, h, status.data_ptr(), L.stream_ptr()), "pointwise")
+        assert bool((guard[m * n * 3 * h:] == -7).all())   # nothing is written behind the planes
+        return dy, hid
+
+    dy, hid = run(slice(0, b))
+    for i in range(0, b, max(1, b // 4)):
+        for got, want in zip((dy, hid), run(slice(i, i + 1))):
+            assert torch.equal(got[i], want[0])
+    kd, vd, l = k[-1].double(), v[-1].double(), [1.0 if t is None else t[-1].double()[:, None] for t in lr]
+    y, dh = kd @ w02[-1].double().T, vd @ w1[-1].double()
+    y0, y2, sg = y[:, :h], y[:, h:], torch.sigmoid(y[:, :h])
+    _close(dy[-1][:, :h], 0.5 * l[0] * dh * y2 * sg * (1 + y0 * (1 - sg)))
+    _close(dy[-1][:, h:], 0.5 * l[2] * dh * y0 * sg)
+    _close(hid[-1], 0.5 * l[1] * y0 * sg * y2)
+    assert int(status[0]) == 0
