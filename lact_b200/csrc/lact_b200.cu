@@ -1161,7 +1161,7 @@ int launch_swa_bwd(const SwaBwdArgs& a, int64_t ctas, cudaStream_t stream) {
     }
   }
   KernelScope scope(kClsOther, stream);
-  kernel<<<static_cast<unsigned>(ctas), 320, smem, stream>>>(a);
+  kernel<<<static_cast<unsigned>(ctas), kSwaBwdThreads, smem, stream>>>(a);
   LACT_CUDA(cudaGetLastError());
   return LACT_OK;
 }
@@ -2621,10 +2621,6 @@ int lact_swa_bwd(const void* q, const void* k, const void* v, const void* o, con
   LACT_TRY(encode_map_heads(&a.k, k, b, lk, n_heads, d, k_ts, k_bs));
   LACT_TRY(encode_map_heads(&a.v, v, b, lk, n_heads, d, v_ts, v_bs));
   LACT_TRY(encode_map_heads(&a.dout, dout, b, l, n_heads, d, do_ts, do_bs));
-  LACT_TRY(encode_map_heads(&a.q64, q, b, l, n_heads, d, q_ts, q_bs, 64));
-  LACT_TRY(encode_map_heads(&a.k64, k, b, lk, n_heads, d, k_ts, k_bs, 64));
-  LACT_TRY(encode_map_heads(&a.v64, v, b, lk, n_heads, d, v_ts, v_bs, 64));
-  LACT_TRY(encode_map_heads(&a.dout64, dout, b, l, n_heads, d, do_ts, do_bs, 64));
   a.lse = static_cast<const float*>(lse);
   a.delta = static_cast<const float*>(delta);
   a.seq_start = seq_start;

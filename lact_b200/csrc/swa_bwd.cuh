@@ -2,28 +2,28 @@
 // visible to every query) for sm_100a.  With P = softmax(q k^T * scale) restricted to the visible keys, recomputed from
 // the forward's log-sum-exp L, and Delta_i = sum_d dO_i O_i:
 //   dV_j = sum_i P_ij dO_i,   dS_ij = P_ij (dO_i . v_j - Delta_i) * scale,   dK_j = sum_i dS_ij q_i,   dQ_i = sum_j dS_ij k_j.
-// One kernel, two modes (a CTA owns a 128-row OUTER tile and walks 64-row INNER tiles of its band):
+// One kernel, two modes (a CTA owns a 128-row OUTER tile and walks the 128-row INNER tiles of its band):
 //   MODE 0  outer = key tile j, inner = query tiles i:  dV_j += P^T dO_i,  dK_j += dS^T Q_i   (two accumulators)
 //   MODE 1  outer = query tile i, inner = key tiles j:  dQ_i += dS K_j                        (one accumulator)
 // The OUTER rows are the tensor-memory lanes in both modes: per inner tile the first products are
-// [128 outer x 64 inner] (mode 0: S^T = K Q^T and dP^T = V dO^T; mode 1: S = Q K^T and dP = dO V^T), two softmax
-// threads per lane (32 columns each) turn them into bf16 tiles [128 outer][64 inner] in shared memory (one 128-byte
-// swizzled row per lane: the K-major A operand of the second products), and the inner tiles, [64 rows][64 columns] TMA
-// boxes, serve as K-major B operands of the first products and as MN-major B operands (rows = k) of the second.
-// Pipeline over the inner tiles: the inner tiles go through a three-stage ring (a stage is held from its load to the end
-// of its second products, so two stages would put the load latency on the critical path), S / dP columns and the
-// P / dS tiles are double-buffered; the issuing thread queues the first products of tile t + 1 BEFORE the second
-// products of tile t, so the tensor pipe works on one tile while the softmax threads work on the other.  Every
-// mbarrier wait is bounded; the one named barrier (mode 0, per-query values staged a tile ahead) is reached by every
-// softmax thread in every iteration, whatever its waits returned.
+// [128 outer x 128 inner] (mode 0: S^T = K Q^T and dP^T = V dO^T; mode 1: S = Q K^T and dP = dO V^T), four softmax
+// threads per lane (32 columns each) turn them into bf16 P and dS, which go back to tensor memory, into the columns the
+// thread has just read, and are the A operands of the second products from there (the shared memory that tiles of them
+// would take holds a third inner stage, and the second products read half as many operand bytes).  The inner tiles
+// serve as K-major B operands of the first products and as MN-major B operands (rows = k) of the second.
+// Order of the products, all issued by one thread and executed in that order:
+//   mode 0  ... dV(t), S(t + 1), dK(t), dP(t + 1) ...   P(t + 1) is worked out while dK(t), dP(t + 1) run, dS(t) during dV(t),
+//                                                       S(t + 1); S and dP have one set of columns each
+//   mode 1  ... dP(t + 1), dQ(t), S(t + 2) ...          S has two sets of columns, dP one
+// The first inner operand (Q or K) is held from its first product to the second products a tile later and goes through a
+// three-stage ring, the other through two stages.  Every mbarrier wait is bounded.
 #pragma once
 #include "swa.cuh"
 
 namespace lact {
 
 struct SwaBwdArgs {
-  CUtensorMap q, k, v, dout;           // 4-D maps (feature, token, head, batch), box {64, 128, 1, 1}: outer tiles
-  CUtensorMap q64, k64, v64, dout64;   // the same tensors with box {64, 64, 1, 1}: inner tiles
+  CUtensorMap q, k, v, dout;           // 4-D maps (feature, token, head, batch), box {64, 128, 1, 1}
   const float* lse;            // [b][h][l]: log2-domain log-sum-exp of the forward (m + log2(l))
   const float* delta;          // [b][h][l]: sum_d dO O
   const int32_t* seq_start;    // optional [l], as in the forward
@@ -36,53 +36,54 @@ struct SwaBwdArgs {
   int32_t* status;
 };
 
+// softmax warps: four per tensor-memory lane quarter, 32 columns of a tile each
+constexpr int kSwaBwdWarps = 16, kSwaBwdThreads = 64 + 32 * kSwaBwdWarps + 32;  // + loads, products, per-query values
+
 template <int HD>
 struct SwaBwdSmem {
-  static constexpr uint32_t kOTile = 128 * HD * 2;   // outer tile
-  static constexpr uint32_t kITile = 64 * HD * 2;    // inner tile
-  static constexpr uint32_t kWTile = 128 * 64 * 2;   // P or dS tile written by the softmax threads
-  static constexpr int kInnerStages = 3;
-  // outer pair | 3 stages x inner pair | 2 stages x (P, dS) | 2 stages x 3 x 64 per-query words (mode 0) | barriers
-  static constexpr uint32_t kOuter = 0, kInner = 2 * kOTile, kW = kInner + kInnerStages * 2 * kITile,
-                            kStats = kW + 4 * kWTile, kBars = kStats + 2 * 3 * 64 * 4;
-  static constexpr uint32_t kBytes = kBars + 256 + 1024;
+  static constexpr uint32_t kTile = 128 * HD * 2;
+  static constexpr int kStagesA = 3, kStagesB = 2;
+  // outer pair | first inner operand x 3 | second inner operand x 2 | 2 stages x (lse, delta) of 128 queries (mode 0) | barriers
+  static constexpr uint32_t kOuter = 0, kA = 2 * kTile, kB = kA + kStagesA * kTile, kStats = kB + kStagesB * kTile,
+                            kBars = kStats + 2 * 2 * 128 * 4;
+  static constexpr uint32_t kBytes = kBars + 256;
 };
 
 template <int HD, int MODE>
-__global__ void __launch_bounds__(320, 1) swa_bwd_kernel(const __grid_constant__ SwaBwdArgs a) {
+__global__ void __launch_bounds__(kSwaBwdThreads, 1) swa_bwd_kernel(const __grid_constant__ SwaBwdArgs a) {
   static_assert(HD == 64 || HD == 128, "head dimensions 64 and 128");
   using SM = SwaBwdSmem<HD>;
-  constexpr int KBD = HD / 64;
-  constexpr uint32_t kBox = 128 * 128;    // [128 rows][64 features] box of an outer tile
-  constexpr uint32_t kIBox = 64 * 128;    // [64 rows][64 features] box of an inner tile
-  constexpr uint32_t kTmemCols = 512;     // 2 stages x (S 64, dP 64) at columns 0 / 128, accumulators from column 256
-  extern __shared__ uint8_t smem_raw[];
-  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  uint8_t* aligned = smem_raw + (base - smem_u32(smem_raw));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(aligned + SM::kBars);
+  constexpr int KBD = HD / 64, NA = SM::kStagesA, NB = SM::kStagesB;
+  constexpr uint32_t kBox = 128 * 128;    // [128 rows][64 features] box of a tile
+  constexpr uint32_t kTmemCols = 512;
+  // tensor memory: S at 0 (mode 1: two sets, 0 and 128), dP at 128 (mode 1: 256), accumulators behind them
+  constexpr uint32_t kDP = MODE == 0 ? 128 : 256, kAcc = kDP + 128;
+  extern __shared__ __align__(1024) uint8_t swa_bwd_smem[];   // (no room for alignment slack: the array itself is aligned)
+  const uint32_t base = smem_u32(swa_bwd_smem);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(swa_bwd_smem + SM::kBars);
   uint64_t* outer_full = bars;        // the CTA's own two tiles have landed
-  constexpr int NI = SM::kInnerStages;
-  uint64_t* inner_full = bars + 1;    // [3] the inner pair of a ring stage has landed
-  uint64_t* inner_empty = bars + 4;   // [3] second products that read a ring stage are done
-  uint64_t* sdp_full = bars + 7;      // [2] S and dP of a stage are in tensor memory
-  uint64_t* pds_full = bars + 9;      // [2] 8 arrivals: P and dS of a stage are in shared memory (S / dP columns read)
-  uint64_t* w_empty = bars + 11;      // [2] second products that read a stage's P / dS tiles are done
-  uint64_t* acc_full = bars + 13;     // all products of this CTA done
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
+  uint64_t* a_full = bars + 1;        // [3] first inner operand (mode 0: Q, mode 1: K)
+  uint64_t* a_empty = bars + 4;       // [3]
+  uint64_t* b_full = bars + 7;        // [2] second inner operand (mode 0: dO, mode 1: V)
+  uint64_t* b_empty = bars + 9;       // [2]
+  uint64_t* s_full = bars + 11;       // [2] S is in tensor memory (mode 0: the first alone)
+  uint64_t* dp_full = bars + 13;      // dP is in tensor memory
+  uint64_t* p_full = bars + 14;       // an arrival per softmax warp, mode 0: S has been read, P written
+  uint64_t* ds_full = bars + 15;      // likewise: dP (and S, mode 1) has been read, dS written
+  uint64_t* acc_full = bars + 16;     // all products of this CTA done
+  uint64_t* st_full = bars + 17;      // [2] mode 0: a tile's per-query values are in shared memory
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 19);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
   const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     mbar_init(outer_full, 1);
-    for (int s = 0; s < NI; ++s) {
-      mbar_init(&inner_full[s], 1);
-      mbar_init(&inner_empty[s], 1);
-    }
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(&sdp_full[s], 1);
-      mbar_init(&pds_full[s], 8);
-      mbar_init(&w_empty[s], 1);
-    }
+    for (int s = 0; s < NA; ++s) { mbar_init(&a_full[s], 1); mbar_init(&a_empty[s], 1); }
+    for (int s = 0; s < NB; ++s) { mbar_init(&b_full[s], 1); mbar_init(&b_empty[s], 1); }
+    for (int s = 0; s < 2; ++s) { mbar_init(&s_full[s], 1); mbar_init(&st_full[s], 1); }
+    mbar_init(dp_full, 1);
+    mbar_init(p_full, kSwaBwdWarps);
+    mbar_init(ds_full, kSwaBwdWarps);
     mbar_init(acc_full, 1);
     *abort_flag = 0;
     fence_mbar_init();
@@ -101,121 +102,149 @@ __global__ void __launch_bounds__(320, 1) swa_bwd_kernel(const __grid_constant__
   const int batch = blockIdx.x / (a.tiles * a.heads);
   const int o0 = ot * 128;   // first row of the outer tile (keys in mode 0, queries in mode 1)
   const int window = a.window > 0 ? a.window : a.L;
-  // inner 64-row tiles [t_lo, t_hi]
+  // inner 128-row tiles [t_lo, t_hi]
   int t_lo, t_hi;
   if (MODE == 0) {   // queries that see any key of this tile: q >= key, q <= key + window - 1
-    t_lo = o0 / 64;
-    const int q_max = o0 + 127 + window - 1;
-    t_hi = (q_max < a.L - 1 ? q_max : a.L - 1) / 64;
-    if (!a.causal) t_lo = 0, t_hi = (a.L - 1) / 64;   // block attention: every query tile
+    t_lo = o0 / 128;
+    const int64_t q_max = static_cast<int64_t>(o0) + 127 + window - 1;
+    t_hi = static_cast<int>(q_max < a.L - 1 ? q_max : a.L - 1) / 128;
+    if (!a.causal) t_lo = 0, t_hi = (a.L - 1) / 128;   // block attention: every query tile
   } else {           // keys this query tile sees: not before the window of its first query, nor before that query's sequence
     int lo = o0 - (window - 1);
     if (lo < 0) lo = 0;
     if (a.seq_start != nullptr && a.seq_start[o0] > lo) lo = a.seq_start[o0];
-    t_lo = lo / 64;
-    t_hi = (o0 + 127 < a.L - 1 ? o0 + 127 : a.L - 1) / 64;
-    if (!a.causal) t_lo = 0, t_hi = (a.Lk - 1) / 64;  // every key tile
+    t_lo = lo / 128;
+    t_hi = (o0 + 127 < a.L - 1 ? o0 + 127 : a.L - 1) / 128;
+    if (!a.causal) t_lo = 0, t_hi = (a.Lk - 1) / 128;  // every key tile
   }
   const int T = t_hi - t_lo + 1;
-  bool failed = uniform(static_cast<uint32_t>(*reinterpret_cast<volatile int32_t*>(a.status))) != kStatusOk;
+  // (swizzled tiles need the alignment asked for above)
+  bool failed = uniform(static_cast<uint32_t>(*reinterpret_cast<volatile int32_t*>(a.status))) != kStatusOk || (base & 1023u) != 0;
   const CUtensorMap* outer_a = MODE == 0 ? &a.k : &a.q;          // outer pair: (K, V) or (Q, dO)
   const CUtensorMap* outer_b = MODE == 0 ? &a.v : &a.dout;
-  const CUtensorMap* inner_a = MODE == 0 ? &a.q64 : &a.k64;      // inner pair: (Q, dO) or (K, V)
-  const CUtensorMap* inner_b = MODE == 0 ? &a.dout64 : &a.v64;
+  const CUtensorMap* inner_a = MODE == 0 ? &a.q : &a.k;          // inner pair: (Q, dO) or (K, V)
+  const CUtensorMap* inner_b = MODE == 0 ? &a.dout : &a.v;
+  float* const stats = reinterpret_cast<float*>(swa_bwd_smem + SM::kStats);   // [stage][lse | delta * scale][128]
+  const int64_t stat_base = (static_cast<int64_t>(batch) * a.heads + head) * a.L;
 
   if (warp == 0) {
     const uint32_t leader = elect_leader();
     if (!failed) {
-      mbar_expect_tx_if(leader, outer_full, 2 * SM::kOTile);
-      for (int j = 0; j < KBD; ++j) {
-        tma_load_4d_if(leader, base + SM::kOuter + j * kBox, outer_a, outer_full, 64 * j, o0, head, batch);
-        tma_load_4d_if(leader, base + SM::kOuter + SM::kOTile + j * kBox, outer_b, outer_full, 64 * j, o0, head, batch);
-      }
+      auto load = [&](uint32_t dst, const CUtensorMap* map, uint64_t* bar, int row) {
+        for (int j = 0; j < KBD; ++j) tma_load_4d_if(leader, dst + j * kBox, map, bar, 64 * j, row, head, batch);
+      };
+      mbar_expect_tx_if(leader, outer_full, 2 * SM::kTile);
+      load(base + SM::kOuter, outer_a, outer_full, o0);
+      load(base + SM::kOuter + SM::kTile, outer_b, outer_full, o0);
       for (int t = 0; t < T && !failed; ++t) {
-        const int s = t % NI;
-        if (t >= NI && !mbar_wait_warp(&inner_empty[s], (t / NI - 1) & 1, abort_flag)) { failed = true; break; }
-        mbar_expect_tx_if(leader, &inner_full[s], 2 * SM::kITile);
-        const uint32_t dst = base + SM::kInner + s * 2 * SM::kITile;
-        for (int j = 0; j < KBD; ++j) {
-          tma_load_4d_if(leader, dst + j * kIBox, inner_a, &inner_full[s], 64 * j, (t_lo + t) * 64, head, batch);
-          tma_load_4d_if(leader, dst + SM::kITile + j * kIBox, inner_b, &inner_full[s], 64 * j, (t_lo + t) * 64, head, batch);
-        }
+        const int sa = t % NA, sb = t % NB;
+        if (t >= NA && !mbar_wait_warp(&a_empty[sa], (t / NA - 1) & 1, abort_flag)) { failed = true; break; }
+        mbar_expect_tx_if(leader, &a_full[sa], SM::kTile);
+        load(base + SM::kA + sa * SM::kTile, inner_a, &a_full[sa], (t_lo + t) * 128);
+        if (t >= NB && !mbar_wait_warp(&b_empty[sb], (t / NB - 1) & 1, abort_flag)) { failed = true; break; }
+        mbar_expect_tx_if(leader, &b_full[sb], SM::kTile);
+        load(base + SM::kB + sb * SM::kTile, inner_b, &b_full[sb], (t_lo + t) * 128);
       }
     }
   } else if (warp == 1) {
     const uint32_t leader = elect_leader();
     if (!failed) {
-      const uint32_t idesc_first = make_idesc_bf16(128, 64, 0, 0);   // [outer x inner], both operands K-major (features)
-      const uint32_t idesc_acc = make_idesc_bf16(128, HD, 0, 1);     // [outer x HD]: A = P / dS tile K-major, B = inner tile MN-major
-      const uint32_t o_a = base + SM::kOuter, o_b = o_a + SM::kOTile;
-      // first products of inner tile t into its stage's columns
-      auto first = [&](int t) -> bool {
-        const int s = t & 1, si = t % NI;
-        if (!mbar_wait_warp(&inner_full[si], (t / NI) & 1, abort_flag)) return false;
+      const uint32_t idesc_first = make_idesc_bf16(128, 128, 0, 0);  // [outer x inner], both operands K-major (features)
+      const uint32_t idesc_acc = make_idesc_bf16(128, HD, 0, 1);     // [outer x HD]: A = P / dS, B = inner tile MN-major
+      const SmemDescBase desc(kBox);   // MN-major: 64-feature atoms a box apart (K-major descriptors ignore it)
+      // 128 x 128 product of two K-major tiles into columns `col`
+      auto first = [&](uint32_t col, uint32_t x, uint32_t y) {
+#pragma unroll
+        for (int kk = 0; kk < KBD; ++kk)
+#pragma unroll
+          for (int k4 = 0; k4 < 4; ++k4)
+            umma_bf16_if(leader, col, desc.at((x + kk * kBox + k4 * 32) >> 4), desc.at((y + kk * kBox + k4 * 32) >> 4), idesc_first,
+                         (kk | k4) != 0);
+      };
+      // accumulator at `col` += A (tensor memory: 32 inner rows in 16 columns from `ta` and every 32 columns on) x inner tile
+      auto second = [&](uint32_t col, uint32_t ta, uint32_t y, bool fresh) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          umma_bf16_ta_if(leader, col, ta + (k >> 1) * 32 + (k & 1) * 8, desc.at((y + k * 2048) >> 4), idesc_acc, !fresh || k != 0);
+      };
+      const uint32_t o_a = base + SM::kOuter, o_b = o_a + SM::kTile;
+      auto tile_a = [&](int t) { return base + SM::kA + (t % NA) * SM::kTile; };
+      auto tile_b = [&](int t) { return base + SM::kB + (t % NB) * SM::kTile; };
+      auto issue_s = [&](int t) -> bool {
+        if (!mbar_wait_warp(&a_full[t % NA], (t / NA) & 1, abort_flag)) return false;
         tc_fence_after();
-        const uint32_t i_a = base + SM::kInner + si * 2 * SM::kITile, i_b = i_a + SM::kITile;
-        const uint32_t col = tmem + s * 128;
-#pragma unroll
-        for (int kk = 0; kk < KBD; ++kk)
-#pragma unroll
-          for (int k4 = 0; k4 < 4; ++k4)
-            umma_bf16_if(leader, col, make_smem_desc(o_a + kk * kBox + k4 * 32, 0, 1024),
-                      make_smem_desc(i_a + kk * kIBox + k4 * 32, 0, 1024), idesc_first, (kk | k4) != 0);
-#pragma unroll
-        for (int kk = 0; kk < KBD; ++kk)
-#pragma unroll
-          for (int k4 = 0; k4 < 4; ++k4)
-            umma_bf16_if(leader, col + 64, make_smem_desc(o_b + kk * kBox + k4 * 32, 0, 1024),
-                      make_smem_desc(i_b + kk * kIBox + k4 * 32, 0, 1024), idesc_first, (kk | k4) != 0);
-        umma_commit_if(leader, &sdp_full[s]);
+        const int set = MODE == 0 ? 0 : t & 1;
+        first(tmem + set * 128, o_a, tile_a(t));
+        umma_commit_if(leader, &s_full[set]);
         return true;
       };
-      if (!mbar_wait_warp(outer_full, 0, abort_flag)) failed = true;
-      if (!failed && !first(0)) failed = true;
-      for (int t = 0; t < T && !failed; ++t) {
-        const int s = t & 1;
-        // (the other stage's columns were read by the softmax threads of tile t - 1: awaited one iteration ago)
-        if (t + 1 < T && !first(t + 1)) { failed = true; break; }
-        if (!mbar_wait_warp(&pds_full[s], (t >> 1) & 1, abort_flag)) { failed = true; break; }
+      auto issue_dp = [&](int t) -> bool {
+        if (!mbar_wait_warp(&b_full[t % NB], (t / NB) & 1, abort_flag)) return false;
         tc_fence_after();
-        const int si = t % NI;
-        const uint32_t i_a = base + SM::kInner + si * 2 * SM::kITile, i_b = i_a + SM::kITile;
-        const uint32_t w_p = base + SM::kW + s * 2 * SM::kWTile, w_ds = w_p + SM::kWTile;
-        // contraction over the 64 inner rows: four 16-row steps
-#pragma unroll
-        for (int k4 = 0; k4 < 4; ++k4) {
-          if (MODE == 0) {
-            umma_bf16_if(leader, tmem + 256, make_smem_desc(w_p + k4 * 32, 0, 1024), make_smem_desc(i_b + k4 * 2048, kIBox, 1024),
-                      idesc_acc, (t | k4) != 0);            // dV += P^T dO
-            umma_bf16_if(leader, tmem + 256 + HD, make_smem_desc(w_ds + k4 * 32, 0, 1024), make_smem_desc(i_a + k4 * 2048, kIBox, 1024),
-                      idesc_acc, (t | k4) != 0);            // dK += dS^T Q
-          } else {
-            umma_bf16_if(leader, tmem + 256, make_smem_desc(w_ds + k4 * 32, 0, 1024), make_smem_desc(i_a + k4 * 2048, kIBox, 1024),
-                      idesc_acc, (t | k4) != 0);            // dQ += dS K
-          }
+        first(tmem + kDP, o_b, tile_b(t));
+        umma_commit_if(leader, dp_full);
+        if (MODE == 1) umma_commit_if(leader, &b_empty[t % NB]);
+        return true;
+      };
+      failed = !mbar_wait_warp(outer_full, 0, abort_flag) || !issue_s(0) || !issue_dp(0) || (MODE == 1 && T > 1 && !issue_s(1));
+      for (int t = 0; t < T && !failed; ++t) {
+        if (MODE == 0) {
+          if (!mbar_wait_warp(p_full, t & 1, abort_flag)) { failed = true; break; }
+          tc_fence_after();
+          second(tmem + kAcc, tmem, tile_b(t), t == 0);                // dV += P^T dO
+          umma_commit_if(leader, &b_empty[t % NB]);
+          if (t + 1 < T && !issue_s(t + 1)) { failed = true; break; }
+          if (!mbar_wait_warp(ds_full, t & 1, abort_flag)) { failed = true; break; }
+          tc_fence_after();
+          second(tmem + kAcc + HD, tmem + kDP, tile_a(t), t == 0);     // dK += dS^T Q
+          umma_commit_if(leader, &a_empty[t % NA]);
+          if (t + 1 < T && !issue_dp(t + 1)) { failed = true; break; }
+        } else {
+          if (!mbar_wait_warp(ds_full, t & 1, abort_flag)) { failed = true; break; }
+          tc_fence_after();
+          if (t + 1 < T && !issue_dp(t + 1)) { failed = true; break; }
+          second(tmem + kAcc, tmem + (t & 1) * 128, tile_a(t), t == 0);  // dQ += dS K
+          umma_commit_if(leader, &a_empty[t % NA]);
+          if (t + 2 < T && !issue_s(t + 2)) { failed = true; break; }
         }
-        umma_commit_if(leader, &inner_empty[si]);
-        umma_commit_if(leader, &w_empty[s]);
       }
       if (!failed) umma_commit_if(leader, acc_full);
     }
+  } else if (warp == 2 + kSwaBwdWarps) {
+    // ---------------- mode 0: the per-query values of an inner tile, fetched a tile ahead; a stage is free again once the tile
+    // before last has been worked out
+    if (MODE == 0) {
+      float x[8];   // lse and delta of queries lane, lane + 32, ...
+      auto fetch = [&](int t) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int qi = (t_lo + t) * 128 + lane + 32 * i;
+          x[i] = qi < a.L ? a.lse[stat_base + qi] : INFINITY;
+          x[4 + i] = qi < a.L ? a.delta[stat_base + qi] : 0.f;
+        }
+      };
+      if (!failed) fetch(0);
+      for (int t = 0; t < T && !failed; ++t) {
+        if (t >= 2 && !mbar_wait_warp(ds_full, t & 1, abort_flag)) { failed = true; break; }  // of tile t - 2
+        float* st = stats + (t & 1) * 256 + lane;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          st[32 * i] = x[i];
+          st[128 + 32 * i] = x[4 + i] * a.scale;
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&st_full[t & 1]);
+        if (t + 1 < T) fetch(t + 1);
+      }
+    }
   } else {
-    // ---------------- softmax / epilogue: two threads per tensor-memory lane (outer row), 32 inner columns each
+    // ---------------- softmax / epilogue: four threads per tensor-memory lane (outer row), 32 inner columns each
     const int quarter = warp & 3;
-    const int half = (warp - 2) >> 2;
+    const int part = (warp - 2) >> 2;
     const int r = quarter * 32 + lane;
-    const int sid = threadIdx.x - 64;   // 0 .. 255
     const uint32_t lane_off = static_cast<uint32_t>(quarter * 32) << 16;
-    const int64_t stat_base = (static_cast<int64_t>(batch) * a.heads + head) * a.L;
     const int row = o0 + r;             // this thread's key (mode 0) or query (mode 1)
-    float* stats = reinterpret_cast<float*>(aligned + SM::kStats);   // [stage][lse | delta * scale | sequence start][64]
-    // mode 0: per-query values of an inner tile, one word per thread 0 .. 191, staged one tile ahead
-    auto stat_load = [&](int t) -> uint32_t {
-      const int arr = sid >> 6, qi = (t_lo + t) * 64 + (sid & 63);
-      if (arr == 0) return __float_as_uint(qi < a.L ? a.lse[stat_base + qi] : INFINITY);
-      if (arr == 1) return __float_as_uint(qi < a.L ? a.delta[stat_base + qi] * a.scale : 0.f);
-      return (a.seq_start != nullptr && qi < a.L) ? static_cast<uint32_t>(a.seq_start[qi]) : 0u;
-    };
+    const int c0 = part * 32;
     float lse_r = INFINITY, delta_r = 0.f;
     int row_start = 0;
     if (MODE == 1 && row < a.L) {
@@ -223,130 +252,119 @@ __global__ void __launch_bounds__(320, 1) swa_bwd_kernel(const __grid_constant__
       delta_r = a.delta[stat_base + row] * a.scale;
       if (a.seq_start != nullptr) row_start = a.seq_start[row];
     }
-    if (MODE == 0 && sid < 192) reinterpret_cast<uint32_t*>(stats)[sid] = stat_load(0);
-    for (int t = 0; t < T; ++t) {
-      const int s = t & 1;
-      // every thread runs every iteration (the named barrier counts all 256), failed or not
-      if (MODE == 0) named_barrier_sync(1, 256);   // stage s of the per-query words is written, stage s ^ 1 no longer read
-      uint32_t next_stat = 0;
-      if (MODE == 0 && sid < 192 && t + 1 < T) next_stat = stat_load(t + 1);
-      if (!failed) {
-        const int i0 = (t_lo + t) * 64;
-        if (!mbar_wait(&sdp_full[s], (t >> 1) & 1, abort_flag) ||
-            (t >= 2 && !mbar_wait(&w_empty[s], ((t >> 1) - 1) & 1, abort_flag))) {
-          failed = true;
-          *abort_flag = 1;
+    // first / last inner row that this outer row meets: mode 0, queries row .. row + window - 1; mode 1, the keys of its window
+    // and sequence.  (The bounds once per thread: tests of every pair took 8500 clocks in each of the two tiles of a band
+    // that are cut by it, a quarter of the kernel at a window of 2048.)
+    int in_lo, in_hi;
+    if (MODE == 0) {
+      const int64_t last = a.causal ? static_cast<int64_t>(row) + window - 1 : a.L - 1;
+      in_lo = a.causal ? row : 0;
+      in_hi = row < a.Lk ? static_cast<int>(last < a.L - 1 ? last : a.L - 1) : -1;
+    } else {
+      in_lo = a.causal ? (row - (window - 1) > row_start ? row - (window - 1) : row_start) : 0;
+      in_hi = row < a.L ? (a.causal ? row : a.Lk - 1) : -1;
+    }
+    const int outer_start = MODE == 1 && a.seq_start != nullptr ? a.seq_start[o0 + 127 < a.L ? o0 + 127 : a.L - 1] : 0;
+    for (int t = 0; t < T && !failed; ++t) {
+      const int i0 = (t_lo + t) * 128, set = MODE == 0 ? 0 : t & 1;
+      const float* st = stats + (t & 1) * 256 + c0;
+      if ((MODE == 0 && !mbar_wait_warp(&st_full[t & 1], (t >> 1) & 1, abort_flag)) ||
+          !mbar_wait_warp(&s_full[set], (MODE == 0 ? t : t >> 1) & 1, abort_flag)) {
+        failed = true;
+        break;
+      }
+      tc_fence_after();
+      uint32_t bits[32];
+      tmem_ld32(tmem + lane_off + set * 128 + c0, bits);
+      bool interior;   // every (row, column) pair of the tile visible: no masks
+      if (MODE == 0) {
+        const int tile_start = a.seq_start != nullptr ? a.seq_start[i0 + 127 < a.L ? i0 + 127 : a.L - 1] : 0;
+        interior = a.causal ? (o0 + 127 <= i0 && o0 >= i0 + 127 - (window - 1) && i0 + 127 < a.L && o0 >= tile_start)
+                            : (i0 + 127 < a.L && o0 + 127 < a.Lk);
+      } else {
+        interior = a.causal ? (i0 + 127 <= o0 && i0 >= o0 + 127 - (window - 1) && o0 + 127 < a.L && i0 >= outer_start)
+                            : (i0 + 127 < a.Lk && o0 + 127 < a.L);
+      }
+      tmem_ld_wait();
+      // p = 2^(s c - lse)
+      float p[32];
+#pragma unroll
+      for (int g = 0; g < 8; ++g) {
+        float lv[4] = {lse_r, lse_r, lse_r, lse_r};
+        if (MODE == 0) {
+          const float4 l4 = *reinterpret_cast<const float4*>(st + g * 4);
+          lv[0] = l4.x; lv[1] = l4.y; lv[2] = l4.z; lv[3] = l4.w;
         }
-        if (!failed) {
-          tc_fence_after();
-          const int c0 = half * 32;
-          uint32_t sb[32], db[32];
-          tmem_ld32(tmem + lane_off + s * 128 + c0, sb);
-          tmem_ld32(tmem + lane_off + s * 128 + 64 + c0, db);
-          tmem_ld_wait();
-          // p = 2^(s c - lse),  dS = p (dP scale - Delta scale); tiles wholly inside the band skip the masks
-          float p[32], ds[32];
-          if (MODE == 0) {
-            // rows = keys, columns = queries i0 + c
-            const int last_q = i0 + 63 < a.L ? i0 + 63 : a.L - 1;
-            const int tile_start = a.seq_start != nullptr ? a.seq_start[last_q] : 0;
-            const bool interior = a.causal ? (o0 + 127 <= i0 && o0 >= i0 + 63 - (window - 1) && i0 + 63 < a.L && o0 >= tile_start)
-                                           : (i0 + 63 < a.L && o0 + 127 < a.Lk);
-            const float* st = stats + s * 192 + c0;
-            if (interior) {
 #pragma unroll
-              for (int g = 0; g < 8; ++g) {
-                const float4 l4 = *reinterpret_cast<const float4*>(st + g * 4);
-                const float4 d4 = *reinterpret_cast<const float4*>(st + 64 + g * 4);
-                const float lv[4] = {l4.x, l4.y, l4.z, l4.w}, dv[4] = {d4.x, d4.y, d4.z, d4.w};
+        for (int e = 0; e < 4; ++e) p[g * 4 + e] = exp2_ftz(fmaf(__uint_as_float(bits[g * 4 + e]), a.scale_log2, -lv[e]));
+      }
+      if (!interior) {
+        const int lo = in_lo - i0 - c0, hi = in_hi - i0 - c0;
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                  const int j = g * 4 + e;
-                  p[j] = exp2_ftz(fmaf(__uint_as_float(sb[j]), a.scale_log2, -lv[e]));
-                  ds[j] = p[j] * fmaf(__uint_as_float(db[j]), a.scale, -dv[e]);
-                }
-              }
-            } else {
+        for (int j = 0; j < 32; ++j)
+          if (j < lo || j > hi) p[j] = 0.f;
+        if (MODE == 0 && a.seq_start != nullptr) {   // queries of a later sequence do not see this key
 #pragma unroll
-              for (int g = 0; g < 8; ++g) {
-                const float4 l4 = *reinterpret_cast<const float4*>(st + g * 4);
-                const float4 d4 = *reinterpret_cast<const float4*>(st + 64 + g * 4);
-                const int4 s4 = *reinterpret_cast<const int4*>(st + 128 + g * 4);
-                const float lv[4] = {l4.x, l4.y, l4.z, l4.w}, dv[4] = {d4.x, d4.y, d4.z, d4.w};
-                const int sv[4] = {s4.x, s4.y, s4.z, s4.w};
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                  const int j = g * 4 + e, qi = i0 + c0 + j;
-                  const bool ok = (!a.causal || (row <= qi && row >= qi - (window - 1) && row >= sv[e])) && qi < a.L && row < a.Lk;
-                  p[j] = ok ? exp2_ftz(fmaf(__uint_as_float(sb[j]), a.scale_log2, -lv[e])) : 0.f;
-                  ds[j] = p[j] * fmaf(__uint_as_float(db[j]), a.scale, -dv[e]);
-                }
-              }
-            }
-          } else {
-            // rows = queries, columns = keys i0 + c
-            const int last_q = o0 + 127 < a.L ? o0 + 127 : a.L - 1;
-            const int tile_start = a.seq_start != nullptr ? a.seq_start[last_q] : 0;
-            const bool interior = a.causal ? (i0 + 63 <= o0 && i0 >= o0 + 127 - (window - 1) && o0 + 127 < a.L && i0 >= tile_start)
-                                           : (i0 + 63 < a.Lk && o0 + 127 < a.L);
-            if (interior) {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) {
-                p[j] = exp2_ftz(fmaf(__uint_as_float(sb[j]), a.scale_log2, -lse_r));
-                ds[j] = p[j] * fmaf(__uint_as_float(db[j]), a.scale, -delta_r);
-              }
-            } else {
-              const int k_hi = row < a.L ? (a.causal ? row : a.Lk - 1) : -1;   // last / first key this query may see
-              const int k_lo = a.causal ? (row - (window - 1) > row_start ? row - (window - 1) : row_start) : 0;
-#pragma unroll
-              for (int j = 0; j < 32; ++j) {
-                const int kv = i0 + c0 + j;
-                const bool ok = kv >= k_lo && kv <= k_hi;
-                p[j] = ok ? exp2_ftz(fmaf(__uint_as_float(sb[j]), a.scale_log2, -lse_r)) : 0.f;
-                ds[j] = p[j] * fmaf(__uint_as_float(db[j]), a.scale, -delta_r);
-              }
-            }
-          }
-          const uint32_t p_row = base + SM::kW + s * 2 * SM::kWTile + r * 128, ds_row = p_row + SM::kWTile;
-#pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            const uint32_t sw = ((half * 4 + g) ^ (r & 7)) << 4;
-            if (MODE == 0)
-              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(p_row + sw), "r"(pack_bf16x2(p[g * 8 + 0], p[g * 8 + 1])),
-                           "r"(pack_bf16x2(p[g * 8 + 2], p[g * 8 + 3])), "r"(pack_bf16x2(p[g * 8 + 4], p[g * 8 + 5])),
-                           "r"(pack_bf16x2(p[g * 8 + 6], p[g * 8 + 7]))
-                           : "memory");
-            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(ds_row + sw), "r"(pack_bf16x2(ds[g * 8 + 0], ds[g * 8 + 1])),
-                         "r"(pack_bf16x2(ds[g * 8 + 2], ds[g * 8 + 3])), "r"(pack_bf16x2(ds[g * 8 + 4], ds[g * 8 + 5])),
-                         "r"(pack_bf16x2(ds[g * 8 + 6], ds[g * 8 + 7]))
-                         : "memory");
-          }
-          tc_fence_before();
-          fence_async_proxy();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&pds_full[s]);
+          for (int j = 0; j < 32; ++j)
+            if (row < a.seq_start[min(i0 + c0 + j, a.L - 1)]) p[j] = 0.f;
         }
       }
-      if (MODE == 0 && sid < 192 && t + 1 < T) reinterpret_cast<uint32_t*>(stats)[(s ^ 1) * 192 + sid] = next_stat;
+      uint32_t w[16];
+      if (MODE == 0) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) w[j] = pack_bf16x2(p[2 * j], p[2 * j + 1]);
+        tmem_st16(tmem + lane_off + c0, w);
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(p_full);
+      }
+      if (!mbar_wait_warp(dp_full, t & 1, abort_flag)) {
+        failed = true;
+        break;
+      }
+      tc_fence_after();
+      // dS = p (dP scale - Delta scale)
+      tmem_ld32(tmem + lane_off + kDP + c0, bits);
+      tmem_ld_wait();
+#pragma unroll
+      for (int g = 0; g < 8; ++g) {
+        float dv[4] = {delta_r, delta_r, delta_r, delta_r};
+        if (MODE == 0) {
+          const float4 d4 = *reinterpret_cast<const float4*>(st + 128 + g * 4);
+          dv[0] = d4.x; dv[1] = d4.y; dv[2] = d4.z; dv[3] = d4.w;
+        }
+        float ds[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) ds[e] = p[g * 4 + e] * fmaf(__uint_as_float(bits[g * 4 + e]), a.scale, -dv[e]);
+        w[g * 2] = pack_bf16x2(ds[0], ds[1]);
+        w[g * 2 + 1] = pack_bf16x2(ds[2], ds[3]);
+      }
+      tmem_st16(tmem + lane_off + (MODE == 0 ? kDP : set * 128u) + c0, w);
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(ds_full);
     }
-    // accumulators: row = outer-tile row (key in mode 0, query in mode 1); this thread stores HD / 2 features of it
-    if (!failed && !mbar_wait(acc_full, 0, abort_flag)) failed = true;
+    if (failed) *abort_flag = 1;
+    // accumulators: row = outer-tile row (key in mode 0, query in mode 1); this thread stores HD / 4 features of it
+    if (!failed && !mbar_wait_warp(acc_full, 0, abort_flag)) failed = true;
     if (!failed) {
       tc_fence_after();
-      constexpr int OC = HD / 2;
+      constexpr int OC = HD / 4;
 #pragma unroll
       for (int acc = 0; acc < (MODE == 0 ? 2 : 1); ++acc) {
         // mode 0: accumulator 0 = dV, accumulator 1 = dK; mode 1: dQ
         bf16* dst_base = MODE == 0 ? (acc == 0 ? a.out1 : a.out0) : a.out0;
-        bf16* dst = dst_base + batch * a.o_bs + static_cast<int64_t>(row) * a.o_ts + head * a.o_hs + half * OC;
+        bf16* dst = dst_base + batch * a.o_bs + static_cast<int64_t>(row) * a.o_ts + head * a.o_hs + part * OC;
 #pragma unroll
-        for (int c = 0; c < OC; c += 32) {
-          uint32_t bits[32];
-          tmem_ld32(tmem + lane_off + 256 + acc * HD + half * OC + c, bits);
+        for (int c = 0; c < OC; c += 16) {
+          uint32_t bits[16];
+          tmem_ld16(tmem + lane_off + kAcc + acc * HD + part * OC + c, bits);
           tmem_ld_wait();
           if (row < (MODE == 0 ? a.Lk : a.L)) {
 #pragma unroll
-            for (int g = 0; g < 4; ++g) {
+            for (int g = 0; g < 2; ++g) {
               uint4 u;
               u.x = pack_bf16x2(__uint_as_float(bits[g * 8 + 0]), __uint_as_float(bits[g * 8 + 1]));
               u.y = pack_bf16x2(__uint_as_float(bits[g * 8 + 2]), __uint_as_float(bits[g * 8 + 3]));
