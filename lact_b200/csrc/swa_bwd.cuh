@@ -17,6 +17,9 @@
 //   mode 1  ... dP(t + 1), dQ(t), S(t + 2) ...          S has two sets of columns, dP one
 // The first inner operand (Q or K) is held from its first product to the second products a tile later and goes through a
 // three-stage ring, the other through two stages.  Every mbarrier wait is bounded.
+// Measured (2 x 32768 tokens, 12 heads of 128, window 2048; 128 x 128 pairs): keys' side 1514 us, queries' side 1079, where
+// 64-row inner tiles with P and dS in shared memory took 1712 and 1287.  About 2900 and 2350 clocks a tile for 2050 and 1540 of
+// products; 1030 of them are exponentials (16 a clock), which no other phase of the same tile can hide.
 #pragma once
 #include "swa.cuh"
 
