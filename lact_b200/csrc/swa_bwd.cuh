@@ -75,7 +75,8 @@ __global__ void __launch_bounds__(kSwaBwdThreads, 1) swa_bwd_kernel(const __grid
   uint64_t* ds_full = bars + 15;      // likewise: dP (and S, mode 1) has been read, dS written
   uint64_t* acc_full = bars + 16;     // all products of this CTA done
   uint64_t* st_full = bars + 17;      // [2] mode 0: a tile's per-query values are in shared memory
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 19);
+  uint64_t* st_empty = bars + 19;     // [2] an arrival per softmax warp: it has read them
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 21);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
   const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
@@ -83,7 +84,7 @@ __global__ void __launch_bounds__(kSwaBwdThreads, 1) swa_bwd_kernel(const __grid
     mbar_init(outer_full, 1);
     for (int s = 0; s < NA; ++s) { mbar_init(&a_full[s], 1); mbar_init(&a_empty[s], 1); }
     for (int s = 0; s < NB; ++s) { mbar_init(&b_full[s], 1); mbar_init(&b_empty[s], 1); }
-    for (int s = 0; s < 2; ++s) { mbar_init(&s_full[s], 1); mbar_init(&st_full[s], 1); }
+    for (int s = 0; s < 2; ++s) { mbar_init(&s_full[s], 1); mbar_init(&st_full[s], 1); mbar_init(&st_empty[s], kSwaBwdWarps); }
     mbar_init(dp_full, 1);
     mbar_init(p_full, kSwaBwdWarps);
     mbar_init(ds_full, kSwaBwdWarps);
@@ -214,8 +215,9 @@ __global__ void __launch_bounds__(kSwaBwdThreads, 1) swa_bwd_kernel(const __grid
       if (!failed) umma_commit_if(leader, acc_full);
     }
   } else if (warp == 2 + kSwaBwdWarps) {
-    // ---------------- mode 0: the per-query values of an inner tile, fetched a tile ahead; a stage is free again once the tile
-    // before last has been worked out
+    // ---------------- mode 0: the per-query values of an inner tile, fetched a tile ahead.  A stage has a barrier of its own for
+    // its way back: the softmax warps may be two tiles past this warp (their tile t - 1 needs nothing more from it), and a wait by
+    // parity on a barrier that completes once per tile, such as ds_full, would then stand for a tile that waits for this warp.
     if (MODE == 0) {
       float x[8];   // lse and delta of queries lane, lane + 32, ...
       auto fetch = [&](int t) {
@@ -228,7 +230,7 @@ __global__ void __launch_bounds__(kSwaBwdThreads, 1) swa_bwd_kernel(const __grid
       };
       if (!failed) fetch(0);
       for (int t = 0; t < T && !failed; ++t) {
-        if (t >= 2 && !mbar_wait_warp(ds_full, t & 1, abort_flag)) { failed = true; break; }  // of tile t - 2
+        if (t >= 2 && !mbar_wait_warp(&st_empty[t & 1], ((t >> 1) - 1) & 1, abort_flag)) { failed = true; break; }  // tile t - 2
         float* st = stats + (t & 1) * 256 + lane;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -347,7 +349,10 @@ __global__ void __launch_bounds__(kSwaBwdThreads, 1) swa_bwd_kernel(const __grid
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(ds_full);
+      if (lane == 0) {
+        mbar_arrive(ds_full);
+        if (MODE == 0) mbar_arrive(&st_empty[t & 1]);
+      }
     }
     if (failed) *abort_flag = 1;
     // accumulators: row = outer-tile row (key in mode 0, query in mode 1); this thread stores HD / 4 features of it
