@@ -52,7 +52,7 @@ ns_bwd_fused_kernel(const __grid_constant__ NsBwdFusedArgs<BT_MM, BT, NITER, SYM
   constexpr int RING = ns_bwd_ring<BT_MM, BT, SYM>();
   constexpr uint32_t kTmemCols = 512;
   griddep_launch_dependents();
-  if (*reinterpret_cast<volatile int32_t*>(args.status) != kStatusOk) return;  // uniform over the grid
+  if (__syncthreads_or(*reinterpret_cast<volatile int32_t*>(args.status) != kStatusOk)) return;  // (all threads of the CTA or none)
   extern __shared__ uint8_t smem_raw[];
   GemmCtx cx;
   gemm_setup(cx, smem_raw, RING, ns_bwd_stride<BT_MM, BT, SYM>(), ns_bwd_staging<BT_MM, BT, SYM>(), kTmemCols);

@@ -72,7 +72,7 @@ ns_fused_kernel(const __grid_constant__ NsFusedArgs<BT_MM, BT_MN, NITER, SYM> ar
   constexpr uint32_t kStride = ns_fused_stage_stride<BT_MM, BT_MN, SYM>();
   constexpr uint32_t kTmemCols = 512;
   griddep_launch_dependents();  // the next kernel may run its prologue while this one works
-  if (*reinterpret_cast<volatile int32_t*>(args.status) != kStatusOk) return;  // uniform over the grid
+  if (__syncthreads_or(*reinterpret_cast<volatile int32_t*>(args.status) != kStatusOk)) return;  // (all threads of the CTA or none)
   extern __shared__ uint8_t smem_raw[];
   GemmCtx cx;
   gemm_setup(cx, smem_raw, RING, kStride, ns_fused_staging<BT_MM, BT_MN, SYM>(), kTmemCols);

@@ -163,7 +163,8 @@ pair_gemm_kernel(const __grid_constant__ GemmArgs<Op, NPROB> args, const int npr
   auto begins = [&](const Run& r) { return r.m == (Op::kReverseBatch ? (r.prob ? tm[1] : tm[0]) - 1 : 0); };
   auto ends = [&](const Run& r) { return r.m == (Op::kReverseBatch ? 0 : (r.prob ? tm[1] : tm[0]) - 1); };
   auto problem = [&](const Run& r) -> const GemmProblem<Op>& { return args.prob[NPROB > 1 ? r.prob : 0]; };
-  bool failed = uniform(*reinterpret_cast<volatile int32_t*>(args.status) != kStatusOk) != 0;
+  // (the CTAs of a pair may differ: every wait for the other has a limit)
+  bool failed = earlier_launch_failed(args.status);
   const bool work = !failed;
   auto term_bytes = [](int t) { return static_cast<uint32_t>(Wire::template b_rows<Op>(t)) * 128u; };  // a k-block of B, per CTA
   constexpr uint32_t b_bytes = pair_b_bytes<Op>(1);

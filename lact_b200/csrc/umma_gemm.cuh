@@ -810,6 +810,17 @@ __device__ __forceinline__ void gemm_teardown(GemmCtx& cx, bool failed, int32_t*
   if ((threadIdx.x >> 5) == 1) tmem_dealloc(cx.tmem_base, tmem_cols);
 }
 
+// Whether an earlier launch has given up.  Calls on other streams may share the word, so it can change while a CTA reads it:
+// the epilogue warps decide together (they would wait for one another at named barriers, which have no time limit; the barrier
+// here costs nothing, they have to wait for the first tile anyway).  The other warps wait at mbarriers alone, with a limit.
+// The answer has to be uniform for the compiler too: with a decision per thread, or one barrier for all warps, the launches of
+// small calls took 0.2 to 0.7 us longer (4 entries of 384, 2048 tokens: apply 15.5 us, 16.1 and 16.1 that way).
+__device__ __forceinline__ bool earlier_launch_failed(const int32_t* status) {
+  bool set = *reinterpret_cast<const volatile int32_t*>(status) != kStatusOk;
+  if (uniform_warp_index() >= 2) set = named_barrier_any(1, kEpiWarps * 32, set);
+  return uniform(set) != 0;
+}
+
 // Persistent single-phase kernel.  The prologue (barriers, tensor memory, descriptor prefetch)
 // touches no global memory and may overlap the tail of the previous kernel in the stream.
 template <class Op, int NPROB>
@@ -834,7 +845,7 @@ umma_gemm_kernel(const __grid_constant__ GemmArgs<Op, NPROB> args, const int npr
   griddep_wait();
   bool failed = false;
   // an earlier launch gave up: do nothing but release the resources
-  if (*reinterpret_cast<volatile int32_t*>(args.status) == kStatusOk)
+  if (!earlier_launch_failed(args.status))
     failed = gemm_phase<Op, Op::STAGES>(cx, args.prob, nprob, NoPatch{});
   gemm_teardown(cx, failed, args.status, kTmemCols);
 }

@@ -75,3 +75,17 @@ def test_per_query_values_of_the_attention_backward(tiles, slowest):
 
     agents = {"values": values(), "softmax": softmax(), "products": products()}
     assert _all_end(agents, slowest)
+
+
+@pytest.mark.parametrize("name", ["umma_gemm.cuh", "pair_gemm.cuh", "ns_fused.cuh", "ns_bwd_fused.cuh", "ns_chip.cuh"])
+def test_whether_to_take_part_is_decided_once_per_cta(name):
+    """The warps of these kernels meet at named barriers, which have no time limit, if they take part: no thread may decide that
+    from its own reading of the status word.  (A thread that reports a failure of its own may look at it, or one that tells all.)"""
+    reads = [line for line in _source(name).splitlines() if ".status) == kStatusOk" in line or ".status) != kStatusOk" in line]
+    assert all(any(w in line for w in ("failed &&", "if (threadIdx.x == 0)", "__syncthreads_or(")) for line in reads), reads
+    assert reads or "earlier_launch_failed(args.status)" in _source(name)
+
+
+def test_the_epilogue_warps_decide_at_a_barrier():
+    body = re.search(r"bool earlier_launch_failed\(.*?\n}", _source("umma_gemm.cuh"), re.S).group(0)
+    assert "if (uniform_warp_index() >= 2) set = named_barrier_any(" in body
