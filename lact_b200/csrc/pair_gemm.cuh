@@ -227,6 +227,12 @@ pair_gemm_kernel(const __grid_constant__ GemmArgs<Op, NPROB> args, const int npr
       }
       if (first) bph ^= 1;
     }
+    // The last products' commits arrive in this CTA's shared memory too: they are waited for, stage by stage, before it goes.
+    for (int i = 0; i < ring && !failed; ++i) {
+      failed = !mbar_wait_warp(&empty[s], ph ^ 1, abort_flag);
+      if (++s == ring) { s = 0; ph ^= 1; }
+    }
+    for (int kb = 0; kb < num_kb && !failed; ++kb) failed = !mbar_wait_warp(&b_empty[kb], bph ^ 1, abort_flag);
   } else if (warp == 1) {
     // ---------------- MMA issuer of the pair
     if (rank == 0) {
