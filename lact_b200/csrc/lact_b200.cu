@@ -274,16 +274,27 @@ int launch_gemm(const GemmArgs<Op, NPROB>& args, cudaStream_t stream, int cls, i
   return LACT_OK;
 }
 
-// Whether a product of `batch` x `M` tokens with N columns in tiles of `bt` goes to pairs of SMs (pair_gemm.cuh).  It does where
-// a pair keeps its weights for at least six tiles of 256 tokens: a launch of clusters costs about 2 us more than a plain one, and
-// with fewer tiles the halves of the last one stand idle.  Measured, us per launch, pairs against single SMs: 1.3 tiles per pair
-// (4 entries of 384, 2048 tokens) gate 16.2 / 14.7, down 12.7 / 10.7, pointwise 21.8 / 21.0; 2.3 to 4.7 (12 entries of 128 x 256,
-// 1560 tokens) 16.8 / 16.6, 12.7 / 10.7, 20.9 / 20.9; 7 to 10.7 (32 of 384, 2048) 43 / 48, 28.8 / 31.5, 96 / 99; 128 (16 of 192,
-// 49152) pointwise 314 / 347.
+// Whether a product of `batch` x `M` tokens and N columns goes to pairs of SMs (pair_gemm.cuh).  All sides measured as us of the
+// call with pairs / with single SMs, pointwise stage and apply, 2 to 16 tiles of 256 tokens per pair:
+//   - a ring of three stages has to fit beside the weights: at K = 512 the pointwise stage has two and takes 1.14 to 1.74 times as
+//     long (18 entries of 512, 4096 tokens: 193 / 154); at 384, three: 0.89 to 0.95;
+//   - six of seven pairs have to find work: a team of pairs has one for every column tile, so that 25 tiles (H = 1600) leave 24 of
+//     74 pairs idle (98.7 / 83.1), 40 (H = 2560) leave 34 (116 / 81); 16 leave 10 (55.1 / 63.5);
+//   - rows are computed in halves of 256: entries of 16 or 128 tokens waste a half or more (394 of 384, 128 tokens: 119 / 90; apply
+//     of 592 entries of 192, 16 tokens: 51 / 32), 384 tokens a quarter (119 / 110).  A tenth may be wasted;
+//   - a set of weights has to serve enough products, or loading the next one shows: 49152 columns x k per 128 rows, 65536 where
+//     tiles are narrow.  At one tile per set 256 or more wide features reach that (197 entries of 384, 256 tokens: 73.9 / 78.1, apply
+//     60.7 / 63.6), 192 do not (apply 76.0 / 64.1), with two the pointwise stage alone (70.2 / 72.1; the gate's 64-wide tiles
+//     51.1 / 43.0), with three all (65.7 / 69.0, apply 57.4 / 58.3);
+//   - six tiles per pair in all, for a launch of clusters costs about 2 us more than a plain one: 1.3 tiles (4 entries of 384, 2048
+//     tokens) gate 16.2 / 14.7, down 12.7 / 10.7; 7 to 10.7 (32 of 384) pointwise 96 / 99, gate 43 / 48, down 28.8 / 31.5.
 inline int64_t pair_tiles(int64_t batch, int64_t M) { return ceil_div(M, kPairRows) * batch; }
-inline bool pair_pays(int64_t tiles, int64_t N, int bt, int64_t K) {
-  const int64_t tn = ceil_div(N, bt);
-  return K <= kPairMaxKb * kBK && tiles * tn >= 6 * (sm_count() / 2) && tn <= sm_count() / 2;
+template <class Op>
+bool pair_pays(int64_t batch, int64_t M, int64_t N, int64_t K) {
+  if (K > kPairMaxKb * kBK || pair_ring<Op>(ceil_div(K, kBK)) < 3) return false;
+  const int64_t pairs = sm_count() / 2, tn = ceil_div(N, Op::BT), cols = Op::NACC * Op::BT, per_set = ceil_div(M, kPairRows);
+  return tn <= pairs && 7 * (pairs / tn * tn) >= 6 * pairs && 20 * per_set <= 11 * ceil_div(M, kBM) &&
+         per_set * cols * K >= (cols > 128 ? 49152 : 65536) && per_set * batch * tn >= 6 * pairs;
 }
 
 // The same launch on pairs of SMs with the weights kept in shared memory; all problems have the same K and N.
@@ -316,23 +327,13 @@ int launch_pair(const GemmArgs<Op, NPROB>& args, cudaStream_t stream, int cls, i
   LACT_CUDA(launch_pdl(kernel, dim3(2 * teams * tn), dim3(kGemmThreadsV2), smem, stream, args, nprob, ring));
   return LACT_OK;
 }
-// c = a b^T of every problem in bf16 tiles `bt` wide; `fill` as for launch_op, with B boxes of half a tile.
-template <int NPROB, class Fill>
-int launch_pair_store(int bt, Fill&& fill, cudaStream_t stream, int cls, int nprob) {
-#define LACT_PAIR_CASE(BTV)                                  \
-  case BTV: {                                                \
-    GemmArgs<OpBmmStore<BTV>, NPROB> g;                      \
-    std::memset(&g, 0, sizeof(g));                           \
-    LACT_TRY(fill(g, BTV / 2));                              \
-    return launch_pair(g, stream, cls, nprob);               \
-  }
-  switch (bt) {
-    LACT_PAIR_CASE(128)
-    LACT_PAIR_CASE(192)
-    LACT_PAIR_CASE(256)
-    default: return LACT_ERR_CONFIG;
-  }
-#undef LACT_PAIR_CASE
+// c = a b^T of every problem in bf16 tiles of Op::BT columns; `fill` as for launch_op, with B boxes of half a tile.
+template <class Op, int NPROB, class Fill>
+int launch_pair_store(Fill&& fill, cudaStream_t stream, int cls, int nprob) {
+  GemmArgs<Op, NPROB> g;
+  std::memset(&g, 0, sizeof(g));
+  LACT_TRY(fill(g, Op::BT / 2));
+  return launch_pair(g, stream, cls, nprob);
 }
 
 // Output-tile width for a single-accumulator GEMM: the candidate with the least padded work over
@@ -436,7 +437,7 @@ int launch_gate(const ApplyArgs& a, const Mat& x, const Mat& w02, int64_t len, i
   P.M = static_cast<int>(len); P.N = static_cast<int>(a.H); P.K = static_cast<int>(a.D);
   P.batch = static_cast<int>(a.B);
   g.status = status;
-  if (pair_pays(pair_tiles(a.B, len), a.H, BT, a.D)) return launch_pair(g, stream, kClsGate);
+  if (pair_pays<OpSwigluGate<BT>>(a.B, len, a.H, a.D)) return launch_pair(g, stream, kClsGate);
   return launch_gemm(g, stream, kClsGate);
 }
 
@@ -462,7 +463,9 @@ int run_apply(const ApplyArgs& a, int32_t* status, cudaStream_t stream) {
     g.status = status;
     return LACT_OK;
   };
-  if (bt >= 128 && pair_pays(pair_tiles(a.B, len), a.D, bt, a.H)) return launch_pair_store<1>(bt, fill, stream, kClsDown, 1);
+  if (bt == 256 && pair_pays<OpBmmStore<256>>(a.B, len, a.D, a.H)) return launch_pair_store<OpBmmStore<256>, 1>(fill, stream, kClsDown, 1);
+  if (bt == 192 && pair_pays<OpBmmStore<192>>(a.B, len, a.D, a.H)) return launch_pair_store<OpBmmStore<192>, 1>(fill, stream, kClsDown, 1);
+  if (bt == 128 && pair_pays<OpBmmStore<128>>(a.B, len, a.D, a.H)) return launch_pair_store<OpBmmStore<128>, 1>(fill, stream, kClsDown, 1);
   return launch_op<OpBmmStore, 1>(bt, fill, stream, kClsDown, 1);
 }
 
@@ -528,7 +531,7 @@ int run_grad_pointwise(const GradArgs& a, int32_t* status, cudaStream_t stream) 
   LACT_TRY(make_output(&P.out[1], &P.oi[1], dy2m, 0, 0));
   LACT_TRY(make_output(&P.out[2], &P.oi[2], hid, 0, 0));
   g.status = status;
-  if (pair_pays(pair_tiles(a.B, len), a.H, BT, a.D)) {
+  if (pair_pays<OpFwGradPointwise>(a.B, len, a.H, a.D)) {
     LACT_TRY(encode_map(&P.b[2], w1, 64, 32));  // a CTA's half of these columns: atoms of 32
     return launch_pair(g, stream, kClsGradPointwise);
   }

@@ -5,11 +5,28 @@ import torch.nn.functional as F
 
 pytestmark = pytest.mark.gpu
 
-# (entries, d, h, tokens): enough tiles of 256 tokens for the pairs in the batch and too few in a single entry.  Token counts at
-# the edges of a tile and of either CTA's half of it, heads whose columns end inside a tile or whose k ends inside a k-block, the
-# longest k that is kept in shared memory, two batch entries per pair and several
-CASES = [(12, 384, 384, 3329), (40, 384, 384, 1025), (48, 192, 192, 1024), (90, 192, 192, 1409), (30, 256, 256, 2048 + 127),
-         (64, 128, 256, 1560), (40, 512, 512, 1281), (60, 144, 80, 2560), (100, 64, 64, 1300), (36, 320, 208, 1152 + 255)]
+# (entries, d, h, tokens, products that go to pairs): enough tiles of 256 tokens for the pairs in the batch and too few in a single
+# entry.  Token counts at the edges of a tile and of either CTA's half of it, heads whose columns end inside a tile or whose k ends
+# inside a k-block, the longest k that is kept in shared memory, two batch entries per pair and several, a tile for every entry
+CASES = [(17, 384, 384, 3329, "gate down pointwise"), (46, 384, 384, 1153, "gate down pointwise"), (152, 192, 192, 1024, "gate down pointwise"),
+         (90, 192, 192, 1409, "gate down pointwise"), (52, 256, 256, 2048 + 127, "gate down pointwise"), (64, 128, 256, 1560, "gate down pointwise"),
+         (40, 512, 512, 1281, "gate down"), (60, 144, 80, 2560, "gate down pointwise"), (100, 64, 64, 2280, "gate pointwise"),
+         (36, 320, 208, 1152 + 255, "gate pointwise"), (230, 384, 384, 250, "gate down pointwise")]
+# calls that leave half of the second SM idle, load weights for every tile, or have column tiles that too few teams of pairs fit
+SINGLE = [(300, 384, 384, 16, ""), (300, 384, 384, 128, ""), (300, 192, 192, 384, ""), (90, 512, 512, 16, ""), (40, 128, 256, 384, ""),
+          (15, 384, 1600, 1024, ""), (9, 384, 2560, 1024, ""), (18, 512, 512, 4096, "gate down")]
+
+
+def _on_pairs(call):
+    """The products of a call that ran on pairs of SMs."""
+    from torch.profiler import ProfilerActivity, profile
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        call()
+        torch.cuda.synchronize()
+    names = [e.name for e in p.events() if "gemm_kernel" in e.name]
+    assert names
+    which = {"OpSwigluGate": "gate", "OpBmmStore": "down", "OpFwGradPointwise": "pointwise"}
+    return {which[k] for k in which for n in names if k in n and "pair_gemm" in n}
 
 
 def _inputs(b, d, h, n, seed):
@@ -25,12 +42,14 @@ def _close(got, want):
     assert float((got.double() - want).norm() / want.norm()) < 2.0 ** -7
 
 
-@pytest.mark.parametrize("b,d,h,n", CASES)
-def test_apply(b, d, h, n):
+@pytest.mark.parametrize("b,d,h,n,pairs", CASES)
+def test_apply(b, d, h, n, pairs):
     import lact_b200 as lb
     w02, w1, k, _, _ = _inputs(b, d, h, n, n)
     x = k.contiguous()
     out = lb.fused_swiglu_ffn_fwd(w02, w1, x)
+    assert _on_pairs(lambda: lb.fused_swiglu_ffn_fwd(w02, w1, x)) == set(pairs.split()) - {"pointwise"}
+    assert _on_pairs(lambda: lb.fused_swiglu_ffn_fwd(w02[:1], w1[:1], x[:1])) == set()
     for i in range(0, b, max(1, b // 4)):
         assert torch.equal(out[i], lb.fused_swiglu_ffn_fwd(w02[i:i + 1], w1[i:i + 1], x[i:i + 1])[0])
     y = x[-1].double() @ w02[-1].double().T
@@ -38,9 +57,9 @@ def test_apply(b, d, h, n):
     lb.synchronize_and_check()
 
 
-@pytest.mark.parametrize("b,d,h,n", CASES)
+@pytest.mark.parametrize("b,d,h,n,pairs", [c for c in CASES if "pointwise" in c[4]])
 @pytest.mark.parametrize("lr_dtype", [torch.float32, torch.bfloat16, None])
-def test_pointwise(b, d, h, n, lr_dtype):
+def test_pointwise(b, d, h, n, pairs, lr_dtype):
     from lact_b200 import _lib as L
     w02, w1, k, v, lr = _inputs(b, d, h, n, n + 1)
     lr = [None] * 3 if lr_dtype is None else [t.to(lr_dtype) for t in lr]
@@ -58,6 +77,7 @@ def test_pointwise(b, d, h, n, lr_dtype):
         return dy, hid
 
     dy, hid = run(slice(0, b))
+    assert _on_pairs(lambda: run(slice(0, b))) == {"pointwise"} and _on_pairs(lambda: run(slice(0, 1))) == set()
     for i in range(0, b, max(1, b // 4)):
         for got, want in zip((dy, hid), run(slice(i, i + 1))):
             assert torch.equal(got[i], want[0])
@@ -68,3 +88,13 @@ def test_pointwise(b, d, h, n, lr_dtype):
     _close(dy[-1][:, h:], 0.5 * l[2] * dh * y0 * sg)
     _close(hid[-1], 0.5 * l[1] * y0 * sg * y2)
     assert int(status[0]) == 0
+
+
+@pytest.mark.parametrize("b,d,h,n,pairs", SINGLE)
+def test_calls_that_pairs_would_slow_down(b, d, h, n, pairs):
+    import lact_b200 as lb
+    w02, w1, k, v, lr = _inputs(b, d, h, n, n + 2)
+    k, v = k.contiguous(), v.contiguous()
+    assert _on_pairs(lambda: lb.fused_swiglu_ffn_fwd(w02, w1, k)) == set(pairs.split())
+    assert _on_pairs(lambda: lb.fused_lact_swiglu_ffn_fast_weight_grads(w02, w1, k, v, *lr)) == set()
+    lb.synchronize_and_check()
