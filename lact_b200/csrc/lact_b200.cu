@@ -288,7 +288,6 @@ int launch_gemm(const GemmArgs<Op, NPROB>& args, cudaStream_t stream, int cls, i
 //     51.1 / 43.0), with three all (65.7 / 69.0, apply 57.4 / 58.3);
 //   - six tiles per pair in all, for a launch of clusters costs about 2 us more than a plain one: 1.3 tiles (4 entries of 384, 2048
 //     tokens) gate 16.2 / 14.7, down 12.7 / 10.7; 7 to 10.7 (32 of 384) pointwise 96 / 99, gate 43 / 48, down 28.8 / 31.5.
-inline int64_t pair_tiles(int64_t batch, int64_t M) { return ceil_div(M, kPairRows) * batch; }
 template <class Op>
 bool pair_pays(int64_t batch, int64_t M, int64_t N, int64_t K) {
   if (K > kPairMaxKb * kBK || pair_ring<Op>(ceil_div(K, kBK)) < 3) return false;
@@ -297,10 +296,10 @@ bool pair_pays(int64_t batch, int64_t M, int64_t N, int64_t K) {
          per_set * cols * K >= (cols > 128 ? 49152 : 65536) && per_set * batch * tn >= 6 * pairs;
 }
 
-// The same launch on pairs of SMs with the weights kept in shared memory; all problems have the same K and N.
-template <class Op, int NPROB>
-int launch_pair(const GemmArgs<Op, NPROB>& args, cudaStream_t stream, int cls, int nprob = NPROB) {
-  auto kernel = pair_gemm_kernel<Op, NPROB>;
+// The same launch on pairs of SMs with the weights kept in shared memory.
+template <class Op>
+int launch_pair(const GemmArgs<Op, 1>& args, cudaStream_t stream, int cls) {
+  auto kernel = pair_gemm_kernel<Op>;
   static std::mutex mu;
   static bool configured[64] = {false};
   int dev = 0;
@@ -312,28 +311,25 @@ int launch_pair(const GemmArgs<Op, NPROB>& args, cudaStream_t stream, int cls, i
       if (dev < 64) configured[dev] = true;
     }
   }
-  int64_t tiles = 0;
-  for (int p = 0; p < nprob; ++p) {
-    const auto& P = args.prob[p];
-    if (P.M < 1 || P.N < 1 || P.batch < 1 || P.K < 1 || P.K != args.prob[0].K || P.N != args.prob[0].N) return LACT_ERR_SHAPE;
-    tiles += pair_tiles(P.batch, P.M);
-  }
-  const int tn = ceil_div(args.prob[0].N, Op::BT), teams = static_cast<int>(std::min<int64_t>(tiles, sm_count() / 2 / tn));
+  const auto& P = args.prob[0];
+  if (P.M < 1 || P.N < 1 || P.batch < 1 || P.K < 1) return LACT_ERR_SHAPE;
+  const int64_t tiles = static_cast<int64_t>(ceil_div(P.M, kPairRows)) * P.batch;
+  const int tn = ceil_div(P.N, Op::BT), teams = static_cast<int>(std::min<int64_t>(tiles, sm_count() / 2 / tn));
   if (tiles > (1ll << 30) || teams < 1) return LACT_ERR_SHAPE;
-  const int num_kb = ceil_div(args.prob[0].K, kBK), ring = pair_ring<Op>(num_kb);
+  const int num_kb = ceil_div(P.K, kBK), ring = pair_ring<Op>(num_kb);
   if (num_kb > kPairMaxKb || ring < 2) return LACT_ERR_CONFIG;
   const size_t smem = 1024 + kPairBars + pair_panels<Op>() * kPairPanel + pair_b_bytes<Op>(num_kb) + ring * pair_stage_bytes<Op>();
   KernelScope scope(cls, stream);
-  LACT_CUDA(launch_pdl(kernel, dim3(2 * teams * tn), dim3(kGemmThreadsV2), smem, stream, args, nprob, ring));
+  LACT_CUDA(launch_pdl(kernel, dim3(2 * teams * tn), dim3(kGemmThreadsV2), smem, stream, args, ring));
   return LACT_OK;
 }
-// c = a b^T of every problem in bf16 tiles of Op::BT columns; `fill` as for launch_op, with B boxes of half a tile.
-template <class Op, int NPROB, class Fill>
-int launch_pair_store(Fill&& fill, cudaStream_t stream, int cls, int nprob) {
-  GemmArgs<Op, NPROB> g;
+// c = a b^T in bf16 tiles of Op::BT columns; `fill` as for launch_op, with B boxes of half a tile.
+template <class Op, class Fill>
+int launch_pair_store(Fill&& fill, cudaStream_t stream, int cls) {
+  GemmArgs<Op, 1> g;
   std::memset(&g, 0, sizeof(g));
   LACT_TRY(fill(g, Op::BT / 2));
-  return launch_pair(g, stream, cls, nprob);
+  return launch_pair(g, stream, cls);
 }
 
 // Output-tile width for a single-accumulator GEMM: the candidate with the least padded work over
@@ -463,9 +459,9 @@ int run_apply(const ApplyArgs& a, int32_t* status, cudaStream_t stream) {
     g.status = status;
     return LACT_OK;
   };
-  if (bt == 256 && pair_pays<OpBmmStore<256>>(a.B, len, a.D, a.H)) return launch_pair_store<OpBmmStore<256>, 1>(fill, stream, kClsDown, 1);
-  if (bt == 192 && pair_pays<OpBmmStore<192>>(a.B, len, a.D, a.H)) return launch_pair_store<OpBmmStore<192>, 1>(fill, stream, kClsDown, 1);
-  if (bt == 128 && pair_pays<OpBmmStore<128>>(a.B, len, a.D, a.H)) return launch_pair_store<OpBmmStore<128>, 1>(fill, stream, kClsDown, 1);
+  if (bt == 256 && pair_pays<OpBmmStore<256>>(a.B, len, a.D, a.H)) return launch_pair_store<OpBmmStore<256>>(fill, stream, kClsDown);
+  if (bt == 192 && pair_pays<OpBmmStore<192>>(a.B, len, a.D, a.H)) return launch_pair_store<OpBmmStore<192>>(fill, stream, kClsDown);
+  if (bt == 128 && pair_pays<OpBmmStore<128>>(a.B, len, a.D, a.H)) return launch_pair_store<OpBmmStore<128>>(fill, stream, kClsDown);
   return launch_op<OpBmmStore, 1>(bt, fill, stream, kClsDown, 1);
 }
 

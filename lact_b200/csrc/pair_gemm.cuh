@@ -76,11 +76,11 @@ __host__ __device__ constexpr int pair_ring(int num_kb) {
   return n < 0 ? 0 : static_cast<int>(n > kPairMaxRing ? kPairMaxRing : n);
 }
 
-template <class Op, int NPROB>
+template <class Op>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreadsV2, 1)
-pair_gemm_kernel(const __grid_constant__ GemmArgs<Op, NPROB> args, const int nprob, const int ring) {
+pair_gemm_kernel(const __grid_constant__ GemmArgs<Op, 1> args, const int ring) {
   using Wire = typename PairWiring<Op>::type;
-  static_assert(NPROB <= 2 && Op::KB == 1 && Op::NOUT > 0 && Op::NTERMS <= 2, "staged single-k-block ops");
+  static_assert(Op::KB == 1 && Op::NOUT > 0 && Op::NTERMS <= 2, "staged single-k-block ops");
   constexpr int BT = Op::BT, NACC = Op::NACC, NOUT = Op::NOUT, PANELS = pair_panels<Op>();
   constexpr uint32_t kAccCols = NACC * BT;
   constexpr uint32_t kTmemCols = tmem_cols_pow2(2 * kAccCols);
@@ -88,8 +88,8 @@ pair_gemm_kernel(const __grid_constant__ GemmArgs<Op, NPROB> args, const int npr
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
-  int num_kb = 0;
-  for (int p = 0; p < nprob; ++p) num_kb = max(num_kb, (args.prob[p].K + kBK - 1) / kBK);
+  const GemmProblem<Op>& P = args.prob[0];
+  const int num_kb = (P.K + kBK - 1) / kBK;
   const uint32_t b_base = base, a_base = base + pair_b_bytes<Op>(num_kb), stg = a_base + ring * pair_stage_bytes<Op>();
   uint64_t* const bars = reinterpret_cast<uint64_t*>(smem_raw + (stg - raw) + PANELS * kPairPanel);
   uint64_t* const full = bars;                         // [ring]           leader's: both CTAs' loads
@@ -116,14 +116,12 @@ pair_gemm_kernel(const __grid_constant__ GemmArgs<Op, NPROB> args, const int npr
     tmem_relinquish_pair();
   }
   if (threadIdx.x == 64) {
-    for (int p = 0; p < nprob; ++p) {
 #pragma unroll
-      for (int i = 0; i < Op::NA; ++i) tma_prefetch_desc(&args.prob[p].a[i]);
+    for (int i = 0; i < Op::NA; ++i) tma_prefetch_desc(&P.a[i]);
 #pragma unroll
-      for (int i = 0; i < Op::NB; ++i) tma_prefetch_desc(&args.prob[p].b[i]);
+    for (int i = 0; i < Op::NB; ++i) tma_prefetch_desc(&P.b[i]);
 #pragma unroll
-      for (int i = 0; i < NOUT; ++i) tma_prefetch_desc(&args.prob[p].out[i]);
-    }
+    for (int i = 0; i < NOUT; ++i) tma_prefetch_desc(&P.out[i]);
   }
   tc_fence_before();
   __syncthreads();
@@ -134,35 +132,24 @@ pair_gemm_kernel(const __grid_constant__ GemmArgs<Op, NPROB> args, const int npr
   griddep_wait();
 
   // The column tiles of one stretch of tokens belong to neighbouring pairs (a team of `tn`), which walk the same tokens at the
-  // same time: they are read from memory once, and whole rows are written together.  The stretches, problem after problem and
-  // batch entry after batch entry, are dealt to the teams in contiguous shares.
-  const int tn = (args.prob[0].N + BT - 1) / BT;
-  int tm[2], tiles_of[2] = {0, 0};
-#pragma unroll
-  for (int p = 0; p < 2; ++p) {
-    const GemmProblem<Op>& P = args.prob[p < nprob ? p : 0];
-    tm[p] = (P.M + kPairRows - 1) / kPairRows;
-    if (p < nprob) tiles_of[p] = tm[p] * P.batch;
-  }
-  const int total = tiles_of[0] + tiles_of[1];
+  // same time: they are read from memory once, and whole rows are written together.  The stretches, batch entry after batch
+  // entry, are dealt to the teams in contiguous shares.
+  const int tn = (P.N + BT - 1) / BT, tm = (P.M + kPairRows - 1) / kPairRows, total = tm * P.batch;
   const int pair = blockIdx.x >> 1, teams = (gridDim.x >> 1) / tn, team = pair / tn;
   const int t_begin = static_cast<int>(static_cast<int64_t>(total) * team / teams);
   const int t_end = static_cast<int>(static_cast<int64_t>(total) * (team + 1) / teams);
   const int n0 = (pair - team * tn) * BT;
-  struct Run { int prob, batch, m; };
+  struct Run { int batch, m; };
   auto locate = [&](int tile) {
     Run r;
     if constexpr (Op::kReverseBatch) tile = total - 1 - tile;
-    r.prob = tile >= tiles_of[0] ? 1 : 0;
-    const int t = r.prob ? tile - tiles_of[0] : tile, per = r.prob ? tm[1] : tm[0];
-    r.batch = t / per;
-    r.m = t - r.batch * per;
+    r.batch = tile / tm;
+    r.m = tile - r.batch * tm;
     return r;
   };
   // first / last tile of a stretch over the same weights
-  auto begins = [&](const Run& r) { return r.m == (Op::kReverseBatch ? (r.prob ? tm[1] : tm[0]) - 1 : 0); };
-  auto ends = [&](const Run& r) { return r.m == (Op::kReverseBatch ? 0 : (r.prob ? tm[1] : tm[0]) - 1); };
-  auto problem = [&](const Run& r) -> const GemmProblem<Op>& { return args.prob[NPROB > 1 ? r.prob : 0]; };
+  auto begins = [&](const Run& r) { return r.m == (Op::kReverseBatch ? tm - 1 : 0); };
+  auto ends = [&](const Run& r) { return r.m == (Op::kReverseBatch ? 0 : tm - 1); };
   // (the CTAs of a pair may differ: every wait for the other has a limit)
   bool failed = earlier_launch_failed(args.status);
   const bool work = !failed;
@@ -179,8 +166,6 @@ pair_gemm_kernel(const __grid_constant__ GemmArgs<Op, NPROB> args, const int npr
     for (int tile = t_begin; tile < t_end && !failed; ++tile) {
       const Run r = locate(tile);
       const bool first = tile == t_begin || begins(r);
-      const GemmProblem<Op>& P = problem(r);
-      const int nkb = (P.K + kBK - 1) / kBK;
       // coordinates of this tile's boxes, per term; one k-block on per stage
       int a_row[Op::NTERMS], a_batch[Op::NTERMS], a_k[Op::NTERMS], b_mn[Op::NTERMS], b_batch[Op::NTERMS], b_k[Op::NTERMS];
       bool b_major[Op::NTERMS];
@@ -196,7 +181,7 @@ pair_gemm_kernel(const __grid_constant__ GemmArgs<Op, NPROB> args, const int npr
         b_k[t] = bi.k_off;
         b_major[t] = bi.mn_major != 0;
       }
-      for (int kb = 0; kb < nkb; ++kb) {
+      for (int kb = 0; kb < num_kb; ++kb) {
         if (first) {
           if (!mbar_wait_warp(&b_empty[kb], bph ^ 1, abort_flag)) { failed = true; break; }
           mbar_expect_tx_if(signaller, &b_full[kb], 2 * b_bytes);
@@ -243,8 +228,6 @@ pair_gemm_kernel(const __grid_constant__ GemmArgs<Op, NPROB> args, const int npr
       for (int tile = t_begin; tile < t_end && !failed; ++tile, ++n) {
         const Run r = locate(tile);
         const bool first = tile == t_begin || begins(r), last = tile == t_end - 1 || ends(r);
-        const GemmProblem<Op>& P = problem(r);
-        const int nkb = (P.K + kBK - 1) / kBK;
         const uint32_t as = n & 1;
         const uint32_t acc = tmem + as * kAccCols;
         if (!mbar_wait_warp(&acc_empty[as], ((n >> 1) & 1) ^ 1, abort_flag)) { failed = true; break; }
@@ -257,7 +240,7 @@ pair_gemm_kernel(const __grid_constant__ GemmArgs<Op, NPROB> args, const int npr
           idesc[t] = make_idesc_bf16(kPairRows, Op::term_n(t), 0, b_mn);
           step_b[t] = half_atom ? 64 : (b_mn ? 128 : 2);  // 16 k-rows of 64 or 128 bytes, or 32 bytes inside a row
         }
-        for (int kb = 0; kb < nkb; ++kb) {
+        for (int kb = 0; kb < num_kb; ++kb) {
           if (first && !mbar_wait_warp(&b_full[kb], bph, abort_flag)) { failed = true; break; }
           if (!mbar_wait_warp(&full[s], ph, abort_flag)) { failed = true; break; }
           tc_fence_after();
@@ -290,13 +273,11 @@ pair_gemm_kernel(const __grid_constant__ GemmArgs<Op, NPROB> args, const int npr
     auto fetch = [&](int tile) {
       if (tile >= t_end) return;
       const Run r = locate(tile);
-      const GemmProblem<Op>& P = problem(r);
       Op::prefetch(P.ep, r.batch, r.m * kPairRows + static_cast<int>(rank) * kBM + row_local, n0, half, P.M, P.N, pf_next);
     };
     fetch(t_begin);
     for (int tile = t_begin; tile < t_end && !stop; ++tile, ++n) {
       const Run r = locate(tile);
-      const GemmProblem<Op>& P = problem(r);
       const int m0 = r.m * kPairRows + static_cast<int>(rank) * kBM, row = m0 + row_local;
       const uint32_t as = n & 1;
       typename Op::Prefetch pf = pf_next;
