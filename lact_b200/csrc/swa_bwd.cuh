@@ -52,6 +52,19 @@ struct SwaBwdSmem {
   static constexpr uint32_t kBytes = kBars + 256;
 };
 
+// Packed sequences: the end of the sequence that holds `row`, at most `limit` (> row); the same answer in all lanes of a full warp.
+// (seq_start never falls; 32 places are looked at together: 3 rounds for 2048 of them.)
+__device__ __forceinline__ int sequence_end(const int32_t* seq_start, int row, int limit) {
+  int lo = row, hi = limit;   // the end is in (lo, hi]
+  while (hi - lo > 1) {
+    const int step = (hi - lo + 31) >> 5, at = lo + (static_cast<int>(threadIdx.x & 31) + 1) * step;
+    const int f = __ffs(__ballot_sync(0xFFFFFFFFu, at >= hi || seq_start[at] > row)) - 1;
+    hi = min(hi, lo + (f + 1) * step);
+    lo += f * step;
+  }
+  return hi;
+}
+
 template <int HD, int MODE>
 __global__ void __launch_bounds__(kSwaBwdThreads, 1) swa_bwd_kernel(const __grid_constant__ SwaBwdArgs a) {
   static_assert(HD == 64 || HD == 128, "head dimensions 64 and 128");
@@ -106,22 +119,18 @@ __global__ void __launch_bounds__(kSwaBwdThreads, 1) swa_bwd_kernel(const __grid
   const int batch = blockIdx.x / (a.tiles * a.heads);
   const int o0 = ot * 128;   // first row of the outer tile (keys in mode 0, queries in mode 1)
   const int window = a.window > 0 ? a.window : a.L;
-  // inner 128-row tiles [t_lo, t_hi]
-  int t_lo, t_hi;
-  if (MODE == 0) {   // queries that see any key of this tile: q >= key, q <= key + window - 1
-    t_lo = o0 / 128;
-    const int64_t q_max = static_cast<int64_t>(o0) + 127 + window - 1;
-    t_hi = static_cast<int>(q_max < a.L - 1 ? q_max : a.L - 1) / 128;
-    if (!a.causal) t_lo = 0, t_hi = (a.L - 1) / 128;   // block attention: every query tile
-  } else {           // keys this query tile sees: not before the window of its first query, nor before that query's sequence
-    int lo = o0 - (window - 1);
-    if (lo < 0) lo = 0;
-    if (a.seq_start != nullptr && a.seq_start[o0] > lo) lo = a.seq_start[o0];
-    t_lo = lo / 128;
-    t_hi = (o0 + 127 < a.L - 1 ? o0 + 127 : a.L - 1) / 128;
-    if (!a.causal) t_lo = 0, t_hi = (a.Lk - 1) / 128;  // every key tile
+  // inner rows [i_lo, i_hi] that any row of this tile meets, in 128-row tiles from t_lo
+  int i_lo = 0, i_hi = (MODE == 0 ? a.L : a.Lk) - 1;   // block attention: all
+  if (a.causal && MODE == 0) {   // queries that see any key of this tile: key <= q <= key + window - 1, of the key's sequence
+    const int64_t past = static_cast<int64_t>(o0) + 127 + window;
+    i_lo = o0;
+    if (past <= i_hi) i_hi = static_cast<int>(past) - 1;
+    if (a.seq_start != nullptr) i_hi = sequence_end(a.seq_start, min(o0 + 127, a.L - 1), i_hi + 1) - 1;
+  } else if (a.causal) {         // keys this query tile sees: not before the window of its first query, nor before that query's sequence
+    i_lo = max(o0 - (window - 1), a.seq_start != nullptr ? a.seq_start[o0] : 0);
+    if (o0 + 127 < i_hi) i_hi = o0 + 127;
   }
-  const int T = t_hi - t_lo + 1;
+  const int t_lo = i_lo / 128, T = i_hi / 128 - t_lo + 1;
   // (swizzled tiles need the alignment asked for above)
   bool failed = uniform(static_cast<uint32_t>(*reinterpret_cast<volatile int32_t*>(a.status))) != kStatusOk || (base & 1023u) != 0;
   const CUtensorMap* outer_a = MODE == 0 ? &a.k : &a.q;          // outer pair: (K, V) or (Q, dO)
@@ -257,19 +266,26 @@ __global__ void __launch_bounds__(kSwaBwdThreads, 1) swa_bwd_kernel(const __grid
       delta_r = a.delta[stat_base + row] * a.scale;
       if (a.seq_start != nullptr) row_start = a.seq_start[row];
     }
-    // first / last inner row that this outer row meets: mode 0, queries row .. row + window - 1; mode 1, the keys of its window
-    // and sequence.  (The bounds once per thread: tests of every pair took 8500 clocks in each of the two tiles of a band
-    // that are cut by it, a quarter of the kernel at a window of 2048.)
-    int in_lo, in_hi;
-    if (MODE == 0) {
+    // first / last inner row that this outer row meets: mode 0, queries row .. row + window - 1 of its sequence; mode 1, the keys of
+    // its window and sequence.  (The bounds once per thread: tests of every pair took 8500 clocks in each of the two tiles of a
+    // band that are cut by it, a quarter of the kernel at a window of 2048.)
+    int in_lo = 0, in_hi = -1;
+    if (MODE == 0 && row < a.Lk) {
       const int64_t last = a.causal ? static_cast<int64_t>(row) + window - 1 : a.L - 1;
       in_lo = a.causal ? row : 0;
-      in_hi = row < a.Lk ? static_cast<int>(last < a.L - 1 ? last : a.L - 1) : -1;
-    } else {
-      in_lo = a.causal ? (row - (window - 1) > row_start ? row - (window - 1) : row_start) : 0;
-      in_hi = row < a.L ? (a.causal ? row : a.Lk - 1) : -1;
+      in_hi = static_cast<int>(last < a.L - 1 ? last : a.L - 1);
+    } else if (MODE == 1 && row < a.L) {
+      in_lo = a.causal ? max(row - (window - 1), row_start) : 0;
+      in_hi = a.causal ? row : a.Lk - 1;
     }
-    const int outer_start = MODE == 1 && a.seq_start != nullptr ? a.seq_start[o0 + 127 < a.L ? o0 + 127 : a.L - 1] : 0;
+    if (MODE == 0 && a.seq_start != nullptr) {   // sequence after sequence of this warp's 32 keys
+      const int first = o0 + quarter * 32;
+      const int limit = static_cast<int>(min(static_cast<int64_t>(a.L), static_cast<int64_t>(first) + 31 + window));
+      for (int end = min(first, a.L); __any_sync(0xFFFFFFFFu, end <= row && row < a.L);) {
+        end = sequence_end(a.seq_start, end, limit);
+        if (row < end && in_hi >= end) in_hi = end - 1;
+      }
+    }
     for (int t = 0; t < T && !failed; ++t) {
       const int i0 = (t_lo + t) * 128, set = MODE == 0 ? 0 : t & 1;
       const float* st = stats + (t & 1) * 256 + c0;
@@ -281,15 +297,8 @@ __global__ void __launch_bounds__(kSwaBwdThreads, 1) swa_bwd_kernel(const __grid
       tc_fence_after();
       uint32_t bits[32];
       tmem_ld32(tmem + lane_off + set * 128 + c0, bits);
-      bool interior;   // every (row, column) pair of the tile visible: no masks
-      if (MODE == 0) {
-        const int tile_start = a.seq_start != nullptr ? a.seq_start[i0 + 127 < a.L ? i0 + 127 : a.L - 1] : 0;
-        interior = a.causal ? (o0 + 127 <= i0 && o0 >= i0 + 127 - (window - 1) && i0 + 127 < a.L && o0 >= tile_start)
-                            : (i0 + 127 < a.L && o0 + 127 < a.Lk);
-      } else {
-        interior = a.causal ? (i0 + 127 <= o0 && i0 >= o0 + 127 - (window - 1) && o0 + 127 < a.L && i0 >= outer_start)
-                            : (i0 + 127 < a.Lk && o0 + 127 < a.L);
-      }
+      const int lo = in_lo - i0 - c0, hi = in_hi - i0 - c0;          // this row's share of the warp's 32 columns
+      const bool interior = __all_sync(0xFFFFFFFFu, lo <= 0 && hi >= 31);   // every pair visible: no masks
       tmem_ld_wait();
       // p = 2^(s c - lse)
       float p[32];
@@ -304,15 +313,9 @@ __global__ void __launch_bounds__(kSwaBwdThreads, 1) swa_bwd_kernel(const __grid
         for (int e = 0; e < 4; ++e) p[g * 4 + e] = exp2_ftz(fmaf(__uint_as_float(bits[g * 4 + e]), a.scale_log2, -lv[e]));
       }
       if (!interior) {
-        const int lo = in_lo - i0 - c0, hi = in_hi - i0 - c0;
 #pragma unroll
         for (int j = 0; j < 32; ++j)
           if (j < lo || j > hi) p[j] = 0.f;
-        if (MODE == 0 && a.seq_start != nullptr) {   // queries of a later sequence do not see this key
-#pragma unroll
-          for (int j = 0; j < 32; ++j)
-            if (row < a.seq_start[min(i0 + c0 + j, a.L - 1)]) p[j] = 0.f;
-        }
       }
       uint32_t w[16];
       if (MODE == 0) {

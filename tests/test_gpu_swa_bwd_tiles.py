@@ -12,14 +12,30 @@ pytestmark = pytest.mark.gpu
                                                (1, 641, 641, 2, 128, 255), (1, 900, 900, 1, 64, 2000), (1, 1, 300, 2, 128, -1),
                                                (2, 130, 127, 2, 64, -1), (1, 256, 513, 1, 128, -1), (1, 500, 1, 2, 128, -1)])
 def test_gradients(b, l, lk, h, d, window):
+    _check(b, l, lk, h, d, window)
+
+
+# sequences packed back to back: many in a tile and one over many, ends on, before and after the edges of tiles and of the 32 rows
+# of a warp, windows shorter and longer than a sequence
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("window", [0, 1, 40, 128, 700])
+@pytest.mark.parametrize("lengths", [(1, 30, 1, 2, 94, 128, 129, 127, 300), (640,), (5,) * 70, (1000, 3, 29, 1, 31), (257, 511)])
+def test_gradients_of_packed_sequences(d, window, lengths):
+    _check(1, sum(lengths), sum(lengths), 2, d, window, lengths)
+
+
+def _check(b, l, lk, h, d, window, lengths=None):
     from lact_b200 import _lib as L
     g = torch.Generator(device="cuda").manual_seed(l * 7 + lk)
     rn = lambda n: torch.randn(b, n, h, d, device="cuda", generator=g).to(torch.bfloat16)
     q, k, v, do = rn(l), rn(lk), rn(lk), rn(l)
     ref = [t.double().transpose(1, 2).requires_grad_(True) for t in (q, k, v)]
-    s = ref[0] @ ref[1].transpose(2, 3) * d ** -0.5
+    s, start = ref[0] @ ref[1].transpose(2, 3) * d ** -0.5, None
     if window >= 0:
         i, j = torch.arange(l, device="cuda")[:, None], torch.arange(lk, device="cuda")[None]
+        if lengths is not None:
+            start = torch.cat([torch.full((n,), sum(lengths[:m]), device="cuda") for m, n in enumerate(lengths)]).int()
+            s = s.masked_fill(j < start[:, None], float("-inf"))
         s = s.masked_fill((j > i) | ((j <= i - window) if window > 0 else torch.zeros_like(j > i)), float("-inf"))
     out = s.softmax(-1) @ ref[2]
     want = [t.transpose(1, 2) for t in torch.autograd.grad(out, ref, do.double().transpose(1, 2))]
@@ -31,7 +47,7 @@ def test_gradients(b, l, lk, h, d, window):
     st = lambda t: (h * d, t.shape[1] * h * d)   # contiguous (strides of length-one axes are anything)
     L.check(L.lib().lact_swa_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr(), lse.data_ptr(), dq.data_ptr(),
                                  dk.data_ptr(), dv.data_ptr(), delta.data_ptr(), b, l, lk, h, d, *st(q), *st(k), *st(v), *st(o), *st(do),
-                                 window, d ** -0.5, None, status.data_ptr(), L.stream_ptr()), "bwd")
+                                 window, d ** -0.5, start.data_ptr() if lengths is not None else None, status.data_ptr(), L.stream_ptr()), "bwd")
     torch.cuda.synchronize()
     assert int(status[0]) == 0
     for got, w, like in zip((dq, dk, dv), want, (q, k, v)):
