@@ -2620,6 +2620,10 @@ int lact_swa_bwd(const void* q, const void* k, const void* v, const void* o, con
   LACT_TRY(encode_map_heads(&a.k, k, b, lk, n_heads, d, k_ts, k_bs));
   LACT_TRY(encode_map_heads(&a.v, v, b, lk, n_heads, d, v_ts, v_bs));
   LACT_TRY(encode_map_heads(&a.dout, dout, b, l, n_heads, d, do_ts, do_bs));
+  LACT_TRY(encode_map_heads(&a.q16, q, b, l, n_heads, d, q_ts, q_bs, 16));
+  LACT_TRY(encode_map_heads(&a.k16, k, b, lk, n_heads, d, k_ts, k_bs, 16));
+  LACT_TRY(encode_map_heads(&a.v16, v, b, lk, n_heads, d, v_ts, v_bs, 16));
+  LACT_TRY(encode_map_heads(&a.dout16, dout, b, l, n_heads, d, do_ts, do_bs, 16));
   a.lse = static_cast<const float*>(lse);
   a.delta = static_cast<const float*>(delta);
   a.seq_start = seq_start;

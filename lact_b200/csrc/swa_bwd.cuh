@@ -27,6 +27,7 @@ namespace lact {
 
 struct SwaBwdArgs {
   CUtensorMap q, k, v, dout;           // 4-D maps (feature, token, head, batch), box {64, 128, 1, 1}
+  CUtensorMap q16, k16, v16, dout16;   // the same, box {64, 16, 1, 1}
   const float* lse;            // [b][h][l]: log2-domain log-sum-exp of the forward (m + log2(l))
   const float* delta;          // [b][h][l]: sum_d dO O
   const int32_t* seq_start;    // optional [l], as in the forward
@@ -146,6 +147,21 @@ __global__ void __launch_bounds__(kSwaBwdThreads, 1) swa_bwd_kernel(const __grid
       auto load = [&](uint32_t dst, const CUtensorMap* map, uint64_t* bar, int row) {
         for (int j = 0; j < KBD; ++j) tma_load_4d_if(leader, dst + j * kBox, map, bar, 64 * j, row, head, batch);
       };
+      // Groups of 16 inner rows that no row of the outer tile meets arrive as zeros (from behind the tensor's end): their
+      // probabilities are zero, but a NaN or an infinity in such a row would reach all rows of the tile, up to 127 past the band.
+      const int rows = MODE == 0 ? a.L : a.Lk;
+      auto load_inner = [&](uint32_t dst, const CUtensorMap* map, const CUtensorMap* map16, uint64_t* bar, int t) {
+        const int row = (t_lo + t) * 128;
+        if (row + 15 >= i_lo && (row + 112 <= i_hi || i_hi == rows - 1)) {
+          load(dst, map, bar, row);
+        } else {
+#pragma unroll 1
+          for (int g = 0; g < 128; g += 16) {
+            const int from = row + g + 15 < i_lo || row + g > i_hi ? rows : row + g;
+            for (int j = 0; j < KBD; ++j) tma_load_4d_if(leader, dst + j * kBox + g * 128, map16, bar, 64 * j, from, head, batch);
+          }
+        }
+      };
       mbar_expect_tx_if(leader, outer_full, 2 * SM::kTile);
       load(base + SM::kOuter, outer_a, outer_full, o0);
       load(base + SM::kOuter + SM::kTile, outer_b, outer_full, o0);
@@ -153,10 +169,10 @@ __global__ void __launch_bounds__(kSwaBwdThreads, 1) swa_bwd_kernel(const __grid
         const int sa = t % NA, sb = t % NB;
         if (t >= NA && !mbar_wait_warp(&a_empty[sa], (t / NA - 1) & 1, abort_flag)) { failed = true; break; }
         mbar_expect_tx_if(leader, &a_full[sa], SM::kTile);
-        load(base + SM::kA + sa * SM::kTile, inner_a, &a_full[sa], (t_lo + t) * 128);
+        load_inner(base + SM::kA + sa * SM::kTile, inner_a, MODE == 0 ? &a.q16 : &a.k16, &a_full[sa], t);
         if (t >= NB && !mbar_wait_warp(&b_empty[sb], (t / NB - 1) & 1, abort_flag)) { failed = true; break; }
         mbar_expect_tx_if(leader, &b_full[sb], SM::kTile);
-        load(base + SM::kB + sb * SM::kTile, inner_b, &b_full[sb], (t_lo + t) * 128);
+        load_inner(base + SM::kB + sb * SM::kTile, inner_b, MODE == 0 ? &a.dout16 : &a.v16, &b_full[sb], t);
       }
     }
   } else if (warp == 1) {
@@ -228,13 +244,14 @@ __global__ void __launch_bounds__(kSwaBwdThreads, 1) swa_bwd_kernel(const __grid
     // its way back: the softmax warps may be two tiles past this warp (their tile t - 1 needs nothing more from it), and a wait by
     // parity on a barrier that completes once per tile, such as ds_full, would then stand for a tile that waits for this warp.
     if (MODE == 0) {
+      // (queries that no key of the tile meets have values like those behind the end: theirs need not be finite)
       float x[8];   // lse and delta of queries lane, lane + 32, ...
       auto fetch = [&](int t) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const int qi = (t_lo + t) * 128 + lane + 32 * i;
-          x[i] = qi < a.L ? a.lse[stat_base + qi] : INFINITY;
-          x[4 + i] = qi < a.L ? a.delta[stat_base + qi] : 0.f;
+          x[i] = qi <= i_hi ? a.lse[stat_base + qi] : INFINITY;
+          x[4 + i] = qi <= i_hi ? a.delta[stat_base + qi] : 0.f;
         }
       };
       if (!failed) fetch(0);
