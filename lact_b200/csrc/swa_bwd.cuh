@@ -312,10 +312,39 @@ __global__ void __launch_bounds__(kSwaBwdThreads, 1) swa_bwd_kernel(const __grid
         break;
       }
       tc_fence_after();
-      uint32_t bits[32];
-      tmem_ld32(tmem + lane_off + set * 128 + c0, bits);
       const int lo = in_lo - i0 - c0, hi = in_hi - i0 - c0;          // this row's share of the warp's 32 columns
       const bool interior = __all_sync(0xFFFFFFFFu, lo <= 0 && hi >= 31);   // every pair visible: no masks
+      if (!__any_sync(0xFFFFFFFFu, lo <= 31 && hi >= 0)) {
+        // None is: zeros without the exponentials.  (Tiles of 128 rows are mostly that where sequences or windows are short: 16384
+        // tokens, window 64, 85.1 -> 76.9 and 66.6 -> 60.5 us, 64 sequences of 64 tokens 27.8 -> 24.8 and 23.9 -> 21.2.  As a case
+        // of the code below instead of a path of its own it took 640 and 438 us instead of 624 and 419 for 32768 tokens of 64.)
+        uint32_t zero[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) zero[j] = 0;
+        if (MODE == 0) {
+          tmem_st16(tmem + lane_off + c0, zero);
+          tmem_st_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(p_full);
+        }
+        if (!mbar_wait_warp(dp_full, t & 1, abort_flag)) {
+          failed = true;
+          break;
+        }
+        tc_fence_after();
+        tmem_st16(tmem + lane_off + (MODE == 0 ? kDP : set * 128u) + c0, zero);
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive(ds_full);
+          if (MODE == 0) mbar_arrive(&st_empty[t & 1]);
+        }
+        continue;
+      }
+      uint32_t bits[32];
+      tmem_ld32(tmem + lane_off + set * 128 + c0, bits);
       tmem_ld_wait();
       // p = 2^(s c - lse)
       float p[32];
