@@ -1,4 +1,6 @@
 """Token x weight products on pairs of SMs: the same bits as the one-SM kernel gives entry by entry, and the fp32 reference."""
+import ctypes as C
+
 import pytest
 import torch
 import torch.nn.functional as F
@@ -98,3 +100,29 @@ def test_calls_that_pairs_would_slow_down(b, d, h, n, pairs):
     assert _on_pairs(lambda: lb.fused_swiglu_ffn_fwd(w02, w1, k)) == set(pairs.split())
     assert _on_pairs(lambda: lb.fused_lact_swiglu_ffn_fast_weight_grads(w02, w1, k, v, *lr)) == set()
     lb.synchronize_and_check()
+
+
+def _products(w02, w1, k, v, lr, status):
+    """Apply and the pointwise stage through the C interface with a status word; the outputs, filled with -7 before."""
+    from lact_b200 import _lib as L
+    b, n, d = k.shape
+    h = w1.shape[2]
+    out, hidden, hid = (torch.full((b, n, w), -7.0, dtype=torch.bfloat16, device="cuda") for w in (d, h, h))
+    dy = torch.full((b, n, 2 * h), -7.0, dtype=torch.bfloat16, device="cuda")
+    ptr = lambda t: C.c_void_p(t.data_ptr())
+    L.check(L.lib().lact_swiglu_ffn_apply(ptr(w02), ptr(w1), ptr(k), ptr(out), ptr(hidden), *map(C.c_int64, (b, n, d, h)), ptr(status),
+                                          C.c_void_p(L.stream_ptr())), "apply")
+    L.check(L.lib().lact_fw_grad_pointwise(w02.data_ptr(), w1.data_ptr(), k.data_ptr(), d, d * n, v.data_ptr(), d, d * n,
+                                           *[t.data_ptr() for t in lr], 0, n, 0.5, dy.data_ptr(), hid.data_ptr(), b, n, d, h,
+                                           status.data_ptr(), L.stream_ptr()), "pointwise")
+    torch.cuda.synchronize()
+    return out, hidden, dy, hid
+
+
+def test_after_an_earlier_failure_nothing_is_written():
+    w02, w1, k, v, lr = _inputs(46, 384, 384, 1153, 3)
+    k, v = k.contiguous(), v.contiguous()
+    word = lambda x: torch.full((64,), x, dtype=torch.int32, device="cuda")
+    assert _on_pairs(lambda: _products(w02, w1, k, v, lr, word(0))) == {"gate", "down", "pointwise"}
+    status = word(101)
+    assert all(bool((t == -7).all()) for t in _products(w02, w1, k, v, lr, status)) and int(status[0]) == 101
