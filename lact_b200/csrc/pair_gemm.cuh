@@ -17,7 +17,7 @@
 // the same program: warp 0 loads the CTA's own operands, warps 2-9 are its epilogue; warp 1 of the leader (rank 0) issues the
 // products of both.  Full barriers live in the leader's shared memory (both CTAs' loads complete there), every other barrier
 // in both, signalled by multicast commits.  All mbarrier waits are bounded; the cluster barriers at either end are reached by
-// every thread whatever its waits returned.
+// every thread whatever its waits returned, and no commit is still on its way then.
 #pragma once
 #include "ops.cuh"
 

@@ -17,9 +17,10 @@
 //   mode 1  ... dP(t + 1), dQ(t), S(t + 2) ...          S has two sets of columns, dP one
 // The first inner operand (Q or K) is held from its first product to the second products a tile later and goes through a
 // three-stage ring, the other through two stages.  Every mbarrier wait is bounded.
-// Measured (2 x 32768 tokens, 12 heads of 128, window 2048; 128 x 128 pairs): keys' side 1514 us, queries' side 1079, where
-// 64-row inner tiles with P and dS in shared memory took 1712 and 1287.  About 2900 and 2350 clocks a tile for 2050 and 1540 of
-// products; 1030 of them are exponentials (16 a clock), which no other phase of the same tile can hide.
+// Measured (2 x 32768 tokens, 12 heads of 128, window 2048; 128 x 128 pairs): keys' side 1469 us, queries' side 1059, where
+// 64-row inner tiles with P and dS in shared memory took 1698 and 1288.  About 2800 and 2300 clocks a tile for 2050 and 1540 of
+// products; 1030 of them are exponentials (16 a clock), which no other phase of the same tile can hide.  One tile of 64 tokens is
+// where the old tiles stay ahead on the queries' side (64 x 8 heads: 21.3 / 18.5, keys' side 24.8 / 24.9).
 #pragma once
 #include "swa.cuh"
 
