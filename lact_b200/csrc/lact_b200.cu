@@ -45,6 +45,7 @@ EncodeFn get_encode_fn() {
 struct Mat {
   const void* ptr;
   int64_t rows, cols, ld, batch, bs;  // ld / bs: row / batch stride in elements
+  int64_t segs = 1, ss = 0;           // segments (ops with `kSegments`) and their stride
 };
 
 // Encodes a 3-D map (cols, rows, batch) with a {64, box_rows, 1} box and 128-byte swizzle, or a {32, box_rows, 1} box and
@@ -88,21 +89,47 @@ int encode_map_kblocks(CUtensorMap* map, const Mat& m, uint32_t box_rows, uint32
   return r == CUDA_SUCCESS ? LACT_OK : LACT_ERR_CUDA;
 }
 
-template <class Op>
-constexpr int kb_of(const GemmProblem<Op>&) { return Op::KB; }
+// As encode_map with a fourth axis, the segments (ops with `kSegments`).
+int encode_map_segments(CUtensorMap* map, const Mat& m, uint32_t box_rows) {
+  EncodeFn fn = get_encode_fn();
+  if (fn == nullptr) return LACT_ERR_CUDA;
+  if ((reinterpret_cast<uintptr_t>(m.ptr) & 15) != 0 || (m.ld % 8) != 0 || (m.batch > 1 && (m.bs % 8) != 0) ||
+      (m.segs > 1 && (m.ss % 8) != 0))
+    return LACT_ERR_SHAPE;
+  if (m.rows < 1 || m.cols < 1 || m.batch < 1 || m.segs < 1 || box_rows > 256) return LACT_ERR_SHAPE;
+  cuuint64_t dims[4] = {static_cast<cuuint64_t>(m.cols), static_cast<cuuint64_t>(m.rows), static_cast<cuuint64_t>(m.batch),
+                        static_cast<cuuint64_t>(m.segs)};
+  const int64_t bs = m.batch > 1 ? m.bs : m.ld * m.rows, ss = m.segs > 1 ? m.ss : bs;
+  cuuint64_t strides[3] = {static_cast<cuuint64_t>(m.ld) * 2, static_cast<cuuint64_t>(bs) * 2, static_cast<cuuint64_t>(ss) * 2};
+  cuuint32_t box[4] = {64, box_rows, 1, 1};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(m.ptr), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? LACT_OK : LACT_ERR_CUDA;
+}
 
-// Operand of a GEMM: `m` used K-major (mn = rows, k = cols) or MN-major (k = rows, mn = cols); `kb` =
-// k-blocks per ring stage of the op that reads it.  With two k-blocks per stage a K-major operand
+// What the maps of a problem's operands depend on: k-blocks per ring stage, and whether there is a segment axis.
+struct OperandForm {
+  int kb;
+  bool segments;
+};
+template <class Op>
+constexpr OperandForm form_of(const GemmProblem<Op>&) { return OperandForm{Op::KB, op_segments<Op>::value}; }
+
+// Operand of a GEMM: `m` used K-major (mn = rows, k = cols) or MN-major (k = rows, mn = cols).  With two k-blocks per stage a K-major operand
 // whose k extent is whole k-blocks gets the 4-D map (one box per stage), an MN-major operand a box of
 // 128 k rows per 64-wide atom.
-int make_operand(int kb, CUtensorMap* map, OperandInfo* info, const Mat& m, int mn_major, int tile_rows, int mn_off,
+int make_operand(OperandForm form, CUtensorMap* map, OperandInfo* info, const Mat& m, int mn_major, int tile_rows, int mn_off,
                  int k_off, int batch_off = 0) {
   info->mn_major = mn_major;
   info->k4d = 0;
   info->mn_off = mn_off;
   info->k_off = k_off;
   info->batch_off = batch_off;
+  const int kb = form.kb;
   if (((mn_major ? mn_off : k_off) % 8) != 0) return LACT_ERR_SHAPE;  // innermost TMA coordinate: 16-byte rule
+  if (form.segments) return encode_map_segments(map, m, static_cast<uint32_t>(mn_major ? 64 * kb : tile_rows));
   if (mn_major) return encode_map(map, m, static_cast<uint32_t>(64 * kb));
   if (kb == 2 && (m.cols % 64) == 0 && (k_off % 64) == 0) {
     info->k4d = 1;
@@ -112,13 +139,13 @@ int make_operand(int kb, CUtensorMap* map, OperandInfo* info, const Mat& m, int 
 }
 
 // Output of a staged epilogue: bf16 matrix `m` whose extents clip the stored tiles.
-int make_output(CUtensorMap* map, OutInfo* info, const Mat& m, int row_off, int col_off, int batch_off = 0) {
+int make_output(OperandForm form, CUtensorMap* map, OutInfo* info, const Mat& m, int row_off, int col_off, int batch_off = 0) {
   info->row_off = row_off;
   info->col_off = col_off;
   info->batch_off = batch_off;
   info->enabled = 1;
   if ((col_off % 8) != 0 || row_off < 0 || col_off < 0) return LACT_ERR_SHAPE;
-  return encode_map(map, m, kBM);
+  return form.segments ? encode_map_segments(map, m, kBM) : encode_map(map, m, kBM);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -416,8 +443,11 @@ struct ApplyArgs {
   void* out;           // [B][*][D] bf16
   int64_t o_bs, o_ts;
   int64_t out_start;
-  bf16* hidden;  // scratch [B][end-start][H]
+  bf16* hidden;  // scratch [segments][B][end-start][H]
   int64_t B, D, H;
+  // Several ranges of one length at once ("segments"), each with its own weights: segment i reads tokens from start + i x_step,
+  // writes from out_start + i o_step and takes its weights w_step elements on.
+  int64_t segs = 1, x_step = 0, o_step = 0, w_step = 0;
 };
 
 template <int BT>
@@ -425,43 +455,47 @@ int launch_gate(const ApplyArgs& a, const Mat& x, const Mat& w02, int64_t len, i
   GemmArgs<OpSwigluGate<BT>, 1> g;
   std::memset(&g, 0, sizeof(g));
   auto& P = g.prob[0];
-  LACT_TRY(make_operand(kb_of(P), &P.a[0], &P.ai[0], x, 0, kBM, static_cast<int>(a.start), 0));
-  LACT_TRY(make_operand(kb_of(P), &P.b[0], &P.bi[0], w02, 0, BT, 0, 0));
-  LACT_TRY(make_operand(kb_of(P), &P.b[1], &P.bi[1], w02, 0, BT, static_cast<int>(a.H), 0));
-  const Mat hid{a.hidden, len, a.H, a.H, a.B, len * a.H};
-  LACT_TRY(make_output(&P.out[0], &P.oi[0], hid, 0, 0));
+  LACT_TRY(make_operand(form_of(P), &P.a[0], &P.ai[0], x, 0, kBM, 0, 0));
+  LACT_TRY(make_operand(form_of(P), &P.b[0], &P.bi[0], w02, 0, BT, 0, 0));
+  LACT_TRY(make_operand(form_of(P), &P.b[1], &P.bi[1], w02, 0, BT, static_cast<int>(a.H), 0));
+  const Mat hid{a.hidden, len, a.H, a.H, a.B, len * a.H, a.segs, a.B * len * a.H};
+  LACT_TRY(make_output(form_of(P), &P.out[0], &P.oi[0], hid, 0, 0));
   P.M = static_cast<int>(len); P.N = static_cast<int>(a.H); P.K = static_cast<int>(a.D);
-  P.batch = static_cast<int>(a.B);
+  P.batch = static_cast<int>(a.segs * a.B);
+  P.entries = static_cast<int>(a.B);
   g.status = status;
-  if (pair_pays<OpSwigluGate<BT>>(a.B, len, a.H, a.D)) return launch_pair(g, stream, kClsGate);
+  if (pair_pays<OpSwigluGate<BT>>(P.batch, len, a.H, a.D)) return launch_pair(g, stream, kClsGate);
   return launch_gemm(g, stream, kClsGate);
 }
 
 int run_apply(const ApplyArgs& a, int32_t* status, cudaStream_t stream) {
   const int64_t len = a.end - a.start;
   if (len <= 0) return LACT_OK;
-  const Mat w02{a.w02b, 2 * a.H, a.D, a.D, a.B, 2 * a.H * a.D};
-  const Mat w1{a.w1b, a.D, a.H, a.H, a.B, a.D * a.H};
-  const Mat x{a.x, a.end, a.D, a.x_ts, a.B, a.x_bs};
-  const Mat hid{a.hidden, len, a.H, a.H, a.B, len * a.H};
+  const Mat w02{a.w02b, 2 * a.H, a.D, a.D, a.B, 2 * a.H * a.D, a.segs, a.w_step};
+  const Mat w1{a.w1b, a.D, a.H, a.H, a.B, a.D * a.H, a.segs, a.w_step};
+  // (token strides are multiples of 16 bytes, so a range may start at any token; the maps end with it: nothing is written
+  // beyond the range)
+  const Mat x{static_cast<const bf16*>(a.x) + a.start * a.x_ts, len, a.D, a.x_ts, a.B, a.x_bs, a.segs, a.x_step * a.x_ts};
+  const Mat om{static_cast<bf16*>(a.out) + a.out_start * a.o_ts, len, a.D, a.o_ts, a.B, a.o_bs, a.segs, a.o_step * a.o_ts};
+  const Mat hid{a.hidden, len, a.H, a.H, a.B, len * a.H, a.segs, a.B * len * a.H};
+  const int64_t batch = a.segs * a.B;
   if (a.H % 128 == 0) LACT_TRY(launch_gate<128>(a, x, w02, len, status, stream));
   else LACT_TRY(launch_gate<64>(a, x, w02, len, status, stream));
   const int bt = choose_bt({{a.D, 1}});
   auto fill = [&](auto& g, int btv) -> int {
     auto& P = g.prob[0];
-    LACT_TRY(make_operand(kb_of(P), &P.a[0], &P.ai[0], hid, 0, kBM, 0, 0));
-    LACT_TRY(make_operand(kb_of(P), &P.b[0], &P.bi[0], w1, 0, btv, 0, 0));
-    // rows beyond the range's end must not be written: the map ends at out_start + len
-    const Mat om{a.out, a.out_start + len, a.D, a.o_ts, a.B, a.o_bs};
-    LACT_TRY(make_output(&P.out[0], &P.oi[0], om, static_cast<int>(a.out_start), 0));
+    LACT_TRY(make_operand(form_of(P), &P.a[0], &P.ai[0], hid, 0, kBM, 0, 0));
+    LACT_TRY(make_operand(form_of(P), &P.b[0], &P.bi[0], w1, 0, btv, 0, 0));
+    LACT_TRY(make_output(form_of(P), &P.out[0], &P.oi[0], om, 0, 0));
     P.M = static_cast<int>(len); P.N = static_cast<int>(a.D); P.K = static_cast<int>(a.H);
-    P.batch = static_cast<int>(a.B);
+    P.batch = static_cast<int>(batch);
+    P.entries = static_cast<int>(a.B);
     g.status = status;
     return LACT_OK;
   };
-  if (bt == 256 && pair_pays<OpBmmStore<256>>(a.B, len, a.D, a.H)) return launch_pair_store<OpBmmStore<256>>(fill, stream, kClsDown);
-  if (bt == 192 && pair_pays<OpBmmStore<192>>(a.B, len, a.D, a.H)) return launch_pair_store<OpBmmStore<192>>(fill, stream, kClsDown);
-  if (bt == 128 && pair_pays<OpBmmStore<128>>(a.B, len, a.D, a.H)) return launch_pair_store<OpBmmStore<128>>(fill, stream, kClsDown);
+  if (bt == 256 && pair_pays<OpBmmStore<256>>(batch, len, a.D, a.H)) return launch_pair_store<OpBmmStore<256>>(fill, stream, kClsDown);
+  if (bt == 192 && pair_pays<OpBmmStore<192>>(batch, len, a.D, a.H)) return launch_pair_store<OpBmmStore<192>>(fill, stream, kClsDown);
+  if (bt == 128 && pair_pays<OpBmmStore<128>>(batch, len, a.D, a.H)) return launch_pair_store<OpBmmStore<128>>(fill, stream, kClsDown);
   return launch_op<OpBmmStore, 1>(bt, fill, stream, kClsDown, 1);
 }
 
@@ -511,21 +545,21 @@ int run_grad_pointwise(const GradArgs& a, int32_t* status, cudaStream_t stream) 
   std::memset(&g, 0, sizeof(g));
   auto& P = g.prob[0];
   constexpr int BT = OpFwGradPointwise::BT;
-  LACT_TRY(make_operand(kb_of(P), &P.a[0], &P.ai[0], km, 0, kBM, static_cast<int>(a.start), 0));
-  LACT_TRY(make_operand(kb_of(P), &P.a[1], &P.ai[1], vm, 0, kBM, static_cast<int>(a.start), 0));
-  LACT_TRY(make_operand(kb_of(P), &P.b[0], &P.bi[0], w02, 0, BT, 0, 0));
-  LACT_TRY(make_operand(kb_of(P), &P.b[1], &P.bi[1], w02, 0, BT, static_cast<int>(a.H), 0));
+  LACT_TRY(make_operand(form_of(P), &P.a[0], &P.ai[0], km, 0, kBM, static_cast<int>(a.start), 0));
+  LACT_TRY(make_operand(form_of(P), &P.a[1], &P.ai[1], vm, 0, kBM, static_cast<int>(a.start), 0));
+  LACT_TRY(make_operand(form_of(P), &P.b[0], &P.bi[0], w02, 0, BT, 0, 0));
+  LACT_TRY(make_operand(form_of(P), &P.b[1], &P.bi[1], w02, 0, BT, static_cast<int>(a.H), 0));
   // dh = v w1: w1 is [D][H], i.e. k (= D) rows with the n (= H) axis contiguous
-  LACT_TRY(make_operand(kb_of(P), &P.b[2], &P.bi[2], w1, 1, BT, 0, 0));
+  LACT_TRY(make_operand(form_of(P), &P.b[2], &P.bi[2], w1, 1, BT, 0, 0));
   P.M = static_cast<int>(len); P.N = static_cast<int>(a.H); P.K = static_cast<int>(a.D);
   P.batch = static_cast<int>(a.B);
   P.ep = EpiFwGrad{a.lr0, a.lr1, a.lr2, a.lr_f32, static_cast<int32_t>(a.start), a.lr_bs, a.w_scale};
   // dy0 and dy2 share the [len][2H] plane: two maps of H columns each, so neither can spill
   const Mat dy0m{a.dy02, len, a.H, 2 * a.H, a.B, len * 2 * a.H};
   const Mat dy2m{a.dy02 + a.H, len, a.H, 2 * a.H, a.B, len * 2 * a.H};
-  LACT_TRY(make_output(&P.out[0], &P.oi[0], dy0m, 0, 0));
-  LACT_TRY(make_output(&P.out[1], &P.oi[1], dy2m, 0, 0));
-  LACT_TRY(make_output(&P.out[2], &P.oi[2], hid, 0, 0));
+  LACT_TRY(make_output(form_of(P), &P.out[0], &P.oi[0], dy0m, 0, 0));
+  LACT_TRY(make_output(form_of(P), &P.out[1], &P.oi[1], dy2m, 0, 0));
+  LACT_TRY(make_output(form_of(P), &P.out[2], &P.oi[2], hid, 0, 0));
   g.status = status;
   if (pair_pays<OpFwGradPointwise>(a.B, len, a.H, a.D)) {
     LACT_TRY(encode_map(&P.b[2], w1, 64, 32));  // a CTA's half of these columns: atoms of 32
@@ -546,15 +580,15 @@ int run_grad(const GradArgs& a, int32_t* status, cudaStream_t stream) {
   const Split split = a.split.part != nullptr ? choose_split(ceil_div(len, kBK)) : Split{1, 0};
   auto fill = [&](auto& g, int btv) -> int {
     auto& P0 = g.prob[0];
-    LACT_TRY(make_operand(kb_of(P0), &P0.a[0], &P0.ai[0], dy, 1, kBM, 0, 0));
-    LACT_TRY(make_operand(kb_of(P0), &P0.b[0], &P0.bi[0], km, 1, btv, 0, static_cast<int>(a.start)));
+    LACT_TRY(make_operand(form_of(P0), &P0.a[0], &P0.ai[0], dy, 1, kBM, 0, 0));
+    LACT_TRY(make_operand(form_of(P0), &P0.b[0], &P0.bi[0], km, 1, btv, 0, static_cast<int>(a.start)));
     P0.M = static_cast<int>(2 * a.H); P0.N = static_cast<int>(a.D); P0.K = static_cast<int>(len);
     P0.batch = static_cast<int>(a.B);
     P0.ep = EpiDW{a.g02, 2 * a.H * a.D, a.D, a.beta, 1, a.g_f32, a.partial02, ceil_div(2 * a.H, kBM),
                   ceil_div(a.D, btv), a.gb02, a.g02_prev, a.fresh};
     auto& P1 = g.prob[1];
-    LACT_TRY(make_operand(kb_of(P1), &P1.a[0], &P1.ai[0], vm, 1, kBM, 0, static_cast<int>(a.start)));
-    LACT_TRY(make_operand(kb_of(P1), &P1.b[0], &P1.bi[0], hid, 1, btv, 0, 0));
+    LACT_TRY(make_operand(form_of(P1), &P1.a[0], &P1.ai[0], vm, 1, kBM, 0, static_cast<int>(a.start)));
+    LACT_TRY(make_operand(form_of(P1), &P1.b[0], &P1.bi[0], hid, 1, btv, 0, 0));
     P1.M = static_cast<int>(a.D); P1.N = static_cast<int>(a.H); P1.K = static_cast<int>(len);
     P1.batch = static_cast<int>(a.B);
     P1.ep = EpiDW{a.g1, a.D * a.H, a.H, a.beta, 1, a.g_f32, a.partial1, ceil_div(a.D, kBM), ceil_div(a.H, btv),
@@ -651,25 +685,25 @@ int wire_ns_group(const NsGroup& G, bf16* cur, bf16* nxt, int bt_mm, int bt_mn, 
   const Mat PB{G.poly, G.m, G.m, G.m, G.nmat, mm};
   const int tall = G.transposed;
   // gram: S = X X^T (wide) / X^T X (tall) + (b / 2c) I
-  LACT_TRY(make_operand(kb_of(gram), &gram.a[0], &gram.ai[0], X, tall, kBM, 0, 0));
-  LACT_TRY(make_operand(kb_of(gram), &gram.b[0], &gram.bi[0], X, tall, bt_mm, 0, 0));
+  LACT_TRY(make_operand(form_of(gram), &gram.a[0], &gram.ai[0], X, tall, kBM, 0, 0));
+  LACT_TRY(make_operand(form_of(gram), &gram.b[0], &gram.bi[0], X, tall, bt_mm, 0, 0));
   gram.M = G.m; gram.N = G.m; gram.K = G.n; gram.batch = G.nmat;
-  LACT_TRY(make_output(&gram.out[0], &gram.oi[0], S, 0, 0));
+  LACT_TRY(make_output(form_of(gram), &gram.out[0], &gram.oi[0], S, 0, 0));
   // poly: P = c S S + (a - b^2 / 4c) I   (S is exactly symmetric: its rows serve as the K-major B operand too)
-  LACT_TRY(make_operand(kb_of(poly), &poly.a[0], &poly.ai[0], S, 0, kBM, 0, 0));
-  LACT_TRY(make_operand(kb_of(poly), &poly.b[0], &poly.bi[0], S, 0, bt_mm, 0, 0));
+  LACT_TRY(make_operand(form_of(poly), &poly.a[0], &poly.ai[0], S, 0, kBM, 0, 0));
+  LACT_TRY(make_operand(form_of(poly), &poly.b[0], &poly.bi[0], S, 0, bt_mm, 0, 0));
   poly.M = G.m; poly.N = G.m; poly.K = G.m; poly.batch = G.nmat;
-  LACT_TRY(make_output(&poly.out[0], &poly.oi[0], PB, 0, 0));
+  LACT_TRY(make_output(form_of(poly), &poly.out[0], &poly.oi[0], PB, 0, 0));
   // update: X' = poly X (wide; X is [k][n]: MN-major B operand) / X' = X poly^T (tall)
   if (!tall) {
-    LACT_TRY(make_operand(kb_of(upd), &upd.a[0], &upd.ai[0], PB, 0, kBM, 0, 0));
-    LACT_TRY(make_operand(kb_of(upd), &upd.b[0], &upd.bi[0], X, 1, bt_mn, 0, 0));
+    LACT_TRY(make_operand(form_of(upd), &upd.a[0], &upd.ai[0], PB, 0, kBM, 0, 0));
+    LACT_TRY(make_operand(form_of(upd), &upd.b[0], &upd.bi[0], X, 1, bt_mn, 0, 0));
   } else {
-    LACT_TRY(make_operand(kb_of(upd), &upd.a[0], &upd.ai[0], X, 0, kBM, 0, 0));
-    LACT_TRY(make_operand(kb_of(upd), &upd.b[0], &upd.bi[0], PB, 0, bt_mn, 0, 0));
+    LACT_TRY(make_operand(form_of(upd), &upd.a[0], &upd.ai[0], X, 0, kBM, 0, 0));
+    LACT_TRY(make_operand(form_of(upd), &upd.b[0], &upd.bi[0], PB, 0, bt_mn, 0, 0));
   }
   upd.M = ns_upd_rows(G); upd.N = ns_upd_cols(G); upd.K = G.m; upd.batch = G.nmat;
-  LACT_TRY(make_output(&upd.out[0], &upd.oi[0], XN, 0, 0));
+  LACT_TRY(make_output(form_of(upd), &upd.out[0], &upd.oi[0], XN, 0, 0));
   return LACT_OK;
 }
 
@@ -1055,33 +1089,33 @@ static int launch_ns_bwd_fused(const NsTrace* tr, const bf16* const* du, int ngr
       auto& pt = args.t[it][g];
       auto& px = args.dx[it][g];
       // Q = dX X^T + X dX^T (wide; the iterate's rows are K-major operands) / dX^T X + X^T dX (tall; MN-major)
-      LACT_TRY(make_operand(1, &pq.a[0], &pq.ai[0], D, tall, kBM, 0, 0));
-      LACT_TRY(make_operand(1, &pq.b[0], &pq.bi[0], X, tall, BT_MM, 0, 0));
-      LACT_TRY(make_operand(1, &pq.a[1], &pq.ai[1], X, tall, kBM, 0, 0));
-      LACT_TRY(make_operand(1, &pq.b[1], &pq.bi[1], D, tall, BT_MM, 0, 0));
+      LACT_TRY(make_operand(OperandForm{1, false}, &pq.a[0], &pq.ai[0], D, tall, kBM, 0, 0));
+      LACT_TRY(make_operand(OperandForm{1, false}, &pq.b[0], &pq.bi[0], X, tall, BT_MM, 0, 0));
+      LACT_TRY(make_operand(OperandForm{1, false}, &pq.a[1], &pq.ai[1], X, tall, kBM, 0, 0));
+      LACT_TRY(make_operand(OperandForm{1, false}, &pq.b[1], &pq.bi[1], D, tall, BT_MM, 0, 0));
       pq.M = G.m; pq.N = G.m; pq.K = G.n; pq.batch = G.nmat;
-      LACT_TRY(make_output(&pq.out[0], &pq.oi[0], Q, 0, 0));
+      LACT_TRY(make_output(form_of(pq), &pq.out[0], &pq.oi[0], Q, 0, 0));
       // T = c (S Q + Q S): all three symmetric, rows serve as K-major operands on either side
-      LACT_TRY(make_operand(1, &pt.a[0], &pt.ai[0], S, 0, kBM, 0, 0));
-      LACT_TRY(make_operand(1, &pt.b[0], &pt.bi[0], Q, 0, BT_MM, 0, 0));
-      LACT_TRY(make_operand(1, &pt.a[1], &pt.ai[1], Q, 0, kBM, 0, 0));
-      LACT_TRY(make_operand(1, &pt.b[1], &pt.bi[1], S, 0, BT_MM, 0, 0));
+      LACT_TRY(make_operand(OperandForm{1, false}, &pt.a[0], &pt.ai[0], S, 0, kBM, 0, 0));
+      LACT_TRY(make_operand(OperandForm{1, false}, &pt.b[0], &pt.bi[0], Q, 0, BT_MM, 0, 0));
+      LACT_TRY(make_operand(OperandForm{1, false}, &pt.a[1], &pt.ai[1], Q, 0, kBM, 0, 0));
+      LACT_TRY(make_operand(OperandForm{1, false}, &pt.b[1], &pt.bi[1], S, 0, BT_MM, 0, 0));
       pt.M = G.m; pt.N = G.m; pt.K = G.m; pt.batch = G.nmat;
-      LACT_TRY(make_output(&pt.out[0], &pt.oi[0], T, 0, 0));
+      LACT_TRY(make_output(form_of(pt), &pt.out[0], &pt.oi[0], T, 0, 0));
       // dX_i = P dX + T X (wide: the [k][n] iterates are MN-major B operands) / dX P + X T (tall)
       if (!tall) {
-        LACT_TRY(make_operand(1, &px.a[0], &px.ai[0], PB, 0, kBM, 0, 0));
-        LACT_TRY(make_operand(1, &px.b[0], &px.bi[0], D, 1, BT, 0, 0));
-        LACT_TRY(make_operand(1, &px.a[1], &px.ai[1], T, 0, kBM, 0, 0));
-        LACT_TRY(make_operand(1, &px.b[1], &px.bi[1], X, 1, BT, 0, 0));
+        LACT_TRY(make_operand(OperandForm{1, false}, &px.a[0], &px.ai[0], PB, 0, kBM, 0, 0));
+        LACT_TRY(make_operand(OperandForm{1, false}, &px.b[0], &px.bi[0], D, 1, BT, 0, 0));
+        LACT_TRY(make_operand(OperandForm{1, false}, &px.a[1], &px.ai[1], T, 0, kBM, 0, 0));
+        LACT_TRY(make_operand(OperandForm{1, false}, &px.b[1], &px.bi[1], X, 1, BT, 0, 0));
       } else {
-        LACT_TRY(make_operand(1, &px.a[0], &px.ai[0], D, 0, kBM, 0, 0));
-        LACT_TRY(make_operand(1, &px.b[0], &px.bi[0], PB, 0, BT, 0, 0));
-        LACT_TRY(make_operand(1, &px.a[1], &px.ai[1], X, 0, kBM, 0, 0));
-        LACT_TRY(make_operand(1, &px.b[1], &px.bi[1], T, 0, BT, 0, 0));
+        LACT_TRY(make_operand(OperandForm{1, false}, &px.a[0], &px.ai[0], D, 0, kBM, 0, 0));
+        LACT_TRY(make_operand(OperandForm{1, false}, &px.b[0], &px.bi[0], PB, 0, BT, 0, 0));
+        LACT_TRY(make_operand(OperandForm{1, false}, &px.a[1], &px.ai[1], X, 0, kBM, 0, 0));
+        LACT_TRY(make_operand(OperandForm{1, false}, &px.b[1], &px.bi[1], T, 0, BT, 0, 0));
       }
       px.M = ns_upd_rows(G); px.N = ns_upd_cols(G); px.K = G.m; px.batch = G.nmat;
-      LACT_TRY(make_output(&px.out[0], &px.oi[0], O, 0, 0));
+      LACT_TRY(make_output(form_of(px), &px.out[0], &px.oi[0], O, 0, 0));
       dX = out;
     }
     args.done[g] = G.done;
@@ -1168,24 +1202,67 @@ int launch_swa_bwd(const SwaBwdArgs& a, int64_t ctas, cudaStream_t stream) {
 struct ScanPlan {
   int32_t* status;
   float *W02, *W1, *W02c, *W1c, *n02, *n1, *G02, *G1, *beta;
-  bf16 *W02b, *W1b, *hidden, *dy02, *hid;
+  bf16 *Wb, *hidden, *dy02, *hid;  // Wb: `w_slots` times [W0W2 | W1]
+  int32_t w_slots;
   SplitScratch split;
   int32_t split_tiles;
   NsPlan ns;
   size_t bytes;
 };
 
+// How many APPLY steps from step `i` on are left to the last of them, which then runs all in one launch (ApplyArgs::segs): steps
+// of one length, evenly spaced, with one UPDATE between each two (so that their weights lie in consecutive slots), whose outputs
+// do not overlap.  A step of few tiles costs its launches' fill and drain, in series with the chain of updates: 12 entries of
+// 128 x 256 and 1560 tokens take 26 us a step alone and 9.5 us in runs of six (21 steps: 1669 -> 1487 us the whole call; 4 entries of
+// 384, 2048 tokens, two steps: 354 -> 343).  Steps are collected until they have kApplyRounds tiles of 128 tokens and hidden
+// features per SM, which also bounds the memory their weights and hidden activations take; a step that has as many by itself
+// gains nothing.  `out_start` nullptr: as if the outputs were disjoint.
+constexpr int64_t kApplyRounds = 12;
+struct ApplyRun {
+  int64_t steps, x_step, o_step;
+};
+ApplyRun apply_run(const lact_scan_config& c, int32_t n_steps, const int32_t* kind, const int64_t* start, const int64_t* end,
+                   const int64_t* out_start, int32_t i) {
+  ApplyRun r{1, 0, 0};
+  const int64_t len = end[i] - start[i];
+  if (len <= 0) return r;
+  const int64_t tiles = c.B * ceil_div(len, kBM) * ceil_div(c.H, kBM);
+  const int64_t most = (kApplyRounds * sm_count() + tiles - 1) / tiles;
+  int64_t at = i;
+  while (r.steps < most && at + 2 < n_steps && kind[at + 1] == LACT_STEP_UPDATE && kind[at + 2] == LACT_STEP_APPLY &&
+         end[at + 2] - start[at + 2] == len) {
+    const int64_t dx = start[at + 2] - start[at], dout = out_start != nullptr ? out_start[at + 2] - out_start[at] : len;
+    if (dx <= 0 || dout < len) break;
+    if (r.steps == 1) {
+      r.x_step = dx;
+      r.o_step = dout;
+    } else if (dx != r.x_step || dout != r.o_step) {
+      break;
+    }
+    ++r.steps;
+    at += 2;
+  }
+  return r;
+}
+
 int plan_scan(const lact_scan_config& c, int32_t n_steps, const int32_t* kind, const int64_t* start,
               const int64_t* end, void* base, ScanPlan* p) {
-  int64_t max_apply = 0, max_update = 0;
+  int64_t max_apply = 0, max_update = 0, slots = 1;
   for (int i = 0; i < n_steps; ++i) {
     if (start[i] < 0 || end[i] > c.L || end[i] < start[i]) return LACT_ERR_STEPS;
     const int64_t len = end[i] - start[i];
-    if (kind[i] == LACT_STEP_APPLY) max_apply = std::max(max_apply, len);
-    else if (kind[i] == LACT_STEP_UPDATE) {
+    if (kind[i] == LACT_STEP_APPLY) {
+      max_apply = std::max(max_apply, len);
+    } else if (kind[i] == LACT_STEP_UPDATE) {
       if (len <= 0) return LACT_ERR_STEPS;
       max_update = std::max(max_update, len);
     } else return LACT_ERR_STEPS;
+  }
+  for (int i = 0; i < n_steps; ++i) {  // (runs from any step: which ones there are also depends on the outputs' places)
+    if (kind[i] != LACT_STEP_APPLY) continue;
+    const int64_t steps = apply_run(c, n_steps, kind, start, end, nullptr, i).steps;
+    slots = std::max(slots, steps);
+    max_apply = std::max(max_apply, steps * (end[i] - start[i]));
   }
   Carver cv(base);
   const size_t B = c.B, D = c.D, H = c.H;
@@ -1199,8 +1276,8 @@ int plan_scan(const lact_scan_config& c, int32_t n_steps, const int32_t* kind, c
   p->G02 = cv.take<float>(B * 2 * H * D);
   p->G1 = cv.take<float>(B * D * H);
   p->beta = cv.take<float>(B * static_cast<size_t>(std::max(1, n_steps)));
-  p->W02b = cv.take<bf16>(B * 2 * H * D);
-  p->W1b = cv.take<bf16>(B * D * H);
+  p->w_slots = static_cast<int32_t>(slots);
+  p->Wb = cv.take<bf16>(B * 3 * H * D * static_cast<size_t>(slots));
   p->hidden = cv.take<bf16>(B * static_cast<size_t>(max_apply) * H);
   p->dy02 = cv.take<bf16>(B * static_cast<size_t>(max_update) * 2 * H);
   p->hid = cv.take<bf16>(B * static_cast<size_t>(max_update) * H);
@@ -1360,10 +1437,11 @@ int scan_fwd(const lact_scan_config& c, const lact_scan_io& io, int32_t n_steps,
   auto slot = [&](int u) { return static_cast<float*>(io.state_dump) + static_cast<size_t>(u) * 2 * (n02 + n1); };
   float* W02cur = dump_in_place ? slot(0) : p.W02;   // master weights in force
   float* W1cur = dump_in_place ? slot(0) + n02 : p.W1;
-  // bf16 copies of the weights in force (MMA operands); training keeps those of every update in the caller's buffer
-  bf16 *W02b = p.W02b, *W1b = p.W1b;
-  auto shadow_slot = [&](int u) { return static_cast<bf16*>(io.shadow_dump) + static_cast<size_t>(u) * (n02 + n1); };
-  if (io.shadow_dump != nullptr) { W02b = shadow_slot(0); W1b = W02b + n02; }
+  // bf16 copies of the weights in force (MMA operands), [W0W2 | W1] per slot; training keeps those of every update in the
+  // caller's buffer, else there are as many slots as one run of APPLY steps needs, used in turn
+  bf16* const Wb = io.shadow_dump != nullptr ? static_cast<bf16*>(io.shadow_dump) : p.Wb;
+  int w_slot = 0;
+  bf16 *W02b = Wb, *W1b = Wb + n02;
   float* G02cur = p.G02;                              // gradient / momentum state after the latest update
   float* G1cur = p.G1;
   {
@@ -1386,11 +1464,20 @@ int scan_fwd(const lact_scan_config& c, const lact_scan_io& io, int32_t n_steps,
   if (ns_keep && (reinterpret_cast<uintptr_t>(io.ns_trace) & 255) != 0) return LACT_ERR_WORKSPACE;
 
   int update_idx = 0;
+  ApplyArgs pending{};     // the run of APPLY steps being collected, none if `missing` is 0
+  int64_t missing = 0;     // how many of its steps are still to come
   for (int i = 0; i < n_steps; ++i) {
     if (kind[i] == LACT_STEP_APPLY) {
-      ApplyArgs a{W02b, W1b, io.q, c.q_bs, c.q_ts, start[i], end[i], io.o, c.o_bs, c.o_ts, out_start[i],
-                  p.hidden, B, D, H};
-      LACT_TRY(run_apply(a, p.status, stream));
+      if (missing == 0) {
+        const ApplyRun run = apply_run(c, n_steps, kind, start, end, out_start, i);
+        pending = ApplyArgs{W02b, W1b, io.q, c.q_bs, c.q_ts, start[i], end[i], io.o, c.o_bs, c.o_ts, out_start[i],
+                            p.hidden, B, D, H};
+        pending.segs = missing = run.steps;
+        pending.x_step = run.x_step;
+        pending.o_step = run.o_step;
+        pending.w_step = static_cast<int64_t>(n02 + n1);
+      }
+      if (--missing == 0) LACT_TRY(run_apply(pending, p.status, stream));
       continue;
     }
     const float* beta = c.use_momentum ? p.beta + static_cast<int64_t>(update_idx) * B : nullptr;
@@ -1445,6 +1532,9 @@ int scan_fwd(const lact_scan_config& c, const lact_scan_io& io, int32_t n_steps,
     // add + renormalise arguments (the update is the Newton-Schulz result when Muon is on)
     // (the fp32 copy of the normalised weights is what pre-norm computes with and what the final export reads)
     const bool want_compute = c.prenorm || ((io.w0_out || io.w1_out || io.w2_out) && !has_later_update(kind, n_steps, i));
+    // (the weights of steps still to run are not overwritten: a run starts in slot 0 or, the first one, where the weights are)
+    const int next_slot = io.shadow_dump != nullptr ? update_idx : (missing > 0 ? w_slot + 1 : 0);
+    if (io.shadow_dump == nullptr && next_slot >= p.w_slots) return LACT_ERR_WORKSPACE;
     RenormArgs rn[2];
     for (int w = 0; w < 2; ++w) {
       RenormArgs& r = rn[w];
@@ -1457,8 +1547,7 @@ int scan_fwd(const lact_scan_config& c, const lact_scan_io& io, int32_t n_steps,
         if (update_idx < n_updates) r.master = w == 0 ? slot(update_idx) : slot(update_idx) + n02;
       }
       r.compute = want_compute ? (w == 0 ? p.W02c : p.W1c) : nullptr;
-      r.shadow = w == 0 ? W02b : W1b;
-      if (io.shadow_dump != nullptr) r.shadow = w == 0 ? shadow_slot(update_idx) : shadow_slot(update_idx) + n02;
+      r.shadow = Wb + static_cast<size_t>(next_slot) * (n02 + n1) + (w == 0 ? 0 : n02);
       r.n0 = w == 0 ? p.n02 : p.n1;
       r.g = w == 0 ? G02cur : G1cur;
       r.x = nullptr;
@@ -1497,8 +1586,9 @@ int scan_fwd(const lact_scan_config& c, const lact_scan_io& io, int32_t n_steps,
       rn[1].x = xres[1];
     }
     LACT_TRY(launch_add_renorm(rn[0], rn[1], stream));
-    W02b = rn[0].shadow;
-    W1b = rn[1].shadow;
+    w_slot = next_slot;
+    W02b = Wb + static_cast<size_t>(w_slot) * (n02 + n1);
+    W1b = W02b + n02;
     if (dump_in_place) {
       W02cur = rn[0].master;
       W1cur = rn[1].master;
@@ -2730,11 +2820,11 @@ static int bmm_group(const lact_bmm_desc* d, int n, int32_t* status_word, void* 
     for (int p = 0; p < n; ++p) {
       const lact_bmm_desc& q = d[p];
       auto& P = g.prob[p];
-      LACT_TRY(make_operand(kb_of(P), &P.a[0], &P.ai[0], mat(q, q.a0, q.a0_mn, q.M, q.a0_ld, q.a0_bs), q.a0_mn, kBM, 0, 0));
-      LACT_TRY(make_operand(kb_of(P), &P.b[0], &P.bi[0], mat(q, q.b0, q.b0_mn, q.N, q.b0_ld, q.b0_bs), q.b0_mn, btv, 0, 0));
+      LACT_TRY(make_operand(form_of(P), &P.a[0], &P.ai[0], mat(q, q.a0, q.a0_mn, q.M, q.a0_ld, q.a0_bs), q.a0_mn, kBM, 0, 0));
+      LACT_TRY(make_operand(form_of(P), &P.b[0], &P.bi[0], mat(q, q.b0, q.b0_mn, q.N, q.b0_ld, q.b0_bs), q.b0_mn, btv, 0, 0));
       if constexpr (std::remove_reference_t<decltype(g)>::OpType::NA == 2) {
-        LACT_TRY(make_operand(kb_of(P), &P.a[1], &P.ai[1], mat(q, q.a1, q.a1_mn, q.M, q.a1_ld, q.a1_bs), q.a1_mn, kBM, 0, 0));
-        LACT_TRY(make_operand(kb_of(P), &P.b[1], &P.bi[1], mat(q, q.b1, q.b1_mn, q.N, q.b1_ld, q.b1_bs), q.b1_mn, btv, 0, 0));
+        LACT_TRY(make_operand(form_of(P), &P.a[1], &P.ai[1], mat(q, q.a1, q.a1_mn, q.M, q.a1_ld, q.a1_bs), q.a1_mn, kBM, 0, 0));
+        LACT_TRY(make_operand(form_of(P), &P.b[1], &P.bi[1], mat(q, q.b1, q.b1_mn, q.N, q.b1_ld, q.b1_bs), q.b1_mn, btv, 0, 0));
       }
       P.M = static_cast<int>(q.M); P.N = static_cast<int>(q.N); P.K = static_cast<int>(q.K);
       P.batch = static_cast<int>(q.batch);
@@ -3123,8 +3213,8 @@ int lact_bmm_bf16(const void* a, int32_t a_mn_major, const void* b, int32_t b_mn
   const Mat Bm = b_mn_major ? Mat{b, K, N, N, batch, K * N} : Mat{b, N, K, K, batch, N * K};
   auto fill = [&](auto& g, int btv) -> int {
     auto& P = g.prob[0];
-    LACT_TRY(make_operand(kb_of(P), &P.a[0], &P.ai[0], A, a_mn_major, kBM, 0, 0));
-    LACT_TRY(make_operand(kb_of(P), &P.b[0], &P.bi[0], Bm, b_mn_major, btv, 0, 0));
+    LACT_TRY(make_operand(form_of(P), &P.a[0], &P.ai[0], A, a_mn_major, kBM, 0, 0));
+    LACT_TRY(make_operand(form_of(P), &P.b[0], &P.bi[0], Bm, b_mn_major, btv, 0, 0));
     P.M = static_cast<int>(M); P.N = static_cast<int>(N); P.K = static_cast<int>(K);
     P.batch = static_cast<int>(batch);
     P.ep = EpiStore{c, M * N, N, 0, 1, 0};
@@ -3133,9 +3223,9 @@ int lact_bmm_bf16(const void* a, int32_t a_mn_major, const void* b, int32_t b_mn
   };
   auto fill_bf16 = [&](auto& g, int btv) -> int {
     auto& P = g.prob[0];
-    LACT_TRY(make_operand(kb_of(P), &P.a[0], &P.ai[0], A, a_mn_major, kBM, 0, 0));
-    LACT_TRY(make_operand(kb_of(P), &P.b[0], &P.bi[0], Bm, b_mn_major, btv, 0, 0));
-    LACT_TRY(make_output(&P.out[0], &P.oi[0], Mat{c, M, N, N, batch, M * N}, 0, 0));
+    LACT_TRY(make_operand(form_of(P), &P.a[0], &P.ai[0], A, a_mn_major, kBM, 0, 0));
+    LACT_TRY(make_operand(form_of(P), &P.b[0], &P.bi[0], Bm, b_mn_major, btv, 0, 0));
+    LACT_TRY(make_output(form_of(P), &P.out[0], &P.oi[0], Mat{c, M, N, N, batch, M * N}, 0, 0));
     P.M = static_cast<int>(M); P.N = static_cast<int>(N); P.K = static_cast<int>(K);
     P.batch = static_cast<int>(batch);
     g.status = status_word;

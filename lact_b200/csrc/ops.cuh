@@ -247,6 +247,7 @@ struct OpDW {
 struct EpiNone {};
 template <int BT_>
 struct OpBmmStore {
+  static constexpr bool kSegments = true;
   static constexpr int NA = 1, NB = 1, NACC = 1, BT = BT_, NTERMS = 1, NOUT = 1;
   static constexpr bool kTileReduce = false;
   static constexpr bool kWarpTranspose = false, kReverseBatch = true;
@@ -384,6 +385,7 @@ using OpNs2 = OpNs2T<BT_, false>;
 // into adjacent accumulator columns.
 template <int BT_>
 struct OpSwigluGate {
+  static constexpr bool kSegments = true;
   static constexpr int KB = 1;  // measured: two-k-block stages (a 2-deep ring here) are 7 % slower for this op
   static constexpr int NA = 1, NB = 2, NACC = 2, BT = BT_, NTERMS = KB, NOUT = 1;
   static constexpr bool kTileReduce = false;

@@ -153,6 +153,11 @@ pair_gemm_kernel(const __grid_constant__ GemmArgs<Op, 1> args, const int ring) {
   // (the CTAs of a pair may differ: every wait for the other has a limit)
   bool failed = earlier_launch_failed(args.status);
   const bool work = !failed;
+  constexpr bool SEG = op_segments<Op>::value;
+  auto load = [](uint32_t leader, uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int entry, int segment) {
+    if constexpr (SEG) tma_load_4d_pair_if(leader, dst, map, bar, c0, c1, entry, segment);
+    else tma_load_3d_pair_if(leader, dst, map, bar, c0, c1, entry);
+  };
   auto term_bytes = [](int t) { return static_cast<uint32_t>(Wire::template b_rows<Op>(t)) * 128u; };  // a k-block of B, per CTA
   constexpr uint32_t b_bytes = pair_b_bytes<Op>(1);
   auto term_base = [&](int t) { return b_base + (t == 0 ? 0u : term_bytes(0) * num_kb); };
@@ -169,15 +174,17 @@ pair_gemm_kernel(const __grid_constant__ GemmArgs<Op, 1> args, const int ring) {
       // coordinates of this tile's boxes, per term; one k-block on per stage
       int a_row[Op::NTERMS], a_batch[Op::NTERMS], a_k[Op::NTERMS], b_mn[Op::NTERMS], b_batch[Op::NTERMS], b_k[Op::NTERMS];
       bool b_major[Op::NTERMS];
+      int entry, segment;
+      entry_of(P, r.batch, entry, segment);
 #pragma unroll
       for (int t = 0; t < Op::NTERMS; ++t) {
         const OperandInfo& ai = P.ai[Op::term_a(t)];
         a_row[t] = ai.mn_off + r.m * kPairRows + static_cast<int>(rank) * kBM;
-        a_batch[t] = ai.batch_off + r.batch;
+        a_batch[t] = ai.batch_off + entry;
         a_k[t] = ai.k_off;
         const OperandInfo& bi = P.bi[Wire::template b_map<Op>(t, rank)];
         b_mn[t] = bi.mn_off + n0 + Wire::template b_col<Op>(t, rank);
-        b_batch[t] = bi.batch_off + r.batch;
+        b_batch[t] = bi.batch_off + entry;
         b_k[t] = bi.k_off;
         b_major[t] = bi.mn_major != 0;
       }
@@ -190,12 +197,12 @@ pair_gemm_kernel(const __grid_constant__ GemmArgs<Op, 1> args, const int ring) {
           for (int t = 0; t < Op::NTERMS; ++t) {
             const CUtensorMap* const map = &P.b[Wire::template b_map<Op>(t, rank)];
             const uint32_t dst = term_base(t) + kb * term_bytes(t);
-            if (!b_major[t]) tma_load_3d_pair_if(leader, dst, map, bar, b_k[t], b_mn[t], b_batch[t]);
-            else if (Wire::kHalfAtom && t == Op::NTERMS - 1) tma_load_3d_pair_if(leader, dst, map, bar, b_mn[t], b_k[t], b_batch[t]);
+            if (!b_major[t]) load(leader, dst, map, bar, b_k[t], b_mn[t], b_batch[t], segment);
+            else if (Wire::kHalfAtom && t == Op::NTERMS - 1) load(leader, dst, map, bar, b_mn[t], b_k[t], b_batch[t], segment);
             else {
 #pragma unroll
               for (int j = 0; j < Wire::template b_rows<Op>(t) / 64; ++j)
-                tma_load_3d_pair_if(leader, dst + j * kAtomBytes, map, bar, b_mn[t] + 64 * j, b_k[t], b_batch[t]);
+                load(leader, dst + j * kAtomBytes, map, bar, b_mn[t] + 64 * j, b_k[t], b_batch[t], segment);
             }
             b_k[t] += kBK;
           }
@@ -205,7 +212,7 @@ pair_gemm_kernel(const __grid_constant__ GemmArgs<Op, 1> args, const int ring) {
         const uint32_t bar = leader_address(&full[s]), st = a_base + s * pair_stage_bytes<Op>();
 #pragma unroll
         for (int t = 0; t < Op::NTERMS; ++t) {
-          tma_load_3d_pair_if(leader, st + Op::term_a(t) * kATileBytes, &P.a[Op::term_a(t)], bar, a_k[t], a_row[t], a_batch[t]);
+          load(leader, st + Op::term_a(t) * kATileBytes, &P.a[Op::term_a(t)], bar, a_k[t], a_row[t], a_batch[t], segment);
           a_k[t] += kBK;
         }
         if (++s == ring) { s = 0; ph ^= 1; }
@@ -288,6 +295,8 @@ pair_gemm_kernel(const __grid_constant__ GemmArgs<Op, 1> args, const int ring) {
       tc_fence_after();
       const uint32_t acc = tmem + as * kAccCols + (static_cast<uint32_t>(quarter * 32) << 16) + half * 32;
       const int panels = min(BT / 64, (P.N - n0 + 63) / 64);
+      int entry, segment;
+      entry_of(P, r.batch, entry, segment);
       for (int pnl = 0; pnl < panels && !stop; ++pnl) {
         uint32_t packed[NOUT][16];
         {
@@ -329,8 +338,9 @@ pair_gemm_kernel(const __grid_constant__ GemmArgs<Op, 1> args, const int ring) {
           named_barrier_sync(2, kEpiWarps * 32);
           if (pnl == 0 && o == 0 && abort_flag[1 + as] != 0) { stop = true; break; }
           if (elected && m0 < P.M) {
-            tma_store_3d(&P.out[o], stg + buf * kPairPanel, P.oi[o].col_off + n0 + pnl * 64, P.oi[o].row_off + m0,
-                         P.oi[o].batch_off + r.batch);
+            const int col = P.oi[o].col_off + n0 + pnl * 64, at = P.oi[o].row_off + m0, b = P.oi[o].batch_off + entry;
+            if constexpr (SEG) tma_store_4d(&P.out[o], stg + buf * kPairPanel, col, at, b, segment);
+            else tma_store_3d(&P.out[o], stg + buf * kPairPanel, col, at, b);
           }
           if (elected) bulk_commit_group();
           if (++buf == PANELS) buf = 0;

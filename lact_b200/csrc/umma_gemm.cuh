@@ -42,6 +42,7 @@ struct GemmProblem {
   OperandInfo bi[Op::NB];
   OutInfo oi[Op::NOUT > 0 ? Op::NOUT : 1];
   int32_t M, N, K, batch;
+  int32_t entries;  // ops with `kSegments`: batch index x is entry x % entries of segment x / entries (0: one segment)
   typename Op::Epi ep;
   // Split contraction (ops with `kSplitK`; `splits` > 1): the k-blocks of every output tile are dealt to `splits` units of
   // `kb_per_split` k-blocks each.  A unit leaves its fp32 sums in `part`; the unit that finds the tile's word of `count` at
@@ -98,20 +99,22 @@ constexpr int kGemmThreadsFlow = kGemmThreadsV2 + 64;  // + dependency scout war
 // MN-major tile as one 128-k-row box per atom.
 // The cursor holds the coordinates of an operand's next boxes: they are worked out once per output tile, so that between two
 // stages the issuing warp only adds.  (What that warp spends per box is what the loads can reach: see gemm_phase.)
-template <int ROWS, int KB>
+// SEG: the maps are 4-D (inner, row, entry, segment), see op_segments.
+template <int ROWS, int KB, bool SEG>
 struct OperandCursor {
   const CUtensorMap* map;
-  int32_t inner, row, batch;  // first box of the stage; 4-D maps: inner = k-block, row = mn
+  int32_t inner, row, batch, segment;  // first box of the stage; 4-D maps: inner = k-block, row = mn
   int32_t d_inner, d_row;     // advance per stage
   int32_t kind;               // 0: K-major, a box per k-block; 1: K-major, one 4-D box; 2: MN-major, a box per atom
-  __device__ __forceinline__ void start(const CUtensorMap* m, const OperandInfo& oi, int mn0, int kc, int b) {
+  __device__ __forceinline__ void start(const CUtensorMap* m, const OperandInfo& oi, int mn0, int kc, int b, int seg) {
     map = m;
     batch = oi.batch_off + b;
+    segment = seg;
     if (oi.mn_major) {
       kind = 2;
       inner = oi.mn_off + mn0; row = oi.k_off + kc;
       d_inner = 0; d_row = KB * kBK;
-    } else if (KB == 2 && oi.k4d) {
+    } else if (!SEG && KB == 2 && oi.k4d) {
       kind = 1;
       inner = (oi.k_off + kc) / kBK; row = oi.mn_off + mn0;
       d_inner = KB; d_row = 0;
@@ -121,15 +124,19 @@ struct OperandCursor {
       d_inner = KB * kBK; d_row = 0;
     }
   }
+  __device__ __forceinline__ void box(uint32_t leader, uint32_t dst, uint32_t bar, int at) const {
+    if constexpr (SEG) tma_load_4d_if(leader, dst, map, bar, at, row, batch, segment);
+    else tma_load_3d_if(leader, dst, map, bar, at, row, batch);
+  }
   __device__ __forceinline__ void load(uint32_t leader, uint32_t dst, uint32_t bar) {
     if (kind == 0) {
 #pragma unroll
-      for (int kk = 0; kk < KB; ++kk) tma_load_3d_if(leader, dst + kk * (ROWS * kBK * 2), map, bar, inner + kk * kBK, row, batch);
-    } else if (KB == 2 && kind == 1) {
+      for (int kk = 0; kk < KB; ++kk) box(leader, dst + kk * (ROWS * kBK * 2), bar, inner + kk * kBK);
+    } else if (!SEG && KB == 2 && kind == 1) {
       tma_load_4d_if(leader, dst, map, bar, 0, row, inner, batch);
     } else {
 #pragma unroll
-      for (int j = 0; j < ROWS / 64; ++j) tma_load_3d_if(leader, dst + j * (KB * kAtomBytes), map, bar, inner + 64 * j, row, batch);
+      for (int j = 0; j < ROWS / 64; ++j) box(leader, dst + j * (KB * kAtomBytes), bar, inner + 64 * j);
     }
     inner += d_inner;
     row += d_row;
@@ -156,6 +163,25 @@ struct op_symmetric<Op, decltype(void(Op::kSymmetric))> { static constexpr bool 
 template <class Op>
 __host__ __device__ constexpr uint32_t gemm_staging_bytes() {
   return (Op::NOUT + (op_symmetric<Op>::value ? 1 : 0)) * kBM * Op::BT * 2 + Op::kEpiScratch;
+}
+
+// Ops whose launches may cover several runs of tokens ("segments") of the same entries, each with weights of its own, declare
+// `kSegments`: all their maps are 4-D, (columns, rows, entry, segment).
+template <class Op, class = void>
+struct op_segments { static constexpr bool value = false; };
+template <class Op>
+struct op_segments<Op, decltype(void(Op::kSegments))> { static constexpr bool value = Op::kSegments; };
+// batch index -> entry and segment
+template <class Op>
+__device__ __forceinline__ void entry_of(const GemmProblem<Op>& P, int batch, int& entry, int& segment) {
+  entry = batch;
+  segment = 0;
+  if constexpr (op_segments<Op>::value) {
+    if (P.entries > 0) {
+      segment = batch / P.entries;
+      entry = batch - segment * P.entries;
+    }
+  }
 }
 
 // Ops whose contraction may be split over several units (see GemmProblem): direct epilogues, single-phase kernels.
@@ -288,6 +314,8 @@ __device__ __forceinline__ bool gemm_phase(GemmCtx& cx, const GemmProblem<Op>* p
 
   constexpr bool SYM = op_symmetric<Op>::value;
   static_assert(!SYM || (BT == kBM && Op::NOUT == 1 && Deps::kOn), "symmetric ops: 128-wide tiles, one staged output, dataflow");
+  constexpr bool SEG = op_segments<Op>::value;
+  static_assert(!SEG || !Deps::kOn, "segments: one phase");
   constexpr bool SPLIT = op_split<Op>::value;
   static_assert(!SPLIT || (Op::NOUT == 0 && Op::kWarpTranspose && !Deps::kOn), "split contractions: direct epilogue, one phase");
   int tiles_of[kMaxProb], tn_of[kMaxProb], tm_of[kMaxProb], per_batch_of[kMaxProb], splits_of[kMaxProb];
@@ -378,12 +406,14 @@ __device__ __forceinline__ bool gemm_phase(GemmCtx& cx, const GemmProblem<Op>* p
         k_range(P, tc, kb0, kb1);
         const int num_sb = (kb1 - kb0 + KB - 1) / KB;  // ring stages of KB k-blocks
         const bool diagonal = SYM && tc.m0 == tc.n0;
-        OperandCursor<kBM, KB> ca[NA];
-        OperandCursor<BT, KB> cb[NB];
+        OperandCursor<kBM, KB, SEG> ca[NA];
+        OperandCursor<BT, KB, SEG> cb[NB];
+        int entry, segment;
+        entry_of(P, tc.batch, entry, segment);
 #pragma unroll
-        for (int i = 0; i < NA; ++i) ca[i].start(&P.a[i], P.ai[i], tc.m0, kb0 * kBK, tc.batch);
+        for (int i = 0; i < NA; ++i) ca[i].start(&P.a[i], P.ai[i], tc.m0, kb0 * kBK, entry, segment);
 #pragma unroll
-        for (int i = 0; i < NB; ++i) cb[i].start(&P.b[i], P.bi[i], tc.n0, kb0 * kBK, tc.batch);
+        for (int i = 0; i < NB; ++i) cb[i].start(&P.b[i], P.bi[i], tc.n0, kb0 * kBK, entry, segment);
         const uint32_t bytes = diagonal ? KB * NA * kATileBytes : kStageBytes;
         if constexpr (Deps::kOn) {
           if (!__all_sync(0xFFFFFFFFu, flow_wait_verified(cx, cx.ptile++))) { failed = true; break; }  // the scout warp checked this tile
@@ -729,13 +759,17 @@ __device__ __forceinline__ bool gemm_phase(GemmCtx& cx, const GemmProblem<Op>* p
           if (elected) mbar_arrive(&cx.stg_full_bar[0]);  // the storing warp issues the stores and publishes the tile
           ++cx.sround;
         } else if (elected) {
+          int entry, segment;
+          entry_of(P, tc.batch, entry, segment);
 #pragma unroll
           for (int o = 0; o < NOUT; ++o) {
             if (!P.oi[o].enabled || Op::skip_store(ep, o)) continue;
             for (int pnl = 0; pnl < BT / 64; ++pnl) {
               if (tc.n0 + pnl * 64 >= P.N) break;
-              tma_store_3d(&P.out[o], stg + o * (kBM * BT * 2) + pnl * (kBM * 128),
-                           P.oi[o].col_off + tc.n0 + pnl * 64, P.oi[o].row_off + tc.m0, P.oi[o].batch_off + tc.batch);
+              const uint32_t src = stg + o * (kBM * BT * 2) + pnl * (kBM * 128);
+              const int col = P.oi[o].col_off + tc.n0 + pnl * 64, at = P.oi[o].row_off + tc.m0, b = P.oi[o].batch_off + entry;
+              if constexpr (SEG) tma_store_4d(&P.out[o], src, col, at, b, segment);
+              else tma_store_3d(&P.out[o], src, col, at, b);
             }
           }
           bulk_commit_group();
