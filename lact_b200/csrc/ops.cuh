@@ -215,7 +215,10 @@ struct OpDW {
   static constexpr bool kWarpTranspose = true;                   // results reach global memory through `EpiDW::warp_block`
   static constexpr bool kReverseBatch = true;                    // reads the planes the pointwise kernel has just written
   static constexpr uint32_t kEpiScratch = kEpiWarps * 32 * 144;  // one 32 x 32 fp32 block (rows padded to 144 bytes) per epilogue warp
-  static constexpr int KB = kb_per_stage(kATileBytes + BT_ * kBK * 2, kEpiScratch);
+  // One k-block per stage: since box coordinates are worked out once per tile, a box costs the loading warp little, and a
+  // ring of four or five small stages refills sooner than one of two large ones (72 tiles of 25 k-blocks 19.4 -> 17.3 us, a call
+  // with 21 of them 1677 -> 1626; 16 entries of 192 and 49152 tokens 815 -> 766 the whole call, 32 of 384 even).
+  static constexpr int KB = 1;
   static constexpr int STAGES = ring_depth(KB * (kATileBytes + BT_ * kBK * 2), kEpiScratch);
   using Epi = EpiDW;
   __host__ __device__ static constexpr int term_a(int) { return 0; }
