@@ -144,6 +144,11 @@ int make_output(OperandForm form, CUtensorMap* map, OutInfo* info, const Mat& m,
   info->col_off = col_off;
   info->batch_off = batch_off;
   info->enabled = 1;
+  info->ptr = const_cast<bf16*>(static_cast<const bf16*>(m.ptr) + batch_off * m.bs + row_off * m.ld + col_off);
+  info->bs = m.bs;
+  info->ld = static_cast<int32_t>(m.ld);
+  info->wide = (reinterpret_cast<uintptr_t>(info->ptr) & 31) == 0 && m.ld % 16 == 0 && m.bs % 16 == 0;
+  if (m.ld > 0x7FFFFFFF) return LACT_ERR_SHAPE;
   if ((col_off % 8) != 0 || row_off < 0 || col_off < 0) return LACT_ERR_SHAPE;
   return form.segments ? encode_map_segments(map, m, kBM) : encode_map(map, m, kBM);
 }
@@ -869,7 +874,7 @@ int try_ns_fused(const NsGroup* grp, int ngroups, int steps, int const_coeffs, i
                ? launch_ns_fused<128, 192, 2, true>(grp, ngroups, steps, const_coeffs, status, stream, unscaled_first)
                : launch_ns_fused<128, 192, 5, true>(grp, ngroups, steps, const_coeffs, status, stream, unscaled_first, keep);
   if (wide && !symmable && gram_tiles(192) >= want) return LACT_NS_FUSED(192);
-  // (a 256-wide update tile leaves no room for a useful ring next to two staging tiles: 128 is used)
+  // (256-wide update tiles would leave a ring of four stages: 128 is used)
   const bool ok128 = (bt_mm == 192 && bt_mn == 192) || (bt_mm == 128 && (bt_mn == 128 || bt_mn == 256));
   if (ok128 && (gram_tiles(128) >= want || gram_tiles(64) == gram_tiles(128))) return LACT_NS_FUSED(128);
   if (ok128 || (bt_mm == 64 && bt_mn == 64)) return LACT_NS_FUSED(64);

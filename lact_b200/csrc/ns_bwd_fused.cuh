@@ -30,17 +30,10 @@ __host__ __device__ constexpr uint32_t ns_bwd_stride() {
                                                                                : gemm_stage_bytes<OpNs2<BT>>();
 }
 template <int BT_MM, int BT, bool SYM>
-__host__ __device__ constexpr uint32_t ns_bwd_staging() {
-  return gemm_staging_bytes<OpNs2T<BT_MM, SYM>>() > gemm_staging_bytes<OpNs2<BT>>() ? gemm_staging_bytes<OpNs2T<BT_MM, SYM>>()
-                                                                                   : gemm_staging_bytes<OpNs2<BT>>();
-}
-template <int BT_MM, int BT, bool SYM>
-__host__ __device__ constexpr int ns_bwd_ring() {
-  return static_cast<int>((232448u - 1024u - 256u - ns_bwd_staging<BT_MM, BT, SYM>()) / ns_bwd_stride<BT_MM, BT, SYM>());
-}
+__host__ __device__ constexpr int ns_bwd_ring() { return flow_ring(ns_bwd_stride<BT_MM, BT, SYM>()); }
 template <int BT_MM, int BT, bool SYM>
 __host__ __device__ constexpr uint32_t ns_bwd_smem_bytes() {
-  return ns_bwd_ring<BT_MM, BT, SYM>() * ns_bwd_stride<BT_MM, BT, SYM>() + ns_bwd_staging<BT_MM, BT, SYM>() + 1024 + 256;
+  return ns_bwd_ring<BT_MM, BT, SYM>() * ns_bwd_stride<BT_MM, BT, SYM>() + kFlowScratch + 1024 + 256;
 }
 
 template <int BT_MM, int BT, int NITER, bool SYM>
@@ -55,7 +48,7 @@ ns_bwd_fused_kernel(const __grid_constant__ NsBwdFusedArgs<BT_MM, BT, NITER, SYM
   if (__syncthreads_or(*reinterpret_cast<volatile int32_t*>(args.status) != kStatusOk)) return;  // (all threads of the CTA or none)
   extern __shared__ uint8_t smem_raw[];
   GemmCtx cx;
-  gemm_setup(cx, smem_raw, RING, ns_bwd_stride<BT_MM, BT, SYM>(), ns_bwd_staging<BT_MM, BT, SYM>(), kTmemCols);
+  gemm_setup(cx, smem_raw, RING, ns_bwd_stride<BT_MM, BT, SYM>(), kFlowScratch, kTmemCols);
   bool failed = false;
   NsPatch patch;
   FlowDeps deps;

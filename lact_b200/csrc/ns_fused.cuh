@@ -47,19 +47,10 @@ __host__ __device__ constexpr uint32_t ns_fused_stage_stride() {
                                                                                 : gemm_stage_bytes<OpNs<BT_MN>>();
 }
 template <int BT_MM, int BT_MN, bool SYM = false>
-__host__ __device__ constexpr uint32_t ns_fused_staging() {
-  return gemm_staging_bytes<OpNsT<BT_MM, SYM>>() > gemm_staging_bytes<OpNs<BT_MN>>() ? gemm_staging_bytes<OpNsT<BT_MM, SYM>>()
-                                                                                    : gemm_staging_bytes<OpNs<BT_MN>>();
-}
-template <int BT_MM, int BT_MN, bool SYM = false>
-__host__ __device__ constexpr int ns_fused_ring() {
-  return static_cast<int>((232448u - 1024u - 256u - ns_fused_staging<BT_MM, BT_MN, SYM>()) /
-                          ns_fused_stage_stride<BT_MM, BT_MN, SYM>());
-}
+__host__ __device__ constexpr int ns_fused_ring() { return flow_ring(ns_fused_stage_stride<BT_MM, BT_MN, SYM>()); }
 template <int BT_MM, int BT_MN, bool SYM = false>
 __host__ __device__ constexpr uint32_t ns_fused_smem_bytes() {
-  return ns_fused_ring<BT_MM, BT_MN, SYM>() * ns_fused_stage_stride<BT_MM, BT_MN, SYM>() +
-         ns_fused_staging<BT_MM, BT_MN, SYM>() + 1024 + 256;
+  return ns_fused_ring<BT_MM, BT_MN, SYM>() * ns_fused_stage_stride<BT_MM, BT_MN, SYM>() + kFlowScratch + 1024 + 256;
 }
 
 template <int BT_MM, int BT_MN, int NITER, bool SYM = false>
@@ -75,7 +66,7 @@ ns_fused_kernel(const __grid_constant__ NsFusedArgs<BT_MM, BT_MN, NITER, SYM> ar
   if (__syncthreads_or(*reinterpret_cast<volatile int32_t*>(args.status) != kStatusOk)) return;  // (all threads of the CTA or none)
   extern __shared__ uint8_t smem_raw[];
   GemmCtx cx;
-  gemm_setup(cx, smem_raw, RING, kStride, ns_fused_staging<BT_MM, BT_MN, SYM>(), kTmemCols);
+  gemm_setup(cx, smem_raw, RING, kStride, kFlowScratch, kTmemCols);
   if (threadIdx.x == 32) {
     for (int par = 0; par < (NITER < 2 ? NITER : 2); ++par)
       for (int g = 0; g < args.ngroups; ++g) {
@@ -83,11 +74,8 @@ ns_fused_kernel(const __grid_constant__ NsFusedArgs<BT_MM, BT_MN, NITER, SYM> ar
         tma_prefetch_desc(&args.gram[par][g].b[0]);
         tma_prefetch_desc(&args.upd[par][g].a[0]);
         tma_prefetch_desc(&args.upd[par][g].b[0]);
-        tma_prefetch_desc(&args.gram[par][g].out[0]);
-        tma_prefetch_desc(&args.upd[par][g].out[0]);
         tma_prefetch_desc(&args.poly[par][g].a[0]);
         tma_prefetch_desc(&args.poly[par][g].b[0]);
-        tma_prefetch_desc(&args.poly[par][g].out[0]);
       }
   }
   bool failed = false;
@@ -128,7 +116,6 @@ ns_fused_kernel(const __grid_constant__ NsFusedArgs<BT_MM, BT_MN, NITER, SYM> ar
     for (int g = 0; g < 2; ++g) deps.need[g] += tiles_mn[g];
   }
   if (failed) *cx.abort_flag = 1;
-  // (the storing thread published every tile of this CTA after its stores had landed)
 
   gemm_teardown(cx, failed, args.status, kTmemCols);
 }

@@ -6,8 +6,6 @@
 
 namespace lact {
 
-using bf16 = __nv_bfloat16;
-
 // one value of an fp32 or bf16 vector
 __device__ __forceinline__ float load_scalar(const void* p, int is_f32, int64_t idx) {
   return is_f32 ? reinterpret_cast<const float*>(p)[idx] : __bfloat162float(reinterpret_cast<const bf16*>(p)[idx]);
@@ -167,12 +165,6 @@ struct EpiFwGrad {
 // Ops without global epilogue operands prefetch nothing.
 struct NoPrefetch {};
 
-// k-blocks per ring stage: two when two such stages fit next to `staging` bytes (each operand tile of a
-// stage then arrives as ONE TMA box spanning both k-blocks: the load path is bound by the number of
-// boxes, not by bytes), else one
-__host__ __device__ constexpr int kb_per_stage(uint32_t kblock_bytes, uint32_t staging) {
-  return (232448u - 1024u - 256u - staging) / (2 * kblock_bytes) >= 2 ? 2 : 1;
-}
 // ring depth that fits 227 KB next to `staging` bytes of output tiles
 __host__ __device__ constexpr int ring_depth(uint32_t stage_bytes, uint32_t staging) {
   return static_cast<int>((232448u - 1024u - 256u - staging) / stage_bytes) > 8
@@ -316,9 +308,8 @@ struct OpNsT {
   static constexpr bool kWarpTranspose = false, kReverseBatch = false;
   static constexpr bool kSymmetric = SYM_;
   static constexpr uint32_t kEpiScratch = 0;
-  static constexpr uint32_t kStagingTiles = (SYM_ ? 2 : 1) * kBM * BT_ * 2;
-  static constexpr int KB = kb_per_stage(kATileBytes + BT_ * kBK * 2, kStagingTiles);
-  static constexpr int STAGES = ring_depth(KB * (kATileBytes + BT_ * kBK * 2), kStagingTiles);
+  static constexpr int KB = 1;
+  static constexpr int STAGES = ring_depth(kATileBytes + BT_ * kBK * 2, kBM * BT_ * 2);  // (one launch per product)
   using Epi = EpiNs;
   __host__ __device__ static constexpr int diag_a(int) { return 0; }  // S = X X^T, P ~ S S: one matrix on both sides
   __host__ __device__ static constexpr int term_a(int) { return 0; }
@@ -339,8 +330,15 @@ struct OpNsT {
   }
   __device__ static __forceinline__ void epilogue_staged(const Epi& ep, int, int row, int col, int, int,
                                                          const float (&v)[1][32], float (&o)[1][32], Prefetch& pf) {
+    // (the diagonal passes through a warp's 32 rows and columns from corner to corner or not at all; the store rounds)
+    const int on = row - col;
+    if (on - static_cast<int>(threadIdx.x & 31) == 0 && ep.diag != 0.f) {
 #pragma unroll
-    for (int j = 0; j < 32; ++j) o[0][j] = bf16_round(v[0][j] * pf.sc + (row == col + j ? ep.diag : 0.f));
+      for (int j = 0; j < 32; ++j) o[0][j] = v[0][j] * pf.sc + (on == j ? ep.diag : 0.f);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) o[0][j] = v[0][j] * pf.sc + 0.f;
+    }
   }
 };
 
@@ -357,7 +355,7 @@ struct OpNs2T {
   static constexpr bool kSymmetric = SYM_;
   static constexpr uint32_t kEpiScratch = 0;
   static constexpr int KB = 1;
-  static constexpr int STAGES = ring_depth(2 * (kATileBytes + BT_ * kBK * 2), (SYM_ ? 2 : 1) * kBM * BT_ * 2);
+  static constexpr int STAGES = ring_depth(2 * (kATileBytes + BT_ * kBK * 2), kBM * BT_ * 2);
   using Epi = EpiNs;
   __host__ __device__ static constexpr int diag_a(int b) { return 1 - b; }  // U V^T + V U^T: a0 = b1 = U, a1 = b0 = V
   __host__ __device__ static constexpr int term_a(int t) { return t; }

@@ -143,6 +143,15 @@ __device__ __forceinline__ void fence_async_proxy() {
   // makes generic-proxy shared-memory writes visible to the async proxy (TMA / tcgen05.mma)
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
+// 16 and 32 bytes to global memory (aligned to their size)
+__device__ __forceinline__ void st_global_16(void* p, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.global.v4.b32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+__device__ __forceinline__ void st_global_32(void* p, const uint32_t* w) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]),
+               "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+               : "memory");
+}
 __device__ __forceinline__ void tc_fence_before() {
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
 }

@@ -13,6 +13,8 @@
 
 namespace lact {
 
+using bf16 = __nv_bfloat16;
+
 constexpr int kBM = 128;   // UMMA M (rows of the accumulator = TMEM lanes)
 constexpr int kBK = 64;    // k-block: 64 bf16 = 128 bytes = one swizzle row
 constexpr int kUmmaK = 16; // K of one tcgen05.mma for 16-bit operands
@@ -29,8 +31,12 @@ struct OperandInfo {
 
 // Where a staged (TMA-stored) output tile lands: tile (m0, n0) of batch entry b is stored at
 // coordinates (col_off + n0, row_off + m0, batch_off + b) of the output map, whose extents clip it.
+// Dataflow kernels store from registers instead: element (r, c) of entry b at ptr[b * bs + r * ld + c].
 struct OutInfo {
   int32_t row_off, col_off, batch_off, enabled;
+  void* ptr;
+  int64_t bs;
+  int32_t ld, wide;  // wide: rows start on 32 bytes
 };
 
 template <class Op>
@@ -90,7 +96,14 @@ constexpr int kEpiWarps = 8;
 constexpr int kGemmThreadsV2 = 64 + 32 * kEpiWarps;  // producer warp + MMA warp + epilogue warps
 // dataflow kernels add a scout warp that walks the tile sequence ahead of the producer and checks
 // every tile's dependency, so that the global-memory latency of that check never stalls the loads
-constexpr int kGemmThreadsFlow = kGemmThreadsV2 + 64;  // + dependency scout warp + storing warp
+constexpr int kGemmThreadsFlow = kGemmThreadsV2 + 32;
+constexpr uint32_t kFlowScratch = kEpiWarps * 32 * 80;  // a 32 x 32 bf16 block (rows padded to 80 bytes) per epilogue warp
+// ring stages of `stride` bytes beside that scratch
+__host__ __device__ constexpr int flow_ring(uint32_t stride) {
+  return static_cast<int>((232448u - 1024u - 256u - kFlowScratch) / stride) > 8
+             ? 8
+             : static_cast<int>((232448u - 1024u - 256u - kFlowScratch) / stride);
+}
 
 // One operand tile of a ring stage: ROWS (mn) x KB k-blocks.  Shared-memory layout:
 //   K-major:  [k-block][ROWS rows][64 k] (KB tiles of ROWS x 128 bytes back to back);
@@ -150,7 +163,7 @@ struct TileCoord {
 
 // Ops whose output is a symmetric M x M matrix (both operands the same rows) may declare `kSymmetric`: only the
 // 128 x 128 tiles on and above the diagonal are computed, and every off-diagonal tile is stored twice, as it is and
-// transposed (from a second staging tile the epilogue fills).  Needs BT = 128, one staged output, dataflow mode.
+// transposed.  Needs BT = 128, one staged output, dataflow mode.
 // On the diagonal the B tiles are the very rows of the A tiles, read the same way: they are not loaded a second time, the
 // products read A tile `diag_a(b)` in place of B tile b.  At three row blocks half of the computed tiles lie on the diagonal: a
 // quarter of the operand bytes of these phases, worth 0.4 % of a forward and 0.8 % of a training step at 32 units of 384 (the
@@ -162,7 +175,7 @@ struct op_symmetric<Op, decltype(void(Op::kSymmetric))> { static constexpr bool 
 
 template <class Op>
 __host__ __device__ constexpr uint32_t gemm_staging_bytes() {
-  return (Op::NOUT + (op_symmetric<Op>::value ? 1 : 0)) * kBM * Op::BT * 2 + Op::kEpiScratch;
+  return Op::NOUT * kBM * Op::BT * 2 + Op::kEpiScratch;
 }
 
 // Ops whose launches may cover several runs of tokens ("segments") of the same entries, each with weights of its own, declare
@@ -207,14 +220,12 @@ struct GemmCtx {
   uint32_t stage_stride;  // bytes between ring stages (>= the op's stage bytes)
   uint32_t staging;       // 1024-byte aligned start of the output staging tiles
   uint64_t *full_bar, *empty_bar, *acc_full_bar, *acc_empty_bar;
-  uint64_t *stg_full_bar, *stg_empty_bar;  // dataflow kernels: staging tile handed to / returned by the storing warp
-  volatile uint32_t* abort_flag;
+  volatile uint32_t* abort_flag;  // [0] raised by anyone, [1], [2] by epilogue warps only
   uint32_t tmem_base;
   uint32_t slot = 0, phase = 0, tcount = 0;  // ring stage in turn and its phase; output tiles so far
   // dataflow mode (multi-phase kernels whose phases are ordered by completion counters, see FlowDeps)
   uint32_t rot = 0;              // tiles handed out by earlier phases, modulo the grid size
   uint32_t ptile = 0;            // tiles whose dependency has been verified (scout) / consumed (producer)
-  uint32_t sround = 0;           // staging hand-overs so far (epilogue threads and the storing thread count alike)
   uint32_t* dep_ok = nullptr;    // shared-memory word: tiles verified by the scout warp, read by the producer thread
   volatile uint32_t* last_unit = nullptr;  // shared-memory word: this unit completes its tile (split contractions)
   template <int RING>
@@ -229,8 +240,8 @@ struct NoPatch {
 };
 
 // Phase ordering of a multi-phase kernel without grid-wide barriers.  Every (problem, batch entry)
-// owns a completion counter in global memory; a tile's stores are followed (once they have landed)
-// by one increment of its batch entry's counter, and a tile of a later phase may load only after the
+// owns a completion counter in global memory; a tile's stores are followed by one releasing increment
+// of its batch entry's counter, and a tile of a later phase may load only after the
 // counter of its batch entry has reached `need` = the number of tiles all earlier phases produce for
 // that entry.  The phases of a batch entry must form a chain (each phase reads only what earlier
 // phases of the same entry wrote, and overwrites only what earlier phases of the same entry read).
@@ -249,6 +260,9 @@ __device__ __forceinline__ uint32_t ld_acquire_gpu_u32(const uint32_t* p) {
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
+__device__ __forceinline__ void red_release_gpu_u32(uint32_t* p, uint32_t v) {
+  asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
 __device__ __forceinline__ uint32_t ld_acquire_cta_shared_u32(const uint32_t* p) {
   uint32_t v;
   asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(smem_u32(p)) : "memory");
@@ -265,13 +279,6 @@ __device__ __forceinline__ bool dep_wait(const uint32_t* ctr, uint32_t need, vol
     if (ld_acquire_gpu_u32(ctr) >= need) return true;
     if ((i & 31u) == 0 && (*abort_flag != 0 || !clock.within_limit())) return false;
   }
-}
-// Storing thread: once all its stores have landed, publish the completion of a tile.
-__device__ __forceinline__ void flow_publish(uint32_t* counter) {
-  bulk_wait_all();
-  asm volatile("fence.proxy.async;" ::: "memory");
-  __threadfence();
-  atomicAdd(counter, 1u);
 }
 // Producer thread: bounded wait until the scout warp has verified the dependency of the tile with
 // running number `seq` (0-based).
@@ -417,7 +424,7 @@ __device__ __forceinline__ bool gemm_phase(GemmCtx& cx, const GemmProblem<Op>* p
         const uint32_t bytes = diagonal ? KB * NA * kATileBytes : kStageBytes;
         if constexpr (Deps::kOn) {
           if (!__all_sync(0xFFFFFFFFu, flow_wait_verified(cx, cx.ptile++))) { failed = true; break; }  // the scout warp checked this tile
-          asm volatile("fence.proxy.async;" ::: "memory");
+          asm volatile("fence.proxy.async.global;" ::: "memory");
         }
         for (int sb = 0; sb < num_sb; ++sb) {
           if (!mbar_wait_warp(&cx.empty_bar[cx.slot], cx.phase ^ 1, cx.abort_flag)) { failed = true; break; }
@@ -496,10 +503,10 @@ __device__ __forceinline__ bool gemm_phase(GemmCtx& cx, const GemmProblem<Op>* p
         ++cx.tcount;
       }
     }
-  } else if (warp == 2 + kEpiWarps) {
-    // ---------------- dependency scout (dataflow kernels only): one thread verifies, in tile order,
-    // that every tile's inputs are complete and publishes the count of verified tiles
-    if constexpr (Deps::kOn) {
+  } else if constexpr (Deps::kOn) {
+    if (warp == 2 + kEpiWarps) {
+      // ---------------- dependency scout (dataflow kernels only): one thread verifies, in tile order,
+      // that every tile's inputs are complete and publishes the count of verified tiles
       if (lane == 0) {
         for (int tile_i = 0; tile_i < rounds && !failed; ++tile_i) {
           const int tile = tile_at(tile_i);
@@ -509,49 +516,98 @@ __device__ __forceinline__ bool gemm_phase(GemmCtx& cx, const GemmProblem<Op>* p
           st_release_cta_shared_u32(cx.dep_ok, ++cx.ptile);
         }
       }
+      return failed;
     }
-  } else if (warp > 2 + kEpiWarps) {
-    // ---------------- storing thread (dataflow kernels only): takes each staged tile from the epilogue
-    // warps, issues its TMA stores, returns the staging tile as soon as the stores have read it, and
-    // publishes the tile's completion as soon as they have landed -- the epilogue warps never wait for
-    // global memory, and no CTA can wait on a tile it has not yet published itself
-    if constexpr (Deps::kOn && Op::NOUT > 0) {
-      if (lane == 0) {
-        for (int tile_i = 0; tile_i < rounds && !failed; ++tile_i) {
-          const int tile = tile_at(tile_i);
-          if (tile >= total_tiles) continue;
-          const TileCoord tc = coord(tile);
-          const GemmProblem<Op>& P = probs[tc.prob];
-          typename Op::Epi ep = P.ep;
-          patch(ep, tc.prob);
-          const uint32_t stg = cx.staging;
-          if (!mbar_wait(&cx.stg_full_bar[0], cx.sround & 1, cx.abort_flag)) { failed = true; break; }
+    // ---------------- epilogue of a dataflow tile: rounded rows go from registers straight to global memory, 64 bytes per thread
+    // and 32 columns.  What counts here is how soon the next phase of the matrix may load.  Clocks inside the kernel at 8 matrices of
+    // side 384 (a tile per SM and phase): bulk stores from a staging tile took 3170 clocks from the hand-over to the counter, and
+    // 5300 with the chip full; stores from registers and the release take 1470.  The loading warp's fence between counter and
+    // loads, for global memory alone, costs 900 clocks less than one for all proxies' state spaces.  Without staging tiles the
+    // ring takes all of shared memory.  8 matrices 97.6 -> 72.9 us a launch, 64 of them (power-limited in a long call) 197 -> 160.
+    static_assert(Op::NOUT == 1, "one output");
+    const int quarter = warp & 3, half = (warp - 2) >> 2, row_local = quarter * 32 + lane;
+    const uint32_t scratch = cx.staging + (warp - 2) * (32 * 80);
+    for (int tile_i = 0; tile_i < rounds; ++tile_i) {
+      const int tile = tile_at(tile_i);
+      if (tile >= total_tiles) continue;
+      const TileCoord tc = coord(tile);
+      const GemmProblem<Op>& P = probs[tc.prob];
+      typename Op::Epi ep = P.ep;
+      patch(ep, tc.prob);
+      const uint32_t as = cx.tcount & 1, aph = (cx.tcount >> 1) & 1;
+      const int row = tc.m0 + row_local;
+      typename Op::Prefetch pf;
+      Op::prefetch(ep, tc.batch, row, tc.n0, half, P.M, P.N, pf);
+      // A warp whose wait ran out tells the others at the tile's barrier, in the word of the tile's parity: by the time it could
+      // raise that word for another tile, all of them have looked.
+      const bool got = mbar_wait(&cx.acc_full_bar[as], aph, cx.abort_flag);
+      if (!got) cx.abort_flag[1 + as] = 1;
+      tc_fence_after();
+      const uint32_t acc_base = cx.tmem_base + as * kAccStride + (static_cast<uint32_t>(quarter * 32) << 16);
+      const int64_t ld = P.oi[0].ld;
+      bf16* const out = static_cast<bf16*>(P.oi[0].ptr) + tc.batch * P.oi[0].bs;
+      const bool wide = P.oi[0].wide != 0;
+      auto release = [&]() {  // all TMEM reads of this warp are complete: hand the buffer back
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&cx.acc_empty_bar[as]);
+      };
+      if (tc.n0 + half * 32 >= P.N) release();
+      for (int c = half * 32; c < BT; c += 64) {
+        const int left = P.N - (tc.n0 + c);  // columns; a multiple of 8
+        if (left <= 0) break;                // warp-uniform
+        float v[1][32], ov[1][32];
+        {
+          uint32_t bits[32];
+          tmem_ld32(acc_base + c, bits);
+          tmem_ld_wait();
 #pragma unroll
-          for (int o = 0; o < Op::NOUT; ++o) {
-            if (!P.oi[o].enabled || Op::skip_store(ep, o)) continue;
-            for (int pnl = 0; pnl < BT / 64; ++pnl) {
-              if (tc.n0 + pnl * 64 >= P.N) break;
-              tma_store_3d(&P.out[o], stg + o * (kBM * BT * 2) + pnl * (kBM * 128), P.oi[o].col_off + tc.n0 + pnl * 64,
-                           P.oi[o].row_off + tc.m0, P.oi[o].batch_off + tc.batch);
-            }
+          for (int j = 0; j < 32; ++j) v[0][j] = __uint_as_float(bits[j]);
+        }
+        if (c + 64 >= BT || left <= 64) release();
+        Op::epilogue_staged(ep, tc.batch, row, tc.n0 + c, P.M, P.N, v, ov, pf);
+        uint32_t w[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) w[j] = pack_bf16x2(ov[0][2 * j], ov[0][2 * j + 1]);
+        if (got && row < P.M) {
+          bf16* const p = out + row * ld + tc.n0 + c;
+          if (wide && left >= 32) {
+            st_global_32(p, w);
+            st_global_32(p + 16, w + 8);
+          } else {
+#pragma unroll
+            for (int g = 0; g < 4; ++g)
+              if (g * 8 < left) st_global_16(p + g * 8, w[4 * g], w[4 * g + 1], w[4 * g + 2], w[4 * g + 3]);
           }
-          if constexpr (SYM) {
-            // the transposed tile (second staging tile) goes below the diagonal
-            if (tc.m0 != tc.n0) {
-              for (int pnl = 0; pnl < BT / 64; ++pnl) {
-                if (tc.m0 + pnl * 64 >= P.N) break;
-                tma_store_3d(&P.out[0], stg + kBM * BT * 2 + pnl * (kBM * 128), P.oi[0].col_off + tc.m0 + pnl * 64,
-                             P.oi[0].row_off + tc.n0, P.oi[0].batch_off + tc.batch);
-              }
+        }
+        if constexpr (SYM) {
+          if (tc.m0 != tc.n0) {  // the block transposed: through the warp's scratch, four lanes per row of 64 bytes
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              const uint16_t h = static_cast<uint16_t>((j & 1) ? w[j >> 1] >> 16 : w[j >> 1]);
+              asm volatile("st.shared.b16 [%0], %1;" ::"r"(scratch + j * 80 + lane * 2), "h"(h) : "memory");
             }
+            __syncwarp();
+            const int u = lane & 3, col = tc.m0 + quarter * 32 + u * 8;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const int rr = i * 8 + (lane >> 2), at = tc.n0 + c + rr;
+              uint32_t x[4];
+              asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                           : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3])
+                           : "r"(scratch + rr * 80 + u * 16)
+                           : "memory");
+              if (got && at < P.N && col < P.M) st_global_16(out + at * ld + col, x[0], x[1], x[2], x[3]);
+            }
+            __syncwarp();
           }
-          bulk_commit_group();
-          bulk_wait_read_all();
-          mbar_arrive(&cx.stg_empty_bar[0]);
-          ++cx.sround;
-          flow_publish(deps.counter[tc.prob] + tc.batch);
         }
       }
+      // (the loading warps of other SMs have the proxy fence between the counter and their bulk loads of these rows)
+      named_barrier_sync(2, kEpiWarps * 32);
+      if (cx.abort_flag[1 + as] != 0) { failed = true; break; }
+      if (threadIdx.x == 64) red_release_gpu_u32(deps.counter[tc.prob] + tc.batch, 1u);
+      ++cx.tcount;
     }
   } else {
     // ---------------- epilogue: warp w may only touch TMEM lanes [32*(w%4), 32*(w%4)+32); the two
@@ -604,14 +660,7 @@ __device__ __forceinline__ bool gemm_phase(GemmCtx& cx, const GemmProblem<Op>* p
         // a flag that only epilogue warps write, and every warp decides after the barrier.
         if (!got) cx.abort_flag[1] = 1;
         // the previous tile's stores must have finished reading the staging tile
-        if (elected) {
-          if constexpr (Deps::kOn) {
-            // the storing warp returns the staging tile once its stores have read it
-            if (cx.sround > 0 && !mbar_wait(&cx.stg_empty_bar[0], (cx.sround - 1) & 1, cx.abort_flag)) cx.abort_flag[1] = 1;
-          } else {
-            bulk_wait_read_all();
-          }
-        }
+        if (elected) bulk_wait_read_all();
         named_barrier_sync(1, kEpiThreads);
         if (cx.abort_flag[1] != 0) { failed = true; break; }
       } else {
@@ -717,21 +766,6 @@ __device__ __forceinline__ bool gemm_phase(GemmCtx& cx, const GemmProblem<Op>* p
                            : "memory");
             }
           }
-          if constexpr (SYM) {
-            if (tc.m0 != tc.n0) {
-              // element (row_local, c + j) lands at (c + j, row_local) of the second staging tile: the 32 lanes of a
-              // warp write 32 consecutive columns of one row (64 contiguous bytes)
-              const uint32_t tbase = stg + kBM * BT * 2 + (row_local >> 6) * (kBM * 128) + (row_local & 7) * 2;
-              const uint32_t tunit = (row_local & 63) >> 3;
-#pragma unroll
-              for (int j = 0; j < 32; ++j) {
-                const uint32_t rt = c + j;
-                const uint32_t addr = tbase + rt * 128 + ((tunit ^ (rt & 7)) << 4);
-                const __nv_bfloat16 hv = __float2bfloat16_rn(ov[0][j]);
-                asm volatile("st.shared.b16 [%0], %1;" ::"r"(addr), "h"(*reinterpret_cast<const uint16_t*>(&hv)) : "memory");
-              }
-            }
-          }
         } else {
           if constexpr (Op::kWarpTranspose)
             Op::epilogue_warp(ep, tc.batch, tc.m0 + quarter * 32, tc.n0 + c, P.M, P.N, v, pf,
@@ -755,10 +789,7 @@ __device__ __forceinline__ bool gemm_phase(GemmCtx& cx, const GemmProblem<Op>* p
       if constexpr (NOUT > 0) {
         fence_async_proxy();
         named_barrier_sync(2, kEpiThreads);
-        if constexpr (Deps::kOn) {
-          if (elected) mbar_arrive(&cx.stg_full_bar[0]);  // the storing warp issues the stores and publishes the tile
-          ++cx.sround;
-        } else if (elected) {
+        if (elected) {
           int entry, segment;
           entry_of(P, tc.batch, entry, segment);
 #pragma unroll
@@ -777,7 +808,7 @@ __device__ __forceinline__ bool gemm_phase(GemmCtx& cx, const GemmProblem<Op>* p
       }
       ++cx.tcount;
     }
-    if constexpr (NOUT > 0 && !Deps::kOn) {
+    if constexpr (NOUT > 0) {
       if (elected) bulk_wait_all();  // this CTA's output tiles are in global memory
     }
   }
@@ -797,12 +828,10 @@ __device__ __forceinline__ void gemm_setup(GemmCtx& cx, uint8_t* smem_raw, int r
   cx.empty_bar = cx.full_bar + ring;
   cx.acc_full_bar = cx.empty_bar + ring;    // [2]
   cx.acc_empty_bar = cx.acc_full_bar + 2;   // [2]
-  cx.stg_full_bar = cx.acc_empty_bar + 2;   // [1]
-  cx.stg_empty_bar = cx.stg_full_bar + 1;   // [1]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(cx.stg_empty_bar + 1);
-  cx.abort_flag = tmem_slot + 1;  // [2]
-  cx.dep_ok = tmem_slot + 3;
-  cx.last_unit = tmem_slot + 4;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(cx.acc_empty_bar + 2);
+  cx.abort_flag = tmem_slot + 1;  // [3]
+  cx.dep_ok = tmem_slot + 4;
+  cx.last_unit = tmem_slot + 5;
   if (threadIdx.x == 0) {
     for (int s = 0; s < ring; ++s) {
       mbar_init(&cx.full_bar[s], 1);
@@ -812,10 +841,9 @@ __device__ __forceinline__ void gemm_setup(GemmCtx& cx, uint8_t* smem_raw, int r
       mbar_init(&cx.acc_full_bar[s], 1);
       mbar_init(&cx.acc_empty_bar[s], kEpiWarps);
     }
-    mbar_init(&cx.stg_full_bar[0], 1);
-    mbar_init(&cx.stg_empty_bar[0], 1);
     cx.abort_flag[0] = 0;
     cx.abort_flag[1] = 0;
+    cx.abort_flag[2] = 0;
     *cx.dep_ok = 0;
     fence_mbar_init();
   }
