@@ -866,16 +866,20 @@ int try_ns_fused(const NsGroup* grp, int ngroups, int steps, int const_coeffs, i
   // (measured at D = H = 384: 16 and 12 units, i.e. under 1.5 Gram tiles of width 192 per SM) the symmetric phases
   // leave a second, nearly empty round of tiles and plain 128-wide tiles are 4-5 % faster; from 20 units up the
   // symmetric variant wins.
+  // Gram sides that 256 divides run on the same tiles; the training forward (`keep`) refuses them as it always has.  One launch per
+  // product took, with four updates of square matrices (us per call, launches / this kernel): side 256, 1 unit 594 / 396, 16 units
+  // 630 / 498, 32 units 810 / 710; side 512 673 / 461, 1434 / 1303, 2740 / 2414.  (Three tiles of four are no gain: 256 stays plain.)
+  const bool by256 = keep == nullptr && bt_mm == 256 && bt_mn != 64;
   const bool wide = bt_mm == 192 && bt_mn == 192;
-  bool symmable = wide;
-  for (int g = 0; g < ngroups; ++g) symmable = symmable && grp[g].m % kBM == 0 && grp[g].m >= 2 * kBM;
+  bool symmable = wide || by256;
+  for (int g = 0; g < ngroups; ++g) symmable = symmable && grp[g].m % kBM == 0 && grp[g].m >= 3 * kBM;
   if (symmable && gram_tiles(192) >= static_cast<int64_t>(sm_count()) * 3 / 2)
     return keep == nullptr
                ? launch_ns_fused<128, 192, 2, true>(grp, ngroups, steps, const_coeffs, status, stream, unscaled_first)
                : launch_ns_fused<128, 192, 5, true>(grp, ngroups, steps, const_coeffs, status, stream, unscaled_first, keep);
   if (wide && !symmable && gram_tiles(192) >= want) return LACT_NS_FUSED(192);
   // (256-wide update tiles would leave a ring of four stages: 128 is used)
-  const bool ok128 = (bt_mm == 192 && bt_mn == 192) || (bt_mm == 128 && (bt_mn == 128 || bt_mn == 256));
+  const bool ok128 = wide || by256 || (bt_mm == 128 && (bt_mn == 128 || bt_mn == 256));
   if (ok128 && (gram_tiles(128) >= want || gram_tiles(64) == gram_tiles(128))) return LACT_NS_FUSED(128);
   if (ok128 || (bt_mm == 64 && bt_mn == 64)) return LACT_NS_FUSED(64);
 #undef LACT_NS_FUSED
