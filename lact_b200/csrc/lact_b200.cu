@@ -14,7 +14,7 @@
 #include <vector>
 
 #include "../../include/lact_b200.h"
-#include "f32_gemm.cuh"
+#include "f32_split.cuh"
 #include "ns_bwd_fused.cuh"
 #include "ns_chip.cuh"
 #include "pair_gemm.cuh"
@@ -1607,7 +1607,7 @@ int scan_fwd(const lact_scan_config& c, const lact_scan_io& io, int32_t n_steps,
 }
 
 // ------------------------------------------------------------------------------------------
-// fp32 mode: the same step programs on fp32 activations (FFMA contractions, f32_gemm.cuh)
+// fp32 mode: the same step programs on fp32 activations (contractions in bf16 pieces, f32_split.cuh)
 // ------------------------------------------------------------------------------------------
 F32Mat f32_mat(const float* p, int64_t ld, int64_t bs, int t, int64_t rows, int64_t k) {
   const int64_t contiguous = t ? rows : k;
@@ -1615,28 +1615,87 @@ F32Mat f32_mat(const float* p, int64_t ld, int64_t bs, int t, int64_t rows, int6
   return F32Mat{p, ld, bs, t, vec ? 1 : 0};
 }
 
-template <int MODE>
-int launch_f32_gemm(F32Args& a, cudaStream_t stream) {
-  const dim3 grid(ceil_div(a.N, MODE == kF32Store ? kFN : 32), ceil_div(a.M, kFM), static_cast<unsigned>(a.batch * a.splits));
-  if (a.M < 1 || a.N < 1 || a.K < 1 || grid.y > 65535 || static_cast<int64_t>(a.batch) * a.splits > 65535) return LACT_ERR_SHAPE;
-  a.c_vec = (reinterpret_cast<uintptr_t>(a.c) & 15) == 0 && (a.c_ld % 4) == 0 && (a.c_bs % 4) == 0;
+template <int MODE, int BT>
+int launch_cut_gemm(CutArgs& a, cudaStream_t stream) {
+  auto kernel = cut_gemm_kernel<MODE, BT>;
+  constexpr uint32_t smem = CutTile<MODE, BT>::kSmem;
+  static_assert(smem <= 232448, "shared memory budget exceeded");
+  static std::mutex mu;
+  static bool configured[64] = {false};
+  int dev = 0;
+  LACT_CUDA(cudaGetDevice(&dev));
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    if (dev >= 64 || !configured[dev]) {
+      LACT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+      if (dev < 64) configured[dev] = true;
+    }
+  }
+  int64_t units = 0;
+  for (int i = 0; i < a.nprob; ++i) {
+    CutProblem& P = a.prob[i];
+    if (P.M < 1 || P.N < 1 || P.K < 1 || ceil_div(P.M, kBM) > 65535 || static_cast<int64_t>(P.batch) * P.splits > 65535)
+      return LACT_ERR_SHAPE;
+    auto starts_on = [&](int bytes) {
+      return reinterpret_cast<uintptr_t>(P.c) % bytes == 0 && P.c_ld % (bytes / 4) == 0 && P.c_bs % (bytes / 4) == 0;
+    };
+    P.c_vec = starts_on(32) ? 2 : starts_on(16) ? 1 : 0;
+    units += static_cast<int64_t>(ceil_div(P.M, kBM)) * ceil_div(P.N, CutTile<MODE, BT>::kOut) * P.batch * P.splits;
+  }
+  if (units > (1ll << 30)) return LACT_ERR_SHAPE;
   KernelScope scope(kClsOther, stream);
-  LACT_CUDA(launch_pdl(f32_gemm_kernel<MODE>, grid, dim3(kFThreads), 0, stream, a));
+  LACT_CUDA(launch_pdl(kernel, dim3(static_cast<unsigned>(std::min<int64_t>(units, sm_count()))), dim3(kCutThreads), smem, stream, a));
   return LACT_OK;
 }
+// (128-wide tiles move half as many bytes per product, 64-wide ones waste less of other sizes)
+int launch_cut_store(CutArgs& a, int bt, cudaStream_t stream) {
+  return bt == 128 ? launch_cut_gemm<kCutStore, 128>(a, stream) : launch_cut_gemm<kCutStore, 64>(a, stream);
+}
 
-// Splits of a token contraction (output R x C per entry, `len` tokens): enough that the grid fills the four CTAs an SM
-// holds, at least 64 tokens each, and no more than the grid's third axis takes (B x splits).  At 4 entries of 192 x 192 and
-// 4096 tokens one split would be 24 CTAs.
-int f32_splits(int64_t R, int64_t C, int64_t B, int64_t len) {
-  const int64_t tiles = B * ceil_div(R, kFM) * ceil_div(C, kFN);
-  const int64_t want = (4 * static_cast<int64_t>(sm_count()) + tiles - 1) / tiles;
-  return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>({want, (len + 63) / 64, 64, 65535 / B})));
+// Pieces of an fp32 matrix: [3][batch][rows][ld].
+struct Pieces {
+  bf16* p;
+  int64_t rows, cols, ld;
+};
+inline int64_t piece_ld(int64_t cols) { return (cols + 7) & ~7ll; }
+inline Mat piece_mat(const Pieces& x, int64_t batch) { return Mat{x.p, x.rows, x.cols, x.ld, 3 * batch, x.rows * x.ld}; }
+
+struct CutPlanes {
+  CutPlanesArgs a;
+  explicit CutPlanes(int64_t batch) {
+    std::memset(&a, 0, sizeof(a));
+    a.batch = static_cast<int32_t>(batch);
+  }
+  void add(const float* src, int64_t ld, int64_t bs, const Pieces& x) {
+    const bool vec = (reinterpret_cast<uintptr_t>(src) & 15) == 0 && ld % 4 == 0 && bs % 4 == 0;
+    a.s[a.n] = CutSource{src, ld, bs, x.p, static_cast<int32_t>(x.rows), static_cast<int32_t>(x.cols), static_cast<int32_t>(x.ld), vec};
+    a.first[a.n + 1] = a.first[a.n] + a.batch * x.rows * (x.ld / 8);
+    ++a.n;
+  }
+  int launch(cudaStream_t stream) {
+    const int64_t blocks = (a.first[a.n] + 255) / 256;
+    if (blocks < 1 || blocks > 0x7FFFFFFF) return LACT_ERR_SHAPE;
+    KernelScope scope(kClsOther, stream);
+    LACT_CUDA(launch_pdl(cut_planes_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, stream, a));
+    return LACT_OK;
+  }
+};
+
+// Splits of the two token contractions of an update ([2H x D] and [D x H] per entry, `len` tokens): two units per SM, at least 64
+// tokens each, and no more than 65535 partial results.  At 4 entries of 192 x 192 and 4096 tokens one split would be 60 units of
+// 64 slabs on 148 SMs.
+inline int cut_bt(int64_t D, int64_t H) { return D % 128 == 0 && H % 128 == 0 ? 128 : 64; }
+int f32_splits(int64_t B, int64_t D, int64_t H, int64_t len) {
+  const int bt = cut_bt(D, H);
+  const int64_t tiles = output_tiles(2 * H, D, B, bt) + output_tiles(D, H, B, bt);
+  return static_cast<int>(
+      std::max<int64_t>(1, std::min<int64_t>({2 * static_cast<int64_t>(sm_count()) / tiles, (len + kBK - 1) / kBK, 64, 65535 / B})));
 }
 
 struct ScanF32Plan {
   int32_t* status;
-  float *W02, *W1, *W02c, *W1c, *n02, *n1, *G02, *G1, *beta, *hidden, *dy02, *part02, *part1;
+  float *W02, *W1, *W02c, *W1c, *n02, *n1, *G02, *G1, *beta, *part02, *part1;
+  bf16 *w02, *w1, *x, *v, *hidden, *dy02;  // pieces of the weights, of q or k, of v, of the hidden activations, of dy0 | dy2
   bool updates;  // some update has tokens
   NsPlan ns;
   size_t bytes;
@@ -1664,12 +1723,18 @@ int plan_scan_f32(const lact_scan_config& c, int32_t n_steps, const int32_t* kin
   p->G02 = cv.take<float>(B * 2 * H * D);
   p->G1 = cv.take<float>(B * D * H);
   p->beta = cv.take<float>(B * static_cast<size_t>(std::max(1, n_steps)));
-  p->hidden = cv.take<float>(B * static_cast<size_t>(std::max(max_apply, max_update)) * H);
-  p->dy02 = cv.take<float>(B * static_cast<size_t>(max_update) * 2 * H);
+  const size_t any = static_cast<size_t>(std::max(max_apply, max_update)), upd = static_cast<size_t>(max_update), Dp = piece_ld(c.D);
+  p->w02 = cv.take<bf16>(3 * B * 2 * H * Dp);
+  p->w1 = cv.take<bf16>(3 * B * D * H);
+  p->x = cv.take<bf16>(3 * B * any * Dp);
+  p->v = cv.take<bf16>(3 * B * upd * Dp);
+  p->hidden = cv.take<bf16>(3 * B * any * H);
+  p->dy02 = cv.take<bf16>(3 * B * upd * 2 * H);
   p->updates = max_update > 0;
   // (splits grow with the token count: the longest update needs the most)
-  p->part02 = cv.take<float>(max_update > 0 ? static_cast<size_t>(f32_splits(2 * c.H, c.D, c.B, max_update)) * B * 2 * H * D : 0);
-  p->part1 = cv.take<float>(max_update > 0 ? static_cast<size_t>(f32_splits(c.D, c.H, c.B, max_update)) * B * D * H : 0);
+  const size_t splits = max_update > 0 ? static_cast<size_t>(f32_splits(c.B, c.D, c.H, max_update)) : 0;
+  p->part02 = cv.take<float>(splits * B * 2 * H * D);
+  p->part1 = cv.take<float>(splits * B * D * H);
   p->ns.ngroups = 0;
   if (c.use_muon && max_update > 0) plan_ns(cv, c.B, c.D, c.H, c.ns_concat, c.ns_gram_right, &p->ns);
   p->bytes = cv.off + 256;
@@ -1715,6 +1780,7 @@ int scan_fwd_f32(const lact_scan_config& c, const lact_scan_io& io, int32_t n_st
   const float* W1 = c.prenorm ? p.W1c : p.W1;
   const float *q = static_cast<const float*>(io.q), *k = static_cast<const float*>(io.k), *v = static_cast<const float*>(io.v);
   int update_idx = 0;
+  bool weights_cut = false;                       // the pieces are those of W02 and W1 as they are
   bool state_written = has_initial_momentum(io);  // by the caller, or by an update that had tokens
   for (int i = 0; i < n_steps; ++i) {
     const int64_t len = end[i] - start[i];
@@ -1722,38 +1788,54 @@ int scan_fwd_f32(const lact_scan_config& c, const lact_scan_io& io, int32_t n_st
       update_idx += kind[i] == LACT_STEP_UPDATE;
       continue;
     }
-    F32Args a;
+    const int64_t Dp = piece_ld(D);
+    const Pieces w02{p.w02, 2 * H, D, Dp}, w1{p.w1, D, H, H}, x{p.x, len, D, Dp}, hidden{p.hidden, len, H, H};
+    CutPlanes cut(B);
+    if (!weights_cut) {
+      cut.add(W02, D, 2 * H * D, w02);
+      cut.add(W1, H, D * H, w1);
+      weights_cut = true;
+    }
+    CutArgs a;
     std::memset(&a, 0, sizeof(a));
-    a.batch = static_cast<int32_t>(B);
-    a.splits = 1;
-    a.M = static_cast<int32_t>(len); a.N = static_cast<int32_t>(H); a.K = a.kper = static_cast<int32_t>(D);
-    a.c = p.hidden; a.c_ld = H; a.c_bs = len * H;
-    a.b = f32_mat(W02, D, 2 * H * D, 0, 2 * H, D);
+    a.status = p.status;
+    a.nprob = 1;
+    a.hidden = p.hidden;
+    {
+      CutProblem& P = a.prob[0];
+      LACT_TRY(encode_map(&P.a, piece_mat(x, B), kBM));
+      LACT_TRY(encode_map(&P.b, piece_mat(w02, B), 64));
+      P.M = static_cast<int32_t>(len); P.N = static_cast<int32_t>(H); P.K = P.kper = static_cast<int32_t>(D);
+      P.batch = static_cast<int32_t>(B);
+      P.splits = 1;
+    }
     if (kind[i] == LACT_STEP_APPLY) {
-      a.a = f32_mat(q + start[i] * c.q_ts, c.q_ts, c.q_bs, 0, len, D);
-      LACT_TRY(launch_f32_gemm<kF32Gate>(a, stream));
-      F32Args d;
-      std::memset(&d, 0, sizeof(d));
-      d.batch = a.batch; d.splits = 1;
-      d.M = a.M; d.N = static_cast<int32_t>(D); d.K = d.kper = static_cast<int32_t>(H);
-      d.a = f32_mat(p.hidden, H, len * H, 0, len, H);
-      d.b = f32_mat(W1, H, D * H, 0, D, H);
-      d.c = static_cast<float*>(io.o) + out_start[i] * c.o_ts; d.c_ld = c.o_ts; d.c_bs = c.o_bs;
-      LACT_TRY(launch_f32_gemm<kF32Store>(d, stream));
+      cut.add(q + start[i] * c.q_ts, c.q_ts, c.q_bs, x);
+      LACT_TRY(cut.launch(stream));
+      LACT_TRY((launch_cut_gemm<kCutGate, 128>(a, stream)));
+      CutProblem& P = a.prob[0];
+      LACT_TRY(encode_map(&P.a, piece_mat(hidden, B), kBM));
+      LACT_TRY(encode_map(&P.b, piece_mat(w1, B), 64));
+      P.N = static_cast<int32_t>(D); P.K = P.kper = static_cast<int32_t>(H);
+      P.c = static_cast<float*>(io.o) + out_start[i] * c.o_ts; P.c_ld = c.o_ts; P.c_bs = c.o_bs;
+      LACT_TRY(launch_cut_store(a, D % 128 == 0 ? 128 : 64, stream));
       continue;
     }
+    const Pieces v_pieces{p.v, len, D, Dp}, dy{p.dy02, len, 2 * H, 2 * H};
+    cut.add(k + start[i] * c.k_ts, c.k_ts, c.k_bs, x);
+    cut.add(v + start[i] * c.v_ts, c.v_ts, c.v_bs, v_pieces);
+    LACT_TRY(cut.launch(stream));
+    LACT_TRY(encode_map(&a.a2, piece_mat(v_pieces, B), kBM));
+    LACT_TRY(encode_map(&a.b2, piece_mat(w1, B), 64));  // dh = v w1: w1 is [D][H], k = D rows
+    a.dy = p.dy02;
     const int u = update_idx++;
-    a.a = f32_mat(k + start[i] * c.k_ts, c.k_ts, c.k_bs, 0, len, D);
-    a.a2 = f32_mat(v + start[i] * c.v_ts, c.v_ts, c.v_bs, 0, len, D);
-    a.b2 = f32_mat(W1, H, D * H, 1, H, D);  // dh = v w1: w1 is [D][H], k = D rows
-    a.c2 = p.dy02; a.c2_ld = 2 * H; a.c2_bs = len * 2 * H;
     const int64_t esz = c.lr_dtype == LACT_F32 ? 4 : 2;
     auto at = [&](const void* t) { return static_cast<const uint8_t*>(t) + start[i] * esz; };
     a.lr0 = at(io.lr0); a.lr1 = at(io.lr1); a.lr2 = at(io.lr2);
     a.lr_f32 = c.lr_dtype == LACT_F32;
     a.lr_bs = c.L;
     a.w_scale = c.w_scale;
-    LACT_TRY(launch_f32_gemm<kF32Grad>(a, stream));
+    LACT_TRY((launch_cut_gemm<kCutGrad, 128>(a, stream)));
     F32ReduceArgs red;
     std::memset(&red, 0, sizeof(red));
     red.batch = static_cast<int32_t>(B);
@@ -1761,30 +1843,26 @@ int scan_fwd_f32(const lact_scan_config& c, const lact_scan_io& io, int32_t n_st
     red.fresh = !state_written;
     red.beta = c.use_momentum ? p.beta + static_cast<int64_t>(u) * B : nullptr;
     state_written = true;
-    for (int w = 0; w < 2; ++w) {  // [dw0; dw2] = dy^T k, dw1 = v^T hidden
-      const int64_t R = w == 0 ? 2 * H : D, C = w == 0 ? D : H;
-      F32Args g;
-      std::memset(&g, 0, sizeof(g));
-      g.batch = a.batch;
-      g.M = static_cast<int32_t>(R); g.N = static_cast<int32_t>(C); g.K = static_cast<int32_t>(len);
-      const int splits = f32_splits(R, C, B, len);
-      g.kper = ceil_div(ceil_div(len, splits), kFK) * kFK;
-      g.splits = ceil_div(len, g.kper);
-      if (w == 0) {
-        g.a = f32_mat(p.dy02, 2 * H, len * 2 * H, 1, R, len);
-        g.b = f32_mat(k + start[i] * c.k_ts, c.k_ts, c.k_bs, 1, C, len);
-      } else {
-        g.a = f32_mat(v + start[i] * c.v_ts, c.v_ts, c.v_bs, 1, R, len);
-        g.b = f32_mat(p.hidden, H, len * H, 1, C, len);
-      }
-      g.c = w == 0 ? p.part02 : p.part1;
-      g.c_ld = C; g.c_bs = R * C;
-      LACT_TRY(launch_f32_gemm<kF32Store>(g, stream));
-      red.part[w] = g.c;
+    // [dw0; dw2] = dy^T k, dw1 = v^T hidden
+    const int splits = f32_splits(B, D, H, len);
+    for (int w = 0; w < 2; ++w) {
+      CutProblem& P = a.prob[w];
+      LACT_TRY(encode_map(&P.a, piece_mat(w == 0 ? dy : v_pieces, B), 64));
+      LACT_TRY(encode_map(&P.b, piece_mat(w == 0 ? x : hidden, B), 64));
+      P.a_mn = P.b_mn = 1;
+      P.M = static_cast<int32_t>(w == 0 ? 2 * H : D); P.N = static_cast<int32_t>(w == 0 ? D : H); P.K = static_cast<int32_t>(len);
+      P.batch = static_cast<int32_t>(B);
+      P.kper = ceil_div(ceil_div(len, splits), kBK) * kBK;
+      P.splits = ceil_div(len, P.kper);
+      P.c = w == 0 ? p.part02 : p.part1;
+      P.c_ld = P.N; P.c_bs = static_cast<int64_t>(P.M) * P.N;
+      red.part[w] = P.c;
       red.c[w] = w == 0 ? p.G02 : p.G1;
-      red.n[w] = R * C;
-      red.splits[w] = g.splits;
+      red.n[w] = P.c_bs;
+      red.splits[w] = P.splits;
     }
+    a.nprob = 2;
+    LACT_TRY(launch_cut_store(a, cut_bt(D, H), stream));
     {
       KernelScope scope(kClsOther, stream);
       LACT_CUDA(launch_pdl(f32_reduce_kernel, dim3(ceil_div((red.n[0] + red.n[1]) * B / 4, 256)), dim3(256), 0, stream, red));
@@ -1809,6 +1887,7 @@ int scan_fwd_f32(const lact_scan_config& c, const lact_scan_io& io, int32_t n_st
       r.mode = c.renorm; r.prenorm = c.prenorm; r.prenorm_bf16 = c.prenorm_bf16; r.quirk = c.overwrite_quirk;
     }
     LACT_TRY(launch_add_renorm(rn[0], rn[1], stream));
+    weights_cut = false;
   }
   return store_state(c, io, W02, W1, p.G02, p.G1, stream);
 }
@@ -3170,13 +3249,18 @@ int lact_sgemm_f32(const void* a, int32_t a_t, const void* b, int32_t b_t, void*
   std::memset(&g, 0, sizeof(g));
   g.a = f32_mat(static_cast<const float*>(a), a_t ? M : K, M * K, a_t ? 1 : 0, M, K);
   g.b = f32_mat(static_cast<const float*>(b), b_t ? N : K, N * K, b_t ? 1 : 0, N, K);
-  g.M = static_cast<int32_t>(M); g.N = static_cast<int32_t>(N); g.K = g.kper = static_cast<int32_t>(K);
+  g.M = static_cast<int32_t>(M); g.N = static_cast<int32_t>(N); g.K = static_cast<int32_t>(K);
   g.batch = static_cast<int32_t>(batch);
-  g.splits = 1;
   g.c = static_cast<float*>(c); g.c_ld = N; g.c_bs = M * N;
   g.accumulate = accumulate;
   g.beta = static_cast<const float*>(beta);
-  return launch_f32_gemm<kF32Store>(g, static_cast<cudaStream_t>(stream));
+  const dim3 grid(ceil_div(N, kFN), ceil_div(M, kFM), static_cast<unsigned>(batch));
+  if (grid.y > 65535) return LACT_ERR_SHAPE;
+  g.c_vec = (reinterpret_cast<uintptr_t>(g.c) & 15) == 0 && (g.c_ld % 4) == 0 && (g.c_bs % 4) == 0;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  KernelScope scope(kClsOther, s);
+  LACT_CUDA(launch_pdl(f32_gemm_kernel, grid, dim3(kFThreads), 0, s, g));
+  return LACT_OK;
 }
 
 int lact_swiglu_planes_f32(const void* y02, const void* dh, const void* lr0, const void* lr1, const void* lr2,

@@ -1159,7 +1159,7 @@ __global__ void __launch_bounds__(256) weight_grad_kernel(const WeightGradArgs a
 }
 
 // ------------------------------------------------------------------------------------------
-// fp32 mode: pointwise stages as kernels of their own (the recurrence itself fuses them, f32_gemm.cuh)
+// fp32 mode: pointwise stages as kernels of their own (the recurrence itself fuses them, f32_split.cuh)
 // ------------------------------------------------------------------------------------------
 // fp32 planes: hidden = silu(y0) * y2 (lr pointers null and dh null), or the lr-weighted gradient
 // planes (hidden*lr1, dy0*lr0, dy2*lr2).  Exact expf / division.  One warp per token row.
