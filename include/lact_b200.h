@@ -171,8 +171,10 @@ int lact_swiglu_ffn_workspace_bytes(int64_t B, int64_t N, int64_t D, int64_t H, 
 int lact_swiglu_ffn_fwd(const void *w0w2, const void *w1, const void *x, void *out, int64_t B, int64_t N,
                         int64_t D, int64_t H, void *workspace, size_t workspace_bytes, void *stream);
 
-/* lact_swiglu_ffn_fwd with its scratch and its status word given one by one: hidden = bf16 [B, N, H]; status_word = device
+/* lact_swiglu_ffn_fwd with its scratch and its status word given one by one: hidden = bf16 [B, N, H], of which
+ * lact_swiglu_ffn_hidden_bytes are used (0: a few tokens per entry need none and hidden may be NULL); status_word = device
  * word the caller has cleared (it is not cleared here, so that consecutive calls can share one). */
+int lact_swiglu_ffn_hidden_bytes(int64_t B, int64_t N, int64_t D, int64_t H, size_t *bytes_out);
 int lact_swiglu_ffn_apply(const void *w0w2, const void *w1, const void *x, void *out, void *hidden, int64_t B, int64_t N,
                           int64_t D, int64_t H, int32_t *status_word, void *stream);
 

@@ -17,6 +17,7 @@
 #include "f32_split.cuh"
 #include "ns_bwd_fused.cuh"
 #include "ns_chip.cuh"
+#include "few_tokens.cuh"
 #include "pair_gemm.cuh"
 #include "row_passes.cuh"
 #include "swa_bwd.cuh"
@@ -473,6 +474,60 @@ int launch_gate(const ApplyArgs& a, const Mat& x, const Mat& w02, int64_t len, i
   return launch_gemm(g, stream, kClsGate);
 }
 
+// Whether apply on `tokens` tokens of `B` entries goes to one cluster per entry (few_tokens.cuh): where the
+// clusters of all entries run at once.  us per call, two launches / one cluster per entry: up to there 12.3 / 8.6 at 256, 192 and 128 x
+// 256 (64 entries of 256, 16 tokens, two CTAs per SM: 12.6 / 10.9), 12.4 / 8.8 at 384, 14.3 / 8.6 at 512; past it 12.7 / 14.2 (32
+// of 384, 32 tokens), 12.3 / 16.6 (64 of 192, 64 tokens), 14.7 / 18.1 (32 of 512, 16 tokens).
+bool few_pays(int64_t B, int64_t tokens, int64_t D, int64_t H) {
+  if (!few_fits(D, H, tokens)) return false;
+  const int64_t nt = (tokens + 15) / 16 * 16;
+  const int64_t per_sm = 233472 / (few_smem_bytes(static_cast<int>(D), static_cast<int>(H), static_cast<int>(nt)) + 1024);
+  return B * (H / 64) <= per_sm * sm_count();
+}
+int launch_few(const ApplyArgs& a, const Mat& x, const Mat& w02, const Mat& w1, int32_t* status, cudaStream_t stream) {
+  static std::mutex mu;
+  static bool configured[64] = {false};
+  int dev = 0;
+  LACT_CUDA(cudaGetDevice(&dev));
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    if (dev >= 64 || !configured[dev]) {
+      LACT_CUDA(cudaFuncSetAttribute(few_tokens_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448));
+      if (dev < 64) configured[dev] = true;
+    }
+  }
+  FewArgs f;
+  std::memset(&f, 0, sizeof(f));
+  f.D = static_cast<int32_t>(a.D); f.H = static_cast<int32_t>(a.H);
+  f.tokens = static_cast<int32_t>(a.end - a.start);
+  f.nt = (f.tokens + 15) / 16 * 16;
+  const int ranks = f.H / 64;
+  f.rows1 = ceil_div(f.D, ranks);
+  f.out = static_cast<bf16*>(a.out) + a.out_start * a.o_ts;
+  f.o_bs = a.o_bs; f.o_ts = a.o_ts;
+  f.status = status;
+  LACT_TRY(encode_map(&f.w02, w02, 64));
+  LACT_TRY(encode_map(&f.w1, w1, 64));
+  LACT_TRY(encode_map(&f.x, x, static_cast<uint32_t>(f.nt)));
+  cudaLaunchConfig_t cfg;
+  std::memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3(static_cast<unsigned>(a.B * ranks));
+  cfg.blockDim = dim3(kFewThreads);
+  cfg.dynamicSmemBytes = few_smem_bytes(f.D, f.H, f.nt);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = static_cast<unsigned>(ranks);
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  KernelScope scope(kClsGate, stream);
+  LACT_CUDA(cudaLaunchKernelEx(&cfg, few_tokens_kernel, f));
+  return LACT_OK;
+}
+
 int run_apply(const ApplyArgs& a, int32_t* status, cudaStream_t stream) {
   const int64_t len = a.end - a.start;
   if (len <= 0) return LACT_OK;
@@ -484,6 +539,7 @@ int run_apply(const ApplyArgs& a, int32_t* status, cudaStream_t stream) {
   const Mat om{static_cast<bf16*>(a.out) + a.out_start * a.o_ts, len, a.D, a.o_ts, a.B, a.o_bs, a.segs, a.o_step * a.o_ts};
   const Mat hid{a.hidden, len, a.H, a.H, a.B, len * a.H, a.segs, a.B * len * a.H};
   const int64_t batch = a.segs * a.B;
+  if (a.segs == 1 && few_pays(a.B, len, a.D, a.H)) return launch_few(a, x, w02, w1, status, stream);
   if (a.H % 128 == 0) LACT_TRY(launch_gate<128>(a, x, w02, len, status, stream));
   else LACT_TRY(launch_gate<64>(a, x, w02, len, status, stream));
   const int bt = choose_bt({{a.D, 1}});
@@ -2111,11 +2167,19 @@ int lact_swiglu_ffn_fwd(const void* w0w2, const void* w1, const void* x, void* o
   return run_apply(a, static_cast<int32_t*>(workspace), s);
 }
 
+int lact_swiglu_ffn_hidden_bytes(int64_t B, int64_t N, int64_t D, int64_t H, size_t* bytes_out) {
+  if (!bytes_out) return LACT_ERR_NULL;
+  LACT_TRY(check_dims(B, N, D, H));
+  *bytes_out = few_pays(B, N, D, H) ? 0 : static_cast<size_t>(B) * N * H * 2;
+  return LACT_OK;
+}
+
 int lact_swiglu_ffn_apply(const void* w0w2, const void* w1, const void* x, void* out, void* hidden, int64_t B, int64_t N,
                           int64_t D, int64_t H, int32_t* status_word, void* stream) {
-  if (!w0w2 || !w1 || !x || !out || !hidden || !status_word) return LACT_ERR_NULL;
+  if (!w0w2 || !w1 || !x || !out || !status_word) return LACT_ERR_NULL;
   LACT_TRY(check_device());
   LACT_TRY(check_dims(B, N, D, H));
+  if (!hidden && !few_pays(B, N, D, H)) return LACT_ERR_NULL;
   const ApplyArgs a{static_cast<const bf16*>(w0w2), static_cast<const bf16*>(w1), x, N * D, D, 0, N, out, N * D, D, 0,
                     static_cast<bf16*>(hidden), B, D, H};
   return run_apply(a, status_word, static_cast<cudaStream_t>(stream));

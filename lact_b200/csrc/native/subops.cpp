@@ -27,8 +27,12 @@ Tensor ffn(const Tensor& w02_, const Tensor& w1_, const Tensor& x_) {
   const c10::cuda::CUDAGuard guard(x_.device());
   const Tensor w02 = w02_.contiguous(), w1 = w1_.contiguous(), x = x_.contiguous();
   const int64_t B = x.size(0), N = x.size(1), D = x.size(2), H = w02.size(1) / 2;
-  Tensor out = empty({B, N, D}, at::kBFloat16, x), hidden = empty({B, N, H}, at::kBFloat16, x);
-  check(lact_swiglu_ffn_apply(ptr(w02), ptr(w1), ptr(x), ptr(out), ptr(hidden), B, N, D, H, status_word(x), stream_of(x)),
+  size_t need = 0;
+  if (lact_swiglu_ffn_hidden_bytes(B, N, D, H, &need) != LACT_OK) need = 0;  // the call below reports it
+  Tensor out = empty({B, N, D}, at::kBFloat16, x), hidden;
+  if (need > 0) hidden = bytes(need, x);
+  check(lact_swiglu_ffn_apply(ptr(w02), ptr(w1), ptr(x), ptr(out), need > 0 ? ptr(hidden) : nullptr, B, N, D, H, status_word(x),
+                              stream_of(x)),
         "lact_swiglu_ffn_fwd");
   return out;
 }
