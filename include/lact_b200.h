@@ -311,6 +311,16 @@ int lact_swa_fwd_split(const void *q, const void *k, const void *v, void *o, int
                  int64_t o_bs, int64_t window, float softmax_scale, const int32_t *seq_start, void *lse,
                  void *counters, void *scratch, size_t scratch_bytes, int32_t *status_word, void *stream);
 
+/* Block attention over a cache and new tokens (every query sees all l_cache + l_new keys) without putting them into one array:
+ * k_cache, v_cache [b, l_cache, n_heads, d], k, v [b, l_new, n_heads, d], q, o [b, l, n_heads, d], bf16.  strides: token and
+ * batch stride of q, k_cache, v_cache, k, v, o in this order (12 values, elements).  counters and scratch as for
+ * lact_swa_fwd_split.  ar_lact_swa_repeat.py:464-531. */
+int lact_swa_fwd_cache_bytes(int64_t b, int64_t l, int64_t l_cache, int64_t l_new, int64_t n_heads, int64_t d, size_t *bytes,
+                             int64_t *counters);
+int lact_swa_fwd_cache(const void *q, const void *k_cache, const void *v_cache, const void *k, const void *v, void *o, int64_t b,
+                       int64_t l, int64_t l_cache, int64_t l_new, int64_t n_heads, int64_t d, const int64_t *strides,
+                       float softmax_scale, void *counters, void *scratch, size_t scratch_bytes, int32_t *status_word, void *stream);
+
 /* Backward of lact_swa_fwd: dq (bf16, contiguous [b, l, n_heads, d]) and dk, dv ([b, lk, n_heads, d]), written, from the forward's inputs, its
  * output o, its lse and the output gradient dout (bf16, token / batch strides in elements).  delta: fp32 scratch
  * [b, n_heads, l].  Three launches: row sums of dout * o, the keys' side (dK, dV), the queries' side (dQ); the

@@ -88,6 +88,11 @@ def _(q, k, v, window, softmax_scale, seq_start=None):
     return [q.new_empty(q.shape), q.new_empty((b, h, l), dtype=F32)]
 
 
+@_fake("swa_fwd_cache")
+def _(q, k_cache, v_cache, k, v, softmax_scale):
+    return q.new_empty(q.shape)
+
+
 @_fake("swa_bwd")
 def _(q, k, v, o, lse, dout, window, softmax_scale, seq_start=None):
     return [q.new_empty(q.shape), q.new_empty(k.shape), q.new_empty(k.shape)]

@@ -172,6 +172,8 @@ def load_ops() -> None:
         raise ImportError(f"{OPS_PATH} was built for another PyTorch than {torch.__version__}: rebuild it with "
                           "`python -m lact_b200.build`")
     torch.ops.load_library(OPS_PATH)
+    if not hasattr(torch.ops.lact_b200, "swa_fwd_cache"):   # the operator that was added last
+        raise ImportError(f"{OPS_PATH} is older than this package: rebuild it with `python -m lact_b200.build`")
     _ops_lib = C.CDLL(OPS_PATH)
     _ops_lib.lact_torch_take_status.argtypes = [C.c_int]
     _ops_lib.lact_torch_take_status.restype = C.c_int

@@ -2768,10 +2768,18 @@ int lact_swa_fwd(const void* q, const void* k, const void* v, void* o, int64_t b
                             seq_start, lse, nullptr, nullptr, 0, status_word, stream);
 }
 
-int lact_swa_fwd_split(const void* q, const void* k, const void* v, void* o, int64_t b, int64_t l, int64_t lk, int64_t n_heads,
-                       int64_t d, int64_t q_ts, int64_t q_bs, int64_t k_ts, int64_t k_bs, int64_t v_ts, int64_t v_bs, int64_t o_ts,
-                       int64_t o_bs, int64_t window, float softmax_scale, const int32_t* seq_start, void* lse, void* counters,
-                       void* scratch, size_t scratch_bytes, int32_t* status_word, void* stream) {
+// Keys of two runs as the kernel counts them: the second begins at the next whole tile.
+static int64_t swa_two_runs(int64_t lk1, int64_t lk2) { return static_cast<int64_t>(ceil_div(lk1, 128)) * 128 + lk2; }
+
+// A second run of keys and values (block attention), or k = nullptr.
+struct SwaSecond {
+  const void *k, *v;
+  int64_t lk, k_ts, k_bs, v_ts, v_bs;
+};
+static int swa_fwd_impl(const void* q, const void* k, const void* v, const SwaSecond& two, void* o, int64_t b, int64_t l, int64_t lk,
+                        int64_t n_heads, int64_t d, int64_t q_ts, int64_t q_bs, int64_t k_ts, int64_t k_bs, int64_t v_ts,
+                        int64_t v_bs, int64_t o_ts, int64_t o_bs, int64_t window, float softmax_scale, const int32_t* seq_start,
+                        void* lse, void* counters, void* scratch, size_t scratch_bytes, int32_t* status_word, void* stream) {
   if (!q || !k || !v || !o || !status_word) return LACT_ERR_NULL;
   if (seq_start != nullptr && b != 1) return LACT_ERR_CONFIG;   // packed sequences live in one batch entry
   const bool causal = window >= 0;
@@ -2788,6 +2796,12 @@ int lact_swa_fwd_split(const void* q, const void* k, const void* v, void* o, int
   LACT_TRY(encode_map_heads(&a.q, q, b, l, n_heads, d, q_ts, q_bs));
   LACT_TRY(encode_map_heads(&a.k, k, b, lk, n_heads, d, k_ts, k_bs));
   LACT_TRY(encode_map_heads(&a.v, v, b, lk, n_heads, d, v_ts, v_bs));
+  if (two.k != nullptr) {
+    LACT_TRY(encode_map_heads(&a.k2, two.k, b, two.lk, n_heads, d, two.k_ts, two.k_bs));
+    LACT_TRY(encode_map_heads(&a.v2, two.v, b, two.lk, n_heads, d, two.v_ts, two.v_bs));
+    a.Lk1 = static_cast<int32_t>(lk);
+    lk = swa_two_runs(lk, two.lk);
+  }
   a.Lk = static_cast<int32_t>(lk);
   a.causal = causal ? 1 : 0;
   a.o = static_cast<bf16*>(o);
@@ -2821,6 +2835,31 @@ int lact_swa_fwd_split(const void* q, const void* k, const void* v, void* o, int
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   return d == 64 ? launch_swa<64>(a, ctas, st) : launch_swa<128>(a, ctas, st);
+}
+
+int lact_swa_fwd_split(const void* q, const void* k, const void* v, void* o, int64_t b, int64_t l, int64_t lk, int64_t n_heads,
+                       int64_t d, int64_t q_ts, int64_t q_bs, int64_t k_ts, int64_t k_bs, int64_t v_ts, int64_t v_bs, int64_t o_ts,
+                       int64_t o_bs, int64_t window, float softmax_scale, const int32_t* seq_start, void* lse, void* counters,
+                       void* scratch, size_t scratch_bytes, int32_t* status_word, void* stream) {
+  return swa_fwd_impl(q, k, v, SwaSecond{}, o, b, l, lk, n_heads, d, q_ts, q_bs, k_ts, k_bs, v_ts, v_bs, o_ts, o_bs, window,
+                      softmax_scale, seq_start, lse, counters, scratch, scratch_bytes, status_word, stream);
+}
+
+int lact_swa_fwd_cache_bytes(int64_t b, int64_t l, int64_t l_cache, int64_t l_new, int64_t n_heads, int64_t d, size_t* bytes,
+                             int64_t* counters) {
+  if (l_cache < 1 || l_new < 1 || l_cache > (1ll << 29) || l_new > (1ll << 29)) return LACT_ERR_SHAPE;
+  return lact_swa_fwd_split_bytes(b, l, swa_two_runs(l_cache, l_new), n_heads, d, -1, bytes, counters);
+}
+
+int lact_swa_fwd_cache(const void* q, const void* k_cache, const void* v_cache, const void* k, const void* v, void* o, int64_t b,
+                       int64_t l, int64_t l_cache, int64_t l_new, int64_t n_heads, int64_t d, const int64_t* strides,
+                       float softmax_scale, void* counters, void* scratch, size_t scratch_bytes, int32_t* status_word, void* stream) {
+  if (!k || !v || !strides) return LACT_ERR_NULL;
+  if (l_cache < 1 || l_new < 1 || l_cache > (1ll << 29) || l_new > (1ll << 29)) return LACT_ERR_SHAPE;
+  const int64_t* s = strides;
+  return swa_fwd_impl(q, k_cache, v_cache, SwaSecond{k, v, l_new, s[6], s[7], s[8], s[9]}, o, b, l, l_cache, n_heads, d, s[0], s[1], s[2],
+                      s[3], s[4], s[5], s[10], s[11], -1, softmax_scale, nullptr, nullptr, counters, scratch, scratch_bytes, status_word,
+                      stream);
 }
 
 int lact_swa_bwd(const void* q, const void* k, const void* v, const void* o, const void* dout, const void* lse, void* dq,

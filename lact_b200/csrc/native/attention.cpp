@@ -50,6 +50,28 @@ std::vector<Tensor> swa(const Tensor& q_, const Tensor& k_, const Tensor& v_, in
   return {o, lse};
 }
 
+// Block attention of q over the keys and values of a cache followed by k, v, where they lie.
+Tensor swa_cache(const Tensor& q_, const Tensor& kc_, const Tensor& vc_, const Tensor& k_, const Tensor& v_, double scale) {
+  const c10::cuda::CUDAGuard guard(q_.device());
+  const Tensor q = head_view(q_), kc = head_view(kc_), vc = head_view(vc_), k = head_view(k_), v = head_view(v_);
+  const int64_t b = q.size(0), l = q.size(1), h = q.size(2), d = q.size(3), lc = kc.size(1), ln = k.size(1);
+  Tensor o = empty({b, l, h, d}, at::kBFloat16, q);
+  size_t need = 0;
+  int64_t words = 0;
+  if (lact_swa_fwd_cache_bytes(b, l, lc, ln, h, d, &need, &words) != LACT_OK) need = 0;  // the call below reports it
+  Tensor scratch, counters;
+  if (need > 0) {
+    scratch = bytes(need, q);
+    counters = at::zeros({words}, q.options().dtype(at::kInt).requires_grad(false));
+  }
+  const int64_t strides[12] = {q.stride(1), q.stride(0), kc.stride(1), kc.stride(0), vc.stride(1), vc.stride(0),
+                               k.stride(1), k.stride(0), v.stride(1),  v.stride(0),  o.stride(1),  o.stride(0)};
+  check(lact_swa_fwd_cache(ptr(q), ptr(kc), ptr(vc), ptr(k), ptr(v), ptr(o), b, l, lc, ln, h, d, strides, static_cast<float>(scale),
+                           need > 0 ? ptr(counters) : nullptr, need > 0 ? ptr(scratch) : nullptr, need, status_word(q), stream_of(q)),
+        "lact_swa_fwd_cache");
+  return o;
+}
+
 // [dq, dk, dv] (bf16, contiguous): probabilities recomputed from lse
 std::vector<Tensor> swa_bwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& o_, const Tensor& lse_,
                             const Tensor& dout_, int64_t window, double scale, const OptTensor& seq) {
@@ -98,6 +120,17 @@ std::vector<Tensor> swa_autograd(const Tensor& q, const Tensor& k, const Tensor&
   return fwd_op().call(q, k, v, window, scale, seq);
 }
 
+using CacheSig = Tensor(const Tensor&, const Tensor&, const Tensor&, const Tensor&, const Tensor&, double);
+// (with gradients the keys and values are put together first: the backward reads them as one array)
+Tensor swa_cache_autograd(const Tensor& q, const Tensor& kc, const Tensor& vc, const Tensor& k, const Tensor& v, double scale) {
+  static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow("lact_b200::swa_fwd_cache", "").typed<CacheSig>();
+  bool grad = false;
+  for (const Tensor* t : {&q, &kc, &vc, &k, &v}) grad = grad || t->requires_grad();
+  if (at::GradMode::is_enabled() && grad) return fwd_op().call(q, at::cat({kc, k}, 1), at::cat({vc, v}, 1), -1, scale, {})[0];
+  at::AutoDispatchBelowADInplaceOrView guard;
+  return op.call(q, kc, vc, k, v, scale);
+}
+
 // int32 [n_tokens]: first token of the packed sequence every token belongs to
 Tensor seq_start(const Tensor& cu_, int64_t n_tokens) {
   const c10::cuda::CUDAGuard guard(cu_.device());
@@ -112,18 +145,21 @@ Tensor seq_start(const Tensor& cu_, int64_t n_tokens) {
 
 TORCH_LIBRARY_FRAGMENT(lact_b200, m) {
   m.def("swa_fwd(Tensor q, Tensor k, Tensor v, int window, float softmax_scale, Tensor? seq_start=None) -> Tensor[]");
+  m.def("swa_fwd_cache(Tensor q, Tensor k_cache, Tensor v_cache, Tensor k, Tensor v, float softmax_scale) -> Tensor");
   m.def("swa_bwd(Tensor q, Tensor k, Tensor v, Tensor o, Tensor lse, Tensor dout, int window, float softmax_scale, "
         "Tensor? seq_start=None) -> Tensor[]");
   m.def("seq_start(Tensor cu_seqlens, int n_tokens) -> Tensor");
 }
 TORCH_LIBRARY_IMPL(lact_b200, CUDA, m) {
   m.impl("swa_fwd", &swa);
+  m.impl("swa_fwd_cache", &swa_cache);
   m.impl("swa_bwd", &swa_bwd);
   m.impl("seq_start", &seq_start);
 }
 TORCH_LIBRARY_IMPL(lact_b200, Autograd, m) {
   m.impl("swa_bwd", torch::autograd::autogradNotImplementedFallback());
   m.impl("swa_fwd", &swa_autograd);
+  m.impl("swa_fwd_cache", &swa_cache_autograd);
 }
 
 }  // namespace lact_torch

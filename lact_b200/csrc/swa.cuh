@@ -22,10 +22,12 @@ namespace lact {
 
 struct SwaArgs {
   CUtensorMap q, k, v;   // 4-D maps (feature, token, head, batch), box {64, 128, 1, 1}
+  CUtensorMap k2, v2;    // keys and values behind the first `Lk1` (block attention over a cache and new tokens), if Lk1 > 0
   bf16* o;               // [b][l][h][d], strides below (elements); feature stride 1
   int64_t o_bs, o_ts, o_hs;
   int32_t L, window;     // queries per batch entry; window <= 0: unbounded (plain causal attention)
   int32_t Lk, causal;    // keys per batch entry (= L when causal); causal = 0: every query sees every key of its entry
+  int32_t Lk1;           // two runs of keys: the second begins at the next whole tile behind Lk1, and Lk counts from there on
   int32_t heads, q_tiles;
   float scale_log2;      // log2(e) / sqrt(d)
   const int32_t* seq_start;  // optional [l]: first token of the packed sequence every token belongs to (nondecreasing;
@@ -130,6 +132,7 @@ __global__ void __launch_bounds__(320, 1) swa_fwd_kernel(const __grid_constant__
     kv_lo += t0 * 128;
   }
   bool failed = uniform(static_cast<uint32_t>(*reinterpret_cast<volatile int32_t*>(a.status))) != kStatusOk;
+  const int second = a.Lk1 > 0 ? (a.Lk1 + 127) / 128 * 128 : 0x7FFFFFFF;  // where the second run of keys begins
 
   if (warp == 0) {
     const uint32_t leader = elect_leader();
@@ -138,14 +141,18 @@ __global__ void __launch_bounds__(320, 1) swa_fwd_kernel(const __grid_constant__
       for (int j = 0; j < KBD; ++j) tma_load_4d_if(leader, base + SM::kQ + j * kBox, &a.q, q_full, 64 * j, q0, head, batch);
       for (int t = 0; t < T && !failed; ++t) {
         const int sb = t & 1;
+        const bool behind = kv_lo + t * 128 >= second;
+        const int row = kv_lo + t * 128 - (behind ? second : 0);
+        const CUtensorMap* const km = behind ? &a.k2 : &a.k;
+        const CUtensorMap* const vm = behind ? &a.v2 : &a.v;
         if (t >= 2 && !mbar_wait_warp(&k_empty[sb], ((t - 2) >> 1) & 1, abort_flag)) { failed = true; break; }
         mbar_expect_tx_if(leader, &k_full[sb], SM::kTile);
         for (int j = 0; j < KBD; ++j)
-          tma_load_4d_if(leader, base + SM::kK + sb * SM::kTile + j * kBox, &a.k, &k_full[sb], 64 * j, kv_lo + t * 128, head, batch);
+          tma_load_4d_if(leader, base + SM::kK + sb * SM::kTile + j * kBox, km, &k_full[sb], 64 * j, row, head, batch);
         if (t >= 2 && !mbar_wait_warp(&pv_done[sb], ((t - 2) >> 1) & 1, abort_flag)) { failed = true; break; }
         mbar_expect_tx_if(leader, &v_full[sb], SM::kTile);
         for (int j = 0; j < KBD; ++j)
-          tma_load_4d_if(leader, base + SM::kV + sb * SM::kTile + j * kBox, &a.v, &v_full[sb], 64 * j, kv_lo + t * 128, head, batch);
+          tma_load_4d_if(leader, base + SM::kV + sb * SM::kTile + j * kBox, vm, &v_full[sb], 64 * j, row, head, batch);
       }
     }
   } else if (warp == 1) {
@@ -242,11 +249,12 @@ __global__ void __launch_bounds__(320, 1) swa_fwd_kernel(const __grid_constant__
         *abort_flag = 1;
       }
       // every (row, key) pair of the tile inside the band and the sequence: no masks
+      const int keys = kv0 < second && a.Lk1 > 0 ? a.Lk1 : a.Lk;  // (not causal) end of the run this tile belongs to
       const bool interior = a.causal ? (kv0 + 127 <= q0 && kv0 >= q0 + 127 - (window - 1) && kv0 + 127 < a.L && kv0 >= tile_start)
-                                     : kv0 + 127 < a.Lk;
+                                     : kv0 + 127 < keys;
       const int c0 = half * 64;                                // this thread's first key column of the tile
       // last / first column of the tile this row may see
-      const int j_hi = (a.causal ? (qi < a.L - 1 ? qi : a.L - 1) : a.Lk - 1) - kv0;
+      const int j_hi = (a.causal ? (qi < a.L - 1 ? qi : a.L - 1) : keys - 1) - kv0;
       const int j_lo = (a.causal ? (qi - (window - 1) > row_start ? qi - (window - 1) : row_start) : 0) - kv0;
       const uint32_t s_addr = tmem + lane_off + sb * 128 + c0;
       uint32_t ba[32], bb[32];   // this thread's 64 scores: read once, kept across the exchange of the row maximum

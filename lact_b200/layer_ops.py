@@ -228,4 +228,9 @@ def sliding_window_attention_inference(q: torch.Tensor, k: torch.Tensor, v: torc
         o_rest = block_attention(q[:, mb:], k[:, mb - kv_cache_size:], v[:, mb - kv_cache_size:])
         return torch.cat([o_clean, o_rest], dim=1)
     k_cache, v_cache = kv_cache.chunk(2, dim=0)
+    every = (q, k_cache, v_cache, k, v)
+    if (all(t.is_cuda and t.dtype == BF16 and t.dim() == 4 and t.device == q.device for t in every) and k.shape == v.shape
+            and k_cache.shape == v_cache.shape and all(t.shape[0] == q.shape[0] and t.shape[2:] == q.shape[2:] for t in every)
+            and q.shape[3] in (64, 128) and min(t.shape[1] for t in every) > 0):
+        return L.call(_op("swa_fwd_cache"), *every, q.shape[3] ** -0.5)   # (the keys are read where they lie)
     return block_attention(q, torch.cat([k_cache, k], dim=1), torch.cat([v_cache, v], dim=1))
