@@ -2,7 +2,9 @@
 // features, V 16-byte units per lane (unit u = lane + LPR * i), so no lane idles and a lane has all its loads in flight.
 // Grid (token blocks, heads [x tensors], batch entries): no index divisions, and a block's rows are consecutive tokens.
 // What bounds them is HBM and the instructions between the loads: 2 batches x 8192 tokens x 4 heads of 384 take 83 us in the
-// prologue forward (302 MB: 3.6 TB/s) and 125 backward, 40 and 52 in the epilogue.  (A warp per row leaves a quarter of the
+// prologue forward (302 MB: 3.6 TB/s) and 107 backward (125 with the sigmoid worked out again behind the row sums: two of the
+// special-function unit's operations per feature, which it takes half of that time for), 40 and 52 in the epilogue.  Persistent
+// blocks with the next row's loads in flight take 12 to 20 % longer (fewer warps).  (A warp per row leaves a quarter of the
 // lanes without a unit at that size and the loads of too few warps in flight: 144, 324, 59 and 111 us.)  Head sizes without a
 // (LPR, V) of this table take the warp-per-row kernels of ops.cuh.
 #pragma once
@@ -151,14 +153,15 @@ __global__ void __launch_bounds__(256, V <= 3 ? 3 : 2) qkv_rows_bwd_kernel(const
   }
   const bool silu = a.silu[t] != 0;
   if (a.l2norm[t]) {
-    float ss = 0.f, dot = 0.f;
+    float ss = 0.f, dot = 0.f, sgm[V][8];
 #pragma unroll
     for (int i = 0; i < V; ++i) {
       float x[8];
       unpack8(rx[i], x);
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
-        const float u = silu ? silu_bf16(x[e]) : x[e];
+        sgm[i][e] = sigmoidf_fast(x[e]);
+        const float u = silu ? bf16_round(x[e] * sgm[i][e]) : x[e];
         ss += u * u;
         dot += g[i][e] * u;
       }
@@ -173,7 +176,7 @@ __global__ void __launch_bounds__(256, V <= 3 ? 3 : 2) qkv_rows_bwd_kernel(const
       unpack8(rx[i], x);
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
-        const float sg = sigmoidf_fast(x[e]);
+        const float sg = sgm[i][e];
         const float u = silu ? bf16_round(x[e] * sg) : x[e];
         const float d = g[i][e] * inv - u * coef;
         g[i][e] = silu ? d * (sg * (1.f + x[e] * (1.f - sg))) : d;
