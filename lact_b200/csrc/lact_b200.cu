@@ -1415,16 +1415,42 @@ int scan_ns_trace_layout(const lact_scan_config& c, size_t* stride, size_t* g0_b
   return LACT_OK;
 }
 
+struct StateCopy {
+  StateCopyArgs a;
+  int64_t longest = 0;
+  explicit StateCopy(int64_t batch) {
+    std::memset(&a, 0, sizeof(a));
+    a.batch = static_cast<int32_t>(batch);
+  }
+  void add(const float* src, int64_t src_bs, void* dst, int64_t dst_bs, int64_t n) {
+    if (dst == nullptr || src == dst) return;
+    const int i = a.copies++;
+    a.src[i] = src;
+    a.dst[i] = static_cast<float*>(dst);
+    a.src_bs[i] = src_bs; a.dst_bs[i] = dst_bs; a.n[i] = n;
+    a.vec[i] = ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0 && (src_bs | dst_bs | n) % 4 == 0;
+    longest = std::max(longest, n);
+  }
+  int launch(cudaStream_t stream) {
+    if (a.copies == 0) return LACT_OK;
+    KernelScope scope(kClsOther, stream);
+    LACT_CUDA(launch_pdl(state_copy_kernel, dim3(ceil_div(longest, 2048), a.copies, a.batch), dim3(256), 0, stream, a));
+    return LACT_OK;
+  }
+};
+
 // Momentum state the program starts from: the caller's.  Without one the first update adds its factor times zero without
 // reading it, and zeros are written only for a program that hands the state back untouched.
 inline bool has_initial_momentum(const lact_scan_io& io) { return io.m0_in && io.m1_in && io.m2_in; }
 int load_momentum_state(const lact_scan_config& c, const lact_scan_io& io, float* G02, float* G1, cudaStream_t stream) {
   const size_t B = c.B, D = c.D, H = c.H;
   if (has_initial_momentum(io)) {
-    LACT_CUDA(cudaMemcpy2DAsync(G02, 2 * H * D * 4, io.m0_in, H * D * 4, H * D * 4, B, cudaMemcpyDeviceToDevice, stream));
-    LACT_CUDA(cudaMemcpy2DAsync(G02 + H * D, 2 * H * D * 4, io.m2_in, H * D * 4, H * D * 4, B, cudaMemcpyDeviceToDevice,
-                                stream));
-    LACT_CUDA(cudaMemcpyAsync(G1, io.m1_in, B * D * H * 4, cudaMemcpyDeviceToDevice, stream));
+    const int64_t n = static_cast<int64_t>(H * D);
+    StateCopy copy(c.B);
+    copy.add(static_cast<const float*>(io.m0_in), n, G02, 2 * n, n);
+    copy.add(static_cast<const float*>(io.m2_in), n, G02 + n, 2 * n, n);
+    copy.add(static_cast<const float*>(io.m1_in), n, G1, n, n);
+    LACT_TRY(copy.launch(stream));
   } else {
     LACT_CUDA(cudaMemsetAsync(G02, 0, B * 2 * H * D * 4, stream));
     LACT_CUDA(cudaMemsetAsync(G1, 0, B * D * H * 4, stream));
@@ -1461,16 +1487,15 @@ int launch_momentum_means(const lact_scan_config& c, const lact_scan_io& io, int
 // Final fast weights and momentum state into the caller's arrays (those that are given).
 int store_state(const lact_scan_config& c, const lact_scan_io& io, const float* W02, const float* W1, const float* G02,
                 const float* G1, cudaStream_t stream) {
-  const size_t B = c.B, D = c.D, H = c.H;
-  auto half = [&](void* dst, const float* src) {
-    return cudaMemcpy2DAsync(dst, H * D * 4, src, 2 * H * D * 4, H * D * 4, B, cudaMemcpyDeviceToDevice, stream);
-  };
-  if (io.w0_out) LACT_CUDA(half(io.w0_out, W02));
-  if (io.w2_out) LACT_CUDA(half(io.w2_out, W02 + H * D));
-  if (io.w1_out) LACT_CUDA(cudaMemcpyAsync(io.w1_out, W1, B * D * H * 4, cudaMemcpyDeviceToDevice, stream));
-  if (io.m0_out) LACT_CUDA(half(io.m0_out, G02));
-  if (io.m2_out) LACT_CUDA(half(io.m2_out, G02 + H * D));
-  if (io.m1_out) LACT_CUDA(cudaMemcpyAsync(io.m1_out, G1, B * D * H * 4, cudaMemcpyDeviceToDevice, stream));
+  const int64_t n = c.D * c.H;
+  StateCopy copy(c.B);
+  copy.add(W02, 2 * n, io.w0_out, n, n);
+  copy.add(W02 + n, 2 * n, io.w2_out, n, n);
+  copy.add(W1, n, io.w1_out, n, n);
+  copy.add(G02, 2 * n, io.m0_out, n, n);
+  copy.add(G02 + n, 2 * n, io.m2_out, n, n);
+  copy.add(G1, n, io.m1_out, n, n);
+  LACT_TRY(copy.launch(stream));
   return LACT_OK;
 }
 

@@ -527,6 +527,32 @@ __global__ void prepare_weights_kernel(const void* w0, const void* w1, const voi
 // beta[u][b] = mean over tokens [s_u, e_u) of momentum[b, t] for up to kMeanBatch update steps per
 // launch; grid (batch entries, steps).
 constexpr int kMeanBatch = 64;
+// Up to six batched copies of fp32 rows in one launch: entry b of copy i is n[i] values from src[i] + b * src_bs[i] to dst[i] +
+// b * dst_bs[i].  (State in and out of a call is three to six arrays whose copies, one after another, were 12 us of a call that
+// updates 12 entries of 128 x 256 once.)
+struct StateCopyArgs {
+  const float* src[6];
+  float* dst[6];
+  int64_t src_bs[6], dst_bs[6], n[6];
+  int32_t vec[6];   // both sides on 16 bytes, n and strides multiples of four
+  int32_t copies, batch;
+};
+__global__ void __launch_bounds__(256) state_copy_kernel(const StateCopyArgs a) {
+  griddep_launch_dependents();
+  griddep_wait();
+  const int i = blockIdx.y, b = blockIdx.z;
+  const float* const src = a.src[i] + b * a.src_bs[i];
+  float* const dst = a.dst[i] + b * a.dst_bs[i];
+  const int64_t at = (static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x) * 8;
+  if (a.vec[i] && at + 8 <= a.n[i]) {
+    const float4 u = *reinterpret_cast<const float4*>(src + at), v = *reinterpret_cast<const float4*>(src + at + 4);
+    *reinterpret_cast<float4*>(dst + at) = u;
+    *reinterpret_cast<float4*>(dst + at + 4) = v;
+  } else {
+    for (int64_t j = at; j < at + 8 && j < a.n[i]; ++j) dst[j] = src[j];
+  }
+}
+
 struct MeanArgs {
   int32_t n;
   int32_t s[kMeanBatch], e[kMeanBatch];
