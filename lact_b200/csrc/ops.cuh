@@ -1401,6 +1401,8 @@ struct LrPrologueArgs {
   int32_t b, s, n_h;
 };
 __global__ void __launch_bounds__(256) lr_prologue_kernel(const LrPrologueArgs a) {
+  griddep_launch_dependents();
+  griddep_wait();
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const int64_t total = static_cast<int64_t>(a.b) * a.s * a.n_h;
   if (i >= total) return;
@@ -1434,6 +1436,8 @@ struct LrPrologueBwdArgs {
   int32_t b, s, n_h;
 };
 __global__ void __launch_bounds__(256) lr_prologue_bwd_kernel(const LrPrologueBwdArgs a) {
+  griddep_launch_dependents();
+  griddep_wait();
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= static_cast<int64_t>(a.b) * a.s * a.n_h) return;
   const int h = static_cast<int>(i % a.n_h);
@@ -1458,6 +1462,8 @@ __global__ void __launch_bounds__(256) lr_prologue_bwd_kernel(const LrPrologueBw
 // Sums of the columns of an [rows][cols] fp32 matrix (partial sums of many blocks) in a fixed order: a block owns 32
 // columns, its eight warps every eighth row.
 __global__ void __launch_bounds__(256) column_sums_kernel(const float* x, float* out, int64_t rows, int64_t cols) {
+  griddep_launch_dependents();
+  griddep_wait();
   __shared__ float part[8][33];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t c = static_cast<int64_t>(blockIdx.x) * 32 + lane;

@@ -50,6 +50,8 @@ __device__ __forceinline__ void rope_partner(const uint4 (&y)[V], int half_units
 
 template <int LPR, int V, bool ROPE>
 __global__ void __launch_bounds__(256, V <= 3 ? 4 : 2) qkv_rows_kernel(const PrologueArgs a) {
+  griddep_launch_dependents();
+  griddep_wait();
   const int lane = threadIdx.x % LPR, t = blockIdx.y / a.n_h, h = blockIdx.y - t * a.n_h, bi = blockIdx.z;
   const int tok = blockIdx.x * (256 / LPR) + threadIdx.x / LPR;
   const bool live = tok < a.s;  // (every lane takes part in the shuffles)
@@ -111,6 +113,8 @@ __global__ void __launch_bounds__(256, V <= 3 ? 4 : 2) qkv_rows_kernel(const Pro
 
 template <int LPR, int V, bool ROPE>
 __global__ void __launch_bounds__(256, V <= 3 ? 3 : 2) qkv_rows_bwd_kernel(const PrologueBwdArgs a) {
+  griddep_launch_dependents();
+  griddep_wait();
   const int lane = threadIdx.x % LPR, t = blockIdx.y / a.n_h, h = blockIdx.y - t * a.n_h, bi = blockIdx.z;
   const int tok = blockIdx.x * (256 / LPR) + threadIdx.x / LPR;
   const bool live = tok < a.s;
@@ -199,6 +203,8 @@ __global__ void __launch_bounds__(256, V <= 3 ? 3 : 2) qkv_rows_bwd_kernel(const
 
 template <int LPR, int V>
 __global__ void __launch_bounds__(256) out_rows_kernel(const EpilogueArgs a) {
+  griddep_launch_dependents();
+  griddep_wait();
   const int lane = threadIdx.x % LPR, h = blockIdx.y, bi = blockIdx.z;
   const int tok = blockIdx.x * (256 / LPR) + threadIdx.x / LPR;
   const bool live = tok < a.s;
@@ -249,6 +255,8 @@ __global__ void __launch_bounds__(256) out_rows_kernel(const EpilogueArgs a) {
 // keeps its share of the norm weight's gradient in registers; the block's shares are added in shared memory.
 template <int LPR, int V>
 __global__ void __launch_bounds__(256, 2) out_rows_bwd_kernel(const EpilogueBwdArgs a) {
+  griddep_launch_dependents();
+  griddep_wait();
   constexpr int kGroups = 256 / LPR, D = 8 * LPR * V;
   __shared__ float red[8][D];
   const int lane = threadIdx.x % LPR, grp = threadIdx.x / LPR;

@@ -101,6 +101,8 @@ __global__ void __launch_bounds__(320, 1) swa_fwd_kernel(const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = uniform(*tmem_slot);
+  griddep_launch_dependents();
+  griddep_wait();
 
   // this CTA's query tile and the key tiles its window touches
   int tile = blockIdx.x, splits = 1, split = 0;
