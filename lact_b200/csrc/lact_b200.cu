@@ -69,27 +69,6 @@ int encode_map(CUtensorMap* map, const Mat& m, uint32_t box_rows, uint32_t box_c
   return r == CUDA_SUCCESS ? LACT_OK : LACT_ERR_CUDA;
 }
 
-// Encodes a 4-D map (64 cols of a k-block, rows, k-blocks, batch) of a matrix whose column count is a
-// multiple of 64, with a {64, box_rows, kb, 1} box: one load brings `kb` consecutive k-blocks of a row
-// block, laid out in shared memory k-block after k-block.
-int encode_map_kblocks(CUtensorMap* map, const Mat& m, uint32_t box_rows, uint32_t kb) {
-  EncodeFn fn = get_encode_fn();
-  if (fn == nullptr) return LACT_ERR_CUDA;
-  if ((reinterpret_cast<uintptr_t>(m.ptr) & 15) != 0 || (m.ld % 8) != 0 || (m.batch > 1 && (m.bs % 8) != 0))
-    return LACT_ERR_SHAPE;
-  if (m.rows < 1 || m.cols < 64 || (m.cols % 64) != 0 || m.batch < 1 || box_rows > 256) return LACT_ERR_SHAPE;
-  cuuint64_t dims[4] = {64, static_cast<cuuint64_t>(m.rows), static_cast<cuuint64_t>(m.cols / 64),
-                        static_cast<cuuint64_t>(m.batch)};
-  const int64_t bs = m.batch > 1 ? m.bs : m.ld * m.rows;
-  cuuint64_t strides[3] = {static_cast<cuuint64_t>(m.ld) * 2, 128, static_cast<cuuint64_t>(bs) * 2};
-  cuuint32_t box[4] = {64, box_rows, kb, 1};
-  cuuint32_t estr[4] = {1, 1, 1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(m.ptr), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? LACT_OK : LACT_ERR_CUDA;
-}
-
 // As encode_map with a fourth axis, the segments (ops with `kSegments`).
 int encode_map_segments(CUtensorMap* map, const Mat& m, uint32_t box_rows) {
   EncodeFn fn = get_encode_fn();
@@ -110,33 +89,27 @@ int encode_map_segments(CUtensorMap* map, const Mat& m, uint32_t box_rows) {
   return r == CUDA_SUCCESS ? LACT_OK : LACT_ERR_CUDA;
 }
 
-// What the maps of a problem's operands depend on: k-blocks per ring stage, and whether there is a segment axis.
+// What the maps of a problem's operands depend on: whether there is a segment axis.
 struct OperandForm {
-  int kb;
   bool segments;
 };
 template <class Op>
-constexpr OperandForm form_of(const GemmProblem<Op>&) { return OperandForm{Op::KB, op_segments<Op>::value}; }
+constexpr OperandForm form_of(const GemmProblem<Op>&) { 
+  static_assert(Op::KB == 1, "operand boxes are one k-block deep");
+  return OperandForm{op_segments<Op>::value};
+}
 
-// Operand of a GEMM: `m` used K-major (mn = rows, k = cols) or MN-major (k = rows, mn = cols).  With two k-blocks per stage a K-major operand
-// whose k extent is whole k-blocks gets the 4-D map (one box per stage), an MN-major operand a box of
-// 128 k rows per 64-wide atom.
+// Operand of a GEMM: `m` used K-major (mn = rows, k = cols; boxes of `tile_rows`) or MN-major (k = rows, mn = cols; boxes of 64 k
+// rows and 64 columns).
 int make_operand(OperandForm form, CUtensorMap* map, OperandInfo* info, const Mat& m, int mn_major, int tile_rows, int mn_off,
                  int k_off, int batch_off = 0) {
   info->mn_major = mn_major;
-  info->k4d = 0;
   info->mn_off = mn_off;
   info->k_off = k_off;
   info->batch_off = batch_off;
-  const int kb = form.kb;
   if (((mn_major ? mn_off : k_off) % 8) != 0) return LACT_ERR_SHAPE;  // innermost TMA coordinate: 16-byte rule
-  if (form.segments) return encode_map_segments(map, m, static_cast<uint32_t>(mn_major ? 64 * kb : tile_rows));
-  if (mn_major) return encode_map(map, m, static_cast<uint32_t>(64 * kb));
-  if (kb == 2 && (m.cols % 64) == 0 && (k_off % 64) == 0) {
-    info->k4d = 1;
-    return encode_map_kblocks(map, m, static_cast<uint32_t>(tile_rows), 2);
-  }
-  return encode_map(map, m, static_cast<uint32_t>(tile_rows));
+  if (form.segments) return encode_map_segments(map, m, static_cast<uint32_t>(mn_major ? kBK : tile_rows));
+  return encode_map(map, m, static_cast<uint32_t>(mn_major ? kBK : tile_rows));
 }
 
 // Output of a staged epilogue: bf16 matrix `m` whose extents clip the stored tiles.
@@ -1157,30 +1130,30 @@ static int launch_ns_bwd_fused(const NsTrace* tr, const bf16* const* du, int ngr
       auto& pt = args.t[it][g];
       auto& px = args.dx[it][g];
       // Q = dX X^T + X dX^T (wide; the iterate's rows are K-major operands) / dX^T X + X^T dX (tall; MN-major)
-      LACT_TRY(make_operand(OperandForm{1, false}, &pq.a[0], &pq.ai[0], D, tall, kBM, 0, 0));
-      LACT_TRY(make_operand(OperandForm{1, false}, &pq.b[0], &pq.bi[0], X, tall, BT_MM, 0, 0));
-      LACT_TRY(make_operand(OperandForm{1, false}, &pq.a[1], &pq.ai[1], X, tall, kBM, 0, 0));
-      LACT_TRY(make_operand(OperandForm{1, false}, &pq.b[1], &pq.bi[1], D, tall, BT_MM, 0, 0));
+      LACT_TRY(make_operand(OperandForm{false}, &pq.a[0], &pq.ai[0], D, tall, kBM, 0, 0));
+      LACT_TRY(make_operand(OperandForm{false}, &pq.b[0], &pq.bi[0], X, tall, BT_MM, 0, 0));
+      LACT_TRY(make_operand(OperandForm{false}, &pq.a[1], &pq.ai[1], X, tall, kBM, 0, 0));
+      LACT_TRY(make_operand(OperandForm{false}, &pq.b[1], &pq.bi[1], D, tall, BT_MM, 0, 0));
       pq.M = G.m; pq.N = G.m; pq.K = G.n; pq.batch = G.nmat;
       LACT_TRY(make_output(form_of(pq), &pq.out[0], &pq.oi[0], Q, 0, 0));
       // T = c (S Q + Q S): all three symmetric, rows serve as K-major operands on either side
-      LACT_TRY(make_operand(OperandForm{1, false}, &pt.a[0], &pt.ai[0], S, 0, kBM, 0, 0));
-      LACT_TRY(make_operand(OperandForm{1, false}, &pt.b[0], &pt.bi[0], Q, 0, BT_MM, 0, 0));
-      LACT_TRY(make_operand(OperandForm{1, false}, &pt.a[1], &pt.ai[1], Q, 0, kBM, 0, 0));
-      LACT_TRY(make_operand(OperandForm{1, false}, &pt.b[1], &pt.bi[1], S, 0, BT_MM, 0, 0));
+      LACT_TRY(make_operand(OperandForm{false}, &pt.a[0], &pt.ai[0], S, 0, kBM, 0, 0));
+      LACT_TRY(make_operand(OperandForm{false}, &pt.b[0], &pt.bi[0], Q, 0, BT_MM, 0, 0));
+      LACT_TRY(make_operand(OperandForm{false}, &pt.a[1], &pt.ai[1], Q, 0, kBM, 0, 0));
+      LACT_TRY(make_operand(OperandForm{false}, &pt.b[1], &pt.bi[1], S, 0, BT_MM, 0, 0));
       pt.M = G.m; pt.N = G.m; pt.K = G.m; pt.batch = G.nmat;
       LACT_TRY(make_output(form_of(pt), &pt.out[0], &pt.oi[0], T, 0, 0));
       // dX_i = P dX + T X (wide: the [k][n] iterates are MN-major B operands) / dX P + X T (tall)
       if (!tall) {
-        LACT_TRY(make_operand(OperandForm{1, false}, &px.a[0], &px.ai[0], PB, 0, kBM, 0, 0));
-        LACT_TRY(make_operand(OperandForm{1, false}, &px.b[0], &px.bi[0], D, 1, BT, 0, 0));
-        LACT_TRY(make_operand(OperandForm{1, false}, &px.a[1], &px.ai[1], T, 0, kBM, 0, 0));
-        LACT_TRY(make_operand(OperandForm{1, false}, &px.b[1], &px.bi[1], X, 1, BT, 0, 0));
+        LACT_TRY(make_operand(OperandForm{false}, &px.a[0], &px.ai[0], PB, 0, kBM, 0, 0));
+        LACT_TRY(make_operand(OperandForm{false}, &px.b[0], &px.bi[0], D, 1, BT, 0, 0));
+        LACT_TRY(make_operand(OperandForm{false}, &px.a[1], &px.ai[1], T, 0, kBM, 0, 0));
+        LACT_TRY(make_operand(OperandForm{false}, &px.b[1], &px.bi[1], X, 1, BT, 0, 0));
       } else {
-        LACT_TRY(make_operand(OperandForm{1, false}, &px.a[0], &px.ai[0], D, 0, kBM, 0, 0));
-        LACT_TRY(make_operand(OperandForm{1, false}, &px.b[0], &px.bi[0], PB, 0, BT, 0, 0));
-        LACT_TRY(make_operand(OperandForm{1, false}, &px.a[1], &px.ai[1], X, 0, kBM, 0, 0));
-        LACT_TRY(make_operand(OperandForm{1, false}, &px.b[1], &px.bi[1], T, 0, BT, 0, 0));
+        LACT_TRY(make_operand(OperandForm{false}, &px.a[0], &px.ai[0], D, 0, kBM, 0, 0));
+        LACT_TRY(make_operand(OperandForm{false}, &px.b[0], &px.bi[0], PB, 0, BT, 0, 0));
+        LACT_TRY(make_operand(OperandForm{false}, &px.a[1], &px.ai[1], X, 0, kBM, 0, 0));
+        LACT_TRY(make_operand(OperandForm{false}, &px.b[1], &px.bi[1], T, 0, BT, 0, 0));
       }
       px.M = ns_upd_rows(G); px.N = ns_upd_cols(G); px.K = G.m; px.batch = G.nmat;
       LACT_TRY(make_output(form_of(px), &px.out[0], &px.oi[0], O, 0, 0));

@@ -380,15 +380,13 @@ struct OpNs2T {
 template <int BT_>
 using OpNs2 = OpNs2T<BT_, false>;
 
-// [y0 | y2] = x [w0 slice ; w2 slice]^T; epilogue = SwiGLU gate, staged.  With one k-block per stage
-// the two weight tiles are adjacent in shared memory and one 128 x 2BT MMA covers both; with two
-// k-blocks per stage each tile holds its k-blocks back to back, so the product is two 128 x BT MMAs
-// into adjacent accumulator columns.
+// [y0 | y2] = x [w0 slice ; w2 slice]^T; epilogue = SwiGLU gate, staged.  The two weight tiles are
+// adjacent in shared memory and one 128 x 2BT MMA covers both.
 template <int BT_>
 struct OpSwigluGate {
   static constexpr bool kSegments = true;
   static constexpr int KB = 1;  // measured: two-k-block stages (a 2-deep ring here) are 7 % slower for this op
-  static constexpr int NA = 1, NB = 2, NACC = 2, BT = BT_, NTERMS = KB, NOUT = 1;
+  static constexpr int NA = 1, NB = 2, NACC = 2, BT = BT_, NTERMS = 1, NOUT = 1;
   static constexpr bool kTileReduce = false;
   static constexpr bool kWarpTranspose = false, kReverseBatch = false;
   static constexpr uint32_t kEpiScratch = 0;
@@ -397,7 +395,7 @@ struct OpSwigluGate {
   __host__ __device__ static constexpr int term_a(int) { return 0; }
   __host__ __device__ static constexpr int term_b(int t) { return t; }
   __host__ __device__ static constexpr int term_col(int t) { return t * BT_; }
-  __host__ __device__ static constexpr int term_n(int) { return KB == 2 ? BT_ : 2 * BT_; }
+  __host__ __device__ static constexpr int term_n(int) { return 2 * BT_; }
   __host__ __device__ static constexpr bool term_first(int) { return true; }
   using Prefetch = NoPrefetch;
   __device__ static __forceinline__ void prefetch(const Epi&, int, int, int, int, int, int, Prefetch&) {}

@@ -23,7 +23,6 @@ constexpr uint32_t kAtomBytes = 64 * kBK * 2;  // one 64(mn) x 64(k) MN-major at
 
 struct OperandInfo {
   int32_t mn_major;   // 0: global [mn][k] (k contiguous); 1: global [k][mn] (mn contiguous)
-  int32_t k4d;        // K-major only: the map is 4-D (64 k, rows, k-blocks, batch) and one box spans the stage's k-blocks
   int32_t mn_off;     // added to the mn coordinate
   int32_t k_off;      // added to the k coordinate
   int32_t batch_off;  // added to the batch coordinate
@@ -108,8 +107,6 @@ __host__ __device__ constexpr int flow_ring(uint32_t stride) {
 // One operand tile of a ring stage: ROWS (mn) x KB k-blocks.  Shared-memory layout:
 //   K-major:  [k-block][ROWS rows][64 k] (KB tiles of ROWS x 128 bytes back to back);
 //   MN-major: per 64-wide mn atom [KB * 64 k rows][64 mn] (atoms KB * 8 KB apart).
-// With KB = 2 a K-major tile arrives as one box of a 4-D map when the operand allows it (k4d), an
-// MN-major tile as one 128-k-row box per atom.
 // The cursor holds the coordinates of an operand's next boxes: they are worked out once per output tile, so that between two
 // stages the issuing warp only adds.  (What that warp spends per box is what the loads can reach: see gemm_phase.)
 // SEG: the maps are 4-D (inner, row, entry, segment), see op_segments.
@@ -118,21 +115,16 @@ struct OperandCursor {
   const CUtensorMap* map;
   int32_t inner, row, batch, segment;  // first box of the stage; 4-D maps: inner = k-block, row = mn
   int32_t d_inner, d_row;     // advance per stage
-  int32_t kind;               // 0: K-major, a box per k-block; 1: K-major, one 4-D box; 2: MN-major, a box per atom
+  int32_t mn_major;           // 0: K-major, a box per k-block; 1: MN-major, a box per atom
   __device__ __forceinline__ void start(const CUtensorMap* m, const OperandInfo& oi, int mn0, int kc, int b, int seg) {
     map = m;
     batch = oi.batch_off + b;
     segment = seg;
-    if (oi.mn_major) {
-      kind = 2;
+    mn_major = oi.mn_major;
+    if (mn_major) {
       inner = oi.mn_off + mn0; row = oi.k_off + kc;
       d_inner = 0; d_row = KB * kBK;
-    } else if (!SEG && KB == 2 && oi.k4d) {
-      kind = 1;
-      inner = (oi.k_off + kc) / kBK; row = oi.mn_off + mn0;
-      d_inner = KB; d_row = 0;
     } else {
-      kind = 0;
       inner = oi.k_off + kc; row = oi.mn_off + mn0;
       d_inner = KB * kBK; d_row = 0;
     }
@@ -142,11 +134,9 @@ struct OperandCursor {
     else tma_load_3d_if(leader, dst, map, bar, at, row, batch);
   }
   __device__ __forceinline__ void load(uint32_t leader, uint32_t dst, uint32_t bar) {
-    if (kind == 0) {
+    if (!mn_major) {
 #pragma unroll
       for (int kk = 0; kk < KB; ++kk) box(leader, dst + kk * (ROWS * kBK * 2), bar, inner + kk * kBK);
-    } else if (!SEG && KB == 2 && kind == 1) {
-      tma_load_4d_if(leader, dst, map, bar, 0, row, inner, batch);
     } else {
 #pragma unroll
       for (int j = 0; j < ROWS / 64; ++j) box(leader, dst + j * (KB * kAtomBytes), bar, inner + 64 * j);
