@@ -1256,18 +1256,19 @@ struct ScanPlan {
 // 128 x 256 and 1560 tokens take 26 us a step alone and 9.5 us in runs of six (21 steps: 1669 -> 1487 us the whole call; 4 entries of
 // 384, 2048 tokens, two steps: 354 -> 343).  Steps are collected until they have kApplyRounds tiles of 128 tokens and hidden
 // features per SM, which also bounds the memory their weights and hidden activations take; a step that has as many by itself
-// gains nothing.  `out_start` nullptr: as if the outputs were disjoint.
+// gains nothing.  `free_slots`: how many weight slots there are from the one of step `i` on; `out_start` nullptr: as if the outputs
+// were disjoint.
 constexpr int64_t kApplyRounds = 12;
 struct ApplyRun {
   int64_t steps, x_step, o_step;
 };
 ApplyRun apply_run(const lact_scan_config& c, int32_t n_steps, const int32_t* kind, const int64_t* start, const int64_t* end,
-                   const int64_t* out_start, int32_t i) {
+                   const int64_t* out_start, int32_t i, int64_t free_slots) {
   ApplyRun r{1, 0, 0};
   const int64_t len = end[i] - start[i];
   if (len <= 0) return r;
   const int64_t tiles = c.B * ceil_div(len, kBM) * ceil_div(c.H, kBM);
-  const int64_t most = (kApplyRounds * sm_count() + tiles - 1) / tiles;
+  const int64_t most = std::min((kApplyRounds * sm_count() + tiles - 1) / tiles, free_slots);
   int64_t at = i;
   while (r.steps < most && at + 2 < n_steps && kind[at + 1] == LACT_STEP_UPDATE && kind[at + 2] == LACT_STEP_APPLY &&
          end[at + 2] - start[at + 2] == len) {
@@ -1298,9 +1299,11 @@ int plan_scan(const lact_scan_config& c, int32_t n_steps, const int32_t* kind, c
       max_update = std::max(max_update, len);
     } else return LACT_ERR_STEPS;
   }
-  for (int i = 0; i < n_steps; ++i) {  // (runs from any step: which ones there are also depends on the outputs' places)
+  // (the longest run, wherever it begins: which runs there are also depends on the outputs' places.  One that does not begin in slot
+  // 0 may find fewer slots and ends earlier.)
+  for (int i = 0; i < n_steps; ++i) {
     if (kind[i] != LACT_STEP_APPLY) continue;
-    const int64_t steps = apply_run(c, n_steps, kind, start, end, nullptr, i).steps;
+    const int64_t steps = apply_run(c, n_steps, kind, start, end, nullptr, i, n_steps).steps;
     slots = std::max(slots, steps);
     max_apply = std::max(max_apply, steps * (end[i] - start[i]));
   }
@@ -1532,7 +1535,8 @@ int scan_fwd(const lact_scan_config& c, const lact_scan_io& io, int32_t n_steps,
   for (int i = 0; i < n_steps; ++i) {
     if (kind[i] == LACT_STEP_APPLY) {
       if (missing == 0) {
-        const ApplyRun run = apply_run(c, n_steps, kind, start, end, out_start, i);
+        const int64_t free_slots = io.shadow_dump != nullptr ? n_steps : p.w_slots - w_slot;
+        const ApplyRun run = apply_run(c, n_steps, kind, start, end, out_start, i, free_slots);
         pending = ApplyArgs{W02b, W1b, io.q, c.q_bs, c.q_ts, start[i], end[i], io.o, c.o_bs, c.o_ts, out_start[i],
                             p.hidden, B, D, H};
         pending.segs = missing = run.steps;
@@ -1595,9 +1599,9 @@ int scan_fwd(const lact_scan_config& c, const lact_scan_io& io, int32_t n_steps,
     // add + renormalise arguments (the update is the Newton-Schulz result when Muon is on)
     // (the fp32 copy of the normalised weights is what pre-norm computes with and what the final export reads)
     const bool want_compute = c.prenorm || ((io.w0_out || io.w1_out || io.w2_out) && !has_later_update(kind, n_steps, i));
-    // (the weights of steps still to run are not overwritten: a run starts in slot 0 or, the first one, where the weights are)
+    // (the weights of steps still to run are not overwritten: a run takes the slots from the one on that the weights are in, and no
+    // more than there are)
     const int next_slot = io.shadow_dump != nullptr ? update_idx : (missing > 0 ? w_slot + 1 : 0);
-    if (io.shadow_dump == nullptr && next_slot >= p.w_slots) return LACT_ERR_WORKSPACE;
     RenormArgs rn[2];
     for (int w = 0; w < 2; ++w) {
       RenormArgs& r = rn[w];
