@@ -1252,13 +1252,27 @@ struct ScanPlan {
 
 // How many APPLY steps from step `i` on are left to the last of them, which then runs all in one launch (ApplyArgs::segs): steps
 // of one length, evenly spaced, with one UPDATE between each two (so that their weights lie in consecutive slots), whose outputs
-// do not overlap.  A step of few tiles costs its launches' fill and drain, in series with the chain of updates: 12 entries of
-// 128 x 256 and 1560 tokens take 26 us a step alone and 9.5 us in runs of six (21 steps: 1669 -> 1487 us the whole call; 4 entries of
-// 384, 2048 tokens, two steps: 354 -> 343).  Steps are collected until they have kApplyRounds tiles of 128 tokens and hidden
-// features per SM, which also bounds the memory their weights and hidden activations take; a step that has as many by itself
-// gains nothing.  `free_slots`: how many weight slots there are from the one of step `i` on; `out_start` nullptr: as if the outputs
-// were disjoint.
-constexpr int64_t kApplyRounds = 12;
+// do not overlap.  A step of few tiles costs its launches' fill and drain, in series with the chain of updates.  Steps are collected
+// until they have kApplyRounds tiles of 128 tokens and hidden features per SM, which bounds the memory of their hidden activations to
+// 58 MB beside one step's, and as long as their weights take no more than kRunWeightBytes: short steps of many weights would fill
+// hundreds of slots.  us per call:
+//   12 entries of 128 x 256, 21 steps of 1560 tokens: single steps 1674, six tiles per SM 1510, twelve 1473, twenty-four 1466; 4 entries of
+//   384, 16 steps of 512 tokens 1795 / 1611 / 1602 / 1617
+//   4 entries of 384, 255 steps of 128 tokens: single steps 10035, weights of 16 MB 7008, 64 MB 6310, 128 MB 6255, no bound 6167 (524 MB);
+//   16 entries of 512, 16 steps of 512 tokens 1833 / 1837 / 1782 / 1740 / 1710
+// `free_slots`: how many weight slots there are from the one of step `i` on.
+constexpr int64_t kApplyRounds = 12, kRunWeightBytes = 128 << 20;
+// The most steps of `len` tokens that share a launch.
+int64_t longest_run(const lact_scan_config& c, int64_t len) {
+  const int64_t tiles = c.B * ceil_div(len, kBM) * ceil_div(c.H, kBM);
+  return std::max<int64_t>(1, std::min((kApplyRounds * sm_count() + tiles - 1) / tiles, kRunWeightBytes / (c.B * 3 * c.H * c.D * 2)));
+}
+// Whether APPLY step `i` and the one two steps on may be neighbours in a run.
+bool run_goes_on(int32_t n_steps, const int32_t* kind, const int64_t* start, const int64_t* end, int32_t i) {
+  const int64_t len = end[i] - start[i];
+  return i + 2 < n_steps && kind[i + 1] == LACT_STEP_UPDATE && kind[i + 2] == LACT_STEP_APPLY && len > 0 &&
+         end[i + 2] - start[i + 2] == len && start[i + 2] > start[i];
+}
 struct ApplyRun {
   int64_t steps, x_step, o_step;
 };
@@ -1267,13 +1281,10 @@ ApplyRun apply_run(const lact_scan_config& c, int32_t n_steps, const int32_t* ki
   ApplyRun r{1, 0, 0};
   const int64_t len = end[i] - start[i];
   if (len <= 0) return r;
-  const int64_t tiles = c.B * ceil_div(len, kBM) * ceil_div(c.H, kBM);
-  const int64_t most = std::min((kApplyRounds * sm_count() + tiles - 1) / tiles, free_slots);
-  int64_t at = i;
-  while (r.steps < most && at + 2 < n_steps && kind[at + 1] == LACT_STEP_UPDATE && kind[at + 2] == LACT_STEP_APPLY &&
-         end[at + 2] - start[at + 2] == len) {
-    const int64_t dx = start[at + 2] - start[at], dout = out_start != nullptr ? out_start[at + 2] - out_start[at] : len;
-    if (dx <= 0 || dout < len) break;
+  const int64_t most = std::min(longest_run(c, len), free_slots);
+  for (int32_t at = i; r.steps < most && run_goes_on(n_steps, kind, start, end, at); at += 2) {
+    const int64_t dx = start[at + 2] - start[at], dout = out_start[at + 2] - out_start[at];
+    if (dout < len) break;
     if (r.steps == 1) {
       r.x_step = dx;
       r.o_step = dout;
@@ -1281,7 +1292,6 @@ ApplyRun apply_run(const lact_scan_config& c, int32_t n_steps, const int32_t* ki
       break;
     }
     ++r.steps;
-    at += 2;
   }
   return r;
 }
@@ -1299,13 +1309,18 @@ int plan_scan(const lact_scan_config& c, int32_t n_steps, const int32_t* kind, c
       max_update = std::max(max_update, len);
     } else return LACT_ERR_STEPS;
   }
-  // (the longest run, wherever it begins: which runs there are also depends on the outputs' places.  One that does not begin in slot
-  // 0 may find fewer slots and ends earlier.)
+  // As many slots as the longest run of evenly spaced steps, wherever it begins (which runs there are also depends on the outputs'
+  // places).  A run that does not begin in slot 0 may find fewer and ends earlier.  `even[i & 1]`: steps of the evenly spaced stretch
+  // that ends with step i.
+  int64_t even[2] = {1, 1};
   for (int i = 0; i < n_steps; ++i) {
-    if (kind[i] != LACT_STEP_APPLY) continue;
-    const int64_t steps = apply_run(c, n_steps, kind, start, end, nullptr, i, n_steps).steps;
+    int64_t& n = even[i & 1];
+    if (i < 2 || kind[i - 2] != LACT_STEP_APPLY || !run_goes_on(n_steps, kind, start, end, i - 2)) n = 1;
+    else n = n > 1 && start[i] - start[i - 2] != start[i - 2] - start[i - 4] ? 2 : n + 1;
+    if (kind[i] != LACT_STEP_APPLY || end[i] == start[i]) continue;
+    const int64_t len = end[i] - start[i], steps = std::min(n, longest_run(c, len));
     slots = std::max(slots, steps);
-    max_apply = std::max(max_apply, steps * (end[i] - start[i]));
+    max_apply = std::max(max_apply, steps * len);
   }
   Carver cv(base);
   const size_t B = c.B, D = c.D, H = c.H;
