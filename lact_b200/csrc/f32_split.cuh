@@ -358,29 +358,31 @@ __global__ void __launch_bounds__(kCutThreads, 1) cut_gemm_kernel(const __grid_c
       }
       if (failed) break;
       if constexpr (MODE == kCutStore) {
-        if (row >= P.M) continue;
-        float* const C = P.c + (static_cast<int64_t>(r.split) * P.batch + r.b) * P.c_bs + static_cast<int64_t>(row) * P.c_ld + r.n0 + part * SUMS;
-        const int left = P.N - r.n0 - part * SUMS;
+        if (row < P.M) {
+          float* const C = P.c + (static_cast<int64_t>(r.split) * P.batch + r.b) * P.c_bs + static_cast<int64_t>(row) * P.c_ld + r.n0 + part * SUMS;
+          const int left = P.N - r.n0 - part * SUMS;
 #pragma unroll
-        for (int j = 0; j < SUMS; j += 8) {
-          if (j + 8 <= left && P.c_vec == 2) {
-            uint32_t w[8];
+          for (int j = 0; j < SUMS; j += 8) {
+            if (j + 8 <= left && P.c_vec == 2) {
+              uint32_t w[8];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) w[e] = __float_as_uint(sum[j + e]);
-            st_global_32(C + j, w);
-          } else {
+              for (int e = 0; e < 8; ++e) w[e] = __float_as_uint(sum[j + e]);
+              st_global_32(C + j, w);
+            } else {
 #pragma unroll
-            for (int e = 0; e < 8; e += 4) {
-              if (j + e + 4 <= left && P.c_vec) {
-                *reinterpret_cast<float4*>(C + j + e) = make_float4(sum[j + e], sum[j + e + 1], sum[j + e + 2], sum[j + e + 3]);
-              } else {
+              for (int e = 0; e < 8; e += 4) {
+                if (j + e + 4 <= left && P.c_vec) {
+                  *reinterpret_cast<float4*>(C + j + e) = make_float4(sum[j + e], sum[j + e + 1], sum[j + e + 2], sum[j + e + 3]);
+                } else {
 #pragma unroll
-                for (int f = e; f < e + 4; ++f)
-                  if (j + f < left) C[j + f] = sum[j + f];
+                  for (int f = e; f < e + 4; ++f)
+                    if (j + f < left) C[j + f] = sum[j + f];
+                }
               }
             }
           }
         }
+        __syncwarp();  // (the next unit's tensor-memory loads want the warp together)
       } else {
         // h, dy0 and dy2 take the places of y0, y2 and dh
 #pragma unroll

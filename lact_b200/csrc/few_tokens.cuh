@@ -185,6 +185,7 @@ __global__ void __launch_bounds__(kFewThreads, 1) few_tokens_kernel(const __grid
         for (int j = 0; j < 16; ++j)
           if (n0 + j < a.tokens) out[(n0 + j) * a.o_ts] = __float2bfloat16_rn(__uint_as_float(v[j]));
       }
+      __syncwarp();  // (the next load of tensor memory wants the warp together; rows1 may end inside it)
     }
     tc_fence_before();
   }

@@ -589,9 +589,9 @@ __device__ __forceinline__ bool gemm_phase(GemmCtx& cx, const GemmProblem<Op>* p
                            : "memory");
               if (got && at < P.N && col < P.M) st_global_16(out + at * ld + col, x[0], x[1], x[2], x[3]);
             }
-            __syncwarp();
           }
         }
+        __syncwarp();  // (scratch; and the next tensor-memory load wants the warp together, whose last rows may lie past M)
       }
       // (the loading warps of other SMs have the proxy fence between the counter and their bulk loads of these rows)
       named_barrier_sync(2, kEpiWarps * 32);

@@ -37,9 +37,10 @@ def _exact(w0, w1, w2, q, k, v, l0, l1, l2):
     return (F.silu(q @ u[0].mT) * (q @ u[2].mT)) @ u[1].mT
 
 
-# tokens around slabs of 64 and rows of 128; sides that 8, 64 and 128 do not divide; contractions cut into many and into one
+# tokens around slabs of 64 and rows of 128; sides that 8, 64 and 128 do not divide; contractions cut into many and into one; rows past
+# the end of a tile in a warp that has another tile to do (more entries than SMs)
 @pytest.mark.parametrize("b,n,d,h", [(1, 1, 64, 64), (2, 63, 12, 8), (1, 65, 68, 72), (3, 129, 128, 128), (2, 1000, 100, 200),
-                                     (1, 4100, 192, 192), (40, 200, 64, 128), (2, 300, 320, 136)])
+                                     (1, 4100, 192, 192), (40, 200, 64, 128), (2, 300, 320, 136), (400, 33, 64, 72)])
 def test_close_to_64_bits(lb, b, n, d, h):
     args = _inputs(b, n, d, h, seed=n)
     o = lb.bidirectional_lact_swiglu(*args, use_muon=False).double()
