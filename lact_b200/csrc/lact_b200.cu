@@ -460,7 +460,9 @@ bool few_pays(int64_t B, int64_t tokens, int64_t D, int64_t H) {
   const int64_t per_sm = 233472 / (few_smem_bytes(static_cast<int>(D), static_cast<int>(H), static_cast<int>(nt)) + 1024);
   return B * (H / 64) <= per_sm * sm_count();
 }
-int launch_few(const ApplyArgs& a, const Mat& x, const Mat& w02, const Mat& w1, int32_t* status, cudaStream_t stream) {
+int launch_few(const ApplyArgs& a, const Mat& x, const Mat& w02, const Mat& w1, const Mat& om, int32_t* status, cudaStream_t stream) {
+  // (outputs that the two launches' maps do not take are refused here too: stores of single values want 2 bytes all the same)
+  if ((reinterpret_cast<uintptr_t>(om.ptr) & 15) != 0 || om.ld % 8 != 0 || (om.batch > 1 && om.bs % 8 != 0)) return LACT_ERR_SHAPE;
   static std::mutex mu;
   static bool configured[64] = {false};
   int dev = 0;
@@ -515,7 +517,7 @@ int run_apply(const ApplyArgs& a, int32_t* status, cudaStream_t stream) {
   const Mat om{static_cast<bf16*>(a.out) + a.out_start * a.o_ts, len, a.D, a.o_ts, a.B, a.o_bs, a.segs, a.o_step * a.o_ts};
   const Mat hid{a.hidden, len, a.H, a.H, a.B, len * a.H, a.segs, a.B * len * a.H};
   const int64_t batch = a.segs * a.B;
-  if (a.segs == 1 && few_pays(a.B, len, a.D, a.H)) return launch_few(a, x, w02, w1, status, stream);
+  if (a.segs == 1 && few_pays(a.B, len, a.D, a.H)) return launch_few(a, x, w02, w1, om, status, stream);
   if (a.H % 128 == 0) LACT_TRY(launch_gate<128>(a, x, w02, len, status, stream));
   else LACT_TRY(launch_gate<64>(a, x, w02, len, status, stream));
   const int bt = choose_bt({{a.D, 1}});

@@ -43,6 +43,24 @@ def test_views_and_neighbours():
     assert torch.equal(parts, whole)
 
 
+@pytest.mark.parametrize("n", [5, 65])
+@pytest.mark.parametrize("which", ["x", "out"])
+def test_rows_off_16_bytes_are_refused(n, which):
+    """As with more tokens, before any launch."""
+    from lact_b200 import _lib as L
+    g = torch.Generator(device="cuda").manual_seed(3)
+    w02, w1 = (w.bfloat16() for w in _weights(2, 64, 64, g))
+    buf = {k: torch.zeros(2 * n * 64 + 8, dtype=torch.bfloat16, device="cuda") for k in ("x", "out")}
+    hidden, word = torch.empty(2 * n * 64, dtype=torch.bfloat16, device="cuda"), torch.zeros(64, dtype=torch.int32, device="cuda")
+    p = lambda t, off=0: C.c_void_p(t.data_ptr() + off)
+    call = lambda off: L.lib().lact_swiglu_ffn_apply(p(w02), p(w1), p(buf["x"], off if which == "x" else 0),
+                                                     p(buf["out"], off if which == "out" else 0), p(hidden),
+                                                     *map(C.c_int64, (2, n, 64, 64)), p(word), C.c_void_p(L.stream_ptr()))
+    assert call(0) == 0
+    torch.cuda.synchronize()
+    assert call(2) == -2 and call(8) == -2
+
+
 def test_nothing_is_written_after_an_earlier_failure():
     """(A status word that is set: the kernel stands aside, and so do all CTAs of a cluster.)"""
     from lact_b200 import _lib as L
