@@ -1413,20 +1413,26 @@ int scan_ns_trace_layout(const lact_scan_config& c, size_t* stride, size_t* g0_b
 struct StateCopy {
   StateCopyArgs a;
   int64_t longest = 0;
-  explicit StateCopy(int64_t batch) {
+  cudaStream_t stream;
+  StateCopy(int64_t batch, cudaStream_t s) : stream(s) {
     std::memset(&a, 0, sizeof(a));
     a.batch = static_cast<int32_t>(batch);
   }
-  void add(const float* src, int64_t src_bs, void* dst, int64_t dst_bs, int64_t n) {
-    if (dst == nullptr || src == dst) return;
+  int add(const float* src, int64_t src_bs, void* dst, int64_t dst_bs, int64_t n) {
+    if (dst == nullptr || src == dst) return LACT_OK;
+    if (((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 3) != 0) {  // (an array packed behind bytes)
+      LACT_CUDA(cudaMemcpy2DAsync(dst, dst_bs * 4, src, src_bs * 4, n * 4, a.batch, cudaMemcpyDeviceToDevice, stream));
+      return LACT_OK;
+    }
     const int i = a.copies++;
     a.src[i] = src;
     a.dst[i] = static_cast<float*>(dst);
     a.src_bs[i] = src_bs; a.dst_bs[i] = dst_bs; a.n[i] = n;
     a.vec[i] = ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0 && (src_bs | dst_bs | n) % 4 == 0;
     longest = std::max(longest, n);
+    return LACT_OK;
   }
-  int launch(cudaStream_t stream) {
+  int launch() {
     if (a.copies == 0) return LACT_OK;
     KernelScope scope(kClsOther, stream);
     LACT_CUDA(launch_pdl(state_copy_kernel, dim3(ceil_div(longest, 2048), a.copies, a.batch), dim3(256), 0, stream, a));
@@ -1441,11 +1447,11 @@ int load_momentum_state(const lact_scan_config& c, const lact_scan_io& io, float
   const size_t B = c.B, D = c.D, H = c.H;
   if (has_initial_momentum(io)) {
     const int64_t n = static_cast<int64_t>(H * D);
-    StateCopy copy(c.B);
-    copy.add(static_cast<const float*>(io.m0_in), n, G02, 2 * n, n);
-    copy.add(static_cast<const float*>(io.m2_in), n, G02 + n, 2 * n, n);
-    copy.add(static_cast<const float*>(io.m1_in), n, G1, n, n);
-    LACT_TRY(copy.launch(stream));
+    StateCopy copy(c.B, stream);
+    LACT_TRY(copy.add(static_cast<const float*>(io.m0_in), n, G02, 2 * n, n));
+    LACT_TRY(copy.add(static_cast<const float*>(io.m2_in), n, G02 + n, 2 * n, n));
+    LACT_TRY(copy.add(static_cast<const float*>(io.m1_in), n, G1, n, n));
+    LACT_TRY(copy.launch());
   } else {
     LACT_CUDA(cudaMemsetAsync(G02, 0, B * 2 * H * D * 4, stream));
     LACT_CUDA(cudaMemsetAsync(G1, 0, B * D * H * 4, stream));
@@ -1483,15 +1489,14 @@ int launch_momentum_means(const lact_scan_config& c, const lact_scan_io& io, int
 int store_state(const lact_scan_config& c, const lact_scan_io& io, const float* W02, const float* W1, const float* G02,
                 const float* G1, cudaStream_t stream) {
   const int64_t n = c.D * c.H;
-  StateCopy copy(c.B);
-  copy.add(W02, 2 * n, io.w0_out, n, n);
-  copy.add(W02 + n, 2 * n, io.w2_out, n, n);
-  copy.add(W1, n, io.w1_out, n, n);
-  copy.add(G02, 2 * n, io.m0_out, n, n);
-  copy.add(G02 + n, 2 * n, io.m2_out, n, n);
-  copy.add(G1, n, io.m1_out, n, n);
-  LACT_TRY(copy.launch(stream));
-  return LACT_OK;
+  StateCopy copy(c.B, stream);
+  LACT_TRY(copy.add(W02, 2 * n, io.w0_out, n, n));
+  LACT_TRY(copy.add(W02 + n, 2 * n, io.w2_out, n, n));
+  LACT_TRY(copy.add(W1, n, io.w1_out, n, n));
+  LACT_TRY(copy.add(G02, 2 * n, io.m0_out, n, n));
+  LACT_TRY(copy.add(G02 + n, 2 * n, io.m2_out, n, n));
+  LACT_TRY(copy.add(G1, n, io.m1_out, n, n));
+  return copy.launch();
 }
 
 int scan_fwd(const lact_scan_config& c, const lact_scan_io& io, int32_t n_steps, const int32_t* kind,

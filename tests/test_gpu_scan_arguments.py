@@ -69,6 +69,47 @@ def test_c_abi_returns_each_weight_by_itself(which):
         assert torch.equal(out[x], want[x]), x
 
 
+@pytest.mark.parametrize("offset", [0, 2, 4])
+def test_state_arrays_on_any_byte(offset):
+    """Momentum in and out and the final weights may start anywhere (they are copied, byte by byte if need be)."""
+    from lact_b200 import _lib as L
+    from lact_b200 import ops
+    from lact_b200 import program as P
+    B, n, D, H = 2, 64, 64, 32
+    i = _inputs(B, n, D, H)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    m = [torch.randn(i[w].shape, device="cuda", generator=g) for w in ("w0", "w1", "w2")]
+    gate = i["momentum"].float().contiguous()
+    steps = [(P.UPDATE, 0, n, 0), (P.APPLY, 0, n, 0)]
+    want = ops.scan(*[i[x] for x in NAMES], steps, momentum=gate, m_init=m, return_state=True, return_momentum=True)
+    cfg, io = L.ScanConfig(), L.ScanIO()
+    cfg.B, cfg.L, cfg.D, cfg.H, cfg.out_len, cfg.act_dtype, cfg.renorm, cfg.w_scale = B, n, D, H, n, L.LACT_BF16, L.RENORM_EPS_OUTSIDE, 1.0
+    cfg.use_momentum = 1
+    for x in ("q", "k", "v", "o"):
+        setattr(cfg, x + "_bs", n * D)
+        setattr(cfg, x + "_ts", D)
+    for x in NAMES:
+        setattr(io, x, i[x].data_ptr())
+    o = torch.empty(B, n, D, dtype=BF16, device="cuda")
+    io.o, io.momentum = o.data_ptr(), gate.data_ptr()
+    size = B * H * D * 4
+    packed = {x: torch.zeros(size + 16, dtype=torch.uint8, device="cuda") for x in ("m0_in", "m1_in", "m2_in", "w0_out", "w1_out", "w2_out",
+                                                                                   "m0_out", "m1_out", "m2_out")}
+    for x, t in zip(("m0_in", "m1_in", "m2_in"), m):
+        packed[x][offset:offset + size] = t.reshape(-1).view(torch.uint8)
+    for x, t in packed.items():
+        setattr(io, x, t.data_ptr() + offset)
+    kind, start, end, outs = ((t * 2)(*[s[j] for s in steps]) for j, t in enumerate((C.c_int32, C.c_int64, C.c_int64, C.c_int64)))
+    need = C.c_size_t(0)
+    L.check(L.lib().lact_scan_workspace_bytes(C.byref(cfg), 2, kind, start, end, C.byref(need)), "bytes")
+    ws = torch.empty(need.value, dtype=torch.uint8, device="cuda")
+    L.check(L.lib().lact_scan_fwd(C.byref(cfg), C.byref(io), 2, kind, start, end, outs, ws.data_ptr(), need, L.stream_ptr()), "scan")
+    torch.cuda.synchronize()
+    assert torch.equal(o, want[0])
+    for x, t in zip(("w0_out", "w1_out", "w2_out", "m0_out", "m1_out", "m2_out"), want[1:]):
+        assert torch.equal(packed[x][offset:offset + size].clone().view(torch.float32).view(t.shape), t), x
+
+
 @pytest.mark.parametrize("act", [BF16, torch.float32])
 @pytest.mark.parametrize("muon", [False, True])
 def test_nan_gate_of_the_first_chunk_reaches_the_weights(act, muon):
