@@ -137,12 +137,6 @@ struct CutArgs {
 constexpr int kCutEpiWarps = 16;
 constexpr int kCutThreads = 64 + 32 * kCutEpiWarps;
 
-// 1 / x of a normal x by the approximation and one Newton step (within an ulp; infinity gives 0)
-__device__ __forceinline__ float cut_reciprocal(float x) {
-  const float r = rcp_ftz(x), e = fmaf(-x, r, 1.0f);
-  return fabsf(e) < 1.0f ? fmaf(r, e, r) : r;
-}
-
 // columns of b per tile and plane
 template <int MODE, int BT>
 struct CutTile {
@@ -388,7 +382,7 @@ __global__ void __launch_bounds__(kCutThreads, 1) cut_gemm_kernel(const __grid_c
 #pragma unroll
         for (int j = 0; j < HC; ++j) {
           const float y0 = sum[j], y2 = sum[HC + j];
-          const float sg = cut_reciprocal(1.0f + expf(-y0)), sw = sg * y0;
+          const float sg = 1.0f / (1.0f + expf(-y0)), sw = sg * y0;
           sum[j] = sw * y2 * l1;
           if constexpr (MODE == kCutGrad) {
             sum[HC + j] = sg * y2 * dh[j] * (1.0f + y0 * (1.0f - sg)) * l0;

@@ -49,6 +49,20 @@ def test_close_to_64_bits(lb, b, n, d, h):
     assert (o - want).norm() <= 2e-6 * want.norm()
 
 
+def test_gate_far_below_zero(lb):
+    """The sigmoid is a plain division: 1 / (1 + e^88) is a subnormal number, not zero."""
+    b, n, d, h = 1, 40, 64, 64
+    w0, w1, w2, q, k, v, *lr = _inputs(b, n, d, h, seed=6)
+    w1 = w1.abs()
+    w0[:, :, 0], w2[:, :, 0] = 1.0, 1e22
+    q = torch.zeros_like(q)
+    q[0, :, 0] = -torch.linspace(80, 88.5, n, device="cuda")   # what the gate sees
+    o = lb.block_causal_lact_swiglu(w0, w1, w2, q, k, v, *lr, chunk_size=64, use_muon=False).double()
+    want = (F.silu(q.double() @ w0.double().mT) * (q.double() @ w2.double().mT)) @ w1.double().mT
+    # a subnormal sigmoid is a multiple of 2^-149 (and at least 2^-128); else an ulp or two of e^88
+    assert ((o - want).abs() <= (2e-6 + 2.0 ** -22) * want.abs()).all()
+
+
 def test_infinities_and_large_values(lb):
     """A token's infinity reaches its own outputs as an infinity, a NaN as a NaN, and no other token; values that bf16 rounds to
     infinity stay finite."""
