@@ -1,11 +1,16 @@
 // fp32 mode (fp32 activations) on the tensor cores.  tcgen05 multiplies no fp32 by fp32, so every operand is kept as three bf16
-// matrices ("pieces"), x = hi + mid + lo, each the rounding of what the ones before it leave (8 + 8 + 8 bits: nothing of a normal
-// value is lost), and six products stand for the one: hi hi, hi mid, mid hi, mid mid, hi lo, lo hi.  What is left out (mid lo,
-// lo mid, lo lo) is below 2^-26 of a term and of either sign.  Each product of two pieces is exact.  The tensor core adds 64 of
+// matrices ("pieces"), x = hi + mid + lo, each the rounding of what the ones before it leave (8 + 8 + 8 bits), and six products
+// stand for the one: hi hi, hi mid, mid hi, mid mid, hi lo, lo hi.  What is left out (mid lo, lo mid, lo lo) is below 2^-23 of a
+// term at worst, about 2^-27 in the mean, and of either sign.  Each product of two pieces is exact.  The tensor core adds 64 of
 // them (four steps of 16) to accumulators that start at zero, hi hi in one and the small five in another; the epilogue warps add
 // the accumulators of all 64-wide slabs of k to fp32 registers with rounding, so its truncating additions never see more than
 // four steps.  An infinity or NaN is its own hi with zeros behind it; where the hi hi sum is not finite it stands alone (infinity
-// times a zero piece would make a NaN of it).  Pieces below 2^-133 vanish: values under 2^-110 keep fewer bits.
+// times a zero piece would make a NaN of it).
+// A bf16 value is a multiple of 2^-133, a float of 2^-149: mid is kept times 2^7 and lo times 2^14, so that nothing is lost down to
+// 2^-124 and at most 2^-148 below (as they are, values under 2^-110 would keep fewer bits).  The products of one order carry one
+// factor: mid mid, hi lo and lo hi are added first, and hi mid, mid hi onto their sum divided by 2^7, which tcgen05.mma does on the
+// way.  With 7 the sum of the small products stays below 1.01 times the sum of the terms' magnitudes; with 8 it could be twice that,
+// and infinite where the result is not.  (Error of results near 1e-36, as pieces are / kept this way: 2e-5 to 6e-4 / 3e-7.)
 // Error against 64 bits of a whole call (update and apply, Muon off; relative 2-norm, FFMA contractions / these), x 1e-7:
 // 4 entries of 192, 4096 tokens 6.0 / 3.3; 4 of 192, 8192 7.3 / 3.6; 16 of 256, 2048 6.2 / 3.1; 8 of 128, 1000 4.3 / 3.0; 2 of
 // 64 x 128, 256 3.4 / 2.8; 2 of 256, 333 5.3 / 2.7.
@@ -24,8 +29,12 @@
 
 namespace lact {
 
+// The middle piece is kept times 2^kCutShift, the last one times 2^(2 kCutShift).
+constexpr int kCutShift = 7;
+
 // The three pieces of eight values, packed.  A finite value that would round to infinity is truncated instead.
 __device__ __forceinline__ void cut8(const float (&x)[8], uint32_t (&hi)[4], uint32_t (&mid)[4], uint32_t (&lo)[4]) {
+  constexpr float kUp = 1 << kCutShift;
   float r[8];
   uint32_t special = 0;
 #pragma unroll
@@ -56,8 +65,9 @@ __device__ __forceinline__ void cut8(const float (&x)[8], uint32_t (&hi)[4], uin
   }
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    mid[j] = pack_bf16x2(r[2 * j], r[2 * j + 1]);
-    lo[j] = pack_bf16x2(r[2 * j] - __uint_as_float(mid[j] << 16), r[2 * j + 1] - __uint_as_float(mid[j] & 0xFFFF0000u));
+    const float r0 = r[2 * j] * kUp, r1 = r[2 * j + 1] * kUp;
+    mid[j] = pack_bf16x2(r0, r1);
+    lo[j] = pack_bf16x2((r0 - __uint_as_float(mid[j] << 16)) * kUp, (r1 - __uint_as_float(mid[j] & 0xFFFF0000u)) * kUp);
   }
 }
 
@@ -271,18 +281,25 @@ __global__ void __launch_bounds__(kCutThreads, 1) cut_gemm_kernel(const __grid_c
         const uint32_t step_a = a_mn ? 128 : 2, step_b = b_mn ? 128 : 2, plane_b = second ? T::kPlaneB / 2 : T::kPlaneB;
         const uint32_t nb = second ? BT / 2 : BT;  // columns of this product
         const uint32_t one = make_idesc_bf16(kBM, nb, a_mn, b_mn), two = make_idesc_bf16(kBM, 2 * nb, a_mn, b_mn);
-        auto product = [&](int pa, int pb, uint32_t col, uint32_t idesc, bool first) {
+        // steps [from, 4) of piece pa of A times piece pb of B, onto what the columns hold or (fresh) in its place
+        auto product = [&](int pa, int pb, uint32_t col, uint32_t idesc, bool fresh, int from) {
           const uint32_t at = (st + pa * T::kPlaneA) >> 4, bt = (sb + pb * plane_b) >> 4;
 #pragma unroll
           for (int k4 = 0; k4 < 4; ++k4)
-            umma_bf16_if(leader, acc + col, desc.at(at + k4 * step_a), desc.at(bt + k4 * step_b), idesc, (k4 != 0 || !first) ? 1u : 0u);
+            if (k4 >= from)
+              umma_bf16_if(leader, acc + col, desc.at(at + k4 * step_a), desc.at(bt + k4 * step_b), idesc, (k4 != from || !fresh) ? 1u : 0u);
         };
-        // hi hi into columns [0, nb), the rest into [nb, 2 nb): B's hi and mid lie next to each other, one product for both
-        product(0, 0, 0, two, true);
-        product(1, 0, nb, one, false);
-        product(1, 1, nb, one, false);
-        product(0, 2, nb, one, false);
-        product(2, 0, nb, one, false);
+        // hi hi into columns [0, nb), the rest into [nb, 2 nb).  The rest: the three products of the order of mid mid, which are
+        // 2^(2 kCutShift) times too large; onto their sum, scaled down by 2^kCutShift, those of the order of hi mid.  B's hi and mid
+        // lie next to each other: from the second step on one product for hi hi and hi mid.
+        product(1, 1, nb, one, true, 0);
+        product(0, 2, nb, one, false, 0);
+        product(2, 0, nb, one, false, 0);
+        umma_bf16_onto_scaled_if<kCutShift>(leader, acc + nb, desc.at((st + T::kPlaneA) >> 4), desc.at(sb >> 4), one);
+        product(1, 0, nb, one, false, 1);
+        umma_bf16_if(leader, acc, desc.at(st >> 4), desc.at(sb >> 4), one, 0);
+        umma_bf16_if(leader, acc + nb, desc.at(st >> 4), desc.at((sb + plane_b) >> 4), one, 1);
+        product(0, 0, 0, two, false, 1);
         umma_commit_if(leader, &empty[s]);
         umma_commit_if(leader, &acc_full[buf]);
         if (++s == RING) { s = 0; ph ^= 1; }
@@ -324,7 +341,7 @@ __global__ void __launch_bounds__(kCutThreads, 1) cut_gemm_kernel(const __grid_c
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           const float v = __uint_as_float(big[j]);
-          x[j] += fabsf(v) <= 3.402823466e38f ? v + __uint_as_float(small[j]) : v;
+          x[j] += fabsf(v) <= 3.402823466e38f ? fmaf(__uint_as_float(small[j]), 1.f / (1 << kCutShift), v) : v;
         }
       };
       const int passes = MODE == kCutGrad ? 2 : 1;

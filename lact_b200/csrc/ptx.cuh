@@ -336,6 +336,17 @@ __device__ __forceinline__ void umma_bf16_if(uint32_t leader, uint32_t tmem_d, u
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(leader)
       : "memory");
 }
+// The same, D = A * B + D / 2^SHIFT (SHIFT of 1 to 15).
+template <int SHIFT>
+__device__ __forceinline__ void umma_bf16_onto_scaled_if(uint32_t leader, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.eq.b32 p, 0, 0;\n\t"
+      "setp.ne.b32 q, %4, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p, %5;\n\t}"
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(leader), "n"(SHIFT)
+      : "memory");
+}
 // The same with A in tensor memory: a row per lane, two bf16 values of consecutive k per column.
 __device__ __forceinline__ void umma_bf16_ta_if(uint32_t leader, uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
                                                 uint32_t accumulate) {

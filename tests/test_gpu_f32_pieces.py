@@ -24,14 +24,17 @@ def _inputs(b, n, d, h, seed=0):
         [F.softplus(rn(b, n, 1) - 2) for _ in range(3)]
 
 
+def _gradients(w0, w1, w2, q, k, v, l0, l1, l2):
+    y0, y2, dh = k @ w0.mT, k @ w2.mT, v @ w1
+    s = torch.sigmoid(y0)
+    return [(dh * y2 * s * (1 + y0 * (1 - s)) * l0).mT @ k, (v * l1).mT @ (y0 * s * y2), (dh * y0 * s * l2).mT @ k]
+
+
 def _exact(w0, w1, w2, q, k, v, l0, l1, l2):
     """One update on all tokens, then apply, in 64 bits."""
     w0, w1, w2, q, k, v, l0, l1, l2 = (t.double() for t in (w0, w1, w2, q, k, v, l0, l1, l2))
-    y0, y2, dh = k @ w0.mT, k @ w2.mT, v @ w1
-    s = torch.sigmoid(y0)
-    g = [(dh * y2 * s * (1 + y0 * (1 - s)) * l0).mT @ k, (v * l1).mT @ (y0 * s * y2), (dh * y0 * s * l2).mT @ k]
     u = []
-    for w, dw in zip((w0, w1, w2), g):
+    for w, dw in zip((w0, w1, w2), _gradients(w0, w1, w2, q, k, v, l0, l1, l2)):
         x = w + dw
         u.append(x / (x.norm(dim=2, keepdim=True) + 1e-5) * w.norm(dim=2, keepdim=True))
     return (F.silu(q @ u[0].mT) * (q @ u[2].mT)) @ u[1].mT
@@ -47,6 +50,32 @@ def test_close_to_64_bits(lb, b, n, d, h):
     want = _exact(*args)
     # fp32 throughout: a few roundings of sums of up to d and 64 terms, 2^-24 each
     assert (o - want).norm() <= 2e-6 * want.norm()
+
+
+@pytest.mark.parametrize("power", [-59, -56, -53, -40, 20])
+def test_small_queries(lb, power):
+    """Gate and hidden activations near the smallest normal number keep their bits (hidden = about q^2)."""
+    b, n, d, h = 2, 200, 64, 136
+    w0, w1, w2, q, k, v, *lr = _inputs(b, n, d, h, seed=7)
+    q = q * 2.0 ** power
+    o = lb.block_causal_lact_swiglu(w0, w1, w2, q, k, v, *lr, chunk_size=256, use_muon=False).double()
+    want = (F.silu(q.double() @ w0.double().mT) * (q.double() @ w2.double().mT)) @ w1.double().mT
+    assert (o - want).norm() <= 2e-6 * want.norm()
+
+
+# (what, times a power of two): the gradients of the weights, read as the momentum that starts at zero
+@pytest.mark.parametrize("what,power", [("v", -116), ("v", -109), ("v", 118), ("lr", -116), ("lr", -109), ("k", -55), ("k", -50)])
+def test_small_and_large_gradients(lb, what, power):
+    b, n, d, h = 2, 200, 72, 128
+    a = _inputs(b, n, d, h, seed=8)
+    for i in {"k": (4,), "v": (5,), "lr": (6, 7, 8)}[what]:
+        a[i] = a[i] * 2.0 ** power
+    zeros = [torch.zeros_like(w) for w in a[:3]]
+    r = lb.ar_fast_weight_swish_glu_weight_norm_mini_batch_inference_with_momentum(
+        *a, 1.0, mini_batch_size=n, do_update=True, use_moun=False, fw_momentum=torch.ones(b, n, 1, device="cuda"),
+        dw0_momentum=zeros[0], dw1_momentum=zeros[1], dw2_momentum=zeros[2], use_momentum=True)
+    for got, want in zip(r[4:7], _gradients(*(t.double() for t in a))):
+        assert (got.double() - want).norm() <= 2e-6 * want.norm()
 
 
 def test_gate_far_below_zero(lb):
