@@ -94,8 +94,7 @@ struct OperandForm {
   bool segments;
 };
 template <class Op>
-constexpr OperandForm form_of(const GemmProblem<Op>&) { 
-  static_assert(Op::KB == 1, "operand boxes are one k-block deep");
+constexpr OperandForm form_of(const GemmProblem<Op>&) {
   return OperandForm{op_segments<Op>::value};
 }
 
@@ -366,14 +365,15 @@ int choose_bt(std::initializer_list<NW> probs) {
 // 25 (12 of 128 x 256) 19 -> 23.  Where the tiles fill the chip anyway the partial sums cost what they are: nothing at 64
 // entries of 192 (204 us either way), 345 -> 378 at 128 of them, 255 -> 288 at 96 of 128 x 256; entries of 384 gain alone
 // (49 -> 33 at 128 k-blocks) and in fours (60 -> 58), and lose in eights (70 -> 82) and beyond (32: 219 -> 256; 64 at 96
-// k-blocks: 365 -> 485).
+// k-blocks: 365 -> 485).  (A unit's k-blocks are rounded up to an even number: where the cuts lie decides an entry's bits, and they
+// stay where they have been.)
 struct Split {
   int splits, kb_per_split;
 };
 Split choose_split(int64_t num_kb) {
   if (num_kb < 96) return Split{1, static_cast<int>(num_kb)};
   const int64_t want = num_kb < 192 ? 3 : 5;
-  const int64_t per = ((num_kb + want - 1) / want + 1) & ~1ll;  // whole ring stages of two k-blocks
+  const int64_t per = ((num_kb + want - 1) / want + 1) & ~1ll;
   return Split{static_cast<int>((num_kb + per - 1) / per), static_cast<int>(per)};
 }
 inline int64_t output_tiles(int64_t M, int64_t N, int64_t batch, int bt) {

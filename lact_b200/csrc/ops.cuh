@@ -180,8 +180,7 @@ struct OpBmm {
   static constexpr bool kTileReduce = false;
   static constexpr bool kWarpTranspose = true, kReverseBatch = false;
   static constexpr uint32_t kEpiScratch = EpiT::kScratch;
-  static constexpr int KB = 1;  // measured: two-k-block stages slow the training backward's products by 7 %
-  static constexpr int STAGES = ring_depth(KB * (kATileBytes + BT_ * kBK * 2), kEpiScratch);
+  static constexpr int STAGES = ring_depth(kATileBytes + BT_ * kBK * 2, kEpiScratch);
   using Epi = EpiT;
   __host__ __device__ static constexpr int term_a(int) { return 0; }
   __host__ __device__ static constexpr int term_b(int) { return 0; }
@@ -207,11 +206,7 @@ struct OpDW {
   static constexpr bool kWarpTranspose = true;                   // results reach global memory through `EpiDW::warp_block`
   static constexpr bool kReverseBatch = true;                    // reads the planes the pointwise kernel has just written
   static constexpr uint32_t kEpiScratch = kEpiWarps * 32 * 144;  // one 32 x 32 fp32 block (rows padded to 144 bytes) per epilogue warp
-  // One k-block per stage: since box coordinates are worked out once per tile, a box costs the loading warp little, and a
-  // ring of four or five small stages refills sooner than one of two large ones (72 tiles of 25 k-blocks 19.4 -> 17.3 us, a call
-  // with 21 of them 1677 -> 1626; 16 entries of 192 and 49152 tokens 815 -> 766 the whole call, 32 of 384 even).
-  static constexpr int KB = 1;
-  static constexpr int STAGES = ring_depth(KB * (kATileBytes + BT_ * kBK * 2), kEpiScratch);
+  static constexpr int STAGES = ring_depth(kATileBytes + BT_ * kBK * 2, kEpiScratch);
   using Epi = EpiDW;
   __host__ __device__ static constexpr int term_a(int) { return 0; }
   __host__ __device__ static constexpr int term_b(int) { return 0; }
@@ -247,8 +242,7 @@ struct OpBmmStore {
   static constexpr bool kTileReduce = false;
   static constexpr bool kWarpTranspose = false, kReverseBatch = true;
   static constexpr uint32_t kEpiScratch = 0;
-  static constexpr int KB = 1;  // measured: two-k-block stages are 5 % slower for this op (K-major operands, short K)
-  static constexpr int STAGES = ring_depth(KB * (kATileBytes + BT_ * kBK * 2), kBM * BT_ * 2);
+  static constexpr int STAGES = ring_depth(kATileBytes + BT_ * kBK * 2, kBM * BT_ * 2);
   using Epi = EpiNone;
   __host__ __device__ static constexpr int term_a(int) { return 0; }
   __host__ __device__ static constexpr int term_b(int) { return 0; }
@@ -272,8 +266,7 @@ struct OpBmm2 {
   static constexpr bool kTileReduce = false;
   static constexpr bool kWarpTranspose = true, kReverseBatch = false;
   static constexpr uint32_t kEpiScratch = EpiT::kScratch;
-  static constexpr int KB = 1;
-  static constexpr int STAGES = ring_depth(KB * (2 * kATileBytes + 2 * BT_ * kBK * 2), kEpiScratch);
+  static constexpr int STAGES = ring_depth(2 * kATileBytes + 2 * BT_ * kBK * 2, kEpiScratch);
   using Epi = EpiT;
   __host__ __device__ static constexpr int term_a(int t) { return t; }
   __host__ __device__ static constexpr int term_b(int t) { return t; }
@@ -308,7 +301,6 @@ struct OpNsT {
   static constexpr bool kWarpTranspose = false, kReverseBatch = false;
   static constexpr bool kSymmetric = SYM_;
   static constexpr uint32_t kEpiScratch = 0;
-  static constexpr int KB = 1;
   static constexpr int STAGES = ring_depth(kATileBytes + BT_ * kBK * 2, kBM * BT_ * 2);  // (one launch per product)
   using Epi = EpiNs;
   __host__ __device__ static constexpr int diag_a(int) { return 0; }  // S = X X^T, P ~ S S: one matrix on both sides
@@ -354,7 +346,6 @@ struct OpNs2T {
   static constexpr bool kWarpTranspose = false, kReverseBatch = false;
   static constexpr bool kSymmetric = SYM_;
   static constexpr uint32_t kEpiScratch = 0;
-  static constexpr int KB = 1;
   static constexpr int STAGES = ring_depth(2 * (kATileBytes + BT_ * kBK * 2), kBM * BT_ * 2);
   using Epi = EpiNs;
   __host__ __device__ static constexpr int diag_a(int b) { return 1 - b; }  // U V^T + V U^T: a0 = b1 = U, a1 = b0 = V
@@ -385,12 +376,11 @@ using OpNs2 = OpNs2T<BT_, false>;
 template <int BT_>
 struct OpSwigluGate {
   static constexpr bool kSegments = true;
-  static constexpr int KB = 1;  // measured: two-k-block stages (a 2-deep ring here) are 7 % slower for this op
   static constexpr int NA = 1, NB = 2, NACC = 2, BT = BT_, NTERMS = 1, NOUT = 1;
   static constexpr bool kTileReduce = false;
   static constexpr bool kWarpTranspose = false, kReverseBatch = false;
   static constexpr uint32_t kEpiScratch = 0;
-  static constexpr int STAGES = ring_depth(KB * (kATileBytes + 2 * BT_ * kBK * 2), kBM * BT_ * 2);
+  static constexpr int STAGES = ring_depth(kATileBytes + 2 * BT_ * kBK * 2, kBM * BT_ * 2);
   using Epi = EpiNone;
   __host__ __device__ static constexpr int term_a(int) { return 0; }
   __host__ __device__ static constexpr int term_b(int t) { return t; }
@@ -418,8 +408,7 @@ struct OpFwGradPointwise {
   static constexpr bool kTileReduce = false;
   static constexpr bool kWarpTranspose = false, kReverseBatch = false;
   static constexpr uint32_t kEpiScratch = 0;
-  static constexpr int KB = 1;  // two k-blocks of this op's five tiles would leave a one-stage ring
-  static constexpr int STAGES = ring_depth(KB * (2 * kATileBytes + 3 * 64 * kBK * 2), 3 * kBM * 64 * 2);
+  static constexpr int STAGES = ring_depth(2 * kATileBytes + 3 * 64 * kBK * 2, 3 * kBM * 64 * 2);
   using Epi = EpiFwGrad;
   __host__ __device__ static constexpr int term_a(int t) { return t; }
   __host__ __device__ static constexpr int term_b(int t) { return t == 0 ? 0 : 2; }

@@ -80,7 +80,7 @@ template <class Op>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreadsV2, 1)
 pair_gemm_kernel(const __grid_constant__ GemmArgs<Op, 1> args, const int ring) {
   using Wire = typename PairWiring<Op>::type;
-  static_assert(Op::KB == 1 && Op::NOUT > 0 && Op::NTERMS <= 2, "staged single-k-block ops");
+  static_assert(Op::NOUT > 0 && Op::NTERMS <= 2, "staged ops");
   constexpr int BT = Op::BT, NACC = Op::NACC, NOUT = Op::NOUT, PANELS = pair_panels<Op>();
   constexpr uint32_t kAccCols = NACC * BT;
   constexpr uint32_t kTmemCols = tmem_cols_pow2(2 * kAccCols);

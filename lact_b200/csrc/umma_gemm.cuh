@@ -80,7 +80,7 @@ __host__ __device__ constexpr uint32_t tmem_cols_pow2(uint32_t n) {
 // of tile i overlaps the main loop of tile i + 1.
 template <class Op>
 __host__ __device__ constexpr uint32_t gemm_stage_bytes() {
-  return Op::KB * (Op::NA * kATileBytes + Op::NB * Op::BT * kBK * 2);
+  return Op::NA * kATileBytes + Op::NB * Op::BT * kBK * 2;
 }
 // bf16 staging tiles for TMA-stored outputs: NOUT x [128 rows][BT columns], 128-byte swizzled in
 // 64-column panels (the layout the output tensor maps expect)
@@ -104,18 +104,20 @@ __host__ __device__ constexpr int flow_ring(uint32_t stride) {
              : static_cast<int>((232448u - 1024u - 256u - kFlowScratch) / stride);
 }
 
-// One operand tile of a ring stage: ROWS (mn) x KB k-blocks.  Shared-memory layout:
-//   K-major:  [k-block][ROWS rows][64 k] (KB tiles of ROWS x 128 bytes back to back);
-//   MN-major: per 64-wide mn atom [KB * 64 k rows][64 mn] (atoms KB * 8 KB apart).
+// One operand tile of a ring stage: ROWS (mn) x one k-block.  Shared-memory layout:
+//   K-major:  [ROWS rows][64 k];
+//   MN-major: per 64-wide mn atom [64 k rows][64 mn] (atoms 8 KB apart).
+// (A ring of four or five small stages refills sooner than one of two stages of two k-blocks: 72 tiles of the token contraction, 25
+// k-blocks each, 19.4 -> 17.3 us.)
 // The cursor holds the coordinates of an operand's next boxes: they are worked out once per output tile, so that between two
 // stages the issuing warp only adds.  (What that warp spends per box is what the loads can reach: see gemm_phase.)
 // SEG: the maps are 4-D (inner, row, entry, segment), see op_segments.
-template <int ROWS, int KB, bool SEG>
+template <int ROWS, bool SEG>
 struct OperandCursor {
   const CUtensorMap* map;
-  int32_t inner, row, batch, segment;  // first box of the stage; 4-D maps: inner = k-block, row = mn
+  int32_t inner, row, batch, segment;  // first box of the stage
   int32_t d_inner, d_row;     // advance per stage
-  int32_t mn_major;           // 0: K-major, a box per k-block; 1: MN-major, a box per atom
+  int32_t mn_major;           // 0: K-major, one box; 1: MN-major, a box per atom
   __device__ __forceinline__ void start(const CUtensorMap* m, const OperandInfo& oi, int mn0, int kc, int b, int seg) {
     map = m;
     batch = oi.batch_off + b;
@@ -123,10 +125,10 @@ struct OperandCursor {
     mn_major = oi.mn_major;
     if (mn_major) {
       inner = oi.mn_off + mn0; row = oi.k_off + kc;
-      d_inner = 0; d_row = KB * kBK;
+      d_inner = 0; d_row = kBK;
     } else {
       inner = oi.k_off + kc; row = oi.mn_off + mn0;
-      d_inner = KB * kBK; d_row = 0;
+      d_inner = kBK; d_row = 0;
     }
   }
   __device__ __forceinline__ void box(uint32_t leader, uint32_t dst, uint32_t bar, int at) const {
@@ -135,11 +137,10 @@ struct OperandCursor {
   }
   __device__ __forceinline__ void load(uint32_t leader, uint32_t dst, uint32_t bar) {
     if (!mn_major) {
-#pragma unroll
-      for (int kk = 0; kk < KB; ++kk) box(leader, dst + kk * (ROWS * kBK * 2), bar, inner + kk * kBK);
+      box(leader, dst, bar, inner);
     } else {
 #pragma unroll
-      for (int j = 0; j < ROWS / 64; ++j) box(leader, dst + j * (KB * kAtomBytes), bar, inner + 64 * j);
+      for (int j = 0; j < ROWS / 64; ++j) box(leader, dst + j * kAtomBytes, bar, inner + 64 * j);
     }
     inner += d_inner;
     row += d_row;
@@ -297,7 +298,7 @@ __device__ __forceinline__ int snake_tile(int round, int grid, int cta) {
 template <class Op, int RING, class EpiPatch, class Deps = NoDeps>
 __device__ __forceinline__ bool gemm_phase(GemmCtx& cx, const GemmProblem<Op>* probs, const int nprob,
                                            EpiPatch patch, Deps deps = Deps{}) {
-  constexpr int BT = Op::BT, NA = Op::NA, NB = Op::NB, NACC = Op::NACC, KB = Op::KB;
+  constexpr int BT = Op::BT, NA = Op::NA, NB = Op::NB, NACC = Op::NACC;
   constexpr uint32_t kBTileBytes = BT * kBK * 2;  // one k-block of a B tile
   constexpr uint32_t kStageBytes = gemm_stage_bytes<Op>();
   constexpr uint32_t kAccCols = NACC * BT;
@@ -401,31 +402,30 @@ __device__ __forceinline__ bool gemm_phase(GemmCtx& cx, const GemmProblem<Op>* p
         const GemmProblem<Op>& P = probs[tc.prob];
         int kb0, kb1;
         k_range(P, tc, kb0, kb1);
-        const int num_sb = (kb1 - kb0 + KB - 1) / KB;  // ring stages of KB k-blocks
         const bool diagonal = SYM && tc.m0 == tc.n0;
-        OperandCursor<kBM, KB, SEG> ca[NA];
-        OperandCursor<BT, KB, SEG> cb[NB];
+        OperandCursor<kBM, SEG> ca[NA];
+        OperandCursor<BT, SEG> cb[NB];
         int entry, segment;
         entry_of(P, tc.batch, entry, segment);
 #pragma unroll
         for (int i = 0; i < NA; ++i) ca[i].start(&P.a[i], P.ai[i], tc.m0, kb0 * kBK, entry, segment);
 #pragma unroll
         for (int i = 0; i < NB; ++i) cb[i].start(&P.b[i], P.bi[i], tc.n0, kb0 * kBK, entry, segment);
-        const uint32_t bytes = diagonal ? KB * NA * kATileBytes : kStageBytes;
+        const uint32_t bytes = diagonal ? NA * kATileBytes : kStageBytes;
         if constexpr (Deps::kOn) {
           if (!__all_sync(0xFFFFFFFFu, flow_wait_verified(cx, cx.ptile++))) { failed = true; break; }  // the scout warp checked this tile
           asm volatile("fence.proxy.async.global;" ::: "memory");
         }
-        for (int sb = 0; sb < num_sb; ++sb) {
+        for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait_warp(&cx.empty_bar[cx.slot], cx.phase ^ 1, cx.abort_flag)) { failed = true; break; }
           const uint32_t bar = smem_u32(&cx.full_bar[cx.slot]);
           mbar_expect_tx_if(leader, bar, bytes);
           const uint32_t st = cx.smem_base + cx.slot * cx.stage_stride;
 #pragma unroll
-          for (int i = 0; i < NA; ++i) ca[i].load(leader, st + i * (KB * kATileBytes), bar);
+          for (int i = 0; i < NA; ++i) ca[i].load(leader, st + i * kATileBytes, bar);
           if (!diagonal) {
 #pragma unroll
-            for (int i = 0; i < NB; ++i) cb[i].load(leader, st + NA * (KB * kATileBytes) + i * (KB * kBTileBytes), bar);
+            for (int i = 0; i < NB; ++i) cb[i].load(leader, st + NA * kATileBytes + i * kBTileBytes, bar);
           }
           cx.next_stage<RING>();
         }
@@ -447,43 +447,36 @@ __device__ __forceinline__ bool gemm_phase(GemmCtx& cx, const GemmProblem<Op>* p
         if (!mbar_wait_warp(&cx.acc_empty_bar[as], aph ^ 1, cx.abort_flag)) { failed = true; break; }
         tc_fence_after();
         const uint32_t acc_base = cx.tmem_base + as * kAccStride;
-        const int num_sb = (num_kb + KB - 1) / KB;
         const bool diagonal = SYM && tc.m0 == tc.n0;
-        // K-major tiles: 16 elements = 32 bytes on inside the swizzled 128-byte row, k-blocks a tile apart; MN-major tiles:
-        // 16 k-rows of 128 bytes on, k-blocks 64 rows apart, 64-wide atoms KB * 8 KB apart (the leading offset)
-        uint32_t idesc[Op::NTERMS], step_a[Op::NTERMS], step_b[Op::NTERMS], blk_a[Op::NTERMS], blk_b[Op::NTERMS];
+        // K-major tiles: 16 elements = 32 bytes on inside the swizzled 128-byte row; MN-major tiles: 16 k-rows of 128 bytes on, 64-wide
+        // atoms 8 KB apart (the leading offset)
+        uint32_t idesc[Op::NTERMS], step_a[Op::NTERMS], step_b[Op::NTERMS];
 #pragma unroll
         for (int t = 0; t < Op::NTERMS; ++t) {
           const int a_mn = P.ai[Op::term_a(t)].mn_major, b_mn = P.bi[Op::term_b(t)].mn_major;
           idesc[t] = make_idesc_bf16(kBM, Op::term_n(t), a_mn, b_mn);
           step_a[t] = a_mn ? 128 : 2;
           step_b[t] = b_mn ? 128 : 2;
-          blk_a[t] = (a_mn ? kAtomBytes : kATileBytes) >> 4;
-          blk_b[t] = (b_mn ? kAtomBytes : kBTileBytes) >> 4;
         }
-        const SmemDescBase desc(KB * kAtomBytes);  // (K-major descriptors ignore the leading offset)
-        for (int sb = 0; sb < num_sb; ++sb) {
+        const SmemDescBase desc(kAtomBytes);  // (K-major descriptors ignore the leading offset)
+        for (int kb = 0; kb < num_kb; ++kb) {
           const uint32_t s = cx.slot;
           if (!mbar_wait_warp(&cx.full_bar[s], cx.phase, cx.abort_flag)) { failed = true; break; }
           tc_fence_after();
           const uint32_t st = (cx.smem_base + s * cx.stage_stride) >> 4;
 #pragma unroll
-          for (int kk = 0; kk < KB; ++kk) {
-            if (sb * KB + kk >= num_kb) break;  // a trailing half-empty stage
+          for (int t = 0; t < Op::NTERMS; ++t) {
+            const uint32_t a_tile = st + Op::term_a(t) * (kATileBytes >> 4);
+            uint32_t b_off = NA * kATileBytes + Op::term_b(t) * kBTileBytes;
+            if constexpr (SYM) {
+              if (diagonal) b_off = Op::diag_a(Op::term_b(t)) * kATileBytes;
+            }
+            const uint32_t b_tile = st + (b_off >> 4);
 #pragma unroll
-            for (int t = 0; t < Op::NTERMS; ++t) {
-              const uint32_t a_tile = st + Op::term_a(t) * (KB * kATileBytes >> 4) + kk * blk_a[t];
-              uint32_t b_off = NA * (KB * kATileBytes) + Op::term_b(t) * (KB * kBTileBytes);
-              if constexpr (SYM) {
-                if (diagonal) b_off = Op::diag_a(Op::term_b(t)) * (KB * kATileBytes);
-              }
-              const uint32_t b_tile = st + (b_off >> 4) + kk * blk_b[t];
-#pragma unroll
-              for (int k4 = 0; k4 < kBK / kUmmaK; ++k4) {
-                const uint32_t acc = (sb > 0 || kk > 0 || k4 > 0 || !Op::term_first(t)) ? 1u : 0u;
-                umma_bf16_if(leader, acc_base + Op::term_col(t), desc.at(a_tile + k4 * step_a[t]), desc.at(b_tile + k4 * step_b[t]),
-                             idesc[t], acc);
-              }
+            for (int k4 = 0; k4 < kBK / kUmmaK; ++k4) {
+              const uint32_t acc = (kb > 0 || k4 > 0 || !Op::term_first(t)) ? 1u : 0u;
+              umma_bf16_if(leader, acc_base + Op::term_col(t), desc.at(a_tile + k4 * step_a[t]), desc.at(b_tile + k4 * step_b[t]),
+                           idesc[t], acc);
             }
           }
           umma_commit_if(leader, &cx.empty_bar[s]);  // frees the stage once these MMAs have read it
