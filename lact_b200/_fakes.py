@@ -1,4 +1,4 @@
-"""Shape-only implementations of the registered operators (tracing, `torch.compile`); imported once the operator library
+"""Shape-only implementations of the registered operators (tracing, `torch.compile`); registered once the operator library
 has been loaded (`_lib.load_ops`)."""
 from __future__ import annotations
 
@@ -12,8 +12,24 @@ from . import program as P
 BF16, F32 = torch.bfloat16, torch.float32
 
 
+_FAKES = {}   # every operator that this package calls
+
+
 def _fake(name):
-    return torch.library.register_fake("lact_b200::" + name)
+    def keep(fn):
+        _FAKES[name] = fn
+        return fn
+    return keep
+
+
+def register() -> None:
+    """Raises ImportError, before it registers anything, if the loaded library lacks one of the operators."""
+    missing = [name for name in _FAKES if not hasattr(torch.ops.lact_b200, name)]
+    if missing:
+        raise ImportError(f"{L.OPS_PATH} is older than this package (it has no {', '.join(missing)}): rebuild it with "
+                          "`python -m lact_b200.build`")
+    for name, fn in _FAKES.items():
+        torch.library.register_fake("lact_b200::" + name, fn)
 
 
 def ns_trace_bytes(B, Ltok, D, H, cfg) -> int:

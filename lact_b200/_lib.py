@@ -172,8 +172,8 @@ def load_ops() -> None:
         raise ImportError(f"{OPS_PATH} was built for another PyTorch than {torch.__version__}: rebuild it with "
                           "`python -m lact_b200.build`")
     torch.ops.load_library(OPS_PATH)
-    if not hasattr(torch.ops.lact_b200, "swa_fwd_cache"):   # the operator that was added last
-        raise ImportError(f"{OPS_PATH} is older than this package: rebuild it with `python -m lact_b200.build`")
+    from . import _fakes
+    _fakes.register()
     _ops_lib = C.CDLL(OPS_PATH)
     _ops_lib.lact_torch_take_status.argtypes = [C.c_int]
     _ops_lib.lact_torch_take_status.restype = C.c_int
@@ -182,7 +182,6 @@ def load_ops() -> None:
     _ops_lib.lact_torch_set_error_type.argtypes = [C.py_object]
     _ops_lib.lact_torch_set_error_type.restype = None
     _ops_lib.lact_torch_set_error_type(LactError)   # what a device status or a CUDA error is raised as
-    from . import _fakes  # noqa: F401
     _ops_loaded = True
 
 

@@ -28,6 +28,27 @@ def test_library_of_another_torch_is_stale_and_refused(tmp_path):
     assert r.returncode == 0, r.stdout + r.stderr
 
 
+MISSING = """
+import lact_b200
+from lact_b200 import _fakes, _lib
+_lib._ops_loaded = False
+_fakes._fake("added_later")(lambda x: x)
+for _ in range(2):
+    try:
+        _lib.load_ops()
+    except ImportError as e:
+        assert "older than this package" in str(e) and "added_later" in str(e), e
+    else:
+        raise SystemExit("loaded")
+"""
+
+
+def test_library_without_an_operator_is_refused():
+    build.build()
+    r = subprocess.run([sys.executable, "-c", MISSING], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
 def test_build_compiles_again_for_another_torch(monkeypatch):
     built = []
     monkeypatch.setattr(build, "build_torch", lambda verbose=False: built.append(1))
