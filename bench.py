@@ -41,7 +41,7 @@ MIN_TRAFFIC_BYTES_FWD = 3.29e9  # q, k, v, o in bf16 + lr, momentum + fast weigh
 
 
 def dram_traffic_table():
-    """Per kernel class: (units in the capture, DRAM bytes read, DRAM bytes written) per launch, from the
+    """Per kernel class: (units in the capture, DRAM bytes read, DRAM bytes written) per launch and chunk, from the
     ncu table committed under profiles/ (rows `| class | units | read | write |`)."""
     table = {}
     if not os.path.exists(TRAFFIC_TABLE):
@@ -70,7 +70,7 @@ def algorithmic_flops(B, L, D, H, C, ns_steps):
 
 
 def class_flops(name, B, D, H, C, ns_steps):
-    """Algorithmic FLOPs of ONE launch of a kernel class at the benchmark shape."""
+    """Algorithmic FLOPs of ONE chunk's launch of a kernel class at the benchmark shape."""
     m1, n1 = min(D, H), max(D, H)
     m2, n2 = min(2 * H, D), max(2 * H, D)
     return {
@@ -639,19 +639,22 @@ def main():
     total_prof = sum(v[0] for v in prof.values())
     top = max((k for k in prof if class_flops(k, B, D, H, C, CFG["ns_steps"])), key=lambda k: prof[k][0])
     top_ms = prof[top][0] / prof[top][1]
-    achieved = class_flops(top, B, D, H, C, CFG["ns_steps"]) / (top_ms * 1e-3) / 1e12
+    # (a launch of the apply's two kernels serves one chunk or, as a run of apply steps, several)
+    n_chunks = len(range(0, L, C))
+    chunks = {k: n_chunks * prof_steps / v[1] if k in ("gemm_swiglu_gate", "gemm_down_proj") else 1 for k, v in prof.items()}
+    achieved = chunks[top] * class_flops(top, B, D, H, C, CFG["ns_steps"]) / (top_ms * 1e-3) / 1e12
     flops = algorithmic_flops(B, L, D, H, C, CFG["ns_steps"])
     step_tflops = flops / (ms_per_step * 1e-3) / 1e12
     # DRAM traffic per launch from the committed ncu table (captured on a smaller case; every class's traffic
     # grows in proportion to the units per launch), and the forward's total against its algorithmic minimum
     table = dram_traffic_table()
-    traffic_of = lambda k: (table[k][1] + table[k][2]) * B / table[k][0] if k in table else None
+    traffic_of = lambda k: chunks[k] * (table[k][1] + table[k][2]) * B / table[k][0] if k in table else None
     classes = {}
     fwd_traffic = 0.0
     for k, v in sorted(prof.items()):
         f = class_flops(k, B, D, H, C, CFG["ns_steps"])
         classes[k] = {"ms_per_launch": v[0] / v[1], "launches_per_step": v[1] / prof_steps, "share": v[0] / total_prof,
-                      "tflops": f / (v[0] / v[1] * 1e-3) / 1e12 if f else None, "dram_bytes_per_launch": traffic_of(k)}
+                      "tflops": chunks[k] * f / (v[0] / v[1] * 1e-3) / 1e12 if f else None, "dram_bytes_per_launch": traffic_of(k)}
         if traffic_of(k) is not None:
             fwd_traffic += traffic_of(k) * v[1] / prof_steps
     roofline = {"bound": "tensor", "kernel": top, "achieved": achieved, "peak": peaks["bf16_sustained"],
