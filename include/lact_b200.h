@@ -98,8 +98,10 @@ typedef struct lact_scan_io {
 /* Library version (major * 1000 + minor).  1001: lact_fw_grad_bwd_pointwise takes entries, tokens and the batch strides of
  * lr* and g_lr* in place of a row count; lact_momentum_bwd reads dg0 / dg1 and no longer adds the carry to them; lact_scan_io
  * ends with shadow_dump.  A caller compiled against 1000 that uses one of these must be compiled again.  1002: new entries
- * lact_swiglu_ffn_hidden_bytes, lact_swa_fwd_cache_bytes and lact_swa_fwd_cache; workspaces of programs with many short
- * steps are larger (they are asked for as before).  No counterpart in the reference. */
+ * lact_swiglu_ffn_hidden_bytes, lact_swa_fwd_cache_bytes and lact_swa_fwd_cache; larger workspaces (asked for as before):
+ * programs of many short steps by up to 128 MB for weights and 58 MB for hidden activations, fp32 programs by their
+ * operands in bf16 pieces (6 bytes a value: an update and apply of D = H take 30 H bytes per token, 12 H before).  No
+ * counterpart in the reference. */
 int lact_version(void);
 
 /* Human-readable text for a return code.  No counterpart in the reference. */

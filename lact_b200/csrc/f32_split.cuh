@@ -22,8 +22,9 @@
 // One persistent CTA per SM: warp 0 loads (TMA; the pieces of one matrix are entries `piece * batch + entry` of one map), warp 1
 // issues, sixteen warps drain and finish.  Accumulators of a slab are double-buffered.  A slab of 128 x 128 is 1536 clocks of
 // products and 96 KB of operands at 64 bytes a clock; what is left above that is the finish of short sums (a gradient-plane tile
-// of three slabs twice).  4 entries of 192, 4096 tokens, us per launch, FFMA / these: gradient planes 138 / 50, gate 83 / 25, token
-// contractions 2 x 48 / 38, down 48 / 17, the cuts - / 18; the call with Muon 431 / 192.
+// of three slabs twice; 18 warps leave 96 registers a thread: the gradient planes spill 78 bytes, 128-wide plain products 40).  4
+// entries of 192, 4096 tokens, us per launch, FFMA / these: gradient planes 138 / 51, gate 83 / 27, token contractions 2 x 48 / 36, down
+// 48 / 17, the cuts - / 18; the call with Muon 434 / 192.
 #pragma once
 #include "f32_gemm.cuh"
 

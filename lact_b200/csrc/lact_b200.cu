@@ -227,9 +227,9 @@ cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t s
   // Measured (10 forward steps of the benchmark shape, same GPU, back to back): 8.16 -> 8.05 ms at 32 (batch x head)
   // units, 3.58 -> 3.39 ms at 8 units, 2.94 -> 2.74 ms at 4 units: the fewer units, the larger the share of the
   // launch gaps that the overlap hides.
-  // The layer's row passes gain 4 % (302 -> 290 us for ten launches), the attention forward and a program's first
-  // kernels 1 to 3 us a call.  The row kernels and attention kernels of the backwards stay plain launches: a training
-  // step of 32 entries took 2.5 % longer with them, 8 entries of 192 718 -> 729 us.
+  // The layer's row passes, forward and backward, gain 4 % (302 -> 290 us for ten launches), the attention forward and
+  // a program's first kernels 1 to 3 us a call.  Plain launches are the row kernels of the recurrence's reverse sweep and
+  // the attention backward: a training step of 32 entries took 2.5 % longer with them, 8 entries of 192 718 -> 729 us.
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
@@ -900,9 +900,10 @@ int try_ns_fused(const NsGroup* grp, int ngroups, int steps, int const_coeffs, i
   // (measured at D = H = 384: 16 and 12 units, i.e. under 1.5 Gram tiles of width 192 per SM) the symmetric phases
   // leave a second, nearly empty round of tiles and plain 128-wide tiles are 4-5 % faster; from 20 units up the
   // symmetric variant wins.
-  // Gram sides that 256 divides run on the same tiles; the training forward (`keep`) refuses them as it always has.  One launch per
-  // product took, with four updates of square matrices (us per call, launches / this kernel): side 256, 1 unit 594 / 396, 16 units
-  // 630 / 498, 32 units 810 / 710; side 512 673 / 461, 1434 / 1303, 2740 / 2414.  (Three tiles of four are no gain: 256 stays plain.)
+  // Gram sides that 256 divides run on the same tiles; the training forward (`keep`) refuses them as it always has.  Five iterations on
+  // 3, 24, 48 and 96 square matrices by themselves, us, one launch per product / this kernel: side 256 125, 128, 134, 189 / 76, 86, 99,
+  // 140; side 512 150, 221, 319, 613 / 94, 154, 233, 469; side 768 195, 422, 855, 1680 / 145, 320, 655, 1357.  (Three tiles of four are
+  // no gain: 256 stays plain.)
   const bool by256 = keep == nullptr && bt_mm == 256 && bt_mn != 64;
   const bool wide = bt_mm == 192 && bt_mn == 192;
   bool symmable = wide || by256;

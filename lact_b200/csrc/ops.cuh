@@ -511,9 +511,6 @@ __global__ void prepare_weights_kernel(const void* w0, const void* w1, const voi
   if (lane == 0) *dn = sqrtf(ss);
 }
 
-// beta[u][b] = mean over tokens [s_u, e_u) of momentum[b, t] for up to kMeanBatch update steps per
-// launch; grid (batch entries, steps).
-constexpr int kMeanBatch = 64;
 // Up to six batched copies of fp32 rows in one launch: entry b of copy i is n[i] values from src[i] + b * src_bs[i] to dst[i] +
 // b * dst_bs[i].  (State in and out of a call is three to six arrays whose copies, one after another, were 12 us of a call that
 // updates 12 entries of 128 x 256 once.)
@@ -540,6 +537,9 @@ __global__ void __launch_bounds__(256) state_copy_kernel(const StateCopyArgs a) 
   }
 }
 
+// beta[u][b] = mean over tokens [s_u, e_u) of momentum[b, t] for up to kMeanBatch update steps per
+// launch; grid (batch entries, steps).
+constexpr int kMeanBatch = 64;
 struct MeanArgs {
   int32_t n;
   int32_t s[kMeanBatch], e[kMeanBatch];

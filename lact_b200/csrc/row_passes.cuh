@@ -3,7 +3,8 @@
 // Grid (token blocks, heads [x tensors], batch entries): no index divisions, and a block's rows are consecutive tokens.
 // What bounds them is HBM and the instructions between the loads: 2 batches x 8192 tokens x 4 heads of 384 take 83 us in the
 // prologue forward (302 MB: 3.6 TB/s) and 107 backward (125 with the sigmoid worked out again behind the row sums: two of the
-// special-function unit's operations per feature, which it takes half of that time for), 40 and 52 in the epilogue.  Persistent
+// special-function unit's operations per feature, which it takes half of that time for; keeping it spills 12 bytes at the 80
+// registers of three blocks per SM), 40 and 52 in the epilogue.  Persistent
 // blocks with the next row's loads in flight take 12 to 20 % longer (fewer warps).  (A warp per row leaves a quarter of the
 // lanes without a unit at that size and the loads of too few warps in flight: 144, 324, 59 and 111 us.)  Head sizes without a
 // (LPR, V) of this table take the warp-per-row kernels of ops.cuh.
