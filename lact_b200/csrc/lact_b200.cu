@@ -21,6 +21,7 @@
 #include "pair_gemm.cuh"
 #include "row_passes.cuh"
 #include "swa_bwd.cuh"
+#include "swa_pairs.cuh"
 
 namespace lact {
 namespace {
@@ -1217,6 +1218,28 @@ int launch_swa(const SwaArgs& a, int64_t ctas, cudaStream_t stream) {
   }
   KernelScope scope(kClsOther, stream);
   LACT_CUDA(launch_pdl(kernel, dim3(static_cast<unsigned>(ctas)), dim3(320), smem, stream, a));
+  return LACT_OK;
+}
+
+template <int HD>
+int launch_swa_pairs(const SwaPairArgs& a, int64_t ctas, cudaStream_t stream) {
+  auto kernel = swa_pairs_kernel<HD>;
+  constexpr uint32_t smem = SwaPairSmem<HD>::kBytes;
+  static_assert(smem <= 232448, "shared memory budget exceeded");
+  static std::mutex mu;
+  static bool configured[64] = {false};
+  int dev = 0;
+  LACT_CUDA(cudaGetDevice(&dev));
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    if (dev >= 64 || !configured[dev]) {
+      LACT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+      if (dev < 64) configured[dev] = true;
+    }
+  }
+  KernelScope scope(kClsOther, stream);
+  LACT_CUDA(launch_pdl(kernel, dim3(static_cast<unsigned>(ctas)), dim3(kSwaPairThreads), smem, stream, a));
+  if (a.cutters > 0) LACT_CUDA(launch_pdl(swa_combine_kernel<HD>, dim3(static_cast<unsigned>(a.rest) * 32), dim3(256), 0, stream, a));
   return LACT_OK;
 }
 
@@ -2757,23 +2780,84 @@ int lact_out_epilogue(const void* fw_x, const void* weight, const void* gate_pro
 struct SwaSplit {
   int64_t whole;
   int splits;
+  double us;
 };
-static SwaSplit swa_split(int64_t b, int64_t l, int64_t lk, int64_t heads, int64_t d, int64_t window) {
+static SwaSplit swa_split(int64_t b, int64_t l, int64_t lk, int64_t heads, int64_t d, int64_t window, bool may_cut) {
   const int64_t sms = sm_count(), tiles = b * heads * ceil_div(l, 128);
   const int64_t span = window < 0 ? (lk > 0 ? lk : l) : window > 0 && window < l ? std::min(l, window + 127) : l;
   const int64_t T = ceil_div(span, 128), rest = tiles % sms;
-  SwaSplit best{tiles, 1};
-  if (rest == 0 || tiles > 64 * sms) return best;
-  const double per_tile = d == 64 ? 1.2 : 1.5;
-  double cost = T * per_tile + 4.0;
+  const double per_tile = d == 64 ? 1.2 : 1.5, round = T * per_tile + 4.0;
+  // (tiles of causal attention without a window are half as long on the average, and the SMs take them as they come)
+  const bool even = window < 0 || (window > 0 && 2 * window <= l);
+  const double rounds = even || tiles <= sms ? static_cast<double>((tiles + sms - 1) / sms) : std::max(1.0, 0.6 * tiles / sms);
+  SwaSplit best{tiles, 1, rounds * round};
+  if (!may_cut || rest == 0 || tiles > 64 * sms) return best;
+  double cost = round;
   for (int s = 2; s <= 16 && s <= T; ++s) {
     const double c = ((rest * s + sms - 1) / sms) * (((T + s - 1) / s) * per_tile + 4.0) + 2.0 + 0.6 * s;
     if (c < 0.9 * cost) {
       cost = c;
-      best = SwaSplit{tiles - rest, s};
+      best = SwaSplit{tiles - rest, s, (even ? static_cast<double>(tiles / sms) : std::max(tiles >= sms ? 1.0 : 0.0, 0.6 * (tiles - rest) / sms)) * round + c};
     }
   }
   return best;
+}
+
+// The same launch on pairs of query tiles (see SwaPairArgs).  Whole pairs fill whole rounds of the SMs; the rest, all pairs where there are
+// fewer than SMs, are cut over their keys if the longest CTA then ends sooner: 2.5 us per pair or piece plus 2.0 us per key tile (1.5
+// at d = 64), a second launch that puts the pieces together and what it waits for 13.  Measured: 1560 queries over 4680 keys, 12 heads of
+// 128 (84 pairs on 148 SMs, 38 key tiles each) whole 84, cut 72 us.  Pairs of causal attention without a window differ in length and
+// are dealt the long ones first: 8 heads of 8192 queries (256 pairs) are left whole, 133 us, 221 with the 108 shortest cut.
+struct SwaPairSplit {
+  int64_t whole, rest, cutters, span;   // cutters = 0: nothing is cut (and rest = 0)
+  double us;
+};
+static SwaPairSplit swa_pair_split(int64_t b, int64_t l, int64_t lk, int64_t heads, int64_t d, int64_t window, bool may_cut) {
+  const int64_t sms = sm_count(), bh = b * heads, pairs = ceil_div(l, 256), items = bh * pairs;
+  const bool causal = window >= 0;
+  const int64_t band = window > 0 && window < l ? window : l;
+  const int64_t span = causal ? std::min<int64_t>(ceil_div(l, 128), ceil_div(band + 255, 128) + 1) : ceil_div(lk > 0 ? lk : l, 128);
+  const double per_tile = d == 64 ? 1.5 : 2.0, per_item = 2.5;
+  // the longest CTA's time for the first n items; only where their lengths differ are they looked at one by one
+  auto dealt = [&](int64_t n) {
+    const int64_t rounds = (n + sms - 1) / sms;
+    if (!causal || n <= sms || rounds > 8 || band + 256 <= l / 2) return rounds * (span * per_tile + per_item);
+    double worst = 0.0;
+    for (int64_t c = 0; c < sms; ++c) {
+      double t = 0.0;
+      for (int64_t r = 0; r < rounds; ++r) {
+        const int64_t item = r * sms + ((r & 1) ? sms - 1 - c : c);
+        if (item >= n) continue;
+        const int64_t q0 = (pairs - 1 - item / bh) * 256;
+        t += (ceil_div(std::min(q0 + 256, l), 128) - std::max<int64_t>(q0 - (band - 1), 0) / 128) * per_tile + per_item;
+      }
+      worst = std::max(worst, t);
+    }
+    return worst;
+  };
+  SwaPairSplit best{items, 0, 0, 0, dealt(items) + 2.0};
+  const int64_t rest = items % sms;
+  if (!may_cut || rest == 0 || items > 64 * sms) return best;
+  const double before = dealt(items - rest) + 13.0 + 2 * per_item;
+  for (int64_t s = 2, last = 0; s <= 16; s += 1 + s / 4) {
+    const int64_t cutters = std::min(rest * std::min(s, span), sms);
+    if (cutters == last) break;
+    last = cutters;
+    const double us = before + ceil_div(rest * span, cutters) * per_tile;
+    if (us < 0.95 * best.us) best = SwaPairSplit{items - rest, rest, cutters, span, us};
+  }
+  return best;
+}
+// Scratch of a cut launch: fewer pieces than cutters and items together, 256 rows each.
+static size_t swa_pair_scratch(const SwaPairSplit& sp, int64_t d) {
+  return static_cast<size_t>(sp.cutters + sp.rest) * 256 * (d * sizeof(float) + sizeof(float2));
+}
+// Whether a launch runs on pairs: by the estimates of both.  Measured (us, single tiles / pairs): 12 heads of 128
+// with 4096 queries and a window of 2048 78 / 47, 8 with 16384 206 / 159, 4 with 1024 and 512 14.6 / 18.7, 8 of 64 with 777 queries over
+// 2777 keys 26 / 32.
+static bool swa_takes_pairs(int64_t b, int64_t l, int64_t lk, int64_t heads, int64_t d, int64_t window, bool may_cut, SwaPairSplit* pairs) {
+  *pairs = swa_pair_split(b, l, lk, heads, d, window, may_cut);
+  return pairs->us < swa_split(b, l, lk, heads, d, window, may_cut).us;
 }
 
 int lact_swa_fwd_split_bytes(int64_t b, int64_t l, int64_t lk, int64_t n_heads, int64_t d, int64_t window, size_t* bytes,
@@ -2781,7 +2865,13 @@ int lact_swa_fwd_split_bytes(int64_t b, int64_t l, int64_t lk, int64_t n_heads, 
   if (!bytes || !counters) return LACT_ERR_NULL;
   if ((d != 64 && d != 128) || b < 1 || l < 1 || n_heads < 1 || b > 65535 || n_heads > 65535 || l > (1ll << 30) || lk > (1ll << 30))
     return LACT_ERR_SHAPE;
-  const SwaSplit sp = swa_split(b, l, lk, n_heads, d, window);
+  SwaPairSplit pairs;
+  if (swa_takes_pairs(b, l, lk, n_heads, d, window, true, &pairs)) {
+    *counters = 0;
+    *bytes = swa_pair_scratch(pairs, d);
+    return LACT_OK;
+  }
+  const SwaSplit sp = swa_split(b, l, lk, n_heads, d, window, true);
   *counters = sp.splits > 1 ? b * n_heads * ceil_div(l, 128) - sp.whole : 0;
   *bytes = static_cast<size_t>(*counters) * sp.splits * (128 * d * sizeof(float) + 256 * sizeof(float2));
   return LACT_OK;
@@ -2841,12 +2931,39 @@ static int swa_fwd_impl(const void* q, const void* k, const void* v, const SwaSe
   a.lse = static_cast<float*>(lse);
   a.seq_start = seq_start;
   a.status = status_word;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
   int64_t ctas = b * n_heads * a.q_tiles;
   if (ctas > 0x7FFFFFFFll) return LACT_ERR_SHAPE;
+  SwaPairSplit sp2;
+  if (swa_takes_pairs(b, l, lk, n_heads, d, window, scratch != nullptr, &sp2)) {
+    SwaPairArgs p;
+    std::memset(&p, 0, sizeof(p));
+    p.q = a.q; p.k = a.k; p.v = a.v; p.k2 = a.k2; p.v2 = a.v2;
+    p.o = a.o; p.o_bs = a.o_bs; p.o_ts = a.o_ts; p.o_hs = a.o_hs;
+    p.L = a.L; p.window = a.window; p.Lk = a.Lk; p.causal = a.causal; p.Lk1 = a.Lk1;
+    p.heads = a.heads;
+    p.entries = static_cast<int32_t>(b);
+    p.pairs = ceil_div(l, 256);
+    p.scale_log2 = a.scale_log2; p.seq_start = a.seq_start; p.lse = a.lse; p.status = a.status;
+    p.whole = static_cast<int32_t>(sp2.whole);
+    if (sp2.cutters > 0) {
+      if (scratch_bytes < swa_pair_scratch(sp2, d) || (reinterpret_cast<uintptr_t>(scratch) & 15) != 0) return LACT_ERR_WORKSPACE;
+      p.rest = static_cast<int32_t>(sp2.rest);
+      p.cutters = static_cast<int32_t>(sp2.cutters);
+      p.span = static_cast<int32_t>(sp2.span);
+      p.share = static_cast<int32_t>(sp2.rest * sp2.span / sp2.cutters);
+      p.longer = static_cast<int32_t>(sp2.rest * sp2.span % sp2.cutters);
+      p.part = static_cast<float*>(scratch);
+      p.ml = reinterpret_cast<float2*>(p.part + (sp2.cutters + sp2.rest) * 256 * d);
+    }
+    ctas = std::max<int64_t>(p.cutters, std::min<int64_t>(p.whole, sm_count()));
+    p.rounds = ceil_div(p.whole, ctas);
+    return d == 64 ? launch_swa_pairs<64>(p, ctas, st) : launch_swa_pairs<128>(p, ctas, st);
+  }
   a.whole = static_cast<int32_t>(ctas);
   a.splits = 1;
   if (scratch != nullptr && counters != nullptr) {
-    const SwaSplit sp = swa_split(b, l, lk, n_heads, d, window);
+    const SwaSplit sp = swa_split(b, l, lk, n_heads, d, window, true);
     const int64_t rest = ctas - sp.whole;
     const size_t rows = static_cast<size_t>(rest) * sp.splits;
     if (sp.splits > 1) {
@@ -2860,7 +2977,6 @@ static int swa_fwd_impl(const void* q, const void* k, const void* v, const SwaSe
       ctas = sp.whole + rest * sp.splits;
     }
   }
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
   return d == 64 ? launch_swa<64>(a, ctas, st) : launch_swa<128>(a, ctas, st);
 }
 

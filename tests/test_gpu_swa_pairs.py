@@ -1,0 +1,98 @@
+"""Attention forward on pairs of query tiles: outputs and log-sum-exps against 64-bit attention where the pairs, the dealing of items to
+SMs and the cut of the last ones have their edges."""
+import pytest
+import torch
+
+from test_gpu_swa_split import _run
+
+pytestmark = pytest.mark.gpu
+
+
+def _reference(q, k, v, window, starts=None):
+    l, lk, d = q.shape[1], k.shape[1], q.shape[-1]
+    qf, kf, vf = (t.double().transpose(1, 2) for t in (q, k, v))
+    s = qf @ kf.transpose(2, 3) * d ** -0.5
+    if window >= 0:
+        i, j = torch.arange(l, device="cuda")[:, None], torch.arange(lk, device="cuda")[None]
+        hidden = j > i
+        if window > 0:
+            hidden |= j <= i - window
+        if starts is not None:
+            hidden |= j < starts[:, None]
+        s = s.masked_fill(hidden, float("-inf"))
+    return (s.softmax(-1) @ vf).transpose(1, 2), torch.logsumexp(s, -1) * 1.4426950408889634
+
+
+def _compare(q, k, v, window, cut, starts=None):
+    from lact_b200 import _lib as L
+    o, lse = _run(L, q, k, v, window, cut, starts)
+    want, want_lse = _reference(q, k, v, window, starts)
+    assert torch.isfinite(o.float()).all()
+    # probabilities and results are rounded to bf16 (2^-9 each)
+    assert float((o.double() - want).norm() / want.norm()) <= 6e-3
+    # the scores' products are summed in fp32 (2^-24 each over d terms), the exponentials are good to 2^-22
+    assert float((lse.double() - want_lse).abs().max()) <= 1e-4
+
+
+# one tile and two, rows on both sides of a tile's and a pair's end, windows that end on tiles and inside them (300 heads: calls with
+# few tiles run on single ones)
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("l,window", [(1, 0), (127, 40), (128, 128), (129, 1), (255, 0), (256, 128), (257, 129), (385, 256), (511, 130),
+                                      (513, 600)])
+def test_ends_of_pairs(l, window, d):
+    g = torch.Generator(device="cuda").manual_seed(l * 7 + window)
+    q, k, v = (torch.randn(1, l, 300, d, device="cuda", generator=g).to(torch.bfloat16) for _ in range(3))
+    _compare(q, k, v, window, False)
+
+
+# more items than SMs: whole rounds and a rest that is cut; one round exactly; keys of block attention on both sides of a tile's end
+@pytest.mark.parametrize("b,l,lk,h,d,window,cut", [(1, 1100, 1100, 40, 128, 0, False), (1, 2600, 2500, 14, 128, -1, True),
+                                                   (2, 1900, 2600, 10, 64, -1, True),
+                                                   (1, 257, 257, 74, 64, 200, False), (1, 300, 1025, 80, 128, -1, False),
+                                                   (3, 130, 127, 30, 64, -1, False)])
+def test_items_over_the_chip(b, l, lk, h, d, window, cut):
+    g = torch.Generator(device="cuda").manual_seed(l + h)
+    rn = lambda n: torch.randn(b, n, h, d, device="cuda", generator=g).to(torch.bfloat16)
+    _compare(rn(l), rn(lk), rn(lk), window, cut)
+
+
+@pytest.mark.parametrize("l,h,window,cut", [(1100, 60, 300, False), (2305, 8, 2048, True)])
+@pytest.mark.parametrize("cuts", [(128, 256, 400), (1, 2, 383), (255, 257, 1000), (64, 640, 896)])
+def test_packed_sequences_across_pairs(l, h, window, cut, cuts):
+    g = torch.Generator(device="cuda").manual_seed(sum(cuts))
+    q, k, v = (torch.randn(1, l, h, 128, device="cuda", generator=g).to(torch.bfloat16) for _ in range(3))
+    starts = torch.zeros(l, dtype=torch.int32, device="cuda")
+    for c in cuts:
+        starts[c:] = c
+    _compare(q, k, v, window, cut, starts)
+
+
+def test_growing_scores_reach_every_row():
+    """Scores that grow along the keys: the maximum changes in every tile, for some rows by more than fp32's range of exponents."""
+    g = torch.Generator(device="cuda").manual_seed(5)
+    q, k, v = (torch.randn(1, 900, 100, 64, device="cuda", generator=g).to(torch.bfloat16) for _ in range(3))
+    k = (k * torch.linspace(0.1, 30, 900, device="cuda")[None, :, None, None]).to(torch.bfloat16)
+    from lact_b200 import _lib as L
+    o, _ = _run(L, q, k, v, 0, False)
+    want, _ = _reference(q, k, v, 0)
+    # one probability of 1 beside small ones: the result is that value's bf16 rounding or near it
+    assert float((o.double() - want).norm() / want.norm()) <= 6e-3
+
+
+@pytest.mark.parametrize("l,h,window,cut", [(300, 200, 0, False), (2305, 8, 2048, True)])
+def test_nothing_is_written_after_an_earlier_failure(l, h, window, cut):
+    import ctypes as C
+    from lact_b200 import _lib as L
+    b, d = 1, 128
+    q, k, v = (torch.randn(b, l, h, d, device="cuda").to(torch.bfloat16) for _ in range(3))
+    o, lse = torch.full_like(q, 7.0), torch.full((b, h, l), 7.0, device="cuda")
+    need, words = C.c_size_t(0), C.c_int64(0)
+    L.check(L.lib().lact_swa_fwd_split_bytes(b, l, l, h, d, window, C.byref(need), C.byref(words)), "split_bytes")
+    scratch = torch.zeros(max(need.value, 256), dtype=torch.uint8, device="cuda")
+    status = torch.zeros(64, dtype=torch.int32, device="cuda")
+    status[0] = 101
+    L.check(L.lib().lact_swa_fwd_split(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), b, l, l, h, d, *[h * d, h * d * l] * 4, window,
+                                       d ** -0.5, None, lse.data_ptr(), None, scratch.data_ptr() if cut else None, need.value,
+                                       status.data_ptr(), L.stream_ptr()), "swa")
+    torch.cuda.synchronize()
+    assert bool((o == 7).all()) and bool((lse == 7).all())
