@@ -20,6 +20,7 @@
 #include "few_tokens.cuh"
 #include "pair_gemm.cuh"
 #include "row_passes.cuh"
+#include "grad_fused.cuh"
 #include "swa_bwd.cuh"
 #include "swa_pairs.cuh"
 
@@ -608,8 +609,55 @@ int run_grad_pointwise(const GradArgs& a, int32_t* status, cudaStream_t stream) 
   return launch_gemm(g, stream, kClsGradPointwise);
 }
 
+// Whether an update of `len` tokens runs as one launch (grad_fused.cuh): by an estimate of both in us, each CTA's chain of tiles against the
+// rounds of the two launches (both give the same bits; sums that choose_split cuts stay cut).  Measured, us per call of five updates, two
+// launches / one: 12 entries of 128 x 256, 384 tokens each 136 / 107, 1560 235 / 199; 32 entries, chunks of 2048 476 / 393; 16 entries,
+// 4096 456 / 353.  Few CTAs with many tokens lose: one entry, 4096 130 / 176; 4 entries of 128 x 128, one update of 6000 97 / 112; so does a
+// short second round: 24 entries, 384 172 / 177.
+bool grad_in_one_launch(int64_t B, int64_t D, int64_t H, int64_t len) {
+  if (D != kGradD || H % kBM != 0 || len < 1 || choose_split(ceil_div(len, kBK)).splits > 1) return false;
+  const double sms = sm_count(), rounds = B * (H / kGradSlice) / sms;
+  const int64_t tiles = ceil_div(len, 128);
+  const double one = std::max(1.0, rounds) * (1.15 * tiles + 5.0) + (rounds > 1.0 ? 3.5 : 0.0);
+  const double two = 5.0 + 2.0 * std::ceil(B * tiles * (H / 64) / sms) + std::ceil(B * (3 * H / kBM) / sms) * (0.6 * tiles + 4.0);
+  return 1.05 * one < two;
+}
+
+int run_grad_fused(const GradArgs& a, int32_t* status, cudaStream_t stream) {
+  GradFusedArgs g;
+  std::memset(&g, 0, sizeof(g));
+  LACT_TRY(encode_map(&g.k, Mat{a.k, a.end, a.D, a.k_ts, a.B, a.k_bs}, 128));
+  LACT_TRY(encode_map(&g.v, Mat{a.v, a.end, a.D, a.v_ts, a.B, a.v_bs}, 128));
+  LACT_TRY(encode_map(&g.w02, Mat{a.w02b, 2 * a.H, a.D, a.D, a.B, 2 * a.H * a.D}, kGradSlice));
+  LACT_TRY(encode_map(&g.w1, Mat{a.w1b, a.D, a.H, a.H, a.B, a.D * a.H}, 128, kGradSlice));
+  g.lr = EpiFwGrad{a.lr0, a.lr1, a.lr2, a.lr_f32, static_cast<int32_t>(a.start), a.lr_bs, a.w_scale};
+  g.e[0] = EpiDW{a.g02, 2 * a.H * a.D, a.D, a.beta, 1, a.g_f32, a.partial02, 0, 0, a.gb02, a.g02_prev, a.fresh};
+  g.e[1] = EpiDW{a.g1, a.D * a.H, a.H, a.beta, 1, a.g_f32, a.partial1, 0, 0, a.gb1, a.g1_prev, a.fresh};
+  g.start = static_cast<int32_t>(a.start);
+  g.len = static_cast<int32_t>(a.end - a.start);
+  g.H = static_cast<int32_t>(a.H);
+  g.status = status;
+  const int64_t ctas = a.B * (a.H / kGradSlice);
+  if (ctas > 0x7FFFFFFFll) return LACT_ERR_SHAPE;
+  static std::mutex mu;
+  static bool configured[64] = {false};
+  int dev = 0;
+  LACT_CUDA(cudaGetDevice(&dev));
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    if (dev >= 64 || !configured[dev]) {
+      LACT_CUDA(cudaFuncSetAttribute(grad_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GradSmem::kBytes));
+      if (dev < 64) configured[dev] = true;
+    }
+  }
+  KernelScope scope(kClsGradContract, stream);
+  LACT_CUDA(launch_pdl(grad_fused_kernel, dim3(static_cast<unsigned>(ctas)), dim3(kGradThreads), GradSmem::kBytes, stream, g));
+  return LACT_OK;
+}
+
 int run_grad(const GradArgs& a, int32_t* status, cudaStream_t stream) {
   const int64_t len = a.end - a.start;
+  if (grad_in_one_launch(a.B, a.D, a.H, len)) return run_grad_fused(a, status, stream);
   LACT_TRY(run_grad_pointwise(a, status, stream));
   const Mat km{a.k, a.end, a.D, a.k_ts, a.B, a.k_bs};
   const Mat vm{a.v, a.end, a.D, a.v_ts, a.B, a.v_bs};

@@ -90,22 +90,38 @@ struct EpiDW {
   // row per lane.  Returns this lane's share of the sum of squares of the bf16-rounded results if `want_ss`.
   __device__ __forceinline__ float warp_block(int batch, int row0, int col, int M, int N, const float* v,
                                               uint32_t scratch, int lane, bool want_ss) const {
+    put_block<false>(v, scratch, lane);
+    float4 old[8];
+    const float bt = load_state(batch, row0, col, M, N, lane, old);
+    return add_block(batch, row0, col, M, N, scratch, lane, want_ss, old, bt);
+  }
+  // Its three parts: the block into `scratch` (TRANSPOSED: thread `lane` holds column `col + lane`, rows row0 to row0 + 31), the momentum
+  // state and its factor, the sum of both out.
+  template <bool TRANSPOSED>
+  __device__ __forceinline__ void put_block(const float* v, uint32_t scratch, int lane) const {
+    if constexpr (TRANSPOSED) {
 #pragma unroll
-    for (int gq = 0; gq < 8; ++gq) {
-      float r[4];
+      for (int j = 0; j < 32; ++j)
+        asm volatile("st.shared.f32 [%0], %1;" ::"r"(scratch + j * 144 + lane * 4), "f"(round_bf16 ? bf16_round(v[j]) : v[j]) : "memory");
+    } else {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) r[j] = round_bf16 ? bf16_round(v[gq * 4 + j]) : v[gq * 4 + j];
-      asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(scratch + lane * 144 + gq * 16), "f"(r[0]), "f"(r[1]),
-                   "f"(r[2]), "f"(r[3])
-                   : "memory");
+      for (int gq = 0; gq < 8; ++gq) {
+        float r[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) r[j] = round_bf16 ? bf16_round(v[gq * 4 + j]) : v[gq * 4 + j];
+        asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(scratch + lane * 144 + gq * 16), "f"(r[0]), "f"(r[1]),
+                     "f"(r[2]), "f"(r[3])
+                     : "memory");
+      }
     }
     __syncwarp();
+  }
+  __device__ __forceinline__ float load_state(int batch, int row0, int col, int M, int N, int lane, float4 (&old)[8]) const {
     const int u = lane & 7, rsub = lane >> 3;
     const bool col_ok = col + u * 4 + 4 <= N;
     const bool rmw = out_f32 && beta != nullptr;
     const float bt = rmw ? beta[batch] : 0.f;
     const int64_t base = batch * bs + col + u * 4;
-    float4 old[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int row = row0 + i * 4 + rsub;
@@ -114,6 +130,13 @@ struct EpiDW {
         old[i] = *reinterpret_cast<const float4*>((g_prev != nullptr ? g_prev : reinterpret_cast<const float*>(g)) + base +
                                                   static_cast<int64_t>(row) * ld);
     }
+    return bt;
+  }
+  __device__ __forceinline__ float add_block(int batch, int row0, int col, int M, int N, uint32_t scratch, int lane, bool want_ss,
+                                             const float4 (&old)[8], float bt) const {
+    const int u = lane & 7, rsub = lane >> 3;
+    const bool col_ok = col + u * 4 + 4 <= N;
+    const int64_t base = batch * bs + col + u * 4;
     float ss = 0.f;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -438,12 +461,11 @@ struct OpFwGradPointwise {
     return __uint_as_float(ep.lr_f32 ? r : r << 16) * ep.w_scale;
   }
   __device__ static __forceinline__ bool skip_store(const Epi&, int) { return false; }
-  __device__ static __forceinline__ void epilogue_staged(const Epi& ep, int, int, int, int, int,
-                                                         const float (&v)[3][32], float (&o)[3][32],
-                                                         Prefetch& pf) {
+  template <int N>
+  __device__ static __forceinline__ void pointwise(const Epi& ep, const float (&v)[3][N], float (&o)[3][N], const Prefetch& pf) {
     const float l0 = rate(ep, pf.r[0]), l1 = rate(ep, pf.r[1]), l2 = rate(ep, pf.r[2]);
 #pragma unroll
-    for (int j = 0; j < 32; ++j) {
+    for (int j = 0; j < N; ++j) {
       const float y0 = v[0][j], y2 = v[1][j], dh = v[2][j];
       const float sg = sigmoidf_fast(y0);
       const float sw = sg * y0;
@@ -451,6 +473,11 @@ struct OpFwGradPointwise {
       o[1][j] = sw * dh * l2;                                     // dy2
       o[2][j] = sw * y2 * l1;                                     // hidden * lr1
     }
+  }
+  __device__ static __forceinline__ void epilogue_staged(const Epi& ep, int, int, int, int, int,
+                                                         const float (&v)[3][32], float (&o)[3][32],
+                                                         Prefetch& pf) {
+    pointwise<32>(ep, v, o, pf);
   }
 };
 

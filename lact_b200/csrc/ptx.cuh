@@ -411,6 +411,10 @@ __device__ __forceinline__ uint32_t leader_address(const void* p) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(smem_u32(p)));
   return a;
 }
+// a value into another CTA's shared memory (an address of the cluster's window)
+__device__ __forceinline__ void st_shared_cluster(uint32_t addr, float x) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(x) : "memory");
+}
 __device__ __forceinline__ void mbar_arrive_leader(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(leader_address(bar)) : "memory");
 }

@@ -1,0 +1,76 @@
+"""The fast-weight gradient of heads of 128 features in one launch against the two launches, bit for bit: the way is chosen by the number
+of entries, and an entry has the same bits in any batch; tokens whose learning rates are zero add nothing."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _inputs(b, n, h, lr_dtype, seed=0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    rn = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    d = 128
+    w = [rn(b, h, d) / d ** 0.5, rn(b, d, h) / h ** 0.5, rn(b, h, d) / d ** 0.5]
+    qkv = [torch.nn.functional.normalize(rn(b, n, d), dim=-1).bfloat16() for _ in range(2)] + [rn(b, n, d).bfloat16()]
+    lrs = [torch.nn.functional.softplus(rn(b, n, 1) - 2.0).to(lr_dtype) for _ in range(3)]
+    return w, qkv, lrs, torch.sigmoid(rn(b, n, 1)), [rn(*x.shape) for x in w]
+
+
+def _step(w, qkv, lrs, gate, m, muon):
+    import lact_b200 as lb
+    n = qkv[0].shape[1]
+    out = lb.ar_fast_weight_swish_glu_weight_norm_mini_batch_inference_with_momentum(
+        *w, *qkv, *lrs, 1.0, mini_batch_size=n, do_update=True, use_moun=muon, num_moun_iters=5, fw_momentum=gate,
+        dw0_momentum=m[0], dw1_momentum=m[1], dw2_momentum=m[2], use_momentum=True)
+    lb.synchronize_and_check()
+    return [t for t in out if torch.is_tensor(t)]
+
+
+def _same(a, b):
+    assert len(a) == len(b) >= 7
+    for x, y in zip(a, b):
+        assert torch.equal(x, y)
+
+
+# an entry alone takes two launches at these lengths, sixteen take one: ends of tiles of 128 tokens, of k-blocks of 64, of both
+@pytest.mark.parametrize("n", [2048, 2049, 2111, 2175, 2177, 2300, 4000])
+@pytest.mark.parametrize("h,muon,lr", [(256, True, torch.float32), (128, False, torch.bfloat16)])
+def test_entries_of_a_batch_and_alone(n, h, muon, lr):
+    w, qkv, lrs, gate, m = _inputs(16, n, h, lr)
+    both = _step(w, qkv, lrs, gate, m, muon)
+    for e in (0, 7, 15):
+        one = lambda ts: [t[e:e + 1].contiguous() for t in ts]
+        _same([t[e:e + 1] for t in both], _step(one(w), one(qkv), one(lrs), gate[e:e + 1].contiguous(), one(m), muon))
+
+
+# few tokens (one launch) against the same tokens in front of others whose learning rates are zero (two launches)
+@pytest.mark.parametrize("n", [1, 5, 63, 64, 65, 127, 128, 129, 200, 256, 257, 385])
+@pytest.mark.parametrize("h", [128, 256, 384])
+def test_few_tokens_and_zero_learning_rates(n, h):
+    w, qkv, lrs, gate, m = _inputs(1, 2300, h, torch.float32, seed=n)
+    for t in lrs:
+        t[:, n:] = 0
+    gate[:] = gate[:, :1]      # (the momentum's factor is the mean gate of the tokens)
+    gate = torch.full_like(gate, 0.5)
+    few = _step(w, [t[:, :n].contiguous() for t in qkv], [t[:, :n].contiguous() for t in lrs], gate[:, :n].contiguous(), m, True)
+    many = _step(w, qkv, lrs, gate, m, True)
+    _same([t[:, :n] if t.dim() == 3 and t.shape[1] == 2300 else t for t in many], few)
+
+
+def test_tokens_before_the_range_and_strided_rows():
+    """An update of a later frame (the tile's rows begin inside the arrays) on rows that are views of a fused projection."""
+    import lact_b200 as lb
+    b, f, h = 12, 1560, 256
+    w, _, lrs, gate, _ = _inputs(b, 3 * f, h, torch.float32, seed=3)
+    g = torch.Generator(device="cuda").manual_seed(4)
+    wide = torch.randn(b, 3 * f, 3 * 128, device="cuda", generator=g).bfloat16()
+    q, k, v = (wide[..., i * 128:(i + 1) * 128] for i in range(3))
+    run = lambda q, k, v, sel: lb.ar_fast_weight_swish_glu_weight_norm_mini_batch_with_momentum(
+        *[t[sel] for t in w], q[sel], k[sel], v[sel], *[t[sel] for t in lrs], 1.0, mini_batch_size=f, update_every=f, use_moun=False,
+        num_moun_iters=5, fw_momentum=gate[sel], use_momentum=True)
+    views = run(q, k, v, slice(None))
+    copies = run(q.contiguous(), k.contiguous(), v.contiguous(), slice(None))
+    alone = run(q.contiguous(), k.contiguous(), v.contiguous(), slice(3, 4))
+    lb.synchronize_and_check()
+    for x, y, z in zip(views, copies, alone):
+        assert torch.equal(x, y) and torch.equal(x[3:4], z)
