@@ -40,7 +40,7 @@ struct GradSmem {
 static_assert(GradSmem::kK % 1024 == 0 && GradSmem::kDy % 1024 == 0 && GradSmem::kHid % 1024 == 0, "swizzled tiles");
 static_assert(kEpiWarps * 32 * 144 <= 6 * GradSmem::kBox, "the gradient's epilogue works in the memory of k");
 
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGradThreads, 1) grad_fused_kernel(const __grid_constant__ GradFusedArgs a) {
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGradThreads, 1) grad_gemm_kernel(const __grid_constant__ GradFusedArgs a) {
   using SM = GradSmem;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -119,7 +119,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGradThreads, 1) gra
     tma_load_3d_if(leader, base + SM::kW1, &a.w1, smem_u32(w_full), slice * kGradSlice, 0, batch);
     load(leader, &a.v, &v_full[0], base + SM::kV, 0);
   }
-  bool failed = earlier_launch_failed(a.status);
+  // (the second issuing warp waits at mbarriers alone and reads the word by itself)
+  bool failed = warp < 2 + kEpiWarps ? earlier_launch_failed(a.status)
+                                     : uniform(static_cast<uint32_t>(*reinterpret_cast<volatile int32_t*>(a.status))) != kStatusOk;
   const bool skip = failed;
   const uint32_t rank = cluster_rank();
   float own1 = 0.f;   // this lane's share of the squares of dw1

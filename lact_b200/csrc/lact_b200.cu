@@ -646,12 +646,12 @@ int run_grad_fused(const GradArgs& a, int32_t* status, cudaStream_t stream) {
   {
     std::lock_guard<std::mutex> lock(mu);
     if (dev >= 64 || !configured[dev]) {
-      LACT_CUDA(cudaFuncSetAttribute(grad_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GradSmem::kBytes));
+      LACT_CUDA(cudaFuncSetAttribute(grad_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GradSmem::kBytes));
       if (dev < 64) configured[dev] = true;
     }
   }
   KernelScope scope(kClsGradContract, stream);
-  LACT_CUDA(launch_pdl(grad_fused_kernel, dim3(static_cast<unsigned>(ctas)), dim3(kGradThreads), GradSmem::kBytes, stream, g));
+  LACT_CUDA(launch_pdl(grad_gemm_kernel, dim3(static_cast<unsigned>(ctas)), dim3(kGradThreads), GradSmem::kBytes, stream, g));
   return LACT_OK;
 }
 

@@ -862,8 +862,7 @@ __device__ __forceinline__ void gemm_teardown(GemmCtx& cx, bool failed, int32_t*
 // small calls took 0.2 to 0.7 us longer (4 entries of 384, 2048 tokens: apply 15.5 us, 16.1 and 16.1 that way).
 __device__ __forceinline__ bool earlier_launch_failed(const int32_t* status) {
   bool set = *reinterpret_cast<const volatile int32_t*>(status) != kStatusOk;
-  const int warp = uniform_warp_index();
-  if (warp >= 2 && warp < 2 + kEpiWarps) set = named_barrier_any(1, kEpiWarps * 32, set);
+  if (uniform_warp_index() >= 2) set = named_barrier_any(1, kEpiWarps * 32, set);
   return uniform(set) != 0;
 }
 
