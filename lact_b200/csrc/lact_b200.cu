@@ -2866,12 +2866,14 @@ static SwaPairSplit swa_pair_split(int64_t b, int64_t l, int64_t lk, int64_t hea
   const int64_t band = window > 0 && window < l ? window : l;
   const int64_t span = causal ? std::min<int64_t>(ceil_div(l, 128), ceil_div(band + 255, 128) + 1) : ceil_div(lk > 0 ? lk : l, 128);
   const double per_tile = d == 64 ? 1.5 : 2.0, per_item = 2.5;
-  // the longest CTA's time for the first n items; only where their lengths differ are they looked at one by one
+  // the longest CTA's time for the first n items; only where their lengths differ are they looked at, those of five CTAs (the call waits
+  // for this)
   auto dealt = [&](int64_t n) {
     const int64_t rounds = (n + sms - 1) / sms;
     if (!causal || n <= sms || rounds > 8 || band + 256 <= l / 2) return rounds * (span * per_tile + per_item);
     double worst = 0.0;
-    for (int64_t c = 0; c < sms; ++c) {
+    for (int64_t i = 0; i <= 4; ++i) {
+      const int64_t c = i * (sms - 1) / 4;
       double t = 0.0;
       for (int64_t r = 0; r < rounds; ++r) {
         const int64_t item = r * sms + ((r & 1) ? sms - 1 - c : c);
