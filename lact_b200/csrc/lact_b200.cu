@@ -2898,9 +2898,10 @@ static SwaPairSplit swa_pair_split(int64_t b, int64_t l, int64_t lk, int64_t hea
   }
   return best;
 }
-// Scratch of a cut launch: fewer pieces than cutters and items together, 256 rows each.
+// Scratch of a cut launch: fewer pieces than cutters and items together, 256 rows each, from the caller's next multiple of 32 bytes on
+// (the caller's own has 16, rows are stored 32 bytes at a time).
 static size_t swa_pair_scratch(const SwaPairSplit& sp, int64_t d) {
-  return static_cast<size_t>(sp.cutters + sp.rest) * 256 * (d * sizeof(float) + sizeof(float2));
+  return sp.cutters > 0 ? static_cast<size_t>(sp.cutters + sp.rest) * 256 * (d * sizeof(float) + sizeof(float2)) + 16 : 0;
 }
 // Whether a launch runs on pairs: by the estimates of both.  Measured (us, single tiles / pairs): 12 heads of 128
 // with 4096 queries and a window of 2048 78 / 47, 8 with 16384 206 / 159, 4 with 1024 and 512 14.6 / 18.7, 8 of 64 with 777 queries over
@@ -3003,7 +3004,7 @@ static int swa_fwd_impl(const void* q, const void* k, const void* v, const SwaSe
       p.span = static_cast<int32_t>(sp2.span);
       p.share = static_cast<int32_t>(sp2.rest * sp2.span / sp2.cutters);
       p.longer = static_cast<int32_t>(sp2.rest * sp2.span % sp2.cutters);
-      p.part = static_cast<float*>(scratch);
+      p.part = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(scratch) + 31) & ~static_cast<uintptr_t>(31));
       p.ml = reinterpret_cast<float2*>(p.part + (sp2.cutters + sp2.rest) * 256 * d);
     }
     ctas = std::max<int64_t>(p.cutters, std::min<int64_t>(p.whole, sm_count()));

@@ -50,7 +50,7 @@ struct SwaPairArgs {
   // maxima and sums of its piece of an item in `part` / `ml`, and swa_combine_kernel puts the pieces together.
   // (Pieces in their order step to the next cutter, the next item or both: the sum of the two numbers is a piece's own.)
   int32_t whole, rounds, rest, cutters, span, share, longer;   // rounds: of whole items over the grid
-  float* part;   // [cutter + item - whole][group][128 rows][HD]
+  float* part;   // [cutter + item - whole][group][128 rows][HD], a multiple of 32 bytes
   float2* ml;    // [cutter + item - whole][group][128 rows]: maximum, sum
 };
 

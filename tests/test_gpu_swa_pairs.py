@@ -96,3 +96,43 @@ def test_nothing_is_written_after_an_earlier_failure(l, h, window, cut):
                                        status.data_ptr(), L.stream_ptr()), "swa")
     torch.cuda.synchronize()
     assert bool((o == 7).all()) and bool((lse == 7).all())
+
+
+def _address(nbytes, off, fill):
+    """A buffer and the first address in it that lies `off` bytes behind a multiple of 256."""
+    buf = torch.full((nbytes + 512,), fill, dtype=torch.uint8, device="cuda")
+    return buf, (buf.data_ptr() + 255) // 256 * 256 + off
+
+
+# scratch and outputs as they are promised to be taken: on 16 bytes
+@pytest.mark.parametrize("d,l,lk,h", [(128, 1560, 4680, 12), (64, 1300, 4500, 30)])
+@pytest.mark.parametrize("off", [16, 48])
+def test_addresses_on_16_bytes(d, l, lk, h, off):
+    import ctypes as C
+    from lact_b200 import _lib as L
+    g = torch.Generator(device="cuda").manual_seed(l)
+    rn = lambda n: torch.randn(1, n, h, d, device="cuda", generator=g).to(torch.bfloat16)
+    q, k, v = rn(l), rn(lk), rn(lk)
+    need, words = C.c_size_t(0), C.c_int64(0)
+    L.check(L.lib().lact_swa_fwd_split_bytes(1, l, lk, h, d, -1, C.byref(need), C.byref(words)), "split_bytes")
+    assert need.value > 0 and words.value == 0   # pairs, the last ones cut
+    counters = torch.zeros(64, dtype=torch.int32, device="cuda")
+    status = torch.zeros(64, dtype=torch.int32, device="cuda")
+    got = []
+    for so, oo in ((0, 0), (off, 0), (0, off), (off, off)):
+        scratch, at = _address(need.value, so, 0xFF)
+        out, to = _address(l * h * d * 2, oo, 7)
+        L.check(L.lib().lact_swa_fwd_split(q.data_ptr(), k.data_ptr(), v.data_ptr(), to, 1, l, lk, h, d, *[h * d, h * d * l],
+                                           *[h * d, h * d * lk] * 2, h * d, h * d * l, -1, d ** -0.5, None, None, counters.data_ptr(), at,
+                                           need.value, status.data_ptr(), L.stream_ptr()), "swa")
+        torch.cuda.synchronize()
+        first = to - out.data_ptr()
+        assert bool((out[:first] == 7).all()) and bool((out[first + l * h * d * 2:] == 7).all())
+        end = at - scratch.data_ptr() + need.value
+        assert bool((scratch[:at - scratch.data_ptr()] == 0xFF).all()) and bool((scratch[end:] == 0xFF).all())
+        got.append(out[first:first + l * h * d * 2].view(torch.bfloat16).view(1, l, h, d).clone())
+    assert int(status[0]) == 0
+    assert all(torch.equal(x, got[0]) for x in got[1:])
+    want, _ = _reference(q, k, v, -1)
+    # probabilities and results are rounded to bf16 (2^-9 each)
+    assert float((got[0].double() - want).norm() / want.norm()) <= 6e-3
