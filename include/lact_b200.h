@@ -306,8 +306,8 @@ int lact_swa_fwd(const void *q, const void *k, const void *v, void *o, int64_t b
                  int32_t *status_word, void *stream);
 /* The same with query tiles cut over their keys where whole tiles would leave SMs idle (few of them, or a short last round).
  * lact_swa_fwd_split_bytes: bytes of scratch (16-byte aligned) and uint32 words of counters (zero before every call) it
- * takes; both 0 where nothing is cut, the counters alone where the pieces are put together by a launch of their own.  scratch NULL, or
- * counters NULL where there are any: nothing is cut. */
+ * takes; both 0 where nothing is cut, counters 0 where a second launch puts the pieces together (any address that is not NULL then
+ * stands for them: it is not read).  counters or scratch NULL: nothing is cut. */
 int lact_swa_fwd_split_bytes(int64_t b, int64_t l, int64_t lk, int64_t n_heads, int64_t d, int64_t window, size_t *bytes,
                              int64_t *counters);
 int lact_swa_fwd_split(const void *q, const void *k, const void *v, void *o, int64_t b, int64_t l, int64_t lk, int64_t n_heads,

@@ -2986,7 +2986,7 @@ static int swa_fwd_impl(const void* q, const void* k, const void* v, const SwaSe
   int64_t ctas = b * n_heads * a.q_tiles;
   if (ctas > 0x7FFFFFFFll) return LACT_ERR_SHAPE;
   SwaPairSplit sp2;
-  if (swa_takes_pairs(b, l, lk, n_heads, d, window, scratch != nullptr, &sp2)) {
+  if (swa_takes_pairs(b, l, lk, n_heads, d, window, scratch != nullptr && counters != nullptr, &sp2)) {
     SwaPairArgs p;
     std::memset(&p, 0, sizeof(p));
     p.q = a.q; p.k = a.k; p.v = a.v; p.k2 = a.k2; p.v2 = a.v2;

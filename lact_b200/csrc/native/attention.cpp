@@ -42,9 +42,10 @@ std::vector<Tensor> swa(const Tensor& q_, const Tensor& k_, const Tensor& v_, in
     scratch = bytes(need, q);
     if (words > 0) counters = at::zeros({words}, q.options().dtype(at::kInt).requires_grad(false));
   }
+  void* const room = need > 0 ? ptr(scratch) : nullptr;
   check(lact_swa_fwd_split(ptr(q), ptr(k), ptr(v), ptr(o), b, l, lk, h, d, q.stride(1), q.stride(0), k.stride(1), k.stride(0), v.stride(1),
                      v.stride(0), o.stride(1), o.stride(0), window, static_cast<float>(scale), static_cast<const int32_t*>(ptr(seq)),
-                     ptr(lse), words > 0 ? ptr(counters) : nullptr, need > 0 ? ptr(scratch) : nullptr, need, status_word(q),
+                     ptr(lse), words > 0 ? ptr(counters) : room, room, need, status_word(q),
                      stream_of(q)),
         "lact_swa_fwd");
   return {o, lse};
@@ -64,10 +65,11 @@ Tensor swa_cache(const Tensor& q_, const Tensor& kc_, const Tensor& vc_, const T
     scratch = bytes(need, q);
     if (words > 0) counters = at::zeros({words}, q.options().dtype(at::kInt).requires_grad(false));
   }
+  void* const room = need > 0 ? ptr(scratch) : nullptr;
   const int64_t strides[12] = {q.stride(1), q.stride(0), kc.stride(1), kc.stride(0), vc.stride(1), vc.stride(0),
                                k.stride(1), k.stride(0), v.stride(1),  v.stride(0),  o.stride(1),  o.stride(0)};
   check(lact_swa_fwd_cache(ptr(q), ptr(kc), ptr(vc), ptr(k), ptr(v), ptr(o), b, l, lc, ln, h, d, strides, static_cast<float>(scale),
-                           words > 0 ? ptr(counters) : nullptr, need > 0 ? ptr(scratch) : nullptr, need, status_word(q), stream_of(q)),
+                           words > 0 ? ptr(counters) : room, room, need, status_word(q), stream_of(q)),
         "lact_swa_fwd_cache");
   return o;
 }

@@ -89,11 +89,12 @@ def test_nothing_is_written_after_an_earlier_failure(l, h, window, cut):
     need, words = C.c_size_t(0), C.c_int64(0)
     L.check(L.lib().lact_swa_fwd_split_bytes(b, l, l, h, d, window, C.byref(need), C.byref(words)), "split_bytes")
     scratch = torch.zeros(max(need.value, 256), dtype=torch.uint8, device="cuda")
+    counters = torch.zeros(max(words.value, 1), dtype=torch.int32, device="cuda")
     status = torch.zeros(64, dtype=torch.int32, device="cuda")
     status[0] = 101
     L.check(L.lib().lact_swa_fwd_split(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), b, l, l, h, d, *[h * d, h * d * l] * 4, window,
-                                       d ** -0.5, None, lse.data_ptr(), None, scratch.data_ptr() if cut else None, need.value,
-                                       status.data_ptr(), L.stream_ptr()), "swa")
+                                       d ** -0.5, None, lse.data_ptr(), counters.data_ptr() if cut else None,
+                                       scratch.data_ptr() if cut else None, need.value, status.data_ptr(), L.stream_ptr()), "swa")
     torch.cuda.synchronize()
     assert bool((o == 7).all()) and bool((lse == 7).all())
 
@@ -136,3 +137,22 @@ def test_addresses_on_16_bytes(d, l, lk, h, off):
     want, _ = _reference(q, k, v, -1)
     # probabilities and results are rounded to bf16 (2^-9 each)
     assert float((got[0].double() - want).norm() / want.norm()) <= 6e-3
+
+
+@pytest.mark.parametrize("l,lk,h,d", [(1560, 4680, 12, 128), (1300, 4500, 30, 64)])
+@pytest.mark.parametrize("scratch,counters", [(True, False), (False, True), (False, False)])
+def test_scratch_or_counters_alone_cut_nothing(l, lk, h, d, scratch, counters):
+    """Either of them NULL: the call does without both, whatever size is given for the scratch."""
+    from lact_b200 import _lib as L
+    g = torch.Generator(device="cuda").manual_seed(l)
+    rn = lambda n: torch.randn(1, n, h, d, device="cuda", generator=g).to(torch.bfloat16)
+    q, k, v = rn(l), rn(lk), rn(lk)
+    o, buf, words = torch.empty_like(q), torch.full((256,), 0xFF, dtype=torch.uint8, device="cuda"), torch.full((64,), 3, device="cuda")
+    status = torch.zeros(64, dtype=torch.int32, device="cuda")
+    L.check(L.lib().lact_swa_fwd_split(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), 1, l, lk, h, d, h * d, h * d * l,
+                                       *[h * d, h * d * lk] * 2, h * d, h * d * l, -1, d ** -0.5, None, None,
+                                       words.data_ptr() if counters else None, buf.data_ptr() if scratch else None, 0, status.data_ptr(),
+                                       L.stream_ptr()), "swa")
+    torch.cuda.synchronize()
+    assert int(status[0]) == 0 and bool((buf == 0xFF).all()) and bool((words == 3).all())
+    assert torch.equal(o, _run(L, q, k, v, -1, False)[0])
