@@ -420,6 +420,7 @@ __global__ void __launch_bounds__(kSwaPairThreads, 1) swa_pairs_kernel(const __g
           };
           if (w.piece < 0) {
             const float inv = finish_row();
+            __syncwarp();   // (rows past the end have stored nothing)
 #pragma unroll 1
             for (int c = 0; c < HD; c += 32) {
               float v[32];

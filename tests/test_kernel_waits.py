@@ -89,3 +89,9 @@ def test_whether_to_take_part_is_decided_once_per_cta(name):
 def test_the_epilogue_warps_decide_at_a_barrier():
     body = re.search(r"bool earlier_launch_failed\(.*?\n}", _source("umma_gemm.cuh"), re.S).group(0)
     assert "if (uniform_warp_index() >= 2) set = named_barrier_any(" in body
+
+
+def test_a_warp_meets_again_before_aligned_loads_of_tensor_memory():
+    """Attention on pairs: the log-sum-exp is stored by the rows below the end alone, the loads behind it want the whole warp."""
+    between = re.search(r"inv = finish_row\(\);(.*?)own\(c, v\);", _source("swa_pairs.cuh"), re.S).group(1)
+    assert "__syncwarp();" in between
