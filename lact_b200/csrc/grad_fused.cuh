@@ -215,6 +215,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGradThreads, 1) gra
       __syncwarp();
       if (lane == 0) mbar_arrive(&y_empty[s]);
       Op::pointwise<16>(a.lr, v, o, pf);
+      // rows past the end are zeros in both contractions (0 times a weight that is not finite is none)
+      if (__builtin_expect(i * 128 + r >= a.len, 0)) {
+#pragma unroll
+        for (int p = 0; p < 3; ++p)
+#pragma unroll
+          for (int j = 0; j < 16; ++j) o[p][j] = 0.f;
+      }
       if (i > 0 && !mbar_wait_warp(planes_empty, (i - 1) & 1, abort_flag)) { failed = true; break; }
       // dy0, dy2: halves of rows of 128 bytes; hidden: rows of 64 bytes
       const uint32_t dy = base + SM::kDy + r * 128, hid = base + SM::kHid + r * 64;

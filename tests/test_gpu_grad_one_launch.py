@@ -74,3 +74,22 @@ def test_tokens_before_the_range_and_strided_rows():
     lb.synchronize_and_check()
     for x, y, z in zip(views, copies, alone):
         assert torch.equal(x, y) and torch.equal(x[3:4], z)
+
+
+# rows past the end of the last tile: their k and v are zeros, and zero times infinity is not
+@pytest.mark.parametrize("n", [2049, 2111, 2177, 2304])
+@pytest.mark.parametrize("h", [128, 256])
+def test_infinite_weights(n, h):
+    import lact_b200 as lb
+    w, (_, k, v), lrs, _, _ = _inputs(16, n, h, torch.float32, seed=n)
+    w02, w1, k, v = torch.cat([w[0], w[2]], 1).bfloat16(), w[1].bfloat16(), k.abs().clamp(min=2.0 ** -10), v.abs().clamp(min=2.0 ** -10)   # (no exact zeros)
+    w02[:, 7] = w02[:, 7].abs()
+    w1[:, 5, 7] = float("inf")      # dh of hidden feature 7 is +inf for every token, and so is dy2
+    w02[:, h + 9, 3] = float("inf")   # y2 of hidden feature 9
+    run = lambda s: lb.fused_lact_swiglu_ffn_fast_weight_grads(w02[s], w1[s], k[s], v[s], *[t[s, :, 0].contiguous() for t in lrs])
+    both = run(slice(None))
+    lb.synchronize_and_check()
+    assert bool((both[0][:, h + 7] == float("inf")).all())
+    for e in (0, 15):
+        for x, y in zip(both, run(slice(e, e + 1))):
+            assert torch.equal(x[e:e + 1].isnan(), y.isnan()) and torch.equal(x[e:e + 1].nan_to_num(), y.nan_to_num())
