@@ -2830,32 +2830,52 @@ struct SwaSplit {
   int splits;
   double us;
 };
+// Estimates of both attention forwards, which swa_takes_pairs compares.  An SM spends `tile` us per key tile and `item` per query tile or
+// pair, fitted to 255 shapes (32 to 32768 queries, windows of 100 to none, caches up to 16384 keys, d = 64 and 128) that were timed on both
+// kernels: the faster one is chosen in all but 3, within 1.18 there.
+struct SwaCost {
+  double tile, item;
+};
+static SwaCost swa_single_cost(int64_t d) { return d == 64 ? SwaCost{1.28, 4.9} : SwaCost{1.4, 6.7}; }
+static SwaCost swa_pair_cost(int64_t d) { return d == 64 ? SwaCost{1.75, 2.0} : SwaCost{2.1, 3.0}; }
+// Causal attention: the first key tile that query tile i meets is i - swa_behind, or 0.
+static int64_t swa_band(int64_t l, int64_t window) { return window > 0 && window < l ? window : l; }
+static int64_t swa_behind(int64_t l, int64_t window) { return ceil_div(swa_band(l, window) - 1, 128); }
+
 static SwaSplit swa_split(int64_t b, int64_t l, int64_t lk, int64_t heads, int64_t d, int64_t window, bool may_cut) {
-  const int64_t sms = sm_count(), tiles = b * heads * ceil_div(l, 128);
+  const int64_t sms = sm_count(), n = ceil_div(l, 128), tiles = b * heads * n;
   const int64_t span = window < 0 ? (lk > 0 ? lk : l) : window > 0 && window < l ? std::min(l, window + 127) : l;
   const int64_t T = ceil_div(span, 128), rest = tiles % sms;
   const double per_tile = d == 64 ? 1.2 : 1.5, round = T * per_tile + 4.0;
-  // (tiles of causal attention without a window are half as long on the average, and the SMs take them as they come)
-  const bool even = window < 0 || (window > 0 && 2 * window <= l);
-  const double rounds = even || tiles <= sms ? static_cast<double>((tiles + sms - 1) / sms) : std::max(1.0, 0.6 * tiles / sms);
-  SwaSplit best{tiles, 1, rounds * round};
+  // Whole tiles: rounds of equal ones; causal ones differ in length, are taken as SMs come free, and the last of them are the long ones of
+  // a head: an equal share of the work and 0.4 of the longest.
+  const SwaCost cost = swa_single_cost(d);
+  const double longest = T * cost.tile + cost.item;
+  double share = 0.0;
+  if (window >= 0) {
+    const int64_t c = swa_behind(l, window), keys = n * (n + 1) / 2 - (n > c ? (n - c) * (n - c - 1) / 2 : 0);
+    share = static_cast<double>(b * heads) * (keys * cost.tile + n * cost.item) / sms;
+  }
+  SwaSplit best{tiles, 1, window < 0 || tiles <= sms ? ((tiles + sms - 1) / sms) * longest : std::max(longest, share + 0.4 * longest)};
   if (!may_cut || rest == 0 || tiles > 64 * sms) return best;
-  double cost = round;
+  double end = round;   // of the rest
   for (int s = 2; s <= 16 && s <= T; ++s) {
-    const double c = ((rest * s + sms - 1) / sms) * (((T + s - 1) / s) * per_tile + 4.0) + 2.0 + 0.6 * s;
-    if (c < 0.9 * cost) {
-      cost = c;
-      best = SwaSplit{tiles - rest, s, (even ? static_cast<double>(tiles / sms) : std::max(tiles >= sms ? 1.0 : 0.0, 0.6 * (tiles - rest) / sms)) * round + c};
+    const int64_t turns = (rest * s + sms - 1) / sms, keys = (T + s - 1) / s;
+    const double c = turns * (keys * per_tile + 4.0) + 2.0 + 0.6 * s;
+    if (c < 0.9 * end) {
+      end = c;
+      const double us = turns * (keys * cost.tile + cost.item) + 2.0 + 0.6 * s;
+      best = SwaSplit{tiles - rest, s, tiles < sms ? us : window < 0 ? (tiles / sms) * longest + us : std::max(longest, share + 0.5 * us)};
     }
   }
   return best;
 }
 
 // The same launch on pairs of query tiles (see SwaPairArgs).  Whole pairs fill whole rounds of the SMs; the rest, all pairs where there are
-// fewer than SMs, are cut over their keys if the longest CTA then ends sooner: 2.5 us per pair or piece plus 2.0 us per key tile (1.5
-// at d = 64), a second launch that puts the pieces together and what it waits for 13.  Measured: 1560 queries over 4680 keys, 12 heads of
-// 128 (84 pairs on 148 SMs, 38 key tiles each) whole 84, cut 72 us.  Pairs of causal attention without a window differ in length and
-// are dealt the long ones first: 8 heads of 8192 queries (256 pairs) are left whole, 133 us, 221 with the 108 shortest cut.
+// fewer than SMs, are cut over their keys if the longest CTA then ends sooner.  A second launch puts the pieces together: it, what it
+// waits for and the pieces' rows take 2 us and 0.08 per piece (60 pieces 6, 232 pieces 20).  Measured: 1560 queries over 4680 keys, 12
+// heads of 128 (84 pairs on 148 SMs, 38 key tiles each) whole 86, cut 73 us.  Pairs of causal attention without a window differ in length and
+// are dealt the long ones first: 8 heads of 8192 queries (256 pairs) are left whole, 134 us, 221 with the 108 shortest cut.
 struct SwaPairSplit {
   int64_t whole, rest, cutters, span;   // cutters = 0: nothing is cut (and rest = 0)
   double us;
@@ -2863,23 +2883,34 @@ struct SwaPairSplit {
 static SwaPairSplit swa_pair_split(int64_t b, int64_t l, int64_t lk, int64_t heads, int64_t d, int64_t window, bool may_cut) {
   const int64_t sms = sm_count(), bh = b * heads, pairs = ceil_div(l, 256), items = bh * pairs;
   const bool causal = window >= 0;
-  const int64_t band = window > 0 && window < l ? window : l;
-  const int64_t span = causal ? std::min<int64_t>(ceil_div(l, 128), ceil_div(band + 255, 128) + 1) : ceil_div(lk > 0 ? lk : l, 128);
-  const double per_tile = d == 64 ? 1.5 : 2.0, per_item = 2.5;
-  // the longest CTA's time for the first n items; only where their lengths differ are they looked at, those of five CTAs (the call waits
-  // for this)
-  auto dealt = [&](int64_t n) {
+  const int64_t behind = swa_behind(l, window);
+  // key tiles of an item, at most (what is cut is laid out by it: none may have more)
+  const int64_t span = causal ? std::min<int64_t>(ceil_div(l, 128), behind + 2) : ceil_div(lk > 0 ? lk : l, 128);
+  const SwaCost cost = swa_pair_cost(d);
+  const double longest = span * cost.tile + cost.item;
+  // key tiles of pair p and of all pairs before it (of the last pair's second tile there may be no rows)
+  auto keys = [&](int64_t p) { return 2 * (p + 1) - std::max<int64_t>(0, 2 * p - behind) - (p + 1 == pairs ? ceil_div(l, 128) % 2 : 0); };
+  auto keys_before = [&](int64_t p) {
+    const int64_t m = (behind + 1) / 2;
+    return p * (p + 1) - (p > m ? (p - m) * (p + m - 1 - behind) : 0);
+  };
+  // The longest CTA's time for the first n items.  Where their lengths differ: up to eight rounds by those of five CTAs (the call waits for
+  // this), beyond by an equal share of the work and a quarter of the longest item.
+  auto dealt = [&](int64_t n) -> double {
     const int64_t rounds = (n + sms - 1) / sms;
-    if (!causal || n <= sms || rounds > 8 || band + 256 <= l / 2) return rounds * (span * per_tile + per_item);
+    if (!causal || n <= sms) return rounds * longest;
+    if (rounds > 8) {
+      const int64_t full = n / bh, part = n % bh;
+      const int64_t all = bh * (keys_before(pairs) - ceil_div(l, 128) % 2 - keys_before(pairs - full)) + (part > 0 ? part * keys(pairs - 1 - full) : 0);
+      return (all * cost.tile + n * cost.item) / sms + 0.25 * longest;
+    }
     double worst = 0.0;
     for (int64_t i = 0; i <= 4; ++i) {
       const int64_t c = i * (sms - 1) / 4;
       double t = 0.0;
       for (int64_t r = 0; r < rounds; ++r) {
         const int64_t item = r * sms + ((r & 1) ? sms - 1 - c : c);
-        if (item >= n) continue;
-        const int64_t q0 = (pairs - 1 - item / bh) * 256;
-        t += (ceil_div(std::min(q0 + 256, l), 128) - std::max<int64_t>(q0 - (band - 1), 0) / 128) * per_tile + per_item;
+        if (item < n) t += keys(pairs - 1 - item / bh) * cost.tile + cost.item;
       }
       worst = std::max(worst, t);
     }
@@ -2888,12 +2919,12 @@ static SwaPairSplit swa_pair_split(int64_t b, int64_t l, int64_t lk, int64_t hea
   SwaPairSplit best{items, 0, 0, 0, dealt(items) + 2.0};
   const int64_t rest = items % sms;
   if (!may_cut || rest == 0 || items > 64 * sms) return best;
-  const double before = dealt(items - rest) + 13.0 + 2 * per_item;
+  const double before = dealt(items - rest) + 2 * cost.item + 4.0;
   for (int64_t s = 2, last = 0; s <= 16; s += 1 + s / 4) {
     const int64_t cutters = std::min(rest * std::min(s, span), sms);
     if (cutters == last) break;
     last = cutters;
-    const double us = before + ceil_div(rest * span, cutters) * per_tile;
+    const double us = before + ceil_div(rest * span, cutters) * cost.tile + 0.08 * (cutters + rest);
     if (us < 0.95 * best.us) best = SwaPairSplit{items - rest, rest, cutters, span, us};
   }
   return best;
@@ -2903,12 +2934,14 @@ static SwaPairSplit swa_pair_split(int64_t b, int64_t l, int64_t lk, int64_t hea
 static size_t swa_pair_scratch(const SwaPairSplit& sp, int64_t d) {
   return sp.cutters > 0 ? static_cast<size_t>(sp.cutters + sp.rest) * 256 * (d * sizeof(float) + sizeof(float2)) + 16 : 0;
 }
-// Whether a launch runs on pairs: by the estimates of both.  Measured (us, single tiles / pairs): 12 heads of 128
-// with 4096 queries and a window of 2048 78 / 47, 8 with 16384 206 / 159, 4 with 1024 and 512 14.6 / 18.7, 8 of 64 with 777 queries over
-// 2777 keys 26 / 32.
+// Whether a launch runs on pairs: by the estimates of both.  Measured (us, single tiles / pairs; heads of 128 unless stated): 4 x 8192 queries,
+// 12 heads, no window 1084 / 769; 16 x 2048 392 / 246, of 64 325 / 184; 12 heads, 32768 queries of packed sequences of 256 under a window of
+// 2048 182 / 75, of 2048 387 / 317; 128 entries of 256 queries 176 / 73; 4096 queries, window 1024 57 / 46.  Few or uneven items lose: 12
+// heads of 1024 queries, window 256 12.6 / 15.8; 8 heads of 2305, window 2048 32 / 46; 4 heads of 8192 121 / 134; 8 of 64 with 777 queries
+// over 2777 keys 28 / 30.  What a launch would not meet (sequences packed into its entry) is not looked at.
 static bool swa_takes_pairs(int64_t b, int64_t l, int64_t lk, int64_t heads, int64_t d, int64_t window, bool may_cut, SwaPairSplit* pairs) {
   *pairs = swa_pair_split(b, l, lk, heads, d, window, may_cut);
-  return pairs->us < swa_split(b, l, lk, heads, d, window, may_cut).us;
+  return pairs->us < 0.98 * swa_split(b, l, lk, heads, d, window, may_cut).us;   // (a tie: single tiles)
 }
 
 int lact_swa_fwd_split_bytes(int64_t b, int64_t l, int64_t lk, int64_t n_heads, int64_t d, int64_t window, size_t* bytes,

@@ -8,6 +8,16 @@ from test_gpu_swa_split import _run
 pytestmark = pytest.mark.gpu
 
 
+def _kernels(call):
+    """The attention kernels that a call launches."""
+    from torch.profiler import ProfilerActivity, profile
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        call()
+        torch.cuda.synchronize()
+    which = {"swa_pairs_kernel": "pairs", "swa_combine_kernel": "combine", "swa_fwd_kernel": "single"}
+    return {which[k] for k in which for e in p.events() if k in e.name}
+
+
 def _reference(q, k, v, window, starts=None):
     l, lk, d = q.shape[1], k.shape[1], q.shape[-1]
     qf, kf, vf = (t.double().transpose(1, 2) for t in (q, k, v))
@@ -156,3 +166,15 @@ def test_scratch_or_counters_alone_cut_nothing(l, lk, h, d, scratch, counters):
     torch.cuda.synchronize()
     assert int(status[0]) == 0 and bool((buf == 0xFF).all()) and bool((words == 3).all())
     assert torch.equal(o, _run(L, q, k, v, -1, False)[0])
+
+
+# many items of uneven length, more than eight rounds of them and fewer, few items: the way that is the faster one (both measured)
+@pytest.mark.parametrize("b,l,h,d,window,way", [(4, 8192, 12, 128, None, "pairs"), (16, 2048, 12, 128, 2048, "pairs"), (16, 2048, 12, 64, None, "pairs"),
+                                                (8, 4096, 12, 128, 3000, "pairs"), (2, 2048, 12, 128, 256, "pairs"), (40, 200, 12, 128, None, "pairs"),
+                                                (1, 3626, 12, 128, 1024, "pairs"), (1, 8192, 8, 128, None, "pairs"),
+                                                (1, 2305, 8, 128, 2048, "single"), (1, 1024, 12, 128, 256, "single"), (1, 8192, 4, 128, None, "single")])
+def test_the_faster_way(b, l, h, d, window, way):
+    from lact_b200 import layer_ops as lo
+    q, k, v = (torch.randn(b, l, h, d, device="cuda", dtype=torch.bfloat16) for _ in range(3))
+    with torch.no_grad():
+        assert _kernels(lambda: lo.sliding_window_attention(q, k, v, window)) == {way}
