@@ -99,12 +99,11 @@ def test_nothing_is_written_after_an_earlier_failure(l, h, window, cut):
     need, words = C.c_size_t(0), C.c_int64(0)
     L.check(L.lib().lact_swa_fwd_split_bytes(b, l, l, h, d, window, C.byref(need), C.byref(words)), "split_bytes")
     scratch = torch.zeros(max(need.value, 256), dtype=torch.uint8, device="cuda")
-    counters = torch.zeros(max(words.value, 1), dtype=torch.int32, device="cuda")
     status = torch.zeros(64, dtype=torch.int32, device="cuda")
     status[0] = 101
     L.check(L.lib().lact_swa_fwd_split(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), b, l, l, h, d, *[h * d, h * d * l] * 4, window,
-                                       d ** -0.5, None, lse.data_ptr(), counters.data_ptr() if cut else None,
-                                       scratch.data_ptr() if cut else None, need.value, status.data_ptr(), L.stream_ptr()), "swa")
+                                       d ** -0.5, None, lse.data_ptr(), None, scratch.data_ptr() if cut else None, need.value,
+                                       status.data_ptr(), L.stream_ptr()), "swa")
     torch.cuda.synchronize()
     assert bool((o == 7).all()) and bool((lse == 7).all())
 
@@ -178,3 +177,71 @@ def test_the_faster_way(b, l, h, d, window, way):
     q, k, v = (torch.randn(b, l, h, d, device="cuda", dtype=torch.bfloat16) for _ in range(3))
     with torch.no_grad():
         assert _kernels(lambda: lo.sliding_window_attention(q, k, v, window)) == {way}
+
+
+PAIRS = {"pairs"}
+CUT = {"pairs", "combine"}
+
+
+# which kernel the calls of this file are compared on.  Uncut: every remainder of a pair at which its second tile or a tile's last rows are
+# missing; block attention; packed sequences.  Cut: the last items of a causal launch and of block attention, all items, with and without sequences
+@pytest.mark.parametrize("b,l,lk,h,d,window,cuts,way", [
+    *[(1, l, l, 300, d, w, (), PAIRS) for d in (64, 128) for l, w in ((1, 0), (127, 40), (128, 128), (129, 1), (255, 0), (256, 128), (257, 129),
+                                                                     (385, 256), (511, 130), (513, 600))],
+    *[(1, l, 700, 148, 128, -1, (), PAIRS) for l in (129, 255, 257)], (1, 300, 1025, 148, 64, -1, (), PAIRS),
+    (1, 1100, 1100, 40, 128, 0, (), PAIRS), (1, 257, 257, 74, 64, 200, (), PAIRS), (3, 130, 127, 30, 64, -1, (), PAIRS),
+    (1, 900, 900, 100, 64, 0, (), PAIRS), (1, 1100, 1100, 60, 128, 300, (255, 257, 1000), PAIRS), (1, 300, 300, 200, 128, 0, (), PAIRS),
+    (1, 2600, 2500, 14, 128, -1, (), CUT), (2, 1900, 2600, 10, 64, -1, (), CUT), (1, 5000, 5000, 2, 128, 0, (), CUT),
+    (1, 4100, 4100, 3, 128, 0, (1, 2, 383, 4099), CUT), (1, 3626, 3626, 3, 64, 0, (128, 1000, 3073), CUT), (1, 4100, 4100, 3, 64, 4096, (), CUT)])
+def test_the_kernel_that_is_compared(b, l, lk, h, d, window, cuts, way):
+    from lact_b200 import _lib as L
+    g = torch.Generator(device="cuda").manual_seed(l + h + d)
+    rn = lambda n: torch.randn(b, n, h, d, device="cuda", generator=g).to(torch.bfloat16)
+    q, k, v = rn(l), rn(lk), rn(lk)
+    starts = None
+    if cuts:
+        starts = torch.zeros(l, dtype=torch.int32, device="cuda")
+        for c in cuts:
+            starts[c:] = c
+    _compare(q, k, v, window, way == CUT, starts)
+    assert _kernels(lambda: _run(L, q, k, v, window, way == CUT, starts)) == way
+
+
+# keys in two runs on pairs that are cut over both: the first ends on a tile's end, just past one, inside one
+@pytest.mark.parametrize("cached", [3120, 3072, 3073, 2999])
+@pytest.mark.parametrize("l,new,h,d", [(1560, 1560, 12, 128), (1300, 1400, 30, 64)])
+def test_cut_over_a_cache_and_new_keys(l, cached, new, h, d):
+    from lact_b200 import layer_ops as lo
+    g = torch.Generator(device="cuda").manual_seed(cached)
+    rn = lambda *s: torch.randn(*s, h, d, device="cuda", generator=g).to(torch.bfloat16)
+    q, k, v, cache = rn(1, l), rn(1, new), rn(1, new), rn(2, cached)
+    call = lambda: lo.sliding_window_attention_inference(q, k, v, new, kv_cache=cache)
+    o = call()
+    assert _kernels(call) == CUT
+    want, _ = _reference(q, torch.cat([cache[:1], k], 1), torch.cat([cache[1:], v], 1), -1)
+    # probabilities and results are rounded to bf16 (2^-9 each)
+    assert float((o.double() - want).norm() / want.norm()) <= 6e-3
+
+
+@pytest.mark.parametrize("l,lk,h,window,way", [(300, 300, 200, 0, PAIRS), (1560, 4680, 12, -1, CUT), (5000, 5000, 2, 0, CUT)])
+def test_pairs_after_an_earlier_failure(l, lk, h, window, way):
+    """Outputs and the status word stay what they were."""
+    import ctypes as C
+    from lact_b200 import _lib as L
+    d = 128
+    rn = lambda n: torch.randn(1, n, h, d, device="cuda").to(torch.bfloat16)
+    q, k, v = rn(l), rn(lk), rn(lk)
+    o, lse = torch.full_like(q, 7.0), torch.full((1, h, l), 7.0, device="cuda")
+    need, words = C.c_size_t(0), C.c_int64(0)
+    L.check(L.lib().lact_swa_fwd_split_bytes(1, l, lk, h, d, window, C.byref(need), C.byref(words)), "split_bytes")
+    assert (need.value > 0) == (way == CUT) and words.value == 0
+    scratch = torch.zeros(max(need.value, 256), dtype=torch.uint8, device="cuda")
+    counters = torch.zeros(1, dtype=torch.int32, device="cuda")
+    status = torch.zeros(64, dtype=torch.int32, device="cuda")
+    status[0] = 101
+    call = lambda: L.check(L.lib().lact_swa_fwd_split(
+        q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), 1, l, lk, h, d, h * d, h * d * l, *[h * d, h * d * lk] * 2, h * d, h * d * l,
+        window, d ** -0.5, None, lse.data_ptr(), counters.data_ptr() if way == CUT else None, scratch.data_ptr() if way == CUT else None,
+        need.value, status.data_ptr(), L.stream_ptr()), "swa")
+    assert _kernels(call) == way
+    assert bool((o == 7).all()) and bool((lse == 7).all()) and int(status[0]) == 101
