@@ -93,3 +93,57 @@ def test_infinite_weights(n, h):
     for e in (0, 15):
         for x, y in zip(both, run(slice(e, e + 1))):
             assert torch.equal(x[e:e + 1].isnan(), y.isnan()) and torch.equal(x[e:e + 1].nan_to_num(), y.nan_to_num())
+
+
+def _launches(call):
+    """The kernels of the gradient that a call launches: "one" for both stages, "pointwise" and "contract" for one each."""
+    from torch.profiler import ProfilerActivity, profile
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        call()
+        torch.cuda.synchronize()
+    which = {"grad_gemm_kernel": "one", "OpFwGradPointwise": "pointwise", "OpDW": "contract"}
+    return sorted(which[k] for e in p.events() for k in which if k in e.name)
+
+
+def _grads(w, qkv, lrs):
+    import lact_b200 as lb
+    w02, w1 = torch.cat([w[0], w[2]], 1).bfloat16(), w[1].bfloat16()
+    lrs = [t[..., 0].contiguous() for t in lrs]
+    return lb.fused_lact_swiglu_ffn_fast_weight_grads(w02, w1, qkv[1], qkv[2], *lrs)
+
+
+# what is compared in this file: a batch that takes one launch, a few of its entries that take two.  More CTAs than SMs (clusters in a second
+# round, full and nearly empty), as many clusters as fit, the most tokens that sixteen entries take in one launch
+@pytest.mark.parametrize("b,n,h", [(32, 2048, 256), (40, 2177, 128), (24, 2300, 256), (16, 4000, 256), (64, 2049, 256), (37, 2111, 128),
+                                   (16, 2048, 128), (16, 2300, 128)])
+def test_one_launch_against_two(b, n, h):
+    import lact_b200 as lb
+    w, qkv, lrs, _, _ = _inputs(b, n, h, torch.float32, seed=b + n)
+    both = _grads(w, qkv, lrs)
+    assert _launches(lambda: _grads(w, qkv, lrs)) == ["one"]
+    for e in (0, b // 2, b - 1):
+        at = lambda ts: [t[e:e + 1].contiguous() for t in ts]
+        alone = _grads(at(w), at(qkv), at(lrs))
+        for x, y in zip(both, alone):
+            assert torch.equal(x[e:e + 1], y)
+    assert _launches(lambda: _grads(at(w), at(qkv), at(lrs))) == ["contract", "pointwise"]
+    lb.synchronize_and_check()
+
+
+# with momentum and Newton-Schulz, whose norms the launch leaves behind as partial sums: the second round of clusters too
+@pytest.mark.parametrize("b,n,h", [(32, 2177, 256), (40, 2048, 128), (16, 4000, 256)])
+def test_a_whole_update_with_more_ctas_than_sms(b, n, h):
+    w, qkv, lrs, gate, m = _inputs(b, n, h, torch.float32, seed=n)
+    both = _step(w, qkv, lrs, gate, m, True)
+    assert "one" in _launches(lambda: _step(w, qkv, lrs, gate, m, True))
+    for e in (0, b // 2, b - 1):
+        one = lambda ts: [t[e:e + 1].contiguous() for t in ts]
+        _same([t[e:e + 1] for t in both], _step(one(w), one(qkv), one(lrs), gate[e:e + 1].contiguous(), one(m), True))
+
+
+# few tokens: one launch on the side with few, two on the side with many
+@pytest.mark.parametrize("n,ways", [(1, ["one"]), (128, ["one"]), (385, ["one"]), (2300, ["contract", "pointwise"])])
+@pytest.mark.parametrize("h", [128, 256, 384])
+def test_the_way_of_one_entry(n, ways, h):
+    w, qkv, lrs, _, _ = _inputs(1, n, h, torch.float32)
+    assert _launches(lambda: _grads(w, qkv, lrs)) == ways
