@@ -126,3 +126,15 @@ def test_after_an_earlier_failure_nothing_is_written():
     assert _on_pairs(lambda: _products(w02, w1, k, v, lr, word(0))) == {"gate", "down", "pointwise"}
     status = word(101)
     assert all(bool((t == -7).all()) for t in _products(w02, w1, k, v, lr, status)) and int(status[0]) == 101
+
+
+@pytest.mark.parametrize("b,d,h,n,_", SINGLE)
+def test_a_pointwise_stage_that_pairs_would_slow_down(b, d, h, n, _):
+    """The stage by itself: a gradient of heads of 128 features may run as one launch without it."""
+    from lact_b200 import _lib as L
+    w02, w1, k, v, lr = _inputs(b, d, h, n, n + 2)
+    dy, hid, status = torch.empty(b, n, 2 * h, device="cuda").bfloat16(), torch.empty(b, n, h, device="cuda").bfloat16(), torch.zeros(64, dtype=torch.int32, device="cuda")
+    call = lambda: L.check(L.lib().lact_fw_grad_pointwise(w02.data_ptr(), w1.data_ptr(), k.data_ptr(), 3 * d, 3 * d * n, v.data_ptr(), 3 * d, 3 * d * n,
+                                                          *[t.data_ptr() for t in lr], 0, n, 0.5, dy.data_ptr(), hid.data_ptr(), b, n, d, h,
+                                                          status.data_ptr(), L.stream_ptr()), "pointwise")
+    assert _on_pairs(call) == set() and int(status[0]) == 0
