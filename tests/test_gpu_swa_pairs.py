@@ -3,6 +3,7 @@ SMs and the cut of the last ones have their edges."""
 import pytest
 import torch
 
+from launched_kernels import kernels
 from test_gpu_swa_split import _run
 
 pytestmark = pytest.mark.gpu
@@ -10,12 +11,27 @@ pytestmark = pytest.mark.gpu
 
 def _kernels(call):
     """The attention kernels that a call launches."""
-    from torch.profiler import ProfilerActivity, profile
-    with profile(activities=[ProfilerActivity.CUDA]) as p:
-        call()
-        torch.cuda.synchronize()
-    which = {"swa_pairs_kernel": "pairs", "swa_combine_kernel": "combine", "swa_fwd_kernel": "single"}
-    return {which[k] for k in which for e in p.events() if k in e.name}
+    return set(kernels(call, {"swa_pairs_kernel": "pairs", "swa_combine_kernel": "combine", "swa_fwd_kernel": "single"}))
+
+
+def _prepared(q, k, v, window, cut, starts=None, failed=False):
+    """A call of the C interface with all that it takes in hand; outputs filled with 7, and its status word."""
+    import ctypes as C
+    from lact_b200 import _lib as L
+    b, l, h, d = q.shape
+    lk = k.shape[1]
+    o, lse = torch.full_like(q, 7.0), torch.full((b, h, l), 7.0, device="cuda")
+    need, words = C.c_size_t(0), C.c_int64(0)
+    L.check(L.lib().lact_swa_fwd_split_bytes(b, l, lk, h, d, window, C.byref(need), C.byref(words)), "split_bytes")
+    scratch = torch.full((max(need.value, 256),), 0xFF, dtype=torch.uint8, device="cuda")
+    counters = torch.zeros(max(words.value, 1), dtype=torch.int32, device="cuda")
+    status = torch.zeros(64, dtype=torch.int32, device="cuda")
+    status[0] = 101 if failed else 0
+    call = lambda: L.check(L.lib().lact_swa_fwd_split(
+        q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), b, l, lk, h, d, h * d, h * d * l, *[h * d, h * d * lk] * 2, h * d, h * d * l,
+        window, d ** -0.5, starts.data_ptr() if starts is not None else None, lse.data_ptr(), counters.data_ptr() if cut else None,
+        scratch.data_ptr() if cut else None, need.value, status.data_ptr(), L.stream_ptr()), "swa")
+    return call, o, lse, status
 
 
 def _reference(q, k, v, window, starts=None):
@@ -194,7 +210,6 @@ CUT = {"pairs", "combine"}
     (1, 2600, 2500, 14, 128, -1, (), CUT), (2, 1900, 2600, 10, 64, -1, (), CUT), (1, 5000, 5000, 2, 128, 0, (), CUT),
     (1, 4100, 4100, 3, 128, 0, (1, 2, 383, 4099), CUT), (1, 3626, 3626, 3, 64, 0, (128, 1000, 3073), CUT), (1, 4100, 4100, 3, 64, 4096, (), CUT)])
 def test_the_kernel_that_is_compared(b, l, lk, h, d, window, cuts, way):
-    from lact_b200 import _lib as L
     g = torch.Generator(device="cuda").manual_seed(l + h + d)
     rn = lambda n: torch.randn(b, n, h, d, device="cuda", generator=g).to(torch.bfloat16)
     q, k, v = rn(l), rn(lk), rn(lk)
@@ -204,7 +219,7 @@ def test_the_kernel_that_is_compared(b, l, lk, h, d, window, cuts, way):
         for c in cuts:
             starts[c:] = c
     _compare(q, k, v, window, way == CUT, starts)
-    assert _kernels(lambda: _run(L, q, k, v, window, way == CUT, starts)) == way
+    assert _kernels(_prepared(q, k, v, window, way == CUT, starts)[0]) == way
 
 
 # keys in two runs on pairs that are cut over both: the first ends on a tile's end, just past one, inside one
@@ -226,22 +241,7 @@ def test_cut_over_a_cache_and_new_keys(l, cached, new, h, d):
 @pytest.mark.parametrize("l,lk,h,window,way", [(300, 300, 200, 0, PAIRS), (1560, 4680, 12, -1, CUT), (5000, 5000, 2, 0, CUT)])
 def test_pairs_after_an_earlier_failure(l, lk, h, window, way):
     """Outputs and the status word stay what they were."""
-    import ctypes as C
-    from lact_b200 import _lib as L
-    d = 128
-    rn = lambda n: torch.randn(1, n, h, d, device="cuda").to(torch.bfloat16)
-    q, k, v = rn(l), rn(lk), rn(lk)
-    o, lse = torch.full_like(q, 7.0), torch.full((1, h, l), 7.0, device="cuda")
-    need, words = C.c_size_t(0), C.c_int64(0)
-    L.check(L.lib().lact_swa_fwd_split_bytes(1, l, lk, h, d, window, C.byref(need), C.byref(words)), "split_bytes")
-    assert (need.value > 0) == (way == CUT) and words.value == 0
-    scratch = torch.zeros(max(need.value, 256), dtype=torch.uint8, device="cuda")
-    counters = torch.zeros(1, dtype=torch.int32, device="cuda")
-    status = torch.zeros(64, dtype=torch.int32, device="cuda")
-    status[0] = 101
-    call = lambda: L.check(L.lib().lact_swa_fwd_split(
-        q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), 1, l, lk, h, d, h * d, h * d * l, *[h * d, h * d * lk] * 2, h * d, h * d * l,
-        window, d ** -0.5, None, lse.data_ptr(), counters.data_ptr() if way == CUT else None, scratch.data_ptr() if way == CUT else None,
-        need.value, status.data_ptr(), L.stream_ptr()), "swa")
+    rn = lambda n: torch.randn(1, n, h, 128, device="cuda").to(torch.bfloat16)
+    call, o, lse, status = _prepared(rn(l), rn(lk), rn(lk), window, way == CUT, failed=True)
     assert _kernels(call) == way
     assert bool((o == 7).all()) and bool((lse == 7).all()) and int(status[0]) == 101
