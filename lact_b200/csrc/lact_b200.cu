@@ -609,18 +609,20 @@ int run_grad_pointwise(const GradArgs& a, int32_t* status, cudaStream_t stream) 
   return launch_gemm(g, stream, kClsGradPointwise);
 }
 
-// Whether an update of `len` tokens runs as one launch (grad_fused.cuh): by an estimate of both in us, each CTA's chain of tiles against the
-// rounds of the two launches (both give the same bits; sums that choose_split cuts stay cut).  Measured, us per call of five updates, two
-// launches / one: 12 entries of 128 x 256, 384 tokens each 136 / 107, 1560 235 / 199; 32 entries, chunks of 2048 476 / 393; 16 entries,
-// 4096 456 / 353.  Few CTAs with many tokens lose: one entry, 4096 130 / 176; 4 entries of 128 x 128, one update of 6000 97 / 112; so does a
-// short second round: 24 entries, 384 172 / 177.
+// Whether an update of `len` tokens runs as one launch (grad_fused.cuh): by an estimate of both in us (they give the same bits; sums that
+// choose_split cuts stay cut).  One launch: rounds of CTAs, two per pair of SMs, each with its chain of tiles; a last round of few CTAs takes as
+// long as a full one.  Two: tiles of both over the SMs and what the planes between them cost in memory.  Fitted to 645 gradients and 436
+// whole updates (1 to 96 entries, h = 128 to 512, 16 to 5632 tokens) timed both ways: in 26 the chosen way is more than 3 % slower, at most
+// 7 %.  Measured, us per gradient, two launches / one: 12 entries of 128 x 256, 384 tokens 17.1 / 12.6, 1560 30 / 23; 32 entries, 2048 70 / 48;
+// 16 entries, 4096 69 / 41.  Chains of few CTAs lose: one entry, 2048 tokens 21 / 25; so does a short last round: 20 entries, 780
+// tokens 26 / 29, 40 entries, 16 tokens 21 / 25.
 bool grad_in_one_launch(int64_t B, int64_t D, int64_t H, int64_t len) {
   if (D != kGradD || H % kBM != 0 || len < 1 || choose_split(ceil_div(len, kBK)).splits > 1) return false;
-  const double sms = sm_count(), rounds = B * (H / kGradSlice) / sms;
-  const int64_t tiles = ceil_div(len, 128);
-  const double one = std::max(1.0, rounds) * (1.15 * tiles + 5.0) + (rounds > 1.0 ? 3.5 : 0.0);
-  const double two = 5.0 + 2.0 * std::ceil(B * tiles * (H / 64) / sms) + std::ceil(B * (3 * H / kBM) / sms) * (0.6 * tiles + 4.0);
-  return 1.05 * one < two;
+  const int64_t sms = sm_count(), tiles = ceil_div(len, 128);
+  const double one = 4.0 + ceil_div(B * (H / kGradSlice), sms) * (0.97 * tiles + 5.9);
+  const double two = 11.8 + 1.03 * ceil_div(B * tiles * (H / 64), sms) + ceil_div(B * (3 * H / kBM), sms) * (0.27 * tiles + 1.9) +
+                     2.03 * (B * tiles * (H / 64)) / sms;
+  return one < two;
 }
 
 int run_grad_fused(const GradArgs& a, int32_t* status, cudaStream_t stream) {

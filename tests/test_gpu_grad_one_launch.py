@@ -144,3 +144,13 @@ def test_a_whole_update_with_more_ctas_than_sms(b, n, h):
 def test_the_way_of_one_entry(n, ways, h):
     w, qkv, lrs, _, _ = _inputs(1, n, h, torch.float32)
     assert _launches(lambda: _grads(w, qkv, lrs)) == ways
+
+
+# the faster way, both measured: chains in whole rounds of the SMs; a last round of few CTAs, few tokens per round, few CTAs
+@pytest.mark.parametrize("b,n,h,one", [(12, 384, 256, True), (12, 1560, 256, True), (18, 5632, 128, True), (16, 4096, 128, True), (37, 780, 512, True),
+                                       (37, 128, 256, True), (20, 16, 512, False), (40, 16, 256, False), (20, 16, 256, False), (40, 16, 128, False),
+                                       (19, 780, 256, False), (38, 780, 128, False), (40, 384, 512, False), (28, 384, 512, False),
+                                       (1, 2048, 256, False), (2, 1560, 256, False)])
+def test_the_faster_way(b, n, h, one):
+    w, qkv, lrs, _, _ = _inputs(b, n, h, torch.float32)
+    assert _launches(lambda: _grads(w, qkv, lrs)) == (["one"] if one else ["contract", "pointwise"])
