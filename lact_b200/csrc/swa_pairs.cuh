@@ -20,8 +20,8 @@
 // Code size counts: roles in 107 KB of code took 919 us, in 78 KB 836, in 67 KB 820 (a quarter of the stalls waits for
 // instructions), which is why rarely run loops are not unrolled and masks are applied in tensor memory.
 // Key and value tiles share one shared-memory layout ([128 rows][64 features] boxes, 128-byte swizzle): the first
-// product reads it K-major (features = k), the second MN-major (keys = k).  Every mbarrier wait is bounded;
-// no others are used.
+// product reads it K-major (features = k), the second MN-major (keys = k).  The roles wait for each
+// other at mbarriers alone, every wait with a limit.
 #pragma once
 #include <type_traits>
 #include "swa.cuh"
@@ -569,7 +569,7 @@ __global__ void __launch_bounds__(kSwaPairThreads, 1) swa_pairs_kernel(const __g
           if (t == lo) {
             if (!swa_wait(&q_full[g], parts++ & 1, abort_flag)) { failed = true; break; }
             // Groups that begin together come to their exponentials at the same time, then both to their products, and stay so: 4300 clocks
-            // per pair of tiles.  Half a tile apart, they alternate: 3500.
+            // per pair of tiles.  Half a tile apart, they alternate: 3500 (d = 128; tiles of d = 64, a fifth shorter, wait as long).
             if (g == 1 && lo == uniform(w.lo[0]) && hi - lo >= 4)
               for (const uint32_t begin = clock(); clock() - begin < 1700u;) __nanosleep(64);
           }
