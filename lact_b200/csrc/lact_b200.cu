@@ -2833,13 +2833,14 @@ struct SwaSplit {
   double us;
 };
 // Estimates of both attention forwards, which swa_takes_pairs compares.  An SM spends `tile` us per key tile and `item` per query tile or
-// pair, fitted to 255 shapes (32 to 32768 queries, windows of 100 to none, caches up to 16384 keys, d = 64 and 128) that were timed on both
-// kernels: the faster one is chosen in all but 3, within 1.18 there.
+// pair, a launch `launch`: fitted to 1722 random shapes (1 to 16 entries, 1 to 32 heads of 64 and 128, 32 to 16384 queries, windows of any
+// share, caches and blocks up to 16384 keys), each timed on single tiles, on pairs whole and on pairs cut in three ways, in replayed graphs, so that
+// small calls show what the device takes.  What is chosen is more than 5 % slower than the fastest way in 92, than single tiles in 9.
 struct SwaCost {
-  double tile, item;
+  double tile, item, launch;
 };
-static SwaCost swa_single_cost(int64_t d) { return d == 64 ? SwaCost{1.28, 4.9} : SwaCost{1.4, 6.7}; }
-static SwaCost swa_pair_cost(int64_t d) { return d == 64 ? SwaCost{1.75, 2.0} : SwaCost{2.1, 3.0}; }
+static SwaCost swa_single_cost(int64_t d) { return d == 64 ? SwaCost{1.19, 5.1, 1.05} : SwaCost{1.12, 6.4, 1.05}; }
+static SwaCost swa_pair_cost(int64_t d) { return d == 64 ? SwaCost{1.62, 1.63, 4.5} : SwaCost{1.87, 2.23, 4.5}; }
 // Causal attention: the first key tile that query tile i meets is i - swa_behind, or 0.
 static int64_t swa_band(int64_t l, int64_t window) { return window > 0 && window < l ? window : l; }
 static int64_t swa_behind(int64_t l, int64_t window) { return ceil_div(swa_band(l, window) - 1, 128); }
@@ -2850,7 +2851,7 @@ static SwaSplit swa_split(int64_t b, int64_t l, int64_t lk, int64_t heads, int64
   const int64_t T = ceil_div(span, 128), rest = tiles % sms;
   const double per_tile = d == 64 ? 1.2 : 1.5, round = T * per_tile + 4.0;
   // Whole tiles: rounds of equal ones; causal ones differ in length, are taken as SMs come free, and the last of them are the long ones of
-  // a head: an equal share of the work and 0.4 of the longest.
+  // a head: an equal share of the work and 0.45 of the longest; where the rest is cut, 0.57 of one of its pieces.
   const SwaCost cost = swa_single_cost(d);
   const double longest = T * cost.tile + cost.item;
   double share = 0.0;
@@ -2858,7 +2859,7 @@ static SwaSplit swa_split(int64_t b, int64_t l, int64_t lk, int64_t heads, int64
     const int64_t c = swa_behind(l, window), keys = n * (n + 1) / 2 - (n > c ? (n - c) * (n - c - 1) / 2 : 0);
     share = static_cast<double>(b * heads) * (keys * cost.tile + n * cost.item) / sms;
   }
-  SwaSplit best{tiles, 1, window < 0 || tiles <= sms ? ((tiles + sms - 1) / sms) * longest : std::max(longest, share + 0.4 * longest)};
+  SwaSplit best{tiles, 1, cost.launch + (window < 0 || tiles <= sms ? ((tiles + sms - 1) / sms) * longest : std::max(longest, share + 0.45 * longest))};
   if (!may_cut || rest == 0 || tiles > 64 * sms) return best;
   double end = round;   // of the rest
   for (int s = 2; s <= 16 && s <= T; ++s) {
@@ -2866,8 +2867,10 @@ static SwaSplit swa_split(int64_t b, int64_t l, int64_t lk, int64_t heads, int64
     const double c = turns * (keys * per_tile + 4.0) + 2.0 + 0.6 * s;
     if (c < 0.9 * end) {
       end = c;
-      const double us = turns * (keys * cost.tile + cost.item) + 2.0 + 0.6 * s;
-      best = SwaSplit{tiles - rest, s, tiles < sms ? us : window < 0 ? (tiles / sms) * longest + us : std::max(longest, share + 0.5 * us)};
+      const double piece = keys * cost.tile + cost.item, put = 2.4 + 0.57 * s;   // (and the pieces put together)
+      const double us = window < 0 || tiles < sms ? (tiles / sms) * longest + turns * piece + put
+                                                  : std::max(longest, share + rest * (s - 1) * cost.item / sms + 0.57 * piece + put);
+      best = SwaSplit{tiles - rest, s, cost.launch + us};
     }
   }
   return best;
@@ -2875,7 +2878,7 @@ static SwaSplit swa_split(int64_t b, int64_t l, int64_t lk, int64_t heads, int64
 
 // The same launch on pairs of query tiles (see SwaPairArgs).  Whole pairs fill whole rounds of the SMs; the rest, all pairs where there are
 // fewer than SMs, are cut over their keys if the longest CTA then ends sooner.  A second launch puts the pieces together: it, what it
-// waits for and the pieces' rows take 2 us and 0.08 per piece (60 pieces 6, 232 pieces 20).  Measured: 1560 queries over 4680 keys, 12
+// waits for and the pieces' rows take 6.9 us and 0.05 per piece.  Measured: 1560 queries over 4680 keys, 12
 // heads of 128 (84 pairs on 148 SMs, 38 key tiles each) whole 86, cut 73 us.  Pairs of causal attention without a window differ in length and
 // are dealt the long ones first: 8 heads of 8192 queries (256 pairs) are left whole, 134 us, 221 with the 108 shortest cut.
 struct SwaPairSplit {
@@ -2897,14 +2900,14 @@ static SwaPairSplit swa_pair_split(int64_t b, int64_t l, int64_t lk, int64_t hea
     return p * (p + 1) - (p > m ? (p - m) * (p + m - 1 - behind) : 0);
   };
   // The longest CTA's time for the first n items.  Where their lengths differ: up to eight rounds by those of five CTAs (the call waits for
-  // this), beyond by an equal share of the work and a quarter of the longest item.
+  // this), beyond by an equal share of the work and 0.27 of the longest item.
   auto dealt = [&](int64_t n) -> double {
     const int64_t rounds = (n + sms - 1) / sms;
     if (!causal || n <= sms) return rounds * longest;
     if (rounds > 8) {
       const int64_t full = n / bh, part = n % bh;
       const int64_t all = bh * (keys_before(pairs) - ceil_div(l, 128) % 2 - keys_before(pairs - full)) + (part > 0 ? part * keys(pairs - 1 - full) : 0);
-      return (all * cost.tile + n * cost.item) / sms + 0.25 * longest;
+      return (all * cost.tile + n * cost.item) / sms + 0.27 * longest;
     }
     double worst = 0.0;
     for (int64_t i = 0; i <= 4; ++i) {
@@ -2918,16 +2921,16 @@ static SwaPairSplit swa_pair_split(int64_t b, int64_t l, int64_t lk, int64_t hea
     }
     return worst;
   };
-  SwaPairSplit best{items, 0, 0, 0, dealt(items) + 2.0};
+  SwaPairSplit best{items, 0, 0, 0, dealt(items) + cost.launch};
   const int64_t rest = items % sms;
   if (!may_cut || rest == 0 || items > 64 * sms) return best;
-  const double before = dealt(items - rest) + 2 * cost.item + 4.0;
+  const double before = dealt(items - rest) + cost.launch + 6.9;
   for (int64_t s = 2, last = 0; s <= 16; s += 1 + s / 4) {
     const int64_t cutters = std::min(rest * std::min(s, span), sms);
     if (cutters == last) break;
     last = cutters;
-    const double us = before + ceil_div(rest * span, cutters) * cost.tile + 0.08 * (cutters + rest);
-    if (us < 0.95 * best.us) best = SwaPairSplit{items - rest, rest, cutters, span, us};
+    const double us = before + ceil_div(rest * span, cutters) * cost.tile + 0.05 * (cutters + rest);
+    if (us < best.us) best = SwaPairSplit{items - rest, rest, cutters, span, us};
   }
   return best;
 }
@@ -2939,11 +2942,11 @@ static size_t swa_pair_scratch(const SwaPairSplit& sp, int64_t d) {
 // Whether a launch runs on pairs: by the estimates of both.  Measured (us, single tiles / pairs; heads of 128 unless stated): 4 x 8192 queries,
 // 12 heads, no window 1084 / 769; 16 x 2048 392 / 246, of 64 325 / 184; 12 heads, 32768 queries of packed sequences of 256 under a window of
 // 2048 182 / 75, of 2048 387 / 317; 128 entries of 256 queries 176 / 73; 4096 queries, window 1024 57 / 46.  Few or uneven items lose: 12
-// heads of 1024 queries, window 256 12.6 / 15.8; 8 heads of 2305, window 2048 32 / 46; 4 heads of 8192 121 / 134; 8 of 64 with 777 queries
+// heads of 1024 queries, window 256 12.6 / 15.8; 24 of 64 with 121 queries 7.8 / 8.7; 24 with 768 over 132 keys 12 / 17; 8 heads of 2305, window 2048 32 / 46; 4 heads of 8192 121 / 134; 8 of 64 with 777 queries
 // over 2777 keys 28 / 30.  What a launch would not meet (sequences packed into its entry) is not looked at.
 static bool swa_takes_pairs(int64_t b, int64_t l, int64_t lk, int64_t heads, int64_t d, int64_t window, bool may_cut, SwaPairSplit* pairs) {
   *pairs = swa_pair_split(b, l, lk, heads, d, window, may_cut);
-  return pairs->us < 0.98 * swa_split(b, l, lk, heads, d, window, may_cut).us;   // (a tie: single tiles)
+  return pairs->us < swa_split(b, l, lk, heads, d, window, may_cut).us;
 }
 
 int lact_swa_fwd_split_bytes(int64_t b, int64_t l, int64_t lk, int64_t n_heads, int64_t d, int64_t window, size_t* bytes,

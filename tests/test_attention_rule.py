@@ -48,7 +48,7 @@ def _scratch(b, l, lk, h, d, window):
 # pairs, the last of them cut (the pieces take a second launch and no counters); single tiles, the last of them cut
 @pytest.mark.parametrize("b,l,lk,h,d,window,pairs", [(1, 1560, 4680, 12, 128, -1, True), (1, 1300, 4500, 30, 64, -1, True),
                                                      (1, 2600, 2500, 14, 128, -1, True), (2, 1900, 2600, 10, 64, -1, True),
-                                                     (1, 4680, 4681, 5, 128, -1, False), (1, 2305, 2305, 8, 128, 2048, False), (1, 100, 4581, 4, 128, -1, False),
+                                                     (1, 4680, 4681, 5, 128, -1, True), (1, 2305, 2305, 8, 128, 2048, False), (1, 100, 4581, 4, 128, -1, False),
                                                      (2, 300, 5384, 4, 64, -1, False), (1, 777, 2777, 8, 64, -1, False)])
 def test_what_is_cut(b, l, lk, h, d, window, pairs):
     need, words = _scratch(b, l, lk, h, d, window)

@@ -208,7 +208,7 @@ CUT = {"pairs", "combine"}
     (1, 1100, 1100, 40, 128, 0, (), PAIRS), (1, 257, 257, 74, 64, 200, (), PAIRS), (3, 130, 127, 30, 64, -1, (), PAIRS),
     (1, 900, 900, 100, 64, 0, (), PAIRS), (1, 1100, 1100, 60, 128, 300, (255, 257, 1000), PAIRS), (1, 300, 300, 200, 128, 0, (), PAIRS),
     (1, 2600, 2500, 14, 128, -1, (), CUT), (2, 1900, 2600, 10, 64, -1, (), CUT), (1, 5000, 5000, 2, 128, 0, (), CUT),
-    (1, 4100, 4100, 3, 128, 0, (1, 2, 383, 4099), CUT), (1, 3626, 3626, 3, 64, 0, (128, 1000, 3073), CUT), (1, 4100, 4100, 3, 64, 4096, (), CUT)])
+    (1, 5000, 5000, 2, 128, 0, (1, 2, 383, 4999), CUT), (1, 5000, 5000, 2, 64, 0, (128, 1000, 3073), CUT), (1, 7000, 7000, 2, 64, 5600, (), CUT)])
 def test_the_kernel_that_is_compared(b, l, lk, h, d, window, cuts, way):
     g = torch.Generator(device="cuda").manual_seed(l + h + d)
     rn = lambda n: torch.randn(b, n, h, d, device="cuda", generator=g).to(torch.bfloat16)
@@ -245,3 +245,15 @@ def test_pairs_after_an_earlier_failure(l, lk, h, window, way):
     call, o, lse, status = _prepared(rn(l), rn(lk), rn(lk), window, way == CUT, failed=True)
     assert _kernels(call) == way
     assert bool((o == 7).all()) and bool((lse == 7).all()) and int(status[0]) == 101
+
+
+# small calls, where a launch of pairs costs more than its rounds save; a launch of uneven items that single tiles cut; and others like them that pairs are
+# faster at (all measured both ways)
+@pytest.mark.parametrize("b,l,lk,h,d,window,way", [
+    (1, 121, 121, 24, 64, 0, "single"), (3, 128, 128, 16, 64, 12, "single"), (2, 239, 239, 3, 64, 0, "single"), (1, 128, 128, 4, 64, 64, "single"),
+    (1, 768, 132, 24, 128, -1, "single"), (1, 4736, 249, 1, 128, -1, "single"), (1, 648, 2912, 24, 64, -1, "single"), (1, 738, 738, 6, 64, 14, "single"),
+    (1, 6234, 6234, 3, 64, 5610, "single"), (1, 8192, 8192, 4, 128, 0, "single"),
+    (4, 5632, 96, 24, 64, -1, "pairs"), (8, 1485, 1485, 32, 128, 29, "pairs"), (3, 130, 127, 30, 64, -1, "pairs"), (1, 257, 257, 74, 64, 200, "pairs")])
+def test_the_faster_way_of_small_and_of_cut_calls(b, l, lk, h, d, window, way):
+    rn = lambda n: torch.randn(b, n, h, d, device="cuda").to(torch.bfloat16)
+    assert _kernels(_prepared(rn(l), rn(lk), rn(lk), window, True)[0]) == {way}
